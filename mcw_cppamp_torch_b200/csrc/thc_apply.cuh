@@ -2,9 +2,10 @@
 //
 // One functor, three data paths, picked on the host from the operands' strides:
 //   contiguous : float4 grid-stride streaming (the HBM-bound fast path)
-//   tiled 2-D  : operands whose unit-stride dimension differs from the output's (transposed views)
-//                are staged through 32x33 shared-memory tiles so that every global access stays
-//                coalesced; counts the same algorithmic bytes as the contiguous case
+//   tiled 2-D  : operands whose unit-stride dimension differs from the output's (transposed views):
+//                4 x 4 blocks transposed in registers where 16-byte accesses are possible, else
+//                64 x 64 shared-memory tiles, so that every global access stays coalesced; counts the
+//                same algorithmic bytes as the contiguous case
 //   strided    : anything else, collapsed dims + div/mod indexing (correct, not fast)
 // This replaces the reference pattern "newContiguous every operand, run, freeCopyTo the result"
 // (gputorch/lib/THC/THCTensorMath.cpp:67-163) and its per-element div/mod copy kernel
@@ -13,6 +14,8 @@
 #define THC_APPLY_CUH
 
 #include "thc_internal.h"
+
+#include <type_traits>
 
 namespace thc {
 
@@ -91,7 +94,7 @@ __global__ void __launch_bounds__(256) apply_contig_kernel(Operands<NIN> p, long
 struct StridedArgs {
   int nd;
   long size[kMaxDims];
-  long stride[3][kMaxDims];
+  long stride[4][kMaxDims];
 };
 
 template <typename Op, int NIN>
@@ -114,62 +117,131 @@ __global__ void __launch_bounds__(256) apply_strided_kernel(Operands<NIN> p, Str
   }
 }
 
-// 2-D index space (n0, n1); the output has unit stride along dim 1.  Inputs flagged in `via_smem`
-// have unit stride along dim 0 and are transposed through shared memory.  kTile2d x kTile2d tiles (32 or 64, chosen
-// by the caller): every global access of a warp is one contiguous 128-byte segment and a thread has
-// kTile2d * kTile2d / 256 independent loads per operand in flight.
-template <typename Op, int NIN, int kTile2d>
-__global__ void __launch_bounds__(256) apply_tiled2d_kernel(Operands<NIN> p, long n0, long n1,
-                                                            long os0, long is0_0, long is1_0,
-                                                            long is0_1, long is1_1, unsigned via_smem,
-                                                            long tiles1, long ntiles, Op op) {
-  extern __shared__ float tile2d_smem[];   // [NIN][kTile2d][kTile2d + 1]
-  const long is0[2] = {is0_0, is0_1}, is1[2] = {is1_0, is1_1};
-  constexpr int TY = 256 / kTile2d;
-  const int tx = threadIdx.x % kTile2d, ty = threadIdx.x / kTile2d;
-  for (long t = blockIdx.x; t < ntiles; t += gridDim.x) {
-    const long b0 = (t / tiles1) * kTile2d, b1 = (t % tiles1) * kTile2d;
+// Order in which the tiles of a transposing kernel are taken: strips of eight tiles along dim 0, inside a strip dim 0
+// fastest.  The blocks that run together then cover a wide rectangle, so that both the rows they write (along dim 1)
+// and the rows they read (transposed inputs, along dim 0) are runs of 2 KB and more instead of one 256-byte piece per
+// DRAM page.
+struct TileWalk {
+  unsigned tiles0, tiles1;
+  __host__ __device__ unsigned count() const { return tiles0 * tiles1; }
+  __device__ __forceinline__ void at(unsigned t, unsigned &t0, unsigned &t1) const {
+    constexpr unsigned G = 8;
+    const unsigned strip = t / (G * tiles1), r = t - strip * G * tiles1;
+    const unsigned h = tiles0 - strip * G < G ? tiles0 - strip * G : G;
+    t1 = r / h;
+    t0 = strip * G + (r - t1 * h);
+  }
+};
+// strides of a 2-D index space: [operand][dim], operand 0 is the output
+struct Strides2d {
+  int s[3][2];
+};
+
+// 2-D index space (n0, n1); the output has unit stride along dim 1.  Inputs flagged in VIA have unit stride along
+// dim 0 and are transposed through 64 x 64 shared-memory tiles: for sizes, pitches or addresses that 16-byte accesses
+// cannot serve.  Every global access of a warp is one contiguous 128-byte segment, eight per thread and operand in
+// flight.  Bound by instruction issue, not by memory, as long as each element pays for 64-bit address arithmetic and
+// bounds tests (58 instructions a warp access, half the issue slots, 3.5 TB/s on 3001 x 5003): hence 32-bit steps from one
+// pointer per tile and a path without tests for the tiles inside.
+template <typename Op, int NIN, unsigned VIA>   // VIA: bit k = operand k is transposed
+__global__ void __launch_bounds__(512, 3) apply_tiled2d_kernel(Operands<NIN> p, int n0, int n1, const Strides2d st,
+                                                                TileWalk walk, Op op) {
+  constexpr int T = 64, PITCH = T + 1, TY = 512 / T, NJ = T / TY;
+  extern __shared__ float tile2d_smem[];   // one [T][PITCH] tile per staged operand
+  const int tx = threadIdx.x % T, ty = threadIdx.x / T;
+  const unsigned ntiles = walk.count();
+  const int slot1 = (NIN > 1 && (VIA & 1u)) ? T * PITCH : 0;   // second staged operand
+  auto one_tile = [&](int b0, int b1, auto inside) {
+    constexpr bool INSIDE = decltype(inside)::value;
+    float direct[NIN > 1 ? NIN : 1][NIN > 1 ? NJ : 1];   // a single input is always the staged one
 #pragma unroll
     for (int k = 0; k < NIN; k++) {
-      if (via_smem & (1u << k)) {
-        float *tile = tile2d_smem + k * kTile2d * (kTile2d + 1);
-        const long i0 = b0 + tx;
+      if (VIA & (1u << k)) {   // rows of the tile run along dim 0
+        const float *src = p.in[k] + (b0 + tx) + (long)(b1 + ty) * st.s[k + 1][1];
+        const int step = TY * st.s[k + 1][1];
+        float *tile = tile2d_smem + (k ? slot1 : 0) + ty * PITCH + tx;
+        float v[NJ];
 #pragma unroll
-        for (int j = ty; j < kTile2d; j += TY) {
-          const long i1 = b1 + j;
-          if (i0 < n0 && i1 < n1) tile[j * (kTile2d + 1) + tx] = p.in[k][i0 * is0[k] + i1 * is1[k]];
-        }
+        for (int j = 0; j < NJ; j++) v[j] = (INSIDE || (b0 + tx < n0 && b1 + ty + j * TY < n1)) ? src[j * step] : 0.f;
+#pragma unroll
+        for (int j = 0; j < NJ; j++) tile[j * TY * PITCH] = v[j];
       }
     }
     // operands that need no transposition are fetched into registers BEFORE the barrier, so that their loads fly
     // together with the staged ones instead of starting after them
-    const long i1 = b1 + tx;
-    float direct[NIN > 1 ? NIN : 1][NIN > 1 ? kTile2d / TY : 1];   // a single input is always the staged one
 #pragma unroll
     for (int k = 0; k < (NIN > 1 ? NIN : 0); k++) {
-      if (!(via_smem & (1u << k))) {
+      if (!(VIA & (1u << k))) {
+        const float *src = p.in[k] + (long)(b0 + ty) * st.s[k + 1][0] + (long)(b1 + tx) * st.s[k + 1][1];
+        const int step = TY * st.s[k + 1][0];
 #pragma unroll
-        for (int jj = 0; jj < kTile2d / TY; jj++) {
-          const long i0 = b0 + ty + jj * TY;
-          direct[k][jj] = (i0 < n0 && i1 < n1) ? p.in[k][i0 * is0[k] + i1 * is1[k]] : 0.f;
-        }
+        for (int j = 0; j < NJ; j++) direct[k][j] = (INSIDE || (b0 + ty + j * TY < n0 && b1 + tx < n1)) ? src[j * step] : 0.f;
       }
     }
     __syncthreads();
+    float *dst = p.out + (long)(b0 + ty) * st.s[0][0] + (b1 + tx);
+    const int step = TY * st.s[0][0];
 #pragma unroll
-    for (int jj = 0; jj < kTile2d / TY; jj++) {
-      const int j = ty + jj * TY;
-      const long i0 = b0 + j;
-      if (i0 < n0 && i1 < n1) {
-        float a[NIN > 0 ? NIN : 1];
+    for (int j = 0; j < NJ; j++) {
+      float a[NIN];
 #pragma unroll
-        for (int k = 0; k < NIN; k++)
-          a[k] = (NIN == 1 || (via_smem & (1u << k))) ? tile2d_smem[k * kTile2d * (kTile2d + 1) + tx * (kTile2d + 1) + j]
-                                                      : direct[NIN > 1 ? k : 0][NIN > 1 ? jj : 0];
-        p.out[i0 * os0 + i1] = op(a);
-      }
+      for (int k = 0; k < NIN; k++)
+        a[k] = (VIA & (1u << k)) ? tile2d_smem[(k ? slot1 : 0) + tx * PITCH + ty + j * TY]
+                                                    : direct[NIN > 1 ? k : 0][NIN > 1 ? j : 0];
+      if (INSIDE || (b0 + ty + j * TY < n0 && b1 + tx < n1)) dst[j * step] = op(a);
     }
     __syncthreads();
+  };
+  for (unsigned t = blockIdx.x; t < ntiles; t += gridDim.x) {
+    unsigned t0, t1;
+    walk.at(t, t0, t1);
+    const int b0 = (int)t0 * T, b1 = (int)t1 * T;
+    if (b0 + T <= n0 && b1 + T <= n1) one_tile(b0, b1, std::true_type());
+    else one_tile(b0, b1, std::false_type());
+  }
+}
+
+// The same index space with 16-byte accesses on both sides and no shared memory: a thread owns a 4 x 4 block, reads a
+// transposed input as four 16-byte rows along dim 0, the others as four along dim 1, and transposes in registers.
+// A warp covers 16 (dim 0) x 32 (dim 1): transposed inputs arrive in whole 64-byte segments whose other half the
+// neighbouring warp of the block fetches, results leave in 128-byte segments.  No barrier, so loads of later
+// tiles fly under the stores of earlier ones.  n0, n1 and all pitches multiples of 4, 16-byte aligned bases.
+template <typename Op, int NIN, unsigned VIA>
+__global__ void __launch_bounds__(256) apply_transpose4_kernel(Operands<NIN> p, int n0, int n1, const Strides2d st, TileWalk walk,
+                                                               Op op) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int o0 = (warp & 3) * 16 + (lane & 3) * 4, o1 = (warp >> 2) * 32 + (lane >> 2) * 4;
+  const unsigned ntiles = walk.count();
+  for (unsigned t = blockIdx.x; t < ntiles; t += gridDim.x) {
+    unsigned t0, t1;
+    walk.at(t, t0, t1);
+    const int i0 = (int)t0 * 64 + o0, i1 = (int)t1 * 64 + o1;
+    if (i0 >= n0 || i1 >= n1) continue;
+    float v[NIN][4][4];   // [operand][row of the access][element]
+#pragma unroll
+    for (int k = 0; k < NIN; k++) {
+      const bool tr = (VIA & (1u << k)) != 0;
+      const int step = tr ? st.s[k + 1][1] : st.s[k + 1][0];
+      const float *b = p.in[k] + (tr ? (long)i1 * step + i0 : (long)i0 * step + i1);
+#pragma unroll
+      for (int r = 0; r < 4; r++) {
+        const float4 q = *reinterpret_cast<const float4 *>(b + r * step);
+        v[k][r][0] = q.x; v[k][r][1] = q.y; v[k][r][2] = q.z; v[k][r][3] = q.w;
+      }
+    }
+    float *dst = p.out + (long)i0 * st.s[0][0] + i1;
+#pragma unroll
+    for (int r = 0; r < 4; r++) {
+      float o[4];
+#pragma unroll
+      for (int c = 0; c < 4; c++) {
+        float a[NIN];
+#pragma unroll
+        for (int k = 0; k < NIN; k++) a[k] = ((VIA & (1u << k)) != 0) ? v[k][c][r] : v[k][r][c];
+        o[c] = op(a);
+      }
+      *reinterpret_cast<float4 *>(dst + r * st.s[0][0]) = make_float4(o[0], o[1], o[2], o[3]);
+    }
   }
 }
 
@@ -177,14 +249,14 @@ inline bool aligned16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 
 
 // out = op(in...) over tensors of equal shape (already resized by the caller); out may alias an input.
 template <int NIN, typename Op>
-void apply(THGPUTensor *out, const THGPUTensor *in0, const THGPUTensor *in1, Op op, const char *name) {
+void apply(THGPUTensor *out, const THGPUTensor *in0, const THGPUTensor *in1, Op op, const char *name,
+           const THGPUTensor *in2 = nullptr) {
   const long n = nelem(out);
   if (n == 0) return;
-  const THGPUTensor *ops[3] = {out, in0, in1};
+  const THGPUTensor *ops[4] = {out, in0, in1, in2};
   Operands<NIN> p;
   p.out = data_ptr(out);
-  if (NIN > 0) p.in[0] = data_ptr(in0);
-  if (NIN > 1) p.in[1] = data_ptr(in1);
+  for (int k = 0; k < NIN; k++) p.in[k] = data_ptr(ops[k + 1]);
   const int max_blocks = ctx().sm_count * 8;
   bool all_contig = is_contiguous(out);
   for (int k = 0; k < NIN; k++) all_contig = all_contig && is_contiguous(ops[k + 1]);
@@ -200,25 +272,41 @@ void apply(THGPUTensor *out, const THGPUTensor *in0, const THGPUTensor *in1, Op 
   }
   Strided s;
   THC_CHECK(collapse(NIN + 1, ops, s), "%s: too many non-collapsible dimensions", name);
-  if (s.nd == 2 && NIN > 0) {
-    // normalise so that the output's unit-stride dim is dim 1
-    int a = 0, b = 1;
-    if (s.stride[0][1] != 1 && s.stride[0][0] == 1) { a = 1; b = 0; }
-    if (s.stride[0][b] == 1) {
-      unsigned via = 0;
-      for (int k = 0; k < NIN; k++)
-        if (s.stride[k + 1][a] == 1 && s.stride[k + 1][b] != 1) via |= 1u << k;
-      if (via) {
+  if constexpr (NIN == 1 || NIN == 2) {
+    if (s.nd == 2) {
+      // normalise so that the output's unit-stride dim is dim 1
+      int a = 0, b = 1;
+      if (s.stride[0][1] != 1 && s.stride[0][0] == 1) { a = 1; b = 0; }
+      if (s.stride[0][b] == 1) {
+        unsigned via = 0;
+        for (int k = 0; k < NIN; k++)
+          if (s.stride[k + 1][a] == 1 && s.stride[k + 1][b] != 1) via |= 1u << k;
+        bool fits = s.size[0] < (1l << 30) && s.size[1] < (1l << 30);   // 32-bit steps inside a tile
+        for (int k = 0; k <= NIN; k++) fits = fits && s.stride[k][0] < (1l << 24) && s.stride[k][1] < (1l << 24);
         const long n0 = s.size[a], n1 = s.size[b];
-        constexpr int kTile2d = 64;   // 32 x 32 tiles measured the same for one input (0.63 / 0.64 of the HBM rate) and worse for two
-        const long tiles0 = (n0 + kTile2d - 1) / kTile2d, tiles1 = (n1 + kTile2d - 1) / kTile2d, ntiles = tiles0 * tiles1;
-        int blocks = (int)(ntiles < max_blocks ? ntiles : max_blocks);
-        const size_t smem = (NIN > 0 ? NIN : 1) * kTile2d * (kTile2d + 1) * sizeof(float);
-        apply_tiled2d_kernel<Op, NIN, kTile2d><<<blocks, 256, smem, stream()>>>(
-            p, n0, n1, s.stride[0][a], s.stride[1][a], s.stride[1][b], NIN > 1 ? s.stride[2][a] : 0,
-            NIN > 1 ? s.stride[2][b] : 0, via, tiles1, ntiles, op);
-        check_launch(name);
-        return;
+        const long tiles0 = (n0 + 63) / 64, tiles1 = (n1 + 63) / 64;
+        if (via && fits && tiles0 * tiles1 < (1l << 30)) {
+          const TileWalk walk{(unsigned)tiles0, (unsigned)tiles1};
+          const unsigned blocks = std::min(walk.count(), (unsigned)max_blocks);
+          Strides2d st = {};
+          for (int k = 0; k <= NIN; k++) { st.s[k][0] = (int)s.stride[k][a]; st.s[k][1] = (int)s.stride[k][b]; }
+          // 16-byte accesses on every operand: pitches and extents multiples of 4, aligned bases
+          bool vec = aligned16(p.out) && n0 % 4 == 0 && n1 % 4 == 0 && st.s[0][0] % 4 == 0;
+          for (int k = 0; k < NIN; k++)
+            vec = vec && aligned16(p.in[k]) && ((via >> k & 1u) ? st.s[k + 1][1] % 4 == 0 : st.s[k + 1][1] == 1 && st.s[k + 1][0] % 4 == 0);
+          if (vec) {
+            if (NIN == 1 || via == 1u) apply_transpose4_kernel<Op, NIN, 1u><<<blocks, 256, 0, stream()>>>(p, (int)n0, (int)n1, st, walk, op);
+            else if (via == 2u) apply_transpose4_kernel<Op, NIN, NIN == 2 ? 2u : 1u><<<blocks, 256, 0, stream()>>>(p, (int)n0, (int)n1, st, walk, op);
+            else apply_transpose4_kernel<Op, NIN, NIN == 2 ? 3u : 1u><<<blocks, 256, 0, stream()>>>(p, (int)n0, (int)n1, st, walk, op);
+          } else {
+            const size_t smem = (via == 3u ? 2 : 1) * 64 * 65 * sizeof(float);
+            if (NIN == 1 || via == 1u) apply_tiled2d_kernel<Op, NIN, 1u><<<blocks, 512, smem, stream()>>>(p, (int)n0, (int)n1, st, walk, op);
+            else if (via == 2u) apply_tiled2d_kernel<Op, NIN, NIN == 2 ? 2u : 1u><<<blocks, 512, smem, stream()>>>(p, (int)n0, (int)n1, st, walk, op);
+            else apply_tiled2d_kernel<Op, NIN, NIN == 2 ? 3u : 1u><<<blocks, 512, smem, stream()>>>(p, (int)n0, (int)n1, st, walk, op);
+          }
+          check_launch(name);
+          return;
+        }
       }
     }
   }
@@ -226,7 +314,7 @@ void apply(THGPUTensor *out, const THGPUTensor *in0, const THGPUTensor *in1, Op 
   sa.nd = s.nd;
   for (int d = 0; d < kMaxDims; d++) {
     sa.size[d] = d < s.nd ? s.size[d] : 1;
-    for (int k = 0; k < 3; k++) sa.stride[k][d] = d < s.nd ? s.stride[k][d] : 0;
+    for (int k = 0; k < 4; k++) sa.stride[k][d] = d < s.nd ? s.stride[k][d] : 0;
   }
   int blocks = (int)((n + 255) / 256);
   if (blocks > max_blocks) blocks = max_blocks;

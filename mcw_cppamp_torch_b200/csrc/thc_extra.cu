@@ -30,10 +30,10 @@ __global__ void __launch_bounds__(256) prod_partial_kernel(const float *__restri
     partial[blockIdx.x] = acc;
   }
 }
-__global__ void prod_finish_kernel(const double *__restrict__ partial, int n, double *result) {
+__global__ void prod_finish_kernel(const double *__restrict__ partial, int n, ScalarSlot *slot, unsigned long long seq) {
   double acc = 1.0;
   for (int i = 0; i < n; i++) acc *= partial[i];
-  *result = acc;
+  scalar_deliver(slot, acc, seq);
 }
 // src viewed as [outer][R][inner] (contiguous): out[o][i] = prod_r src[o][r][i].  inner > 1: one thread per output,
 // neighbouring threads read neighbouring addresses.
@@ -176,17 +176,15 @@ THC_API float THGPUTensor_prodall(THGPUTensor *self) {
   THC_ARG(n > 0, 1, "empty tensor");
   WsScope ws_scope;
   TensorRef c(tensor_new_contiguous(self));
-  double *partial = (double *)ws_alloc(sizeof(double) * (kProdBlocks + 1));
+  double *partial = (double *)ws_alloc(sizeof(double) * kProdBlocks);
   int blocks = (int)((n + 255) / 256);
   if (blocks > kProdBlocks) blocks = kProdBlocks;
   prod_partial_kernel<<<blocks, 256, 0, stream()>>>(data_ptr(c), n, partial);
   check_launch("prod_partial");
-  prod_finish_kernel<<<1, 1, 0, stream()>>>(partial, blocks, partial + kProdBlocks);
+  const unsigned long long seq = scalar_expect();
+  prod_finish_kernel<<<1, 1, 0, stream()>>>(partial, blocks, ctx().scalar_slot_dev, seq);
   check_launch("prod_finish");
-  double *host = (double *)ctx().host_pinned;
-  THC_CUDA(cudaMemcpyAsync(host, partial + kProdBlocks, sizeof(double), cudaMemcpyDeviceToHost, stream()));
-  sync_stream();
-  return (float)*host;
+  return (float)scalar_wait(seq);
   THC_END(0.f)
 }
 

@@ -3,6 +3,7 @@
 // empty device stubs of gputorch/init.cpp:10-66 with real CUDA device management.
 #include "thc_internal.h"
 
+#include <atomic>
 #include <cstring>
 #include <map>
 #include <mutex>
@@ -70,7 +71,13 @@ static void init_device(Context &c, int device) {
       g_pool_ready[device] = true;
     }
   }
-  if (!c.host_pinned) THC_CUDA(cudaMallocHost((void **)&c.host_pinned, 64));
+  if (!c.scalar_slot) {
+    THC_CUDA(cudaHostAlloc((void **)&c.scalar_slot, sizeof(ScalarSlot), cudaHostAllocMapped | cudaHostAllocPortable));
+    c.scalar_slot->seq = 0;
+    THC_CUDA(cudaHostAlloc((void **)&c.small_stage, sizeof(float) * kSmallStage, cudaHostAllocMapped | cudaHostAllocPortable));
+  }
+  THC_CUDA(cudaHostGetDevicePointer((void **)&c.small_stage_dev, c.small_stage, 0));
+  THC_CUDA(cudaHostGetDevicePointer((void **)&c.scalar_slot_dev, c.scalar_slot, 0));
   if (!c.stall_host) {
     THC_CUDA(cudaHostAlloc((void **)&c.stall_host, sizeof(int), cudaHostAllocMapped | cudaHostAllocPortable));
     *c.stall_host = 0;
@@ -146,6 +153,28 @@ void check_stall() {
 void sync_stream() {
   THC_CUDA(cudaStreamSynchronize(stream()));
   check_stall();
+}
+
+unsigned long long scalar_expect() { return ++ctx().scalar_seq; }
+
+double scalar_wait(unsigned long long seq) {
+  Context &c = ctx();
+  volatile ScalarSlot *slot = c.scalar_slot;
+  for (unsigned polls = 1; slot->seq != seq; polls++) {
+    if ((polls & 4095) == 0) {   // a failed launch never delivers: ask the stream now and then
+      const cudaError_t e = cudaStreamQuery(c.stream);
+      if (e == cudaErrorNotReady) continue;
+      THC_CUDA(e);
+      THC_CHECK(slot->seq == seq, "internal: a scalar result was not delivered");
+    }
+#if defined(__x86_64__)
+    __builtin_ia32_pause();
+#endif
+  }
+  std::atomic_thread_fence(std::memory_order_acquire);
+  const double v = slot->value;
+  check_stall();
+  return v;
 }
 int device_if_initialised() { return g_ctx.device; }
 

@@ -3,6 +3,7 @@
 #define THC_INTERNAL_H
 
 #include <cuda_runtime.h>
+#include <algorithm>
 #include <cstdarg>
 #include <cstdint>
 #include <cstdio>
@@ -43,6 +44,15 @@ struct StallCtl {
 };
 }  // namespace mm
 
+// Scalar results (sums, maxima, single elements) travel to the host through one mapped pinned record: the kernel
+// writes the value, then the sequence number the host polls for (scalar_expect / scalar_wait).
+struct ScalarSlot {
+  double value;
+  unsigned long long seq;
+};
+
+constexpr long kSmallStage = 16384;
+
 struct Context {
   int device = -1;            // current device of this host thread, -1 = not yet initialised
   cudaStream_t stream = nullptr;
@@ -53,7 +63,11 @@ struct Context {
   // small device scratch reused by reductions and the GEMM error flag (lazy, per device)
   void *scratch = nullptr;
   size_t scratch_bytes = 0;
-  float *host_pinned = nullptr;  // 64 B pinned staging for scalar results
+  ScalarSlot *scalar_slot = nullptr;      // mapped pinned host record
+  ScalarSlot *scalar_slot_dev = nullptr;  // its device alias
+  float *small_stage = nullptr;           // kSmallStage floats of mapped pinned memory behind small downloads
+  float *small_stage_dev = nullptr;
+  unsigned long long scalar_seq = 0;      // number of the last scalar asked for
   // stall flags of the tensor-core kernels (see mm::StallCtl)
   int *stall_host = nullptr;      // mapped pinned host word
   int *stall_host_dev = nullptr;  // its device alias
@@ -79,6 +93,19 @@ cudaStream_t stream();
 // Every entry point that hands results to the host synchronises through this.
 void sync_stream();
 void check_stall();               // the check alone, for callers that have just synchronised themselves
+// The next scalar's sequence number, for a kernel that ends in scalar_deliver(ctx().scalar_slot_dev, value, number);
+// scalar_wait returns the value once the number has arrived (or fails with the stream's error).  Everything queued
+// on the stream before that kernel is then complete too, and a pipeline stall is reported as by sync_stream.
+unsigned long long scalar_expect();
+double scalar_wait(unsigned long long seq);
+#ifdef __CUDACC__
+__device__ __forceinline__ void scalar_deliver(ScalarSlot *slot, double v, unsigned long long seq) {
+  volatile ScalarSlot *s = slot;
+  s->value = v;
+  __threadfence_system();
+  s->seq = seq;
+}
+#endif
 mm::StallCtl stall_ctl();         // kernel parameter of the tensor-core kernels
 // A zeroed device word for one persistent launch to hand out its work items from.  The words come from a block of
 // 4096 that is cleared on the stream each time it has been used up (the launches that used it are ahead of the
@@ -139,13 +166,13 @@ struct TensorRef {
   THGPUTensor *operator->() const { return t; }
 };
 
-// Collapsed strided description of up to 3 operands over one index space (used by the generic
+// Collapsed strided description of up to 4 operands over one index space (used by the generic
 // elementwise / copy kernels).  dims are merged wherever every operand allows it.
 constexpr int kMaxDims = 8;
 struct Strided {
   int nd;
   long size[kMaxDims];
-  long stride[3][kMaxDims];
+  long stride[4][kMaxDims];
 };
 // Builds the description for operands that all have nelem equal; returns false if more than
 // kMaxDims dims remain after collapsing.

@@ -6,7 +6,7 @@
 // double (TH's accreal), max/min use strict comparisons so the first extremum wins.
 #include <cfloat>
 
-#include "thc_apply.cuh"
+#include "thc_reduce.cuh"
 
 namespace thc {
 
@@ -22,115 +22,8 @@ struct CdivOp { __device__ float operator()(const float *a) const { return a[0] 
 
 static void resize_as(THGPUTensor *r, const THGPUTensor *t) { tensor_resize_as(r, t); }
 
-// ------------------------------------------------------------------ full reductions
-// Pass 1: every block reduces a grid-strided slice (fp32 runs of 4 folded into a double
-// accumulator per thread), writes one partial; the last block to finish (atomic ticket) folds the
-// partials in fixed order, so the result is deterministic.  No block ever waits on another.
-enum { RED_SUM = 0, RED_MAX = 1, RED_MIN = 2, RED_DOT = 3 };
-
-struct RedScratch {
-  double partial[1024];
-  unsigned int ticket;
-  unsigned int pad;
-  double result;
-};
-
-template <int MODE> struct RedTraits;
-template <> struct RedTraits<RED_SUM> {
-  __device__ static double init(float) { return 0.0; }
-  __device__ static double fold4(float4 v) { return (double)((v.x + v.y) + (v.z + v.w)); }
-  __device__ static double one(float v) { return (double)v; }
-  __device__ static double comb(double a, double b) { return a + b; }
-};
-template <> struct RedTraits<RED_MAX> {
-  __device__ static double init(float first) { return (double)first; }
-  __device__ static double fold4(float4 v) { return (double)fmaxf(fmaxf(v.x, v.y), fmaxf(v.z, v.w)); }
-  __device__ static double one(float v) { return (double)v; }
-  __device__ static double comb(double a, double b) { return a > b ? a : b; }
-};
-template <> struct RedTraits<RED_MIN> {
-  __device__ static double init(float first) { return (double)first; }
-  __device__ static double fold4(float4 v) { return (double)fminf(fminf(v.x, v.y), fminf(v.z, v.w)); }
-  __device__ static double one(float v) { return (double)v; }
-  __device__ static double comb(double a, double b) { return a < b ? a : b; }
-};
-
-template <int MODE>
-__device__ __forceinline__ double block_reduce(double v, double *smem) {
-  typedef RedTraits<MODE> T;
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v = T::comb(v, __shfl_xor_sync(0xffffffffu, v, o));
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
-  if (lane == 0) smem[warp] = v;
-  __syncthreads();
-  if (warp == 0) {
-    // lanes beyond the warp count re-use entry 0 for max/min (idempotent) and contribute 0 to sums
-    v = lane < nwarps ? smem[lane] : (MODE == RED_SUM ? 0.0 : smem[0]);
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v = T::comb(v, __shfl_xor_sync(0xffffffffu, v, o));
-  }
-  __syncthreads();
-  return v;  // valid in warp 0
-}
-
-template <int MODE>
-__global__ void __launch_bounds__(512) reduce_all_kernel(const float *__restrict__ x, const float *__restrict__ y,
-                                                         long n, bool vec, RedScratch *s) {
-  typedef RedTraits<MODE == RED_DOT ? RED_SUM : MODE> T;
-  __shared__ double smem[32];
-  __shared__ bool is_last;
-  const long tid = (long)blockIdx.x * blockDim.x + threadIdx.x, nthreads = (long)gridDim.x * blockDim.x;
-  double acc = T::init(x[0]);
-  long done = 0;
-  if (vec) {
-    const long nvec = n >> 2;
-    const float4 *x4 = reinterpret_cast<const float4 *>(x);
-    const float4 *y4 = reinterpret_cast<const float4 *>(y);
-    long i = tid;
-    if (MODE != RED_DOT) {  // four independent 16-byte loads per thread in flight
-      for (; i + 3 * nthreads < nvec; i += 4 * nthreads) {
-        const float4 v0 = x4[i], v1 = x4[i + nthreads], v2 = x4[i + 2 * nthreads], v3 = x4[i + 3 * nthreads];
-        acc = T::comb(acc, T::comb(T::comb(T::fold4(v0), T::fold4(v1)), T::comb(T::fold4(v2), T::fold4(v3))));
-      }
-    }
-    for (; i < nvec; i += nthreads) {
-      float4 v = x4[i];
-      if (MODE == RED_DOT) {
-        const float4 w = y4[i];
-        // products are exact in double; keeps the dot product faithful to a double accumulator
-        acc += (double)v.x * w.x + (double)v.y * w.y + (double)v.z * w.z + (double)v.w * w.w;
-      } else
-        acc = T::comb(acc, T::fold4(v));
-    }
-    done = nvec << 2;
-  }
-  for (long i = done + tid; i < n; i += nthreads) {
-    if (MODE == RED_DOT) acc += (double)x[i] * y[i];
-    else acc = T::comb(acc, T::one(x[i]));
-  }
-  acc = block_reduce<(MODE == RED_DOT ? RED_SUM : MODE)>(acc, smem);
-  if (threadIdx.x == 0) {
-    s->partial[blockIdx.x] = acc;
-    __threadfence();
-    const unsigned int t = atomicAdd(&s->ticket, 1u);
-    is_last = (t == gridDim.x - 1);
-  }
-  __syncthreads();
-  if (is_last) {
-    __threadfence();
-    double v = T::init(x[0]);
-    for (int i = threadIdx.x; i < (int)gridDim.x; i += blockDim.x) v = T::comb(v, ((volatile double *)s->partial)[i]);
-    v = block_reduce<(MODE == RED_DOT ? RED_SUM : MODE)>(v, smem);
-    if (threadIdx.x == 0) {
-      s->result = v;
-      s->ticket = 0;  // ready for the next launch on this stream
-    }
-  }
-}
-
-// A tensor whose elements occupy one gap-free block of memory in some dim order (contiguous, or a
-// transposed / permuted view of a contiguous block): order-free reductions can run over the block.
-static bool is_dense_block(const THGPUTensor *t) {
+// ------------------------------------------------------------------ full reductions (thc_reduce.cuh)
+bool is_dense_block(const THGPUTensor *t) {
   int order[kMaxDims * 4];
   int nd = 0;
   for (int d = 0; d < t->nDimension; d++)
@@ -147,52 +40,19 @@ static bool is_dense_block(const THGPUTensor *t) {
   return true;
 }
 
-static bool same_layout(const THGPUTensor *a, const THGPUTensor *b) {
+bool same_layout(const THGPUTensor *a, const THGPUTensor *b) {
   if (a->nDimension != b->nDimension) return false;
   for (int d = 0; d < a->nDimension; d++)
     if (a->size[d] != b->size[d] || (a->size[d] != 1 && a->stride[d] != b->stride[d])) return false;
   return true;
 }
 
-template <int MODE>
-static double reduce_all(THGPUTensor *t, THGPUTensor *u) {
-  const long n = nelem(t);
-  THC_ARG(n > 0, 1, "tensor must have one dimension");
-  THGPUTensor *tc = nullptr, *uc = nullptr;
-  const float *x, *y = nullptr;
-  if (MODE == RED_DOT) {
-    THC_ARG(nelem(u) == n, 2, "sizes do not match");
-    if (is_dense_block(t) && same_layout(t, u)) { x = data_ptr(t); y = data_ptr(u); }
-    else { tc = tensor_new_contiguous(t); uc = tensor_new_contiguous(u); x = data_ptr(tc); y = data_ptr(uc); }
-  } else {
-    if (is_dense_block(t)) x = data_ptr(t);
-    else { tc = tensor_new_contiguous(t); x = data_ptr(tc); }
-  }
-  Context &c = ctx();
-  RedScratch *s = (RedScratch *)scratch(sizeof(RedScratch));
-  // the ticket starts at 0 (scratch is zero-filled when allocated); each launch resets it
-  const bool vec = aligned16(x) && (MODE != RED_DOT || aligned16(y));
-  long work = vec ? (n + 3) / 4 : n;
-  int blocks = (int)((work + 511) / 512);
-  int cap = c.sm_count * 4;   // 4 blocks of 512 threads per SM = full occupancy
-  if (cap > 1024) cap = 1024;
-  if (blocks > cap) blocks = cap;
-  reduce_all_kernel<MODE><<<blocks, 512, 0, stream()>>>(x, y, n, vec, s);
-  check_launch("reduce_all");
-  double *host = (double *)c.host_pinned;
-  THC_CUDA(cudaMemcpyAsync(host, &s->result, sizeof(double), cudaMemcpyDeviceToHost, stream()));
-  sync_stream();
-  if (tc) tensor_free(tc);
-  if (uc) tensor_free(uc);
-  return *host;
-}
-
 // ------------------------------------------------------------------ dim-wise reductions
 // The source is described as out(o, j) <- reduce_r src[base + o*so + j*sj + r*sr].
-//   row kernel   : sr == 1 (reduced dim is the unit-stride one).  One block per output.
-//   column kernel: sj == 1 (outputs are unit-stride neighbours).  Threads own 1 column each, the
-//                  reduced dim is additionally split over threadIdx.y and blockIdx.y; a second tiny
-//                  kernel folds the blockIdx.y partials in ascending order.
+//   row kernel   : sr == 1 (reduced dim is the unit-stride one).  One block per output, or one warp.
+//   column kernel: sj == 1 (outputs are unit-stride neighbours).  Threads own 1 or 4 columns each, the
+//                  reduced dim is additionally split over threadIdx.y and blockIdx.y; the last block of a
+//                  column range folds the blockIdx.y partials in ascending order.
 template <int MODE, class I = long> __device__ __forceinline__ bool better(float a, I ia, float b, I ib) {
   // true when (a, ia) should replace (b, ib): strictly better value, or equal value at a lower index
   if (MODE == RED_MAX) return a > b || (a == b && ia < ib);
@@ -292,95 +152,218 @@ __global__ void __launch_bounds__(256) reduce_rows_kernel(const float *__restric
   }
 }
 
-// grid (ceil(J/32), splits, O); block (32, 8).  Partials: [O][splits][J].
+// Rows of a few hundred elements: a warp per row, eight rows per block (a block per row would leave most of its
+// threads, or most of the SM's block slots, without work).
 template <int MODE>
-__global__ void __launch_bounds__(256) reduce_cols_kernel(const float *__restrict__ src, long so, long sr, long J,
-                                                          long R, long rows_per_split, double *__restrict__ psum,
-                                                          float *__restrict__ pval, long *__restrict__ pidx) {
+__global__ void __launch_bounds__(256) reduce_rows_warp_kernel(const float *__restrict__ src, long so, long J, int R,
+                                                               float *__restrict__ out, float *__restrict__ idx, float scale) {
+  const long j = (long)blockIdx.x * 8 + (threadIdx.x >> 5);
+  if (j >= J) return;
+  const int lane = threadIdx.x & 31;
+  const float *row = src + j * so;
+  if (MODE == RED_SUM) {
+    double acc = 0;
+    int i = lane;
+    for (; i + 96 < R; i += 128) {
+      const float v0 = row[i], v1 = row[i + 32], v2 = row[i + 64], v3 = row[i + 96];
+      acc += (double)v0 + (double)v1 + (double)v2 + (double)v3;
+    }
+    for (; i < R; i += 32) acc += (double)row[i];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+    if (lane == 0) out[j] = (float)(acc * (double)scale);
+  } else {
+    float bv = row[0];
+    int bi = 0;
+#pragma unroll 4
+    for (int i = lane; i < R; i += 32) {
+      const float v = row[i];
+      if (better<MODE, int>(v, i, bv, bi)) { bv = v; bi = i; }
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      const float ov = __shfl_xor_sync(0xffffffffu, bv, o);
+      const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
+      if (better<MODE, int>(ov, oi, bv, bi)) { bv = ov; bi = oi; }
+    }
+    if (lane == 0) {
+      out[j] = bv;
+      if (idx) idx[j] = (float)(bi + 1);
+    }
+  }
+}
+
+// Where a column reduction leaves its results.  With more than one slice of the reduced dimension the partials of
+// slice s go to psum / (pval, pidx)[(o * splits + s) * J + j], and the block that finishes last among the slices of its
+// columns (tickets[o * gridDim.x + blockIdx.x], zero between launches) folds them in slice order: no second launch.
+struct ColOut {
+  double *psum;
+  float *pval;
+  int *pidx;
+  unsigned *tickets;
+  float *out, *idx;
+  float scale;
+};
+template <int MODE>
+__device__ __forceinline__ void cols_emit(const ColOut &w, long t, double acc, float v, int i) {
+  if (MODE == RED_SUM) {
+    w.out[t] = (float)(acc * (double)w.scale);
+  } else {
+    w.out[t] = v;
+    if (w.idx) w.idx[t] = (float)(i + 1);
+  }
+}
+// Called by all threads of the block once its partials are written; COLS columns from j0 on belong to the block.
+template <int MODE, int COLS>
+__device__ __forceinline__ void cols_fold_if_last(const ColOut &w, long J, long j0) {
+  __shared__ bool is_last;
+  const int tid = threadIdx.y * 32 + threadIdx.x, splits = gridDim.y;
+  __threadfence();
+  __syncthreads();
+  if (tid == 0) {
+    unsigned *ticket = w.tickets + (long)blockIdx.z * gridDim.x + blockIdx.x;
+    is_last = atomicAdd(ticket, 1u) == (unsigned)splits - 1;
+    if (is_last) *ticket = 0;   // ready for the next launch on this stream
+  }
+  __syncthreads();
+  if (!is_last) return;
+  __threadfence();
+  // `COLS` columns, 256 / COLS interleaved groups of slices per column, folded in group order
+  __shared__ double fd[256];
+  __shared__ float fv[256];
+  __shared__ int fi[256];
+  const int c = tid % COLS, grp = tid / COLS;
+  constexpr int GROUPS = 256 / COLS;
+  const long j = j0 + c, first = (long)blockIdx.z * splits * J + j;
+  double acc = 0;
+  float bv = 0;
+  int bi = -1;
+  if (j < J) {
+    if (MODE == RED_SUM) {
+#pragma unroll 8
+      for (int s = grp; s < splits; s += GROUPS) acc += __ldcg(w.psum + first + (long)s * J);
+    } else {
+      for (int s0 = grp; s0 < splits; s0 += 8 * GROUPS) {
+        float ov[8];
+        int oi[8];
+#pragma unroll
+        for (int u = 0; u < 8; u++) {
+          const int s = s0 + u * GROUPS;
+          ov[u] = s < splits ? __ldcg(w.pval + first + (long)s * J) : 0.f;
+          oi[u] = s < splits ? __ldcg(w.pidx + first + (long)s * J) : -1;
+        }
+#pragma unroll
+        for (int u = 0; u < 8; u++)
+          if (oi[u] >= 0 && (bi < 0 || better<MODE, int>(ov[u], oi[u], bv, bi))) { bv = ov[u]; bi = oi[u]; }
+      }
+    }
+  }
+  if (MODE == RED_SUM) fd[tid] = acc;
+  else { fv[tid] = bv; fi[tid] = bi; }
+  __syncthreads();
+  if (grp == 0 && j < J) {
+    for (int k = 1; k < GROUPS; k++) {
+      if (MODE == RED_SUM) {
+        acc += fd[k * COLS + c];
+      } else {
+        const float ov = fv[k * COLS + c];
+        const int oi = fi[k * COLS + c];
+        if (oi >= 0 && (bi < 0 || better<MODE, int>(ov, oi, bv, bi))) { bv = ov; bi = oi; }
+      }
+    }
+    cols_emit<MODE>(w, (long)blockIdx.z * J + j, acc, bv, bi);
+  }
+}
+
+// grid (ceil(J/32), splits, O); block (32, 8).
+template <int MODE>
+__global__ void __launch_bounds__(256) reduce_cols_kernel(const float *__restrict__ src, long so, long sr, long J, int R,
+                                                          int rows_per_split, const ColOut w) {
   __shared__ double sd[8][33];
   __shared__ float sv[8][33];
-  __shared__ long si[8][33];
+  __shared__ int si[8][33];
   const long j = (long)blockIdx.x * 32 + threadIdx.x;
-  const long r0 = (long)blockIdx.y * rows_per_split;
-  long r1 = r0 + rows_per_split;
-  if (r1 > R) r1 = R;
+  const int r0 = blockIdx.y * rows_per_split, r1 = min(R, r0 + rows_per_split);
   const float *base = src + (long)blockIdx.z * so + j;
   double acc = 0;
   float bv = 0;
-  long bi = -1;
+  int bi = -1;
   if (j < J) {
-    long r = r0 + threadIdx.y;
-    for (; r + 24 < r1; r += 32) {  // four independent loads in flight per thread
-      const float v0 = base[r * sr], v1 = base[(r + 8) * sr], v2 = base[(r + 16) * sr], v3 = base[(r + 24) * sr];
-      if (MODE == RED_SUM) acc += ((double)v0 + (double)v1) + ((double)v2 + (double)v3);
-      else {
-        if (bi < 0 || better<MODE>(v0, r, bv, bi)) { bv = v0; bi = r; }
-        if (better<MODE>(v1, r + 8, bv, bi)) { bv = v1; bi = r + 8; }
-        if (better<MODE>(v2, r + 16, bv, bi)) { bv = v2; bi = r + 16; }
-        if (better<MODE>(v3, r + 24, bv, bi)) { bv = v3; bi = r + 24; }
+    int r = r0 + threadIdx.y;
+    for (; r + 56 < r1; r += 64) {  // eight independent loads in flight per thread
+      float v[8];
+#pragma unroll
+      for (int u = 0; u < 8; u++) v[u] = base[(long)(r + 8 * u) * sr];
+      if (MODE == RED_SUM) {
+        acc += (((double)v[0] + (double)v[1]) + ((double)v[2] + (double)v[3])) + (((double)v[4] + (double)v[5]) + ((double)v[6] + (double)v[7]));
+      } else {
+#pragma unroll
+        for (int u = 0; u < 8; u++)
+          if (bi < 0 || better<MODE, int>(v[u], r + 8 * u, bv, bi)) { bv = v[u]; bi = r + 8 * u; }
       }
     }
     for (; r < r1; r += 8) {
-      const float v = base[r * sr];
+      const float v = base[(long)r * sr];
       if (MODE == RED_SUM) acc += (double)v;
-      else if (bi < 0 || better<MODE>(v, r, bv, bi)) { bv = v; bi = r; }
+      else if (bi < 0 || better<MODE, int>(v, r, bv, bi)) { bv = v; bi = r; }
     }
   }
   if (MODE == RED_SUM) sd[threadIdx.y][threadIdx.x] = acc;
   else { sv[threadIdx.y][threadIdx.x] = bv; si[threadIdx.y][threadIdx.x] = bi; }
   __syncthreads();
   if (threadIdx.y == 0 && j < J) {
-    const long o = ((long)blockIdx.z * gridDim.y + blockIdx.y) * J + j;
     if (MODE == RED_SUM) {
       for (int k = 1; k < 8; k++) acc += sd[k][threadIdx.x];
-      psum[o] = acc;
     } else {
       for (int k = 1; k < 8; k++) {
         const float ov = sv[k][threadIdx.x];
-        const long oi = si[k][threadIdx.x];
-        if (oi >= 0 && (bi < 0 || better<MODE>(ov, oi, bv, bi))) { bv = ov; bi = oi; }
+        const int oi = si[k][threadIdx.x];
+        if (oi >= 0 && (bi < 0 || better<MODE, int>(ov, oi, bv, bi))) { bv = ov; bi = oi; }
       }
-      pval[o] = bv;
-      pidx[o] = bi;
+    }
+    if (gridDim.y == 1) {
+      cols_emit<MODE>(w, (long)blockIdx.z * J + j, acc, bv, bi);
+    } else {
+      const long o = ((long)blockIdx.z * gridDim.y + blockIdx.y) * J + j;
+      if (MODE == RED_SUM) w.psum[o] = acc;
+      else { w.pval[o] = bv; w.pidx[o] = bi; }
     }
   }
+  if (gridDim.y > 1) cols_fold_if_last<MODE, 32>(w, J, (long)blockIdx.x * 32);
 }
 
 // The same with four adjacent columns per thread (16-byte loads: a warp fetches 512 contiguous bytes per row, and
 // eight rows are requested before the first is used).  J % 4 == 0, 16-byte aligned rows.  grid (ceil(J/128), splits, O).
 template <int MODE>
-__global__ void __launch_bounds__(256) reduce_cols4_kernel(const float *__restrict__ src, long so, long sr, long J, long R,
-                                                           long rows_per_split, double *__restrict__ psum,
-                                                           float *__restrict__ pval, long *__restrict__ pidx) {
+__global__ void __launch_bounds__(256) reduce_cols4_kernel(const float *__restrict__ src, long so, long sr, long J, int R,
+                                                           int rows_per_split, const ColOut w) {
   __shared__ double sd[8][129];
   __shared__ float sv[8][129];
-  __shared__ long si[8][129];
+  __shared__ int si[8][129];
   const long j = ((long)blockIdx.x * 32 + threadIdx.x) * 4;
-  const long r0 = (long)blockIdx.y * rows_per_split;
-  long r1 = r0 + rows_per_split;
-  if (r1 > R) r1 = R;
+  const int r0 = blockIdx.y * rows_per_split, r1 = min(R, r0 + rows_per_split);
   const float *base = src + (long)blockIdx.z * so + j;
   double acc[4] = {0, 0, 0, 0};
   float bv[4] = {0, 0, 0, 0};
-  long bi[4] = {-1, -1, -1, -1};
-  auto take = [&](const float4 &v, long r) {
+  int bi[4] = {-1, -1, -1, -1};
+  auto take = [&](const float4 &v, int r) {
     const float e[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
     for (int c = 0; c < 4; c++) {
       if (MODE == RED_SUM) acc[c] += (double)e[c];
-      else if (bi[c] < 0 || better<MODE>(e[c], r, bv[c], bi[c])) { bv[c] = e[c]; bi[c] = r; }
+      else if (bi[c] < 0 || better<MODE, int>(e[c], r, bv[c], bi[c])) { bv[c] = e[c]; bi[c] = r; }
     }
   };
   if (j < J) {
-    long r = r0 + threadIdx.y;
+    int r = r0 + threadIdx.y;
     for (; r + 56 < r1; r += 64) {
       float4 v[8];
 #pragma unroll
-      for (int u = 0; u < 8; u++) v[u] = *reinterpret_cast<const float4 *>(base + (r + 8 * u) * sr);
+      for (int u = 0; u < 8; u++) v[u] = *reinterpret_cast<const float4 *>(base + (long)(r + 8 * u) * sr);
 #pragma unroll
       for (int u = 0; u < 8; u++) take(v[u], r + 8 * u);
     }
-    for (; r < r1; r += 8) take(*reinterpret_cast<const float4 *>(base + r * sr), r);
+    for (; r < r1; r += 8) take(*reinterpret_cast<const float4 *>(base + (long)r * sr), r);
   }
 #pragma unroll
   for (int c = 0; c < 4; c++) {
@@ -390,52 +373,39 @@ __global__ void __launch_bounds__(256) reduce_cols4_kernel(const float *__restri
   __syncthreads();
   // 128 columns of the block, folded over the eight row slices in slice order
   const int col = threadIdx.y * 32 + threadIdx.x;
-  if (col < 128) {
-    const long jc = (long)blockIdx.x * 128 + col;
-    if (jc < J) {
-      const long o = ((long)blockIdx.z * gridDim.y + blockIdx.y) * J + jc;
-      if (MODE == RED_SUM) {
-        double a = sd[0][col];
-        for (int k = 1; k < 8; k++) a += sd[k][col];
-        psum[o] = a;
-      } else {
-        float v = sv[0][col];
-        long i = si[0][col];
-        for (int k = 1; k < 8; k++) {
-          const float ov = sv[k][col];
-          const long oi = si[k][col];
-          if (oi >= 0 && (i < 0 || better<MODE>(ov, oi, v, i))) { v = ov; i = oi; }
-        }
-        pval[o] = v;
-        pidx[o] = i;
+  const long jc = (long)blockIdx.x * 128 + col;
+  if (col < 128 && jc < J) {
+    double a = 0;
+    float v = 0;
+    int i = -1;
+    if (MODE == RED_SUM) {
+      a = sd[0][col];
+      for (int k = 1; k < 8; k++) a += sd[k][col];
+    } else {
+      v = sv[0][col];
+      i = si[0][col];
+      for (int k = 1; k < 8; k++) {
+        const float ov = sv[k][col];
+        const int oi = si[k][col];
+        if (oi >= 0 && (i < 0 || better<MODE, int>(ov, oi, v, i))) { v = ov; i = oi; }
       }
     }
+    if (gridDim.y == 1) {
+      cols_emit<MODE>(w, (long)blockIdx.z * J + jc, a, v, i);
+    } else {
+      const long o = ((long)blockIdx.z * gridDim.y + blockIdx.y) * J + jc;
+      if (MODE == RED_SUM) w.psum[o] = a;
+      else { w.pval[o] = v; w.pidx[o] = i; }
+    }
   }
+  if (gridDim.y > 1) cols_fold_if_last<MODE, 128>(w, J, (long)blockIdx.x * 128);
 }
 
-template <int MODE>
-__global__ void reduce_cols_finish_kernel(const double *__restrict__ psum, const float *__restrict__ pval,
-                                          const long *__restrict__ pidx, int splits, long J, long O,
-                                          float *__restrict__ out, float *__restrict__ idx, float scale) {
-  const long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= O * J) return;
-  const long o = t / J, j = t - o * J;
-  if (MODE == RED_SUM) {
-    double acc = 0;
-    for (int s = 0; s < splits; s++) acc += psum[(o * splits + s) * J + j];
-    out[t] = (float)(acc * (double)scale);
-  } else {
-    float bv = 0;
-    long bi = -1;
-    for (int s = 0; s < splits; s++) {
-      const float ov = pval[(o * splits + s) * J + j];
-      const long oi = pidx[(o * splits + s) * J + j];
-      if (oi >= 0 && (bi < 0 || better<MODE>(ov, oi, bv, bi))) { bv = ov; bi = oi; }
-    }
-    out[t] = bv;
-    if (idx) idx[t] = (float)(bi + 1);
-  }
-}
+// zero-initialised words in the reductions' scratch block: the full reductions' record, then the column ranges' tickets
+struct DimScratch {
+  RedScratch all;
+  unsigned tickets[4096];
+};
 
 template <int MODE>
 static void reduce_dim(THGPUTensor *values, THGPUTensor *indices, THGPUTensor *src, long dim, float scale) {
@@ -446,9 +416,8 @@ static void reduce_dim(THGPUTensor *values, THGPUTensor *indices, THGPUTensor *s
   for (int d = 0; d < src->nDimension; d++) osize[d] = src->size[d];
   osize[dim] = 1;
   const long R = src->size[dim];
-  // The result is produced into contiguous temporaries when the destinations alias the source or
-  // are not contiguous after resizing.
-  THGPUTensor *src_keep = nullptr;
+  TensorRef src_keep;
+  const THGPUTensor *orig = src;
   long O, J, so, sj, sr;
   const float *base;
   auto describe = [&](THGPUTensor *t) -> bool {
@@ -485,57 +454,66 @@ static void reduce_dim(THGPUTensor *values, THGPUTensor *indices, THGPUTensor *s
     return;
   }
   if (!describe(src)) {
-    src_keep = tensor_new_contiguous(src);
+    src_keep.reset(tensor_new_contiguous(src));
     src = src_keep;
     describe(src);
   }
   THC_CHECK(O <= 65535, "outer dimension too large for the column reducer");
+  THC_CHECK(R < (1l << 31) - 4096, "reduced dimension too long");
   base = data_ptr(src);
-  THGPUTensor *vtmp = tensor_new_sized(src->nDimension, osize);
-  THGPUTensor *itmp = indices ? tensor_new_sized(src->nDimension, osize) : nullptr;
-  float *out = data_ptr(vtmp), *idx = itmp ? data_ptr(itmp) : nullptr;
+  const int ond = src->nDimension;
+  // Results go where they belong unless a destination shares memory with the source or is not contiguous after
+  // resizing: then through a temporary.
+  auto place = [&](THGPUTensor *dst, TensorRef &tmp) -> float * {
+    if (!dst) return nullptr;
+    if (!dst->storage || dst->storage != orig->storage) {
+      resize_nd(dst, ond, osize, nullptr);
+      if (is_contiguous(dst)) return data_ptr(dst);
+    }
+    tmp.reset(tensor_new_sized(ond, osize));
+    return data_ptr(tmp);
+  };
+  TensorRef vtmp, itmp;
+  float *out = place(values, vtmp), *idx = place(indices, itmp);
   if (sr == 1) {
     THC_CHECK(O == 1, "internal: row reduce with outer dim");
-    THC_CHECK(R < (1l << 31), "reduced dimension too long");
     const bool vec = aligned16(base) && (sj % 4 == 0);
-    int threads = R >= 4096 ? 256 : (R >= 512 ? 128 : 32);
-    reduce_rows_kernel<MODE><<<(unsigned)J, threads, 0, stream()>>>(base, sj, R, out, idx, scale, vec);
+    if (R < 512) {
+      reduce_rows_warp_kernel<MODE><<<(unsigned)((J + 7) / 8), 256, 0, stream()>>>(base, sj, J, (int)R, out, idx, scale);
+    } else {
+      const int threads = R >= 4096 ? 256 : 128;
+      reduce_rows_kernel<MODE><<<(unsigned)J, threads, 0, stream()>>>(base, sj, R, out, idx, scale, vec);
+    }
     check_launch("reduce_rows");
   } else {
     THC_CHECK(sj == 1, "internal: column reduce needs unit stride");
     const bool vec4 = J % 4 == 0 && sr % 4 == 0 && so % 4 == 0 && aligned16(base) && J >= 128;
     const long colblocks = vec4 ? (J + 127) / 128 : (J + 31) / 32;
-    long want = (long)ctx().sm_count * 8;
-    long splits = want / (colblocks * O);
-    if (splits < 1) splits = 1;
-    if (splits > (R + 63) / 64) splits = (R + 63) / 64;
-    if (splits > 512) splits = 512;
-    long rows_per_split = (R + splits - 1) / splits;
+    const long want = (long)ctx().sm_count * 8;
+    // slices of at least 64 rows (a thread's eight loads in flight), and none for what one block reads in four rounds
+    long splits = R <= 256 ? 1 : std::max(1l, std::min(std::min(want / (colblocks * O), (R + 63) / 64), 512l));
+    const long rows_per_split = (R + splits - 1) / splits;
     splits = (R + rows_per_split - 1) / rows_per_split;
-    const size_t nparts = (size_t)O * splits * J;
+    const size_t nparts = splits > 1 ? (size_t)O * splits * J : 0;
     WsScope ws_scope;
-    char *scr = (char *)ws_alloc(nparts * (MODE == RED_SUM ? sizeof(double) : sizeof(float) + sizeof(long)));
-    double *psum = (double *)scr;
-    long *pidx = (long *)scr;
-    float *pval = (float *)(scr + (MODE == RED_SUM ? 0 : nparts * sizeof(long)));
+    ColOut w = {};
+    if (splits > 1) {
+      char *scr = (char *)ws_alloc(nparts * sizeof(double));
+      w.psum = (double *)scr;
+      w.pidx = (int *)scr;
+      w.pval = (float *)scr + nparts;
+      DimScratch *ds = (DimScratch *)scratch(sizeof(DimScratch));
+      THC_CHECK(colblocks * O <= (long)(sizeof(ds->tickets) / sizeof(ds->tickets[0])), "internal: too many column ranges to split");
+      w.tickets = ds->tickets;
+    }
+    w.out = out; w.idx = idx; w.scale = scale;
     dim3 grid((unsigned)colblocks, (unsigned)splits, (unsigned)O), block(32, 8);
-    if (vec4) reduce_cols4_kernel<MODE><<<grid, block, 0, stream()>>>(base, so, sr, J, R, rows_per_split, psum, pval, pidx);
-    else reduce_cols_kernel<MODE><<<grid, block, 0, stream()>>>(base, so, sr, J, R, rows_per_split, psum, pval, pidx);
+    if (vec4) reduce_cols4_kernel<MODE><<<grid, block, 0, stream()>>>(base, so, sr, J, (int)R, (int)rows_per_split, w);
+    else reduce_cols_kernel<MODE><<<grid, block, 0, stream()>>>(base, so, sr, J, (int)R, (int)rows_per_split, w);
     check_launch("reduce_cols");
-    const long total = O * J;
-    reduce_cols_finish_kernel<MODE><<<ceil_div(total, 256), 256, 0, stream()>>>(psum, pval, pidx, (int)splits, J, O, out, idx, scale);
-    check_launch("reduce_cols_finish");
   }
-  const int ond = src->nDimension;
-  if (src_keep) tensor_free(src_keep);
-  resize_nd(values, ond, osize, nullptr);
-  tensor_copy(values, vtmp);
-  tensor_free(vtmp);
-  if (indices) {
-    resize_nd(indices, ond, osize, nullptr);
-    tensor_copy(indices, itmp);
-    tensor_free(itmp);
-  }
+  if (vtmp.t) { resize_nd(values, ond, osize, nullptr); tensor_copy(values, vtmp); }
+  if (itmp.t) { resize_nd(indices, ond, osize, nullptr); tensor_copy(indices, itmp); }
 }
 
 }  // namespace thc
@@ -576,13 +554,13 @@ THC_API void THGPUTensor_cdiv(THGPUTensor *self, THGPUTensor *src1, THGPUTensor 
   THC_END()
 }
 
-THC_API float THGPUTensor_dot(THGPUTensor *self, THGPUTensor *src) { THC_BEGIN return (float)reduce_all<RED_DOT>(self, src); THC_END(0.f) }
-THC_API float THGPUTensor_minall(THGPUTensor *self) { THC_BEGIN return (float)reduce_all<RED_MIN>(self, nullptr); THC_END(0.f) }
-THC_API float THGPUTensor_maxall(THGPUTensor *self) { THC_BEGIN return (float)reduce_all<RED_MAX>(self, nullptr); THC_END(0.f) }
-THC_API float THGPUTensor_sumall(THGPUTensor *self) { THC_BEGIN return (float)reduce_all<RED_SUM>(self, nullptr); THC_END(0.f) }
+THC_API float THGPUTensor_dot(THGPUTensor *self, THGPUTensor *src) { THC_BEGIN return (float)reduce_all<RED_DOT>(self, src, IdTerm()); THC_END(0.f) }
+THC_API float THGPUTensor_minall(THGPUTensor *self) { THC_BEGIN return (float)reduce_all<RED_MIN>(self, nullptr, IdTerm()); THC_END(0.f) }
+THC_API float THGPUTensor_maxall(THGPUTensor *self) { THC_BEGIN return (float)reduce_all<RED_MAX>(self, nullptr, IdTerm()); THC_END(0.f) }
+THC_API float THGPUTensor_sumall(THGPUTensor *self) { THC_BEGIN return (float)reduce_all<RED_SUM>(self, nullptr, IdTerm()); THC_END(0.f) }
 THC_API float THGPUTensor_meanall(THGPUTensor *self) {
   THC_BEGIN
-  return (float)(reduce_all<RED_SUM>(self, nullptr) / (double)nelem(self));
+  return (float)(reduce_all<RED_SUM>(self, nullptr, IdTerm()) / (double)nelem(self));
   THC_END(0.f)
 }
 

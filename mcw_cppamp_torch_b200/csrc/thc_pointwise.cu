@@ -10,7 +10,7 @@
 // (thc_apply.cuh): contiguous float4 streaming, tiled transposes, generic strides.
 #include <cmath>
 
-#include "thc_apply.cuh"
+#include "thc_reduce.cuh"
 
 namespace thc {
 
@@ -54,14 +54,20 @@ template <int C> struct CmpTensorOp { __device__ float operator()(const float *a
 // (value * src1) * src2 and (value * src1) / src2, each step rounded to float as in the C expression
 struct ScaledMulOp { float v; __device__ float operator()(const float *a) const { return __fmul_rn(__fmul_rn(v, a[0]), a[1]); } };
 struct ScaledDivOp { float v; __device__ float operator()(const float *a) const { return __fdiv_rn(__fmul_rn(v, a[0]), a[1]); } };
-struct SumOp { __device__ float operator()(const float *a) const { return __fadd_rn(a[0], a[1]); } };
+// a[0] + op(a[1], a[2])
+template <class Op> struct AddOp { Op op; __device__ float operator()(const float *a) const { return __fadd_rn(a[0], op(a + 1)); } };
 
-// terms of the whole-tensor norms
-struct NonZeroOp { __device__ float operator()(const float *a) const { return a[0] != 0.f ? 1.f : 0.f; } };
-struct SquareOp { __device__ float operator()(const float *a) const { const double z = (double)a[0]; return (float)(z * z); } };
-struct AbsPowOp { float v; __device__ float operator()(const float *a) const { return powf(fabsf(a[0]), v); } };
-struct AbsDiffPowOp { float v; __device__ float operator()(const float *a) const { return powf(fabsf(a[0] - a[1]), v); } };
-struct CenteredSquareOp { double mean; __device__ float operator()(const float *a) const { const double d = (double)a[0] - mean; return (float)(d * d); } };
+// terms of the whole-tensor norms (NIN operands each, rounded to float)
+struct NonZeroOp { static constexpr int NIN = 1; __device__ float operator()(const float *a) const { return a[0] != 0.f ? 1.f : 0.f; } };
+struct AbsTermOp { static constexpr int NIN = 1; __device__ float operator()(const float *a) const { return fabsf(a[0]); } };
+struct SquareOp { static constexpr int NIN = 1; __device__ float operator()(const float *a) const { return __fmul_rn(a[0], a[0]); } };
+struct AbsPowOp { static constexpr int NIN = 1; float v; __device__ float operator()(const float *a) const { return powf(fabsf(a[0]), v); } };
+struct AbsDiffPowOp { static constexpr int NIN = 2; float v; __device__ float operator()(const float *a) const { return powf(fabsf(a[0] - a[1]), v); } };
+struct CenteredSquareOp {
+  static constexpr int NIN = 1;
+  double mean;
+  __device__ float operator()(const float *a) const { const double d = (double)a[0] - mean; return (float)(d * d); }
+};
 
 template <typename Op>
 static void unary(THGPUTensor *self, THGPUTensor *src, Op op, const char *name) {
@@ -74,33 +80,32 @@ static void binary(THGPUTensor *self, THGPUTensor *a, THGPUTensor *b, Op op, con
   tensor_resize_as(self, a);
   apply<2>(self, a, b, op, name);
 }
-// sum over all elements of op(a) or op(a, b), through a temporary of a's shape
+// sum over all elements of op(a) or op(a, b).  Operands of another shape with the same number of elements are taken in
+// their own logical order.
 template <typename Op>
-static double sum_of(THGPUTensor *a, THGPUTensor *b, Op op, const char *name) {
-  THGPUTensor *tmp = tensor_new();
-  tensor_resize_as(tmp, a);
-  if (b) apply<2>(tmp, a, b, op, name);
-  else apply<1>(tmp, a, nullptr, op, name);
-  const double s = (double)THGPUTensor_sumall(tmp);
-  tensor_free(tmp);
-  return s;
-}
-// r = t + op(src1, src2).  TH walks the three tensors element by element in memory order, so operands of another
-// shape with the same number of elements are taken as contiguous copies seen under t's sizes.
+static double sum_of(THGPUTensor *a, THGPUTensor *b, Op op) { return reduce_all<RED_SUM>(a, b, op); }
+// r = t + op(src1, src2) in one pass.  TH walks the three tensors element by element in memory order, so operands of
+// another shape with the same number of elements are taken as contiguous copies seen under t's sizes.
 template <typename Op>
 static void add_scaled(THGPUTensor *self, THGPUTensor *t, THGPUTensor *src1, THGPUTensor *src2, Op op, const char *name) {
   THC_ARG(nelem(src1) == nelem(t) && nelem(src2) == nelem(t), 3, "sizes do not match");
-  THGPUTensor *v1 = nullptr, *v2 = nullptr;
-  if (!THGPUTensor_isSameSizeAs(src1, t)) { v1 = THGPUTensor_newClone(src1); tensor_resize_as(v1, t); }
-  if (!THGPUTensor_isSameSizeAs(src2, t)) { v2 = THGPUTensor_newClone(src2); tensor_resize_as(v2, t); }
-  THGPUTensor *tmp = tensor_new();
-  tensor_resize_as(tmp, t);
-  apply<2>(tmp, v1 ? v1 : src1, v2 ? v2 : src2, op, name);
+  // an operand that overlaps the result in memory without being the same view has to be read before anything is written
+  auto entangled = [&](const THGPUTensor *a) {
+    if (a->storage != self->storage || (data_ptr(a) == data_ptr(self) && same_layout(a, self))) return false;
+    auto last = [](const THGPUTensor *x) {
+      long e = x->storageOffset;
+      for (int d = 0; d < x->nDimension; d++) e += (x->size[d] - 1) * x->stride[d];
+      return e;
+    };
+    return last(a) >= self->storageOffset && last(self) >= a->storageOffset;
+  };
+  TensorRef v0, v1, v2;
+  if (self != t && entangled(t)) { v0.reset(THGPUTensor_newClone(t)); t = v0; }
+  const bool own1 = !THGPUTensor_isSameSizeAs(src1, t), own2 = !THGPUTensor_isSameSizeAs(src2, t);
+  if (own1 || entangled(src1)) { v1.reset(THGPUTensor_newClone(src1)); tensor_resize_as(v1, t); src1 = v1; }
+  if (own2 || entangled(src2)) { v2.reset(THGPUTensor_newClone(src2)); tensor_resize_as(v2, t); src2 = v2; }
   if (self != t) tensor_resize_as(self, t);
-  apply<2>(self, t, tmp, SumOp(), name);
-  if (v1) tensor_free(v1);
-  if (v2) tensor_free(v2);
-  tensor_free(tmp);
+  apply<3>(self, t, src1, AddOp<Op>{op}, name, src2);
 }
 
 }  // namespace thc
@@ -162,17 +167,17 @@ THC_API void THGPUTensor_addcdiv(THGPUTensor *self, THGPUTensor *t, float value,
 THC_API float THGPUTensor_normall(THGPUTensor *self, float value) {
   THC_BEGIN
   if (nelem(self) == 0) return 0.f;
-  if (value == 0.f) return (float)sum_of(self, nullptr, NonZeroOp(), "normall");
-  if (value == 1.f) return (float)sum_of(self, nullptr, AbsOp(), "normall");
-  if (value == 2.f) return (float)sqrt(sum_of(self, nullptr, SquareOp(), "normall"));
-  return (float)pow(sum_of(self, nullptr, AbsPowOp{value}, "normall"), 1.0 / (double)value);
+  if (value == 0.f) return (float)sum_of(self, nullptr, NonZeroOp());
+  if (value == 1.f) return (float)sum_of(self, nullptr, AbsTermOp());
+  if (value == 2.f) return (float)sqrt(sum_of(self, nullptr, SquareOp()));
+  return (float)pow(sum_of(self, nullptr, AbsPowOp{value}), 1.0 / (double)value);
   THC_END(0.f)
 }
 THC_API float THGPUTensor_dist(THGPUTensor *self, THGPUTensor *src, float value) {
   THC_BEGIN
   THC_ARG(nelem(self) == nelem(src), 2, "sizes do not match");
   if (nelem(self) == 0) return 0.f;
-  return (float)pow(sum_of(self, src, AbsDiffPowOp{value}, "dist"), 1.0 / (double)value);
+  return (float)pow(sum_of(self, src, AbsDiffPowOp{value}), 1.0 / (double)value);
   THC_END(0.f)
 }
 THC_API float THGPUTensor_varall(THGPUTensor *self) {
@@ -180,7 +185,7 @@ THC_API float THGPUTensor_varall(THGPUTensor *self) {
   const long n = nelem(self);
   THC_ARG(n > 0, 1, "empty Tensor");
   const double mean = (double)THGPUTensor_sumall(self) / (double)n;
-  return (float)(sum_of(self, nullptr, CenteredSquareOp{mean}, "varall") / (double)(n - 1));
+  return (float)(sum_of(self, nullptr, CenteredSquareOp{mean}) / (double)(n - 1));
   THC_END(0.f)
 }
 THC_API float THGPUTensor_stdall(THGPUTensor *self) {
@@ -188,7 +193,7 @@ THC_API float THGPUTensor_stdall(THGPUTensor *self) {
   const long n = nelem(self);
   THC_ARG(n > 0, 1, "empty Tensor");
   const double mean = (double)THGPUTensor_sumall(self) / (double)n;
-  return (float)sqrt(sum_of(self, nullptr, CenteredSquareOp{mean}, "stdall") / (double)(n - 1));
+  return (float)sqrt(sum_of(self, nullptr, CenteredSquareOp{mean}) / (double)(n - 1));
   THC_END(0.f)
 }
 // norm along a dimension (mcw_torch7_core/lib/TH/generic/THTensorMath.c:1401-1427): the terms |x|^value (or

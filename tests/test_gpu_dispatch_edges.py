@@ -1,0 +1,82 @@
+"""The elementwise, reduction and host-copy kernels at the sizes where their dispatch changes: tile edges and 16-byte
+alignment of transposed operands, one block or many and one slice or several in the reductions, the staging limit of
+small downloads."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def gt():
+    import mcw_cppamp_torch_b200 as gt
+    return gt
+
+
+@pytest.mark.parametrize("r,c", [(64, 64), (4, 8), (63, 65), (128, 68), (130, 3), (3, 130), (200, 516), (577, 129)])
+def test_transposed_operands(gt, r, c):
+    g = np.random.default_rng(r * 1000 + c)
+    x, y, z = (g.standard_normal(s).astype(np.float32) for s in ((r, c), (c, r), (c, r)))
+    X, Y, Z, R = gt.gpu(x), gt.gpu(y), gt.gpu(z), gt.GPUTensor(r, c)
+    half = np.float32(0.5)
+    assert np.array_equal(R.copy(Y.t()).float(), y.T)
+    assert np.array_equal(R.add(X, 0.5, Y.t()).float(), x + half * y.T)                  # second operand transposed
+    assert np.array_equal(R.add(Y.t(), 0.5, X).float(), y.T + half * x)                  # first
+    assert np.array_equal(R.add(Y.t(), 0.5, Z.t()).float(), y.T + half * z.T)            # both
+    out = gt.GPUTensor(c, r)
+    out.t().cmul(X, Y.t())
+    assert np.array_equal(out.float(), (x * y.T).T)                                      # result transposed
+    sub = gt.GPUTensor(r, c + 3).zero()
+    sub.narrow(2, 2, c).copy(Y.t())                                                      # pitch and address off 16 bytes
+    want = np.zeros((r, c + 3), np.float32)
+    want[:, 1:1 + c] = y.T
+    assert np.array_equal(sub.float(), want)
+
+
+def test_addcmul_in_place_with_overlapping_operand(gt):
+    x = np.random.default_rng(3).standard_normal((96, 96)).astype(np.float32)
+    X = gt.gpu(x)
+    X.addcmul(0.5, X.t(), X)
+    assert np.array_equal(X.float(), x + np.float32(0.5) * x.T * x)
+
+
+@pytest.mark.parametrize("n", [1, 3, 4096 * 4, 4096 * 4 + 4, 4096 * 4 + 1, 300007])
+def test_full_reductions(gt, n):
+    x = (np.random.default_rng(n).standard_normal(n) + 0.5).astype(np.float32)
+    X = gt.gpu(x)
+    # a float32 run of four and the final rounding: 3 roundings of terms bounded by the sum of magnitudes
+    bound = 4 * 2.0 ** -24 * np.abs(x.astype(np.float64)).sum() + 1e-12
+    assert abs(X.sum() - x.astype(np.float64).sum()) <= bound
+    assert X.max() == x.max() and X.min() == x.min()
+    exact = np.sqrt((x.astype(np.float64) ** 2).sum())
+    assert abs(X.norm() - exact) <= 8 * 2.0 ** -24 * exact
+    assert abs(X.dist(gt.gpu(np.zeros_like(x))) - exact) <= 64 * 2.0 ** -24 * exact      # powf: a few ulp a term
+    last = gt.lib().THGPUTensor_get1d(X.cdata, n - 1)
+    assert last == x[-1]
+
+
+@pytest.mark.parametrize("shape", [(256, 40), (257, 40), (8200, 33), (700, 128), (5000, 132), (1000, 516), (3, 511), (3, 512),
+                                   (9, 31), (7, 4097), (3, 300, 130), (2, 5000, 8)])
+def test_dim_reductions(gt, shape):
+    g = np.random.default_rng(sum(shape))
+    x = g.standard_normal(shape).astype(np.float32)
+    x.reshape(-1)[::7] = 5.0            # ties across slices: the first maximum wins
+    X = gt.gpu(x)
+    for dim in range(x.ndim):
+        s, (v, i) = X.sum(dim + 1).float(), X.max(dim + 1)
+        x64 = x.astype(np.float64)
+        assert np.all(np.abs(s - x64.sum(dim, keepdims=True)) <= 2.0 ** -23 * np.abs(x64).sum(dim, keepdims=True))
+        assert np.array_equal(v.float(), x.max(dim, keepdims=True))
+        assert np.array_equal(i.float(), np.expand_dims(x.argmax(dim), dim) + 1)
+        lo, k = X.min(dim + 1)
+        assert np.array_equal(lo.float(), x.min(dim, keepdims=True)) and np.array_equal(k.float(), np.expand_dims(x.argmin(dim), dim) + 1)
+    X.sum(X, 1)                          # the result in the source's own storage
+    assert X.size() == (1,) + shape[1:]
+    assert np.all(np.abs(X.float() - x.astype(np.float64).sum(0, keepdims=True)) <= 2.0 ** -23 * np.abs(x.astype(np.float64)).sum(0, keepdims=True))
+
+
+@pytest.mark.parametrize("n", [1, 1023, 16384, 16385])
+def test_download_sizes(gt, n):
+    x = np.random.default_rng(n).standard_normal(n).astype(np.float32)
+    out = np.zeros(n, np.float32)
+    assert gt.gpu(x).float(out) is out and np.array_equal(out, x)
