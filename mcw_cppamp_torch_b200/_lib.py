@@ -211,17 +211,28 @@ class THCError(RuntimeError):
 
 
 class _Lib:
+    """The library's functions as attributes.  Each raises THCError when the call left an error; those with an invoker in
+    the native module `_calls` go through it, the others (and odd arguments) through ctypes."""
+
     def __init__(self):
         if not os.path.exists(LIB_PATH):
             raise ImportError("%s is missing: build it with `python -m mcw_cppamp_torch_b200.build` "
                               "(there is no CPU fallback)" % LIB_PATH)
+        from . import _calls
         self.cdll = C.CDLL(LIB_PATH)
+
+        def address(fn):
+            return C.cast(fn, C.c_void_p).value
+        _calls.setup(address(self.cdll.THGPUGetLastError), address(self.cdll.THGPUClearError), THCError, (TP, SP, C.c_void_p))
+        _calls.functions(*(address(getattr(self.cdll, n)) for n in ("THGPUTensor_setStorage", "THGPUTensor_copyFloat",
+                                                                    "THFloatTensor_copyGPU")))
         for name, (res, args) in SIGNATURES.items():
             fn = getattr(self.cdll, name)
             fn.restype = res
             fn.argtypes = args
             if name not in ("THGPUGetLastError", "THGPUClearError"):
-                setattr(self, name, self._checked(fn))
+                slow = self._checked(fn)
+                setattr(self, name, _calls.wrap(name, address(fn), slow) or slow)
             else:
                 setattr(self, name, fn)
 
@@ -236,7 +247,6 @@ class _Lib:
                 clear()
                 raise THCError(msg)
             return r
-        call.raw = fn
         return call
 
 

@@ -1,4 +1,4 @@
-"""In-tree nvcc build of libTHC.so (sm_100a only).
+"""In-tree build of libTHC.so (nvcc, sm_100a only) and of the Python call module _calls.so.
 
     python -m mcw_cppamp_torch_b200.build [--force] [--verbose]
 
@@ -9,12 +9,14 @@ import glob
 import os
 import subprocess
 import sys
+import sysconfig
 
 PKG = os.path.dirname(os.path.abspath(__file__))
 ROOT = os.path.dirname(PKG)
 CSRC = os.path.join(PKG, "csrc")
 OBJ = os.path.join(CSRC, "build")
 LIB = os.path.join(PKG, "libTHC.so")
+CALLS = os.path.join(PKG, "_calls.so")
 
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
@@ -57,7 +59,18 @@ def build(force=False, verbose=False):
     if jobs or not os.path.exists(LIB):
         cmd = [NVCC, "-shared", "-o", LIB] + objs + ["-lcudart"]
         subprocess.check_call(cmd)
+    build_calls(force)
     return LIB
+
+
+def build_calls(force=False):
+    """_calls.so: the CPython module behind lib()'s functions (csrc/py_calls.cpp), compiled by the host compiler."""
+    src, hdr = os.path.join(CSRC, "py_calls.cpp"), os.path.join(ROOT, "include", "THC.h")
+    if not force and os.path.exists(CALLS) and os.path.getmtime(CALLS) > max(os.path.getmtime(src), os.path.getmtime(hdr)):
+        return CALLS
+    subprocess.check_call([os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-shared", "-fPIC", "-fvisibility=hidden",
+                           "-I", os.path.join(ROOT, "include"), "-I", sysconfig.get_paths()["include"], src, "-o", CALLS])
+    return CALLS
 
 
 if __name__ == "__main__":

@@ -6,9 +6,11 @@ Method names, argument order and overloads follow the Lua methods the reference 
 (`torch.FloatTensor` in the reference) are numpy float32 arrays here.  All arithmetic happens in
 the CUDA library; nothing in this file computes on the CPU."""
 import ctypes as C
+import math
 
 import numpy as np
 
+from . import _calls
 from ._lib import (HOST_TYPES, THLongStorage, lib)
 
 # numpy dtype -> TH host type name
@@ -92,9 +94,8 @@ class GPUTensor:
     nDimension = dim
 
     def size(self, d=None):
-        t = self._p.contents
         if d is None:
-            return tuple(t.size[k] for k in range(t.nDimension))
+            return _calls.sizes(self._p)
         return lib().THGPUTensor_size(self._p, d - 1)
 
     def stride(self, d=None):
@@ -122,6 +123,9 @@ class GPUTensor:
     def resize(self, *sizes):
         if len(sizes) == 1 and isinstance(sizes[0], (tuple, list)):
             sizes = tuple(sizes[0])
+        if 1 <= len(sizes) <= 5:
+            getattr(lib(), "THGPUTensor_resize%dd" % len(sizes))(self._p, *[int(v) for v in sizes])
+            return self
         s = _long_storage([int(v) for v in sizes])
         lib().THGPUTensor_resize(self._p, C.byref(s), None)
         return self
@@ -153,13 +157,11 @@ class GPUTensor:
         sizes = list(sizes)
         if -1 in sizes:
             k = sizes.index(-1)
-            rest = int(np.prod([s for s in sizes if s != -1])) or 1
+            rest = math.prod(s for s in sizes if s != -1) or 1
             sizes[k] = n // rest
-        assert int(np.prod(sizes)) == n
-        L = lib()
+        assert math.prod(sizes) == n
         r = GPUTensor()
-        s = _long_storage(sizes)
-        L.THGPUTensor_setStorage(r._p, self._p.contents.storage, self._p.contents.storageOffset, C.byref(s), None)
+        _calls.set_view(r._p, self._p, tuple(sizes))
         return r
 
     def contiguous(self):
@@ -176,6 +178,8 @@ class GPUTensor:
         else:
             # a host tensor of any TH type: THGPUTensor_copy<Type> (gputorch/Tensor.cpp:38-65 dispatches the same way)
             a = np.asarray(src)
+            if _calls.upload(self._p, a):
+                return self
             if a.dtype not in _TH_NAME:
                 a = a.astype(np.float32)
             name, h = _host_view(a)
@@ -186,7 +190,7 @@ class GPUTensor:
         shape = self.size() if self.dim() else (0,)
         if out is None:
             out = np.empty(shape, dtype)
-        if out.size:
+        if out.size and not (out.dtype == np.float32 and _calls.download(out, self._p)):
             name, h = _host_view(out)
             getattr(lib(), "TH%sTensor_copyGPU" % name)(C.byref(h), self._p)
         return out
