@@ -384,6 +384,7 @@ THC_API int THGPUNN_Threshold_updateGradInput(THGPUTensor *input, THGPUTensor *g
     THGPUTensor *gradInput, double threshold);
 /* Classifier tail: gpunn-impl/LogSoftMax.cpp:116-194, gpunn-impl/ClassNLLCriterion.cpp:96-198
  * (targets are a float GPU tensor of 1-based class ids; loss averaged over the batch). */
+THC_API int THGPUNN_Linear_updateOutput(THGPUTensor *input, THGPUTensor *output, THGPUTensor *weight, THGPUTensor *bias);
 THC_API int THGPUNN_LogSoftMax_updateOutput(THGPUTensor *input, THGPUTensor *output);
 THC_API int THGPUNN_LogSoftMax_updateGradInput(THGPUTensor *input, THGPUTensor *gradOutput,
     THGPUTensor *gradInput, THGPUTensor *output);

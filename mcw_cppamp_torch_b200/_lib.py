@@ -184,6 +184,7 @@ SIGNATURES = {
     "THGPUNN_SpatialMaxPooling_updateOutput": (i, [TP, TP, TP, i, i, i, i]),
     "THGPUNN_SpatialMaxPooling_updateGradInput": (i, [TP, TP, TP, TP, i, i, i, i]),
     "THGPUNN_Threshold_updateOutput": (i, [TP, TP, d, d]), "THGPUNN_Threshold_updateGradInput": (i, [TP, TP, TP, d]),
+    "THGPUNN_Linear_updateOutput": (i, [TP, TP, TP, TP]),
     "THGPUNN_LogSoftMax_updateOutput": (i, [TP, TP]), "THGPUNN_LogSoftMax_updateGradInput": (i, [TP, TP, TP, TP]),
     "THGPUNN_ClassNLLCriterion_updateOutput": (i, [TP, TP, TP, i]),
     "THGPUNN_ClassNLLCriterion_updateGradInput": (i, [TP, TP, TP, i]),

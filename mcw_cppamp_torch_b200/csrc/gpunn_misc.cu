@@ -186,6 +186,21 @@ THC_API int THGPUNN_Threshold_updateGradInput(THGPUTensor *input, THGPUTensor *g
   THC_END(1)
 }
 
+// output = input * weight^T + bias (mcw_nn/Linear.lua:46-58, batch mode) in one product whose epilogue adds the bias
+THC_API int THGPUNN_Linear_updateOutput(THGPUTensor *input, THGPUTensor *output, THGPUTensor *weight, THGPUTensor *bias) {
+  THC_BEGIN
+  THC_ARG(input->nDimension == 2 && weight->nDimension == 2 && bias->nDimension == 1, 1, "batch of rows, matrix and vector expected");
+  const long rows = input->size[0], in = input->size[1], out = weight->size[0];
+  THC_ARG(weight->size[1] == in && bias->size[0] == out, 3, "size mismatch");
+  TensorRef x(tensor_new_contiguous(input)), w(tensor_new_contiguous(weight)), b(tensor_new_contiguous(bias));
+  const long s[2] = {rows, out};
+  resize_nd(output, 2, s, nullptr);
+  THC_CHECK(is_contiguous(output), "output must be contiguous");
+  gemm('t', 'n', out, rows, in, 1.f, data_ptr(w), in, data_ptr(x), in, 0.f, data_ptr(output), out, data_ptr(b));
+  return 0;
+  THC_END(1)
+}
+
 THC_API int THGPUNN_LogSoftMax_updateOutput(THGPUTensor *input, THGPUTensor *output) {
   THC_BEGIN
   long nframe, dim;

@@ -5,8 +5,10 @@
 
 #include <algorithm>
 #include <climits>
+#include <cmath>
 
 #include "mm_simt.cuh"
+#include "mm_small.cuh"
 #include "mm_tc.cuh"
 #include "mm_tc2.cuh"
 #include "mm_tc2h.cuh"
@@ -92,14 +94,14 @@ static int choose_tail_splits(long tail, long ktiles, int slots) {
   return best;
 }
 
-// `allow_split` lets long-K problems with few output tiles spread over the SMs.  TC_ONLY problems
-// (operands that only the tensor-core engine can read) never instantiate the FP32 FMA engine.
-template <class P, bool TC_ONLY>
+// `allow_split` lets long-K problems with few output tiles spread over the SMs.  ENGINES: which of the one-SM tensor-core
+// engine (1) and the FP32 FMA engine (2) the problem may reach, so that the other is not instantiated for it.
+template <class P, int ENGINES>
 static void launch_impl(P p, bool allow_split) {
   if (p.M <= 0 || p.N <= 0) return;
   THC_CHECK(p.K > 0, "internal: matrix product with empty reduction");
   const int mode = ctx().math_mode;
-  THC_CHECK(mode == 0 || mode == 2 || (mode == 1 && !TC_ONLY), "math mode %d cannot run this product", mode);
+  THC_CHECK(mode == 1 ? (ENGINES & 2) != 0 : (ENGINES & 1) != 0, "math mode %d cannot run this product", mode);
   const int sms = ctx().sm_count;
   const bool tc = mode != 1;   // the BF16 mode runs what its own engine does not take in the FP32-accurate one
   const int bm = tc ? TC_BM : SIMT_BM;
@@ -117,12 +119,15 @@ static void launch_impl(P p, bool allow_split) {
   }
   if (splits > 1) p.ws = (float *)ws_alloc(sizeof(float) * splits * p.M * p.N);
   dim3 grid((unsigned)gm, (unsigned)gn, (unsigned)splits);
-  if (tc) {
-    if (bn == 128) launch_tc<P, 128>(p, grid);
-    else launch_tc<P, 64>(p, grid);
-  } else if constexpr (!TC_ONLY) {
-    simt_kernel<P><<<grid, 256, 0, stream()>>>(p);
-    check_launch("simt_kernel");
+  if constexpr ((ENGINES & 1) != 0) {
+    if (tc && bn == 128) launch_tc<P, 128>(p, grid);
+    else if (tc) launch_tc<P, 64>(p, grid);
+  }
+  if constexpr ((ENGINES & 2) != 0) {
+    if (!tc) {
+      simt_kernel<P><<<grid, 256, 0, stream()>>>(p);
+      check_launch("simt_kernel");
+    }
   }
   if (splits > 1) {
     splitk_finish_kernel<<<dim3((unsigned)ceil_div(p.M, 256), (unsigned)(p.N < 32768 ? p.N : 32768)), 256, 0, stream()>>>(
@@ -130,8 +135,9 @@ static void launch_impl(P p, bool allow_split) {
     check_launch("splitk_finish");
   }
 }
-template <class P> static void launch(const P &p, bool allow_split = true) { launch_impl<P, false>(p, allow_split); }
-template <class P> static void launch_tc_only(const P &p, bool allow_split = true) { launch_impl<P, true>(p, allow_split); }
+template <class P> static void launch(const P &p, bool allow_split = true) { launch_impl<P, 3>(p, allow_split); }
+template <class P> static void launch_tc_only(const P &p, bool allow_split = true) { launch_impl<P, 1>(p, allow_split); }
+template <class P> static void launch_simt(const P &p, bool allow_split = true) { launch_impl<P, 2>(p, allow_split); }
 
 // cuTensorMapEncodeTiled through the runtime's driver entry point (no link-time dependency on libcuda).
 typedef CUresult (*EncodeTiledFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *, const cuuint64_t *,
@@ -357,6 +363,54 @@ static void launch_raw(P p, Attach attach, bool allow_split = true) {
         p.ws, p.tail_splits, bn2, p.tail_first, gm, p.M, p.N, p.epi);
     check_launch("tail_finish");
   }
+}
+
+// ---- small and narrow products (mm_small.cuh) ----------------------------------------------------------------------
+template <int BN, int WM, int WN, bool A_K, bool B_K>
+static void launch_small_kernel(const SmallProblem &p) {
+  constexpr int BM = 64, SMEM = SM_STAGES * (SmallTile<BM, A_K>::FLOATS + SmallTile<BN, B_K>::FLOATS) * 4;
+  static thread_local int configured_for = -1;
+  if (SMEM > 47 * 1024 && configured_for != ctx().device) {
+    THC_CUDA(cudaFuncSetAttribute(small_kernel<BM, BN, WM, WN, A_K, B_K>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM));
+    configured_for = ctx().device;
+  }
+  const dim3 grid((unsigned)ceil_div(p.M, BM), (unsigned)ceil_div(p.N, BN), (unsigned)p.slices);
+  small_kernel<BM, BN, WM, WN, A_K, B_K><<<grid, SM_THREADS, SMEM, stream()>>>(p);
+  check_launch("small_kernel");
+}
+template <int BN, int WM, int WN>
+static void launch_small_layout(const SmallProblem &p, bool a_k, bool b_k) {
+  if (a_k && b_k) launch_small_kernel<BN, WM, WN, true, true>(p);
+  else if (a_k) launch_small_kernel<BN, WM, WN, true, false>(p);
+  else if (b_k) launch_small_kernel<BN, WM, WN, false, true>(p);
+  else launch_small_kernel<BN, WM, WN, false, false>(p);
+}
+inline SmallOperand small_operand(const float *base, long ld) {
+  return SmallOperand{base, ld, ((uintptr_t)base & 15) == 0 && ld % 4 == 0 ? 1 : 0};
+}
+// D = alpha * A * B^T + beta * D (+ bias) for A [M][K] and B [N][K]; a_k / b_k: the operand's memory runs along k.
+static void launch_small(SmallProblem p, bool a_k, bool b_k) {
+  if (p.N > p.M) {   // the longer side takes the 64-row tiles
+    std::swap(p.a, p.b); std::swap(a_k, b_k); std::swap(p.M, p.N); std::swap(p.sm, p.sn); std::swap(p.bias_m, p.bias_n);
+  }
+  p.stalled = stall_ctl().dev_flag;
+  const int bn = p.N <= 8 ? 8 : p.N <= 16 ? 16 : p.N <= 32 ? 32 : 64;
+  const long tiles = (long)ceil_div(p.M, 64) * ceil_div(p.N, bn), ktiles = ceil_div(p.K, TC_BK);
+  // Slices until the tiles fill the device as deep as registers and shared memory allow, each at least two k tiles, and
+  // not so many that the block that folds them, one after the other, takes longer than a slice's own k tiles.
+  const long depth = bn == 64 ? 3 : bn == 8 ? 5 : 4;
+  const long fold = (long)std::sqrt((double)ktiles * 64 / bn);   // a slice costs the folding block about bn / 64 of a k tile's time
+  const long slices = std::max(1l, std::min(std::min(depth * ctx().sm_count / tiles, ktiles / 2), std::min(fold, 32l)));
+  p.tiles_per_slice = ceil_div(ktiles, slices);
+  p.slices = ceil_div(ktiles, p.tiles_per_slice);
+  if (p.slices > 1) {
+    p.ws = (float *)ws_alloc(sizeof(float) * tiles * p.slices * 64 * bn);
+    p.tickets = zero_words();
+  }
+  if (bn == 8) launch_small_layout<8, 4, 1>(p, a_k, b_k);
+  else if (bn == 16) launch_small_layout<16, 4, 1>(p, a_k, b_k);
+  else if (bn == 32) launch_small_layout<32, 4, 1>(p, a_k, b_k);
+  else launch_small_layout<64, 2, 2>(p, a_k, b_k);
 }
 
 // Products over ready-made planes: the two-SM engine when the tile fits the problem, else the one-SM engine.

@@ -681,6 +681,8 @@ struct Epilogue {
   // n = (parity, plane): out[img * pair_img + plane * nstride + y * pair_oW + 2 * x2 + parity]; with an odd
   // output width the last pair of a row has no parity-1 pixel.
   long pair_K = 0, pair_oH = 1, pair_oW2 = 1, pair_oW = 0, pair_img = 0;
+  const float *row_bias = nullptr;   // added per row (Linear: the output features are the rows); beta == 0, no `bias`
+  __device__ __forceinline__ float rb(long m) const { return row_bias ? __ldg(row_bias + m) : 0.f; }
   static constexpr long kLastOdd = 1l << 62;
   // PAIR is a compile-time property of the problem: the common path carries none of the pair arithmetic
   template <bool PAIR = false>
@@ -718,7 +720,7 @@ struct Epilogue {
     out[mo + n * nstride] = v;
   }
   template <bool PAIR = false>
-  __device__ __forceinline__ void store(long mo, long n, float acc) const {
+  __device__ __forceinline__ void store(long mo, long n, float acc, float row_b = 0.f) const {
     if (PAIR) {
       const long par = n >= pair_K ? 1 : 0, plane = n - par * pair_K;
       if (par && (mo & kLastOdd)) return;
@@ -728,7 +730,7 @@ struct Epilogue {
       return;
     }
     const long o = mo + n * nstride;
-    float v = alpha * acc;
+    float v = alpha * acc + row_b;
     if (bias) v += bias[n];
     if (beta != 0.f) v += beta * out[o];
     out[o] = v;
@@ -819,6 +821,7 @@ __device__ __forceinline__ void tc2_store_rows(const P &p, const float (&acc)[NC
     float4 *o = reinterpret_cast<float4 *>(p.epi.out + mo + nb);
     const float alpha = p.epi.alpha, beta = p.epi.beta;
     const float *bias = p.epi.bias;
+    const float row_b = p.epi.rb(m);
 #pragma unroll
     for (int j0 = 0; j0 < NCOL; j0 += 16) {
       float4 old[4];
@@ -828,7 +831,7 @@ __device__ __forceinline__ void tc2_store_rows(const P &p, const float (&acc)[NC
         for (int q = 0; q < 4; q++) old[q] = o[j0 / 4 + q];
       }
 #pragma unroll
-      for (int j = 0; j < 16; j++) b[j] = bias ? __ldg(bias + nb + j0 + j) : 0.f;
+      for (int j = 0; j < 16; j++) b[j] = bias ? __ldg(bias + nb + j0 + j) : row_b;
 #pragma unroll
       for (int q = 0; q < 4; q++) {
         float4 v;
@@ -850,11 +853,12 @@ __device__ __forceinline__ void tc2_store_rows(const P &p, const float (&acc)[NC
       float *o = p.epi.out + mo + nb * p.epi.nstride;
       const long st = p.epi.nstride;
       const float *bias = p.epi.bias;
+      const float row_b = p.epi.rb(m);
 #pragma unroll
       for (int j0 = 0; j0 < NCOL; j0 += 16) {
         float b[16];
 #pragma unroll
-        for (int j = 0; j < 16; j++) b[j] = bias ? __ldg(bias + nb + j0 + j) : 0.f;
+        for (int j = 0; j < 16; j++) b[j] = bias ? __ldg(bias + nb + j0 + j) : row_b;
 #pragma unroll
         for (int j = 0; j < 16; j++) o[(j0 + j) * st] = alpha * acc[j0 + j] + b[j];
       }
@@ -884,11 +888,12 @@ __device__ __forceinline__ void tc2_store_rows(const P &p, const float (&acc)[NC
       }
       return;
     }
+    const float row_b = P::PAIR ? 0.f : p.epi.rb(m);
 #pragma unroll
     for (int j0 = 0; j0 < NCOL; j0 += 16) {
       float b[16];
 #pragma unroll
-      for (int j = 0; j < 16; j++) b[j] = nb + j0 + j < p.N ? p.epi.template bias_of<P::PAIR>(nb + j0 + j) : 0.f;
+      for (int j = 0; j < 16; j++) b[j] = row_b + (nb + j0 + j < p.N ? p.epi.template bias_of<P::PAIR>(nb + j0 + j) : 0.f);
 #pragma unroll
       for (int j = 0; j < 16; j++)
         if (nb + j0 + j < p.N) p.epi.template store_biased<P::PAIR>(mo, nb + j0 + j, acc[j0 + j], b[j]);
@@ -969,11 +974,12 @@ static __global__ void __launch_bounds__(256) splitk_finish_kernel(const float *
   if (m >= M) return;
   const bool pair = epi.pair_K != 0;
   const long mo = pair ? epi.moff<true>(m) : epi.moff<false>(m);
+  const float row_b = epi.rb(m);
   for (long n = blockIdx.y; n < N; n += gridDim.y) {
     float acc = 0.f;
     for (int z = 0; z < splits; z++) acc += ws[((long)z * N + n) * M + m];
     if (pair) epi.store<true>(mo, n, acc);
-    else epi.store<false>(mo, n, acc);
+    else epi.store<false>(mo, n, acc, row_b);
   }
 }
 
@@ -988,6 +994,7 @@ static __global__ void __launch_bounds__(256) tail_finish_kernel(const float *__
   if (m >= M) return;
   const bool pair = epi.pair_K != 0;
   const long mo = pair ? epi.moff<true>(m) : epi.moff<false>(m);
+  const float row_b = epi.rb(m);
   const float *base = ws + (long)blockIdx.x * splits * bn2 * 256 + threadIdx.x;
   for (int c = blockIdx.y; c < bn2; c += gridDim.y) {
     const long n = nt * bn2 + c;
@@ -995,7 +1002,7 @@ static __global__ void __launch_bounds__(256) tail_finish_kernel(const float *__
     float acc = 0.f;
     for (int z = 0; z < splits; z++) acc += base[((long)z * bn2 + c) * 256];
     if (pair) epi.store<true>(mo, n, acc);
-    else epi.store<false>(mo, n, acc);
+    else epi.store<false>(mo, n, acc, row_b);
   }
 }
 

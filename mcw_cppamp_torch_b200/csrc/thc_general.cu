@@ -193,6 +193,8 @@ void *scratch(size_t bytes) {
   return c.scratch;
 }
 
+unsigned *zero_words() { return (unsigned *)((char *)scratch(1 << 20) + (1 << 17)); }
+
 void *dev_alloc(size_t bytes) {
   if (bytes == 0) return nullptr;
   void *p = nullptr;

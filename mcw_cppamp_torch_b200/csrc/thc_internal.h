@@ -113,6 +113,10 @@ mm::StallCtl stall_ctl();         // kernel parameter of the tensor-core kernels
 unsigned *sched_counter();
 int device_if_initialised();       // -1 before the first CUDA use on this thread; never initialises
 void *scratch(size_t bytes);      // grow-only device scratch of the reductions, zero-filled when (re)allocated
+// Device words that are zero between launches: tickets of kernels that put them back to zero when they are done.  One
+// block for all of them, since the launches of a context run one after the other on its stream.
+constexpr int kZeroWords = 16384;
+unsigned *zero_words();
 void *dev_alloc(size_t bytes);    // stream-ordered allocation (caching pool): storages
 void dev_free(void *p);
 // Temporaries of one entry-point call (operand planes, split-K partials, repacked weights ...) come from a
@@ -183,7 +187,7 @@ void sgd_update_async(float *w, const float *g, float *v, long n, float lr, floa
 
 // device-side GEMM front (col-major BLAS semantics) shared by addmm / conv / Linear
 void gemm(char transa, char transb, long m, long n, long k, float alpha, const float *a, long lda,
-          const float *b, long ldb, float beta, float *c, long ldc);
+          const float *b, long ldb, float beta, float *c, long ldc, const float *row_bias = nullptr);   // bias[i] added to row i (beta 0)
 
 }  // namespace thc
 

@@ -401,12 +401,6 @@ __global__ void __launch_bounds__(256) reduce_cols4_kernel(const float *__restri
   if (gridDim.y > 1) cols_fold_if_last<MODE, 128>(w, J, (long)blockIdx.x * 128);
 }
 
-// zero-initialised words in the reductions' scratch block: the full reductions' record, then the column ranges' tickets
-struct DimScratch {
-  RedScratch all;
-  unsigned tickets[4096];
-};
-
 template <int MODE>
 static void reduce_dim(THGPUTensor *values, THGPUTensor *indices, THGPUTensor *src, long dim, float scale) {
   THC_ARG(dim >= 0 && dim < src->nDimension, 3, "dimension out of range");
@@ -502,9 +496,8 @@ static void reduce_dim(THGPUTensor *values, THGPUTensor *indices, THGPUTensor *s
       w.psum = (double *)scr;
       w.pidx = (int *)scr;
       w.pval = (float *)scr + nparts;
-      DimScratch *ds = (DimScratch *)scratch(sizeof(DimScratch));
-      THC_CHECK(colblocks * O <= (long)(sizeof(ds->tickets) / sizeof(ds->tickets[0])), "internal: too many column ranges to split");
-      w.tickets = ds->tickets;
+      THC_CHECK(colblocks * O <= kZeroWords, "internal: too many column ranges to split");
+      w.tickets = zero_words();
     }
     w.out = out; w.idx = idx; w.scale = scale;
     dim3 grid((unsigned)colblocks, (unsigned)splits, (unsigned)O), block(32, 8);

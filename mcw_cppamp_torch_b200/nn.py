@@ -320,7 +320,7 @@ class View(Module):
 
 
 class Linear(Module):
-    """mcw_nn/Linear.lua:33-94, batch mode: addr for the bias broadcast, addmm for the products."""
+    """mcw_nn/Linear.lua:33-94, batch mode: addmm for the products, the bias added in the forward product's epilogue."""
 
     def __init__(self, inputSize, outputSize, rng=None):
         super().__init__()
@@ -350,10 +350,7 @@ class Linear(Module):
     def updateOutput(self, input):
         _need_gpu(input, "Linear"); _need_gpu(self.weight, "Linear.weight")
         assert input.dim() == 2, "batch (2-D) input expected"
-        nframe, nunit = input.size(1), self.bias.size(1)
-        self.output.resize(nframe, nunit)
-        self.output.zero().addr(1, self._ones_vec(nframe), self.bias)
-        self.output.addmm(1, input, self.weight.t())
+        lib().THGPUNN_Linear_updateOutput(input._p, self.output._p, self.weight._p, self.bias._p)
         return self.output
 
     def updateGradInput(self, input, gradOutput):
