@@ -219,7 +219,9 @@ class _Lib:
         if not os.path.exists(LIB_PATH):
             raise ImportError("%s is missing: build it with `python -m mcw_cppamp_torch_b200.build` "
                               "(there is no CPU fallback)" % LIB_PATH)
+        global calls
         from . import _calls
+        calls = _calls
         self.cdll = C.CDLL(LIB_PATH)
 
         def address(fn):
@@ -251,6 +253,7 @@ class _Lib:
         return call
 
 
+calls = None    # the native module, imported with the library: the package itself imports before either is built
 _lib = None
 
 

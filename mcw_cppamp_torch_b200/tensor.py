@@ -10,7 +10,7 @@ import math
 
 import numpy as np
 
-from . import _calls
+from . import _lib
 from ._lib import (HOST_TYPES, THLongStorage, lib)
 
 # numpy dtype -> TH host type name
@@ -95,7 +95,7 @@ class GPUTensor:
 
     def size(self, d=None):
         if d is None:
-            return _calls.sizes(self._p)
+            return _lib.calls.sizes(self._p)
         return lib().THGPUTensor_size(self._p, d - 1)
 
     def stride(self, d=None):
@@ -161,7 +161,7 @@ class GPUTensor:
             sizes[k] = n // rest
         assert math.prod(sizes) == n
         r = GPUTensor()
-        _calls.set_view(r._p, self._p, tuple(sizes))
+        _lib.calls.set_view(r._p, self._p, tuple(sizes))
         return r
 
     def contiguous(self):
@@ -178,7 +178,7 @@ class GPUTensor:
         else:
             # a host tensor of any TH type: THGPUTensor_copy<Type> (gputorch/Tensor.cpp:38-65 dispatches the same way)
             a = np.asarray(src)
-            if _calls.upload(self._p, a):
+            if _lib.calls.upload(self._p, a):
                 return self
             if a.dtype not in _TH_NAME:
                 a = a.astype(np.float32)
@@ -190,7 +190,7 @@ class GPUTensor:
         shape = self.size() if self.dim() else (0,)
         if out is None:
             out = np.empty(shape, dtype)
-        if out.size and not (out.dtype == np.float32 and _calls.download(out, self._p)):
+        if out.size and not (out.dtype == np.float32 and _lib.calls.download(out, self._p)):
             name, h = _host_view(out)
             getattr(lib(), "TH%sTensor_copyGPU" % name)(C.byref(h), self._p)
         return out
