@@ -5,13 +5,11 @@
 //
 //     D(m, n) = sum_k  A(m, k) * B(n, k)          m < M, n < N, k < K
 //
-// where an operand element is found by adding a per-row and a per-k memory offset and passing a
-// small box test that realises zero padding.  That is the implicit-GEMM form of what the reference
-// does by materialising a column matrix per image and calling a generic SGEMM on it
-// (gputorch/lib/THC/gpunn-impl/SpatialConvolutionMM.cpp:10-92 im2col / col2im, :185-217 host loop;
-// operand mapping in the table of the gemm call sites :194-216, :289-300, :404-417).  The engines
-// (mm_simt.cuh: FP32 FMA; mm_tc.cuh: tcgen05 tensor cores with a 3xTF32 split) only see these
-// descriptions, so the index rules are written, and tested, exactly once.
+// which is the implicit-GEMM form of what the reference does by materialising a column matrix per image and calling a
+// generic SGEMM on it (gputorch/lib/THC/gpunn-impl/SpatialConvolutionMM.cpp:10-92 im2col / col2im, :185-217 host loop;
+// operand mapping in the table of the gemm call sites :194-216, :289-300, :404-417).  The tensor-core engine
+// (mm_tc2r.cuh) reads its operands through TMA maps; the FP32 FMA engine (mm_simt.cuh) finds an element by adding a per-row
+// and a per-k memory offset and passing a small box test that realises zero padding.
 #ifndef THC_MM_PROBLEM_CUH
 #define THC_MM_PROBLEM_CUH
 
@@ -51,7 +49,6 @@ struct FastDiv {
 
 // idx -> idx * stride
 struct LinearMap {
-  static constexpr bool kLinear = true;   // cheap enough to evaluate inline, no staging needed
   long count, stride;
   __device__ __forceinline__ Info operator()(long idx) const {
     Info r;
@@ -64,7 +61,6 @@ struct LinearMap {
 
 // idx = (img, y, x) over a [count/PP, PP/XW, XW] grid of pixels
 struct PixelMap {
-  static constexpr bool kLinear = false;
   long count;            // < 2^31 (checked by set())
   FastDiv PP, XW;
   unsigned p_valid;      // pixels of a plane that exist; indices in [p_valid, PP) are padding (zeros)
@@ -91,7 +87,6 @@ struct PixelMap {
 
 // idx = (c, i, j) over [count/kHW, kHW/kW, kW] filter taps
 struct TapMap {
-  static constexpr bool kLinear = false;
   long count;            // < 2^31 (checked by set())
   FastDiv kHW, kW;
   long c_stride, i_stride, j_stride;
@@ -116,38 +111,18 @@ struct TapMap {
 // BOX 0: valid rows/ks only.  BOX 1: additionally 0 <= y < H and 0 <= x < W (zero padding).
 // BOX 2: the summed coordinates must be non-negative multiples of (dH, dW) and the quotients index
 //        an H x W plane (gradInput of a strided convolution).
-template <class RowMap_, class KMap_, int BOX_, bool ALONG_K_>
+template <class RowMap_, class KMap_, int BOX_>
 struct Operand {
   typedef RowMap_ RowMap;
   typedef KMap_ KMap;
-  static constexpr int BOX = BOX_;
-  static constexpr bool ALONG_K = ALONG_K_;  // memory is contiguous along k (else along rows)
-  // plain matrices whose k runs are contiguous can be read 16 bytes at a time when vec4 is set
-  static constexpr bool VECTORIZABLE = ALONG_K_ && BOX_ == 0 && RowMap_::kLinear && KMap_::kLinear;
-  static constexpr bool PRESPLIT = false;
-  static constexpr bool MN_MAJOR = false;
-  static constexpr bool TMA_CAPABLE = false;
-  static constexpr bool TMA_IM2COL = false;
   const float *base;
   RowMap rows;
   KMap ks;
   int H, W, dH, dW;
-  int vec4;  // host promise: base 16-byte aligned, row stride a multiple of 4 floats, k stride 1
-  // Where element (r, k) lives, or nullptr when it is a structural zero (padding / out of range).
-  __device__ __forceinline__ const float *locate(const Info &r, const Info &k) const {
-    const int ty = r.y + k.y, tx = r.x + k.x;
-    if (BOX == 0) return ty >= 0 ? base + (r.off + k.off) : nullptr;
-    if (BOX == 1)
-      return ((unsigned)ty < (unsigned)H && (unsigned)tx < (unsigned)W) ? base + (r.off + k.off) : nullptr;
-    if (ty < 0 || tx < 0) return nullptr;
-    const int y = ty / dH, x = tx / dW;
-    if (y * dH != ty || x * dW != tx || y >= H || x >= W) return nullptr;
-    return base + (r.off + k.off + (long)y * W + x);
-  }
   __device__ __forceinline__ float fetch(const Info &r, const Info &k) const {
     const int ty = r.y + k.y, tx = r.x + k.x;
-    if (BOX == 0) return ty >= 0 ? base[r.off + k.off] : 0.f;
-    if (BOX == 1)
+    if (BOX_ == 0) return ty >= 0 ? base[r.off + k.off] : 0.f;
+    if (BOX_ == 1)
       return ((unsigned)ty < (unsigned)H && (unsigned)tx < (unsigned)W) ? base[r.off + k.off] : 0.f;
     if (ty < 0 || tx < 0) return 0.f;
     const int y = ty / dH, x = tx / dW;
@@ -156,91 +131,32 @@ struct Operand {
   }
 };
 
-// A plain matrix that a preparation pass (split_planes_kernel) has already rounded into two K-major
-// planes of TF32 values, hi and lo = tf32(x - hi), each [rows][ld] with ld a multiple of 32 floats
-// and zeros beyond the real K.  The tensor-core engine copies both planes straight into their tiles
-// (16-byte cp.async, no per-element work in the main loop).
-struct SplitOperand {
-  typedef LinearMap RowMap;
-  typedef LinearMap KMap;
-  static constexpr int BOX = 0;
-  static constexpr bool ALONG_K = true;
-  static constexpr bool VECTORIZABLE = true;
-  static constexpr bool PRESPLIT = true;
-  static constexpr bool MN_MAJOR = false;
-  static constexpr bool TMA_CAPABLE = false;
-  static constexpr bool TMA_IM2COL = false;
-  const float *base;  // hi plane (BF16 mode: one plane of BF16 values, offsets then count 4-byte units)
-  const float *lo;    // lo plane
-  RowMap rows;        // {row count, ld}
-  KMap ks;            // {ld, 1}
-  int H, W, dH, dW, vec4;
-  // optional second level along k: k = outer * k_inner + inner lives at outer * k_outer_stride + inner
-  // (k_inner a multiple of 32, so a k tile never straddles two outer blocks); k_inner.d == 0: plain
-  FastDiv k_inner;
-  long k_outer_stride;
-  __device__ __forceinline__ long ktile_off(long k0) const {
-    if (k_inner.d == 0) return k0;
-    unsigned q, r;
-    k_inner.divmod((unsigned)k0, q, r);
-    return (long)q * k_outer_stride + r;
-  }
-  // what 16-byte chunk `chunk` of the 32-k tile starting at k0 adds to a row's offset / box coordinates
-  __device__ __forceinline__ Info ktile(long k0, int chunk) const {
-    Info t;
-    t.off = ktile_off(k0) + chunk * 4; t.y = 0; t.x = 0;
-    return t;
-  }
-  __device__ __forceinline__ bool valid(const Info &r, const Info &) const { return r.y >= 0; }
-  __device__ __forceinline__ float fetch(const Info &r, const Info &k) const {
-    return (r.y | k.y) >= 0 ? base[r.off + k.off] + lo[r.off + k.off] : 0.f;
-  }
-  __device__ __forceinline__ const float *locate(const Info &r, const Info &k) const {
-    return (r.y | k.y) >= 0 ? base + (r.off + k.off) : nullptr;
-  }
+// ---------------------------------------------------------------------------------------------
+// Operands of the two-SM engine, all fetched by TMA.  A tile row holds one swizzle span of 128 bytes: KV = 32 FP32 values
+// (3xTF32 products) or 64 BF16 values.
+//
+// A plain matrix: K-major (memory runs along k) or MN-major (memory runs along the rows).  tmap: K-major {K, rows} with
+// a {KV, tile rows} box and the 128-byte swizzle; MN-major {rows, K} with a {KV rows, KV k} box per KV-row block (FP32: the
+// 32-byte-granule swizzle).  Elements beyond either extent read as zeros.
+template <bool MN_>
+struct RawOperand {
+  static constexpr bool MN_MAJOR = MN_;
+  CUtensorMap tmap;
 };
 
-
-// ---------------------------------------------------------------------------------------------
-// Channels-last hi / lo planes of an activation tensor: P[img][y][x][c], c contiguous and padded with zero
-// planes to a multiple of 4, every value already rounded to TF32 (hi) and tf32(x - hi) (lo) by
-// nchw_to_planes_kernel.  With channels innermost, a 16-byte chunk of the implicit column matrix is ONE
-// filter tap and 4 consecutive channels, so the tensor-core engine fills its tiles with 16-byte copies
-// and one box test per (pixel, chunk) instead of per element; with 32 or more channels a whole 32-k tile
-// (128 contiguous bytes per pixel) belongs to one tap.  Tensor-core engine only (no fetch()).
-//
-// Window view (K-major): row = pixel (img, y, x) of the product's output grid, k = (i, j, c); K is
-// taps * C rounded up to 32, the tail reads as zero.
+// Convolution windows over a channels-last plane [n_img][H][W][C] (C a multiple of KV), as rows (K-major): row = window (img,
+// y, x) of the product's grid, k = (i, j, c).  tmap: im2col map {C, W, H, n_img}, KV channels of 128 consecutive windows at
+// one filter tap per load, padding read as zeros.
 struct PlanesWindowOperand {
-  typedef PixelMap RowMap;
-  typedef LinearMap KMap;   // unused; k chunks are decoded by ktile()
-  static constexpr int BOX = 1;
-  static constexpr bool ALONG_K = true;
-  static constexpr bool VECTORIZABLE = true;
-  static constexpr bool PRESPLIT = true;
   static constexpr bool MN_MAJOR = false;
-  static constexpr bool TMA_CAPABLE = true;
-  static constexpr bool TMA_IM2COL = true;
-  // When use_tma is set (one FP32 plane, raw-operand engine), tmap is an im2col tensor map over the plane seen
-  // as a channels-last tensor {C, W, H, n_img}: 32 channels of 128 consecutive windows per load, the 128-byte
-  // swizzle of the operand tiles, padding read as zeros: one TMA load per k tile (one tap, 32 channels).
   CUtensorMap tmap;
-  int use_tma;
-  int n_img;                // images per plane
-  int n_planes;             // 2: hi / lo planes; 1: one plane of FP32 values (raw-operand engine)
-  FastDiv ctiles;           // C / 32 (TMA form only)
-  const float *base, *lo;
-  RowMap rows;              // off = plane offset of the window's top-left pixel, (y, x) = its coordinates
-  KMap ks;
-  int H, W, dH, dW, vec4;   // H x W: the plane's pixel grid (box test)
-  FastDiv cquads;           // C / 4
-  FastDiv kW;
-  unsigned taps;            // kH * kW
-  long i_stride, j_stride;  // W*C, C
-  // Window corner (x, y) and image of row m, the start coordinates of an im2col load; rows past the end map
-  // beyond the last image, where every read is out of bounds (zeros).
+  int n_img;
+  PixelMap rows;            // window -> coordinates of its corner
+  FastDiv ctiles, kW;       // C / KV
+  // Corner (x, y) and image of row m, the start coordinates of an im2col load; rows past the end map beyond the last
+  // image, where every read is out of bounds (zeros).
   __device__ __forceinline__ void tile_origin(long m, int &x, int &y, int &img) const {
-    if (m >= rows.count) { x = rows.x0; y = rows.y0; img = n_planes * n_img; return; }
+    if (m >= rows.count) { x = rows.x0; y = rows.y0; img = n_img; return; }
     unsigned im, px, yy, xx;
     rows.PP.divmod((unsigned)m, im, px);
     rows.XW.divmod(px, yy, xx);
@@ -248,55 +164,22 @@ struct PlanesWindowOperand {
     y = (int)yy * rows.sy + rows.y0;
     img = (int)im;
   }
-  // Tap (i, j) and first channel of the k tile starting at k0.
-  __device__ __forceinline__ void tile_tap(long k0, int &i, int &j, int &c0) const {
+  // Tap (i, j) and channel tile of k tile t.
+  __device__ __forceinline__ void tile_tap(unsigned t, int &i, int &j, int &ct) const {
     unsigned tap, cb, ii, jj;
-    ctiles.divmod((unsigned)(k0 >> 5), tap, cb);
+    ctiles.divmod(t, tap, cb);
     kW.divmod(tap, ii, jj);
-    i = (int)ii; j = (int)jj; c0 = (int)cb * 32;
-  }
-  __device__ __forceinline__ Info ktile(long k0, int chunk) const {
-    unsigned tap, cq, i, j;
-    cquads.divmod((unsigned)(k0 >> 2) + (unsigned)chunk, tap, cq);
-    kW.divmod(tap, i, j);
-    Info t;
-    t.off = (long)i * i_stride + (long)j * j_stride + (long)cq * 4;
-    t.y = tap < taps ? (int)i : kInvalid;
-    t.x = (int)j;
-    return t;
-  }
-  __device__ __forceinline__ bool valid(const Info &r, const Info &t) const {
-    return (unsigned)(r.y + t.y) < (unsigned)H && (unsigned)(r.x + t.x) < (unsigned)W;
+    i = (int)ii; j = (int)jj; ct = (int)cb;
   }
 };
 
-// A plain FP32 matrix read by TMA alone (raw-operand engine, mm_tc2r.cuh): K-major (memory runs along k) or
-// MN-major (memory runs along the rows).  tmap: K-major {K, rows} with a {32 k, tile rows} box and the 128-byte
-// swizzle; MN-major {rows, K} with a {32 rows, 32 k} box per 32-row block and the 32-byte-granule swizzle.
-// Elements beyond either extent read as zeros.
-template <bool MN_>
-struct RawOperand {
-  static constexpr bool PRESPLIT = true;
-  static constexpr bool MN_MAJOR = MN_;
-  static constexpr bool TMA_CAPABLE = true;
-  static constexpr bool TMA_IM2COL = false;
-  CUtensorMap tmap;
-  int use_tma;
-};
-
-// Input windows of a convolution as the MN-major operand of the weight-gradient product, read by TMA alone
-// (raw-operand engine): rows = (tap, c) of one channels-last FP32 plane [n_img][H][W][C], C % 32 == 0,
-// k = output pixels.  tmap: im2col map {C, W, H, n_img}, 32 channels of 32 consecutive windows per load (one
-// 32-row block of a k tile), the 32-byte-granule swizzle.
+// The same windows as the MN-major operand of the weight-gradient product: rows = (tap, c), k = windows.  tmap: im2col
+// map, KV channels of KV consecutive windows per load (one KV-row block of a k tile).
 struct WindowRowsOperand {
-  static constexpr bool PRESPLIT = true;
   static constexpr bool MN_MAJOR = true;
-  static constexpr bool TMA_CAPABLE = true;
-  static constexpr bool TMA_IM2COL = false;
   CUtensorMap tmap;
-  int use_tma;
   int n_img;
-  PixelMap ks;              // output pixel -> window corner
+  PixelMap ks;              // window -> coordinates of its corner
   FastDiv C, kW;
   __device__ __forceinline__ void pixel_origin(long k, int &x, int &y, int &img) const {
     if (k >= ks.count) { x = ks.x0; y = ks.y0; img = n_img; return; }
@@ -315,108 +198,67 @@ struct WindowRowsOperand {
   }
 };
 
-// A pixel map cheap enough for every thread to evaluate for itself once per stage.
-struct InlinePixelMap : PixelMap {
-  static constexpr bool kLinear = true;
-};
-
-// Pixel view (MN-major): k = pixel (img, y, x) of the reduction grid, row = (tap, c) (TAPS) or just c.
-// Memory runs along the rows, which tcgen05 reads as an "MN-major" operand: the tile is stored as
-// [32-channel block][32 pixels][128 bytes] and the instruction descriptor carries the transpose bit.
-// This is the weight-gradient form: both gradOutput and the input windows are reduced over pixels.
-template <bool TAPS_>
-struct PlanesPixelOperand {
-  typedef LinearMap RowMap;
-  typedef InlinePixelMap KMap;
-  static constexpr int BOX = 1;
-  static constexpr bool ALONG_K = false;
-  static constexpr bool VECTORIZABLE = true;
-  static constexpr bool PRESPLIT = true;
-  static constexpr bool MN_MAJOR = true;
-  static constexpr bool TMA_CAPABLE = false;
-  static constexpr bool TMA_IM2COL = false;
-  static constexpr bool TAPS = TAPS_;
-  const float *base, *lo;
-  RowMap rows;              // {row count, 1}
-  KMap ks;                  // pixel -> plane offset of the window's top-left pixel + its coordinates
-  int H, W, dH, dW, vec4;
-  FastDiv C;                // channels per tap (rows = taps * C)
-  FastDiv kW;
-  long i_stride, j_stride;
-  __device__ __forceinline__ Info rowblock(long r0) const {   // 4-row chunk starting at r0 (never straddles a tap)
-    Info t;
-    if (!TAPS) { t.off = r0; t.y = 0; t.x = 0; return t; }
-    unsigned tap, c, i, j;
-    C.divmod((unsigned)r0, tap, c);
-    kW.divmod(tap, i, j);
-    t.off = (long)i * i_stride + (long)j * j_stride + (long)c;
-    t.y = (int)i; t.x = (int)j;
-    return t;
-  }
-  __device__ __forceinline__ bool valid(const Info &px, const Info &t) const {
-    return (unsigned)(px.y + t.y) < (unsigned)H && (unsigned)(px.x + t.x) < (unsigned)W;
-  }
-};
-
-// NCHW fp32 -> channels-last hi / lo planes.  One 32-channel x 32-pixel tile per step through shared
-// memory: reads coalesced along pixels, writes coalesced along channels.  C % 32 == 0.
+// ---------------------------------------------------------------------------------------------
+// Channels-last planes of an activation tensor, FP32 or BF16, channels padded with zeros to Cp = a multiple of KV.
+//
+// NCHW fp32 -> [img][pixel][Cp].  CT channels x PT pixels per pass through shared memory, sixteen loads per thread in flight
+// before the barrier (32 x 32 tiles with four left the kernel at half the HBM rate): reads coalesced along pixels, writes in
+// whole 128-byte lines along channels.
 // `chan_partial` (optional): [gridDim.x][C] sums over the pixels this block transposed, per channel -- the gradBias
 // reduction of a convolution rides on the transposition of gradOutput instead of reading the tensor a second time.
 // A channel of a tile belongs to one warp, tiles are taken in a fixed order, so the sums are reproducible.
-static __global__ void __launch_bounds__(256) nchw_to_planes_kernel(const float *__restrict__ src, long N, long C, long HW,
-                                                                    float *__restrict__ hi, float *__restrict__ lo,
-                                                                    float *__restrict__ chan_partial) {
-  // 32 channels x 128 pixels per pass: sixteen loads per thread in flight before the barrier (32 x 32 tiles with
-  // four left the kernel at half the HBM rate)
-  constexpr int PT = 128;
-  __shared__ float tile[32][PT + 1];
+template <bool HALF>
+static __global__ void __launch_bounds__(256) nchw_to_planes_kernel(const float *__restrict__ src, long N, int C, int HW, int Cp,
+                                                                    void *__restrict__ dst, float *__restrict__ chan_partial) {
+  constexpr int CT = HALF ? 64 : 32, PT = HALF ? 64 : 128;
+  __shared__ float tile[CT][PT + 1];
   extern __shared__ float chan_sum[];   // [C] when chan_partial is given
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-  const long ptiles = (HW + PT - 1) / PT, ctiles = C / 32;
+  const unsigned ptiles = (unsigned)((HW + PT - 1) / PT), ctiles = (unsigned)(Cp / CT);
   const long ntiles = N * ptiles * ctiles;
   if (chan_partial) {
-    for (long c = threadIdx.x; c < C; c += blockDim.x) chan_sum[c] = 0.f;
+    for (int c = threadIdx.x; c < C; c += blockDim.x) chan_sum[c] = 0.f;
     __syncthreads();
   }
   for (long t = blockIdx.x; t < ntiles; t += gridDim.x) {
-    const long pt = t % ptiles, q = t / ptiles, ct = q % ctiles, img = q / ctiles;
-    const long p0 = pt * PT, c0 = ct * 32;
-    const float *s = src + (img * C + c0) * HW + p0;
-    const int np = HW - p0 < PT ? (int)(HW - p0) : PT;
+    const unsigned r = (unsigned)(t % (ptiles * ctiles));
+    const long img = t / (ptiles * ctiles);
+    const int ct = (int)(r / ptiles), p0 = (int)(r - ct * ptiles) * PT, c0 = ct * CT;
+    const int np = min(HW - p0, PT), nc = min(C - c0, CT);
+    const float *s = src + (img * C + c0) * HW + p0 + tx;
+    float v[CT / 8][PT / 32];
 #pragma unroll
-    for (int j = ty; j < 32; j += 8) {
+    for (int j = 0; j < CT / 8; j++)
+#pragma unroll
+      for (int g = 0; g < PT / 32; g++)
+        v[j][g] = (g * 32 + tx < np && ty + 8 * j < nc) ? s[(long)(ty + 8 * j) * HW + g * 32] : 0.f;
+#pragma unroll
+    for (int j = 0; j < CT / 8; j++) {
       float part = 0.f;
 #pragma unroll
-      for (int g = 0; g < PT; g += 32) {
-        const float v = (g + tx < np) ? s[(long)j * HW + g + tx] : 0.f;
-        tile[j][g + tx] = v;
-        part += v;
+      for (int g = 0; g < PT / 32; g++) {
+        tile[ty + 8 * j][g * 32 + tx] = v[j][g];
+        part += v[j][g];
       }
       if (chan_partial) {
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
-        if (tx == 0) chan_sum[c0 + j] += part;
+        if (tx == 0 && ty + 8 * j < nc) chan_sum[c0 + ty + 8 * j] += part;
       }
     }
     __syncthreads();
-#pragma unroll 4
+    const long o0 = (img * HW + p0) * Cp + c0;
+#pragma unroll 8
     for (int j = ty; j < np; j += 8) {
-      const float x = tile[tx][j];
-      const long o = (img * HW + p0 + j) * C + c0 + tx;
-      if (lo) {
-        unsigned h, l;
-        asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(h) : "f"(x));
-        const float xl = x - __uint_as_float(h);
-        asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(l) : "f"(xl));
-        hi[o] = __uint_as_float(h); lo[o] = __uint_as_float(l);
-      } else {
-        hi[o] = x;   // one plane of plain FP32 values (raw-operand engine)
-      }
+      if constexpr (HALF)
+        reinterpret_cast<__nv_bfloat162 *>(dst)[(o0 + (long)j * Cp) / 2 + tx] = __floats2bfloat162_rn(tile[2 * tx][j], tile[2 * tx + 1][j]);
+      else
+        reinterpret_cast<float *>(dst)[o0 + (long)j * Cp + tx] = tile[tx][j];
     }
     __syncthreads();
   }
   if (chan_partial)
-    for (long c = threadIdx.x; c < C; c += blockDim.x) chan_partial[(long)blockIdx.x * C + c] = chan_sum[c];
+    for (int c = threadIdx.x; c < C; c += blockDim.x) chan_partial[(long)blockIdx.x * C + c] = chan_sum[c];
 }
 // out[c] += scale * sum_b partial[b][c]: 32 row slices per channel (one warp each, eight loads in flight per
 // thread), folded in a fixed order.  The partials are a few MB at most; what this kernel costs is the chain of
@@ -450,223 +292,224 @@ static __global__ void __launch_bounds__(1024) chan_partial_finish_kernel(const 
   }
 }
 
-// The same for channel counts that are not multiples of 32: one thread per pixel walks the planes (reads
-// coalesced across threads) and writes its pixel's Cp = round_up(C, 4) channels 16 bytes at a time.
-static __global__ void __launch_bounds__(256) nchw_to_planes_any_kernel(const float *__restrict__ src, long N, long C, long HW,
-                                                                        long Cp, float *__restrict__ hi, float *__restrict__ lo) {
-  const long total = N * HW;
-  const long nthreads = (long)gridDim.x * blockDim.x;
-  for (long t = (long)blockIdx.x * blockDim.x + threadIdx.x; t < total; t += nthreads) {
-    const long img = t / HW, px = t - img * HW;
-    const float *s = src + img * C * HW + px;
-    for (long c0 = 0; c0 < Cp; c0 += 4) {
-      float h[4], l[4];
+
+// A convolution layer restated over "cells": pixel (Y, X) of the restated input carries, as channels, the eH x eW input
+// pixels at offsets (dy, dx) from (Y * dH - pad, X * dW - pad), all planes of each:
+//   S[n][Y][X][ch = (dy * eW + dx) * Cq + c] = in[n][c][Y * dH + dy - pad][X * dW + dx - pad]
+// and filter tap (i, j) is tap ((i - dy) / stepH, (j - dx) / stepW) at the channels of (dy, dx).  Per axis either
+//   fold    e = min(d, k): the pixels of a stride cell become channels, ceil(k / d) taps remain, or
+//   unfold  e = k: one tap remains (along both axes: the column matrix).
+// `direct`: the input's own planes (e = 1, all taps, stride and padding left to the TMA window map).
+// Which one costs least depends on how far the channel count is from a multiple of KV: see restate() in gpunn_conv.cu.
+struct Cells {
+  int C, kH, kW, dH, dW, pad;      // the layer
+  int H, W;
+  int eH, eW, kHs, kWs, stepH, stepW;
+  int Cq;                          // channels per offset: C, or padded where that costs no further span
+  int Cr, Cs;                      // eH * eW * Cq, and that padded to a multiple of KV
+  int Hs, Ws;                      // grid of S
+  bool direct;
+  // place of channel `ch`; false: padding
+  __host__ __device__ __forceinline__ bool channel(int ch, int &c, int &dy, int &dx) const {
+    const int q = ch / Cq;
+    c = ch - q * Cq;
+    dy = q / eW;
+    dx = q - dy * eW;
+    return ch < Cr && c < C;
+  }
+};
+
+// S of one image row per block.  A thread produces 16 bytes of a pixel: 4 FP32 or 8 BF16 channels, whose source offsets it
+// looks up in a table; neighbouring threads hold neighbouring channels, i.e. neighbouring columns of a few input rows.
+template <bool HALF>
+static __global__ void __launch_bounds__(256) cells_input_kernel(const float *__restrict__ in, void *__restrict__ S, const Cells u) {
+  constexpr int V = HALF ? 8 : 4;
+  extern __shared__ int2 chan_src[];      // per channel: offset in the image, (dy << 16 | dx) or -1
+  for (int ch = threadIdx.x; ch < u.Cs; ch += blockDim.x) {
+    int c, dy, dx;
+    chan_src[ch] = u.channel(ch, c, dy, dx) ? make_int2((c * u.H + dy) * u.W + dx, dy << 16 | dx) : make_int2(0, -1);
+  }
+  __syncthreads();
+  const long n = blockIdx.x / u.Hs;
+  const int Y = (int)(blockIdx.x - n * u.Hs);
+  const int q = u.Cs / V, chunks = u.Ws * q, y0 = Y * u.dH - u.pad;
+  const float *img = in + n * u.C * (long)u.H * u.W;
+  uint4 *dst = reinterpret_cast<uint4 *>(S) + ((n * u.Hs + Y) * u.Ws) * (long)q;
+  for (int o = threadIdx.x; o < chunks; o += blockDim.x) {
+    const int X = o / q, ch0 = (o - X * q) * V, x0 = X * u.dW - u.pad;
+    const float *base = img + (long)y0 * u.W + x0;
+    float v[V];
 #pragma unroll
-      for (int e = 0; e < 4; e++) {
-        const float x = c0 + e < C ? s[(c0 + e) * HW] : 0.f;
-        unsigned hh, ll;
-        asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(hh) : "f"(x));
-        const float xl = x - __uint_as_float(hh);
-        asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(ll) : "f"(xl));
-        h[e] = lo ? __uint_as_float(hh) : x; l[e] = __uint_as_float(ll);
-      }
-      *reinterpret_cast<float4 *>(hi + t * Cp + c0) = make_float4(h[0], h[1], h[2], h[3]);
-      if (lo) *reinterpret_cast<float4 *>(lo + t * Cp + c0) = make_float4(l[0], l[1], l[2], l[3]);
+    for (int e = 0; e < V; e++) {
+      const int2 s = chan_src[ch0 + e];
+      const int y = y0 + (s.y >> 16), x = x0 + (s.y & 0xffff);
+      v[e] = s.y >= 0 && (unsigned)y < (unsigned)u.H && (unsigned)x < (unsigned)u.W ? __ldg(base + s.x) : 0.f;
+    }
+    if constexpr (HALF) {
+      __nv_bfloat162 h[4];
+#pragma unroll
+      for (int e = 0; e < 4; e++) h[e] = __floats2bfloat162_rn(v[2 * e], v[2 * e + 1]);
+      dst[o] = *reinterpret_cast<const uint4 *>(h);
+    } else {
+      dst[o] = make_uint4(__float_as_uint(v[0]), __float_as_uint(v[1]), __float_as_uint(v[2]), __float_as_uint(v[3]));
     }
   }
 }
 
-// Weight matrix W[ko][(c, tap)] -> hi / lo planes in the k order of the planes operands, channel counts
-// padded to multiples of 4 (Cp, Kp) and rows to `ld` floats (a multiple of 32); padding is zero.
-//   flip == 0: out[ko][(tap, c)],          rows = K, row length taps * Cp   (forward: k = (i, j, c))
-//   flip == 1: out[c][(kHW-1-tap, ko)],    rows = C, row length taps * Kp   (gradInput as a forward pass over
-//              gradOutput with the filter rotated by 180 degrees: k = (i', j', ko))
-// pair_shift > 0 (pixel-pair mode, see Epilogue): the filter is widened to kWe = kW + pair_shift columns and
+// The column matrix in BF16 with eight channels per tap (Cq = 8, C <= 8): 16 bytes of S are one tap of one pixel.  A block makes
+// the rows of one output row: the kH input rows it needs go to shared memory once, as 16-byte pixels, and leave from there
+// kH * kW times over, so that the kernel is bound by the writes (gathering each value from the image took four times as
+// long: 1105 -> 280 us for 256 images under the 11 x 11 / 4 filter, 1.6 GB).
+static __global__ void __launch_bounds__(256) columns8_kernel(const float *__restrict__ in, uint4 *__restrict__ S, const Cells u) {
+  extern __shared__ uint4 px_rows[];   // [kH][W + 2 pad]
+  const long n = blockIdx.x / u.Hs;
+  const int Y = (int)(blockIdx.x - n * u.Hs), Wp = u.W + 2 * u.pad, taps = u.kH * u.kW, q = u.Cs / 8;
+  const float *img = in + n * u.C * (long)u.H * u.W;
+  for (int t = threadIdx.x; t < u.kH * Wp; t += blockDim.x) {
+    const int i = t / Wp, y = Y * u.dH + i - u.pad, x = t - i * Wp - u.pad;
+    float v[8];
+#pragma unroll
+    for (int c = 0; c < 8; c++)
+      v[c] = c < u.C && (unsigned)y < (unsigned)u.H && (unsigned)x < (unsigned)u.W ? __ldg(img + ((long)c * u.H + y) * u.W + x) : 0.f;
+    __nv_bfloat162 h[4];
+#pragma unroll
+    for (int e = 0; e < 4; e++) h[e] = __floats2bfloat162_rn(v[2 * e], v[2 * e + 1]);
+    px_rows[t] = *reinterpret_cast<const uint4 *>(h);
+  }
+  __syncthreads();
+  uint4 *dst = S + (n * u.Hs + Y) * u.Ws * (long)q;
+  const int chunks = u.Ws * q, step_x = (int)blockDim.x / q, step_t = (int)blockDim.x - step_x * q;
+  int X = (int)threadIdx.x / q, tap = (int)threadIdx.x - X * q;
+  for (int o = threadIdx.x; o < chunks; o += blockDim.x) {
+    const int i = tap / u.kW, j = tap - i * u.kW;
+    dst[o] = tap < taps ? px_rows[i * Wp + X * u.dW + j] : make_uint4(0, 0, 0, 0);
+    X += step_x; tap += step_t;
+    if (tap >= q) { tap -= q; X++; }
+  }
+}
+
+// Weights of the restated layer in the k order of the window operand, four values per thread:
+//   FLIP false: out[ko][(bi, bj, ch)]           (forward)
+//   FLIP true : out[ch][(bi', bj', ko)], bi' = kHs - 1 - bi: gradInput as a forward pass over gradOutput (channels padded to
+//               `chans`) under the filter rotated by 180 degrees
+// pair_shift > 0 (pixel-pair mode, see Epilogue): the filter is widened to kWs + pair_shift columns and
 // stored twice, rows [0, rows) as it is (output parity 0) and rows [rows, 2 rows) shifted right by pair_shift
 // columns (parity 1, whose window starts one stride later); the new columns are zero.
-static __global__ void __launch_bounds__(256) repack_weight_planes_kernel(const float *__restrict__ w, long K, long C, long kHW,
-                                                                          long Cp, long Kp, long ld, int flip, int kW,
-                                                                          int pair_shift, float *__restrict__ hi,
-                                                                          float *__restrict__ lo) {
-  const long rows = flip ? C : K;
-  const long total = (pair_shift ? 2 : 1) * rows * ld;
-  const long nthreads = (long)gridDim.x * blockDim.x;
-  const long chans = flip ? Kp : Cp;
-  const long kWe = kW + pair_shift, kH = kHW / kW;
-  for (long t = (long)blockIdx.x * blockDim.x + threadIdx.x; t < total; t += nthreads) {
-    long r = t / ld;
-    const long k = t - r * ld;
-    const long par = r >= rows ? 1 : 0;
+template <bool HALF, bool FLIP>
+static __global__ void __launch_bounds__(256) repack_weight_kernel(const float *__restrict__ w, const Cells u, int K, int rows, int chans,
+                                                                   int pair_shift, void *__restrict__ out) {
+  const int kWe = u.kWs + pair_shift, quads = u.kHs * kWe * (chans / 4);
+  const unsigned total = (unsigned)((pair_shift ? 2 : 1) * rows) * (unsigned)quads;
+  for (unsigned t = blockIdx.x * blockDim.x + threadIdx.x; t < total; t += gridDim.x * blockDim.x) {
+    int r = (int)(t / (unsigned)quads);
+    const int k = (int)(t - (unsigned)r * quads) * 4, tap = k / chans, k0 = k - tap * chans;
+    const int par = r >= rows ? 1 : 0;
     r -= par * rows;
-    const long tape = k / chans, ch = k - tape * chans;       // tap in the widened filter
-    const long i = tape / kWe, j = tape - i * kWe - par * pair_shift;
-    float x = 0.f;
-    if (i < kH && j >= 0 && j < kW) {
-      const long tap = i * kW + j;
-      if (!flip) { if (ch < C) x = w[(r * C + ch) * kHW + tap]; }
-      else if (ch < K) x = w[(ch * C + r) * kHW + (kHW - 1 - tap)];
-    }
-    unsigned h, l;
-    asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(h) : "f"(x));
-    const float xl = x - __uint_as_float(h);
-    asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(l) : "f"(xl));
-    if (lo) { hi[t] = __uint_as_float(h); lo[t] = __uint_as_float(l); }
-    else hi[t] = x;
-  }
-}
-
-// gradW[ko][(c, tap)] += scale * tmp[ko][(tap, c)], tmp rows of length kHW * Cp (channels padded to Cp)
-static __global__ void __launch_bounds__(256) unpack_grad_weight_kernel(const float *__restrict__ tmp, float *__restrict__ gw,
-                                                                        long K, long C, long kHW, long Cp, float scale) {
-  const long total = K * C * kHW;
-  const long nthreads = (long)gridDim.x * blockDim.x;
-  for (long t = (long)blockIdx.x * blockDim.x + threadIdx.x; t < total; t += nthreads) {
-    const long tap = t % kHW, q = t / kHW, c = q % C, ko = q / C;
-    gw[t] += scale * tmp[(ko * kHW + tap) * Cp + c];
-  }
-}
-
-
-// ---------------------------------------------------------------------------------------------
-// BF16 planes (math mode 2): the same layouts with one plane of BF16 values; rows are padded so that a row
-// is a whole number of 16-byte chunks (8 values), k extents to 64 values.
-//
-// NCHW fp32 -> channels-last BF16 plane [N * HW][Cp], Cp a multiple of 8.  One thread per pixel.
-static __global__ void __launch_bounds__(256) nchw_to_planes_bf16_kernel(const float *__restrict__ src, long N, long C, long HW,
-                                                                         long Cp, __nv_bfloat16 *__restrict__ out) {
-  const long total = N * HW;
-  const long nthreads = (long)gridDim.x * blockDim.x;
-  for (long t = (long)blockIdx.x * blockDim.x + threadIdx.x; t < total; t += nthreads) {
-    const long img = t / HW, px = t - img * HW;
-    const float *s = src + img * C * HW + px;
-    for (long c0 = 0; c0 < Cp; c0 += 8) {
-      __align__(16) __nv_bfloat16 v[8];
+    int bi = tap / kWe, bj = tap - bi * kWe - par * pair_shift;
+    if (FLIP) { bi = u.kHs - 1 - bi; bj = u.kWs - 1 - bj; }
+    float v[4];
 #pragma unroll
-      for (int e = 0; e < 8; e++) v[e] = __float2bfloat16(c0 + e < C ? s[(c0 + e) * HW] : 0.f);
-      *reinterpret_cast<uint4 *>(out + t * Cp + c0) = *reinterpret_cast<const uint4 *>(v);
+    for (int e = 0; e < 4; e++) {
+      const int ch = FLIP ? r : k0 + e, ko = FLIP ? k0 + e : r;
+      int c, dy, dx;
+      const bool real = u.channel(ch, c, dy, dx);
+      const int i = dy + bi * u.stepH, j = dx + bj * u.stepW;
+      v[e] = real && ko < K && bj >= 0 && bj < u.kWs && i < u.kH && j < u.kW ? w[(((long)ko * u.C + c) * u.kH + i) * u.kW + j] : 0.f;
+    }
+    if constexpr (HALF) {
+      const __nv_bfloat162 a = __floats2bfloat162_rn(v[0], v[1]), b = __floats2bfloat162_rn(v[2], v[3]);
+      reinterpret_cast<uint2 *>(out)[t] = make_uint2(*reinterpret_cast<const unsigned *>(&a), *reinterpret_cast<const unsigned *>(&b));
+    } else {
+      reinterpret_cast<float4 *>(out)[t] = make_float4(v[0], v[1], v[2], v[3]);
     }
   }
 }
-// The same for C % 32 == 0 through 32 x 32 shared-memory tiles (reads coalesced along pixels, writes along channels).
-static __global__ void __launch_bounds__(256) nchw_to_planes_bf16_tiled_kernel(const float *__restrict__ src, long N, long C,
-                                                                               long HW, __nv_bfloat16 *__restrict__ out) {
-  __shared__ float tile[32][33];
-  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-  const long ptiles = (HW + 31) / 32, ctiles = C / 32;
-  const long ntiles = N * ptiles * ctiles;
-  for (long t = blockIdx.x; t < ntiles; t += gridDim.x) {
-    const long pt = t % ptiles, q = t / ptiles, ct = q % ctiles, img = q / ctiles;
-    const long p0 = pt * 32, c0 = ct * 32;
-    const float *s = src + (img * C + c0) * HW + p0;
-#pragma unroll
-    for (int j = ty; j < 32; j += 8) tile[j][tx] = (p0 + tx < HW) ? s[(long)j * HW + tx] : 0.f;
-    __syncthreads();
-    // thread (pixel row j, channel pair tx % 16): two passes of 16 pixel rows
-#pragma unroll
-    for (int j = ty * 2 + (tx >> 4); j < 32; j += 16) {
-      if (p0 + j < HW) {
-        const int cp = (tx & 15) * 2;
-        const __nv_bfloat162 v = __floats2bfloat162_rn(tile[cp][j], tile[cp + 1][j]);
-        *reinterpret_cast<__nv_bfloat162 *>(out + (img * HW + p0 + j) * C + c0 + cp) = v;
-      }
-    }
-    __syncthreads();
+
+// gw[ko][(c, i, j)] += scale * T at the restated tap and channel of (c, i, j).  ko_stride, ch_stride, bi_stride, bj_stride: where T
+// keeps them (bj counted from the other end when bj_stride is negative: `first` is then the place of tap (0, 0)).
+// `copies` partial sums of each, copy_stride apart.
+struct WgradPlace { long ko_stride, ch_stride, bi_stride, bj_stride, first; int copies; long copy_stride; };
+static __global__ void __launch_bounds__(256) unpack_grad_weight_kernel(const float *__restrict__ T, float *__restrict__ gw, const Cells u,
+                                                                        int K, const WgradPlace p, float scale) {
+  const unsigned kHW = (unsigned)(u.kH * u.kW), per = (unsigned)u.C * kHW, total = (unsigned)K * per;
+  for (unsigned t = blockIdx.x * blockDim.x + threadIdx.x; t < total; t += gridDim.x * blockDim.x) {
+    const unsigned ko = t / per, r = t - ko * per, c = r / kHW, tap = r - c * kHW, i = tap / (unsigned)u.kW, j = tap - i * u.kW;
+    const int bi = u.kHs > 1 ? (int)i / u.stepH : 0, bj = u.kWs > 1 ? (int)j / u.stepW : 0;
+    const int dy = (int)i - bi * u.stepH, dx = (int)j - bj * u.stepW;
+    const long ch = (dy * u.eW + dx) * u.Cq + (int)c;
+    const float *s = T + (p.first + ko * p.ko_stride + ch * p.ch_stride + bi * p.bi_stride + bj * p.bj_stride);
+    float sum = *s;
+    for (int q = 1; q < p.copies; q++) sum += s[q * p.copy_stride];
+    gw[t] += scale * sum;
   }
 }
-// BF16 plane of a strided matrix: element (r, k) at src[r*rs + k*ks]; out [rows][ld], zero for k >= K.
+
+// gin[n][c][h][w] = gS[n][ch][Y][X], the inverse of a fold along both axes (a bijection between the input pixels that any
+// window reaches and the cells' channels; the others get zero).  gS: [N][Cr][Hs][Ws].
+static __global__ void __launch_bounds__(256) unfold_grad_input_kernel(const float *__restrict__ gS, float *__restrict__ gin, long N,
+                                                                       const Cells u) {
+  const unsigned HW = (unsigned)(u.H * u.W);
+  const long planes = N * u.C;
+  for (long pl = blockIdx.y; pl < planes; pl += gridDim.y) {
+    const long n = pl / u.C;
+    const int c = (int)(pl - n * u.C);
+    const float *src = gS + n * u.Cr * (long)(u.Hs * u.Ws);
+    for (unsigned t = blockIdx.x * blockDim.x + threadIdx.x; t < HW; t += gridDim.x * blockDim.x) {
+      const int h = (int)(t / (unsigned)u.W) + u.pad, w = (int)(t % (unsigned)u.W) + u.pad;
+      const int Y = h / u.dH, dy = h - Y * u.dH, X = w / u.dW, dx = w - X * u.dW;
+      float v = 0.f;
+      if (Y < u.Hs && X < u.Ws && dy < u.eH && dx < u.eW) v = src[((long)((dy * u.eW + dx) * u.Cq + c) * u.Hs + Y) * u.Ws + X];
+      gin[pl * HW + t] = v;
+    }
+  }
+}
+
+// BF16 plane of a strided matrix: element (r, k) at src[r*rs + k*ks]; out [rows][ld], zero for k >= K (ld a multiple of 64).
+// 64 x 64 tiles: along k as they lie, else through shared memory.
 static __global__ void __launch_bounds__(256) bf16_rows_kernel(const float *__restrict__ src, long rs, long ks, long rows, long K,
                                                                __nv_bfloat16 *__restrict__ out, long ld) {
-  __shared__ float tile[32][33];
+  __shared__ float tile[64][65];
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-  const long tiles_k = ld / 32;
-  const long ntiles = ((rows + 31) / 32) * tiles_k;
+  const long tiles_k = ld / 64;
+  const long ntiles = ((rows + 63) / 64) * tiles_k;
   for (long t = blockIdx.x; t < ntiles; t += gridDim.x) {
-    const long r0 = (t / tiles_k) * 32, k0 = (t % tiles_k) * 32;
-    if (rs == 1 && ks != 1) {
+    const long r0 = (t / tiles_k) * 64, k0 = (t % tiles_k) * 64;
+    if (rs == 1 && ks != 1) {   // memory runs along the rows: warp = k, lanes = rows
+      float v[8][2];
 #pragma unroll
-      for (int j = ty; j < 32; j += 8) {
-        const long r = r0 + tx, k = k0 + j;
-        tile[tx][j] = (r < rows && k < K) ? src[r + k * ks] : 0.f;
+      for (int j = 0; j < 8; j++)
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+          const long r = r0 + tx + 32 * h, k = k0 + ty + 8 * j;
+          v[j][h] = (r < rows && k < K) ? src[r + k * ks] : 0.f;
+        }
+#pragma unroll
+      for (int j = 0; j < 8; j++)
+#pragma unroll
+        for (int h = 0; h < 2; h++) tile[tx + 32 * h][ty + 8 * j] = v[j][h];
+      __syncthreads();
+#pragma unroll
+      for (int j = 0; j < 8; j++) {
+        const long r = r0 + ty + 8 * j;
+        if (r < rows)
+          *reinterpret_cast<__nv_bfloat162 *>(out + r * ld + k0 + 2 * tx) = __floats2bfloat162_rn(tile[ty + 8 * j][2 * tx], tile[ty + 8 * j][2 * tx + 1]);
       }
+      __syncthreads();
     } else {
+      float v[8][2];
 #pragma unroll
-      for (int j = ty; j < 32; j += 8) {
-        const long r = r0 + j, k = k0 + tx;
-        tile[j][tx] = (r < rows && k < K) ? src[r * rs + k * ks] : 0.f;
+      for (int j = 0; j < 8; j++)
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+          const long r = r0 + ty + 8 * j, k = k0 + 2 * tx + h;
+          v[j][h] = (r < rows && k < K) ? src[r * rs + k * ks] : 0.f;
+        }
+#pragma unroll
+      for (int j = 0; j < 8; j++) {
+        const long r = r0 + ty + 8 * j;
+        if (r < rows) *reinterpret_cast<__nv_bfloat162 *>(out + r * ld + k0 + 2 * tx) = __floats2bfloat162_rn(v[j][0], v[j][1]);
       }
     }
-    __syncthreads();
-#pragma unroll
-    for (int j = ty; j < 32; j += 8) {
-      const long r = r0 + j;
-      if (r < rows) out[r * ld + k0 + tx] = __float2bfloat16(tile[j][tx]);
-    }
-    __syncthreads();
-  }
-}
-// Weight matrix -> one BF16 plane in the k order of the planes operands (see repack_weight_planes_kernel).
-static __global__ void __launch_bounds__(256) repack_weight_bf16_kernel(const float *__restrict__ w, long K, long C, long kHW,
-                                                                        long Cp, long Kp, long ld, int flip,
-                                                                        __nv_bfloat16 *__restrict__ out) {
-  const long rows = flip ? C : K;
-  const long total = rows * ld;
-  const long nthreads = (long)gridDim.x * blockDim.x;
-  for (long t = (long)blockIdx.x * blockDim.x + threadIdx.x; t < total; t += nthreads) {
-    const long r = t / ld, k = t - r * ld;
-    float x = 0.f;
-    if (!flip) {
-      const long tap = k / Cp, c = k - tap * Cp;
-      if (tap < kHW && c < C) x = w[(r * C + c) * kHW + tap];
-    } else {
-      const long tapf = k / Kp, ko = k - tapf * Kp;
-      if (tapf < kHW && ko < K) x = w[(ko * C + r) * kHW + (kHW - 1 - tapf)];
-    }
-    out[t] = __float2bfloat16(x);
-  }
-}
-// gradW[ko][(c, tap)] += scale * tmp[...] is shared with the FP32 path (tmp is FP32 in both modes).
-
-// hi/lo planes of a strided matrix: element (r, k) at src[r*rs + k*ks]; out planes [rows][ld], zero for k >= K.
-// 32x32 tiles through shared memory so that reads are coalesced along whichever source dimension is
-// contiguous and writes are coalesced along k.
-static __global__ void __launch_bounds__(256) split_planes_kernel(const float *__restrict__ src, long rs, long ks, long rows,
-                                                                  long K, float *__restrict__ hi, float *__restrict__ lo,
-                                                                  long ld) {
-  __shared__ float tile[32][33];
-  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-  const long tiles_k = ld / 32;
-  const long ntiles = ((rows + 31) / 32) * tiles_k;
-  for (long t = blockIdx.x; t < ntiles; t += gridDim.x) {
-    const long r0 = (t / tiles_k) * 32, k0 = (t % tiles_k) * 32;
-    if (rs == 1 && ks != 1) {  // contiguous along rows: read transposed
-#pragma unroll
-      for (int j = ty; j < 32; j += 8) {
-        const long r = r0 + tx, k = k0 + j;
-        tile[tx][j] = (r < rows && k < K) ? src[r + k * ks] : 0.f;
-      }
-    } else {
-#pragma unroll
-      for (int j = ty; j < 32; j += 8) {
-        const long r = r0 + j, k = k0 + tx;
-        tile[j][tx] = (r < rows && k < K) ? src[r * rs + k * ks] : 0.f;
-      }
-    }
-    __syncthreads();
-#pragma unroll
-    for (int j = ty; j < 32; j += 8) {
-      const long r = r0 + j;
-      if (r < rows) {
-        const float x = tile[j][tx];
-        unsigned h;
-        asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(h) : "f"(x));
-        const float xl = x - __uint_as_float(h);
-        unsigned l;
-        asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(l) : "f"(xl));
-        hi[r * ld + k0 + tx] = __uint_as_float(h);
-        lo[r * ld + k0 + tx] = __uint_as_float(l);
-      }
-    }
-    __syncthreads();
   }
 }
 
@@ -737,11 +580,13 @@ struct Epilogue {
   }
 };
 
-template <class OpA_, class OpB_, bool PAIR_ = false>
+template <class OpA_, class OpB_, bool PAIR_ = false, bool HALF_ = false>
 struct Problem {
   typedef OpA_ OpA;
   typedef OpB_ OpB;
   static constexpr bool PAIR = PAIR_;   // pixel-pair epilogue (see Epilogue)
+  static constexpr bool HALF = HALF_;   // BF16 operands (two-SM engine)
+  static constexpr int KV = HALF_ ? 64 : 32;   // k per tile of the two-SM engine
   OpA a;
   OpB b;
   Epilogue epi;
@@ -758,11 +603,9 @@ struct Problem {
   int tail_splits = 1;
 };
 
-// Epilogue of one drain thread: its row m of the tile, NCOL columns from nb on (split-K partials go to the
-// workspace instead).
+// Epilogue of one drain thread: its row m of the tile, NCOL columns from nb on.
 template <class P, int NCOL>
-__device__ __forceinline__ void tc2_store_rows(const P &p, const float (&acc)[NCOL], long m, long nb, long z = -1,
-                                               bool direct = false) {
+__device__ __forceinline__ void tc2_store_rows(const P &p, const float (&acc)[NCOL], long m, long nb) {
   if constexpr (!P::PAIR) {
     // Plain accumulation into a destination whose ROWS are neighbours in memory (column-major gradWeight of a Linear
     // layer: out[m + n * nstride]): 16-byte reductions at the L2.  A thread holds one row and NCOL columns, a 16-byte
@@ -770,8 +613,7 @@ __device__ __forceinline__ void tc2_store_rows(const P &p, const float (&acc)[NC
     // through two rounds of shuffles (every lane of the warp takes part, also those whose row lies past M).  A
     // quarter of the memory-side operations of the per-element form below, which is what bounds a weight gradient
     // with a short reduction.
-    const bool to_out = !(p.ws && !direct);
-    if (to_out && p.epi.beta == 1.f && !p.epi.bias && p.epi.mdiv >= p.M && (p.epi.nstride & 3) == 0 &&
+    if (p.epi.beta == 1.f && !p.epi.bias && p.epi.mdiv >= p.M && (p.epi.nstride & 3) == 0 &&
         nb + NCOL <= p.N && (reinterpret_cast<uintptr_t>(p.epi.out) & 15) == 0) {
       const unsigned full = 0xffffffffu;
       const int i = threadIdx.x & 3;
@@ -804,14 +646,8 @@ __device__ __forceinline__ void tc2_store_rows(const P &p, const float (&acc)[NC
     }
   }
   if (m >= p.M) return;
-  if (z < 0) z = blockIdx.z;   // split-K slice: the launch's z index unless the (persistent) caller names it
-  const bool to_ws = p.ws && !direct;   // `direct`: a whole-reduction tile of a launch that splits only its tail
-  const long mo = to_ws ? 0 : p.epi.template moff<P::PAIR>(m);
-  if (to_ws) {
-#pragma unroll
-    for (int j = 0; j < NCOL; j++)
-      if (nb + j < p.N) p.ws[(z * p.N + nb + j) * p.M + m] = acc[j];
-  } else if (!P::PAIR && p.epi.nstride == 1 && nb + NCOL <= p.N &&
+  const long mo = p.epi.template moff<P::PAIR>(m);
+  if (!P::PAIR && p.epi.nstride == 1 && nb + NCOL <= p.N &&
              ((reinterpret_cast<uintptr_t>(p.epi.out + mo + nb) & 15) == 0)) {
     // Row-major destination (the columns of a row are neighbours in memory) and this thread's NCOL columns start on
     // a 16-byte boundary: 16-byte loads and stores.  Neighbouring lanes are a whole row apart, so every access of a
@@ -1000,6 +836,7 @@ static __global__ void __launch_bounds__(256) tail_finish_kernel(const float *__
     const long n = nt * bn2 + c;
     if (n >= N) break;
     float acc = 0.f;
+#pragma unroll 8
     for (int z = 0; z < splits; z++) acc += base[((long)z * bn2 + c) * 256];
     if (pair) epi.store<true>(mo, n, acc);
     else epi.store<false>(mo, n, acc, row_b);

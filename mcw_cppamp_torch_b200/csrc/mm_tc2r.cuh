@@ -1,52 +1,66 @@
-// Two-SM tcgen05 engine over plain FP32 operands: the 3xTF32 split happens inside the SM.
+// Two-SM tcgen05 engine over operands fetched by TMA: FP32 values as 3xTF32 products split inside the SM, or BF16 values.
 //
-// The plane engine (mm_tc2.cuh) reads a TF32 hi and a TF32 lo copy of every operand element, eight bytes per
-// element and k tile, and its main loop runs at the pace of L2 -> SM traffic, not of the tensor pipe.  Here
-// TMA brings the FP32 values themselves (four bytes per element) straight into the `hi` slot of a stage, in
-// the swizzled layout the MMAs read; kind::tf32 ignores the low 13 mantissa bits of its operands, so that
-// slot already is the hi operand, hi = trunc_tf32(x).  Four splitter warps per CTA read the slot back and
-// write lo = tf32(x - hi) into the `lo` slot at the same offsets (both slots share one layout, K-major or
-// MN-major alike).  Products Alo*Bhi + Ahi*Blo + Ahi*Bhi and the drain into FP32 registers are those of
-// the plane engine.
+// A cluster of two CTAs on neighbouring SMs computes one 256 x BN2 tile of D (BN2 = 64, 128, 192 or 256): CTA r of the pair
+// stages rows [128 r, 128 r + 128) of the A tile and rows [BN2/2 r, BN2/2 (r+1)) of the B tile in its own shared
+// memory; the MMAs, issued by CTA 0, read both CTAs' shared memory and leave rows [128 r, +128) of the result in CTA
+// r's tensor memory, so that every byte fetched from L2 feeds twice the arithmetic of a one-SM tile.
+//
+// FP32: TMA brings the values themselves (four bytes per element) straight into the `hi` slot of a stage, in the swizzled
+// layout the MMAs read; kind::tf32 ignores the low 13 mantissa bits of its operands, so that slot already is the
+// hi operand, hi = trunc_tf32(x).  Four splitter warps per CTA read the slot back and write lo = tf32(x - hi) into
+// the `lo` slot at the same offsets (both slots share one layout, K-major or MN-major alike).  Twelve MMAs per 32-k tile,
+// Alo*Bhi + Ahi*Blo + Ahi*Bhi, go into one of two TMEM buffers and are added into FP32 registers with
+// round-to-nearest (the tensor core's own accumulation truncates, so chains stay 12 MMAs long).
+//
+// BF16 (opt-in math mode): no splitters and no lo slots, four kind::f16 MMAs per 64-k tile, one MMA thread; products are exact
+// in FP32 and the tolerance of the mode is BF16's, so four k tiles (16 MMAs) chain in one accumulator before a drain.  In
+// each CTA one thread passes the arrival of a tile's bytes on to CTA 0's `full` barrier.  What bounds it is L2 -> SM traffic:
+// 64 KB per 256 x 256 x 64 step of the pair.
 //
 // Rings: R `hi` slots (loads in flight, tiles being split, tiles being multiplied) and L <= R `lo` slots
-// (only tiles being split or multiplied), so that the load queue can be deep although shared memory holds
-// no more than the plane engine's.
+// (only tiles being split or multiplied), so that the load queue can be deep.
 //
-// Roles (512 threads per CTA, cluster of two CTAs as in mm_tc2.cuh):
+// Roles (512 threads per CTA):
 //   warps 0-3   splitters, two groups of two warps taking alternate k tiles: wait for the tile's TMA bytes
 //               (`raw_full`, CTA-local) and for its lo slot to be free, split, publish to the async proxy,
 //               arrive on CTA 0's `full`.
 //   warps 4, 6  (CTA 0) one MMA-issuing thread each, for the even and the odd k tiles.
 //   warp 5      one thread per CTA issues the TMA loads of this CTA's A rows and B rows, R - 1 tiles ahead,
 //               as soon as the MMAs that read a slot have completed (`empty`).
-//   warps 8-15  drain + epilogue, as in the plane engine.
+//   warps 8-15  drain: tcgen05.ld every finished partial tile and add it into FP32 registers; then the epilogue.
+// Registers are rebalanced with setmaxnreg: the drain warps hold BN2/2 accumulators per thread.
 // The kernel is persistent: see tc2r_kernel.
 // Every wait is bounded; on expiry the CTA tells its peer, raises the stall flags (StallCtl, mm_tc.cuh), skips
 // its stores and still joins the final cluster barrier.
 #ifndef THC_MM_TC2R_CUH
 #define THC_MM_TC2R_CUH
 
-#include "mm_tc2.cuh"
+#include "mm_tc.cuh"
 
 namespace thc {
 namespace mm {
 
+constexpr int T2_PRODUCERS = 128;
+constexpr int T2_MMA_WARP = 4;
+constexpr int T2_DRAIN_WARP0 = 8;
+constexpr int T2_DRAIN_WARPS = 8;
+constexpr int T2_THREADS = 512;
+constexpr int T2R_HALF_CHAIN = 4;   // BF16: k tiles accumulated in tensor memory before the drain warps fold them
 constexpr int T2R_TMA_WARP = 5;
 constexpr int T2R_MMA_WARP2 = 6;
 
-template <int BN2> struct Tc2rCfg {
+template <int BN2, bool HALF> struct Tc2rCfg {
   static constexpr int BH = BN2 / 2;
   static constexpr int A_BYTES = TC_BM * 128;
   static constexpr int B_BYTES = BH * 128;
   static constexpr int SLOT_BYTES = A_BYTES + B_BYTES;          // one precision of this CTA's A rows and B rows
-  static constexpr int LO_SLOTS = 3;
+  static constexpr int LO_SLOTS = HALF ? 0 : 3;
   static constexpr int HI_MAX = (227 * 1024 - 1024 - 512) / SLOT_BYTES - LO_SLOTS;
-  static constexpr int HI_SLOTS = HI_MAX > 6 ? 6 : HI_MAX;
+  static constexpr int HI_SLOTS = HI_MAX > (HALF ? 8 : 6) ? (HALF ? 8 : 6) : HI_MAX;
   static constexpr int TMEM_COLS = 2 * BN2 > 256 ? 512 : 256;
   static constexpr int SMEM_BYTES = (HI_SLOTS + LO_SLOTS) * SLOT_BYTES + 512 + 1024;
   static_assert(HI_SLOTS >= LO_SLOTS, "ring sizes");
-  static_assert(HI_SLOTS % 2 == 0 || HI_SLOTS <= LO_SLOTS + 2, "an odd hi ring must not be longer than the lo ring + 2 (parity waits of the two MMA threads)");
+  static_assert(HALF || HI_SLOTS % 2 == 0 || HI_SLOTS <= LO_SLOTS + 2, "an odd hi ring must not be longer than the lo ring + 2 (parity waits of the two MMA threads)");
 };
 
 // lo = tf32(x - trunc_tf32(x)) of four values
@@ -90,34 +104,36 @@ __device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity) {
       : "memory");
   return done != 0;
 }
-template <int ROWS, bool MN>
+template <int ROWS, int KV, bool MN>
 __device__ __forceinline__ void tma_issue(const RawOperand<MN> &op, uint32_t dst, long row0, long k0, uint32_t mbar) {
   if constexpr (MN) {
+    static_assert(ROWS % KV == 0, "whole row blocks");
 #pragma unroll
-    for (int a = 0; a < ROWS / 32; a++) tma_load_2d(dst + a * 4096, &op.tmap, (int)row0 + 32 * a, (int)k0, mbar);
+    for (int a = 0; a < ROWS / KV; a++) tma_load_2d(dst + a * KV * 128, &op.tmap, (int)row0 + KV * a, (int)k0, mbar);
   } else {
     tma_load_2d(dst, &op.tmap, (int)k0, (int)row0, mbar);
   }
 }
-// Convolution windows as rows (K-major): one im2col load of 32 channels of ROWS = 128 consecutive windows.
-template <int ROWS>
+// Convolution windows as rows (K-major): one im2col load of KV channels of ROWS = 128 consecutive windows.
+template <int ROWS, int KV>
 __device__ __forceinline__ void tma_issue(const PlanesWindowOperand &op, uint32_t dst, long row0, long k0, uint32_t mbar) {
   static_assert(ROWS == TC_BM, "the window map loads 128 windows");
-  int x, y, img, i, j, c0;
+  int x, y, img, i, j, ct;
   op.tile_origin(row0, x, y, img);
-  op.tile_tap(k0, i, j, c0);
-  tma_load_windows(dst, &op.tmap, c0, x, y, img, j, i, mbar);
+  op.tile_tap((unsigned)(k0 / KV), i, j, ct);
+  tma_load_windows(dst, &op.tmap, ct * KV, x, y, img, j, i, mbar);
 }
-// Convolution windows as the reduction (MN-major): per 32-row block, 32 channels of 32 consecutive windows.
-template <int ROWS>
+// Convolution windows as the reduction (MN-major): per KV-row block, KV channels of KV consecutive windows.
+template <int ROWS, int KV>
 __device__ __forceinline__ void tma_issue(const WindowRowsOperand &op, uint32_t dst, long row0, long k0, uint32_t mbar) {
+  static_assert(ROWS % KV == 0, "whole row blocks");
   int x, y, img;
   op.pixel_origin(k0, x, y, img);
 #pragma unroll
-  for (int a = 0; a < ROWS / 32; a++) {
+  for (int a = 0; a < ROWS / KV; a++) {
     int i, j, c0;
-    op.row_tap(row0 + 32 * a, i, j, c0);
-    tma_load_windows(dst + a * 4096, &op.tmap, c0, x, y, img, j, i, mbar);
+    op.row_tap(row0 + KV * a, i, j, c0);
+    tma_load_windows(dst + a * KV * 128, &op.tmap, c0, x, y, img, j, i, mbar);
   }
 }
 
@@ -136,8 +152,8 @@ constexpr int T2R_SCHED = 8;
 constexpr int T2R_SCHED_WARP = 7;
 constexpr uint32_t T2R_NO_ITEM = 0xffffffffu;
 constexpr int T2R_ITEM_WAIT_SHIFT = 6;   // item-level waits may take 64 k-tile limits (see mbar_wait)
-// readers per slot: TMA thread, 4 splitter warps, 8 drain warps in each CTA, the two MMA threads in the leader
-constexpr int T2R_SCHED_READERS = 2 * (1 + 4 + T2_DRAIN_WARPS) + 2;
+// readers per slot: TMA thread, 4 splitter warps (BF16: one relay), 8 drain warps in each CTA, the MMA threads in the leader
+template <bool HALF> struct Tc2rReaders { static constexpr uint32_t count = 2 * (1 + (HALF ? 1 : 4) + T2_DRAIN_WARPS) + (HALF ? 1 : 2); };
 
 __device__ __forceinline__ void mbar_arrive_local(uint32_t bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
@@ -177,8 +193,10 @@ struct Tc2rItem {
 template <class P, int BN2>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(T2_THREADS, 1) tc2r_kernel(const __grid_constant__ P p, const StallCtl ctl,
                                                                                                 unsigned *sched_counter) {
-  typedef Tc2rCfg<BN2> Cfg;
-  constexpr int R = Cfg::HI_SLOTS, L = Cfg::LO_SLOTS;
+  constexpr bool HALF = P::HALF;
+  constexpr int KV = P::KV;
+  typedef Tc2rCfg<BN2, HALF> Cfg;
+  constexpr int R = Cfg::HI_SLOTS, L = Cfg::LO_SLOTS, LM = L > 0 ? L : 1;
   constexpr int BH = Cfg::BH;
   extern __shared__ uint8_t smem_raw[];
   uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
@@ -189,7 +207,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(T2_THREADS, 1) tc2r_
   uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + 3 * R + 4 + L + 2 * T2R_SCHED + 1);
   volatile WaitCtl *abort_flag = reinterpret_cast<volatile WaitCtl *>(tmem_slot + 2);
   uint32_t *sched_ring = tmem_slot + 2 + sizeof(WaitCtl) / 4;
-  static_assert((3 * 6 + 4 + Cfg::LO_SLOTS + 2 * T2R_SCHED + 1) * 8 + 8 + sizeof(WaitCtl) + 4 * T2R_SCHED <= 512, "auxiliary shared memory");
+  static_assert((3 * R + 4 + L + 2 * T2R_SCHED + 1) * 8 + 8 + sizeof(WaitCtl) + 4 * T2R_SCHED <= 512, "auxiliary shared memory");
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const uint32_t rank = cluster_ctarank();
@@ -217,7 +235,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(T2_THREADS, 1) tc2r_
     }
     const uint32_t nt = tile / gm, mt = tile - nt * gm;
     t.m_tile0 = (long)mt * 256; t.n_tile0 = (long)nt * BN2;
-    t.num_k_tiles = (int)((k_end - t.k_begin + TC_BK - 1) / TC_BK);
+    t.num_k_tiles = (int)((k_end - t.k_begin + KV - 1) / KV);
     return t;
   };
 
@@ -232,14 +250,14 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(T2_THREADS, 1) tc2r_
   sched.ring = smem_u32(sched_ring);
   if (tid == 0) {
     for (int s = 0; s < R; s++) {
-      mbar_init(bar_full + 8 * s, 2 * T2_PRODUCERS / 64);   // one group of two splitter warps in each CTA (used in CTA 0)
+      mbar_init(bar_full + 8 * s, HALF ? 2 : 2 * T2_PRODUCERS / 64);   // one relay / group of two splitter warps in each CTA (used in CTA 0)
       mbar_init(bar_empty + 8 * s, 1);
       mbar_init(bar_raw + 8 * s, 1);                        // this CTA's TMA thread + the bytes it announces
     }
     for (int l = 0; l < L; l++) mbar_init(bar_lo_empty + 8 * l, 1);
     for (int k = 0; k < T2R_SCHED; k++) {
       mbar_init(bar_sched_full + 8 * k, 1);
-      mbar_init(bar_sched_empty + 8 * k, T2R_SCHED_READERS);   // used in CTA 0
+      mbar_init(bar_sched_empty + 8 * k, Tc2rReaders<HALF>::count);   // used in CTA 0
     }
     mbar_init(bar_sched_go, 1);                                // used in CTA 0
     for (int b = 0; b < 2; b++) {
@@ -263,6 +281,28 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(T2_THREADS, 1) tc2r_
     // ------------------------------------------------------------ splitters
     setmaxnreg_dec<72>();
     const uint32_t full_leader = mapa_shared(bar_full, 0);
+    if constexpr (HALF) {
+      // BF16 tiles are ready as they land: one thread tells CTA 0 so
+      if (warp == 0 && lane == 0) {
+        int g0 = 0;
+        for (uint32_t n = 0; ok; n++) {
+          uint32_t w = T2R_NO_ITEM;
+          ok = sched.next(n, w, abort_flag);
+          if (!ok) break;
+          sched.done(n);
+          if (w == T2R_NO_ITEM) break;
+          const int nk = item_at(w).num_k_tiles;
+          for (int it = 0; it < nk; it++) {
+            const int g = g0 + it, s = g % R;
+            ok = mbar_wait(bar_raw + 8 * s, (uint32_t)(g / R) & 1u, abort_flag, kWaitRawTile);
+            if (!ok) break;
+            mbar_arrive_cluster(full_leader + 8 * s);
+          }
+          g0 += nk;
+        }
+      }
+      __syncwarp();
+    } else {
     // Two groups of two warps take alternate k tiles, so that one group's barrier round trips and proxy fence
     // overlap the other group's copying: under the MMAs' own shared-memory traffic every access here waits
     // hundreds of cycles.
@@ -277,12 +317,12 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(T2_THREADS, 1) tc2r_
       const int nk = item_at(w).num_k_tiles;
       for (int it = (g0 + grp) & 1; it < nk; it += 2) {
         const int g = g0 + it;
-        const int s = g % R, ls = g % L;
+        const int s = g % R, ls = g % LM;
         const uint32_t raw_bar = bar_raw + 8 * s, raw_par = (uint32_t)(g / R) & 1u;
         // The lo slot is free once the MMAs of tile g - L have read it.  It has a barrier of its own: the hi slots'
         // `empty` barriers can run two phases ahead of a splitter group that was slow to wake up (the other group and
         // the other MMA thread do not wait for it), and a parity wait cannot tell two completed phases from none.
-        const uint32_t lo_bar = bar_lo_empty + 8 * ls, lo_par = (uint32_t)(g / L + 1) & 1u;
+        const uint32_t lo_bar = bar_lo_empty + 8 * ls, lo_par = (uint32_t)(g / LM + 1) & 1u;
         const bool r1 = mbar_try_wait(raw_bar, raw_par), r2 = g < L || mbar_try_wait(lo_bar, lo_par);
         ok = (r1 || mbar_wait(raw_bar, raw_par, abort_flag, kWaitRawTile)) && (r2 || mbar_wait(lo_bar, lo_par, abort_flag, kWaitLoSlot));
         ok = __all_sync(0xffffffffu, ok);
@@ -306,9 +346,41 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(T2_THREADS, 1) tc2r_
       }
       g0 += nk;
     }
+    }
   } else if (warp < T2_DRAIN_WARP0) {
     setmaxnreg_dec<40>();
-    if ((warp == T2_MMA_WARP || warp == T2R_MMA_WARP2) && lane == 0 && rank == 0) {
+    if (HALF && warp == T2_MMA_WARP && lane == 0 && rank == 0) {
+      // ---------------------------------------------------------- MMA issuer, BF16: one thread, T2R_HALF_CHAIN k tiles per buffer
+      constexpr uint32_t idesc = umma2_idesc_bf16(BN2, P::OpA::MN_MAJOR, P::OpB::MN_MAJOR);
+      int g = 0, grp = 0;
+      for (uint32_t n = 0; ok; n++) {
+        uint32_t w = T2R_NO_ITEM;
+        ok = sched.next(n, w, abort_flag);
+        if (!ok) break;
+        sched.done(n);
+        if (w == T2R_NO_ITEM) break;
+        const int nk = item_at(w).num_k_tiles;
+        for (int it = 0; it < nk; it++, g++) {
+          const int s = g % R, buf = grp & 1;
+          const bool first = it % T2R_HALF_CHAIN == 0, last = it % T2R_HALF_CHAIN == T2R_HALF_CHAIN - 1 || it == nk - 1;
+          if (first) ok = mbar_wait_spin(bar_acc_empty + 8 * buf, ((uint32_t)(grp >> 1) & 1u) ^ 1u, abort_flag, kWaitAccEmpty);
+          ok = ok && mbar_wait_spin(bar_full + 8 * s, (uint32_t)(g / R) & 1u, abort_flag, kWaitTileFull);
+          if (!ok) break;
+          tc_fence_after();
+          const uint32_t st = smem_u32(smem + s * Cfg::SLOT_BYTES);
+          const uint64_t a_d = umma_desc_half<P::OpA::MN_MAJOR>(st), b_d = umma_desc_half<P::OpB::MN_MAJOR>(st + Cfg::A_BYTES);
+          const uint32_t d = tmem_base + (uint32_t)(buf * BN2);
+#pragma unroll
+          for (int kk = 0; kk < 4; kk++) {   // 16 k per MMA
+            const uint64_t adv_a = (uint64_t)((kk * umma_kstep_bytes_half<P::OpA::MN_MAJOR>()) >> 4);
+            const uint64_t adv_b = (uint64_t)((kk * umma_kstep_bytes_half<P::OpB::MN_MAJOR>()) >> 4);
+            umma2_bf16(d, a_d + adv_a, b_d + adv_b, idesc, (kk || !first) ? 1u : 0u);
+          }
+          umma2_commit_both(bar_empty + 8 * s);
+          if (last) { umma2_commit_both(bar_acc_full + 8 * buf); grp++; }
+        }
+      }
+    } else if (!HALF && (warp == T2_MMA_WARP || warp == T2R_MMA_WARP2) && lane == 0 && rank == 0) {
       // ---------------------------------------------------------- MMA issuers
       // Two threads take alternate k tiles (and with them alternate accumulator buffers): while one is blocked on
       // the tensor pipe's queue the other sits through its barrier polls, each a shared-memory round trip of
@@ -332,7 +404,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(T2_THREADS, 1) tc2r_
         const int nk = item_at(w).num_k_tiles;
         for (int it = (g0 + buf) & 1; it < nk; it += 2) {
           const int g = g0 + it;
-          const int s = g % R, ls = g % L;
+          const int s = g % R, ls = g % LM;
           const uint32_t phase = (uint32_t)(g / R) & 1u, acc_phase = (uint32_t)(g >> 1) & 1u;
           ok = mbar_wait_spin(bar_acc_empty + 8 * buf, acc_phase ^ 1u, abort_flag, kWaitAccEmpty);
           ok = ok && mbar_wait_spin(bar_full + 8 * s, phase, abort_flag, kWaitTileFull);
@@ -343,14 +415,14 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(T2_THREADS, 1) tc2r_
           const uint64_t b_hi = umma_desc_sw128<B_MN>(hs + Cfg::A_BYTES), b_lo = umma_desc_sw128<B_MN>(lsl + Cfg::A_BYTES);
           const uint32_t d = tmem_base + (uint32_t)(buf * BN2);
 #pragma unroll
-          for (int kk = 0; kk < TC_BK / 8; kk++) {
+          for (int kk = 0; kk < 4; kk++) {   // 8 k per MMA
             const uint64_t adv_a = (uint64_t)((kk * umma_kstep_bytes<A_MN>()) >> 4);
             const uint64_t adv_b = (uint64_t)((kk * umma_kstep_bytes<B_MN>()) >> 4);
             umma2_tf32(d, a_lo + adv_a, b_hi + adv_b, idesc, kk ? 1u : 0u);
             umma2_tf32(d, a_hi + adv_a, b_lo + adv_b, idesc, 1u);
           }
 #pragma unroll
-          for (int kk = 0; kk < TC_BK / 8; kk++) {
+          for (int kk = 0; kk < 4; kk++) {   // 8 k per MMA
             const uint64_t adv_a = (uint64_t)((kk * umma_kstep_bytes<A_MN>()) >> 4);
             const uint64_t adv_b = (uint64_t)((kk * umma_kstep_bytes<B_MN>()) >> 4);
             umma2_tf32(d, a_hi + adv_a, b_hi + adv_b, idesc, 1u);
@@ -377,11 +449,11 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(T2_THREADS, 1) tc2r_
           const int g = g0 + t;
           const int s = g % R;
           if (g >= R && !mbar_wait(bar_empty + 8 * s, (uint32_t)((g - R) / R) & 1u, abort_flag, kWaitSlotEmpty)) { ok = false; break; }
-          const long k0 = item.k_begin + (long)t * TC_BK;
+          const long k0 = item.k_begin + (long)t * KV;
           const uint32_t slot = smem_u32(smem + s * Cfg::SLOT_BYTES);
           mbar_arrive_expect_tx(bar_raw + 8 * s, (uint32_t)Cfg::SLOT_BYTES);
-          tma_issue<TC_BM>(p.a, slot, m0, k0, bar_raw + 8 * s);
-          tma_issue<BH>(p.b, slot + Cfg::A_BYTES, n0, k0, bar_raw + 8 * s);
+          tma_issue<TC_BM, KV>(p.a, slot, m0, k0, bar_raw + 8 * s);
+          tma_issue<BH, KV>(p.b, slot + Cfg::A_BYTES, n0, k0, bar_raw + 8 * s);
         }
         g0 += item.num_k_tiles;
       }
@@ -423,7 +495,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(T2_THREADS, 1) tc2r_
       float acc[NCOL];
 #pragma unroll
       for (int j = 0; j < NCOL; j++) acc[j] = 0.f;
-      for (int it = 0; it < item.num_k_tiles; it++) {
+      const int folds = HALF ? (item.num_k_tiles + T2R_HALF_CHAIN - 1) / T2R_HALF_CHAIN : item.num_k_tiles;   // accumulators of this item
+      for (int it = 0; it < folds; it++) {
         const int g = g0 + it;
         const int buf = g & 1;
         const uint32_t acc_phase = (uint32_t)(g >> 1) & 1u;
@@ -444,7 +517,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(T2_THREADS, 1) tc2r_
         __syncwarp();
         if (lane == 0) mbar_arrive_cluster(acc_empty_leader + 8 * buf);
       }
-      g0 += item.num_k_tiles;
+      g0 += folds;
       if (ok) {
         const long m = item.m_tile0 + (long)rank * TC_BM + q * 32 + lane;
         if (item.z >= 0) {
@@ -454,9 +527,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(T2_THREADS, 1) tc2r_
           for (int j = 0; j < NCOL; j++) o[j * 256] = acc[j];
         } else if constexpr (P::PAIR && BN2 == 128) {
           if (pair_lines) tc2_store_pair_rows<P>(p, acc, m, h * 32);
-          else tc2_store_rows<P, NCOL>(p, acc, m, item.n_tile0 + h * NCOL, 0, true);
+          else tc2_store_rows<P, NCOL>(p, acc, m, item.n_tile0 + h * NCOL);
         } else {
-          tc2_store_rows<P, NCOL>(p, acc, m, item.n_tile0 + h * NCOL, 0, true);
+          tc2_store_rows<P, NCOL>(p, acc, m, item.n_tile0 + h * NCOL);
         }
       }
     }

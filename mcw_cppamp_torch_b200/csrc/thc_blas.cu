@@ -26,121 +26,122 @@ static __global__ void broadcast_rows_kernel(float *c, long m, long n, long ldc,
 // Up to two matrices copied to pitches that TMA can address (blockIdx.y: which): lines of `run` floats.
 struct PackJob { const float *src; float *dst; long lines, run, src_ld, dst_ld; };
 static __global__ void __launch_bounds__(256) pack_matrix_kernel(const PackJob a, const PackJob b) {
+  // a warp copies up to 1024 floats of a line, all its loads in flight before the first store
   const PackJob &j = blockIdx.y ? b : a;
   const int lane = threadIdx.x & 31;
-  const long warps = (long)gridDim.x * (blockDim.x >> 5);
-  for (long l = (long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); l < j.lines; l += warps) {
+  const long warps = (long)gridDim.x * (blockDim.x >> 5), parts = (j.run + 1023) / 1024;
+  for (long w = (long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); w < j.lines * parts; w += warps) {
+    const long l = w / parts, i0 = (w - l * parts) * 1024 + lane;
     const float *s = j.src + l * j.src_ld;
     float *d = j.dst + l * j.dst_ld;
-#pragma unroll 8
-    for (long i = lane; i < j.run; i += 32) d[i] = s[i];
+    float v[32];
+#pragma unroll
+    for (int i = 0; i < 32; i++) v[i] = i0 + 32 * i < j.run ? s[i0 + 32 * i] : 0.f;
+#pragma unroll
+    for (int i = 0; i < 32; i++)
+      if (i0 + 32 * i < j.run) d[i0 + 32 * i] = v[i];
   }
 }
 
 // Tensor-core path over the matrices as they lie in memory (raw-operand engine): TMA reads either layout of
 // either operand, so no pass over the operands precedes the product.
-template <bool TA, bool TB>
-static void gemm_raw_t(long m, long n, long k, float alpha, const float *a, long lda, const float *b, long ldb, float beta,
-                       float *c, long ldc, const float *row_bias) {
+template <bool A_MN, bool B_MN>
+static void gemm_raw_t(const float *a, long lda, const float *b, long ldb, long m, long n, long k, const mm::Epilogue &epi) {
   using namespace mm;
-  // A(i,l): 'n' a[i + l*lda] runs along the rows (MN-major), 't' a[l + i*lda] along k.  B(j,l): 'n' b[l + j*ldb]
-  // runs along k, 't' b[j + l*ldb] along the rows.
-  typedef RawOperand<!TA> OpA;
-  typedef RawOperand<TB> OpB;
-  Problem<OpA, OpB> p;
-  p.epi = Epilogue{c, nullptr, alpha, beta, LONG_MAX, 0, ldc};
-  p.epi.row_bias = row_bias;
+  Problem<RawOperand<A_MN>, RawOperand<B_MN>> p;
+  p.epi = epi;
   p.M = m; p.N = n; p.K = k;
-  launch_raw(p, [&](Problem<OpA, OpB> &q, int bn2) {
-    attach_raw_map(q.a, a, m, k, lda, TC_BM);
-    attach_raw_map(q.b, b, n, k, ldb, bn2 / 2);
+  launch_raw(p, [&](auto &q, int bn2) {
+    attach_raw_map<false>(q.a, a, m, k, lda, TC_BM);
+    attach_raw_map<false>(q.b, b, n, k, ldb, bn2 / 2);
   });
 }
-static void gemm_raw(bool ta, bool tb, long m, long n, long k, float alpha, const float *a, long lda, const float *b,
-                     long ldb, float beta, float *c, long ldc, const float *row_bias) {
-  if (!mm::raw_matrix_ok(a, lda) || !mm::raw_matrix_ok(b, ldb)) {
+// One side of a product: element (r, l) at p[l + r * ld] (along_k) or p[r + l * ld].
+struct GemmSide { const float *p; long ld; bool along_k; long rows; };
+// Orientation of the 256-row tiles and the epilogue for D(i, j) at c[i + j * ldc]: the first side takes the rows unless it has
+// no more than half a tile of them and the other has more.
+static mm::Epilogue gemm_sides(GemmSide &x, GemmSide &y, float alpha, float beta, float *c, long ldc, const float *row_bias) {
+  if (x.rows <= 128 && y.rows > x.rows) {
+    std::swap(x, y);
+    mm::Epilogue e{c, row_bias, alpha, beta, 1, ldc, 1};   // rows of the product are columns of c: out[m * ldc + n]
+    return e;
+  }
+  mm::Epilogue e{c, nullptr, alpha, beta, LONG_MAX, 0, ldc};
+  e.row_bias = row_bias;
+  return e;
+}
+// BF16 math mode: one K-major BF16 plane per operand, BF16 products.  For results of more than half a tile's rows and more
+// than 32 columns; smaller ones stay FP32-accurate.
+static void gemm_half(GemmSide x, GemmSide y, long k, float alpha, float beta, float *c, long ldc, const float *row_bias) {
+  using namespace mm;
+  Problem<RawOperand<false>, RawOperand<false>, false, true> p;
+  p.epi = gemm_sides(x, y, alpha, beta, c, ldc, row_bias);
+  const HalfMatrix hx = make_half_matrix(x.p, x.along_k ? x.ld : 1, x.along_k ? 1 : x.ld, x.rows, k);
+  const HalfMatrix hy = make_half_matrix(y.p, y.along_k ? y.ld : 1, y.along_k ? 1 : y.ld, y.rows, k);
+  p.M = x.rows; p.N = y.rows; p.K = hx.ld;
+  launch_raw(p, [&](auto &q, int bn2) {
+    attach_raw_map<true>(q.a, hx.p, x.rows, hx.ld, hx.ld, TC_BM);
+    attach_raw_map<true>(q.b, hy.p, y.rows, hy.ld, hy.ld, bn2 / 2);
+  });
+}
+static void gemm_raw(GemmSide x, GemmSide y, long k, float alpha, float beta, float *c, long ldc, const float *row_bias) {
+  const mm::Epilogue epi = gemm_sides(x, y, alpha, beta, c, ldc, row_bias);
+  if (!mm::raw_matrix_ok(x.p, x.ld) || !mm::raw_matrix_ok(y.p, y.ld)) {
     // a pitch or address that TMA cannot take: copy that matrix (a hundredth of the product's time at the sizes that come
     // here) instead of feeding the product through per-thread copies
-    PackJob ja = {}, jb = {};
-    auto job = [](const float *src, long lines, long run, long ld, PackJob &j) {
-      j = PackJob{src, nullptr, lines, run, ld, (run + 3) / 4 * 4};
+    PackJob jobs[2] = {};
+    GemmSide *sides[2] = {&x, &y};
+    for (int i = 0; i < 2; i++) {
+      GemmSide &s = *sides[i];
+      if (mm::raw_matrix_ok(s.p, s.ld)) continue;
+      PackJob &j = jobs[i];
+      j = PackJob{s.p, nullptr, s.along_k ? s.rows : k, s.along_k ? k : s.rows, s.ld, ((s.along_k ? k : s.rows) + 3) / 4 * 4};
       j.dst = (float *)ws_alloc(sizeof(float) * j.lines * j.dst_ld);
-    };
-    if (!mm::raw_matrix_ok(a, lda)) { job(a, ta ? m : k, ta ? k : m, lda, ja); a = ja.dst; lda = ja.dst_ld; }
-    if (!mm::raw_matrix_ok(b, ldb)) { job(b, tb ? k : n, tb ? n : k, ldb, jb); b = jb.dst; ldb = jb.dst_ld; }
-    const long lines = std::max(ja.lines, jb.lines);
-    pack_matrix_kernel<<<dim3((unsigned)std::min<long>((lines + 7) / 8, ctx().sm_count * 8l), 2), 256, 0, stream()>>>(ja, jb);
+      s.p = j.dst; s.ld = j.dst_ld;
+    }
+    const long pieces = std::max(jobs[0].lines * ((jobs[0].run + 1023) / 1024), jobs[1].lines * ((jobs[1].run + 1023) / 1024));
+    pack_matrix_kernel<<<dim3((unsigned)std::min<long>((pieces + 7) / 8, ctx().sm_count * 8l), 2), 256, 0, stream()>>>(jobs[0], jobs[1]);
     check_launch("pack_matrix");
   }
-  if (!ta && !tb) gemm_raw_t<false, false>(m, n, k, alpha, a, lda, b, ldb, beta, c, ldc, row_bias);
-  else if (ta && !tb) gemm_raw_t<true, false>(m, n, k, alpha, a, lda, b, ldb, beta, c, ldc, row_bias);
-  else if (!ta && tb) gemm_raw_t<false, true>(m, n, k, alpha, a, lda, b, ldb, beta, c, ldc, row_bias);
-  else gemm_raw_t<true, true>(m, n, k, alpha, a, lda, b, ldb, beta, c, ldc, row_bias);
+  if (!x.along_k && y.along_k) gemm_raw_t<true, false>(x.p, x.ld, y.p, y.ld, x.rows, y.rows, k, epi);
+  else if (x.along_k && y.along_k) gemm_raw_t<false, false>(x.p, x.ld, y.p, y.ld, x.rows, y.rows, k, epi);
+  else if (!x.along_k) gemm_raw_t<true, true>(x.p, x.ld, y.p, y.ld, x.rows, y.rows, k, epi);
+  else gemm_raw_t<false, true>(x.p, x.ld, y.p, y.ld, x.rows, y.rows, k, epi);
 }
-// Whether the warp-level engine (mm_small.cuh) finishes before the two-SM one: both times in microseconds, as measured for
-// m, n in 32 .. 2048 and k in 32 .. 2048.  Small: 5 to start, 22 per GFLOP (30 with 4-byte copies; n counts in tiles), about
-// 1 us per MB of results.  Two-SM: 11 to start and 0.033 per k up to 512 (a tile's pipeline fill), 2.9 per GFLOP; tiles of
-// 128 columns and less wait longer for each k tile; packing adds a launch and a pass over the operand.
+// Whether the warp-level engine (mm_small.cuh) finishes before the two-SM one.  The latter, as measured for the same sizes: 11 us to
+// start, then the fill and fold of its long pipeline (0.026 per k up to 512) and 2.9 per GFLOP, or the operands' bytes
+// at 3.3 TB/s; packing adds a launch and a pass over the operands.
 static bool small_is_faster(long m, long n, long k, bool aligned) {
-  if (!mm::tc2_tile_width(m, n)) return true;
-  const double lo = (double)std::min(m, n), hi = (double)std::max(m, n), bn = lo <= 8 ? 8 : lo <= 16 ? 16 : lo <= 32 ? 32 : 64;
-  const double gf = 2e-9 * (double)m * (double)n * (double)k, padded = gf * (std::ceil(lo / bn) * bn / lo) * (std::ceil(hi / 64) * 64 / hi);
-  const double small = 5 + (aligned ? 22 : 30) * padded + 0.95e-6 * 4 * (double)m * (double)n;
-  double raw = 11 + 0.033 * (double)std::min(k, 512l) + 2.9 * gf;
-  if (n <= 128) raw += 0.0083 * (double)std::min(k, 2048l);
-  if (!aligned) raw += 5 + 1e-6 * 4 * (double)k * (hi + lo);
-  return small < raw;
-}
-
-// BF16 math mode: one BF16 plane per operand, the BF16 two-SM engine; products too small for it run FP32-accurate.
-static void gemm_half(bool ta, bool tb, long m, long n, long k, float alpha, const float *a, long lda, const float *b,
-                      long ldb, float beta, float *c, long ldc, const float *row_bias) {
-  using namespace mm;
-  HalfPlane pa = make_half_plane(a, ta ? lda : 1, ta ? 1 : lda, m, k);
-  HalfPlane pb = make_half_plane(b, tb ? 1 : ldb, tb ? ldb : 1, n, k);
-  Problem<SplitOperand, SplitOperand> p;
-  p.a = half_operand(pa.p, m, pa.ld);
-  p.b = half_operand(pb.p, n, pb.ld);
-  p.epi = Epilogue{c, nullptr, alpha, beta, LONG_MAX, 0, ldc};
-  p.epi.row_bias = row_bias;
-  p.M = m; p.N = n; p.K = pa.ld / 2;
-  launch_planes_half(p);
+  const double gf = 2e-9 * (double)((m + 63) / 64 * 64) * (double)((n + 63) / 64 * 64) * (double)k, bytes = 4 * (double)k * (double)(m + n);
+  double raw = 11 + std::max(0.026 * (double)std::min(k, 512l) + 2.9 * gf, bytes / 3.3e6);
+  if (!aligned) raw += 5 + bytes / 2e6;
+  return mm::small_product_us(m, n, k, aligned) < raw;
 }
 
 // Small and narrow products: operands as they lie, whatever their layout and alignment.
-static void gemm_small(bool ta, bool tb, long m, long n, long k, float alpha, const float *a, long lda, const float *b,
-                       long ldb, float beta, float *c, long ldc, const float *row_bias) {
+static void gemm_small(const GemmSide &x, const GemmSide &y, long k, float alpha, float beta, float *c, long ldc, const float *row_bias) {
   mm::SmallProblem p = {};
-  p.a = mm::small_operand(a, lda); p.b = mm::small_operand(b, ldb);
-  p.M = (int)m; p.N = (int)n; p.K = (int)k;
+  p.a = mm::small_operand(x.p, x.ld); p.b = mm::small_operand(y.p, y.ld);
+  p.M = (int)x.rows; p.N = (int)y.rows; p.K = (int)k;
   p.c = c; p.sm = 1; p.sn = ldc;
   p.alpha = alpha; p.beta = beta;
   p.bias = row_bias; p.bias_m = 1;
-  mm::launch_small(p, ta, !tb);
+  mm::launch_small(p, x.along_k, y.along_k);
 }
 
-template <bool TA, bool TB>
-static void gemm_t(long m, long n, long k, float alpha, const float *a, long lda, const float *b, long ldb,
-                   float beta, float *c, long ldc) {
+// FP32 FMA mode
+static void gemm_simt(const GemmSide &x, const GemmSide &y, long k, float alpha, float beta, float *c, long ldc) {
   using namespace mm;
-  typedef Operand<LinearMap, LinearMap, 0, TA> OpA;     // 't': memory runs along k
-  typedef Operand<LinearMap, LinearMap, 0, !TB> OpB;    // 'n': b[l + j*ldb] runs along k
-  Problem<OpA, OpB> p;
-  p.a.base = a;
-  p.a.rows = LinearMap{m, TA ? lda : 1};
-  p.a.ks = LinearMap{k, TA ? 1 : lda};
-  p.b.base = b;
-  p.b.rows = LinearMap{n, TB ? 1 : ldb};
-  p.b.ks = LinearMap{k, TB ? ldb : 1};
-  auto vec_ok = [](const float *base, long row_stride, long k_stride) {
-    return (int)(((uintptr_t)base & 15) == 0 && row_stride % 4 == 0 && k_stride == 1);
+  Problem<Operand<LinearMap, LinearMap, 0>, Operand<LinearMap, LinearMap, 0>> p;
+  auto side = [&](auto &op, const GemmSide &s) {
+    op.base = s.p;
+    op.rows = LinearMap{s.rows, s.along_k ? s.ld : 1};
+    op.ks = LinearMap{k, s.along_k ? 1 : s.ld};
+    op.H = op.W = 0; op.dH = op.dW = 1;
   };
-  p.a.vec4 = vec_ok(a, p.a.rows.stride, p.a.ks.stride);
-  p.b.vec4 = vec_ok(b, p.b.rows.stride, p.b.ks.stride);
-  p.a.H = p.a.W = p.b.H = p.b.W = 0;
-  p.a.dH = p.a.dW = p.b.dH = p.b.dW = 1;
+  side(p.a, x); side(p.b, y);
   p.epi = Epilogue{c, nullptr, alpha, beta, LONG_MAX, 0, ldc};
-  p.M = m; p.N = n; p.K = k;
+  p.M = x.rows; p.N = y.rows; p.K = k;
   launch_simt(p);
 }
 
@@ -172,17 +173,13 @@ void gemm(char transa, char transb, long m, long n, long k, float alpha, const f
     check_launch("scale_matrix");
     return;
   }
-  if (mode != 1) {
-    const bool aligned = mm::raw_matrix_ok(a, lda) && mm::raw_matrix_ok(b, ldb);
-    if (small_is_faster(m, n, k, aligned)) gemm_small(ta, tb, m, n, k, alpha, a, lda, b, ldb, beta, c, ldc, row_bias);
-    else if (mode == 2 && mm::tc2h_tile_width(m, n, false)) gemm_half(ta, tb, m, n, k, alpha, a, lda, b, ldb, beta, c, ldc, row_bias);
-    else gemm_raw(ta, tb, m, n, k, alpha, a, lda, b, ldb, beta, c, ldc, row_bias);
-    return;
-  }
-  if (!ta && !tb) gemm_t<false, false>(m, n, k, alpha, a, lda, b, ldb, beta, c, ldc);
-  else if (ta && !tb) gemm_t<true, false>(m, n, k, alpha, a, lda, b, ldb, beta, c, ldc);
-  else if (!ta && tb) gemm_t<false, true>(m, n, k, alpha, a, lda, b, ldb, beta, c, ldc);
-  else gemm_t<true, true>(m, n, k, alpha, a, lda, b, ldb, beta, c, ldc);
+  // A(i,l): 'n' a[i + l*lda], 't' a[l + i*lda].  B(j,l): 'n' b[l + j*ldb], 't' b[j + l*ldb].
+  const GemmSide x{a, lda, ta, m}, y{b, ldb, !tb, n};
+  if (mode == 1) { gemm_simt(x, y, k, alpha, beta, c, ldc); return; }
+  const bool aligned = mm::raw_matrix_ok(a, lda) && mm::raw_matrix_ok(b, ldb);
+  if (mode == 2 && m > 128 && n > 32) gemm_half(x, y, k, alpha, beta, c, ldc, row_bias);
+  else if (small_is_faster(m, n, k, aligned)) gemm_small(x, y, k, alpha, beta, c, ldc, row_bias);
+  else gemm_raw(x, y, k, alpha, beta, c, ldc, row_bias);
 }
 
 // y = beta*y + alpha*op(A)*x.  'n': A is m x n column-major, y has m entries: threads own rows

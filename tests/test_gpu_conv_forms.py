@@ -1,0 +1,69 @@
+"""The forms in which the tensor-core convolution passes state a layer: planes padded to whole swizzle spans, folded and unfolded
+cells, the column matrix with stacked weight-gradient pixels, pixel pairs; both precisions, at remainders and smallest sizes."""
+import numpy as np
+import pytest
+
+from util import conv_exact, conv_grad_input_exact, conv_grad_weight_exact
+
+pytestmark = pytest.mark.gpu
+
+CASES = [
+    # N, C, H, W, K, kH, kW, dH, dW, pad
+    (2, 3, 20, 18, 64, 3, 3, 1, 1, 1),     # column matrix, four pixels stacked in the weight gradient
+    (1, 3, 19, 17, 64, 3, 3, 1, 1, 1),     # odd pixel count: not stacked
+    (3, 1, 11, 13, 40, 5, 5, 1, 1, 2),     # one plane
+    (6, 17, 25, 17, 29, 5, 5, 1, 1, 1),    # nothing a multiple of anything
+    (2, 35, 14, 15, 18, 11, 11, 1, 1, 5),
+    (2, 33, 9, 9, 65, 3, 3, 1, 1, 1),      # one plane more than a span (FP32; BF16 in the next)
+    (2, 65, 9, 9, 129, 3, 3, 1, 1, 1),
+    (3, 6, 21, 23, 50, 5, 5, 2, 2, 1),     # strided, ragged
+    (2, 40, 16, 17, 48, 7, 7, 4, 4, 2),
+    (2, 64, 15, 13, 64, 3, 3, 2, 2, 1),    # strided with whole spans: direct windows, folded gradInput
+    (2, 64, 16, 16, 64, 1, 1, 2, 2, 0),    # window smaller than the stride: pixels that no window reaches
+    (1, 5, 17, 19, 33, 3, 2, 4, 3, 0),
+    (2, 8, 6, 5, 40, 2, 3, 1, 1, 3),       # padding not below the window
+    (1, 2, 4, 4, 1, 4, 4, 1, 1, 0),        # one output
+    (150, 3, 6, 6, 16, 3, 3, 1, 1, 0),
+]
+
+
+@pytest.mark.parametrize("mode", ["fp32x3", "bf16"])
+@pytest.mark.parametrize("case", CASES)
+def test_conv_forms(mode, case):
+    import mcw_cppamp_torch_b200 as gt
+    N, C, H, W, K, kH, kW, dH, dW, pad = case
+    geo = (kH, kW, dH, dW, pad)
+    g = np.random.default_rng(sum(case))
+    x = g.uniform(-1, 1, (N, C, H, W)).astype(np.float32)
+    s = 1.0 / np.sqrt(C * kH * kW)
+    w, b = g.uniform(-s, s, (K, C * kH * kW)).astype(np.float32), g.uniform(-s, s, K).astype(np.float32)
+    want = conv_exact(x, w, b, *geo)
+    go = g.standard_normal(want.shape).astype(np.float32)
+    gw0, gb0 = g.standard_normal(w.shape).astype(np.float32), g.standard_normal(K).astype(np.float32)
+    gt.set_math_mode(mode)
+    try:
+        m = gt.nn.SpatialConvolutionMM(C, K, kW, kH, dW, dH, pad)
+        m.weight, m.bias, m.gradWeight, m.gradBias = w.copy(), b.copy(), gw0.copy(), gb0.copy()
+        m.gpu()
+        xg, gog = gt.gpu(x), gt.gpu(go)
+        out = m.forward(xg).float()
+        gi = m.backward(xg, gog, 0.5).float()
+        gw, gb = m.gradWeight.float(), m.gradBias.float()
+        apart = gt.nn.SpatialConvolutionMM(C, K, kW, kH, dW, dH, pad)          # no forward pass, separate calls
+        apart.weight, apart.bias, apart.gradWeight, apart.gradBias = w.copy(), b.copy(), gw0.copy(), gb0.copy()
+        apart.gpu()
+        assert np.array_equal(apart.updateGradInput(xg, gog).float(), gi)
+        apart.accGradParameters(xg, gog, 0.5)
+        assert np.array_equal(apart.gradWeight.float(), gw) and np.array_equal(apart.gradBias.float(), gb)
+    finally:
+        gt.set_math_mode("fp32x3")
+    a = np.abs
+    # 3xTF32: dropped terms and truncating chains are 2^-19 of the sum of |products|; BF16 operands: 2^-8 per product
+    rel = 2.0 ** -19 if mode == "fp32x3" else 2.0 ** -7
+    gw_e, gb_e = conv_grad_weight_exact(x, go, *geo)
+    gw_s, gb_s = conv_grad_weight_exact(a(x), a(go), *geo)
+    long = 2.0 ** -24 * (go.size / K / 32 + 64)                                    # one rounding per k tile of the pixel sum
+    assert np.all(a(out - want) <= rel * conv_exact(a(x), a(w), a(b), *geo) + 1e-30)
+    assert np.all(a(gi - conv_grad_input_exact(go, w, x.shape, *geo)) <= rel * conv_grad_input_exact(a(go), a(w), x.shape, *geo) + 1e-30)
+    assert np.all(a(gw - (gw0 + 0.5 * gw_e)) <= (rel + long) * (gw_s + a(gw0)))
+    assert np.all(a(gb - (gb0 + 0.5 * gb_e)) <= (2.0 ** -19 + long) * (gb_s + a(gb0)))

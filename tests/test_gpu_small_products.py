@@ -65,5 +65,6 @@ def test_linear_forward_bias(gt, rows, inputs, outputs, mode):
 def test_nan_and_infinity_reach_the_result(gt):
     A = np.ones((70, 40), np.float32)
     A[3, 5], A[4, 6] = np.nan, np.inf
+    A[2, 1:2].view(np.uint32)[:] = 0x7fffffff           # the NaN that device arithmetic makes
     r = gt.GPUTensor(70, 20).zero().addmm(0.0, 1.0, gt.gpu(A), gt.gpu(np.ones((40, 20), np.float32))).float()
-    assert np.isnan(r[3]).all() and not np.isfinite(r[4]).any() and np.all(r[5] == 40)
+    assert np.isnan(r[2:4]).all() and not np.isfinite(r[4]).any() and np.all(r[5] == 40)
