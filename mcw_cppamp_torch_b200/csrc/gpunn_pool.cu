@@ -9,6 +9,7 @@
 // visiting them in ascending (y, x) order, which is the order in which the CPU loop
 // (mcw_nn/generic/SpatialMaxPooling.c:147-176) adds them: no atomics, deterministic, and bit-equal
 // to the CPU result for overlapping windows too.
+#include <algorithm>
 #include <cfloat>
 
 #include "thc_internal.h"
@@ -33,15 +34,11 @@ struct Div32 {
   __device__ __forceinline__ unsigned div(unsigned n) const { return d > 1 ? (__umulhi(n, mul) >> shr) : n; }
 };
 
-// grid.y strides over planes, grid.x * block over the plane's outputs: no division by the plane size.
-// KH, KW, DH, DW: compile-time window and stride (0 = use the runtime arguments); the common 3x3 / 2 and
-// 2x2 / 2 windows get fully unrolled scans and shifts instead of divisions.
-template <int KH, int KW, int DH, int DW>
+// Any window and stride: grid.y strides over planes, grid.x * block over the plane's outputs (no division by the plane size).
 static __global__ void __launch_bounds__(256) maxpool_forward_kernel(const float *__restrict__ in, float *__restrict__ out,
                                                                      float *__restrict__ indy, float *__restrict__ indx,
                                                                      long planes, int H, int W, int oH, int oW, Div32 doW,
-                                                                     int kH_, int kW_, int dH_, int dW_) {
-  const int kH = KH ? KH : kH_, kW = KW ? KW : kW_, dH = DH ? DH : dH_, dW = DW ? DW : dW_;
+                                                                     int kH, int kW, int dH, int dW) {
   const unsigned P = (unsigned)(oH * oW);
   for (long plane = blockIdx.y; plane < planes; plane += gridDim.y) {
     const float *ip0 = in + plane * H * W;
@@ -51,9 +48,7 @@ static __global__ void __launch_bounds__(256) maxpool_forward_kernel(const float
       const float *ip = ip0 + (y * dH) * W + x * dW;
       float best = -INFINITY;  // the CPU starts from (float)(-DBL_MAX) = -inf
       int bi = -1, cnt = 0;
-#pragma unroll
       for (int i = 0; i < kH; i++)
-#pragma unroll
         for (int j = 0; j < kW; j++) {
           const float v = ip[i * W + j];
           if (v > best) { best = v; bi = cnt; }
@@ -71,19 +66,15 @@ static __global__ void __launch_bounds__(256) maxpool_forward_kernel(const float
 // Phase 1 turns every window that can reach the item's pixels into (flat position of its maximum, gradOutput
 // value) in shared memory, reading indices and gradOutput exactly once and coalesced; phase 2 lets every input
 // pixel scan the windows covering it.  Global traffic is the algorithmic minimum.
-static __device__ __forceinline__ float *gi_plane(float *gin, long plane, int HW) { return gin + plane * HW; }
-
-template <int KH, int KW, int DH, int DW>
 static __global__ void __launch_bounds__(256) maxpool_backward_kernel(const float *__restrict__ gout,
                                                                       const float *__restrict__ indy,
                                                                       const float *__restrict__ indx, float *__restrict__ gin,
                                                                       long planes, int H, int W, Div32 dW_in, int oH, int oW,
-                                                                      Div32 doW, int kH_, int kW_, int dH_, int dW_, Div32 ddH,
+                                                                      Div32 doW, int kH, int kW, int dH, int dW, Div32 ddH,
                                                                       Div32 ddW, int G, int band_rows, int bands) {
   extern __shared__ int pool_sm[];
-  const int kH = KH ? KH : kH_, kW = KW ? KW : kW_, dH = DH ? DH : dH_, dW = DW ? DW : dW_;
-  auto div_dH = [&](unsigned v) { return DH ? (int)(v / (unsigned)(DH ? DH : 1)) : (int)ddH.div(v); };
-  auto div_dW = [&](unsigned v) { return DW ? (int)(v / (unsigned)(DW ? DW : 1)) : (int)ddW.div(v); };
+  auto div_dH = [&](unsigned v) { return (int)ddH.div(v); };
+  auto div_dW = [&](unsigned v) { return (int)ddW.div(v); };
   const int HW = H * W, oHW = oH * oW;
   const long groups = (planes + G - 1) / G;
   const long items = groups * bands;
@@ -111,50 +102,6 @@ static __global__ void __launch_bounds__(256) maxpool_backward_kernel(const floa
       val[t] = gout[o];
     }
     __syncthreads();
-    if (KH && KW && DH && DW) {
-      // Fixed window shape: a thread owns one stride cell of DH x DW pixels.  The windows that can reach the
-      // cell are those of the cells up to NY-1 rows / NX-1 columns before it; each is fetched once and tested
-      // against every pixel of the cell, in ascending (y, x) order, which keeps the CPU's order of additions.
-      constexpr int cDH = DH ? DH : 1, cDW = DW ? DW : 1;
-      constexpr int NY = (KH + cDH - 1) / cDH, NX = (KW + cDW - 1) / cDW;
-      const int cW = (W + cDW - 1) / cDW, cH = (h1 - h0 + cDH - 1) / cDH, cells = cH * cW;
-      const int a0 = h0 / cDH;                       // band_rows is a multiple of dH
-      for (int t = threadIdx.x; t < np * cells; t += blockDim.x) {
-        int pl = 0, r = t;
-        if (np > 1) { pl = t / cells; r = t - pl * cells; }
-        const int ca = r / cW, b = r - ca * cW, a = a0 + ca;
-        const int *tp = tgt + pl * nwin;
-        const float *vp = val + pl * nwin;
-        float acc[cDH][cDW];
-#pragma unroll
-        for (int rr = 0; rr < cDH; rr++)
-#pragma unroll
-          for (int ss = 0; ss < cDW; ss++) acc[rr][ss] = 0.f;
-        const int me0 = a * cDH * W + b * cDW;       // flat position of the cell's first pixel
-#pragma unroll
-        for (int dy = 0; dy < NY; dy++) {
-          const int y = a - (NY - 1) + dy;
-#pragma unroll
-          for (int dx = 0; dx < NX; dx++) {
-            const int x = b - (NX - 1) + dx;
-            const bool in = y >= ylo && y <= yhi && x >= 0 && x < oW;
-            const int i = in ? (y - ylo) * oW + x : 0;
-            const int tg = in ? tp[i] : -1;
-            const float v = vp[i];
-#pragma unroll
-            for (int rr = 0; rr < cDH; rr++)
-#pragma unroll
-              for (int ss = 0; ss < cDW; ss++) acc[rr][ss] = tg == me0 + rr * W + ss ? acc[rr][ss] + v : acc[rr][ss];
-          }
-        }
-        float *gp = gi_plane(gin, p0 + pl, HW) + (long)a * cDH * W + b * cDW;
-#pragma unroll
-        for (int rr = 0; rr < cDH; rr++)
-#pragma unroll
-          for (int ss = 0; ss < cDW; ss++)
-            if (a * cDH + rr < h1 && b * cDW + ss < W) gp[rr * W + ss] = acc[rr][ss];
-      }
-    } else {
     const int npix = (h1 - h0) * W;            // per plane
     for (int t = threadIdx.x; t < np * npix; t += blockDim.x) {
       int pl = 0, r = t;
@@ -180,91 +127,203 @@ static __global__ void __launch_bounds__(256) maxpool_backward_kernel(const floa
         }
       gin[(p0 + pl) * HW + (long)h0 * W + r] = acc;
     }
-    }
     __syncthreads();
   }
 }
 
-// Backward for planes of at most 32 stride cells per row (the 55 / 27 / 13-wide planes of the AlexNet-style net, the
-// 56-wide and smaller ones of the VGG-style net), stride 2, windows of 2 or 3.  A group of LP lanes walks one plane
-// from the top, one row of windows per step; lane b holds window (y, b), read from global memory exactly once,
-// coalesced, with the next rows' loads already in flight.  Every window has ONE target pixel, so instead of testing
-// each pixel against each window that covers it, the window adds its value to its target in a three-row buffer in
-// shared memory (input rows 2y, 2y+1, 2y+2).  Two windows of a row can share a target only when they are
-// neighbours; then the right-hand lane adds both, left one first.  Together with the top-to-bottom walk this is the
-// CPU's order of additions (ascending window row, then column), so the result is bit-equal to it.  After a step
-// rows 2y and 2y+1 are final and leave as whole lines; row 2y+2 carries over as the next step's first row.
-template <int KH, int KW, int LP>
-static __global__ void __launch_bounds__(256, 8) maxpool_backward_rows_kernel(const float *__restrict__ gout,
-                                                                              const float *__restrict__ indy,
-                                                                              const float *__restrict__ indx,
-                                                                              float *__restrict__ gin, long planes, int H, int W,
-                                                                              int oH, int oW) {
-  static_assert(KH <= 3 && KW <= 3, "a window reaches at most one stride cell further");
-  constexpr int PPW = 32 / LP, RW = 2 * LP;          // planes per warp, floats per buffered row of one plane
-  __shared__ float rows_sm[8][3][64];
+// The 2 x 2 and 3 x 3 windows at stride 2.  A group of LP lanes takes a band of kBand rows of one plane (planes of more than LP
+// columns in tiles): all loads of the band are issued before the first is used, which is what keeps enough of them in flight
+// (a walk with two rows' prefetch reached 60 % of the HBM rate), and no index arithmetic is left per element.
+constexpr int kBand = 4;
+struct PoolGeom {
+  long planes;
+  int H, W, oH, oW, xtiles, bands;   // bands of output rows (forward) or cell rows (backward)
+};
+
+// Forward.  Lane `sub` owns window column x and reads input columns 2x and 2x + 1 of each row once (column 2x + 2 is the right-hand
+// lane's first); a row's maximum over the window's columns serves both windows it belongs to: 4.5 loads an output where a
+// thread per output issues 9.
+template <int K, int LP>
+static __global__ void __launch_bounds__(256) maxpool_forward_band_kernel(const float *__restrict__ in, float *__restrict__ out,
+                                                                          float *__restrict__ indy, float *__restrict__ indx, const PoolGeom p) {
+  constexpr int PPW = 32 / LP, ROWS = 2 * kBand + K - 2;
   const unsigned full = 0xffffffffu;
-  const int lane = threadIdx.x & 31, sub = lane % LP, seg = lane / LP, wib = threadIdx.x >> 5;
+  const int lane = threadIdx.x & 31, sub = lane % LP, seg = lane / LP;
   const long warps = ((long)gridDim.x * blockDim.x) >> 5, warp0 = ((long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int oHW = oH * oW;
-  const long groups = (planes + PPW - 1) / PPW;
-  const int i0 = seg * RW + sub, i1 = i0 + LP;       // this lane's two elements of a buffered row
-  for (long grp = warp0; grp < groups; grp += warps) {
+  const unsigned per_plane = (unsigned)(p.xtiles * p.bands);
+  const long items = (p.planes + PPW - 1) / PPW * per_plane;
+  for (long item = warp0; item < items; item += warps) {
+    const long grp = item / per_plane;
+    const unsigned r = (unsigned)(item - grp * per_plane), band = r / (unsigned)p.xtiles, xt = r - band * p.xtiles;
     const long plane = grp * PPW + seg;
-    const bool live = plane < planes;
-    const bool mine = live && sub < oW, st0 = live && sub < W, st1 = live && LP + sub < W;
-    const float *go = gout + plane * oHW + sub, *iy = indy + plane * oHW + sub, *ix = indx + plane * oHW + sub;
-    float *outp = gin + plane * (long)H * W + sub;   // this lane's first element of the row being written
-    float *r0 = rows_sm[wib][0], *r1 = rows_sm[wib][1], *r2 = rows_sm[wib][2];
-    r0[lane] = 0.f; r0[lane + 32] = 0.f; r1[lane] = 0.f; r1[lane + 32] = 0.f; r2[lane] = 0.f; r2[lane + 32] = 0.f;
-    __syncwarp();
-    // (target row - 2y) * 128 + target column, or -1 for "no window here"; value
-    auto load = [&](int y, int &t, float &v) {
-      t = -1; v = 0.f;
-      if (mine && y < oH) {
-        const int o = y * oW;
-        t = ((int)iy[o] - 1) * 128 + ((int)ix[o] - 1 + 2 * sub);
-        v = go[o];
-      }
-    };
-    int ct, qt[3], nt;
-    float cv, qv[3], nv;
-    load(0, ct, cv);
+    const int x = (int)xt * LP + sub, y0 = (int)band * kBand, h0 = 2 * y0;
+    const bool live = plane < p.planes, l0 = live && 2 * x < p.W, l1 = live && 2 * x + 1 < p.W;
+    const bool edge = K == 3 && sub == LP - 1 && live && 2 * x + 2 < p.W;   // the next lane's first column is in the next tile
+    const float *src = in + (plane * p.H + h0) * (long)p.W + 2 * x;
+    const float none = -INFINITY;   // the CPU starts from (float)(-DBL_MAX) = -inf
+    float a[ROWS], b[ROWS], c[ROWS];
 #pragma unroll
-    for (int d = 0; d < 3; d++) load(1 + d, qt[d], qv[d]);
-    // A finished row leaves as a line (lane `sub` writes elements sub and LP + sub) and its buffer is cleared by the
-    // lanes that read it: only columns below W can ever be targets.
-    auto flush = [&](float *row) {
-      if (st0) { outp[0] = row[i0]; row[i0] = 0.f; }
-      if (st1) { outp[LP] = row[i1]; row[i1] = 0.f; }
-      outp += W;
-    };
-    for (int y = 0; y < oH; y++) {
-      load(y + 4, nt, nv);
-      const int lt = __shfl_up_sync(full, ct, 1, LP), rt = __shfl_down_sync(full, ct, 1, LP);
-      const float lv = __shfl_up_sync(full, cv, 1, LP);
-      const bool with_left = sub > 0 && lt == ct;
-      const bool right_takes_it = sub < LP - 1 && rt == ct;
-      if (ct >= 0 && !right_takes_it) {
-        float *row = (ct >> 7) == 0 ? r0 : ((ct >> 7) == 1 ? r1 : r2);
-        float x = row[seg * RW + (ct & 127)];
-        if (with_left) x += lv;
-        row[seg * RW + (ct & 127)] = x + cv;
-      }
-      __syncwarp();
-      flush(r0);                                      // rows 2y and 2y + 1 are final (H >= 2 oH: both exist)
-      flush(r1);
-      __syncwarp();
-      float *z = r0; r0 = r2; r2 = r1; r1 = z;      // row 2y+2 becomes the next step's row 0; two cleared rows follow
-      ct = qt[0]; cv = qv[0];
-      qt[0] = qt[1]; qv[0] = qv[1]; qt[1] = qt[2]; qv[1] = qv[2]; qt[2] = nt; qv[2] = nv;
+    for (int k = 0; k < ROWS; k++) {
+      const bool ok = h0 + k < p.H;
+      a[k] = ok && l0 ? src[k * p.W] : none;
+      b[k] = ok && l1 ? src[k * p.W + 1] : none;
     }
-    // what lies below the last window row: the carried row, then rows no window reaches (zeros)
-    for (int h = 2 * oH; h < H; h++) flush(r0);
-    __syncwarp();
+    if (K == 3) {
+#pragma unroll
+      for (int k = 0; k < ROWS; k++) c[k] = edge && h0 + k < p.H ? src[k * p.W + 2] : none;
+    }
+    // maximum and its column of every row of the band (first one wins, NaN never does)
+    float m[ROWS];
+    int j[ROWS];
+#pragma unroll
+    for (int k = 0; k < ROWS; k++) {
+      m[k] = none; j[k] = -1;
+      if (a[k] > m[k]) { m[k] = a[k]; j[k] = 0; }
+      if (b[k] > m[k]) { m[k] = b[k]; j[k] = 1; }
+      if (K == 3) {
+        const float n = __shfl_down_sync(full, a[k], 1, LP), cc = sub < LP - 1 ? n : c[k];
+        if (cc > m[k]) { m[k] = cc; j[k] = 2; }
+      }
+    }
+    if (live && x < p.oW) {
+      const long o = (plane * p.oH + y0) * (long)p.oW + x;
+#pragma unroll
+      for (int y = 0; y < kBand; y++) {
+        if (y0 + y >= p.oH) break;
+        float best = m[2 * y];
+        int bi = 0, bj = j[2 * y];
+#pragma unroll
+        for (int k = 1; k < K; k++)
+          if (m[2 * y + k] > best) { best = m[2 * y + k]; bi = k; bj = j[2 * y + k]; }
+        // nothing found (all NaN / -inf): row 1, column 0, the CPU's (int)(-1 / kW) + 1 and (-1 % kW) + 1
+        out[o + y * p.oW] = best;
+        indy[o + y * p.oW] = (float)(bi + 1);
+        indx[o + y * p.oW] = (float)(bj + 1);
+      }
+    }
   }
 }
 
+// Backward for 3 x 3 windows.  Lane `sub` holds the windows (y, b) of its column and owns the four pixels of each cell (y, b), rows
+// 2y and 2y + 1, columns 2b and 2b + 1.  Those are reached by windows (y-1, b-1), (y-1, b), (y, b-1), (y, b) only, whose
+// target codes and values sit in this lane's and the left lane's registers: each pixel adds those that aim at it in that order,
+// the CPU's order of additions (ascending window row, then column), so the result is bit-equal to it.  A row of the result
+// leaves as 8-byte pairs, on odd addresses as the pairs one column to the left.
+// Planes of more than 32 cells: tiles of 31 cells whose first lane holds the window left of the tile.
+template <int LP>
+static __global__ void __launch_bounds__(256) maxpool3_backward_kernel(const float *__restrict__ gout, const float *__restrict__ indy,
+                                                                       const float *__restrict__ indx, float *__restrict__ gin, const PoolGeom p) {
+  constexpr int PPW = 32 / LP;
+  const unsigned full = 0xffffffffu;
+  const int lane = threadIdx.x & 31, sub = lane % LP, seg = lane / LP;
+  const long warps = ((long)gridDim.x * blockDim.x) >> 5, warp0 = ((long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const unsigned per_plane = (unsigned)(p.xtiles * p.bands);
+  const long items = (p.planes + PPW - 1) / PPW * per_plane;
+  const bool halo = p.xtiles > 1;
+  for (long item = warp0; item < items; item += warps) {
+    const long grp = item / per_plane;
+    const unsigned r = (unsigned)(item - grp * per_plane), band = r / (unsigned)p.xtiles, xt = r - band * p.xtiles;
+    const long plane = grp * PPW + seg;
+    const bool live = plane < p.planes;
+    const int b = halo ? (int)xt * (LP - 1) + sub - 1 : sub, y0 = (int)band * kBand;
+    const bool mine = live && b >= 0 && b < p.oW;
+    const bool keep = live && !(halo && sub == 0), c0 = keep && 2 * b < p.W, c1 = keep && 2 * b + 1 < p.W;
+    const long w0 = (plane * p.oH + y0) * (long)p.oW + b;
+    // windows y0 - 1 .. y0 + kBand - 1: 3 * row + column of the target, counted from 1 (4 .. 12; 0: no window), and value
+    float iy[kBand + 1], ix[kBand + 1], v[kBand + 1];
+#pragma unroll
+    for (int d = 0; d <= kBand; d++) {
+      const bool ok = mine && (unsigned)(y0 + d - 1) < (unsigned)p.oH;
+      const long o = w0 + (d - 1) * p.oW;
+      iy[d] = ok ? indy[o] : 0.f; ix[d] = ok ? indx[o] : 0.f; v[d] = ok ? gout[o] : 0.f;
+    }
+    float *dst = gin + (plane * p.H + 2 * y0) * (long)p.W + 2 * b;
+    bool odd = (reinterpret_cast<uintptr_t>(dst) & 4) != 0;
+    auto put = [&](float p0, float p1) {
+      const float left = __shfl_up_sync(full, p1, 1, LP);
+      if (!odd) {
+        if (c1) *reinterpret_cast<float2 *>(dst) = make_float2(p0, p1);
+        else if (c0) dst[0] = p0;
+      } else {
+        // the pair (2b - 1, 2b); the first lane of a row has no left column, the last column of an even row no right one
+        if (c0) {
+          if (sub > (halo ? 1 : 0)) *reinterpret_cast<float2 *>(dst - 1) = make_float2(left, p0);
+          else dst[0] = p0;
+        }
+        if (c1 && (sub == LP - 1 || 2 * b + 2 >= p.W)) dst[1] = p1;
+      }
+      dst += p.W;
+      odd ^= (p.W & 1) != 0;
+    };
+    auto add = [](float acc, bool hit, float x) { return hit ? acc + x : acc; };
+    float pt = fmaf(3.f, iy[0], ix[0]), pv = v[0];
+    float plt = __shfl_up_sync(full, pt, 1, LP), plv = __shfl_up_sync(full, pv, 1, LP);
+    if (sub == 0) plt = 0.f;
+#pragma unroll
+    for (int d = 1; d <= kBand; d++) {
+      if (2 * (y0 + d - 1) >= p.H) break;
+      const float t = fmaf(3.f, iy[d], ix[d]), x = v[d];
+      float lt = __shfl_up_sync(full, t, 1, LP);
+      const float lx = __shfl_up_sync(full, x, 1, LP);
+      if (sub == 0) lt = 0.f;
+      const float p00 = add(add(add(add(0.f, plt == 12.f, plv), pt == 10.f, pv), lt == 6.f, lx), t == 4.f, x);
+      const float p01 = add(add(0.f, pt == 11.f, pv), t == 5.f, x);
+      const float p10 = add(add(0.f, lt == 9.f, lx), t == 7.f, x);
+      const float p11 = add(0.f, t == 8.f, x);
+      put(p00, p01);
+      if (2 * (y0 + d - 1) + 1 < p.H) put(p10, p11);
+      pt = t; pv = x; plt = lt; plv = lx;
+    }
+  }
+}
+
+// Backward for windows of 2 x 2 at stride 2: every pixel belongs to one window.  A thread owns V neighbouring windows and writes
+// their 2 x 2V pixels (V = 2 where 16-byte stores are possible); rows and columns below and right of the last window are zero.
+template <int V>
+static __global__ void __launch_bounds__(256) maxpool2_backward_kernel(const float *__restrict__ gout, const float *__restrict__ indy,
+                                                                       const float *__restrict__ indx, float *__restrict__ gin, long rows,
+                                                                       int H, int W, int oH, int oW, int cells_h, int cells_w, Div32 dcw) {
+  // rows = planes * cells_h; a cell row has cells_w / V items
+  const int per = cells_w / V;
+  for (long row0 = blockIdx.y; row0 * 64 < rows; row0 += gridDim.y) {
+    const unsigned n = (unsigned)(min(64l, rows - row0 * 64) * per);
+    for (unsigned t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
+      const unsigned q = dcw.div(t);
+      const int x = (int)(t - q * per) * V;
+      const long row = row0 * 64 + q, plane = row / cells_h;
+      const int y = (int)(row - plane * cells_h);
+      float top[2 * V], low[2 * V];
+#pragma unroll
+      for (int k = 0; k < V; k++) {
+        float iy = 0.f, ix = 0.f, v = 0.f;
+        if (y < oH && x + k < oW) {
+          const long o = (plane * oH + y) * oW + x + k;
+          iy = indy[o]; ix = indx[o]; v = gout[o];
+        }
+        top[2 * k] = iy == 1.f && ix == 1.f ? v : 0.f; top[2 * k + 1] = iy == 1.f && ix == 2.f ? v : 0.f;
+        low[2 * k] = iy == 2.f && ix == 1.f ? v : 0.f; low[2 * k + 1] = iy == 2.f && ix == 2.f ? v : 0.f;
+      }
+      float *d = gin + (plane * H + 2 * y) * (long)W + 2 * x;
+      if constexpr (V == 2) {
+        *reinterpret_cast<float4 *>(d) = make_float4(top[0], top[1], top[2], top[3]);
+        if (2 * y + 1 < H) *reinterpret_cast<float4 *>(d + W) = make_float4(low[0], low[1], low[2], low[3]);
+      } else {
+        const bool second = 2 * x + 1 < W;
+        d[0] = top[0];
+        if (second) d[1] = top[1];
+        if (2 * y + 1 < H) {
+          d[W] = low[0];
+          if (second) d[W + 1] = low[1];
+        }
+      }
+    }
+  }
+}
+
+static unsigned band_blocks(const PoolGeom &p, int planes_per_warp) {
+  const long items = (p.planes + planes_per_warp - 1) / planes_per_warp * p.xtiles * p.bands;
+  return (unsigned)std::min((items + 7) / 8, (long)ctx().sm_count * 64);
+}
 static dim3 plane_grid(long planes, long per_plane) {
   long gx = (per_plane + 255) / 256;
   if (gx > 64) gx = 64;
@@ -347,15 +406,21 @@ THC_API int THGPUNN_SpatialMaxPooling_updateOutput(THGPUTensor *input, THGPUTens
   const long total = N * C * oH * oW;
   THC_CHECK(H * W < (1l << 31), "image plane too large");
   if (total > 0) {
-    const dim3 grid = plane_grid(N * C, oH * oW);
-#define THC_POOL_FWD(KH, KW, DH, DW)                                                                               \
-  maxpool_forward_kernel<KH, KW, DH, DW><<<grid, 256, 0, stream()>>>(                                              \
-      data_ptr(in), data_ptr(output), data_ptr(indices), data_ptr(indices) + total, N * C, (int)H, (int)W, (int)oH, \
-      (int)oW, Div32::make(oW), kH, kW, dH, dW)
-    if (kH == 3 && kW == 3 && dH == 2 && dW == 2) THC_POOL_FWD(3, 3, 2, 2);
-    else if (kH == 2 && kW == 2 && dH == 2 && dW == 2) THC_POOL_FWD(2, 2, 2, 2);
-    else THC_POOL_FWD(0, 0, 0, 0);
+    const float *src = data_ptr(in);
+    float *o = data_ptr(output), *iy = data_ptr(indices), *ix = iy + total;
+    if (dH == 2 && dW == 2 && kH == kW && (kH == 2 || kH == 3)) {
+      // lanes per plane: as many as it has window columns, up to a warp; wider planes are cut into tiles of 32 columns
+      const int LP = (W + 1) / 2 <= 8 ? 8 : (W + 1) / 2 <= 16 ? 16 : 32;
+      const int xtiles = (int)((oW + LP - 1) / LP);
+      const PoolGeom pg{N * C, (int)H, (int)W, (int)oH, (int)oW, xtiles, (int)((oH + kBand - 1) / kBand)};
+#define THC_POOL_FWD(K, LPV) maxpool_forward_band_kernel<K, LPV><<<band_blocks(pg, 32 / LP), 256, 0, stream()>>>(src, o, iy, ix, pg)
+      if (kH == 3) { if (LP == 8) THC_POOL_FWD(3, 8); else if (LP == 16) THC_POOL_FWD(3, 16); else THC_POOL_FWD(3, 32); }
+      else { if (LP == 8) THC_POOL_FWD(2, 8); else if (LP == 16) THC_POOL_FWD(2, 16); else THC_POOL_FWD(2, 32); }
 #undef THC_POOL_FWD
+    } else {
+      maxpool_forward_kernel<<<plane_grid(N * C, oH * oW), 256, 0, stream()>>>(src, o, iy, ix, N * C, (int)H, (int)W, (int)oH, (int)oW,
+                                                                               Div32::make(oW), kH, kW, dH, dW);
+    }
     check_launch("maxpool_forward");
   }
   return 0;
@@ -380,6 +445,29 @@ THC_API int THGPUNN_SpatialMaxPooling_updateGradInput(THGPUTensor *input, THGPUT
   const long total = N * C * H * W, ototal = N * C * oH * oW;
   THC_CHECK(H * W < (1l << 31), "image plane too large");
   if (total > 0) {
+    const float *g = data_ptr(go), *iy = data_ptr(ind), *ix = iy + ototal;
+    float *gi = data_ptr(gradInput);
+    const long cells_h = (H + 1) / 2, cells_w = (W + 1) / 2;
+    if (dH == 2 && dW == 2 && kH == 3 && kW == 3) {
+      const int LP = cells_w <= 8 ? 8 : cells_w <= 16 ? 16 : 32;
+      const int xtiles = cells_w <= 32 ? 1 : (int)((cells_w + 30) / 31);
+      const PoolGeom pg{N * C, (int)H, (int)W, (int)oH, (int)oW, xtiles, (int)((cells_h + kBand - 1) / kBand)};
+#define THC_POOL_BWD3(LPV) maxpool3_backward_kernel<LPV><<<band_blocks(pg, 32 / LP), 256, 0, stream()>>>(g, iy, ix, gi, pg)
+      if (LP == 8) THC_POOL_BWD3(8); else if (LP == 16) THC_POOL_BWD3(16); else THC_POOL_BWD3(32);
+#undef THC_POOL_BWD3
+      check_launch("maxpool_backward");
+      return 0;
+    }
+    if (dH == 2 && dW == 2 && kH == 2 && kW == 2 && cells_w < (1l << 24)) {
+      const bool vec = W % 4 == 0 && ((uintptr_t)gi & 15) == 0;
+      const long rows = N * C * cells_h, per = vec ? cells_w / 2 : cells_w;
+      const unsigned bx = (unsigned)std::min<long>((64 * per + 255) / 256, 16);
+      const unsigned by = (unsigned)std::min<long>((rows + 63) / 64, std::max<long>(1, ctx().sm_count * 32l / bx));
+      if (vec) maxpool2_backward_kernel<2><<<dim3(bx, by), 256, 0, stream()>>>(g, iy, ix, gi, rows, (int)H, (int)W, (int)oH, (int)oW, (int)cells_h, (int)cells_w, Div32::make(per));
+      else maxpool2_backward_kernel<1><<<dim3(bx, by), 256, 0, stream()>>>(g, iy, ix, gi, rows, (int)H, (int)W, (int)oH, (int)oW, (int)cells_h, (int)cells_w, Div32::make(per));
+      check_launch("maxpool_backward");
+      return 0;
+    }
     // shared memory holds (position, value) of up to kMaxWin windows per work item
     const int kMaxWin = 5120;
     int G = 1, band_rows = (int)H, bands = 1;
@@ -396,38 +484,15 @@ THC_API int THGPUNN_SpatialMaxPooling_updateGradInput(THGPUTensor *input, THGPUT
       if (band_rows < 1) band_rows = 1;
       bands = (int)((H + band_rows - 1) / band_rows);
     }
-    // narrow planes with the common windows: the row-buffer kernel
-    const long cW = (W + dW - 1) / dW;
-    const bool k33 = kH == 3 && kW == 3 && dH == 2 && dW == 2, k22 = kH == 2 && kW == 2 && dH == 2 && dW == 2;
-    if ((k33 || k22) && cW <= 32) {
-      const int LP = cW <= 8 ? 8 : (cW <= 16 ? 16 : 32);
-      const long groups = (N * C + 32 / LP - 1) / (32 / LP);
-      long blocks = (groups + 7) / 8;
-      const long cap = (long)ctx().sm_count * 8;
-      if (blocks > cap) blocks = cap;
-#define THC_POOL_BWD_WARP(KH, KW, LPV)                                                                                \
-  maxpool_backward_rows_kernel<KH, KW, LPV><<<(unsigned)blocks, 256, 0, stream()>>>(                                  \
-      data_ptr(go), data_ptr(ind), data_ptr(ind) + ototal, data_ptr(gradInput), N * C, (int)H, (int)W, (int)oH, (int)oW)
-      if (k33) { if (LP == 8) THC_POOL_BWD_WARP(3, 3, 8); else if (LP == 16) THC_POOL_BWD_WARP(3, 3, 16); else THC_POOL_BWD_WARP(3, 3, 32); }
-      else { if (LP == 8) THC_POOL_BWD_WARP(2, 2, 8); else if (LP == 16) THC_POOL_BWD_WARP(2, 2, 16); else THC_POOL_BWD_WARP(2, 2, 32); }
-#undef THC_POOL_BWD_WARP
-      check_launch("maxpool_backward");
-      return 0;
-    }
     const long items = ((N * C + G - 1) / G) * bands;
     // shared memory actually needed per work item: (position, value) per window
     const size_t smem = bands > 1 ? (size_t)kMaxWin * 8 : (size_t)G * oH * oW * 8;
     long blocks = items;
     const long cap = (long)ctx().sm_count * 8;
     if (blocks > cap) blocks = cap;
-#define THC_POOL_BWD(KH, KW, DH, DW)                                                                                \
-  maxpool_backward_kernel<KH, KW, DH, DW><<<(unsigned)blocks, 256, smem, stream()>>>(                         \
-      data_ptr(go), data_ptr(ind), data_ptr(ind) + ototal, data_ptr(gradInput), N * C, (int)H, (int)W, Div32::make(W), \
-      (int)oH, (int)oW, Div32::make(oW), kH, kW, dH, dW, Div32::make(dH), Div32::make(dW), G, band_rows, bands)
-    if (kH == 3 && kW == 3 && dH == 2 && dW == 2) THC_POOL_BWD(3, 3, 2, 2);
-    else if (kH == 2 && kW == 2 && dH == 2 && dW == 2) THC_POOL_BWD(2, 2, 2, 2);
-    else THC_POOL_BWD(0, 0, 0, 0);
-#undef THC_POOL_BWD
+    maxpool_backward_kernel<<<(unsigned)blocks, 256, smem, stream()>>>(g, iy, ix, gi, N * C, (int)H, (int)W, Div32::make(W), (int)oH, (int)oW,
+                                                                       Div32::make(oW), kH, kW, dH, dW, Div32::make(dH), Div32::make(dW), G,
+                                                                       band_rows, bands);
     check_launch("maxpool_backward");
   }
   return 0;
