@@ -169,7 +169,7 @@ static void window_product_t(const void *act, const mm::Windows &full, const mm:
   THC_CHECK(wrows * Kd < (1l << 31), "filter too large");
   void *wp = ws_alloc((size_t)wrows * Kd * (HALF ? 2 : 4));
   const long blocks = std::min<long>((wrows * (Kd / 4) + 255) / 256, ctx().sm_count * 8l);
-  repack_weight_kernel<HALF, FLIP><<<(unsigned)blocks, 256, 0, stream()>>>(w, u, (int)K, (int)rows, (int)v.C, PAIR ? full.dW : 0, wp);
+  pdl_launch(repack_weight_kernel<HALF, FLIP>, (unsigned)blocks, 256, 0, w, u, (int)K, (int)rows, (int)v.C, PAIR ? full.dW : 0, wp);
   check_launch("repack_weight");
   Problem<PlanesWindowOperand, RawOperand<false>, PAIR, HALF> p;
   attach_window_map<HALF>(p.a, act, v);
@@ -211,12 +211,12 @@ static const void *restated_input(const ConvGeom &g, const mm::Cells &u, const f
         THC_CUDA(cudaFuncSetAttribute(mm::columns8_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
         configured_for = ctx().device;
       }
-      mm::columns8_kernel<<<(unsigned)(g.N * u.Hs), 256, smem, stream()>>>(in, (uint4 *)dst, u);
+      pdl_launch(mm::columns8_kernel, (unsigned)(g.N * u.Hs), 256, smem, in, (uint4 *)dst, u);
       check_launch("columns8");
       return dst;
     }
   }
-  mm::cells_input_kernel<HALF><<<(unsigned)(g.N * u.Hs), 256, sizeof(int2) * u.Cs, stream()>>>(in, dst, u);
+  pdl_launch(mm::cells_input_kernel<HALF>, (unsigned)(g.N * u.Hs), 256, sizeof(int2) * u.Cs, in, dst, u);
   check_launch("cells_input");
   return dst;
 }
@@ -239,7 +239,7 @@ static void conv_grad_input_tc(const ConvGeom &g, const mm::ActPlanes &pgo, cons
   const long planes = g.N * g.C;
   const unsigned bx = (unsigned)std::min<long>((g.H * g.W + 255) / 256, 64);
   const unsigned by = (unsigned)std::min<long>(planes, std::max<long>(1, ctx().sm_count * 32l / bx));
-  mm::unfold_grad_input_kernel<<<dim3(bx, by), 256, 0, stream()>>>(gS, gin, g.N, u);
+  pdl_launch(mm::unfold_grad_input_kernel, dim3(bx, by), 256, 0, gS, gin, g.N, u);
   check_launch("unfold_grad_input");
 }
 
@@ -282,7 +282,7 @@ static void conv_acc_grad_tc(const ConvGeom &g, const mm::Cells &u, const void *
     });
     const WgradPlace pl{Nf, 1, 0, 0, 0, (int)f, Kp * Nf + Cs};
     const long total = g.K * g.R;
-    unpack_grad_weight_kernel<<<(unsigned)std::min<long>((total + 255) / 256, ctx().sm_count * 8l), 256, 0, stream()>>>(T, gw, u, (int)g.K, pl, scale);
+    pdl_launch(unpack_grad_weight_kernel, (unsigned)std::min<long>((total + 255) / 256, ctx().sm_count * 8l), 256, 0, T, gw, u, (int)g.K, pl, scale);
     check_launch("unpack_grad_weight");
     return;
   }
@@ -313,7 +313,7 @@ static void conv_acc_grad_tc(const ConvGeom &g, const mm::Cells &u, const void *
     pl = WgradPlace{1, N2, Cs * N2, -Kp, (u.kWs - 1) * Kp, 1, 0};
   }
   const long total = g.K * g.R;
-  unpack_grad_weight_kernel<<<(unsigned)std::min<long>((total + 255) / 256, ctx().sm_count * 8l), 256, 0, stream()>>>(T, gw, u, (int)g.K, pl, scale);
+  pdl_launch(unpack_grad_weight_kernel, (unsigned)std::min<long>((total + 255) / 256, ctx().sm_count * 8l), 256, 0, T, gw, u, (int)g.K, pl, scale);
   check_launch("unpack_grad_weight");
 }
 
@@ -351,6 +351,7 @@ static void conv_forward_simt(const ConvGeom &g, const float *in, const float *w
 // Wt[c][(ko, i, j)] = W[ko][(c, i, j)]: the weight matrix as the gathered gradInput product reads it.
 static __global__ void __launch_bounds__(256) transpose_weight_kernel(const float *__restrict__ w, float *__restrict__ wt,
                                                                       long K, long C, long kHW) {
+  pdl_begin();
   const long total = K * C * kHW;
   const long nthreads = (long)gridDim.x * blockDim.x;
   for (long t = (long)blockIdx.x * blockDim.x + threadIdx.x; t < total; t += nthreads) {
@@ -363,7 +364,7 @@ static void conv_grad_input_simt(const ConvGeom &g, const float *gout, const flo
   using namespace mm;
   const long kHW = (long)g.kH * g.kW, Kd = g.K * kHW;
   float *wt = (float *)ws_alloc(sizeof(float) * g.C * Kd);
-  transpose_weight_kernel<<<(unsigned)std::min<long>((g.C * Kd + 255) / 256, ctx().sm_count * 8l), 256, 0, stream()>>>(w, wt, g.K, g.C, kHW);
+  pdl_launch(transpose_weight_kernel, (unsigned)std::min<long>((g.C * Kd + 255) / 256, ctx().sm_count * 8l), 256, 0, w, wt, g.K, g.C, kHW);
   check_launch("transpose_weight");
   // rows = input pixels, k = (ko, i, j); only taps with (h + pad - i) % dH == 0 contribute
   Problem<Operand<PixelMap, TapMap, 2>, Operand<LinearMap, LinearMap, 0>> p;
@@ -402,6 +403,7 @@ static void conv_acc_grad_simt(const ConvGeom &g, const float *in, const float *
 static __global__ void __launch_bounds__(256) conv_grad_bias_partial_kernel(const float *__restrict__ gout,
                                                                             float *__restrict__ partial, long N, long K,
                                                                             long P) {
+  pdl_begin();
   __shared__ float sm[8];
   const long k = blockIdx.x;
   // One image per warp at a time (eight images in flight per block), four independent partial sums per lane:
@@ -429,6 +431,7 @@ static __global__ void __launch_bounds__(256) conv_grad_bias_partial_kernel(cons
 }
 static __global__ void conv_grad_bias_finish_kernel(const float *__restrict__ partial, float *gbias, long K, int S,
                                                     float scale) {
+  pdl_begin();
   const long k = (long)blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= K) return;
   float acc = 0.f;
@@ -441,9 +444,9 @@ static void grad_bias(const ConvGeom &g, const float *gout, float *gb, float sca
   if (S > g.N) S = g.N;
   if (S < 1) S = 1;
   float *partial = (float *)ws_alloc(sizeof(float) * g.K * S);
-  conv_grad_bias_partial_kernel<<<dim3((unsigned)g.K, (unsigned)S), 256, 0, stream()>>>(gout, partial, g.N, g.K, g.P);
+  pdl_launch(conv_grad_bias_partial_kernel, dim3((unsigned)g.K, (unsigned)S), 256, 0, gout, partial, g.N, g.K, g.P);
   check_launch("conv_grad_bias_partial");
-  conv_grad_bias_finish_kernel<<<ceil_div(g.K, 128), 128, 0, stream()>>>(partial, gb, g.K, (int)S, scale);
+  pdl_launch(conv_grad_bias_finish_kernel, ceil_div(g.K, 128), 128, 0, partial, gb, g.K, (int)S, scale);
   check_launch("conv_grad_bias_finish");
 }
 
@@ -492,7 +495,7 @@ static void conv_backward_tc(const ConvGeom &g, const float *in, const float *go
     conv_acc_grad_simt(g, in, gout, gw, scale);
   }
   if (pgo.chan_partial) {   // gradBias came along with the transposition of gradOutput
-    mm::chan_partial_finish_kernel<<<ceil_div(g.K, 32), 1024, 0, stream()>>>(pgo.chan_partial, pgo.chan_blocks, g.K, gb, scale);
+    pdl_launch(mm::chan_partial_finish_kernel, ceil_div(g.K, 32), 1024, 0, pgo.chan_partial, pgo.chan_blocks, g.K, gb, scale);
     check_launch("conv_grad_bias_finish");
   } else {
     grad_bias(g, gout, gb, scale);

@@ -48,6 +48,7 @@ static __device__ __forceinline__ double exp_minus_approx(double x) {
 
 // one block per row: out = x - (max + log(sum exp(x - max)))
 static __global__ void __launch_bounds__(256) logsoftmax_forward_kernel(const float *__restrict__ in, float *__restrict__ out, long dim) {
+  pdl_begin();
   __shared__ float smf[8];
   __shared__ double smd[8];
   const float *x = in + (long)blockIdx.x * dim;
@@ -64,6 +65,7 @@ static __global__ void __launch_bounds__(256) logsoftmax_forward_kernel(const fl
 // gradIn = gradOut - exp(out) * sum(gradOut)
 static __global__ void __launch_bounds__(256) logsoftmax_backward_kernel(const float *__restrict__ gout, const float *__restrict__ out,
                                                                          float *__restrict__ gin, long dim) {
+  pdl_begin();
   __shared__ double smd[8];
   const long b = (long)blockIdx.x * dim;
   double s = 0;
@@ -77,6 +79,7 @@ static __global__ void __launch_bounds__(256) logsoftmax_backward_kernel(const f
 // in double, out_d = z_d * (float)(1 / sum).  Backward: gradIn_d = out_d * (gradOut_d - sum_e gradOut_e * out_e),
 // the sum in double.
 static __global__ void __launch_bounds__(256) softmax_forward_kernel(const float *__restrict__ in, float *__restrict__ out, long dim) {
+  pdl_begin();
   __shared__ float smf[8];
   __shared__ double smd[8];
   const float *x = in + (long)blockIdx.x * dim;
@@ -96,6 +99,7 @@ static __global__ void __launch_bounds__(256) softmax_forward_kernel(const float
 }
 static __global__ void __launch_bounds__(256) softmax_backward_kernel(const float *__restrict__ gout, const float *__restrict__ out,
                                                                       float *__restrict__ gin, long dim) {
+  pdl_begin();
   __shared__ double smd[8];
   const long b = (long)blockIdx.x * dim;
   double s = 0;
@@ -107,6 +111,7 @@ static __global__ void __launch_bounds__(256) softmax_backward_kernel(const floa
 // loss = -sum_i in[i][target_i - 1] (/ nframe)
 static __global__ void __launch_bounds__(256) classnll_forward_kernel(const float *__restrict__ in, const float *__restrict__ target,
                                                                       float *out, long nframe, long dim, int size_average) {
+  pdl_begin();
   __shared__ double smd[8];
   double s = 0;
   for (long i = threadIdx.x; i < nframe; i += blockDim.x) {
@@ -117,6 +122,7 @@ static __global__ void __launch_bounds__(256) classnll_forward_kernel(const floa
   if (threadIdx.x == 0) out[0] = (float)(size_average ? s / (double)nframe : s);
 }
 static __global__ void classnll_backward_kernel(const float *__restrict__ target, float *gin, long nframe, long dim, float z) {
+  pdl_begin();
   const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= nframe) return;
   const long t = (long)target[i] - 1;
@@ -125,6 +131,7 @@ static __global__ void classnll_backward_kernel(const float *__restrict__ target
 
 static __global__ void __launch_bounds__(256) sgd_kernel(float *__restrict__ w, const float *__restrict__ g, float *__restrict__ v,
                                                          long n, float lr, float momentum) {
+  pdl_begin();
   const long nthreads = (long)gridDim.x * blockDim.x;
   const long tid = (long)blockIdx.x * blockDim.x + threadIdx.x;
   const long nvec = (((uintptr_t)w | (uintptr_t)g | (uintptr_t)v) & 15) == 0 ? n >> 2 : 0;
@@ -209,7 +216,7 @@ THC_API int THGPUNN_LogSoftMax_updateOutput(THGPUTensor *input, THGPUTensor *out
   tensor_resize_as(output, input);
   THC_CHECK(is_contiguous(output), "output must be contiguous");
   if (nframe > 0 && dim > 0) {
-    logsoftmax_forward_kernel<<<(unsigned)nframe, 256, 0, stream()>>>(data_ptr(in), data_ptr(output), dim);
+    pdl_launch(logsoftmax_forward_kernel, (unsigned)nframe, 256, 0, data_ptr(in), data_ptr(output), dim);
     check_launch("logsoftmax_forward");
   }
   return 0;
@@ -226,7 +233,7 @@ THC_API int THGPUNN_LogSoftMax_updateGradInput(THGPUTensor *input, THGPUTensor *
   tensor_resize_as(gradInput, output);
   THC_CHECK(is_contiguous(gradInput), "gradInput must be contiguous");
   if (nframe > 0 && dim > 0) {
-    logsoftmax_backward_kernel<<<(unsigned)nframe, 256, 0, stream()>>>(data_ptr(go), data_ptr(out), data_ptr(gradInput), dim);
+    pdl_launch(logsoftmax_backward_kernel, (unsigned)nframe, 256, 0, data_ptr(go), data_ptr(out), data_ptr(gradInput), dim);
     check_launch("logsoftmax_backward");
   }
   return 0;
@@ -241,7 +248,7 @@ THC_API int THGPUNN_ClassNLLCriterion_updateOutput(THGPUTensor *input, THGPUTens
   TensorRef in(tensor_new_contiguous(input)); TensorRef tg(tensor_new_contiguous(target));
   const long one[1] = {1};
   resize_nd(outputTensor, 1, one, nullptr);
-  classnll_forward_kernel<<<1, 256, 0, stream()>>>(data_ptr(in), data_ptr(tg), data_ptr(outputTensor), nframe, dim, sizeAverage);
+  pdl_launch(classnll_forward_kernel, 1, 256, 0, data_ptr(in), data_ptr(tg), data_ptr(outputTensor), nframe, dim, sizeAverage);
   check_launch("classnll_forward");
   return 0;
   THC_END(1)
@@ -257,7 +264,7 @@ THC_API int THGPUNN_ClassNLLCriterion_updateGradInput(THGPUTensor *input, THGPUT
   THC_CHECK(is_contiguous(gradInput), "gradInput must be contiguous");
   THC_CUDA(cudaMemsetAsync(data_ptr(gradInput), 0, sizeof(float) * nframe * dim, stream()));
   const float z = sizeAverage ? -1.f / (float)nframe : -1.f;
-  classnll_backward_kernel<<<ceil_div(nframe, 128), 128, 0, stream()>>>(data_ptr(tg), data_ptr(gradInput), nframe, dim, z);
+  pdl_launch(classnll_backward_kernel, ceil_div(nframe, 128), 128, 0, data_ptr(tg), data_ptr(gradInput), nframe, dim, z);
   check_launch("classnll_backward");
   return 0;
   THC_END(1)
@@ -286,7 +293,7 @@ THC_API int THGPUNN_SoftMax_updateOutput(THGPUTensor *input, THGPUTensor *output
   tensor_resize_as(output, input);
   THC_CHECK(is_contiguous(output), "output must be contiguous");
   if (nframe > 0 && dim > 0) {
-    softmax_forward_kernel<<<(unsigned)nframe, 256, 0, stream()>>>(data_ptr(in), data_ptr(output), dim);
+    pdl_launch(softmax_forward_kernel, (unsigned)nframe, 256, 0, data_ptr(in), data_ptr(output), dim);
     check_launch("SoftMax_updateOutput");
   }
   return 0;
@@ -304,7 +311,7 @@ THC_API int THGPUNN_SoftMax_updateGradInput(THGPUTensor *input, THGPUTensor *gra
   tensor_resize_as(gradInput, output);
   THC_CHECK(is_contiguous(gradInput), "gradInput must be contiguous");
   if (nframe > 0 && dim > 0) {
-    softmax_backward_kernel<<<(unsigned)nframe, 256, 0, stream()>>>(data_ptr(go), data_ptr(out), data_ptr(gradInput), dim);
+    pdl_launch(softmax_backward_kernel, (unsigned)nframe, 256, 0, data_ptr(go), data_ptr(out), data_ptr(gradInput), dim);
     check_launch("SoftMax_updateGradInput");
   }
   return 0;

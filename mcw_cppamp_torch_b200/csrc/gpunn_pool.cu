@@ -39,6 +39,7 @@ static __global__ void __launch_bounds__(256) maxpool_forward_kernel(const float
                                                                      float *__restrict__ indy, float *__restrict__ indx,
                                                                      long planes, int H, int W, int oH, int oW, Div32 doW,
                                                                      int kH, int kW, int dH, int dW) {
+  pdl_begin();
   const unsigned P = (unsigned)(oH * oW);
   for (long plane = blockIdx.y; plane < planes; plane += gridDim.y) {
     const float *ip0 = in + plane * H * W;
@@ -72,6 +73,7 @@ static __global__ void __launch_bounds__(256) maxpool_backward_kernel(const floa
                                                                       long planes, int H, int W, Div32 dW_in, int oH, int oW,
                                                                       Div32 doW, int kH, int kW, int dH, int dW, Div32 ddH,
                                                                       Div32 ddW, int G, int band_rows, int bands) {
+  pdl_begin();
   extern __shared__ int pool_sm[];
   auto div_dH = [&](unsigned v) { return (int)ddH.div(v); };
   auto div_dW = [&](unsigned v) { return (int)ddW.div(v); };
@@ -146,6 +148,7 @@ struct PoolGeom {
 template <int K, int LP>
 static __global__ void __launch_bounds__(256) maxpool_forward_band_kernel(const float *__restrict__ in, float *__restrict__ out,
                                                                           float *__restrict__ indy, float *__restrict__ indx, const PoolGeom p) {
+  pdl_begin();
   constexpr int PPW = 32 / LP, ROWS = 2 * kBand + K - 2;
   const unsigned full = 0xffffffffu;
   const int lane = threadIdx.x & 31, sub = lane % LP, seg = lane / LP;
@@ -213,6 +216,7 @@ static __global__ void __launch_bounds__(256) maxpool_forward_band_kernel(const 
 template <int LP>
 static __global__ void __launch_bounds__(256) maxpool3_backward_kernel(const float *__restrict__ gout, const float *__restrict__ indy,
                                                                        const float *__restrict__ indx, float *__restrict__ gin, const PoolGeom p) {
+  pdl_begin();
   constexpr int PPW = 32 / LP;
   const unsigned full = 0xffffffffu;
   const int lane = threadIdx.x & 31, sub = lane % LP, seg = lane / LP;
@@ -283,6 +287,7 @@ template <int V>
 static __global__ void __launch_bounds__(256) maxpool2_backward_kernel(const float *__restrict__ gout, const float *__restrict__ indy,
                                                                        const float *__restrict__ indx, float *__restrict__ gin, long rows,
                                                                        int H, int W, int oH, int oW, int cells_h, int cells_w, Div32 dcw) {
+  pdl_begin();
   // rows = planes * cells_h; a cell row has cells_w / V items
   const int per = cells_w / V;
   for (long row0 = blockIdx.y; row0 * 64 < rows; row0 += gridDim.y) {
@@ -343,6 +348,7 @@ static dim3 plane_grid(long planes, long per_plane) {
 static __global__ void __launch_bounds__(256) sumpool_forward_kernel(const float *__restrict__ in, float *__restrict__ out,
                                                                      long planes, int H, int W, int oH, int oW, int kH, int kW,
                                                                      int dH, int dW) {
+  pdl_begin();
   const long total = planes * oH * oW;
   for (long t = (long)blockIdx.x * blockDim.x + threadIdx.x; t < total; t += (long)gridDim.x * blockDim.x) {
     const int x = (int)(t % oW);
@@ -359,6 +365,7 @@ static __global__ void __launch_bounds__(256) sumpool_forward_kernel(const float
 static __global__ void __launch_bounds__(256) sumpool_backward_kernel(const float *__restrict__ gout, float *__restrict__ gin,
                                                                       long planes, int H, int W, int oH, int oW, int kH, int kW,
                                                                       int dH, int dW) {
+  pdl_begin();
   const long total = planes * H * W;
   for (long t = (long)blockIdx.x * blockDim.x + threadIdx.x; t < total; t += (long)gridDim.x * blockDim.x) {
     const int w = (int)(t % W);
@@ -413,12 +420,12 @@ THC_API int THGPUNN_SpatialMaxPooling_updateOutput(THGPUTensor *input, THGPUTens
       const int LP = (W + 1) / 2 <= 8 ? 8 : (W + 1) / 2 <= 16 ? 16 : 32;
       const int xtiles = (int)((oW + LP - 1) / LP);
       const PoolGeom pg{N * C, (int)H, (int)W, (int)oH, (int)oW, xtiles, (int)((oH + kBand - 1) / kBand)};
-#define THC_POOL_FWD(K, LPV) maxpool_forward_band_kernel<K, LPV><<<band_blocks(pg, 32 / LP), 256, 0, stream()>>>(src, o, iy, ix, pg)
+#define THC_POOL_FWD(K, LPV) pdl_launch(maxpool_forward_band_kernel<K, LPV>, band_blocks(pg, 32 / LP), 256, 0, src, o, iy, ix, pg)
       if (kH == 3) { if (LP == 8) THC_POOL_FWD(3, 8); else if (LP == 16) THC_POOL_FWD(3, 16); else THC_POOL_FWD(3, 32); }
       else { if (LP == 8) THC_POOL_FWD(2, 8); else if (LP == 16) THC_POOL_FWD(2, 16); else THC_POOL_FWD(2, 32); }
 #undef THC_POOL_FWD
     } else {
-      maxpool_forward_kernel<<<plane_grid(N * C, oH * oW), 256, 0, stream()>>>(src, o, iy, ix, N * C, (int)H, (int)W, (int)oH, (int)oW,
+      pdl_launch(maxpool_forward_kernel, plane_grid(N * C, oH * oW), 256, 0, src, o, iy, ix, N * C, (int)H, (int)W, (int)oH, (int)oW,
                                                                                Div32::make(oW), kH, kW, dH, dW);
     }
     check_launch("maxpool_forward");
@@ -452,7 +459,7 @@ THC_API int THGPUNN_SpatialMaxPooling_updateGradInput(THGPUTensor *input, THGPUT
       const int LP = cells_w <= 8 ? 8 : cells_w <= 16 ? 16 : 32;
       const int xtiles = cells_w <= 32 ? 1 : (int)((cells_w + 30) / 31);
       const PoolGeom pg{N * C, (int)H, (int)W, (int)oH, (int)oW, xtiles, (int)((cells_h + kBand - 1) / kBand)};
-#define THC_POOL_BWD3(LPV) maxpool3_backward_kernel<LPV><<<band_blocks(pg, 32 / LP), 256, 0, stream()>>>(g, iy, ix, gi, pg)
+#define THC_POOL_BWD3(LPV) pdl_launch(maxpool3_backward_kernel<LPV>, band_blocks(pg, 32 / LP), 256, 0, g, iy, ix, gi, pg)
       if (LP == 8) THC_POOL_BWD3(8); else if (LP == 16) THC_POOL_BWD3(16); else THC_POOL_BWD3(32);
 #undef THC_POOL_BWD3
       check_launch("maxpool_backward");
@@ -463,8 +470,8 @@ THC_API int THGPUNN_SpatialMaxPooling_updateGradInput(THGPUTensor *input, THGPUT
       const long rows = N * C * cells_h, per = vec ? cells_w / 2 : cells_w;
       const unsigned bx = (unsigned)std::min<long>((64 * per + 255) / 256, 16);
       const unsigned by = (unsigned)std::min<long>((rows + 63) / 64, std::max<long>(1, ctx().sm_count * 32l / bx));
-      if (vec) maxpool2_backward_kernel<2><<<dim3(bx, by), 256, 0, stream()>>>(g, iy, ix, gi, rows, (int)H, (int)W, (int)oH, (int)oW, (int)cells_h, (int)cells_w, Div32::make(per));
-      else maxpool2_backward_kernel<1><<<dim3(bx, by), 256, 0, stream()>>>(g, iy, ix, gi, rows, (int)H, (int)W, (int)oH, (int)oW, (int)cells_h, (int)cells_w, Div32::make(per));
+      if (vec) pdl_launch(maxpool2_backward_kernel<2>, dim3(bx, by), 256, 0, g, iy, ix, gi, rows, (int)H, (int)W, (int)oH, (int)oW, (int)cells_h, (int)cells_w, Div32::make(per));
+      else pdl_launch(maxpool2_backward_kernel<1>, dim3(bx, by), 256, 0, g, iy, ix, gi, rows, (int)H, (int)W, (int)oH, (int)oW, (int)cells_h, (int)cells_w, Div32::make(per));
       check_launch("maxpool_backward");
       return 0;
     }
@@ -490,7 +497,7 @@ THC_API int THGPUNN_SpatialMaxPooling_updateGradInput(THGPUTensor *input, THGPUT
     long blocks = items;
     const long cap = (long)ctx().sm_count * 8;
     if (blocks > cap) blocks = cap;
-    maxpool_backward_kernel<<<(unsigned)blocks, 256, smem, stream()>>>(g, iy, ix, gi, N * C, (int)H, (int)W, Div32::make(W), (int)oH, (int)oW,
+    pdl_launch(maxpool_backward_kernel, (unsigned)blocks, 256, smem, g, iy, ix, gi, N * C, (int)H, (int)W, Div32::make(W), (int)oH, (int)oW,
                                                                        Div32::make(oW), kH, kW, dH, dW, Div32::make(dH), Div32::make(dW), G,
                                                                        band_rows, bands);
     check_launch("maxpool_backward");
@@ -516,7 +523,7 @@ THC_API int THGPUNN_SpatialAveragePooling_updateOutput(THGPUTensor *input, THGPU
   if (total > 0) {
     long blocks = (total + 255) / 256;
     if (blocks > (long)ctx().sm_count * 16) blocks = (long)ctx().sm_count * 16;
-    sumpool_forward_kernel<<<(unsigned)blocks, 256, 0, stream()>>>(data_ptr(in), data_ptr(output), N * C, (int)H, (int)W, (int)oH,
+    pdl_launch(sumpool_forward_kernel, (unsigned)blocks, 256, 0, data_ptr(in), data_ptr(output), N * C, (int)H, (int)W, (int)oH,
                                                                   (int)oW, kH, kW, dH, dW);
     check_launch("SpatialAveragePooling_updateOutput");
   }
@@ -543,7 +550,7 @@ THC_API int THGPUNN_SpatialAveragePooling_updateGradInput(THGPUTensor *input, TH
   if (total > 0) {
     long blocks = (total + 255) / 256;
     if (blocks > (long)ctx().sm_count * 16) blocks = (long)ctx().sm_count * 16;
-    sumpool_backward_kernel<<<(unsigned)blocks, 256, 0, stream()>>>(data_ptr(go), data_ptr(gradInput), N * C, (int)H, (int)W, (int)oH,
+    pdl_launch(sumpool_backward_kernel, (unsigned)blocks, 256, 0, data_ptr(go), data_ptr(gradInput), N * C, (int)H, (int)W, (int)oH,
                                                                    (int)oW, kH, kW, dH, dW);
     check_launch("SpatialAveragePooling_updateGradInput");
   }

@@ -51,11 +51,10 @@ static void launch_simt(P p) {
     splits = (p.K + p.k_per_split - 1) / p.k_per_split;
   }
   if (splits > 1) p.ws = (float *)ws_alloc(sizeof(float) * splits * p.M * p.N);
-  simt_kernel<P><<<dim3((unsigned)gm, (unsigned)gn, (unsigned)splits), 256, 0, stream()>>>(p);
+  pdl_launch(simt_kernel<P>, dim3((unsigned)gm, (unsigned)gn, (unsigned)splits), 256, 0, p);
   check_launch("simt_kernel");
   if (splits > 1) {
-    splitk_finish_kernel<<<dim3((unsigned)ceil_div(p.M, 256), (unsigned)(p.N < 32768 ? p.N : 32768)), 256, 0, stream()>>>(
-        p.ws, (int)splits, p.M, p.N, p.epi);
+    pdl_launch(splitk_finish_kernel, dim3((unsigned)ceil_div(p.M, 256), (unsigned)(p.N < 32768 ? p.N : 32768)), 256, 0, p.ws, (int)splits, p.M, p.N, p.epi);
     check_launch("splitk_finish");
   }
 }
@@ -188,6 +187,32 @@ static void attach_window_rows_map(WindowRowsOperand &op, const void *base, cons
   encode_windows<HALF>(&op.tmap, base, v, HALF ? 64 : 32, true);
 }
 
+// Width of the two-SM tile that pads N least (wider wins ties).  An MN-major BF16 operand on the N side comes in blocks of
+// 64 rows per CTA, which leaves 256 and 128.
+static int tc2_tile_width(long N, bool half_mn = false) {
+  int best = 0;
+  long best_pad = 0;
+  const int widths[4] = {256, 192, 128, 64};
+  for (int w : widths) {
+    if (half_mn && w % 128 != 0) continue;
+    const long pad = (N + w - 1) / w * w;
+    if (!best || pad < best_pad) { best = w; best_pad = pad; }
+  }
+  return best;
+}
+// Microseconds a cluster takes for one k tile of a tile of this width, as the convolution and addmm launches at full size show it.
+static double tc2_tile_us(int bn2, bool half) {
+  if (half) return bn2 == 256 ? 0.55 : bn2 == 192 ? 0.47 : 0.4;
+  return bn2 == 256 ? 1.25 : bn2 == 192 ? 1.0 : bn2 == 128 ? 0.79 : 0.7;
+}
+// Model of a product's time, for choices between ways of stating it.
+static double tc2_product_us(long M, long N, long K, bool half, bool half_mn = false) {
+  const int w = tc2_tile_width(N, half && half_mn), kv = half ? 64 : 32;
+  const double tiles = (double)((M + 255) / 256) * (double)((N + w - 1) / w), ktiles = (double)((K + kv - 1) / kv);
+  // a tile's epilogue and hand-over take about as long as two k tiles; a tile cut along k keeps at least six
+  return std::max(tiles * (ktiles + 2) / (ctx().sm_count / 2), std::min(ktiles, 6.0) + 2) * tc2_tile_us(w, half) + 8;
+}
+
 // Clusters of the two-SM kernel that the device runs at once (the kernel is persistent: a launch has no more).
 template <class P, int BN2>
 static int tc2r_resident_clusters() {
@@ -219,35 +244,10 @@ template <class P, int BN2>
 static void launch_tc2r_kernel(const P &p, long items) {
   typedef Tc2rCfg<BN2, P::HALF> Cfg;
   const long clusters = std::min<long>(items, tc2r_resident_clusters<P, BN2>());
-  tc2r_kernel<P, BN2><<<dim3((unsigned)(2 * clusters), 1, 1), T2_THREADS, Cfg::SMEM_BYTES, stream()>>>(p, stall_ctl(),
-                                                                                                                sched_counter());
+  // a long launch gains nothing from starting early, and measured 1.5 % slower when it did (4096^3: 671 -> 682 us)
+  const bool early = tc2_product_us(p.M, p.N, p.K, P::HALF, P::HALF && P::OpB::MN_MAJOR) < 100;
+  launch_on_stream(early, tc2r_kernel<P, BN2>, dim3((unsigned)(2 * clusters), 1, 1), T2_THREADS, Cfg::SMEM_BYTES, p, stall_ctl(), sched_counter());
   check_launch("tc2r_kernel");
-}
-
-// Width of the two-SM tile that pads N least (wider wins ties).  An MN-major BF16 operand on the N side comes in blocks of
-// 64 rows per CTA, which leaves 256 and 128.
-static int tc2_tile_width(long N, bool half_mn = false) {
-  int best = 0;
-  long best_pad = 0;
-  const int widths[4] = {256, 192, 128, 64};
-  for (int w : widths) {
-    if (half_mn && w % 128 != 0) continue;
-    const long pad = (N + w - 1) / w * w;
-    if (!best || pad < best_pad) { best = w; best_pad = pad; }
-  }
-  return best;
-}
-// Microseconds a cluster takes for one k tile of a tile of this width, as the convolution and addmm launches at full size show it.
-static double tc2_tile_us(int bn2, bool half) {
-  if (half) return bn2 == 256 ? 0.55 : bn2 == 192 ? 0.47 : 0.4;
-  return bn2 == 256 ? 1.25 : bn2 == 192 ? 1.0 : bn2 == 128 ? 0.79 : 0.7;
-}
-// Model of a product's time, for choices between ways of stating it.
-static double tc2_product_us(long M, long N, long K, bool half, bool half_mn = false) {
-  const int w = tc2_tile_width(N, half && half_mn), kv = half ? 64 : 32;
-  const double tiles = (double)((M + 255) / 256) * (double)((N + w - 1) / w), ktiles = (double)((K + kv - 1) / kv);
-  // a tile's epilogue and hand-over take about as long as two k tiles; a tile cut along k keeps at least six
-  return std::max(tiles * (ktiles + 2) / (ctx().sm_count / 2), std::min(ktiles, 6.0) + 2) * tc2_tile_us(w, half) + 8;
 }
 
 // Products over operands that TMA can fetch.  `attach(p, bn2)` writes the operands' tensor maps for the chosen tile width.
@@ -300,8 +300,7 @@ static void launch_raw(P p, Attach attach) {
   if (p.ws) {
     // a few thousand blocks whatever the number of tail tiles: a lone tile cut into many slices gets a block per column
     const long by = std::min<long>(bn2, std::max<long>(32, ceil_div(8l * ctx().sm_count, tail)));
-    tail_finish_kernel<<<dim3((unsigned)tail, (unsigned)by), 256, 0, stream()>>>(
-        p.ws, p.tail_splits, bn2, p.tail_first, gm, p.M, p.N, p.epi);
+    pdl_launch(tail_finish_kernel, dim3((unsigned)tail, (unsigned)by), 256, 0, p.ws, p.tail_splits, bn2, p.tail_first, gm, p.M, p.N, p.epi);
     check_launch("tail_finish");
   }
 }
@@ -316,7 +315,7 @@ static void launch_small_kernel(const SmallProblem &p) {
     configured_for = ctx().device;
   }
   const dim3 grid((unsigned)ceil_div(p.M, BM), (unsigned)ceil_div(p.N, BN), (unsigned)p.slices);
-  small_kernel<BM, BN, WM, WN, A_K, B_K><<<grid, SM_THREADS, SMEM, stream()>>>(p);
+  pdl_launch(small_kernel<BM, BN, WM, WN, A_K, B_K>, grid, SM_THREADS, SMEM, p);
   check_launch("small_kernel");
 }
 template <int BN, int WM, int WN>
@@ -399,7 +398,7 @@ static ActPlanes make_act_planes(const float *src, long N, long C, long H, long 
     ap.chan_partial = (float *)ws_alloc(sizeof(float) * blocks * C);
     smem = sizeof(float) * C;
   }
-  nchw_to_planes_kernel<HALF><<<(unsigned)blocks, 256, smem, stream()>>>(src, N, (int)C, (int)HW, (int)ap.Cp, ap.p, ap.chan_partial);
+  pdl_launch(nchw_to_planes_kernel<HALF>, (unsigned)blocks, 256, smem, src, N, (int)C, (int)HW, (int)ap.Cp, ap.p, ap.chan_partial);
   check_launch("nchw_to_planes");
   return ap;
 }
@@ -414,7 +413,7 @@ static HalfMatrix make_half_matrix(const float *src, long rs, long ks, long rows
   hm.ld = (K + 63) / 64 * 64;
   hm.p = (__nv_bfloat16 *)ws_alloc(sizeof(__nv_bfloat16) * rows * hm.ld);
   const long blocks = std::min(((rows + 63) / 64) * (hm.ld / 64), (long)ctx().sm_count * 16);
-  bf16_rows_kernel<<<(unsigned)blocks, 256, 0, stream()>>>(src, rs, ks, rows, K, hm.p, hm.ld);
+  pdl_launch(bf16_rows_kernel, (unsigned)blocks, 256, 0, src, rs, ks, rows, K, hm.p, hm.ld);
   check_launch("bf16_rows");
   return hm;
 }

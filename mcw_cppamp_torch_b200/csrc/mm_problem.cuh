@@ -210,6 +210,7 @@ struct WindowRowsOperand {
 template <bool HALF>
 static __global__ void __launch_bounds__(256) nchw_to_planes_kernel(const float *__restrict__ src, long N, int C, int HW, int Cp,
                                                                     void *__restrict__ dst, float *__restrict__ chan_partial) {
+  pdl_begin();
   constexpr int CT = HALF ? 64 : 32, PT = HALF ? 64 : 128;
   __shared__ float tile[CT][PT + 1];
   extern __shared__ float chan_sum[];   // [C] when chan_partial is given
@@ -265,6 +266,7 @@ static __global__ void __launch_bounds__(256) nchw_to_planes_kernel(const float 
 // dependent loads per thread, hence the wide block.
 static __global__ void __launch_bounds__(1024) chan_partial_finish_kernel(const float *__restrict__ partial, int nblocks, long C,
                                                                           float *out, float scale) {
+  pdl_begin();
   __shared__ float sm[32][33];
   const int lane = threadIdx.x & 31, s = threadIdx.x >> 5;
   const long c = (long)blockIdx.x * 32 + lane;
@@ -323,6 +325,7 @@ struct Cells {
 // looks up in a table; neighbouring threads hold neighbouring channels, i.e. neighbouring columns of a few input rows.
 template <bool HALF>
 static __global__ void __launch_bounds__(256) cells_input_kernel(const float *__restrict__ in, void *__restrict__ S, const Cells u) {
+  pdl_begin();
   constexpr int V = HALF ? 8 : 4;
   extern __shared__ int2 chan_src[];      // per channel: offset in the image, (dy << 16 | dx) or -1
   for (int ch = threadIdx.x; ch < u.Cs; ch += blockDim.x) {
@@ -361,6 +364,7 @@ static __global__ void __launch_bounds__(256) cells_input_kernel(const float *__
 // kH * kW times over, so that the kernel is bound by the writes (gathering each value from the image took four times as
 // long: 1105 -> 280 us for 256 images under the 11 x 11 / 4 filter, 1.6 GB).
 static __global__ void __launch_bounds__(256) columns8_kernel(const float *__restrict__ in, uint4 *__restrict__ S, const Cells u) {
+  pdl_begin();
   extern __shared__ uint4 px_rows[];   // [kH][W + 2 pad]
   const long n = blockIdx.x / u.Hs;
   const int Y = (int)(blockIdx.x - n * u.Hs), Wp = u.W + 2 * u.pad, taps = u.kH * u.kW, q = u.Cs / 8;
@@ -398,6 +402,7 @@ static __global__ void __launch_bounds__(256) columns8_kernel(const float *__res
 template <bool HALF, bool FLIP>
 static __global__ void __launch_bounds__(256) repack_weight_kernel(const float *__restrict__ w, const Cells u, int K, int rows, int chans,
                                                                    int pair_shift, void *__restrict__ out) {
+  pdl_begin();
   const int kWe = u.kWs + pair_shift, quads = u.kHs * kWe * (chans / 4);
   const unsigned total = (unsigned)((pair_shift ? 2 : 1) * rows) * (unsigned)quads;
   for (unsigned t = blockIdx.x * blockDim.x + threadIdx.x; t < total; t += gridDim.x * blockDim.x) {
@@ -431,6 +436,7 @@ static __global__ void __launch_bounds__(256) repack_weight_kernel(const float *
 struct WgradPlace { long ko_stride, ch_stride, bi_stride, bj_stride, first; int copies; long copy_stride; };
 static __global__ void __launch_bounds__(256) unpack_grad_weight_kernel(const float *__restrict__ T, float *__restrict__ gw, const Cells u,
                                                                         int K, const WgradPlace p, float scale) {
+  pdl_begin();
   const unsigned kHW = (unsigned)(u.kH * u.kW), per = (unsigned)u.C * kHW, total = (unsigned)K * per;
   for (unsigned t = blockIdx.x * blockDim.x + threadIdx.x; t < total; t += gridDim.x * blockDim.x) {
     const unsigned ko = t / per, r = t - ko * per, c = r / kHW, tap = r - c * kHW, i = tap / (unsigned)u.kW, j = tap - i * u.kW;
@@ -448,6 +454,7 @@ static __global__ void __launch_bounds__(256) unpack_grad_weight_kernel(const fl
 // window reaches and the cells' channels; the others get zero).  gS: [N][Cr][Hs][Ws].
 static __global__ void __launch_bounds__(256) unfold_grad_input_kernel(const float *__restrict__ gS, float *__restrict__ gin, long N,
                                                                        const Cells u) {
+  pdl_begin();
   const unsigned HW = (unsigned)(u.H * u.W);
   const long planes = N * u.C;
   for (long pl = blockIdx.y; pl < planes; pl += gridDim.y) {
@@ -468,6 +475,7 @@ static __global__ void __launch_bounds__(256) unfold_grad_input_kernel(const flo
 // 64 x 64 tiles: along k as they lie, else through shared memory.
 static __global__ void __launch_bounds__(256) bf16_rows_kernel(const float *__restrict__ src, long rs, long ks, long rows, long K,
                                                                __nv_bfloat16 *__restrict__ out, long ld) {
+  pdl_begin();
   __shared__ float tile[64][65];
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
   const long tiles_k = ld / 64;
@@ -806,6 +814,7 @@ __device__ __forceinline__ void tc2_store_pair_rows(const P &p, const float (&ac
 // m, which is contiguous in the workspace.
 static __global__ void __launch_bounds__(256) splitk_finish_kernel(const float *__restrict__ ws, int splits, long M, long N,
                                                             Epilogue epi) {
+  pdl_begin();
   const long m = (long)blockIdx.x * blockDim.x + threadIdx.x;
   if (m >= M) return;
   const bool pair = epi.pair_K != 0;
@@ -824,6 +833,7 @@ static __global__ void __launch_bounds__(256) splitk_finish_kernel(const float *
 // workspace.
 static __global__ void __launch_bounds__(256) tail_finish_kernel(const float *__restrict__ ws, int splits, int bn2, long tail_first,
                                                           long gm, long M, long N, Epilogue epi) {
+  pdl_begin();
   const long tile = tail_first + blockIdx.x;
   const long nt = tile / gm, mt = tile - nt * gm;
   const long m = mt * 256 + threadIdx.x;

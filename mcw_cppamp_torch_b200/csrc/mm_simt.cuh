@@ -15,6 +15,7 @@ constexpr int SIMT_BM = 64, SIMT_BN = 64, SIMT_BK = 16;
 
 template <class P>
 __global__ void __launch_bounds__(256) simt_kernel(const P p) {
+  pdl_begin();
   __shared__ float As[SIMT_BK][SIMT_BM + 4];
   __shared__ float Bs[SIMT_BK][SIMT_BN + 4];
   __shared__ Info kiA[SIMT_BK], kiB[SIMT_BK];

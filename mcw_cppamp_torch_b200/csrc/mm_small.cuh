@@ -138,6 +138,7 @@ __device__ __forceinline__ void split_tf32(float x, uint32_t &hi, uint32_t &lo) 
 // WM x WN warps, each (BM / WM) x (BN / WN)
 template <int BM, int BN, int WM, int WN, bool A_K, bool B_K>
 __global__ void __launch_bounds__(SM_THREADS) small_kernel(const SmallProblem p) {
+  pdl_begin();
   static_assert(WM * WN * 32 == SM_THREADS && BM % (16 * WM) == 0 && BN % (8 * WN) == 0, "warp layout");
   constexpr int MT = BM / WM / 16, NT = BN / WN / 8;
   constexpr int A_FLOATS = SmallTile<BM, A_K>::FLOATS, B_FLOATS = SmallTile<BN, B_K>::FLOATS, STAGE = A_FLOATS + B_FLOATS;

@@ -199,6 +199,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(T2_THREADS, 1) tc2r_
   constexpr int R = Cfg::HI_SLOTS, L = Cfg::LO_SLOTS, LM = L > 0 ? L : 1;
   constexpr int BH = Cfg::BH;
   extern __shared__ uint8_t smem_raw[];
+  pdl_wait();
   uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   uint8_t *lo_ring = smem + R * Cfg::SLOT_BYTES;
   uint8_t *aux = lo_ring + L * Cfg::SLOT_BYTES;

@@ -27,6 +27,7 @@ struct Operands {
 
 template <typename Op, int NIN>
 __global__ void __launch_bounds__(256) apply_contig_kernel(Operands<NIN> p, long n, bool vec, Op op) {
+  pdl_begin();
   const long tid = (long)blockIdx.x * blockDim.x + threadIdx.x;
   const long nthreads = (long)gridDim.x * blockDim.x;
   long done = 0;
@@ -99,6 +100,7 @@ struct StridedArgs {
 
 template <typename Op, int NIN>
 __global__ void __launch_bounds__(256) apply_strided_kernel(Operands<NIN> p, StridedArgs s, long n, Op op) {
+  pdl_begin();
   const long nthreads = (long)gridDim.x * blockDim.x;
   for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += nthreads) {
     long rem = i, off[NIN + 1];
@@ -146,6 +148,7 @@ struct Strides2d {
 template <typename Op, int NIN, unsigned VIA>   // VIA: bit k = operand k is transposed
 __global__ void __launch_bounds__(512, 3) apply_tiled2d_kernel(Operands<NIN> p, int n0, int n1, const Strides2d st,
                                                                 TileWalk walk, Op op) {
+  pdl_begin();
   constexpr int T = 64, PITCH = T + 1, TY = 512 / T, NJ = T / TY;
   extern __shared__ float tile2d_smem[];   // one [T][PITCH] tile per staged operand
   const int tx = threadIdx.x % T, ty = threadIdx.x / T;
@@ -209,6 +212,7 @@ __global__ void __launch_bounds__(512, 3) apply_tiled2d_kernel(Operands<NIN> p, 
 template <typename Op, int NIN, unsigned VIA>
 __global__ void __launch_bounds__(256) apply_transpose4_kernel(Operands<NIN> p, int n0, int n1, const Strides2d st, TileWalk walk,
                                                                Op op) {
+  pdl_begin();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int o0 = (warp & 3) * 16 + (lane & 3) * 4, o1 = (warp >> 2) * 32 + (lane >> 2) * 4;
   const unsigned ntiles = walk.count();
@@ -266,7 +270,7 @@ void apply(THGPUTensor *out, const THGPUTensor *in0, const THGPUTensor *in1, Op 
     long work = vec ? (n + 3) / 4 : n;
     int blocks = (int)((work + 255) / 256);
     if (blocks > max_blocks) blocks = max_blocks;
-    apply_contig_kernel<Op, NIN><<<blocks, 256, 0, stream()>>>(p, n, vec, op);
+    pdl_launch(apply_contig_kernel<Op, NIN>, blocks, 256, 0, p, n, vec, op);
     check_launch(name);
     return;
   }
@@ -295,14 +299,14 @@ void apply(THGPUTensor *out, const THGPUTensor *in0, const THGPUTensor *in1, Op 
           for (int k = 0; k < NIN; k++)
             vec = vec && aligned16(p.in[k]) && ((via >> k & 1u) ? st.s[k + 1][1] % 4 == 0 : st.s[k + 1][1] == 1 && st.s[k + 1][0] % 4 == 0);
           if (vec) {
-            if (NIN == 1 || via == 1u) apply_transpose4_kernel<Op, NIN, 1u><<<blocks, 256, 0, stream()>>>(p, (int)n0, (int)n1, st, walk, op);
-            else if (via == 2u) apply_transpose4_kernel<Op, NIN, NIN == 2 ? 2u : 1u><<<blocks, 256, 0, stream()>>>(p, (int)n0, (int)n1, st, walk, op);
-            else apply_transpose4_kernel<Op, NIN, NIN == 2 ? 3u : 1u><<<blocks, 256, 0, stream()>>>(p, (int)n0, (int)n1, st, walk, op);
+            if (NIN == 1 || via == 1u) pdl_launch(apply_transpose4_kernel<Op, NIN, 1u>, blocks, 256, 0, p, (int)n0, (int)n1, st, walk, op);
+            else if (via == 2u) pdl_launch(apply_transpose4_kernel<Op, NIN, NIN == 2 ? 2u : 1u>, blocks, 256, 0, p, (int)n0, (int)n1, st, walk, op);
+            else pdl_launch(apply_transpose4_kernel<Op, NIN, NIN == 2 ? 3u : 1u>, blocks, 256, 0, p, (int)n0, (int)n1, st, walk, op);
           } else {
             const size_t smem = (via == 3u ? 2 : 1) * 64 * 65 * sizeof(float);
-            if (NIN == 1 || via == 1u) apply_tiled2d_kernel<Op, NIN, 1u><<<blocks, 512, smem, stream()>>>(p, (int)n0, (int)n1, st, walk, op);
-            else if (via == 2u) apply_tiled2d_kernel<Op, NIN, NIN == 2 ? 2u : 1u><<<blocks, 512, smem, stream()>>>(p, (int)n0, (int)n1, st, walk, op);
-            else apply_tiled2d_kernel<Op, NIN, NIN == 2 ? 3u : 1u><<<blocks, 512, smem, stream()>>>(p, (int)n0, (int)n1, st, walk, op);
+            if (NIN == 1 || via == 1u) pdl_launch(apply_tiled2d_kernel<Op, NIN, 1u>, blocks, 512, smem, p, (int)n0, (int)n1, st, walk, op);
+            else if (via == 2u) pdl_launch(apply_tiled2d_kernel<Op, NIN, NIN == 2 ? 2u : 1u>, blocks, 512, smem, p, (int)n0, (int)n1, st, walk, op);
+            else pdl_launch(apply_tiled2d_kernel<Op, NIN, NIN == 2 ? 3u : 1u>, blocks, 512, smem, p, (int)n0, (int)n1, st, walk, op);
           }
           check_launch(name);
           return;
@@ -318,7 +322,7 @@ void apply(THGPUTensor *out, const THGPUTensor *in0, const THGPUTensor *in1, Op 
   }
   int blocks = (int)((n + 255) / 256);
   if (blocks > max_blocks) blocks = max_blocks;
-  apply_strided_kernel<Op, NIN><<<blocks, 256, 0, stream()>>>(p, sa, n, op);
+  pdl_launch(apply_strided_kernel<Op, NIN>, blocks, 256, 0, p, sa, n, op);
   check_launch(name);
 }
 

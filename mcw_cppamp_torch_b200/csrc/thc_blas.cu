@@ -10,6 +10,7 @@ namespace thc {
 struct ScaleOp { float v; __device__ float operator()(const float *a) const { return a[0] * v; } };
 
 static __global__ void scale_matrix_kernel(float *c, long m, long n, long ldc, float beta) {
+  pdl_begin();
   const long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= m * n) return;
   const long j = t / m, i = t - j * m;
@@ -18,6 +19,7 @@ static __global__ void scale_matrix_kernel(float *c, long m, long n, long ldc, f
 
 // out[i + j * ldc] = bias[i]
 static __global__ void broadcast_rows_kernel(float *c, long m, long n, long ldc, const float *__restrict__ bias) {
+  pdl_begin();
   const long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= m * n) return;
   const long j = t / m, i = t - j * m;
@@ -26,6 +28,7 @@ static __global__ void broadcast_rows_kernel(float *c, long m, long n, long ldc,
 // Up to two matrices copied to pitches that TMA can address (blockIdx.y: which): lines of `run` floats.
 struct PackJob { const float *src; float *dst; long lines, run, src_ld, dst_ld; };
 static __global__ void __launch_bounds__(256) pack_matrix_kernel(const PackJob a, const PackJob b) {
+  pdl_begin();
   // a warp copies up to 1024 floats of a line, all its loads in flight before the first store
   const PackJob &j = blockIdx.y ? b : a;
   const int lane = threadIdx.x & 31;
@@ -100,7 +103,7 @@ static void gemm_raw(GemmSide x, GemmSide y, long k, float alpha, float beta, fl
       s.p = j.dst; s.ld = j.dst_ld;
     }
     const long pieces = std::max(jobs[0].lines * ((jobs[0].run + 1023) / 1024), jobs[1].lines * ((jobs[1].run + 1023) / 1024));
-    pack_matrix_kernel<<<dim3((unsigned)std::min<long>((pieces + 7) / 8, ctx().sm_count * 8l), 2), 256, 0, stream()>>>(jobs[0], jobs[1]);
+    pdl_launch(pack_matrix_kernel, dim3((unsigned)std::min<long>((pieces + 7) / 8, ctx().sm_count * 8l), 2), 256, 0, jobs[0], jobs[1]);
     check_launch("pack_matrix");
   }
   if (!x.along_k && y.along_k) gemm_raw_t<true, false>(x.p, x.ld, y.p, y.ld, x.rows, y.rows, k, epi);
@@ -162,14 +165,14 @@ void gemm(char transa, char transb, long m, long n, long k, float alpha, const f
   WsScope ws_scope;
   const int mode = ctx().math_mode;
   if (row_bias && (mode == 1 || k <= 0 || alpha == 0.f)) {   // engines without a bias input: D starts as the bias
-    broadcast_rows_kernel<<<ceil_div(m * n, 256), 256, 0, stream()>>>(c, m, n, ldc, row_bias);
+    pdl_launch(broadcast_rows_kernel, ceil_div(m * n, 256), 256, 0, c, m, n, ldc, row_bias);
     check_launch("broadcast_rows");
     row_bias = nullptr;
     beta = 1.f;
   }
   if (k <= 0 || alpha == 0.f) {
     if (beta == 1.f) return;
-    scale_matrix_kernel<<<ceil_div(m * n, 256), 256, 0, stream()>>>(c, m, n, ldc, beta);
+    pdl_launch(scale_matrix_kernel, ceil_div(m * n, 256), 256, 0, c, m, n, ldc, beta);
     check_launch("scale_matrix");
     return;
   }
@@ -188,6 +191,7 @@ void gemm(char transa, char transb, long m, long n, long k, float alpha, const f
 static __global__ void __launch_bounds__(1024) gemv_n_kernel(long m, long n, float alpha, const float *__restrict__ a, long lda,
                                                              const float *__restrict__ x, long incx, float beta, float *y,
                                                              long incy) {
+  pdl_begin();
   __shared__ float part[32][33];
   const long i = (long)blockIdx.x * 32 + threadIdx.x;
   float acc = 0.f;
@@ -204,6 +208,7 @@ static __global__ void __launch_bounds__(1024) gemv_n_kernel(long m, long n, flo
 }
 static __global__ void gemv_t_kernel(long m, long n, float alpha, const float *__restrict__ a, long lda,
                                      const float *__restrict__ x, long incx, float beta, float *y, long incy) {
+  pdl_begin();
   const long j = (long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (j >= n) return;
   const int lane = threadIdx.x & 31;
@@ -214,12 +219,14 @@ static __global__ void gemv_t_kernel(long m, long n, float alpha, const float *_
   if (lane == 0) y[j * incy] = (beta == 0.f ? 0.f : beta * y[j * incy]) + alpha * acc;
 }
 static __global__ void axpy_kernel(long n, float a, const float *__restrict__ x, long incx, float *y, long incy) {
+  pdl_begin();
   const long nthreads = (long)gridDim.x * blockDim.x;
   for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += nthreads)
     y[i * incy] = __fadd_rn(y[i * incy], __fmul_rn(a, x[i * incx]));
 }
 static __global__ void ger_kernel(long m, long n, float alpha, const float *__restrict__ x, long incx,
                                   const float *__restrict__ y, long incy, float *a, long lda) {
+  pdl_begin();
   const long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= m * n) return;
   const long j = t / m, i = t - j * m;
@@ -242,10 +249,10 @@ THC_API void THGPUBlas_gemv(char trans, long m, long n, float alpha, const float
   THC_BEGIN
   if (m <= 0 || n <= 0) return;
   if (trans == 't' || trans == 'T') {
-    gemv_t_kernel<<<ceil_div(n, 8), 256, 0, stream()>>>(m, n, alpha, a, lda, x, incx, beta, y, incy);
+    pdl_launch(gemv_t_kernel, ceil_div(n, 8), 256, 0, m, n, alpha, a, lda, x, incx, beta, y, incy);
     check_launch("gemv_t");
   } else {
-    gemv_n_kernel<<<ceil_div(m, 32), dim3(32, 32), 0, stream()>>>(m, n, alpha, a, lda, x, incx, beta, y, incy);
+    pdl_launch(gemv_n_kernel, ceil_div(m, 32), dim3(32, 32), 0, m, n, alpha, a, lda, x, incx, beta, y, incy);
     check_launch("gemv_n");
   }
   THC_END()
@@ -257,7 +264,7 @@ THC_API void THGPUBlas_axpy(long n, float a, const float *x, long incx, float *y
   int blocks = ceil_div(n, 256);
   const int cap = ctx().sm_count * 8;
   if (blocks > cap) blocks = cap;
-  axpy_kernel<<<blocks, 256, 0, stream()>>>(n, a, x, incx, y, incy);
+  pdl_launch(axpy_kernel, blocks, 256, 0, n, a, x, incx, y, incy);
   check_launch("axpy");
   THC_END()
 }
@@ -266,7 +273,7 @@ THC_API void THGPUBlas_ger(long m, long n, float alpha, const float *x, long inc
                            float *a, long lda) {
   THC_BEGIN
   if (m <= 0 || n <= 0) return;
-  ger_kernel<<<ceil_div(m * n, 256), 256, 0, stream()>>>(m, n, alpha, x, incx, y, incy, a, lda);
+  pdl_launch(ger_kernel, ceil_div(m * n, 256), 256, 0, m, n, alpha, x, incx, y, incy, a, lda);
   check_launch("ger");
   THC_END()
 }
@@ -276,6 +283,7 @@ THC_API void THGPUBlas_ger(long m, long n, float alpha, const float *x, long inc
 // what an engine CTA does: raises the stall flags and returns.  It faults nothing and waits no longer than
 // `limit` SM cycles (plus one polling interval of a few tens of microseconds).
 static __global__ void stall_probe_kernel(const mm::StallCtl ctl) {
+  pdl_begin();
   __shared__ uint64_t bar;
   __shared__ mm::WaitCtl w;
   if (threadIdx.x == 0) {
@@ -307,7 +315,7 @@ THC_API int THGPUStallProbe(long limit_cycles) {
   THC_CHECK(limit_cycles >= 1024 && limit_cycles <= (1l << 27), "probe limit must lie in [2^10, 2^27] SM cycles");
   mm::StallCtl ctl = stall_ctl();
   ctl.limit = limit_cycles;
-  stall_probe_kernel<<<1, 32, 0, stream()>>>(ctl);
+  pdl_launch(stall_probe_kernel, 1, 32, 0, ctl);
   check_launch("stall_probe");
   return 0;
   THC_END(1)

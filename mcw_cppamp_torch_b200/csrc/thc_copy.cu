@@ -70,6 +70,7 @@ template <> __device__ __forceinline__ float from_float<float>(float x) { return
 // Four consecutive elements per thread and step: the FP32 side moves 16 bytes per access.
 template <class T>
 __global__ void __launch_bounds__(256) widen_kernel(const T *__restrict__ src, float *__restrict__ dst, long n) {
+  pdl_begin();
   const long nthreads = (long)gridDim.x * blockDim.x;
   const long n4 = n / 4;
   const bool vec = (reinterpret_cast<uintptr_t>(dst) & 15) == 0;
@@ -82,6 +83,7 @@ __global__ void __launch_bounds__(256) widen_kernel(const T *__restrict__ src, f
 }
 template <class T>
 __global__ void __launch_bounds__(256) narrow_kernel(const float *__restrict__ src, T *__restrict__ dst, long n) {
+  pdl_begin();
   const long nthreads = (long)gridDim.x * blockDim.x;
   const long n4 = n / 4;
   const bool vec = (reinterpret_cast<uintptr_t>(src) & 15) == 0;
@@ -110,7 +112,7 @@ template <class T> void upload(float *dst, const T *hsrc, long n) {
   else {
   T *stage = (T *)ws_alloc(sizeof(T) * n);
   THC_CUDA(cudaMemcpyAsync(stage, hsrc, sizeof(T) * n, cudaMemcpyHostToDevice, stream()));
-  widen_kernel<T><<<convert_blocks(n), 256, 0, stream()>>>(stage, dst, n);
+  pdl_launch(widen_kernel<T>, convert_blocks(n), 256, 0, stage, dst, n);
   check_launch("widen");
   }
 }
@@ -122,7 +124,7 @@ template <class T> void download(T *hdst, const float *src, long n) {
   }
   else {
   T *stage = (T *)ws_alloc(sizeof(T) * n);
-  narrow_kernel<T><<<convert_blocks(n), 256, 0, stream()>>>(src, stage, n);
+  pdl_launch(narrow_kernel<T>, convert_blocks(n), 256, 0, src, stage, n);
   check_launch("narrow");
   THC_CUDA(cudaMemcpyAsync(hdst, stage, sizeof(T) * n, cudaMemcpyDeviceToHost, stream()));
   }
@@ -132,6 +134,7 @@ template <class T> void download(T *hdst, const float *src, long n) {
 // the host polls for, instead of a pageable device-to-host copy and a stream synchronisation.
 __global__ void __launch_bounds__(1024) deliver_kernel(const float *__restrict__ src, float *stage, int n, ScalarSlot *slot,
                                                        unsigned long long seq) {
+  pdl_begin();
   for (int i = threadIdx.x; i < n; i += blockDim.x) stage[i] = src[i];
   __threadfence_system();
   __syncthreads();
@@ -140,7 +143,7 @@ __global__ void __launch_bounds__(1024) deliver_kernel(const float *__restrict__
 void download_small(float *hdst, const float *src, long n) {
   Context &c = ctx();
   const unsigned long long seq = scalar_expect();
-  deliver_kernel<<<1, 1024, 0, stream()>>>(src, c.small_stage_dev, (int)n, c.scalar_slot_dev, seq);
+  pdl_launch(deliver_kernel, 1, 1024, 0, src, c.small_stage_dev, (int)n, c.scalar_slot_dev, seq);
   check_launch("deliver");
   scalar_wait(seq);
   std::memcpy(hdst, c.small_stage, sizeof(float) * n);

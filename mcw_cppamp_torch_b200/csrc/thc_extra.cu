@@ -18,6 +18,7 @@ namespace {
 // ---- products ------------------------------------------------------------------------------------
 constexpr int kProdBlocks = 512;
 __global__ void __launch_bounds__(256) prod_partial_kernel(const float *__restrict__ x, long n, double *__restrict__ partial) {
+  pdl_begin();
   __shared__ double sm[8];
   double acc = 1.0;
   for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) acc *= (double)x[i];
@@ -31,6 +32,7 @@ __global__ void __launch_bounds__(256) prod_partial_kernel(const float *__restri
   }
 }
 __global__ void prod_finish_kernel(const double *__restrict__ partial, int n, ScalarSlot *slot, unsigned long long seq) {
+  pdl_begin();
   double acc = 1.0;
   for (int i = 0; i < n; i++) acc *= partial[i];
   scalar_deliver(slot, acc, seq);
@@ -39,6 +41,7 @@ __global__ void prod_finish_kernel(const double *__restrict__ partial, int n, Sc
 // neighbouring threads read neighbouring addresses.
 __global__ void __launch_bounds__(256) prod_dim_kernel(const float *__restrict__ src, long outer, long R, long inner,
                                                        float *__restrict__ out) {
+  pdl_begin();
   const long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= outer * inner) return;
   const long o = t / inner, i = t - o * inner;
@@ -49,6 +52,7 @@ __global__ void __launch_bounds__(256) prod_dim_kernel(const float *__restrict__
 }
 // inner == 1: one warp per row, lanes stride the row, partial products folded in lane order.
 __global__ void __launch_bounds__(256) prod_rows_kernel(const float *__restrict__ src, long rows, long R, float *__restrict__ out) {
+  pdl_begin();
   const long row = (long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (row >= rows) return;
   const int lane = threadIdx.x & 31;
@@ -62,6 +66,7 @@ __global__ void __launch_bounds__(256) prod_rows_kernel(const float *__restrict_
 
 // ---- renorm: one block per row of a contiguous [rows][size] matrix, in place -----------------------
 __global__ void __launch_bounds__(256) renorm_rows_kernel(float *__restrict__ data, long size, float value, float maxnorm) {
+  pdl_begin();
   __shared__ double sm[8];
   __shared__ float factor;
   float *row = data + (long)blockIdx.x * size;
@@ -92,6 +97,7 @@ template <int MODE>
 __global__ void __launch_bounds__(256) index_kernel(float *__restrict__ dst, const float *__restrict__ src,
                                                     const long *__restrict__ idx, long outer, long D, long nidx, long inner,
                                                     float val) {
+  pdl_begin();
   const long total = outer * nidx * inner;
   for (long t = (long)blockIdx.x * blockDim.x + threadIdx.x; t < total; t += (long)gridDim.x * blockDim.x) {
     const long i = t % inner, q = t / inner, k = q % nidx, o = q / nidx;
@@ -179,10 +185,10 @@ THC_API float THGPUTensor_prodall(THGPUTensor *self) {
   double *partial = (double *)ws_alloc(sizeof(double) * kProdBlocks);
   int blocks = (int)((n + 255) / 256);
   if (blocks > kProdBlocks) blocks = kProdBlocks;
-  prod_partial_kernel<<<blocks, 256, 0, stream()>>>(data_ptr(c), n, partial);
+  pdl_launch(prod_partial_kernel, blocks, 256, 0, data_ptr(c), n, partial);
   check_launch("prod_partial");
   const unsigned long long seq = scalar_expect();
-  prod_finish_kernel<<<1, 1, 0, stream()>>>(partial, blocks, ctx().scalar_slot_dev, seq);
+  pdl_launch(prod_finish_kernel, 1, 1, 0, partial, blocks, ctx().scalar_slot_dev, seq);
   check_launch("prod_finish");
   return (float)scalar_wait(seq);
   THC_END(0.f)
@@ -201,10 +207,10 @@ THC_API void THGPUTensor_prod(THGPUTensor *self, THGPUTensor *src, long dimensio
   TensorRef out(tensor_new_sized(nd, osize));   // src may alias self: compute aside, then hand over
   if (b.outer * b.inner > 0) {
     if (b.inner == 1) {
-      prod_rows_kernel<<<(unsigned)((b.outer + 7) / 8), 256, 0, stream()>>>(data_ptr(c), b.outer, b.D, data_ptr(out));
+      pdl_launch(prod_rows_kernel, (unsigned)((b.outer + 7) / 8), 256, 0, data_ptr(c), b.outer, b.D, data_ptr(out));
       check_launch("prod_rows");
     } else {
-      prod_dim_kernel<<<(unsigned)((b.outer * b.inner + 255) / 256), 256, 0, stream()>>>(data_ptr(c), b.outer, b.D, b.inner,
+      pdl_launch(prod_dim_kernel, (unsigned)((b.outer * b.inner + 255) / 256), 256, 0, data_ptr(c), b.outer, b.D, b.inner,
                                                                                          data_ptr(out));
       check_launch("prod_dim");
     }
@@ -226,7 +232,7 @@ THC_API void THGPUTensor_renorm(THGPUTensor *self, THGPUTensor *src, float value
   tensor_copy(data, srct);
   const long rows = data->size[0], size = rows ? nelem(data) / rows : 0;
   if (rows > 0 && size > 0) {
-    renorm_rows_kernel<<<(unsigned)rows, 256, 0, stream()>>>(data_ptr(data), size, value, maxnorm);
+    pdl_launch(renorm_rows_kernel, (unsigned)rows, 256, 0, data_ptr(data), size, value, maxnorm);
     check_launch("renorm_rows");
   }
   TensorRef back(THGPUTensor_newTranspose(data, (int)dimension, 0));
@@ -253,7 +259,7 @@ THC_API void THGPUTensor_indexSelect(THGPUTensor *res_, THGPUTensor *src, int di
   TensorRef out(tensor_new_sized(nd, osize));
   const long total = b.outer * nidx * b.inner;
   if (total > 0) {
-    index_kernel<0><<<grid_for(total), 256, 0, stream()>>>(data_ptr(out), data_ptr(c), idx, b.outer, b.D, nidx, b.inner, 0.f);
+    pdl_launch(index_kernel<0>, grid_for(total), 256, 0, data_ptr(out), data_ptr(c), idx, b.outer, b.D, nidx, b.inner, 0.f);
     check_launch("indexSelect");
   }
   resize_nd(res_, nd, osize, nullptr);
@@ -277,7 +283,7 @@ THC_API void THGPUTensor_indexCopy(THGPUTensor *res_, int dim, THLongTensor *ind
   const Block3 b = split_at(rc, dim);
   const long total = b.outer * nidx * b.inner;
   if (total > 0) {
-    index_kernel<1><<<grid_for(total), 256, 0, stream()>>>(data_ptr(rc), data_ptr(c), idx, b.outer, b.D, nidx, b.inner, 0.f);
+    pdl_launch(index_kernel<1>, grid_for(total), 256, 0, data_ptr(rc), data_ptr(c), idx, b.outer, b.D, nidx, b.inner, 0.f);
     check_launch("indexCopy");
   }
   if (rc.t != res_) tensor_copy(res_, rc);
@@ -295,7 +301,7 @@ THC_API void THGPUTensor_indexFill(THGPUTensor *res_, int dim, THLongTensor *ind
   const Block3 b = split_at(rc, dim);
   const long total = b.outer * nidx * b.inner;
   if (total > 0) {
-    index_kernel<2><<<grid_for(total), 256, 0, stream()>>>(data_ptr(rc), nullptr, idx, b.outer, b.D, nidx, b.inner, val);
+    pdl_launch(index_kernel<2>, grid_for(total), 256, 0, data_ptr(rc), nullptr, idx, b.outer, b.D, nidx, b.inner, val);
     check_launch("indexFill");
   }
   if (rc.t != res_) tensor_copy(res_, rc);

@@ -189,6 +189,31 @@ void sgd_update_async(float *w, const float *g, float *v, long n, float lr, floa
 void gemm(char transa, char transb, long m, long n, long k, float alpha, const float *a, long lda,
           const float *b, long ldb, float beta, float *c, long ldc, const float *row_bias = nullptr);   // bias[i] added to row i (beta 0)
 
+#ifdef __CUDACC__
+// Kernels of a stream follow one another as programmatic dependents: a kernel's blocks may take their places, and set up what is
+// theirs alone, while the previous kernel drains, and wait in pdl_wait() for its results.  Every kernel launched this way
+// executes the wait, which is what keeps the order transitive.  Worth about 1.5 us a launch (a step of 100 launches at 128
+// images: 4.10 -> 3.95 ms).
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_begin() { pdl_wait(); pdl_trigger(); }
+// `early` false: the ordinary order, the whole device free before the first block starts.
+template <class... P, class... A>
+void launch_on_stream(bool early, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, A &&...args) {
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = stream();
+  cfg.attrs = &attr; cfg.numAttrs = early ? 1 : 0;
+  cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);   // check_launch() picks an error up
+}
+template <class... P, class... A>
+void pdl_launch(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, A &&...args) {
+  launch_on_stream(true, kernel, grid, block, smem, args...);
+}
+#endif
+
 }  // namespace thc
 
 #endif

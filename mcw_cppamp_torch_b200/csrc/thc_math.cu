@@ -63,6 +63,7 @@ template <int MODE>
 __global__ void __launch_bounds__(256) reduce_rows_kernel(const float *__restrict__ src, long so, long R,
                                                           float *__restrict__ out, float *__restrict__ idx,
                                                           float scale, bool vec) {
+  pdl_begin();
   __shared__ double sd[32];
   __shared__ float sv[32];
   __shared__ long si[32];
@@ -157,6 +158,7 @@ __global__ void __launch_bounds__(256) reduce_rows_kernel(const float *__restric
 template <int MODE>
 __global__ void __launch_bounds__(256) reduce_rows_warp_kernel(const float *__restrict__ src, long so, long J, int R,
                                                                float *__restrict__ out, float *__restrict__ idx, float scale) {
+  pdl_begin();
   const long j = (long)blockIdx.x * 8 + (threadIdx.x >> 5);
   if (j >= J) return;
   const int lane = threadIdx.x & 31;
@@ -279,6 +281,7 @@ __device__ __forceinline__ void cols_fold_if_last(const ColOut &w, long J, long 
 template <int MODE>
 __global__ void __launch_bounds__(256) reduce_cols_kernel(const float *__restrict__ src, long so, long sr, long J, int R,
                                                           int rows_per_split, const ColOut w) {
+  pdl_begin();
   __shared__ double sd[8][33];
   __shared__ float sv[8][33];
   __shared__ int si[8][33];
@@ -337,6 +340,7 @@ __global__ void __launch_bounds__(256) reduce_cols_kernel(const float *__restric
 template <int MODE>
 __global__ void __launch_bounds__(256) reduce_cols4_kernel(const float *__restrict__ src, long so, long sr, long J, int R,
                                                            int rows_per_split, const ColOut w) {
+  pdl_begin();
   __shared__ double sd[8][129];
   __shared__ float sv[8][129];
   __shared__ int si[8][129];
@@ -473,10 +477,10 @@ static void reduce_dim(THGPUTensor *values, THGPUTensor *indices, THGPUTensor *s
     THC_CHECK(O == 1, "internal: row reduce with outer dim");
     const bool vec = aligned16(base) && (sj % 4 == 0);
     if (R < 512) {
-      reduce_rows_warp_kernel<MODE><<<(unsigned)((J + 7) / 8), 256, 0, stream()>>>(base, sj, J, (int)R, out, idx, scale);
+      pdl_launch(reduce_rows_warp_kernel<MODE>, (unsigned)((J + 7) / 8), 256, 0, base, sj, J, (int)R, out, idx, scale);
     } else {
       const int threads = R >= 4096 ? 256 : 128;
-      reduce_rows_kernel<MODE><<<(unsigned)J, threads, 0, stream()>>>(base, sj, R, out, idx, scale, vec);
+      pdl_launch(reduce_rows_kernel<MODE>, (unsigned)J, threads, 0, base, sj, R, out, idx, scale, vec);
     }
     check_launch("reduce_rows");
   } else {
@@ -501,8 +505,8 @@ static void reduce_dim(THGPUTensor *values, THGPUTensor *indices, THGPUTensor *s
     }
     w.out = out; w.idx = idx; w.scale = scale;
     dim3 grid((unsigned)colblocks, (unsigned)splits, (unsigned)O), block(32, 8);
-    if (vec4) reduce_cols4_kernel<MODE><<<grid, block, 0, stream()>>>(base, so, sr, J, (int)R, (int)rows_per_split, w);
-    else reduce_cols_kernel<MODE><<<grid, block, 0, stream()>>>(base, so, sr, J, (int)R, (int)rows_per_split, w);
+    if (vec4) pdl_launch(reduce_cols4_kernel<MODE>, grid, block, 0, base, so, sr, J, (int)R, (int)rows_per_split, w);
+    else pdl_launch(reduce_cols_kernel<MODE>, grid, block, 0, base, so, sr, J, (int)R, (int)rows_per_split, w);
     check_launch("reduce_cols");
   }
   if (vtmp.t) { resize_nd(values, ond, osize, nullptr); tensor_copy(values, vtmp); }

@@ -71,6 +71,7 @@ __device__ __forceinline__ double block_reduce(double v, double *smem) {
 template <int MODE, class Term>
 __global__ void __launch_bounds__(512) reduce_all_kernel(const float *__restrict__ x, const float *__restrict__ y, long n, bool vec,
                                                          RedScratch *s, Term term, ScalarSlot *slot, unsigned long long seq) {
+  pdl_begin();
   constexpr bool DOT = MODE == RED_DOT;
   constexpr int BASE = DOT ? RED_SUM : MODE;
   constexpr int NIN = DOT ? 2 : Term::NIN;
@@ -146,7 +147,7 @@ double reduce_flat(const float *x, const float *y, long n, Term term) {
   // one block up to eight loads per thread: below that the ticket's round trips cost more than a second block gains
   int blocks = work <= 8 * 512 ? 1 : (int)std::min<long>((work + 511) / 512, std::min(1024, c.sm_count * 4));   // 4 x 512 threads fill an SM
   const unsigned long long seq = scalar_expect();
-  reduce_all_kernel<MODE, Term><<<blocks, 512, 0, stream()>>>(x, y, n, vec, s, term, c.scalar_slot_dev, seq);
+  pdl_launch(reduce_all_kernel<MODE, Term>, blocks, 512, 0, x, y, n, vec, s, term, c.scalar_slot_dev, seq);
   check_launch("reduce_all");
   return scalar_wait(seq);
 }

@@ -270,13 +270,14 @@ THC_API void THGPUStorage_set(THGPUStorage *self, long index, float value) {
 // One element to the host: a kernel that writes it into the mapped scalar record (a third of the time of a 4-byte
 // device-to-host copy followed by a stream synchronisation).  A float survives the trip through the record's double.
 static __global__ void fetch_scalar_kernel(const float *src, ScalarSlot *slot, unsigned long long seq) {
+  pdl_begin();
   scalar_deliver(slot, (double)*src, seq);
 }
 THC_API float THGPUStorage_get(const THGPUStorage *self, long index) {
   THC_BEGIN
   THC_ARG(index >= 0 && index < self->size, 2, "index out of bounds");
   const unsigned long long seq = scalar_expect();
-  fetch_scalar_kernel<<<1, 1, 0, stream()>>>(self->data + index, ctx().scalar_slot_dev, seq);
+  pdl_launch(fetch_scalar_kernel, 1, 1, 0, self->data + index, ctx().scalar_slot_dev, seq);
   check_launch("fetch_scalar");
   return (float)scalar_wait(seq);
   THC_END(0.f)
