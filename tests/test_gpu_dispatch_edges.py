@@ -80,3 +80,24 @@ def test_download_sizes(gt, n):
     x = np.random.default_rng(n).standard_normal(n).astype(np.float32)
     out = np.zeros(n, np.float32)
     assert gt.gpu(x).float(out) is out and np.array_equal(out, x)
+
+
+@pytest.mark.parametrize("n", [(1 << 21) - 1, 1 << 21, (1 << 21) + 1, 17 << 17, 2500007])
+def test_large_uploads_from_several_threads(gt, n):
+    """Staged uploads around their smallest size and piece boundaries; a second thread that finds the stager busy."""
+    import threading
+    x = np.random.default_rng(n).standard_normal(n).astype(np.float32)
+    bad = []
+
+    def work(k):
+        y = x + np.float32(k)
+        for _ in range(4):
+            if not np.array_equal(gt.gpu(y).float(), y):
+                bad.append(k)
+    ts = [threading.Thread(target=work, args=(k,)) for k in range(3)]
+    for t in ts:
+        t.start()
+    for t in ts:
+        t.join()
+    assert not bad
+    assert np.array_equal(gt.gpu(np.arange(n)).float(), np.arange(n).astype(np.float32))      # another element type
