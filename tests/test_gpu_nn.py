@@ -418,12 +418,27 @@ def test_alexnet_step_matches_cpu(gt, oracle_port):
     cpu = "reference" if oracle.ref.available() else "port"
     _, loss_cpu, d = bench.cpu_alexnet_step(cpu, 8, details=True)
     assert len(d["params"]) == 8
-    loss, layers = _device_step(gt, configs.alexnet(rng=oracle_port.rng(1)), d["params"], d["x"], d["labels"])
+    net = configs.alexnet(rng=oracle_port.rng(1))
+    loss, layers = _device_step(gt, net, d["params"], d["x"], d["labels"])
     assert abs(loss - loss_cpu) <= 1e-5 + 1e-4 * abs(loss_cpu)
     for i, (m, (gw, gb)) in enumerate(zip(layers, d["grads"])):
         got = m.gradWeight.float()
-        close_scaled(got, gw.reshape(got.shape), "alexnet 8 images vs %s: layer %d gradWeight" % (cpu, i + 1))
-        close_scaled(m.gradBias.float(), gb, "alexnet 8 images vs %s: layer %d gradBias" % (cpu, i + 1))
+        gw, gb, got_b = gw.reshape(got.shape), gb.copy(), m.gradBias.float()
+        if cpu == "port" and i == 3:
+            # The plain-C path rounds its sums otherwise than the device, and one pre-activation of this layer lies
+            # within that rounding of zero: image 7, plane 70, (4, 3) is -1.3e-8 exactly, -5.7e-8 on the CPU and +1.4e-7
+            # on the device, so one side passes the ReLU's gradient g there and the other does not.  That adds
+            # g * (the unit's window of the input) to row 70 of gradWeight and g to its gradBias; every other row keeps
+            # the bound, and row 70 gets |g| max|window| (|g|) beside it.
+            at = net.modules.index(m)
+            g = abs(float(net.modules[at + 2].gradInput.float()[7, 70, 4, 3]))
+            window = float(np.abs(net.modules[at - 1].output.float()[7, :, 3:6, 2:5]).max())
+            close_scaled(got[70], gw[70], "alexnet 8 images vs port: layer 4 gradWeight, plane 70", atol=1e-5 + g * window)
+            close_scaled(got_b[70:71], gb[70:71], "alexnet 8 images vs port: layer 4 gradBias, plane 70", atol=1e-5 + g)
+            got, gw = np.delete(got, 70, 0), np.delete(gw, 70, 0)
+            got_b, gb = np.delete(got_b, 70), np.delete(gb, 70)
+        close_scaled(got, gw, "alexnet 8 images vs %s: layer %d gradWeight" % (cpu, i + 1))
+        close_scaled(got_b, gb, "alexnet 8 images vs %s: layer %d gradBias" % (cpu, i + 1))
 
 
 def test_vgg_a_step_matches_cpu(gt, oracle_port):
