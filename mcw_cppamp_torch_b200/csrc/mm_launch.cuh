@@ -347,12 +347,29 @@ inline double small_product_us(long m, long n, long k, bool aligned) {
   const double waves = std::max(1.0, blocks / depth);
   return 5 + (aligned ? 1.0 : 1.3) * step * waves * (double)((ktiles + slices - 1) / slices) + (slices > 1 ? 0.25 * (double)slices : 0);
 }
+// few_rows_kernel, for both operands along k in whole 16-byte pieces: up to 4 rows on the short side, and up to 8 while the
+// matrix stays in L2 many times over (a 4096 x 1000 one: 12.8 -> 9 us); beyond, the reads of the rows outweigh those
+// of the matrix and the MMA tiles win (8 rows against 4096 x 9216: 43 us, here 53).
+static bool launch_few_rows(const SmallProblem &p, bool a_k, bool b_k) {
+  if (!(a_k && b_k && p.a.vec4 && p.b.vec4 && p.K % 4 == 0 && p.K <= 1 << 30 && p.N <= 8 && (p.N <= 4 || (long)p.M * p.K <= 1l << 23))) return false;
+  const int ra = p.N == 1 || (p.N > 2 && p.N <= 4) ? 4 : 8;
+  int groups = 8;   // sets of rows per block: as many as leave two blocks per SM, since they share the few rows
+  while (groups > 1 && ceil_div(p.M, ra * groups) < 2 * ctx().sm_count) groups /= 2;
+  const unsigned blocks = (unsigned)ceil_div(p.M, ra * groups);
+  if (p.N == 1) pdl_launch(few_rows_kernel<1, 4, 2>, blocks, 256, 0, p, groups);
+  else if (p.N == 2) pdl_launch(few_rows_kernel<2, 8, 2>, blocks, 256, 0, p, groups);
+  else if (p.N <= 4) pdl_launch(few_rows_kernel<4, 4, 3>, blocks, 256, 0, p, groups);
+  else pdl_launch(few_rows_kernel<8, 8, 1>, blocks, 256, 0, p, groups);
+  check_launch("few_rows");
+  return true;
+}
 // D = alpha * A * B^T + beta * D (+ bias) for A [M][K] and B [N][K]; a_k / b_k: the operand's memory runs along k.
 static void launch_small(SmallProblem p, bool a_k, bool b_k) {
   if (p.N > p.M) {   // the longer side takes the 64-row tiles
     std::swap(p.a, p.b); std::swap(a_k, b_k); std::swap(p.M, p.N); std::swap(p.sm, p.sn); std::swap(p.bias_m, p.bias_n);
   }
   p.stalled = stall_ctl().dev_flag;
+  if (launch_few_rows(p, a_k, b_k)) return;
   const int bn = small_tile_width(p.N);
   const long tiles = (long)ceil_div(p.M, 64) * ceil_div(p.N, bn), ktiles = ceil_div(p.K, TC_BK), slices = small_slices(tiles, ktiles, bn);
   p.tiles_per_slice = ceil_div(ktiles, slices);

@@ -68,3 +68,21 @@ def test_nan_and_infinity_reach_the_result(gt):
     A[2, 1:2].view(np.uint32)[:] = 0x7fffffff           # the NaN that device arithmetic makes
     r = gt.GPUTensor(70, 20).zero().addmm(0.0, 1.0, gt.gpu(A), gt.gpu(np.ones((40, 20), np.float32))).float()
     assert np.isnan(r[2:4]).all() and not np.isfinite(r[4]).any() and np.all(r[5] == 40)
+
+
+@pytest.mark.parametrize("rows", [1, 2, 3, 4, 5, 8, 9])
+@pytest.mark.parametrize("inputs,outputs", [(4, 9), (124, 33), (516, 4099), (9216, 260), (4096, 2049)])
+def test_few_rows(gt, rows, inputs, outputs):
+    """Few rows against a K-major matrix: remainders of rows, outputs and k chunks, both sides of the size rule."""
+    g = np.random.default_rng(rows * 31 + inputs)
+    x, w, b = (g.standard_normal(s).astype(np.float32) for s in ((rows, inputs), (outputs, inputs), (outputs,)))
+    m = gt.nn.Linear(inputs, outputs)
+    m.weight, m.bias = w, b
+    got = m.gpu().forward(gt.gpu(x)).float()
+    exact = x.astype(np.float64) @ w.T.astype(np.float64) + b
+    tol = bound(x, w.T, inputs) + 2.0 ** -22 * (np.abs(exact) + np.abs(b))
+    assert np.all(np.abs(got - exact) <= tol)
+    c = g.standard_normal((rows, outputs)).astype(np.float32)
+    r = gt.gpu(c).addmm(0.5, 0.75, gt.gpu(x), gt.gpu(w).t()).float()
+    exact = 0.5 * c.astype(np.float64) + 0.75 * (x.astype(np.float64) @ w.T.astype(np.float64))
+    assert np.all(np.abs(r - exact) <= bound(x, w.T, inputs) + 2.0 ** -22 * (np.abs(exact) + np.abs(c)))
