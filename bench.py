@@ -348,8 +348,8 @@ def tensor_math_report(gt, nn, torch, ts, hbm_gbs):
     bw("tanh", 8 * ne, lambda: R.tanh(X))
     bw("clamp", 8 * ne, lambda: R.clamp(X, -0.5, 0.5))
     bw("ltTensor", 12 * ne, lambda: R.lt(X, Y))
-    bw("addcmul", 24 * ne, lambda: R.addcmul(X, 0.5, X, Y))    # product pass (12 B) + sum pass (12 B)
-    bw("normall_2", 12 * ne, lambda: X.norm(2.0))             # squares pass (8 B) + sum (4 B)
+    bw("addcmul", 12 * ne, lambda: R.addcmul(X, 0.5, X, Y))    # one pass: X and Y in, R out
+    bw("normall_2", 4 * ne, lambda: X.norm(2.0))              # one pass
     bw("sumall", 4 * ne, lambda: X.sum())
     bw("maxall", 4 * ne, lambda: X.max())
     bw("sumall_transposed", 4 * ne, lambda: X.t().sum())

@@ -98,15 +98,17 @@ static EncodeIm2colFn encode_im2col_fn() {
 }
 // Slices for the `tail` tiles a persistent launch has left after its whole rounds over `slots` clusters.  A model in
 // microseconds: a k tile step of a lone item takes `tile_us` (1.2; BF16 0.5); a partial-sum block (256 x BN2 floats) costs
-// about 0.17 us of device-wide write + read-back; the folding kernel about 5 us to launch.  Every slice keeps at
-// least six k tiles (the pipeline fill of an item is two to three).
+// about 0.06 us of device-wide write + read-back, which the L2 holds; the folding kernel, queued as a programmatic
+// dependent, 2 us.  Every slice keeps at least three k tiles, the pipeline fill of an item.  (With six tiles, 0.17 and 5 us,
+// which fitted launches in ordinary order, products of few tiles left most clusters idle: the small convolution blocks
+// 208 -> 202 and 91.7 -> 86.0 us, the VGG-A-style classifier over 13 images 1955 -> 1924.)
 static int choose_tail_splits(long tail, long ktiles, int slots, double tile_us) {
   int best = 1;
   double best_us = tile_us * (double)ktiles;
-  const long max_s = std::min<long>(ktiles / 6, 4l * slots);
+  const long max_s = std::min<long>(ktiles / 3, 4l * slots);
   for (long s = 2; s <= max_s; s++) {
     const long rounds = (tail * s + slots - 1) / slots, per = (ktiles + s - 1) / s;
-    const double us = tile_us * (double)(rounds * per) + 0.17 * (double)(tail * s) + 5.0;
+    const double us = tile_us * (double)(rounds * per) + 0.06 * (double)(tail * s) + 2.0;
     if (us < best_us * 0.9) { best = (int)s; best_us = us; }
   }
   return best;

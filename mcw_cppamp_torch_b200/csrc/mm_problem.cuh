@@ -338,7 +338,7 @@ static __global__ void __launch_bounds__(256) cells_input_kernel(const float *__
   const int q = u.Cs / V, chunks = u.Ws * q, y0 = Y * u.dH - u.pad;
   const float *img = in + n * u.C * (long)u.H * u.W;
   uint4 *dst = reinterpret_cast<uint4 *>(S) + ((n * u.Hs + Y) * u.Ws) * (long)q;
-  for (int o = threadIdx.x; o < chunks; o += blockDim.x) {
+  for (int o = blockIdx.y * blockDim.x + threadIdx.x; o < chunks; o += gridDim.y * blockDim.x) {
     const int X = o / q, ch0 = (o - X * q) * V, x0 = X * u.dW - u.pad;
     const float *base = img + (long)y0 * u.W + x0;
     float v[V];

@@ -249,9 +249,8 @@ __global__ void __launch_bounds__(1024) deliver_kernel(const float *__restrict__
                                                        unsigned long long seq) {
   pdl_begin();
   for (int i = threadIdx.x; i < n; i += blockDim.x) stage[i] = src[i];
-  __threadfence_system();
   __syncthreads();
-  if (threadIdx.x == 0) scalar_deliver(slot, 0.0, seq);
+  if (threadIdx.x == 0) scalar_deliver(slot, 0.0, seq);   // its system fence comes after every thread's values, through the barrier
 }
 void download_small(float *hdst, const float *src, long n) {
   Context &c = ctx();
