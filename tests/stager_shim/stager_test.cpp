@@ -1,0 +1,34 @@
+// Staged uploads over the stand-in runtime: one scenario per argument, exit code 0 when the bytes arrived.
+#include <cstdio>
+#include <cstring>
+#include <string>
+#include <vector>
+
+#include "thc_stager.h"
+
+using thc::Stager;
+
+struct Upload {
+  std::vector<char> src, dst;
+  FakeStream *stream = new FakeStream;   // outlives the upload, as the stager's events may
+  bool taken = false;
+  cudaError_t err = cudaSuccess;
+  Upload(long bytes, int seed) : src(bytes), dst(bytes, 0) { for (long i = 0; i < bytes; i++) src[i] = (char)(i * 31 + i / 4096 + seed * 7 + 1); }
+  void run(int device) { taken = Stager::get().upload(dst.data(), src.data(), (long)src.size(), device, stream, err); }
+  bool arrived() { cudaStreamSynchronize(stream); return taken && err == cudaSuccess && std::memcmp(src.data(), dst.data(), src.size()) == 0; }
+};
+
+int main(int, char **argv) {
+  const std::string what = argv[1];
+  const long n = 17 * thc::kPiece + 12345;
+  if (what == "devices") {   // the last pieces for device 0 are still in flight when an upload to device 1 begins
+    for (int round = 0; round < 8; round++) {
+      Upload a(n, 2 * round), b(n, 2 * round + 1);
+      a.run(0);
+      b.run(1);
+      if (!a.arrived() || !b.arrived()) { std::printf("round %d: device 0 %d, device 1 %d\n", round, a.arrived(), b.arrived()); return 1; }
+    }
+    return 0;
+  }
+  return 2;
+}
