@@ -59,6 +59,7 @@ class Stager {
       threads_ = true;
     }
     if (device == device_) return true;
+    device_ = -1;   // until every slot has its event: a failure half-way leaves no device whose events are gone
     for (Slot &s : slots_)
       for (int k = 0; k < 2; k++) {
         // upload() returns with its last pieces still on their way: the pinned slot is this device's once they have left

@@ -30,5 +30,21 @@ int main(int, char **argv) {
     }
     return 0;
   }
+  if (what == "event") {   // an event of the new device cannot be made: the driver's way this time, and no trace of it later
+    for (int fail = 1; fail <= 4; fail++) {
+      Upload a(n, 1), b(n, 2), c(n, 3), d(n, 4);
+      a.run(0);
+      fake_fail_event_create() = fail;
+      b.run(1);
+      fake_fail_event_create() = 0;
+      c.run(0);
+      d.run(1);
+      if (!a.arrived() || b.taken || !c.arrived() || !d.arrived()) {
+        std::printf("creation %d: %d %d %d (error %d) %d\n", fail, a.arrived(), b.taken, c.arrived(), (int)c.err, d.arrived());
+        return 1;
+      }
+    }
+    return 0;
+  }
   return 2;
 }

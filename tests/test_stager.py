@@ -24,3 +24,7 @@ def run(driver, what):
 
 def test_an_upload_to_another_device_waits_for_the_pieces_in_flight(driver):
     run(driver, "devices")
+
+
+def test_a_device_whose_events_cannot_be_made_leaves_the_others_usable(driver):
+    run(driver, "event")
