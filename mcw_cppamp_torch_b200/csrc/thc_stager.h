@@ -16,6 +16,7 @@
 #include <condition_variable>
 #include <cstring>
 #include <mutex>
+#include <system_error>
 #include <thread>
 
 namespace thc {
@@ -54,9 +55,10 @@ class Stager {
   struct Slot { char *p[2] = {}; cudaEvent_t free[2] = {}; };
   // threads once, slots and events for the device last used
   bool ready(int device) {
-    if (!threads_) {
-      for (int i = 1; i < kStagers; i++) std::thread([this, i] { loop(i); }).detach();
-      threads_ = true;
+    try {
+      for (; threads_ < kStagers - 1; threads_++) std::thread([this, i = threads_ + 1] { loop(i); }).detach();
+    } catch (const std::system_error &) {
+      return false;   // the process may not have another thread now; the next upload asks again
     }
     if (device == device_) return true;
     device_ = -1;   // until every slot has its event: a failure half-way leaves no device whose events are gone
@@ -104,7 +106,7 @@ class Stager {
   }
   std::mutex busy_, m_;
   std::condition_variable cv_, done_;
-  bool threads_ = false;
+  int threads_ = 0;   // helpers started
   int device_ = -1, wanted_ = 0, working_ = 0;
   long job_ = 0, bytes_ = 0;
   char *dst_ = nullptr;

@@ -28,3 +28,7 @@ def test_an_upload_to_another_device_waits_for_the_pieces_in_flight(driver):
 
 def test_a_device_whose_events_cannot_be_made_leaves_the_others_usable(driver):
     run(driver, "event")
+
+
+def test_without_a_second_thread_uploads_take_the_drivers_way(driver):
+    run(driver, "thread")
