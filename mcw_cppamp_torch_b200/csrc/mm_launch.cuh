@@ -11,6 +11,7 @@
 #include "mm_simt.cuh"
 #include "mm_small.cuh"
 #include "mm_tc2r.cuh"
+#include "per_device.h"
 
 namespace thc {
 namespace mm {
@@ -219,28 +220,27 @@ static double tc2_product_us(long M, long N, long K, bool half, bool half_mn = f
 template <class P, int BN2>
 static int tc2r_resident_clusters() {
   typedef Tc2rCfg<BN2, P::HALF> Cfg;
-  static int n = 0;
-  if (n) return n;
-  THC_CUDA(cudaFuncSetAttribute(tc2r_kernel<P, BN2>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM_BYTES));
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(2 * ctx().sm_count, 1, 1);
-  cfg.blockDim = dim3(T2_THREADS, 1, 1);
-  cfg.dynamicSmemBytes = Cfg::SMEM_BYTES;
-  int c = 0;
-  if (cudaOccupancyMaxActiveClusters(&c, tc2r_kernel<P, BN2>, &cfg) != cudaSuccess || c < 1) {
-    cudaGetLastError();
-    cudaLaunchAttribute attr;
-    attr.id = cudaLaunchAttributeClusterDimension;
-    attr.val.clusterDim.x = 2; attr.val.clusterDim.y = 1; attr.val.clusterDim.z = 1;
-    cfg.attrs = &attr; cfg.numAttrs = 1;
+  static PerDevice resident;
+  return resident.get(ctx().device, [] {
+    THC_CUDA(cudaFuncSetAttribute(tc2r_kernel<P, BN2>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM_BYTES));
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(2 * ctx().sm_count, 1, 1);
+    cfg.blockDim = dim3(T2_THREADS, 1, 1);
+    cfg.dynamicSmemBytes = Cfg::SMEM_BYTES;
+    int c = 0;
     if (cudaOccupancyMaxActiveClusters(&c, tc2r_kernel<P, BN2>, &cfg) != cudaSuccess || c < 1) {
       cudaGetLastError();
-      c = ctx().sm_count / 2;
+      cudaLaunchAttribute attr;
+      attr.id = cudaLaunchAttributeClusterDimension;
+      attr.val.clusterDim.x = 2; attr.val.clusterDim.y = 1; attr.val.clusterDim.z = 1;
+      cfg.attrs = &attr; cfg.numAttrs = 1;
+      if (cudaOccupancyMaxActiveClusters(&c, tc2r_kernel<P, BN2>, &cfg) != cudaSuccess || c < 1) {
+        cudaGetLastError();
+        c = ctx().sm_count / 2;
+      }
     }
-  }
-  if (c > ctx().sm_count / 2) c = ctx().sm_count / 2;
-  n = c;
-  return n;
+    return std::min(c, ctx().sm_count / 2);
+  });
 }
 template <class P, int BN2>
 static void launch_tc2r_kernel(const P &p, long items) {
