@@ -101,3 +101,22 @@ def test_large_uploads_from_several_threads(gt, n):
         t.join()
     assert not bad
     assert np.array_equal(gt.gpu(np.arange(n)).float(), np.arange(n).astype(np.float32))      # another element type
+
+
+def test_first_products_of_a_process_from_several_threads():
+    """What the engines look up once per process is there for every thread that comes while it is being looked up."""
+    import subprocess
+    import sys
+    code = """if True:
+        import threading, numpy as np, mcw_cppamp_torch_b200 as gt
+        a = np.random.default_rng(1).standard_normal((640, 640)).astype(np.float32)
+        start, got = threading.Barrier(8), []
+        def work():
+            x, r = gt.gpu(a), gt.GPUTensor(640, 640)
+            start.wait()
+            got.append(r.addmm(0.0, 1.0, x, x).float())
+        ts = [threading.Thread(target=work) for _ in range(8)]
+        [t.start() for t in ts]; [t.join() for t in ts]
+        assert len(got) == 8 and all(np.array_equal(g, got[0]) for g in got)
+        """
+    subprocess.check_call([sys.executable, "-c", code], timeout=300)
