@@ -460,19 +460,22 @@ static void reduce_dim(THGPUTensor *values, THGPUTensor *indices, THGPUTensor *s
   THC_CHECK(R < (1l << 31) - 4096, "reduced dimension too long");
   base = data_ptr(src);
   const int ond = src->nDimension;
-  // Results go where they belong unless a destination shares memory with the source or is not contiguous after
-  // resizing: then through a temporary.
-  auto place = [&](THGPUTensor *dst, TensorRef &tmp) -> float * {
+  // Results go where they belong unless a destination shares memory with the source or the other destination, or is not
+  // contiguous after resizing: then through a temporary.  Both are resized before either pointer is taken: two views of one
+  // storage, the second of which makes it grow, must not leave the first with memory that is gone.
+  auto apart = [&](const THGPUTensor *dst) { return !dst->storage || dst->storage != orig->storage; };
+  const bool twins = indices && values->storage && values->storage == indices->storage;
+  const bool direct_v = !twins && apart(values), direct_i = indices && !twins && apart(indices);
+  if (direct_v) resize_nd(values, ond, osize, nullptr);
+  if (direct_i) resize_nd(indices, ond, osize, nullptr);
+  auto place = [&](THGPUTensor *dst, bool direct, TensorRef &tmp) -> float * {
     if (!dst) return nullptr;
-    if (!dst->storage || dst->storage != orig->storage) {
-      resize_nd(dst, ond, osize, nullptr);
-      if (is_contiguous(dst)) return data_ptr(dst);
-    }
+    if (direct && is_contiguous(dst)) return data_ptr(dst);
     tmp.reset(tensor_new_sized(ond, osize));
     return data_ptr(tmp);
   };
   TensorRef vtmp, itmp;
-  float *out = place(values, vtmp), *idx = place(indices, itmp);
+  float *out = place(values, direct_v, vtmp), *idx = place(indices, direct_i, itmp);
   if (sr == 1) {
     THC_CHECK(O == 1, "internal: row reduce with outer dim");
     const bool vec = aligned16(base) && (sj % 4 == 0);

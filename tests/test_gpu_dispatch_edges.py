@@ -75,6 +75,19 @@ def test_dim_reductions(gt, shape):
     assert np.all(np.abs(X.float() - x.astype(np.float64).sum(0, keepdims=True)) <= 2.0 ** -23 * np.abs(x.astype(np.float64)).sum(0, keepdims=True))
 
 
+@pytest.mark.parametrize("shape,dim", [((300, 64), 1), ((64, 300), 2), ((700, 64), 1)])
+def test_values_and_indices_in_one_storage(gt, shape, dim):
+    """Two views of one buffer, both of which have to grow: the values are written, then the indices over what they share."""
+    x = np.random.default_rng(5).standard_normal(shape).astype(np.float32)
+    buf = gt.GPUTensor(8).fill(-1)
+    v, i = buf.narrow(1, 1, 4), buf.narrow(1, 5, 4)
+    src = gt.gpu(x)
+    gt.lib().THGPUTensor_max(v.cdata, i.cdata, src.cdata, dim - 1)
+    val, pos = x.max(dim - 1), x.argmax(dim - 1) + 1
+    assert np.array_equal(i.float().ravel(), pos)
+    assert np.array_equal(v.float().ravel(), np.concatenate([val[:4], pos[:-4]]))
+
+
 @pytest.mark.parametrize("n", [1, 1023, 16384, 16385])
 def test_download_sizes(gt, n):
     x = np.random.default_rng(n).standard_normal(n).astype(np.float32)
