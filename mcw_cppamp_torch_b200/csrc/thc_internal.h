@@ -156,6 +156,9 @@ void tensor_copy(THGPUTensor *dst, THGPUTensor *src);
 THGPUTensor *tensor_new_contiguous(THGPUTensor *t);   // retains t when it already is contiguous
 THGPUTensor *tensor_new_sized(int nd, const long *size);
 void tensor_resize_as(THGPUTensor *r, const THGPUTensor *t);
+// Whether the memory from a tensor's first element to its last meets another's.  By address: two storages may borrow the same
+// memory (THGPUStorage_newWithData).
+bool overlap(const THGPUTensor *a, const THGPUTensor *b);
 
 // Scope guard: one reference to a tensor, released when the scope is left by any route, so that a THC_CHECK that
 // throws between THC_BEGIN and THC_END does not leak it.

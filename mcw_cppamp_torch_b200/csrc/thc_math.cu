@@ -465,9 +465,11 @@ static void reduce_dim(THGPUTensor *values, THGPUTensor *indices, THGPUTensor *s
   // storage, the second of which makes it grow, must not leave the first with memory that is gone.
   auto apart = [&](const THGPUTensor *dst) { return !dst->storage || dst->storage != orig->storage; };
   const bool twins = indices && values->storage && values->storage == indices->storage;
-  const bool direct_v = !twins && apart(values), direct_i = indices && !twins && apart(indices);
+  bool direct_v = !twins && apart(values), direct_i = indices && !twins && apart(indices);
   if (direct_v) resize_nd(values, ond, osize, nullptr);
   if (direct_i) resize_nd(indices, ond, osize, nullptr);
+  direct_v = direct_v && !overlap(values, orig);
+  direct_i = direct_i && !overlap(indices, orig) && !overlap(indices, values);
   auto place = [&](THGPUTensor *dst, bool direct, TensorRef &tmp) -> float * {
     if (!dst) return nullptr;
     if (direct && is_contiguous(dst)) return data_ptr(dst);

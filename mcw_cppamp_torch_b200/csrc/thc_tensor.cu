@@ -251,6 +251,16 @@ void tensor_resize_as(THGPUTensor *r, const THGPUTensor *t) {
   if (!same) resize_nd(r, t->nDimension, t->size, nullptr);
 }
 
+bool overlap(const THGPUTensor *a, const THGPUTensor *b) {
+  if (nelem(a) == 0 || nelem(b) == 0) return false;
+  auto last = [](const THGPUTensor *t) {
+    const float *p = data_ptr(t);
+    for (int d = 0; d < t->nDimension; d++) p += (t->size[d] - 1) * t->stride[d];
+    return p;
+  };
+  return data_ptr(a) <= last(b) && data_ptr(b) <= last(a);
+}
+
 }  // namespace thc
 
 using namespace thc;

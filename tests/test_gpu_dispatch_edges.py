@@ -88,6 +88,34 @@ def test_values_and_indices_in_one_storage(gt, shape, dim):
     assert np.array_equal(v.float().ravel(), np.concatenate([val[:4], pos[:-4]]))
 
 
+def borrowed(gt, ptr, *shape):
+    """A tensor over memory that some other storage owns."""
+    L = gt.lib()
+    n = int(np.prod(shape))
+    s = L.THGPUStorage_newWithData(ptr, n)
+    t = gt.GPUTensor(_ptr=L.THGPUTensor_newWithStorage1d(s, 0, n, 1))
+    L.THGPUStorage_free(s)
+    return t.view(*shape)
+
+
+@pytest.mark.parametrize("shape,dim", [((3000, 600), 2), ((1000, 4096), 1), ((5000, 40), 2)])
+def test_dim_reductions_into_memory_the_source_borrows(gt, shape, dim):
+    """Destination and source over the same memory through storages of their own: the source is read before it is written."""
+    x = np.random.default_rng(6).standard_normal(shape).astype(np.float32)
+    out = tuple(1 if d == dim - 1 else n for d, n in enumerate(shape))
+    for _ in range(5):
+        src = gt.gpu(x)
+        v, i = borrowed(gt, src.data_ptr(), *out), gt.GPUTensor()
+        gt.lib().THGPUTensor_max(v.cdata, i.cdata, src.cdata, dim - 1)
+        assert np.array_equal(v.float(), x.max(dim - 1, keepdims=True))
+        assert np.array_equal(i.float(), np.expand_dims(x.argmax(dim - 1), dim - 1) + 1)
+        src = gt.gpu(x)
+        i, v = borrowed(gt, src.data_ptr(), *out), gt.GPUTensor()
+        gt.lib().THGPUTensor_max(v.cdata, i.cdata, src.cdata, dim - 1)
+        assert np.array_equal(v.float(), x.max(dim - 1, keepdims=True))
+        assert np.array_equal(i.float(), np.expand_dims(x.argmax(dim - 1), dim - 1) + 1)
+
+
 @pytest.mark.parametrize("n", [1, 1023, 16384, 16385])
 def test_download_sizes(gt, n):
     x = np.random.default_rng(n).standard_normal(n).astype(np.float32)
