@@ -91,13 +91,7 @@ static void add_scaled(THGPUTensor *self, THGPUTensor *t, THGPUTensor *src1, THG
   THC_ARG(nelem(src1) == nelem(t) && nelem(src2) == nelem(t), 3, "sizes do not match");
   // an operand that overlaps the result in memory without being the same view has to be read before anything is written
   auto entangled = [&](const THGPUTensor *a) {
-    if (a->storage != self->storage || (data_ptr(a) == data_ptr(self) && same_layout(a, self))) return false;
-    auto last = [](const THGPUTensor *x) {
-      long e = x->storageOffset;
-      for (int d = 0; d < x->nDimension; d++) e += (x->size[d] - 1) * x->stride[d];
-      return e;
-    };
-    return last(a) >= self->storageOffset && last(self) >= a->storageOffset;
+    return overlap(a, self) && !(data_ptr(a) == data_ptr(self) && same_layout(a, self));
   };
   TensorRef v0, v1, v2;
   if (self != t && entangled(t)) { v0.reset(THGPUTensor_newClone(t)); t = v0; }

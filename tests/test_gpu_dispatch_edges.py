@@ -13,6 +13,16 @@ def gt():
     return gt
 
 
+def borrowed(gt, ptr, *shape):
+    """A tensor over memory that some other storage owns."""
+    L = gt.lib()
+    n = int(np.prod(shape))
+    s = L.THGPUStorage_newWithData(ptr, n)
+    t = gt.GPUTensor(_ptr=L.THGPUTensor_newWithStorage1d(s, 0, n, 1))
+    L.THGPUStorage_free(s)
+    return t.view(*shape)
+
+
 @pytest.mark.parametrize("r,c", [(64, 64), (4, 8), (63, 65), (128, 68), (130, 3), (3, 130), (200, 516), (577, 129)])
 def test_transposed_operands(gt, r, c):
     g = np.random.default_rng(r * 1000 + c)
@@ -38,6 +48,21 @@ def test_addcmul_in_place_with_overlapping_operand(gt):
     X = gt.gpu(x)
     X.addcmul(0.5, X.t(), X)
     assert np.array_equal(X.float(), x + np.float32(0.5) * x.T * x)
+
+
+@pytest.mark.parametrize("r", [96, 1031])
+def test_addcmul_over_borrowed_memory(gt, r):
+    """The result's memory seen through another storage: transposed, and one element further on."""
+    x = np.random.default_rng(4).standard_normal((r, r)).astype(np.float32)
+    half = np.float32(0.5)
+    for _ in range(5):
+        X = gt.gpu(x)
+        X.addcmul(0.5, borrowed(gt, X.data_ptr(), r, r).t(), X)
+        assert np.array_equal(X.float(), x + half * x.T * x)
+        buf = gt.gpu(x.ravel())
+        a = buf.narrow(1, 2, r * r - 1)
+        a.addcdiv(0.5, borrowed(gt, buf.data_ptr(), r * r - 1), a)
+        assert np.array_equal(a.float(), x.ravel()[1:] + half * x.ravel()[:-1] / x.ravel()[1:])
 
 
 @pytest.mark.parametrize("n", [1, 3, 4096 * 4, 4096 * 4 + 4, 4096 * 4 + 1, 300007])
@@ -86,16 +111,6 @@ def test_values_and_indices_in_one_storage(gt, shape, dim):
     val, pos = x.max(dim - 1), x.argmax(dim - 1) + 1
     assert np.array_equal(i.float().ravel(), pos)
     assert np.array_equal(v.float().ravel(), np.concatenate([val[:4], pos[:-4]]))
-
-
-def borrowed(gt, ptr, *shape):
-    """A tensor over memory that some other storage owns."""
-    L = gt.lib()
-    n = int(np.prod(shape))
-    s = L.THGPUStorage_newWithData(ptr, n)
-    t = gt.GPUTensor(_ptr=L.THGPUTensor_newWithStorage1d(s, 0, n, 1))
-    L.THGPUStorage_free(s)
-    return t.view(*shape)
 
 
 @pytest.mark.parametrize("shape,dim", [((3000, 600), 2), ((1000, 4096), 1), ((5000, 40), 2)])
