@@ -89,8 +89,17 @@ static double sum_of(THGPUTensor *a, THGPUTensor *b, Op op) { return reduce_all<
 template <typename Op>
 static void add_scaled(THGPUTensor *self, THGPUTensor *t, THGPUTensor *src1, THGPUTensor *src2, Op op, const char *name) {
   THC_ARG(nelem(src1) == nelem(t) && nelem(src2) == nelem(t), 3, "sizes do not match");
-  // an operand that overlaps the result in memory without being the same view has to be read before anything is written
+  // an operand that overlaps the result in memory without being the same view has to be read before anything is written;
+  // so has, where the result is about to be resized, whatever shares its storage or lies where it will reach
+  const bool grows = self != t && !THGPUTensor_isSameSizeAs(self, t);
   auto entangled = [&](const THGPUTensor *a) {
+    if (grows && self->storage && nelem(a) > 0) {
+      if (a->storage == self->storage) return true;
+      THGPUTensor after = *self;   // where it reaches afterwards, its memory staying where it is
+      long n = nelem(t), one = 1;
+      after.size = &n; after.stride = &one; after.nDimension = 1;
+      return data_ptr(self) && overlap(a, &after);
+    }
     return overlap(a, self) && !(data_ptr(a) == data_ptr(self) && same_layout(a, self));
   };
   TensorRef v0, v1, v2;

@@ -65,6 +65,16 @@ def test_addcmul_over_borrowed_memory(gt, r):
         assert np.array_equal(a.float(), x.ravel()[1:] + half * x.ravel()[:-1] / x.ravel()[1:])
 
 
+@pytest.mark.parametrize("offset", [0, 5, 40])
+def test_addcmul_into_a_view_that_grows_over_its_operands(gt, offset):
+    x = np.random.default_rng(7).standard_normal(9000).astype(np.float32)
+    want = x[2000:5000] + np.float32(0.5) * x[40:3040] * x[offset:offset + 3000]
+    buf = gt.gpu(x)
+    r = buf.narrow(1, 1, 4)                                                              # the first four, 3000 in a moment
+    r.addcmul(buf.narrow(1, 2001, 3000), 0.5, buf.narrow(1, 41, 3000), buf.narrow(1, offset + 1, 3000))
+    assert np.array_equal(r.float(), want) and np.array_equal(buf.float()[3000:], x[3000:])
+
+
 @pytest.mark.parametrize("n", [1, 3, 4096 * 4, 4096 * 4 + 4, 4096 * 4 + 1, 300007])
 def test_full_reductions(gt, n):
     x = (np.random.default_rng(n).standard_normal(n) + 0.5).astype(np.float32)
