@@ -13,6 +13,7 @@
 #ifndef THC_APPLY_CUH
 #define THC_APPLY_CUH
 
+#include "per_device.h"
 #include "thc_internal.h"
 
 #include <type_traits>
@@ -136,24 +137,30 @@ struct TileWalk {
 };
 // strides of a 2-D index space: [operand][dim], operand 0 is the output
 struct Strides2d {
-  int s[3][2];
+  int s[4][2];
 };
+// How many of an operand set's inputs before `k` are staged in shared memory, i.e. the place of its tile.
+__host__ __device__ constexpr int staged_before(unsigned via, int k) {
+  int n = 0;
+  for (int i = 0; i < k; i++) n += via >> i & 1u;
+  return n;
+}
 
 // 2-D index space (n0, n1); the output has unit stride along dim 1.  Inputs flagged in VIA have unit stride along
 // dim 0 and are transposed through 64 x 64 shared-memory tiles: for sizes, pitches or addresses that 16-byte accesses
 // cannot serve.  Every global access of a warp is one contiguous 128-byte segment, eight per thread and operand in
 // flight.  Bound by instruction issue, not by memory, as long as each element pays for 64-bit address arithmetic and
 // bounds tests (58 instructions a warp access, half the issue slots, 3.5 TB/s on 3001 x 5003): hence 32-bit steps from one
-// pointer per tile and a path without tests for the tiles inside.
+// pointer per tile and a path without tests for the tiles inside.  Three inputs (addcmul) need 64 registers: two blocks an SM
+// (3001 x 5003: 51 us with one input transposed, 43 contiguous; element by element 128, the result transposed 465).
 template <typename Op, int NIN, unsigned VIA>   // VIA: bit k = operand k is transposed
-__global__ void __launch_bounds__(512, 3) apply_tiled2d_kernel(Operands<NIN> p, int n0, int n1, const Strides2d st,
+__global__ void __launch_bounds__(512, NIN == 3 ? 2 : 3) apply_tiled2d_kernel(Operands<NIN> p, int n0, int n1, const Strides2d st,
                                                                 TileWalk walk, Op op) {
   pdl_begin();
   constexpr int T = 64, PITCH = T + 1, TY = 512 / T, NJ = T / TY;
   extern __shared__ float tile2d_smem[];   // one [T][PITCH] tile per staged operand
   const int tx = threadIdx.x % T, ty = threadIdx.x / T;
   const unsigned ntiles = walk.count();
-  const int slot1 = (NIN > 1 && (VIA & 1u)) ? T * PITCH : 0;   // second staged operand
   auto one_tile = [&](int b0, int b1, auto inside) {
     constexpr bool INSIDE = decltype(inside)::value;
     float direct[NIN > 1 ? NIN : 1][NIN > 1 ? NJ : 1];   // a single input is always the staged one
@@ -162,7 +169,7 @@ __global__ void __launch_bounds__(512, 3) apply_tiled2d_kernel(Operands<NIN> p, 
       if (VIA & (1u << k)) {   // rows of the tile run along dim 0
         const float *src = p.in[k] + (b0 + tx) + (long)(b1 + ty) * st.s[k + 1][1];
         const int step = TY * st.s[k + 1][1];
-        float *tile = tile2d_smem + (k ? slot1 : 0) + ty * PITCH + tx;
+        float *tile = tile2d_smem + staged_before(VIA, k) * T * PITCH + ty * PITCH + tx;
         float v[NJ];
 #pragma unroll
         for (int j = 0; j < NJ; j++) v[j] = (INSIDE || (b0 + tx < n0 && b1 + ty + j * TY < n1)) ? src[j * step] : 0.f;
@@ -189,8 +196,8 @@ __global__ void __launch_bounds__(512, 3) apply_tiled2d_kernel(Operands<NIN> p, 
       float a[NIN];
 #pragma unroll
       for (int k = 0; k < NIN; k++)
-        a[k] = (VIA & (1u << k)) ? tile2d_smem[(k ? slot1 : 0) + tx * PITCH + ty + j * TY]
-                                                    : direct[NIN > 1 ? k : 0][NIN > 1 ? j : 0];
+        a[k] = (VIA & (1u << k)) ? tile2d_smem[staged_before(VIA, k) * T * PITCH + tx * PITCH + ty + j * TY]
+                                 : direct[NIN > 1 ? k : 0][NIN > 1 ? j : 0];
       if (INSIDE || (b0 + ty + j * TY < n0 && b1 + tx < n1)) dst[j * step] = op(a);
     }
     __syncthreads();
@@ -208,7 +215,8 @@ __global__ void __launch_bounds__(512, 3) apply_tiled2d_kernel(Operands<NIN> p, 
 // transposed input as four 16-byte rows along dim 0, the others as four along dim 1, and transposes in registers.
 // A warp covers 16 (dim 0) x 32 (dim 1): transposed inputs arrive in whole 64-byte segments whose other half the
 // neighbouring warp of the block fetches, results leave in 128-byte segments.  No barrier, so loads of later
-// tiles fly under the stores of earlier ones.  n0, n1 and all pitches multiples of 4, 16-byte aligned bases.
+// tiles fly under the stores of earlier ones.  addcmul on 8192 x 8192: 160 us contiguous, 170 - 194 with any operands
+// transposed (527 - 1346 element by element).  n0, n1 and all pitches multiples of 4, 16-byte aligned bases.
 template <typename Op, int NIN, unsigned VIA>
 __global__ void __launch_bounds__(256) apply_transpose4_kernel(Operands<NIN> p, int n0, int n1, const Strides2d st, TileWalk walk,
                                                                Op op) {
@@ -251,6 +259,14 @@ __global__ void __launch_bounds__(256) apply_transpose4_kernel(Operands<NIN> p, 
 
 inline bool aligned16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 
+// f(integral constant `via`) for via in [FIRST, END)
+template <unsigned FIRST, unsigned END, class F> void with_via(unsigned via, F f) {
+  if constexpr (FIRST < END) {
+    if (via == FIRST) f(std::integral_constant<unsigned, FIRST>());
+    else with_via<FIRST + 1, END>(via, f);
+  }
+}
+
 // out = op(in...) over tensors of equal shape (already resized by the caller); out may alias an input.
 template <int NIN, typename Op>
 void apply(THGPUTensor *out, const THGPUTensor *in0, const THGPUTensor *in1, Op op, const char *name,
@@ -276,7 +292,7 @@ void apply(THGPUTensor *out, const THGPUTensor *in0, const THGPUTensor *in1, Op 
   }
   Strided s;
   THC_CHECK(collapse(NIN + 1, ops, s), "%s: too many non-collapsible dimensions", name);
-  if constexpr (NIN == 1 || NIN == 2) {
+  if constexpr (NIN >= 1) {
     if (s.nd == 2) {
       // normalise so that the output's unit-stride dim is dim 1
       int a = 0, b = 1;
@@ -298,16 +314,23 @@ void apply(THGPUTensor *out, const THGPUTensor *in0, const THGPUTensor *in1, Op 
           bool vec = aligned16(p.out) && n0 % 4 == 0 && n1 % 4 == 0 && st.s[0][0] % 4 == 0;
           for (int k = 0; k < NIN; k++)
             vec = vec && aligned16(p.in[k]) && ((via >> k & 1u) ? st.s[k + 1][1] % 4 == 0 : st.s[k + 1][1] == 1 && st.s[k + 1][0] % 4 == 0);
-          if (vec) {
-            if (NIN == 1 || via == 1u) pdl_launch(apply_transpose4_kernel<Op, NIN, 1u>, blocks, 256, 0, p, (int)n0, (int)n1, st, walk, op);
-            else if (via == 2u) pdl_launch(apply_transpose4_kernel<Op, NIN, NIN == 2 ? 2u : 1u>, blocks, 256, 0, p, (int)n0, (int)n1, st, walk, op);
-            else pdl_launch(apply_transpose4_kernel<Op, NIN, NIN == 2 ? 3u : 1u>, blocks, 256, 0, p, (int)n0, (int)n1, st, walk, op);
-          } else {
-            const size_t smem = (via == 3u ? 2 : 1) * 64 * 65 * sizeof(float);
-            if (NIN == 1 || via == 1u) pdl_launch(apply_tiled2d_kernel<Op, NIN, 1u>, blocks, 512, smem, p, (int)n0, (int)n1, st, walk, op);
-            else if (via == 2u) pdl_launch(apply_tiled2d_kernel<Op, NIN, NIN == 2 ? 2u : 1u>, blocks, 512, smem, p, (int)n0, (int)n1, st, walk, op);
-            else pdl_launch(apply_tiled2d_kernel<Op, NIN, NIN == 2 ? 3u : 1u>, blocks, 512, smem, p, (int)n0, (int)n1, st, walk, op);
-          }
+          const auto launch = [&](auto v) {
+            constexpr unsigned VIA = decltype(v)::value;
+            if (vec) {
+              pdl_launch(apply_transpose4_kernel<Op, NIN, VIA>, blocks, 256, 0, p, (int)n0, (int)n1, st, walk, op);
+            } else {
+              constexpr size_t smem = (size_t)staged_before(VIA, NIN) * 64 * 65 * sizeof(float);
+              if constexpr (smem > 48 * 1024) {   // three staged tiles
+                static PerDevice allowed;
+                allowed.get(ctx().device, [] {
+                  THC_CUDA(cudaFuncSetAttribute(apply_tiled2d_kernel<Op, NIN, VIA>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+                  return 1;
+                });
+              }
+              pdl_launch(apply_tiled2d_kernel<Op, NIN, VIA>, blocks, 512, smem, p, (int)n0, (int)n1, st, walk, op);
+            }
+          };
+          with_via<1, (1u << NIN)>(via, launch);
           check_launch(name);
           return;
         }

@@ -43,6 +43,48 @@ def test_transposed_operands(gt, r, c):
     assert np.array_equal(sub.float(), want)
 
 
+@pytest.mark.parametrize("r,c", [(64, 64), (4, 8), (63, 65), (128, 68), (130, 3), (200, 516), (577, 129)])
+def test_transposed_operands_of_addcmul(gt, r, c):
+    """Every set of transposed operands, contiguous and transposed results, in whole 16-byte pieces and off them."""
+    g = np.random.default_rng(r * 1000 + c)
+    v = [g.standard_normal((r, c)).astype(np.float32) + np.float32(3) for _ in range(3)]
+    half = np.float32(0.5)
+    mul, div = v[0] + half * v[1] * v[2], v[0] + half * v[1] / v[2]
+    for turned in range(8):
+        a, b, d = (gt.gpu(np.ascontiguousarray(x.T)).t() if turned >> k & 1 else gt.gpu(x) for k, x in enumerate(v))
+        assert np.array_equal(gt.GPUTensor(r, c).addcmul(a, 0.5, b, d).float(), mul)
+        assert np.array_equal(gt.GPUTensor(r, c).addcdiv(a, 0.5, b, d).float(), div)
+        out = gt.GPUTensor(c, r)
+        out.t().addcmul(a, 0.5, b, d)
+        assert np.array_equal(out.float(), mul.T)
+        a.addcmul(0.5, b, d)
+        assert np.array_equal(a.float(), mul)
+
+
+def device_us(gt, f, n=5):
+    """Median time of f() on the library's stream."""
+    import torch
+    s, times = torch.cuda.ExternalStream(gt.lib().THGPUGetStream()), []
+    for _ in range(n + 2):
+        a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        a.record(s)
+        f()
+        b.record(s)
+        b.synchronize()
+        times.append(a.elapsed_time(b) * 1e3)
+    return sorted(times[2:])[n // 2]
+
+
+def test_addcmul_reads_transposed_operands_by_lines(gt):
+    """At 8192 x 8192: 161 us contiguous; one operand (the result) transposed 527 (1346) when elements are fetched one by one a
+    row apart, 170 (194) through tiles."""
+    n = 8192
+    t, a, b, at, tt = (gt.GPUTensor(n, n).fill(1.0) for _ in range(5))
+    plain = device_us(gt, lambda: t.addcmul(0.5, a, b))
+    assert device_us(gt, lambda: t.addcmul(0.5, at.t(), b)) < 2 * plain
+    assert device_us(gt, lambda: tt.t().addcmul(0.5, a, b)) < 2 * plain
+
+
 def test_addcmul_in_place_with_overlapping_operand(gt):
     x = np.random.default_rng(3).standard_normal((96, 96)).astype(np.float32)
     X = gt.gpu(x)
