@@ -6,7 +6,7 @@
 //                4 x 4 blocks transposed in registers where 16-byte accesses are possible, else
 //                64 x 64 shared-memory tiles, so that every global access stays coalesced; counts the
 //                same algorithmic bytes as the contiguous case
-//   strided    : anything else, collapsed dims + div/mod indexing (correct, not fast)
+//   strided    : anything else (and transposed operands of a few rows or columns), collapsed dims + div/mod indexing (correct, not fast)
 // This replaces the reference pattern "newContiguous every operand, run, freeCopyTo the result"
 // (gputorch/lib/THC/THCTensorMath.cpp:67-163) and its per-element div/mod copy kernel
 // (gputorch/lib/THC/THCTensorCopy.cpp:170-218).
@@ -137,7 +137,7 @@ struct TileWalk {
 };
 // strides of a 2-D index space: [operand][dim], operand 0 is the output
 struct Strides2d {
-  int s[4][2];
+  long s[4][2];
 };
 // How many of an operand set's inputs before `k` are staged in shared memory, i.e. the place of its tile.
 __host__ __device__ constexpr int staged_before(unsigned via, int k) {
@@ -149,10 +149,10 @@ __host__ __device__ constexpr int staged_before(unsigned via, int k) {
 // 2-D index space (n0, n1); the output has unit stride along dim 1.  Inputs flagged in VIA have unit stride along
 // dim 0 and are transposed through 64 x 64 shared-memory tiles: for sizes, pitches or addresses that 16-byte accesses
 // cannot serve.  Every global access of a warp is one contiguous 128-byte segment, eight per thread and operand in
-// flight.  Bound by instruction issue, not by memory, as long as each element pays for 64-bit address arithmetic and
-// bounds tests (58 instructions a warp access, half the issue slots, 3.5 TB/s on 3001 x 5003): hence 32-bit steps from one
-// pointer per tile and a path without tests for the tiles inside.  Three inputs (addcmul) need 64 registers: two blocks an SM
-// (3001 x 5003: 51 us with one input transposed, 43 contiguous; element by element 128, the result transposed 465).
+// flight.  Bound by instruction issue, not by memory, as long as each element pays for its whole address and bounds tests (58
+// instructions a warp access, half the issue slots, 3.5 TB/s on 3001 x 5003): hence steps from one pointer per tile (64 bits
+// wide: any pitch; 32-bit ones measured no faster) and a path without tests for the tiles inside.  Three inputs (addcmul)
+// need 64 registers: two blocks an SM (3001 x 5003: 51 us with one input transposed, 43 contiguous; element by element 128, the result transposed 465).
 template <typename Op, int NIN, unsigned VIA>   // VIA: bit k = operand k is transposed
 __global__ void __launch_bounds__(512, NIN == 3 ? 2 : 3) apply_tiled2d_kernel(Operands<NIN> p, int n0, int n1, const Strides2d st,
                                                                 TileWalk walk, Op op) {
@@ -167,8 +167,8 @@ __global__ void __launch_bounds__(512, NIN == 3 ? 2 : 3) apply_tiled2d_kernel(Op
 #pragma unroll
     for (int k = 0; k < NIN; k++) {
       if (VIA & (1u << k)) {   // rows of the tile run along dim 0
-        const float *src = p.in[k] + (b0 + tx) + (long)(b1 + ty) * st.s[k + 1][1];
-        const int step = TY * st.s[k + 1][1];
+        const float *src = p.in[k] + (b0 + tx) + (b1 + ty) * st.s[k + 1][1];
+        const long step = TY * st.s[k + 1][1];
         float *tile = tile2d_smem + staged_before(VIA, k) * T * PITCH + ty * PITCH + tx;
         float v[NJ];
 #pragma unroll
@@ -182,15 +182,15 @@ __global__ void __launch_bounds__(512, NIN == 3 ? 2 : 3) apply_tiled2d_kernel(Op
 #pragma unroll
     for (int k = 0; k < (NIN > 1 ? NIN : 0); k++) {
       if (!(VIA & (1u << k))) {
-        const float *src = p.in[k] + (long)(b0 + ty) * st.s[k + 1][0] + (long)(b1 + tx) * st.s[k + 1][1];
-        const int step = TY * st.s[k + 1][0];
+        const float *src = p.in[k] + (b0 + ty) * st.s[k + 1][0] + (b1 + tx) * st.s[k + 1][1];
+        const long step = TY * st.s[k + 1][0];
 #pragma unroll
         for (int j = 0; j < NJ; j++) direct[k][j] = (INSIDE || (b0 + ty + j * TY < n0 && b1 + tx < n1)) ? src[j * step] : 0.f;
       }
     }
     __syncthreads();
-    float *dst = p.out + (long)(b0 + ty) * st.s[0][0] + (b1 + tx);
-    const int step = TY * st.s[0][0];
+    float *dst = p.out + (b0 + ty) * st.s[0][0] + (b1 + tx);
+    const long step = TY * st.s[0][0];
 #pragma unroll
     for (int j = 0; j < NJ; j++) {
       float a[NIN];
@@ -233,15 +233,15 @@ __global__ void __launch_bounds__(256) apply_transpose4_kernel(Operands<NIN> p, 
 #pragma unroll
     for (int k = 0; k < NIN; k++) {
       const bool tr = (VIA & (1u << k)) != 0;
-      const int step = tr ? st.s[k + 1][1] : st.s[k + 1][0];
-      const float *b = p.in[k] + (tr ? (long)i1 * step + i0 : (long)i0 * step + i1);
+      const long step = tr ? st.s[k + 1][1] : st.s[k + 1][0];
+      const float *b = p.in[k] + (tr ? i1 * step + i0 : i0 * step + i1);
 #pragma unroll
       for (int r = 0; r < 4; r++) {
         const float4 q = *reinterpret_cast<const float4 *>(b + r * step);
         v[k][r][0] = q.x; v[k][r][1] = q.y; v[k][r][2] = q.z; v[k][r][3] = q.w;
       }
     }
-    float *dst = p.out + (long)i0 * st.s[0][0] + i1;
+    float *dst = p.out + i0 * st.s[0][0] + i1;
 #pragma unroll
     for (int r = 0; r < 4; r++) {
       float o[4];
@@ -301,19 +301,23 @@ void apply(THGPUTensor *out, const THGPUTensor *in0, const THGPUTensor *in1, Op 
         unsigned via = 0;
         for (int k = 0; k < NIN; k++)
           if (s.stride[k + 1][a] == 1 && s.stride[k + 1][b] != 1) via |= 1u << k;
-        bool fits = s.size[0] < (1l << 30) && s.size[1] < (1l << 30);   // 32-bit steps inside a tile
-        for (int k = 0; k <= NIN; k++) fits = fits && s.stride[k][0] < (1l << 24) && s.stride[k][1] < (1l << 24);
+        const bool fits = s.size[0] < (1l << 31) - 128 && s.size[1] < (1l << 31) - 128;   // 32-bit places
         const long n0 = s.size[a], n1 = s.size[b];
         const long tiles0 = (n0 + 63) / 64, tiles1 = (n1 + 63) / 64;
-        if (via && fits && tiles0 * tiles1 < (1l << 30)) {
+        Strides2d st = {};
+        for (int k = 0; k <= NIN; k++) { st.s[k][0] = s.stride[k][a]; st.s[k][1] = s.stride[k][b]; }
+        // 16-byte accesses on every operand: pitches and extents multiples of 4, aligned bases
+        bool vec = aligned16(p.out) && n0 % 4 == 0 && n1 % 4 == 0 && st.s[0][0] % 4 == 0;
+        for (int k = 0; k < NIN; k++)
+          vec = vec && aligned16(p.in[k]) && ((via >> k & 1u) ? st.s[k + 1][1] % 4 == 0 : st.s[k + 1][1] == 1 && st.s[k + 1][0] % 4 == 0);
+        // A few rows or columns fill a few of a tile's 64, and the tile takes as long.  33.5 M elements in 2 / 6 rows: cadd 1593 / 553
+        // us through shared-memory tiles, 243 / 263 element by element (addcmul 2178 / 748 against 263 / 275, copy 1087 / 382
+        // against 235 / 255); the former falls as one over the rows, which puts the line at 9 - 16.  Blocks turned in
+        // registers, in 4 / 8 rows: copy 180 / 105 us, cadd 307 / 183, addcmul 324 / 194 against 235, 248 and 266.
+        const bool wide = std::min(n0, n1) >= (vec ? (NIN == 3 ? 8 : 4) : 12);
+        if (via && fits && wide && tiles0 * tiles1 < (1l << 30)) {
           const TileWalk walk{(unsigned)tiles0, (unsigned)tiles1};
           const unsigned blocks = std::min(walk.count(), (unsigned)max_blocks);
-          Strides2d st = {};
-          for (int k = 0; k <= NIN; k++) { st.s[k][0] = (int)s.stride[k][a]; st.s[k][1] = (int)s.stride[k][b]; }
-          // 16-byte accesses on every operand: pitches and extents multiples of 4, aligned bases
-          bool vec = aligned16(p.out) && n0 % 4 == 0 && n1 % 4 == 0 && st.s[0][0] % 4 == 0;
-          for (int k = 0; k < NIN; k++)
-            vec = vec && aligned16(p.in[k]) && ((via >> k & 1u) ? st.s[k + 1][1] % 4 == 0 : st.s[k + 1][1] == 1 && st.s[k + 1][0] % 4 == 0);
           const auto launch = [&](auto v) {
             constexpr unsigned VIA = decltype(v)::value;
             if (vec) {

@@ -61,6 +61,14 @@ def test_transposed_operands_of_addcmul(gt, r, c):
         assert np.array_equal(a.float(), mul)
 
 
+@pytest.mark.parametrize("few", [2, 4, 7, 8, 11, 12, 13])
+@pytest.mark.parametrize("many", [129, 4096])
+def test_transposed_operands_of_a_few_rows(gt, few, many):
+    for r, c in ((few, many), (many, few)):
+        test_transposed_operands(gt, r, c)
+        test_transposed_operands_of_addcmul(gt, r, c)
+
+
 def device_us(gt, f, n=5):
     """Median time of f() on the library's stream."""
     import torch
@@ -83,6 +91,22 @@ def test_addcmul_reads_transposed_operands_by_lines(gt):
     plain = device_us(gt, lambda: t.addcmul(0.5, a, b))
     assert device_us(gt, lambda: t.addcmul(0.5, at.t(), b)) < 2 * plain
     assert device_us(gt, lambda: tt.t().addcmul(0.5, a, b)) < 2 * plain
+
+
+@pytest.mark.parametrize("cols", [(1 << 24) + 4, (1 << 24) + 5])
+def test_transposed_copy_of_very_long_rows(gt, cols):
+    """Rows of 16.8 M floats: 2.0 ms through tiles, 8.7 element by element (1.3 for the contiguous copy)."""
+    x, y = gt.GPUTensor(64, cols), gt.GPUTensor(cols, 64)
+    for r in range(1, 65):
+        x.narrow(1, r, 1).fill(r)
+    x.narrow(2, 12345678, 1).fill(77)
+    y.copy(x.t())
+    want = np.arange(1, 65, dtype=np.float32)
+    lo, hi = y.min(1)[0].float().ravel(), y.max(1)[0].float().ravel()
+    assert np.array_equal(lo, want) and np.all(hi == 77)
+    assert np.all(y.narrow(1, 12345678, 1).float() == 77) and np.array_equal(y.narrow(1, cols, 1).float().ravel(), want)
+    flat = y.view(64, cols)
+    assert device_us(gt, lambda: y.copy(x.t()), 3) < 3 * device_us(gt, lambda: flat.copy(x), 3)
 
 
 def test_addcmul_in_place_with_overlapping_operand(gt):
