@@ -127,12 +127,25 @@ __device__ __forceinline__ void mma_tf32(float (&d)[4], const uint32_t (&a)[4], 
 }
 // hi = tf32(x) rounded to nearest in integer arithmetic, lo = x - hi scaled by 1 + 2^-12, of which the tensor core drops the
 // low 13 bits (within 3/4 of a unit of the nearest): the conversion instruction shares a pipe that takes a quarter of
-// the ALU's rate and was what bounded this kernel (4096 x 1 x 9216: 45 us with it, 37 without).  A NaN whose mantissa
-// overflows in hi stays a NaN in lo.
+// the ALU's rate and was what bounded this kernel (4096 x 1 x 9216: 45 us with it, 37 without).
+// A value next to the largest rounds to infinity, and lo to its opposite; an infinite one or a NaN has a NaN in lo.  All of
+// them leave a NaN in every sum they reach, whatever the other operand: fp32_sum().
 __device__ __forceinline__ void split_tf32(float x, uint32_t &hi, uint32_t &lo) {
   hi = (__float_as_uint(x) + 0x1000u) & 0xffffe000u;
   const float d = x - __uint_as_float(hi);
   lo = __float_as_uint(fmaf(d, 0x1p-12f, d));
+}
+
+// The sum over [k0, k1) in plain FP32, for one that came out as NaN: values near the largest and infinities then give what FP32
+// arithmetic gives.  (Keeping hi finite by a clamp in split_tf32 costs 2 - 14 % of the whole kernel, 4096 x 16 x 4096 27.0 -> 30.7
+// us; a second pass over the tiles with the clamp costs the 64 x 64 tile its registers.)
+template <bool A_K, bool B_K>
+__device__ __forceinline__ float fp32_sum(const SmallProblem &p, long m, long n, int k0, int k1) {
+  const float *a = p.a.base + (A_K ? m * p.a.ld + k0 : m + k0 * p.a.ld), *b = p.b.base + (B_K ? n * p.b.ld + k0 : n + k0 * p.b.ld);
+  float sum = 0.f;
+#pragma unroll 1
+  for (int k = k0; k < k1; k++, a += A_K ? 1 : p.a.ld, b += B_K ? 1 : p.b.ld) sum = fmaf(*a, *b, sum);
+  return sum;
 }
 
 // WM x WN warps, each (BM / WM) x (BN / WN)
@@ -241,6 +254,25 @@ __global__ void __launch_bounds__(SM_THREADS) small_kernel(const SmallProblem p)
         for (int e = 0; e < 4; e++) acc[i][j][e] += big[i][j][e] + cross[i][j][e];
   }
   cp_async_wait<0>();
+  bool nan = false;
+#pragma unroll
+  for (int i = 0; i < MT; i++)
+#pragma unroll
+    for (int j = 0; j < NT; j++)
+#pragma unroll
+      for (int e = 0; e < 4; e++) nan = nan || acc[i][j][e] != acc[i][j][e];
+  if (nan) {
+    const int k0 = kt0 * TC_BK, k1 = min(p.K, k0 + nk * TC_BK);
+#pragma unroll
+    for (int i = 0; i < MT; i++)
+#pragma unroll
+      for (int j = 0; j < NT; j++)
+#pragma unroll
+        for (int e = 0; e < 4; e++) {
+          const int m = m0 + a_row(i, g, e >> 1), n = n0 + b_row(j, 2 * t + (e & 1));
+          if (acc[i][j][e] != acc[i][j][e] && m < p.M && n < p.N) acc[i][j][e] = fp32_sum<A_K, B_K>(p, m, n, k0, k1);
+        }
+  }
   if (p.slices > 1) {
     const long tile = (long)blockIdx.y * gridDim.x + blockIdx.x;
     constexpr int NV = MT * NT * 4;

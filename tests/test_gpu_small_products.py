@@ -67,7 +67,30 @@ def test_nan_and_infinity_reach_the_result(gt):
     A[3, 5], A[4, 6] = np.nan, np.inf
     A[2, 1:2].view(np.uint32)[:] = 0x7fffffff           # the NaN that device arithmetic makes
     r = gt.GPUTensor(70, 20).zero().addmm(0.0, 1.0, gt.gpu(A), gt.gpu(np.ones((40, 20), np.float32))).float()
-    assert np.isnan(r[2:4]).all() and not np.isfinite(r[4]).any() and np.all(r[5] == 40)
+    assert np.isnan(r[2:4]).all() and np.all(r[4] == np.inf) and np.all(r[5] == 40)
+
+
+@pytest.mark.filterwarnings("ignore:invalid value encountered")
+@pytest.mark.parametrize("n", [2, 8, 12, 20, 33, 70])
+@pytest.mark.parametrize("k", [40, 44, 700])
+def test_values_next_to_the_largest(gt, n, k):
+    """Operands whose TF32 part would round to infinity, on either side, and infinities: what FP32 arithmetic gives.  (Products of
+    the two-SM engine keep the finite ones; an infinity there meets its own NaN low part.)"""
+    top = np.finfo(np.float32).max
+    g = np.random.default_rng(n + k)
+    A, B = (g.standard_normal(s).astype(np.float32) for s in ((70, k), (k, n)))
+    A[:4] = 0
+    A[0, 5], A[1, 5], A[2, 7], A[3, 9] = top, -3.4028e38, np.inf, -np.inf
+    B[5], B[7], B[9] = 0.5, 2, 4096                                                      # exact in TF32: no low part
+    exact = A.astype(np.float64) @ B.astype(np.float64)
+    for a in (gt.gpu(A), gt.gpu(np.ascontiguousarray(A.T)).t()):
+        for b in (gt.gpu(B), gt.gpu(np.ascontiguousarray(B.T)).t()):
+            r = gt.GPUTensor(70, n).zero().addmm(0.0, 1.0, a, b).float()
+            assert np.all(np.abs(r[:2] / exact[:2] - 1) <= 2.0 ** -21)
+            assert np.all(r[2] == np.inf) and np.all(r[3] == -np.inf)
+            assert np.all(np.abs(r[4:] - exact[4:]) <= (bound(A, B, k) + 2.0 ** -22 * np.abs(exact))[4:])
+            other = gt.GPUTensor(n, 70).zero().addmm(0.0, 1.0, b.t(), a.t()).float()     # the huge ones on the other side
+            assert np.array_equal(other.T[2:4], r[2:4]) and np.all(np.abs(other.T[:2] / exact[:2] - 1) <= 2.0 ** -21)
 
 
 @pytest.mark.parametrize("rows", [1, 2, 3, 4, 5, 8, 9])
