@@ -57,16 +57,6 @@ void stamp_planes(const THGPUTensor *finput, const float *input, const ConvGeom 
 void forget_planes(const THGPUTensor *finput) {
   if (finput && finput->storage) g_plane_stamps.erase(data_ptr(finput));
 }
-// The planes the forward pass of this very layer over this very input left in `finput`, or null.
-const void *planes_made_from(const THGPUTensor *finput, const float *input, const ConvGeom &g, bool half) {
-  if (!finput || !finput->storage || !is_contiguous(finput)) return nullptr;
-  auto it = g_plane_stamps.find(data_ptr(finput));
-  if (it == g_plane_stamps.end()) return nullptr;
-  const PlaneStamp &s = it->second;
-  const bool same = s.input == input && s.half == half && s.N == g.N && s.C == g.C && s.H == g.H && s.W == g.W && s.K == g.K &&
-                    s.kH == g.kH && s.kW == g.kW && s.dH == g.dH && s.dW == g.dW && s.pad == g.pad;
-  return same ? data_ptr(finput) : nullptr;
-}
 }  // namespace
 
 // ------------------------------------------------------------------------------------------------
@@ -223,6 +213,20 @@ static const void *restated_input(const ConvGeom &g, const mm::Cells &u, const f
   pdl_launch(mm::cells_input_kernel<HALF>, dim3((unsigned)rows, parts), 256, sizeof(int2) * u.Cs, in, dst, u);
   check_launch("cells_input");
   return dst;
+}
+
+// The planes the forward pass of this very layer over this very input left in `finput`, or null.  A `finput` that has been given
+// another shape since has been used for something else.
+static const void *planes_made_from(const THGPUTensor *finput, const float *input, const ConvGeom &g, const mm::Cells &u, bool half) {
+  if (!finput || !finput->storage || finput->nDimension != 5 || !is_contiguous(finput)) return nullptr;
+  const long shape[5] = {1, g.N, u.Hs, u.Ws, half ? u.Cs / 2 : u.Cs};
+  if (!std::equal(shape, shape + 5, finput->size)) return nullptr;
+  auto it = g_plane_stamps.find(data_ptr(finput));
+  if (it == g_plane_stamps.end()) return nullptr;
+  const PlaneStamp &s = it->second;
+  const bool same = s.input == input && s.half == half && s.N == g.N && s.C == g.C && s.H == g.H && s.W == g.W && s.K == g.K &&
+                    s.kH == g.kH && s.kW == g.kW && s.dH == g.dH && s.dW == g.dW && s.pad == g.pad;
+  return same ? data_ptr(finput) : nullptr;
 }
 
 template <bool HALF>
@@ -492,7 +496,7 @@ static void conv_backward_tc(const ConvGeom &g, const float *in, const float *go
   if (w_ok) {
     // the input's planes: those the forward pass left in finput (as the CPU nn path reuses its finput,
     // mcw_nn/generic/SpatialConvolutionMM.c:284-346), else made here
-    const void *act = planes_made_from(finput, in, g, HALF);
+    const void *act = planes_made_from(finput, in, g, u, HALF);
     if (!act) act = restated_input<HALF>(g, u, in, nullptr);
     conv_acc_grad_tc<HALF>(g, u, act, pgo, gw, scale);
   } else {

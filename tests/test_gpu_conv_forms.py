@@ -67,3 +67,23 @@ def test_conv_forms(mode, case):
     assert np.all(a(gi - conv_grad_input_exact(go, w, x.shape, *geo)) <= rel * conv_grad_input_exact(a(go), a(w), x.shape, *geo) + 1e-30)
     assert np.all(a(gw - (gw0 + 0.5 * gw_e)) <= (rel + long) * (gw_s + a(gw0)))
     assert np.all(a(gb - (gb0 + 0.5 * gb_e)) <= (2.0 ** -19 + long) * (gb_s + a(gb0)))
+
+
+@pytest.mark.parametrize("C", [3, 32])
+def test_planes_of_a_finput_put_to_another_use_are_not_taken(C):
+    """`finput` resized (its memory stays where it is) and written to between the forward pass and accGradParameters."""
+    import mcw_cppamp_torch_b200 as gt
+    g = np.random.default_rng(C)
+    m = gt.nn.SpatialConvolutionMM(C, 40, 3, 3, 1, 1, 1).gpu()
+    x, go = (gt.gpu(g.standard_normal((4, c, 16, 16)).astype(np.float32)) for c in (C, 40))
+
+    def weight_gradient(touch):
+        m.gradWeight.zero(); m.gradBias.zero()
+        m.forward(x)
+        if touch:
+            at = m.finput.data_ptr()
+            m.finput.resize(100, 7).fill(3)
+            assert m.finput.data_ptr() == at
+        m.accGradParameters(x, go)
+        return m.gradWeight.float()
+    assert np.array_equal(weight_gradient(False), weight_gradient(True))
