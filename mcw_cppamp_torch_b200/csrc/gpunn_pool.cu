@@ -305,6 +305,7 @@ static __global__ void __launch_bounds__(256) maxpool2_backward_kernel(const flo
           const long o = (plane * oH + y) * oW + x + k;
           iy = indy[o]; ix = indx[o]; v = gout[o];
         }
+        v = __fadd_rn(v, 0.f);   // what the CPU's addition to a zeroed pixel leaves: -0 becomes +0
         top[2 * k] = iy == 1.f && ix == 1.f ? v : 0.f; top[2 * k + 1] = iy == 1.f && ix == 2.f ? v : 0.f;
         low[2 * k] = iy == 2.f && ix == 1.f ? v : 0.f; low[2 * k + 1] = iy == 2.f && ix == 2.f ? v : 0.f;
       }

@@ -31,3 +31,15 @@ def test_pooling_edges(oracle_port, shape, k):
     go = g.standard_normal(want.shape).astype(np.float32)
     gi = m.updateGradInput(gt.gpu(x), gt.gpu(go)).float()
     assert np.array_equal(gi, oracle_port.maxpool_backward(go, wind, x.shape, 2, 2))
+
+
+@pytest.mark.parametrize("k", [2, 3])
+@pytest.mark.parametrize("W", [8, 9])
+def test_negative_zero_gradients(k, W):
+    """The CPU adds a gradient to a zeroed pixel, which turns -0 into +0; no pixel of the result has a sign bit."""
+    import mcw_cppamp_torch_b200 as gt
+    x = gt.gpu(np.random.default_rng(W).standard_normal((2, 3, 9, W)).astype(np.float32))
+    p = gt.nn.SpatialMaxPooling(k, k, 2, 2)
+    out = p.forward(x).size()
+    gi = p.updateGradInput(x, gt.gpu(np.full(out, -0.0, np.float32))).float()
+    assert np.all(gi == 0) and not np.signbit(gi).any()
