@@ -226,7 +226,7 @@ class _Lib:
 
         def address(fn):
             return C.cast(fn, C.c_void_p).value
-        _calls.setup(address(self.cdll.THGPUGetLastError), address(self.cdll.THGPUClearError), THCError, (TP, SP, C.c_void_p))
+        _calls.setup(address(self.cdll.THGPUGetLastError), address(self.cdll.THGPUClearError), THCError, TP, SP)
         _calls.functions(*(address(getattr(self.cdll, n)) for n in ("THGPUTensor_setStorage", "THGPUTensor_copyFloat",
                                                                     "THFloatTensor_copyGPU")))
         for name, (res, args) in SIGNATURES.items():

@@ -22,27 +22,25 @@ namespace {
 const char *(*g_last_error)(void) = nullptr;
 void (*g_clear_error)(void) = nullptr;
 PyObject *g_error_type = nullptr;
-PyTypeObject *g_pointer_types[8];   // ctypes types whose instances are one pointer: POINTER(THGPUTensor), c_void_p ...
-int g_npointer_types = 0;
+// ctypes types whose instances are one pointer: POINTER(THGPUTensor), POINTER(THGPUStorage)
+PyTypeObject *g_tensor_type = nullptr, *g_storage_type = nullptr;
 
-bool pointer_of(PyObject *o, void **out) {
+// None, or an instance of exactly this type: a pointer to something else is for ctypes to convert or reject.
+bool pointer_of(PyObject *o, PyTypeObject *type, void **out) {
   if (o == Py_None) { *out = nullptr; return true; }
-  PyTypeObject *t = Py_TYPE(o);
-  for (int i = 0; i < g_npointer_types; i++)
-    if (t == g_pointer_types[i]) {
-      Py_buffer b;
-      if (PyObject_GetBuffer(o, &b, PyBUF_SIMPLE) != 0) { PyErr_Clear(); return false; }
-      std::memcpy(out, b.buf, sizeof(void *));
-      PyBuffer_Release(&b);
-      return true;
-    }
-  return false;
+  if (Py_TYPE(o) != type) return false;
+  Py_buffer b;
+  if (PyObject_GetBuffer(o, &b, PyBUF_SIMPLE) != 0) { PyErr_Clear(); return false; }
+  std::memcpy(out, b.buf, sizeof(void *));
+  PyBuffer_Release(&b);
+  return true;
 }
 
 template <class T> bool take(PyObject *o, T &out) {
-  if constexpr (std::is_pointer<T>::value && !std::is_function<typename std::remove_pointer<T>::type>::value) {
+  typedef typename std::remove_cv<typename std::remove_pointer<T>::type>::type Pointee;
+  if constexpr (std::is_same<Pointee, THGPUTensor>::value || std::is_same<Pointee, THGPUStorage>::value) {
     void *p;
-    if (!pointer_of(o, &p)) return false;
+    if (!pointer_of(o, std::is_same<Pointee, THGPUTensor>::value ? g_tensor_type : g_storage_type, &p)) return false;
     out = (T)p;
     return true;
   } else if constexpr (std::is_floating_point<T>::value) {
@@ -164,21 +162,19 @@ PyObject *call_get_slow(PyObject *self, void *) {
 PyGetSetDef call_getset[] = {{"slow", call_get_slow, nullptr, "the ctypes route of this function", nullptr}, {}};
 PyTypeObject CallType = {PyVarObject_HEAD_INIT(nullptr, 0)};
 
-// setup(last_error address, clear_error address, error class, pointer types)
+// setup(last_error address, clear_error address, error class, tensor pointer type, storage pointer type)
 PyObject *setup(PyObject *, PyObject *args) {
   unsigned long long le, ce;
-  PyObject *cls, *types;
-  if (!PyArg_ParseTuple(args, "KKOO!", &le, &ce, &cls, &PyTuple_Type, &types)) return nullptr;
+  PyObject *cls, *tensor, *storage;
+  if (!PyArg_ParseTuple(args, "KKOO!O!", &le, &ce, &cls, &PyType_Type, &tensor, &PyType_Type, &storage)) return nullptr;
   g_last_error = (const char *(*)(void))le;
   g_clear_error = (void (*)(void))ce;
   Py_INCREF(cls);
   g_error_type = cls;
-  g_npointer_types = 0;
-  for (Py_ssize_t i = 0; i < PyTuple_GET_SIZE(types) && i < 8; i++) {
-    PyObject *t = PyTuple_GET_ITEM(types, i);
-    Py_INCREF(t);
-    g_pointer_types[g_npointer_types++] = (PyTypeObject *)t;
-  }
+  Py_INCREF(tensor);
+  g_tensor_type = (PyTypeObject *)tensor;
+  Py_INCREF(storage);
+  g_storage_type = (PyTypeObject *)storage;
   Py_RETURN_NONE;
 }
 // wrap(name, address, slow) -> callable, or None for a function without an invoker
@@ -217,7 +213,7 @@ PyObject *functions(PyObject *, PyObject *args) {
 }
 THGPUTensor *tensor_arg(PyObject *o) {
   void *p;
-  if (!pointer_of(o, &p) || !p) {
+  if (!pointer_of(o, g_tensor_type, &p) || !p) {
     PyErr_SetString(PyExc_TypeError, "pointer to a THGPUTensor expected");
     return nullptr;
   }

@@ -87,6 +87,21 @@ def test_errors_are_reported_not_fatal():
     L.THGPUStorage_free(st)
 
 
+def test_a_pointer_to_something_else_is_rejected():
+    """A storage where a tensor belongs, and the other way round, as ctypes rejects them."""
+    from mcw_cppamp_torch_b200 import lib
+    L = lib()
+    st = L.THGPUStorage_newWithData(C.c_void_p(0x1000), 8)
+    t = L.THGPUTensor_newWithStorage1d(st, 0, 8, 1)
+    for call in (lambda: L.THGPUTensor_nDimension(st), lambda: L.THGPUStorage_size(t), lambda: L.THGPUTensor_isSameSizeAs(t, st),
+                 lambda: L.THGPUTensor_nDimension(C.c_void_p(C.cast(t, C.c_void_p).value))):
+        with pytest.raises(C.ArgumentError):
+            call()
+    assert L.THGPUTensor_nDimension(t) == 1 and L.THGPUStorage_size(st) == 8 and L.THGPUTensor_isSameSizeAs(t, t) == 1
+    L.THGPUTensor_free(t)
+    L.THGPUStorage_free(st)
+
+
 def test_compute_fails_loudly_without_a_device():
     import torch
     if torch.cuda.is_available():
