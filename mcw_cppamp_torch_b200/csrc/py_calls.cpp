@@ -14,6 +14,7 @@
 #include <tuple>
 #include <type_traits>
 #include <utility>
+#include <vector>
 
 #include "THC.h"
 
@@ -229,15 +230,15 @@ PyObject *sizes(PyObject *, PyObject *o) {
 }
 // set_view(dst, src, sizes): dst becomes a contiguous view of src's storage from src's offset on
 PyObject *set_view(PyObject *, PyObject *const *args, Py_ssize_t n) {
-  if (n != 3 || !PyTuple_Check(args[2]) || PyTuple_GET_SIZE(args[2]) > kMaxNd) {
+  if (n != 3 || !PyTuple_Check(args[2])) {
     PyErr_SetString(PyExc_TypeError, "set_view(dst, src, tuple of sizes)");
     return nullptr;
   }
   THGPUTensor *dst = tensor_arg(args[0]), *src = dst ? tensor_arg(args[1]) : nullptr;
   if (!src) return nullptr;
-  long v[kMaxNd];
+  std::vector<long> v((size_t)PyTuple_GET_SIZE(args[2]));
   THLongStorage st = {};
-  st.data = v; st.size = PyTuple_GET_SIZE(args[2]); st.refcount = 1;
+  st.data = v.data(); st.size = (long)v.size(); st.refcount = 1;
   for (long d = 0; d < st.size; d++) {
     v[d] = PyLong_AsLong(PyTuple_GET_ITEM(args[2], d));
     if (v[d] == -1 && PyErr_Occurred()) return nullptr;

@@ -87,6 +87,17 @@ def test_errors_are_reported_not_fatal():
     L.THGPUStorage_free(st)
 
 
+@pytest.mark.parametrize("dims", [1, 16, 17, 40])
+def test_views_of_any_number_of_dimensions(dims):
+    from mcw_cppamp_torch_b200 import GPUTensor, lib
+    L = lib()
+    st = L.THGPUStorage_newWithData(C.c_void_p(0x1000), 24)
+    t = GPUTensor(_ptr=L.THGPUTensor_newWithStorage1d(st, 0, 24, 1))
+    L.THGPUStorage_free(st)
+    shape = (24,) + (1,) * (dims - 1)
+    assert t.view(*shape).size() == shape
+
+
 def test_a_pointer_to_something_else_is_rejected():
     """A storage where a tensor belongs, and the other way round, as ctypes rejects them."""
     from mcw_cppamp_torch_b200 import lib
