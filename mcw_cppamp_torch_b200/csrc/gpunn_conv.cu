@@ -474,8 +474,12 @@ static void conv_forward(const ConvGeom &g, const float *in, const float *w, con
   mm::Cells u;
   const bool half = half_forward(g);
   if (ctx().math_mode != 1 && restate(g, half, u)) {
-    if (half) conv_forward_tc<true>(g, u, in, w, bias, out, finput);
-    else conv_forward_tc<false>(g, u, in, w, bias, out, finput);
+    // kept for a weight gradient of the same precision only, no other reads them back: the BF16 column matrix of the 11 x 11 / 4
+    // layer over 3 planes is 6.2 MB an image, and its weight gradient FP32-accurate
+    THGPUTensor *keep = half == half_acc_grad(g) ? finput : nullptr;
+    if (!keep) forget_planes(finput);
+    if (half) conv_forward_tc<true>(g, u, in, w, bias, out, keep);
+    else conv_forward_tc<false>(g, u, in, w, bias, out, keep);
     return;
   }
   forget_planes(finput);   // this pass leaves finput alone: what it holds belongs to an earlier input

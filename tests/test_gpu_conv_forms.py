@@ -87,3 +87,16 @@ def test_planes_of_a_finput_put_to_another_use_are_not_taken(C):
         m.accGradParameters(x, go)
         return m.gradWeight.float()
     assert np.array_equal(weight_gradient(False), weight_gradient(True))
+
+
+def test_planes_no_weight_gradient_reads_are_not_kept():
+    """BF16 mode: the first layer's column matrix is not its FP32-accurate weight gradient's input; a wide layer's planes are."""
+    import mcw_cppamp_torch_b200 as gt
+    gt.set_math_mode("bf16")
+    try:
+        first, wide = gt.nn.SpatialConvolutionMM(3, 64, 11, 11, 4, 4, 2).gpu(), gt.nn.SpatialConvolutionMM(64, 192, 5, 5, 1, 1, 2).gpu()
+        first.forward(gt.gpu(np.ones((4, 3, 63, 63), np.float32)))
+        wide.forward(gt.gpu(np.ones((4, 64, 27, 27), np.float32)))
+        assert first.finput.dim() == 0 and wide.finput.size() == (1, 4, 27, 27, 32)
+    finally:
+        gt.set_math_mode("fp32x3")
