@@ -106,6 +106,20 @@ static double windows_us(const mm::Windows &v, long Kout, bool half) {
   return mm::tc2_product_us(v.N * v.oH * v.oW, Kout, (long)v.kH * v.kW * v.C, half);
 }
 
+// Scratch of a pass.  A layer over one plane is restated over 32 channels, so a batch of a few GB may come to planes of a hundred:
+// such batches are taken in groups of images, shared out evenly, whose planes are used and given up one after the other.  A
+// group of kGroupScratch bytes is still some hundred tiles, many more than there are clusters, so that nothing is lost on
+// whole rounds and no BF16 tile is cut where it was not before.
+constexpr double kGroupScratch = 2e9, kImageScratch = 64e9;
+// Images per group of a batch whose planes take `bytes` an image, when the whole may have `allowed`.
+static long images_per_group(long N, double bytes, double allowed) {
+  if (bytes * (double)N <= allowed) return N;
+  const long fit = std::max(1l, (long)(kGroupScratch / bytes)), groups = (N + fit - 1) / fit;
+  return (N + groups - 1) / groups;
+}
+// What planes may take in one piece: twice the tensors they restate, which is no blow-up, or a tenth of the device.
+static double whole_scratch(double floats) { return std::max(16e9, 2 * 4 * floats); }
+
 // How a layer is restated for its forward and weight-gradient products: the form that costs least by the model of the product's
 // time plus one pass that writes it and one that reads it back for the weight gradient (5 TB/s).  Channel counts that
 // are multiples of a swizzle span stay direct; few planes become cells, in the extreme (3 planes, 3 x 3) columns, because
@@ -121,7 +135,7 @@ static bool restate(const ConvGeom &g, bool half, mm::Cells &best) {
     best = cells_of(g, true, true, true);
     best.Cq = 8;
     best.Cr = best.eH * best.eW * 8; best.Cs = (int)mm::padded_channels(best.Cr, true);
-    if (mm::windows_ok(forward_windows(g, best)) && (double)mm::planes_bytes(g.N, g.P, best.Cs, true) < 64e9) return true;
+    if (mm::windows_ok(forward_windows(g, best)) && (double)mm::planes_bytes(1, g.P, best.Cs, true) < kImageScratch) return true;
   }
   for (int o = 0; o < 5; o++) {
     if (o > 0 && g.N * g.oH >= (1l << 31)) continue;
@@ -131,7 +145,7 @@ static bool restate(const ConvGeom &g, bool half, mm::Cells &best) {
     if (o > 0 && u.Cs > 6144) continue;   // the channel table of cells_input_kernel
     const mm::Windows v = forward_windows(g, u);
     const double bytes = (double)mm::planes_bytes(g.N, (long)u.Hs * u.Ws, u.Cs, half);
-    if (!mm::windows_ok(v) || (o > 0 && bytes > 64e9)) continue;
+    if (!mm::windows_ok(v) || bytes > (double)g.N * kImageScratch) continue;
     const double us = windows_us(v, g.K, half) + 2 * bytes / 5e6;
     if (!found || us < best_us) { best = u; best_us = us; found = true; }
     if (o == 0 && u.Cs == u.C) break;   // nothing is padded
@@ -232,8 +246,16 @@ static const void *planes_made_from(const THGPUTensor *finput, const float *inpu
 template <bool HALF>
 static void conv_forward_tc(const ConvGeom &g, const mm::Cells &u, const float *in, const float *w, const float *bias, float *out,
                             THGPUTensor *finput) {
-  const void *act = restated_input<HALF>(g, u, in, finput);
-  window_product<HALF, false>(act, forward_windows(g, u), w, u, g.K, g.K, bias, out);
+  const double bytes = (double)mm::planes_bytes(1, (long)u.Hs * u.Ws, u.Cs, HALF), floats = (double)g.N * g.C * g.H * g.W;
+  if (finput && bytes * (double)g.N > whole_scratch(floats)) { forget_planes(finput); finput = nullptr; }
+  const long per = finput ? g.N : images_per_group(g.N, bytes, kGroupScratch);
+  for (long n0 = 0; n0 < g.N; n0 += per) {
+    WsScope ws_scope;
+    ConvGeom s = g;
+    s.N = std::min(per, g.N - n0);
+    const void *act = restated_input<HALF>(s, u, in + n0 * g.C * g.H * g.W, finput);
+    window_product<HALF, false>(act, forward_windows(s, u), w, u, g.K, g.K, bias, out + n0 * g.K * g.P);
+  }
 }
 
 // gradInput = forward pass of gradOutput's planes under the filter rotated by 180 degrees with its plane roles swapped.
@@ -487,20 +509,17 @@ static void conv_forward(const ConvGeom &g, const float *in, const float *w, con
 }
 
 // gradInput (when gin is given) and gradWeight / gradBias (when gw is) of one precision, sharing one transposition of gradOutput.
+// `act`: the input's planes, or null; w_ok / in_ok: whether the weight gradient / gradInput runs over planes.
 template <bool HALF>
-static void conv_backward_tc(const ConvGeom &g, const float *in, const float *gout, const float *w, float *gin, float *gw, float *gb, float scale,
-                             const THGPUTensor *finput) {
-  mm::Cells u;
-  const bool in_ok = gin && mm::windows_ok(grad_input_windows(g, grad_input_cells(g, HALF), HALF)), w_ok = gw && restate(g, HALF, u);
+static void conv_backward_group(const ConvGeom &g, const mm::Cells &u, bool in_ok, bool w_ok, const float *in, const void *act, const float *gout,
+                                const float *w, float *gin, float *gw, float *gb, float scale) {
+  WsScope ws_scope;
   mm::ActPlanes pgo;
   if (in_ok || w_ok) pgo = mm::make_act_planes<HALF>(gout, g.N, g.K, g.oH, g.oW, nullptr, gw != nullptr);
   if (in_ok) conv_grad_input_tc<HALF>(g, pgo, w, gin);
   else if (gin) conv_grad_input_simt(g, gout, w, gin);
   if (!gw) return;
   if (w_ok) {
-    // the input's planes: those the forward pass left in finput (as the CPU nn path reuses its finput,
-    // mcw_nn/generic/SpatialConvolutionMM.c:284-346), else made here
-    const void *act = planes_made_from(finput, in, g, u, HALF);
     if (!act) act = restated_input<HALF>(g, u, in, nullptr);
     conv_acc_grad_tc<HALF>(g, u, act, pgo, gw, scale);
   } else {
@@ -511,6 +530,28 @@ static void conv_backward_tc(const ConvGeom &g, const float *in, const float *go
     check_launch("conv_grad_bias_finish");
   } else {
     grad_bias(g, gout, gb, scale);
+  }
+}
+template <bool HALF>
+static void conv_backward_tc(const ConvGeom &g, const float *in, const float *gout, const float *w, float *gin, float *gw, float *gb, float scale,
+                             const THGPUTensor *finput) {
+  mm::Cells u;
+  const mm::Cells ui = grad_input_cells(g, HALF);
+  const bool in_ok = gin && mm::windows_ok(grad_input_windows(g, ui, HALF)), w_ok = gw && restate(g, HALF, u);
+  // the input's planes: those the forward pass left in finput (as the CPU nn path reuses its finput,
+  // mcw_nn/generic/SpatialConvolutionMM.c:284-346), else made group by group
+  const char *act = w_ok ? (const char *)planes_made_from(finput, in, g, u, HALF) : nullptr;
+  const size_t act_image = w_ok ? mm::planes_bytes(1, (long)u.Hs * u.Ws, u.Cs, HALF) : 0;
+  double bytes = 0;
+  if (in_ok || w_ok) bytes += (double)mm::planes_bytes(1, g.P, mm::padded_channels(g.K, HALF), HALF);
+  if (in_ok && !ui.direct) bytes += 4. * ui.Cr * ui.Hs * ui.Ws;
+  if (w_ok && !act) bytes += (double)act_image;
+  const long image = g.C * g.H * g.W, per = images_per_group(g.N, bytes, whole_scratch((double)g.N * (image + g.K * g.P)));
+  for (long n0 = 0; n0 < g.N; n0 += per) {
+    ConvGeom s = g;
+    s.N = std::min(per, g.N - n0);
+    conv_backward_group<HALF>(s, u, in_ok, w_ok, in ? in + n0 * image : nullptr, act ? act + n0 * act_image : nullptr, gout + n0 * g.K * g.P, w,
+                              gin ? gin + n0 * image : nullptr, gw, gb, scale);
   }
 }
 static void conv_backward(const ConvGeom &g, const float *in, const float *gout, const float *w, float *gin, float *gw, float *gb, float scale,

@@ -100,3 +100,49 @@ def test_planes_no_weight_gradient_reads_are_not_kept():
         assert first.finput.dim() == 0 and wide.finput.size() == (1, 4, 27, 27, 32)
     finally:
         gt.set_math_mode("fp32x3")
+
+
+def test_bf16_columns_in_groups_of_images():
+    """400 images of the 11 x 11 / 4 layer are 2.5 GB of columns: two groups.  Each image's result is its own, bit for bit."""
+    import mcw_cppamp_torch_b200 as gt
+    x = np.random.default_rng(1).standard_normal((400, 3, 224, 224), dtype=np.float32)
+    gt.set_math_mode("bf16")
+    try:
+        m = gt.nn.SpatialConvolutionMM(3, 64, 11, 11, 4, 4, 2).gpu()
+        out = m.forward(gt.gpu(x))
+        for n in (1, 198, 201, 397):
+            assert np.array_equal(out.narrow(1, n, 4).float(), m.clone().forward(gt.gpu(x[n - 1:n + 3])).float())
+    finally:
+        gt.set_math_mode("fp32x3")
+
+
+@pytest.mark.parametrize("stride", [1, 2])
+def test_planes_that_would_outgrow_the_batch_many_times(stride):
+    """125 images of one 1024 x 1024 plane: 0.5 GB, 17 GB as padded planes, which are made in groups and not kept.  Whole numbers,
+    whose sums are exact in any order, against the FP32 FMA engine."""
+    import mcw_cppamp_torch_b200 as gt
+    g = np.random.default_rng(stride)
+    N, K, side = 125, 2, 1024
+    x = g.integers(-1, 2, (N, 1, side, side), np.int8).astype(np.float32)
+    go = g.integers(-1, 2, (N, K, (side - 1) // stride + 1, (side - 1) // stride + 1), np.int8).astype(np.float32)
+    got = {}
+    try:
+        for mode in ("fp32x3", "simt"):
+            gt.set_math_mode(mode)
+            m = gt.nn.SpatialConvolutionMM(1, K, 3, 3, stride, stride, 1)
+            m.weight = g.integers(-2, 3, m.weight.shape).astype(np.float32) if not got else got["weight"]
+            m.bias = np.zeros_like(m.bias)
+            got["weight"] = m.weight
+            m.gpu()
+            X = gt.gpu(x)
+            out = m.forward(X)
+            m.gradWeight.zero(); m.gradBias.zero()
+            gi = m.backward(X, gt.gpu(go))
+            assert stride > 1 or m.finput.dim() == 0
+            now = [out.float(), gi.float(), m.gradWeight.float(), m.gradBias.float()]
+            if mode == "simt":
+                assert all(np.array_equal(a, b) for a, b in zip(got["planes"], now))
+            got["planes"] = now
+            del m, X, out, gi
+    finally:
+        gt.set_math_mode("fp32x3")
