@@ -198,16 +198,17 @@ __global__ void __launch_bounds__(256) reduce_rows_warp_kernel(const float *__re
 // Where a column reduction leaves its results.  With more than one slice of the reduced dimension the partials of
 // slice s go to psum / (pval, pidx)[(o * splits + s) * J + j], and the block that finishes last among the slices of its
 // columns (tickets[o * gridDim.x + blockIdx.x], zero between launches) folds them in slice order: no second launch.
+template <class I>   // positions along the reduced dimension
 struct ColOut {
   double *psum;
   float *pval;
-  int *pidx;
+  I *pidx;
   unsigned *tickets;
   float *out, *idx;
   float scale;
 };
-template <int MODE>
-__device__ __forceinline__ void cols_emit(const ColOut &w, long t, double acc, float v, int i) {
+template <int MODE, class I>
+__device__ __forceinline__ void cols_emit(const ColOut<I> &w, long t, double acc, float v, I i) {
   if (MODE == RED_SUM) {
     w.out[t] = (float)(acc * (double)w.scale);
   } else {
@@ -216,8 +217,8 @@ __device__ __forceinline__ void cols_emit(const ColOut &w, long t, double acc, f
   }
 }
 // Called by all threads of the block once its partials are written; COLS columns from j0 on belong to the block.
-template <int MODE, int COLS>
-__device__ __forceinline__ void cols_fold_if_last(const ColOut &w, long J, long j0) {
+template <int MODE, int COLS, class I>
+__device__ __forceinline__ void cols_fold_if_last(const ColOut<I> &w, long J, long j0) {
   __shared__ bool is_last;
   const int tid = threadIdx.y * 32 + threadIdx.x, splits = gridDim.y;
   __threadfence();
@@ -233,13 +234,13 @@ __device__ __forceinline__ void cols_fold_if_last(const ColOut &w, long J, long 
   // `COLS` columns, 256 / COLS interleaved groups of slices per column, folded in group order
   __shared__ double fd[256];
   __shared__ float fv[256];
-  __shared__ int fi[256];
+  __shared__ I fi[256];
   const int c = tid % COLS, grp = tid / COLS;
   constexpr int GROUPS = 256 / COLS;
   const long j = j0 + c, first = (long)blockIdx.z * splits * J + j;
   double acc = 0;
   float bv = 0;
-  int bi = -1;
+  I bi = -1;
   if (j < J) {
     if (MODE == RED_SUM) {
 #pragma unroll 8
@@ -247,7 +248,7 @@ __device__ __forceinline__ void cols_fold_if_last(const ColOut &w, long J, long 
     } else {
       for (int s0 = grp; s0 < splits; s0 += 8 * GROUPS) {
         float ov[8];
-        int oi[8];
+        I oi[8];
 #pragma unroll
         for (int u = 0; u < 8; u++) {
           const int s = s0 + u * GROUPS;
@@ -256,7 +257,7 @@ __device__ __forceinline__ void cols_fold_if_last(const ColOut &w, long J, long 
         }
 #pragma unroll
         for (int u = 0; u < 8; u++)
-          if (oi[u] >= 0 && (bi < 0 || better<MODE, int>(ov[u], oi[u], bv, bi))) { bv = ov[u]; bi = oi[u]; }
+          if (oi[u] >= 0 && (bi < 0 || better<MODE, I>(ov[u], oi[u], bv, bi))) { bv = ov[u]; bi = oi[u]; }
       }
     }
   }
@@ -269,30 +270,30 @@ __device__ __forceinline__ void cols_fold_if_last(const ColOut &w, long J, long 
         acc += fd[k * COLS + c];
       } else {
         const float ov = fv[k * COLS + c];
-        const int oi = fi[k * COLS + c];
-        if (oi >= 0 && (bi < 0 || better<MODE, int>(ov, oi, bv, bi))) { bv = ov; bi = oi; }
+        const I oi = fi[k * COLS + c];
+        if (oi >= 0 && (bi < 0 || better<MODE, I>(ov, oi, bv, bi))) { bv = ov; bi = oi; }
       }
     }
-    cols_emit<MODE>(w, (long)blockIdx.z * J + j, acc, bv, bi);
+    cols_emit<MODE, I>(w, (long)blockIdx.z * J + j, acc, bv, bi);
   }
 }
 
 // grid (ceil(J/32), splits, O); block (32, 8).
-template <int MODE>
-__global__ void __launch_bounds__(256) reduce_cols_kernel(const float *__restrict__ src, long so, long sr, long J, int R,
-                                                          int rows_per_split, const ColOut w) {
+template <int MODE, class I>
+__global__ void __launch_bounds__(256) reduce_cols_kernel(const float *__restrict__ src, long so, long sr, long J, I R,
+                                                          I rows_per_split, const ColOut<I> w) {
   pdl_begin();
   __shared__ double sd[8][33];
   __shared__ float sv[8][33];
-  __shared__ int si[8][33];
+  __shared__ I si[8][33];
   const long j = (long)blockIdx.x * 32 + threadIdx.x;
-  const int r0 = blockIdx.y * rows_per_split, r1 = min(R, r0 + rows_per_split);
+  const I r0 = blockIdx.y * rows_per_split, r1 = min(R, r0 + rows_per_split);
   const float *base = src + (long)blockIdx.z * so + j;
   double acc = 0;
   float bv = 0;
-  int bi = -1;
+  I bi = -1;
   if (j < J) {
-    int r = r0 + threadIdx.y;
+    I r = r0 + (I)threadIdx.y;
     for (; r + 56 < r1; r += 64) {  // eight independent loads in flight per thread
       float v[8];
 #pragma unroll
@@ -302,13 +303,13 @@ __global__ void __launch_bounds__(256) reduce_cols_kernel(const float *__restric
       } else {
 #pragma unroll
         for (int u = 0; u < 8; u++)
-          if (bi < 0 || better<MODE, int>(v[u], r + 8 * u, bv, bi)) { bv = v[u]; bi = r + 8 * u; }
+          if (bi < 0 || better<MODE, I>(v[u], r + 8 * u, bv, bi)) { bv = v[u]; bi = r + 8 * u; }
       }
     }
     for (; r < r1; r += 8) {
       const float v = base[(long)r * sr];
       if (MODE == RED_SUM) acc += (double)v;
-      else if (bi < 0 || better<MODE, int>(v, r, bv, bi)) { bv = v; bi = r; }
+      else if (bi < 0 || better<MODE, I>(v, r, bv, bi)) { bv = v; bi = r; }
     }
   }
   if (MODE == RED_SUM) sd[threadIdx.y][threadIdx.x] = acc;
@@ -320,46 +321,46 @@ __global__ void __launch_bounds__(256) reduce_cols_kernel(const float *__restric
     } else {
       for (int k = 1; k < 8; k++) {
         const float ov = sv[k][threadIdx.x];
-        const int oi = si[k][threadIdx.x];
-        if (oi >= 0 && (bi < 0 || better<MODE, int>(ov, oi, bv, bi))) { bv = ov; bi = oi; }
+        const I oi = si[k][threadIdx.x];
+        if (oi >= 0 && (bi < 0 || better<MODE, I>(ov, oi, bv, bi))) { bv = ov; bi = oi; }
       }
     }
     if (gridDim.y == 1) {
-      cols_emit<MODE>(w, (long)blockIdx.z * J + j, acc, bv, bi);
+      cols_emit<MODE, I>(w, (long)blockIdx.z * J + j, acc, bv, bi);
     } else {
       const long o = ((long)blockIdx.z * gridDim.y + blockIdx.y) * J + j;
       if (MODE == RED_SUM) w.psum[o] = acc;
       else { w.pval[o] = bv; w.pidx[o] = bi; }
     }
   }
-  if (gridDim.y > 1) cols_fold_if_last<MODE, 32>(w, J, (long)blockIdx.x * 32);
+  if (gridDim.y > 1) cols_fold_if_last<MODE, 32, I>(w, J, (long)blockIdx.x * 32);
 }
 
 // The same with four adjacent columns per thread (16-byte loads: a warp fetches 512 contiguous bytes per row, and
 // eight rows are requested before the first is used).  J % 4 == 0, 16-byte aligned rows.  grid (ceil(J/128), splits, O).
-template <int MODE>
-__global__ void __launch_bounds__(256) reduce_cols4_kernel(const float *__restrict__ src, long so, long sr, long J, int R,
-                                                           int rows_per_split, const ColOut w) {
+template <int MODE, class I>
+__global__ void __launch_bounds__(256) reduce_cols4_kernel(const float *__restrict__ src, long so, long sr, long J, I R,
+                                                           I rows_per_split, const ColOut<I> w) {
   pdl_begin();
   __shared__ double sd[8][129];
   __shared__ float sv[8][129];
-  __shared__ int si[8][129];
+  __shared__ I si[8][129];
   const long j = ((long)blockIdx.x * 32 + threadIdx.x) * 4;
-  const int r0 = blockIdx.y * rows_per_split, r1 = min(R, r0 + rows_per_split);
+  const I r0 = blockIdx.y * rows_per_split, r1 = min(R, r0 + rows_per_split);
   const float *base = src + (long)blockIdx.z * so + j;
   double acc[4] = {0, 0, 0, 0};
   float bv[4] = {0, 0, 0, 0};
-  int bi[4] = {-1, -1, -1, -1};
-  auto take = [&](const float4 &v, int r) {
+  I bi[4] = {-1, -1, -1, -1};
+  auto take = [&](const float4 &v, I r) {
     const float e[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
     for (int c = 0; c < 4; c++) {
       if (MODE == RED_SUM) acc[c] += (double)e[c];
-      else if (bi[c] < 0 || better<MODE, int>(e[c], r, bv[c], bi[c])) { bv[c] = e[c]; bi[c] = r; }
+      else if (bi[c] < 0 || better<MODE, I>(e[c], r, bv[c], bi[c])) { bv[c] = e[c]; bi[c] = r; }
     }
   };
   if (j < J) {
-    int r = r0 + threadIdx.y;
+    I r = r0 + (I)threadIdx.y;
     for (; r + 56 < r1; r += 64) {
       float4 v[8];
 #pragma unroll
@@ -381,7 +382,7 @@ __global__ void __launch_bounds__(256) reduce_cols4_kernel(const float *__restri
   if (col < 128 && jc < J) {
     double a = 0;
     float v = 0;
-    int i = -1;
+    I i = -1;
     if (MODE == RED_SUM) {
       a = sd[0][col];
       for (int k = 1; k < 8; k++) a += sd[k][col];
@@ -390,19 +391,19 @@ __global__ void __launch_bounds__(256) reduce_cols4_kernel(const float *__restri
       i = si[0][col];
       for (int k = 1; k < 8; k++) {
         const float ov = sv[k][col];
-        const int oi = si[k][col];
-        if (oi >= 0 && (i < 0 || better<MODE, int>(ov, oi, v, i))) { v = ov; i = oi; }
+        const I oi = si[k][col];
+        if (oi >= 0 && (i < 0 || better<MODE, I>(ov, oi, v, i))) { v = ov; i = oi; }
       }
     }
     if (gridDim.y == 1) {
-      cols_emit<MODE>(w, (long)blockIdx.z * J + jc, a, v, i);
+      cols_emit<MODE, I>(w, (long)blockIdx.z * J + jc, a, v, i);
     } else {
       const long o = ((long)blockIdx.z * gridDim.y + blockIdx.y) * J + jc;
       if (MODE == RED_SUM) w.psum[o] = a;
       else { w.pval[o] = v; w.pidx[o] = i; }
     }
   }
-  if (gridDim.y > 1) cols_fold_if_last<MODE, 128>(w, J, (long)blockIdx.x * 128);
+  if (gridDim.y > 1) cols_fold_if_last<MODE, 128, I>(w, J, (long)blockIdx.x * 128);
 }
 
 template <int MODE>
@@ -457,7 +458,6 @@ static void reduce_dim(THGPUTensor *values, THGPUTensor *indices, THGPUTensor *s
     describe(src);
   }
   THC_CHECK(O <= 65535, "outer dimension too large for the column reducer");
-  THC_CHECK(R < (1l << 31) - 4096, "reduced dimension too long");
   base = data_ptr(src);
   const int ond = src->nDimension;
   // Results go where they belong unless a destination shares memory with the source or the other destination, or is not
@@ -480,6 +480,7 @@ static void reduce_dim(THGPUTensor *values, THGPUTensor *indices, THGPUTensor *s
   float *out = place(values, direct_v, vtmp), *idx = place(indices, direct_i, itmp);
   if (sr == 1) {
     THC_CHECK(O == 1, "internal: row reduce with outer dim");
+    THC_CHECK(R < (1l << 31), "reduced dimension too long");
     const bool vec = aligned16(base) && (sj % 4 == 0);
     if (R < 512) {
       pdl_launch(reduce_rows_warp_kernel<MODE>, (unsigned)((J + 7) / 8), 256, 0, base, sj, J, (int)R, out, idx, scale);
@@ -499,19 +500,24 @@ static void reduce_dim(THGPUTensor *values, THGPUTensor *indices, THGPUTensor *s
     splits = (R + rows_per_split - 1) / rows_per_split;
     const size_t nparts = splits > 1 ? (size_t)O * splits * J : 0;
     WsScope ws_scope;
-    ColOut w = {};
-    if (splits > 1) {
-      char *scr = (char *)ws_alloc(nparts * sizeof(double));
-      w.psum = (double *)scr;
-      w.pidx = (int *)scr;
-      w.pval = (float *)scr + nparts;
-      THC_CHECK(colblocks * O <= kZeroWords, "internal: too many column ranges to split");
-      w.tickets = zero_words();
-    }
-    w.out = out; w.idx = idx; w.scale = scale;
-    dim3 grid((unsigned)colblocks, (unsigned)splits, (unsigned)O), block(32, 8);
-    if (vec4) pdl_launch(reduce_cols4_kernel<MODE>, grid, block, 0, base, so, sr, J, (int)R, (int)rows_per_split, w);
-    else pdl_launch(reduce_cols_kernel<MODE>, grid, block, 0, base, so, sr, J, (int)R, (int)rows_per_split, w);
+    const dim3 grid((unsigned)colblocks, (unsigned)splits, (unsigned)O), block(32, 8);
+    auto launch = [&](auto position) {
+      typedef decltype(position) I;
+      ColOut<I> w = {};
+      if (splits > 1) {
+        char *scr = (char *)ws_alloc(nparts * std::max(sizeof(double), sizeof(I) + sizeof(float)));
+        w.psum = (double *)scr;
+        w.pidx = (I *)scr;
+        w.pval = (float *)(scr + nparts * sizeof(I));
+        THC_CHECK(colblocks * O <= kZeroWords, "internal: too many column ranges to split");
+        w.tickets = zero_words();
+      }
+      w.out = out; w.idx = idx; w.scale = scale;
+      if (vec4) pdl_launch(reduce_cols4_kernel<MODE, I>, grid, block, 0, base, so, sr, J, (I)R, (I)rows_per_split, w);
+      else pdl_launch(reduce_cols_kernel<MODE, I>, grid, block, 0, base, so, sr, J, (I)R, (I)rows_per_split, w);
+    };
+    if (R < (1l << 31) - 4096) launch(0);   // a thread steps at most 64 rows past the end
+    else launch(0l);
     check_launch("reduce_cols");
   }
   if (vtmp.t) { resize_nd(values, ond, osize, nullptr); tensor_copy(values, vtmp); }

@@ -176,6 +176,18 @@ def test_dim_reductions(gt, shape):
     assert np.all(np.abs(X.float() - x.astype(np.float64).sum(0, keepdims=True)) <= 2.0 ** -23 * np.abs(x.astype(np.float64)).sum(0, keepdims=True))
 
 
+def test_dim_reductions_over_more_than_2_31_rows(gt):
+    rows = (1 << 31) + 8
+    x = gt.GPUTensor(rows, 2).fill(0)
+    for first, value in ((5, 1), (1 << 31, 7), (rows, 2)):
+        x.narrow(1, first, 1).fill(value)
+    x.narrow(1, rows - 6, 1).narrow(2, 2, 1).fill(-3)
+    (hi, i), (lo, k) = x.max(1), x.min(1)
+    assert hi.float().tolist() == [[7, 7]] and i.float().tolist() == [[float(1 << 31)] * 2]
+    assert lo.float().tolist() == [[0, -3]] and k.float().tolist() == [[1, float(np.float32(rows - 6))]]
+    assert x.sum(1).float().tolist() == [[10, 7]]
+
+
 @pytest.mark.parametrize("shape,dim", [((300, 64), 1), ((64, 300), 2), ((700, 64), 1)])
 def test_values_and_indices_in_one_storage(gt, shape, dim):
     """Two views of one buffer, both of which have to grow: the values are written, then the indices over what they share."""
