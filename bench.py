@@ -170,7 +170,8 @@ def cpu_alexnet_step(backend_name, n_images, seed=SEED, details=False):
     backend 'reference': the reference's own TH/nn code (oracle/_ref); conv1 (stride 4) goes through its
     stride-capable nn.SpatialConvolution, the other convs through nn.SpatialConvolutionMM.
     backend 'port': the plain-C restatement (oracle/oracle.c).  Returns (seconds, loss); with details=True
-    also the inputs, labels, initial parameters and their gradients (for the parity test of a whole step)."""
+    also the inputs, labels, initial parameters and their gradients, and each layer's input and output before the ReLU
+    (for the parity test of a whole step)."""
     import oracle
     from mcw_cppamp_torch_b200 import configs
     port, ref = oracle.port, oracle.ref
@@ -263,7 +264,8 @@ def cpu_alexnet_step(backend_name, n_images, seed=SEED, details=False):
     if details:
         # grads were appended classifier first (fc8 w, b, fc7 ..., conv5 ..., conv1): return them layer by layer
         pairs = [(grad_copy[2 * i], grad_copy[2 * i + 1]) for i in range(len(grad_copy) // 2)][::-1]
-        return dt, float(loss), {"x": x, "labels": labels, "params": init, "grads": pairs}
+        return dt, float(loss), {"x": x, "labels": labels, "params": init, "grads": pairs,
+                                 "layers": [(inp, c) for inp, c, _, _ in acts] + fc_acts}
     return dt, float(loss)
 
 

@@ -405,6 +405,41 @@ def _device_step(gt, net, params, x, labels):
     return loss, layers
 
 
+def _turned_relus(net, m, params, inp, pre, x):
+    """What the ReLU behind layer `m` lets through on one side only: a pre-activation within rounding of zero may come out
+    positive on the device and not on the CPU (`inp`: the layer's input there, `pre`: its output before the ReLU), or the
+    other way round.  One side then passes the gradient g there and the other does not, which adds g times the unit's
+    window of the input to its row of gradWeight and g to its gradBias.  Returns the sums of |g| max|window| and |g| per
+    row, zero for rows without such a unit.  Every such unit must have both values within both sides' rounding: K terms
+    of a sequential FP32 sum, and the weights times how far the two inputs are apart."""
+    w, b = (p.astype(np.float64) for p in params)
+    extra_w, extra_b = np.zeros(len(b)), np.zeros(len(b))
+    at = net.modules.index(m)
+    if at + 2 >= len(net.modules) or type(net.modules[at + 1]).__name__ != "ReLU":
+        return extra_w, extra_b
+    out = m.output.float().reshape(pre.shape)
+    turned = np.argwhere((out > 0) != (pre > 0))
+    if len(turned) == 0:
+        return extra_w, extra_b
+    g = np.abs(net.modules[at + 2].gradInput.float().reshape(pre.shape))
+    inputs = [(net.modules[at - 1].output.float() if at else x).reshape(inp.shape), inp]
+    if inp.ndim == 4:
+        p = m.padding
+        inputs = [np.pad(a, ((0, 0), (0, 0), (p, p), (p, p))) for a in inputs]
+    for unit in map(tuple, turned):
+        n, k = unit[:2]
+        if inp.ndim == 4:
+            y, z = unit[2] * m.dH, unit[3] * m.dW
+            dev, cpu = (a[n, :, y:y + m.kH, z:z + m.kW].ravel().astype(np.float64) for a in inputs)
+        else:
+            dev, cpu = (a[n].astype(np.float64) for a in inputs)
+        rounding = 2 * len(dev) * 2.0 ** -24 * (np.abs(w[k]) @ np.abs(dev) + abs(b[k])) + np.abs(w[k]) @ np.abs(dev - cpu)
+        assert max(abs(out[unit]), abs(pre[unit])) <= rounding, (at, unit, out[unit], pre[unit], rounding)
+        extra_w[k] += g[unit] * np.abs(dev).max()
+        extra_b[k] += g[unit]
+    return extra_w, extra_b
+
+
 def test_alexnet_step_matches_cpu(gt, oracle_port):
     """One whole SGD step of the AlexNet-style classifier over 8 images: the loss and all 16 gradient tensors
     against the CPU path run on the same parameters, inputs and labels -- the reference's own TH/nn code when it was
@@ -422,23 +457,16 @@ def test_alexnet_step_matches_cpu(gt, oracle_port):
     loss, layers = _device_step(gt, net, d["params"], d["x"], d["labels"])
     assert abs(loss - loss_cpu) <= 1e-5 + 1e-4 * abs(loss_cpu)
     for i, (m, (gw, gb)) in enumerate(zip(layers, d["grads"])):
-        got = m.gradWeight.float()
-        gw, gb, got_b = gw.reshape(got.shape), gb.copy(), m.gradBias.float()
-        if cpu == "port" and i == 3:
-            # The plain-C path rounds its sums otherwise than the device, and one pre-activation of this layer lies
-            # within that rounding of zero: image 7, plane 70, (4, 3) is -1.3e-8 exactly, -5.7e-8 on the CPU and +1.4e-7
-            # on the device, so one side passes the ReLU's gradient g there and the other does not.  That adds
-            # g * (the unit's window of the input) to row 70 of gradWeight and g to its gradBias; every other row keeps
-            # the bound, and row 70 gets |g| max|window| (|g|) beside it.
-            at = net.modules.index(m)
-            g = abs(float(net.modules[at + 2].gradInput.float()[7, 70, 4, 3]))
-            window = float(np.abs(net.modules[at - 1].output.float()[7, :, 3:6, 2:5]).max())
-            close_scaled(got[70], gw[70], "alexnet 8 images vs port: layer 4 gradWeight, plane 70", atol=1e-5 + g * window)
-            close_scaled(got_b[70:71], gb[70:71], "alexnet 8 images vs port: layer 4 gradBias, plane 70", atol=1e-5 + g)
-            got, gw = np.delete(got, 70, 0), np.delete(gw, 70, 0)
-            got_b, gb = np.delete(got_b, 70), np.delete(gb, 70)
-        close_scaled(got, gw, "alexnet 8 images vs %s: layer %d gradWeight" % (cpu, i + 1))
-        close_scaled(got_b, gb, "alexnet 8 images vs %s: layer %d gradBias" % (cpu, i + 1))
+        got, got_b = m.gradWeight.float(), m.gradBias.float()
+        gw = gw.reshape(got.shape)
+        extra_w, extra_b = _turned_relus(net, m, d["params"][i], *d["layers"][i], x=d["x"])
+        for k in np.flatnonzero(extra_b):
+            what = "alexnet 8 images vs %s: layer %d %%s, plane %d" % (cpu, i + 1, k)
+            close_scaled(got[k], gw[k], what % "gradWeight", atol=1e-5 + extra_w[k])
+            close_scaled(got_b[k:k + 1], gb[k:k + 1], what % "gradBias", atol=1e-5 + extra_b[k])
+        rest = np.flatnonzero(extra_b == 0)
+        close_scaled(got[rest], gw[rest], "alexnet 8 images vs %s: layer %d gradWeight" % (cpu, i + 1))
+        close_scaled(got_b[rest], gb[rest], "alexnet 8 images vs %s: layer %d gradBias" % (cpu, i + 1))
 
 
 def test_vgg_a_step_matches_cpu(gt, oracle_port):
