@@ -2,11 +2,12 @@
 //
 // The reference (gputorch/lib/THC/gpunn-impl/SpatialConvolutionMM.cpp: updateOutput :110-225,
 // updateGradInput :227-311, accGradParameters :313-429) loops over the images of a batch on the
-// host and, per image, launches im2col / col2im and a 16x16-tile SGEMM.  Here each pass is ONE
-// implicit-GEMM launch over the whole batch: the operand maps below state where element (row, k) of
-// the would-be column matrix lives in the NCHW tensor, and the matrix-multiply engine gathers it on
-// the fly.  Results follow the CPU nn semantics (mcw_nn/generic/SpatialConvolutionMM.c) and also
-// cover dW/dH > 1, which the CPU MM path rejects (:148-149) and the reference GPU path supports.
+// host and, per image, launches im2col / col2im and a 16x16-tile SGEMM.  Here each pass is one
+// implicit-GEMM product over the whole batch: the activations are brought into channels-last form once per
+// call, from which the tensor-core engine's TMA loads fetch the windows (the FP32 FMA engine gathers them
+// from the NCHW tensor element by element).  Results follow the CPU nn semantics
+// (mcw_nn/generic/SpatialConvolutionMM.c) and also cover dW/dH > 1, which the CPU MM path rejects
+// (:148-149) and the reference GPU path supports.
 #include "mm_launch.cuh"
 
 #include <unordered_map>

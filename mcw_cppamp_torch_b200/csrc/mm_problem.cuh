@@ -63,20 +63,17 @@ struct LinearMap {
 struct PixelMap {
   long count;            // < 2^31 (checked by set())
   FastDiv PP, XW;
-  unsigned p_valid;      // pixels of a plane that exist; indices in [p_valid, PP) are padding (zeros)
   long img_stride, y_stride, x_stride, off0;
   int sy, y0, sx, x0;
-  void set(long count_, long pp, long xw, long pp_valid = -1) {
+  void set(long count_, long pp, long xw) {
     THC_CHECK(count_ < (1l << 31) && pp > 0 && xw > 0, "problem too large for 32-bit pixel indices");
     count = count_; PP = FastDiv::make(pp); XW = FastDiv::make(xw);
-    p_valid = (unsigned)(pp_valid < 0 ? pp : pp_valid);
   }
   __device__ __forceinline__ Info operator()(long idx) const {
     Info r;
     if (idx >= count) { r.off = 0; r.y = kInvalid; r.x = 0; return r; }
     unsigned img, p, y, x;
     PP.divmod((unsigned)idx, img, p);
-    if (p >= p_valid) { r.off = 0; r.y = kInvalid; r.x = 0; return r; }
     XW.divmod(p, y, x);
     r.off = (long)img * img_stride + (long)y * y_stride + (long)x * x_stride + off0;
     r.y = (int)y * sy + y0;

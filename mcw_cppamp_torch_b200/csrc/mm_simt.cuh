@@ -1,5 +1,5 @@
 // FP32 FMA engine for mm::Problem ("simt" math mode): 64x64 output tile per 256-thread block, 4x4
-// micro-tile per thread, operands gathered through the same row / k maps as the tensor-core engine.
+// micro-tile per thread, operands gathered from the tensors as they lie through row / k maps.
 // It is the exact-FP32 alternative to the 3xTF32 path and the on-device cross-check for it; it
 // stands where the reference had its 16x16-tile one-output-per-thread SGEMM kernels
 // (gputorch/lib/THC/THCBlas.cpp:10-246).
