@@ -88,7 +88,7 @@ static EncodeIm2colFn encode_im2col_fn() {
 // about 0.06 us of device-wide write + read-back, which the L2 holds; the folding kernel, queued as a programmatic
 // dependent, 2 us.  Every slice keeps at least three k tiles, the pipeline fill of an item.  (With six tiles, 0.17 and 5 us,
 // which fitted launches in ordinary order, products of few tiles left most clusters idle: the small convolution blocks
-// 208 -> 202 and 91.7 -> 86.0 us, the VGG-A-style classifier over 13 images 1955 -> 1924.)
+// 208 -> 202 and 91.7 -> 86.0 us; the VGG-A-style classifier over 13 images moved within its noise, 1.92 - 1.95 ms.)
 static int choose_tail_splits(long tail, long ktiles, int slots, double tile_us) {
   int best = 1;
   double best_us = tile_us * (double)ktiles;

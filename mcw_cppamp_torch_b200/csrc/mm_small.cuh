@@ -336,8 +336,10 @@ __global__ void __launch_bounds__(SM_THREADS) small_kernel(const SmallProblem p)
 // the matrix and every (8 / groups)-th 128-k chunk, the RA x UNROLL 16-byte loads of UNROLL chunks in flight before the
 // first multiply-add (8 to 16, as registers allow); the 8 warps of a block are `groups` sets of rows times 8 / groups
 // interleaved slices of k, whose sums meet in shared memory, so no second launch or workspace follows.  The warps of a slice
-// read the same chunk of the few rows at about the same time, which the L1 serves.  9216 -> 4096 outputs (151 MB): 42.5 -> 26 us
-// for one and two rows (5.8 TB/s), 33 for four; 4096 -> 1000: 12.5 -> 6.5; 512 -> 512: 5.0 -> 3.3, against the tiles above.
+// read the same chunk of the few rows at about the same time, which the L1 serves.  In a loop over one
+// matrix, against the tiles above: 9216 -> 4096 outputs (151 MB) 42.5 -> 26 us for one and two rows (5.8 TB/s), 33 for four;
+// 4096 -> 1000 (16 MB, which then stays in L2) 12.5 -> 6.5; 512 -> 512 5.0 -> 3.3.  With the matrix in DRAM: 32, 18 (4096 -> 4096) and
+// 11 us, i.e. 4.7, 3.7 and 1.5 TB/s: the shorter the launch, the more of it is its start.
 template <int R, int RA, int UNROLL>
 __global__ void __launch_bounds__(256) few_rows_kernel(const SmallProblem p, int groups) {
   pdl_begin();
