@@ -14,7 +14,6 @@
 #include <tuple>
 #include <type_traits>
 #include <utility>
-#include <vector>
 
 #include "THC.h"
 
@@ -236,17 +235,24 @@ PyObject *set_view(PyObject *, PyObject *const *args, Py_ssize_t n) {
   }
   THGPUTensor *dst = tensor_arg(args[0]), *src = dst ? tensor_arg(args[1]) : nullptr;
   if (!src) return nullptr;
-  std::vector<long> v((size_t)PyTuple_GET_SIZE(args[2]));
+  const Py_ssize_t nd = PyTuple_GET_SIZE(args[2]);
+  long few[kMaxNd], *v = nd <= kMaxNd ? few : PyMem_New(long, nd);
+  if (!v) return PyErr_NoMemory();
   THLongStorage st = {};
-  st.data = v.data(); st.size = (long)v.size(); st.refcount = 1;
-  for (long d = 0; d < st.size; d++) {
+  st.data = v; st.size = nd; st.refcount = 1;
+  bool ok = true;
+  for (long d = 0; ok && d < nd; d++) {
     v[d] = PyLong_AsLong(PyTuple_GET_ITEM(args[2], d));
-    if (v[d] == -1 && PyErr_Occurred()) return nullptr;
+    ok = !(v[d] == -1 && PyErr_Occurred());
   }
-  Py_BEGIN_ALLOW_THREADS
-  g_set_storage(dst, src->storage, src->storageOffset, &st, nullptr);
-  Py_END_ALLOW_THREADS
-  if (raised()) return nullptr;
+  if (ok) {
+    Py_BEGIN_ALLOW_THREADS
+    g_set_storage(dst, src->storage, src->storageOffset, &st, nullptr);
+    Py_END_ALLOW_THREADS
+    ok = !raised();
+  }
+  if (v != few) PyMem_Free(v);
+  if (!ok) return nullptr;
   Py_RETURN_NONE;
 }
 // A dense float32 array as a TH tensor; false: not one (the caller takes the general route).
