@@ -138,18 +138,25 @@ static bool restate(const ConvGeom &g, bool half, mm::Cells &best) {
     best.Cr = best.eH * best.eW * 8; best.Cs = (int)mm::padded_channels(best.Cr, true);
     if (mm::windows_ok(forward_windows(g, best)) && (double)mm::planes_bytes(1, g.P, best.Cs, true) < kImageScratch) return true;
   }
-  for (int o = 0; o < 5; o++) {
-    if (o > 0 && g.N * g.oH >= (1l << 31)) continue;
-    if ((o == 1 && g.dH == 1 && g.dW == 1) || (o == 2 && g.kW == 1) || (o == 3 && g.kH == 1)) continue;   // the same as another
-    if (o && g.dH * (long)g.kH * g.dW * g.kW * g.C > (1l << 28)) continue;
-    const mm::Cells u = o == 0 ? direct_cells(g, half) : cells_of(g, o >= 3, o == 2 || o == 4, half);
-    if (o > 0 && u.Cs > 6144) continue;   // the channel table of cells_input_kernel
-    const mm::Windows v = forward_windows(g, u);
-    const double bytes = (double)mm::planes_bytes(g.N, (long)u.Hs * u.Ws, u.Cs, half);
-    if (!mm::windows_ok(v) || bytes > (double)g.N * kImageScratch) continue;
-    const double us = windows_us(v, g.K, half) + 2 * bytes / 5e6;
-    if (!found || us < best_us) { best = u; best_us = us; found = true; }
-    if (o == 0 && u.Cs == u.C) break;   // nothing is padded
+  // Forms of more channels than the table of cells_input_kernel holds only where there is no other: strides beyond the eight
+  // that a window map takes, over many planes, and windows beyond 128 taps (as columns).  64 planes under 16 x 16 / 16, 16 images:
+  // 300 us forward and 155 for the weight gradient, 1911 and 1870 on the FMA engine; 131 x 131 taps over 16 planes: 6.6 and
+  // 2.2 ms, 13.6 and 11.9 there.
+  for (const long most : {(long)mm::kCellTable, 1l << 28}) {
+    for (int o = 0; o < 5; o++) {
+      if (o > 0 && g.N * g.oH >= (1l << 31)) continue;
+      if ((o == 1 && g.dH == 1 && g.dW == 1) || (o == 2 && g.kW == 1) || (o == 3 && g.kH == 1)) continue;   // the same as another
+      if (o && g.dH * (long)g.kH * g.dW * g.kW * g.C > (1l << 28)) continue;
+      const mm::Cells u = o == 0 ? direct_cells(g, half) : cells_of(g, o >= 3, o == 2 || o == 4, half);
+      if (o > 0 && (u.Cs > most || (long)u.Ws * u.Cs >= (1l << 31))) continue;
+      const mm::Windows v = forward_windows(g, u);
+      const double bytes = (double)mm::planes_bytes(g.N, (long)u.Hs * u.Ws, u.Cs, half);
+      if (!mm::windows_ok(v) || bytes > (double)g.N * kImageScratch) continue;
+      const double us = windows_us(v, g.K, half) + 2 * bytes / 5e6;
+      if (!found || us < best_us) { best = u; best_us = us; found = true; }
+      if (o == 0 && u.Cs == u.C) break;   // nothing is padded
+    }
+    if (found) break;
   }
   return found;
 }
@@ -225,7 +232,8 @@ static const void *restated_input(const ConvGeom &g, const mm::Cells &u, const f
   // 224 x 224 image: 8.4 us with one block each)
   const long rows = g.N * u.Hs, chunks = (long)u.Ws * u.Cs / (HALF ? 8 : 4);
   const unsigned parts = (unsigned)std::max(1l, std::min((chunks + 255) / 256, 4l * ctx().sm_count / rows));
-  pdl_launch(mm::cells_input_kernel<HALF>, dim3((unsigned)rows, parts), 256, sizeof(int2) * u.Cs, in, dst, u);
+  if (u.Cs <= mm::kCellTable) pdl_launch(mm::cells_input_kernel<HALF, true>, dim3((unsigned)rows, parts), 256, sizeof(int2) * u.Cs, in, dst, u);
+  else pdl_launch(mm::cells_input_kernel<HALF, false>, dim3((unsigned)rows, parts), 256, 0, in, dst, u);
   check_launch("cells_input");
   return dst;
 }

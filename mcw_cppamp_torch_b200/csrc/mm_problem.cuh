@@ -319,17 +319,21 @@ struct Cells {
 };
 
 // S of one image row per block.  A thread produces 16 bytes of a pixel: 4 FP32 or 8 BF16 channels, whose source offsets it
-// looks up in a table; neighbouring threads hold neighbouring channels, i.e. neighbouring columns of a few input rows.
-template <bool HALF>
+// looks up in a table; neighbouring threads hold neighbouring channels, i.e. neighbouring columns of a few input rows.  More
+// channels than the table holds (kCellTable: 48 KB of it) are found by division, once per 16 bytes.
+constexpr int kCellTable = 6144;
+template <bool HALF, bool TABLE>
 static __global__ void __launch_bounds__(256) cells_input_kernel(const float *__restrict__ in, void *__restrict__ S, const Cells u) {
   pdl_begin();
   constexpr int V = HALF ? 8 : 4;
   extern __shared__ int2 chan_src[];      // per channel: offset in the image, (dy << 16 | dx) or -1
-  for (int ch = threadIdx.x; ch < u.Cs; ch += blockDim.x) {
-    int c, dy, dx;
-    chan_src[ch] = u.channel(ch, c, dy, dx) ? make_int2((c * u.H + dy) * u.W + dx, dy << 16 | dx) : make_int2(0, -1);
+  if constexpr (TABLE) {
+    for (int ch = threadIdx.x; ch < u.Cs; ch += blockDim.x) {
+      int c, dy, dx;
+      chan_src[ch] = u.channel(ch, c, dy, dx) ? make_int2((c * u.H + dy) * u.W + dx, dy << 16 | dx) : make_int2(0, -1);
+    }
+    __syncthreads();
   }
-  __syncthreads();
   const long n = blockIdx.x / u.Hs;
   const int Y = (int)(blockIdx.x - n * u.Hs);
   const int q = u.Cs / V, chunks = u.Ws * q, y0 = Y * u.dH - u.pad;
@@ -337,13 +341,28 @@ static __global__ void __launch_bounds__(256) cells_input_kernel(const float *__
   uint4 *dst = reinterpret_cast<uint4 *>(S) + ((n * u.Hs + Y) * u.Ws) * (long)q;
   for (int o = blockIdx.y * blockDim.x + threadIdx.x; o < chunks; o += gridDim.y * blockDim.x) {
     const int X = o / q, ch0 = (o - X * q) * V, x0 = X * u.dW - u.pad;
-    const float *base = img + (long)y0 * u.W + x0;
     float v[V];
+    if constexpr (TABLE) {
+      const float *base = img + (long)y0 * u.W + x0;
 #pragma unroll
-    for (int e = 0; e < V; e++) {
-      const int2 s = chan_src[ch0 + e];
-      const int y = y0 + (s.y >> 16), x = x0 + (s.y & 0xffff);
-      v[e] = s.y >= 0 && (unsigned)y < (unsigned)u.H && (unsigned)x < (unsigned)u.W ? __ldg(base + s.x) : 0.f;
+      for (int e = 0; e < V; e++) {
+        const int2 s = chan_src[ch0 + e];
+        const int y = y0 + (s.y >> 16), x = x0 + (s.y & 0xffff);
+        v[e] = s.y >= 0 && (unsigned)y < (unsigned)u.H && (unsigned)x < (unsigned)u.W ? __ldg(base + s.x) : 0.f;
+      }
+    } else {
+      int c, dy, dx;
+      u.channel(ch0, c, dy, dx);
+#pragma unroll
+      for (int e = 0; e < V; e++) {
+        const int y = y0 + dy, x = x0 + dx;
+        v[e] = ch0 + e < u.Cr && c < u.C && (unsigned)y < (unsigned)u.H && (unsigned)x < (unsigned)u.W
+                   ? __ldg(img + ((long)c * u.H + y) * u.W + x) : 0.f;
+        if (++c == u.Cq) {
+          c = 0;
+          if (++dx == u.eW) { dx = 0; dy++; }
+        }
+      }
     }
     if constexpr (HALF) {
       __nv_bfloat162 h[4];

@@ -24,6 +24,9 @@ CASES = [
     (2, 8, 6, 5, 40, 2, 3, 1, 1, 3),       # padding not below the window
     (1, 2, 4, 4, 1, 4, 4, 1, 1, 0),        # one output
     (150, 3, 6, 6, 16, 3, 3, 1, 1, 0),
+    (2, 32, 32, 48, 40, 16, 16, 16, 16, 0),   # cells of more channels than the table holds
+    (1, 44, 37, 29, 140, 14, 13, 13, 12, 2),  # the same, ragged
+    (1, 7, 135, 140, 34, 131, 133, 1, 1, 0),  # a window beyond what a window map takes: columns
 ]
 
 
