@@ -109,3 +109,24 @@ def test_few_rows(gt, rows, inputs, outputs):
     r = gt.gpu(c).addmm(0.5, 0.75, gt.gpu(x), gt.gpu(w).t()).float()
     exact = 0.5 * c.astype(np.float64) + 0.75 * (x.astype(np.float64) @ w.T.astype(np.float64))
     assert np.all(np.abs(r - exact) <= bound(x, w.T, inputs) + 2.0 ** -22 * (np.abs(exact) + np.abs(c)))
+
+
+def test_accumulating_costs_no_round_trip_per_element(gt):
+    """1574 x 1276 x 2, bound by its result: 15 us overwriting it, 18 adding to it (53 with a load behind every store)."""
+    import torch
+    a, b, r = gt.GPUTensor(1574, 2).fill(1), gt.GPUTensor(2, 1276).fill(1), gt.GPUTensor(1574, 1276).fill(0)
+    stream = torch.cuda.ExternalStream(gt.lib().THGPUGetStream())
+
+    def us(beta):
+        times = []
+        for _ in range(7):
+            t0, t1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            t0.record(stream)
+            for _ in range(20):
+                r.addmm(beta, 1.0, a, b)
+            t1.record(stream)
+            t1.synchronize()
+            times.append(t0.elapsed_time(t1) * 50)
+        return sorted(times)[3]
+    us(0.0)
+    assert us(1.0) < 2 * us(0.0)
