@@ -267,6 +267,40 @@ static void conv_forward_tc(const ConvGeom &g, const mm::Cells &u, const float *
   }
 }
 
+// Wt[c][(ko, i, j)] = W[ko][(c, i, j)]: the weight matrix as the gathered gradInput product reads it; `turned`: with the filter rotated
+// by 180 degrees, the weights of gradInput as a layer over gradOutput.
+static __global__ void __launch_bounds__(256) transpose_weight_kernel(const float *__restrict__ w, float *__restrict__ wt,
+                                                                      long K, long C, long kHW, bool turned) {
+  pdl_begin();
+  const long total = K * C * kHW;
+  const long nthreads = (long)gridDim.x * blockDim.x;
+  for (long t = (long)blockIdx.x * blockDim.x + threadIdx.x; t < total; t += nthreads) {
+    const long tap = t % kHW, q = t / kHW, ko = q % K, c = q / K;
+    wt[t] = w[(ko * C + c) * kHW + (turned ? kHW - 1 - tap : tap)];
+  }
+}
+static const float *transposed_weight(const ConvGeom &g, const float *w, bool turned) {
+  const long kHW = (long)g.kH * g.kW, total = g.C * g.K * kHW;
+  float *wt = (float *)ws_alloc(sizeof(float) * total);
+  pdl_launch(transpose_weight_kernel, (unsigned)std::min<long>((total + 255) / 256, ctx().sm_count * 8l), 256, 0, w, wt, g.K, g.C, kHW, turned);
+  check_launch("transpose_weight");
+  return wt;
+}
+
+// gradInput of a layer with few output planes stated as a layer of its own, whose input is gradOutput: padding two planes to a span of
+// channels multiplies the product by 16, which restate() knows to avoid (13 x 13 taps, 271 <- 2 planes of 110 x 118, four images in
+// BF16: 915 us over padded planes, 177 so; 9 x 9, 32 <- 2, 46 of 87 x 88: 516 and 121).  False: the padded planes cost less.
+static bool grad_input_layer(const ConvGeom &g, bool half, ConvGeom &t, mm::Cells &u) {
+  if (g.dH != 1 || g.dW != 1 || g.kH != g.kW || g.pad >= g.kH || 2 * g.K > mm::padded_channels(g.K, half)) return false;
+  t = g;
+  t.C = g.K; t.K = g.C; t.H = g.oH; t.W = g.oW; t.oH = g.H; t.oW = g.W; t.P = g.H * g.W;
+  t.pad = g.kH - 1 - g.pad; t.R = g.K * g.kH * g.kW;
+  if (!restate(t, half, u) || u.direct) return false;
+  const double bytes = (double)mm::planes_bytes(g.N, (long)u.Hs * u.Ws, u.Cs, half);
+  const double own = windows_us(forward_windows(t, u), t.K, half) + 2 * bytes / 5e6 + 10;   // and two launches more
+  return own < windows_us(grad_input_windows(g, grad_input_cells(g, half), half), g.C, half);
+}
+
 // gradInput = forward pass of gradOutput's planes under the filter rotated by 180 degrees with its plane roles swapped.
 template <bool HALF>
 static void conv_grad_input_tc(const ConvGeom &g, const mm::ActPlanes &pgo, const float *w, float *gin) {
@@ -387,24 +421,10 @@ static void conv_forward_simt(const ConvGeom &g, const float *in, const float *w
   launch_simt(p);
 }
 
-// Wt[c][(ko, i, j)] = W[ko][(c, i, j)]: the weight matrix as the gathered gradInput product reads it.
-static __global__ void __launch_bounds__(256) transpose_weight_kernel(const float *__restrict__ w, float *__restrict__ wt,
-                                                                      long K, long C, long kHW) {
-  pdl_begin();
-  const long total = K * C * kHW;
-  const long nthreads = (long)gridDim.x * blockDim.x;
-  for (long t = (long)blockIdx.x * blockDim.x + threadIdx.x; t < total; t += nthreads) {
-    const long tap = t % kHW, q = t / kHW, ko = q % K, c = q / K;
-    wt[t] = w[(ko * C + c) * kHW + tap];
-  }
-}
-
 static void conv_grad_input_simt(const ConvGeom &g, const float *gout, const float *w, float *gin) {
   using namespace mm;
   const long kHW = (long)g.kH * g.kW, Kd = g.K * kHW;
-  float *wt = (float *)ws_alloc(sizeof(float) * g.C * Kd);
-  pdl_launch(transpose_weight_kernel, (unsigned)std::min<long>((g.C * Kd + 255) / 256, ctx().sm_count * 8l), 256, 0, w, wt, g.K, g.C, kHW);
-  check_launch("transpose_weight");
+  const float *wt = transposed_weight(g, w, false);
   // rows = input pixels, k = (ko, i, j); only taps with (h + pad - i) % dH == 0 contribute
   Problem<Operand<PixelMap, TapMap, 2>, Operand<LinearMap, LinearMap, 0>> p;
   PixelMap rows;
@@ -523,6 +543,13 @@ template <bool HALF>
 static void conv_backward_group(const ConvGeom &g, const mm::Cells &u, bool in_ok, bool w_ok, const float *in, const void *act, const float *gout,
                                 const float *w, float *gin, float *gw, float *gb, float scale) {
   WsScope ws_scope;
+  ConvGeom t;
+  mm::Cells ut;
+  if (gin && grad_input_layer(g, HALF, t, ut)) {
+    conv_forward_tc<HALF>(t, ut, gout, transposed_weight(g, w, true), nullptr, gin, nullptr);
+    gin = nullptr;
+    in_ok = false;
+  }
   mm::ActPlanes pgo;
   if (in_ok || w_ok) pgo = mm::make_act_planes<HALF>(gout, g.N, g.K, g.oH, g.oW, nullptr, gw != nullptr);
   if (in_ok) conv_grad_input_tc<HALF>(g, pgo, w, gin);

@@ -26,6 +26,9 @@ CASES = [
     (150, 3, 6, 6, 16, 3, 3, 1, 1, 0),
     (2, 32, 32, 48, 40, 16, 16, 16, 16, 0),   # cells of more channels than the table holds
     (1, 44, 37, 29, 140, 14, 13, 13, 12, 2),  # the same, ragged
+    (2, 60, 40, 37, 2, 13, 13, 1, 1, 6),      # few output planes: gradInput as a layer over gradOutput
+    (3, 33, 31, 30, 1, 9, 9, 1, 1, 0),
+    (2, 70, 28, 33, 9, 7, 7, 1, 1, 6),
     (1, 7, 135, 140, 34, 131, 133, 1, 1, 0),  # a window beyond what a window map takes: columns
 ]
 
@@ -149,3 +152,23 @@ def test_planes_that_would_outgrow_the_batch_many_times(stride):
             del m, X, out, gi
     finally:
         gt.set_math_mode("fp32x3")
+
+
+def test_grad_input_of_few_output_planes_does_not_pay_for_padding():
+    """9 x 9 taps, 32 <- K planes, 46 of 87 x 88: 516 us for 32 planes and as much for two padded to 32; 121 as a layer over two."""
+    import torch
+    import mcw_cppamp_torch_b200 as gt
+    stream = torch.cuda.ExternalStream(gt.lib().THGPUGetStream())
+
+    def us(K):
+        m = gt.nn.SpatialConvolutionMM(32, K, 9, 9, 1, 1, 4).gpu()
+        x, go, times = gt.GPUTensor(46, 32, 87, 88).fill(1), gt.GPUTensor(46, K, 87, 88).fill(1), []
+        for _ in range(7):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            a.record(stream)
+            m.updateGradInput(x, go)
+            b.record(stream)
+            b.synchronize()
+            times.append(a.elapsed_time(b) * 1e3)
+        return sorted(times[2:])[2]
+    assert us(2) < us(32) / 2
