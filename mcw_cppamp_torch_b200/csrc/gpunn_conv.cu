@@ -11,6 +11,7 @@
 #include "mm_launch.cuh"
 
 #include <unordered_map>
+#include <utility>
 
 namespace thc {
 
@@ -48,12 +49,12 @@ static ConvGeom conv_geom(const THGPUTensor *input, const THGPUTensor *weight, i
 // that does not write `finput` forgets the entry, so planes of an earlier pass are never taken for fresh ones.
 // Keyed by the address of finput's data; one table per host thread, as the rest of the library's state.
 namespace {
-struct PlaneStamp { const float *input; bool half; long N, C, H, W, K; int kH, kW, dH, dW, pad; };
+struct PlaneStamp { const float *input; int prec; long N, C, H, W, K; int kH, kW, dH, dW, pad; };
 thread_local std::unordered_map<const float *, PlaneStamp> g_plane_stamps;
-void stamp_planes(const THGPUTensor *finput, const float *input, const ConvGeom &g, bool half) {
+void stamp_planes(const THGPUTensor *finput, const float *input, const ConvGeom &g, int prec) {
   if (!finput || !finput->storage) return;
   if (g_plane_stamps.size() > 4096) g_plane_stamps.clear();
-  g_plane_stamps[data_ptr(finput)] = PlaneStamp{input, half, g.N, g.C, g.H, g.W, g.K, g.kH, g.kW, g.dH, g.dW, g.pad};
+  g_plane_stamps[data_ptr(finput)] = PlaneStamp{input, prec, g.N, g.C, g.H, g.W, g.K, g.kH, g.kW, g.dH, g.dW, g.pad};
 }
 void forget_planes(const THGPUTensor *finput) {
   if (finput && finput->storage) g_plane_stamps.erase(data_ptr(finput));
@@ -64,23 +65,23 @@ void forget_planes(const THGPUTensor *finput) {
 // Tensor-core passes.  The activations are brought into channels-last form once per call (planes, or cells: see mm::Cells),
 // channel counts padded to whole swizzle spans, after which every operand tile of the three products is one TMA load.
 
-static mm::Cells cells_of(const ConvGeom &g, bool unfoldH, bool unfoldW, bool half) {
+static mm::Cells cells_of(const ConvGeom &g, bool unfoldH, bool unfoldW, int prec) {
   mm::Cells u;
   u.C = (int)g.C; u.kH = g.kH; u.kW = g.kW; u.dH = g.dH; u.dW = g.dW; u.pad = g.pad; u.H = (int)g.H; u.W = (int)g.W;
   u.eH = unfoldH ? g.kH : std::min(g.dH, g.kH); u.eW = unfoldW ? g.kW : std::min(g.dW, g.kW);
   u.kHs = unfoldH ? 1 : (g.kH + g.dH - 1) / g.dH; u.kWs = unfoldW ? 1 : (g.kW + g.dW - 1) / g.dW;
   u.stepH = g.dH; u.stepW = g.dW;
   const int e = u.eH * u.eW, q4 = (u.C + 3) / 4 * 4;
-  u.Cq = mm::padded_channels(e * q4, half) == mm::padded_channels(e * u.C, half) ? q4 : u.C;
-  u.Cr = e * u.Cq; u.Cs = (int)mm::padded_channels(u.Cr, half);
+  u.Cq = mm::padded_channels(e * q4, prec) == mm::padded_channels(e * u.C, prec) ? q4 : u.C;
+  u.Cr = e * u.Cq; u.Cs = (int)mm::padded_channels(u.Cr, prec);
   u.Hs = (int)g.oH + u.kHs - 1; u.Ws = (int)g.oW + u.kWs - 1;
   u.direct = false;
   return u;
 }
-static mm::Cells direct_cells(const ConvGeom &g, bool half) {
-  mm::Cells u = cells_of(g, false, false, half);
+static mm::Cells direct_cells(const ConvGeom &g, int prec) {
+  mm::Cells u = cells_of(g, false, false, prec);
   u.eH = u.eW = 1; u.kHs = g.kH; u.kWs = g.kW; u.stepH = u.stepW = 1;
-  u.Cq = u.Cr = u.C; u.Cs = (int)mm::padded_channels(u.C, half);
+  u.Cq = u.Cr = u.C; u.Cs = (int)mm::padded_channels(u.C, prec);
   u.Hs = (int)g.H; u.Ws = (int)g.W;
   u.direct = true;
   return u;
@@ -92,19 +93,19 @@ static mm::Windows forward_windows(const ConvGeom &g, const mm::Cells &u) {
 }
 
 // A tcgen05.mma occupies the tensor pipe about 80 cycles however narrow it is, so with up to 64 output planes two horizontally
-// adjacent output pixels share a row of the product (pixel-pair mode): half the rows, twice the columns, a window one
+// adjacent output pixels share a row of the product (pixel-pair mode): prec the rows, twice the columns, a window one
 // stride wider.  Worth it when the wider window costs less than the rows save; not for windows of one column.
 // FP32 only: BF16 products are bound by their operands' bytes, which the wider window adds to.
-static bool pair_windows(const mm::Windows &v, long Kout, bool half, mm::Windows &p) {
-  if (half) return false;
+static bool pair_windows(const mm::Windows &v, long Kout, int prec, mm::Windows &p) {
+  if (prec == mm::kBf16) return false;
   p = v;
   p.oW = (v.oW + 1) / 2; p.dW = 2 * v.dW; p.kW = v.kW + v.dW;
   return Kout <= 64 && Kout > 16 && v.oW >= 2 && 4 * p.kW <= 7 * v.kW && v.N * v.oH * p.oW > 128 && mm::windows_ok(p);
 }
-static double windows_us(const mm::Windows &v, long Kout, bool half) {
+static double windows_us(const mm::Windows &v, long Kout, int prec) {
   mm::Windows p;
-  if (pair_windows(v, Kout, half, p)) return mm::tc2_product_us(p.N * p.oH * p.oW, 2 * Kout, (long)p.kH * p.kW * p.C, half);
-  return mm::tc2_product_us(v.N * v.oH * v.oW, Kout, (long)v.kH * v.kW * v.C, half);
+  if (pair_windows(v, Kout, prec, p)) return mm::tc2_product_us(p.N * p.oH * p.oW, 2 * Kout, (long)p.kH * p.kW * p.C, prec);
+  return mm::tc2_product_us(v.N * v.oH * v.oW, Kout, (long)v.kH * v.kW * v.C, prec);
 }
 
 // Scratch of a pass.  A layer over one plane is restated over 32 channels, so a batch of a few GB may come to planes of a hundred:
@@ -125,18 +126,18 @@ static double whole_scratch(double floats) { return std::max(16e9, 2 * 4 * float
 // time plus one pass that writes it and one that reads it back for the weight gradient (5 TB/s).  Channel counts that
 // are multiples of a swizzle span stay direct; few planes become cells, in the extreme (3 planes, 3 x 3) columns, because
 // padding 3 planes to 32 would multiply the products tenfold.  False: no form that TMA can express.
-static bool restate(const ConvGeom &g, bool half, mm::Cells &best) {
+static bool restate(const ConvGeom &g, int prec, mm::Cells &best) {
   if (g.K * g.R >= (1l << 31) || g.N * g.P >= (1l << 31)) return false;
   double best_us = 0;
   bool found = false;
-  if (half && g.C <= 8 && (long)g.kH * g.kW * 8 <= 6144) {
+  if (prec == mm::kBf16 && g.C <= 8 && (long)g.kH * g.kW * 8 <= 6144) {
     // Few planes in BF16: the column matrix with eight planes per tap, k = (tap, plane).  The reduction keeps that order
     // because a step in this mode rounds every layer's result to BF16 again, which turns a different order's last bit into
     // other masks and maxima further up.
-    best = cells_of(g, true, true, true);
+    best = cells_of(g, true, true, mm::kBf16);
     best.Cq = 8;
-    best.Cr = best.eH * best.eW * 8; best.Cs = (int)mm::padded_channels(best.Cr, true);
-    if (mm::windows_ok(forward_windows(g, best)) && (double)mm::planes_bytes(1, g.P, best.Cs, true) < kImageScratch) return true;
+    best.Cr = best.eH * best.eW * 8; best.Cs = (int)mm::padded_channels(best.Cr, mm::kBf16);
+    if (mm::windows_ok(forward_windows(g, best)) && (double)mm::planes_bytes(1, g.P, best.Cs, mm::kBf16) < kImageScratch) return true;
   }
   // Forms of more channels than the table of cells_input_kernel holds only where there is no other: strides beyond the eight
   // that a window map takes, over many planes, and windows beyond 128 taps (as columns).  64 planes under 16 x 16 / 16, 16 images:
@@ -147,12 +148,12 @@ static bool restate(const ConvGeom &g, bool half, mm::Cells &best) {
       if (o > 0 && g.N * g.oH >= (1l << 31)) continue;
       if ((o == 1 && g.dH == 1 && g.dW == 1) || (o == 2 && g.kW == 1) || (o == 3 && g.kH == 1)) continue;   // the same as another
       if (o && g.dH * (long)g.kH * g.dW * g.kW * g.C > (1l << 28)) continue;
-      const mm::Cells u = o == 0 ? direct_cells(g, half) : cells_of(g, o >= 3, o == 2 || o == 4, half);
+      const mm::Cells u = o == 0 ? direct_cells(g, prec) : cells_of(g, o >= 3, o == 2 || o == 4, prec);
       if (o > 0 && (u.Cs > most || (long)u.Ws * u.Cs >= (1l << 31))) continue;
       const mm::Windows v = forward_windows(g, u);
-      const double bytes = (double)mm::planes_bytes(g.N, (long)u.Hs * u.Ws, u.Cs, half);
+      const double bytes = (double)mm::planes_bytes(g.N, (long)u.Hs * u.Ws, u.Cs, prec);
       if (!mm::windows_ok(v) || bytes > (double)g.N * kImageScratch) continue;
-      const double us = windows_us(v, g.K, half) + 2 * bytes / 5e6;
+      const double us = windows_us(v, g.K, prec) + 2 * bytes / 5e6;
       if (!found || us < best_us) { best = u; best_us = us; found = true; }
       if (o == 0 && u.Cs == u.C) break;   // nothing is padded
     }
@@ -163,59 +164,65 @@ static bool restate(const ConvGeom &g, bool half, mm::Cells &best) {
 
 // Whether the gradInput product can be stated: over gradOutput's planes, stride 1 as it is, strided layers through the folded
 // cells (their gradient, brought back by unfold_grad_input_kernel).
-static mm::Windows grad_input_windows(const ConvGeom &g, const mm::Cells &u, bool half) {
+static mm::Windows grad_input_windows(const ConvGeom &g, const mm::Cells &u, int prec) {
   const int padH = u.direct ? g.kH - 1 - g.pad : u.kHs - 1, padW = u.direct ? g.kW - 1 - g.pad : u.kWs - 1;
-  return mm::Windows{g.N, g.oH, g.oW, mm::padded_channels(g.K, half), u.direct ? g.H : u.Hs, u.direct ? g.W : u.Ws, u.kHs, u.kWs, 1, 1, padH, padW};
+  return mm::Windows{g.N, g.oH, g.oW, mm::padded_channels(g.K, prec), u.direct ? g.H : u.Hs, u.direct ? g.W : u.Ws, u.kHs, u.kWs, 1, 1, padH, padW};
 }
-static mm::Cells grad_input_cells(const ConvGeom &g, bool half) {
-  return g.dH == 1 && g.dW == 1 ? direct_cells(g, half) : cells_of(g, false, false, half);
+static mm::Cells grad_input_cells(const ConvGeom &g, int prec) {
+  return g.dH == 1 && g.dW == 1 ? direct_cells(g, prec) : cells_of(g, false, false, prec);
 }
 
+// kPairs: the records of the tensors that a call's products read, whose form is decided together (mm::RangeRec).
+struct Records {
+  const mm::RangeRec *act = nullptr, *weight = nullptr, *gout = nullptr;
+  // `own` first, then the others
+  mm::Ranges joint(const mm::RangeRec *own) const {
+    mm::Ranges r;
+    int n = 0;
+    r.rec[n++] = own;
+    for (const mm::RangeRec *x : {act, weight, gout})
+      if (x != own) r.rec[n++] = x;
+    return r;
+  }
+};
+
 // out[n, r, y, x] = bias[r] + the product of the windows `v` over `act` with rows r < rows of the repacked weights
-template <bool HALF, bool FLIP, bool PAIR>
+template <int PREC, bool FLIP, bool PAIR>
 static void window_product_t(const void *act, const mm::Windows &full, const mm::Windows &v, const float *w, const mm::Cells &u, long K,
-                             long rows, const float *bias, float *out) {
+                             long rows, const float *bias, float *out, const Records &rec) {
   using namespace mm;
   const long Kd = (long)v.kH * v.kW * v.C;
   const long wrows = (PAIR ? 2 : 1) * rows;
   THC_CHECK(wrows * Kd < (1l << 31), "filter too large");
-  void *wp = ws_alloc((size_t)wrows * Kd * (HALF ? 2 : 4));
+  void *wp = ws_alloc((size_t)wrows * Kd * (PREC == mm::kBf16 ? 2 : 4));
   const long blocks = std::min<long>((wrows * (Kd / 4) + 255) / 256, ctx().sm_count * 8l);
-  pdl_launch(repack_weight_kernel<HALF, FLIP>, (unsigned)blocks, 256, 0, w, u, (int)K, (int)rows, (int)v.C, PAIR ? full.dW : 0, wp);
+  pdl_launch(repack_weight_kernel<PREC, FLIP>, (unsigned)blocks, 256, 0, w, u, (int)K, (int)rows, (int)v.C, PAIR ? full.dW : 0, wp, rec.joint(rec.weight));
   check_launch("repack_weight");
-  Problem<PlanesWindowOperand, RawOperand<false>, PAIR, HALF> p;
-  attach_window_map<HALF>(p.a, act, v);
+  Problem<PlanesWindowOperand<PREC>, RawOperand<false, PREC>, PAIR, PREC> p;
+  p.range_a = rec.act; p.range_b = rec.weight; p.ranges = rec.joint(rec.act);
+  attach_window_map<PREC>(p.a, act, v);
   const long P = full.oH * full.oW;
   p.epi = Epilogue{out, bias, 1.f, 0.f, P, rows * P, P};
   if (PAIR) {
     p.epi.pair_K = rows; p.epi.pair_oH = full.oH; p.epi.pair_oW2 = v.oW; p.epi.pair_oW = full.oW; p.epi.pair_img = rows * P;
   }
   p.M = v.N * v.oH * v.oW; p.N = wrows; p.K = Kd;
-  launch_raw(p, [&](auto &q, int bn2) { attach_raw_map<HALF>(q.b, wp, wrows, Kd, Kd, bn2 / 2); });
+  launch_raw(p, [&](auto &q, int bn2) { attach_raw_map<PREC>(q.b, wp, wrows, Kd, Kd, bn2 / 2); });
 }
-template <bool HALF, bool FLIP>
+template <int PREC, bool FLIP>
 static void window_product(const void *act, const mm::Windows &v, const float *w, const mm::Cells &u, long K, long rows, const float *bias,
-                           float *out) {
+                           float *out, const Records &rec) {
   mm::Windows p;
-  if constexpr (!HALF)
-    if (pair_windows(v, rows, HALF, p)) { window_product_t<HALF, FLIP, true>(act, v, p, w, u, K, rows, bias, out); return; }
-  window_product_t<HALF, FLIP, false>(act, v, v, w, u, K, rows, bias, out);
+  if constexpr (PREC != mm::kBf16)
+    if (pair_windows(v, rows, PREC, p)) { window_product_t<PREC, FLIP, true>(act, v, p, w, u, K, rows, bias, out, rec); return; }
+  window_product_t<PREC, FLIP, false>(act, v, v, w, u, K, rows, bias, out, rec);
 }
 
-// The restated input, written into `finput` when given (the counterpart of the column matrix the reference keeps there):
-// a [1, N, Hs, Ws, floats per pixel] tensor that accGradParameters reads back instead of making it again.
-template <bool HALF>
-static const void *restated_input(const ConvGeom &g, const mm::Cells &u, const float *in, THGPUTensor *finput) {
-  void *dst = nullptr;
-  if (finput) {
-    const long s[5] = {1, g.N, u.Hs, u.Ws, HALF ? u.Cs / 2 : u.Cs};
-    resize_nd(finput, 5, s, nullptr);
-    forget_planes(finput);
-    if (is_contiguous(finput) && ((uintptr_t)data_ptr(finput) & 15) == 0) { dst = data_ptr(finput); stamp_planes(finput, in, g, HALF); }
-  }
-  if (u.direct) return mm::make_act_planes<HALF>(in, g.N, g.C, g.H, g.W, dst, false).p;
-  if (!dst) dst = ws_alloc(mm::planes_bytes(g.N, (long)u.Hs * u.Ws, u.Cs, HALF));
-  if constexpr (HALF) {
+// The restated input in `dst`.
+template <int PREC>
+static void restate_input(const ConvGeom &g, const mm::Cells &u, const float *in, void *dst, const mm::PairForm &form) {
+  if (u.direct) { mm::make_act_planes<PREC>(in, g.N, g.C, g.H, g.W, dst, false, form); return; }
+  if constexpr (PREC == mm::kBf16) {
     const size_t smem = sizeof(uint4) * g.kH * (g.W + 2 * g.pad);
     if (u.Cq == 8 && u.kHs == 1 && u.kWs == 1 && g.C <= 8 && smem <= 200 * 1024) {
       static thread_local int configured_for = -1;
@@ -225,45 +232,76 @@ static const void *restated_input(const ConvGeom &g, const mm::Cells &u, const f
       }
       pdl_launch(mm::columns8_kernel, (unsigned)(g.N * u.Hs), 256, smem, in, (uint4 *)dst, u);
       check_launch("columns8");
-      return dst;
+      return;
     }
   }
   // a block per row of cells; a row is shared by several blocks where the rows of few images leave SMs idle (one
-  // 224 x 224 image: 8.4 us with one block each)
-  const long rows = g.N * u.Hs, chunks = (long)u.Ws * u.Cs / (HALF ? 8 : 4);
+  // 224 x 224 image: 8.4 us with one block each).  Planes that are hardly ever made again get few blocks to find that out.
+  const long rows = g.N * u.Hs, chunks = (long)u.Ws * u.Cs / (PREC != mm::kTf32 ? 8 : 4);
+  const unsigned bx = (unsigned)(form.remake ? std::min(rows, 4l * ctx().sm_count) : rows);
   const unsigned parts = (unsigned)std::max(1l, std::min((chunks + 255) / 256, 4l * ctx().sm_count / rows));
-  if (u.Cs <= mm::kCellTable) pdl_launch(mm::cells_input_kernel<HALF, true>, dim3((unsigned)rows, parts), 256, sizeof(int2) * u.Cs, in, dst, u);
-  else pdl_launch(mm::cells_input_kernel<HALF, false>, dim3((unsigned)rows, parts), 256, 0, in, dst, u);
+  if (u.Cs <= mm::kCellTable) pdl_launch(mm::cells_input_kernel<PREC, true>, dim3(bx, parts), 256, sizeof(int2) * u.Cs, in, dst, g.N, u, form);
+  else pdl_launch(mm::cells_input_kernel<PREC, false>, dim3(bx, parts), 256, 0, in, dst, g.N, u, form);
   check_launch("cells_input");
-  return dst;
+}
+
+// Room for the restated input in `finput` (the counterpart of the column matrix the reference keeps there): a
+// [1, N, Hs, Ws, floats per pixel] tensor that accGradParameters reads back instead of making it again.  Pairs have their
+// record behind the tensor, in the same storage.  Null: no room that a TMA map can address.
+static void *planes_in(THGPUTensor *finput, const ConvGeom &g, const mm::Cells &u, const float *in, int prec) {
+  const long s[5] = {1, g.N, u.Hs, u.Ws, prec == mm::kBf16 ? u.Cs / 2 : u.Cs}, n = s[1] * s[2] * s[3] * s[4];
+  resize_nd(finput, 5, s, nullptr);
+  if (prec == mm::kPairs && finput->storage && finput->storage->size < finput->storageOffset + n + mm::kRangeWords)
+    storage_resize(finput->storage, finput->storageOffset + n + mm::kRangeWords);
+  forget_planes(finput);
+  if (!is_contiguous(finput) || ((uintptr_t)data_ptr(finput) & 15) != 0) return nullptr;
+  stamp_planes(finput, in, g, prec);
+  return data_ptr(finput);
+}
+static mm::RangeRec *record_behind(const void *planes, const ConvGeom &g, const mm::Cells &u) {
+  return (mm::RangeRec *)((char *)planes + mm::planes_bytes(g.N, (long)u.Hs * u.Ws, u.Cs, mm::kPairs));
 }
 
 // The planes the forward pass of this very layer over this very input left in `finput`, or null.  A `finput` that has been given
 // another shape since has been used for something else.
-static const void *planes_made_from(const THGPUTensor *finput, const float *input, const ConvGeom &g, const mm::Cells &u, bool half) {
+static const void *planes_made_from(const THGPUTensor *finput, const float *input, const ConvGeom &g, const mm::Cells &u, int prec) {
   if (!finput || !finput->storage || finput->nDimension != 5 || !is_contiguous(finput)) return nullptr;
-  const long shape[5] = {1, g.N, u.Hs, u.Ws, half ? u.Cs / 2 : u.Cs};
+  const long shape[5] = {1, g.N, u.Hs, u.Ws, prec == mm::kBf16 ? u.Cs / 2 : u.Cs};
   if (!std::equal(shape, shape + 5, finput->size)) return nullptr;
+  if (prec == mm::kPairs && finput->storage->size < finput->storageOffset + nelem(finput) + mm::kRangeWords) return nullptr;
   auto it = g_plane_stamps.find(data_ptr(finput));
   if (it == g_plane_stamps.end()) return nullptr;
   const PlaneStamp &s = it->second;
-  const bool same = s.input == input && s.half == half && s.N == g.N && s.C == g.C && s.H == g.H && s.W == g.W && s.K == g.K &&
+  const bool same = s.input == input && s.prec == prec && s.N == g.N && s.C == g.C && s.H == g.H && s.W == g.W && s.K == g.K &&
                     s.kH == g.kH && s.kW == g.kW && s.dH == g.dH && s.dW == g.dW && s.pad == g.pad;
   return same ? data_ptr(finput) : nullptr;
 }
 
-template <bool HALF>
+template <int PREC>
 static void conv_forward_tc(const ConvGeom &g, const mm::Cells &u, const float *in, const float *w, const float *bias, float *out,
                             THGPUTensor *finput) {
-  const double bytes = (double)mm::planes_bytes(1, (long)u.Hs * u.Ws, u.Cs, HALF), floats = (double)g.N * g.C * g.H * g.W;
+  const double bytes = (double)mm::planes_bytes(1, (long)u.Hs * u.Ws, u.Cs, PREC), floats = (double)g.N * g.C * g.H * g.W;
   if (finput && bytes * (double)g.N > whole_scratch(floats)) { forget_planes(finput); finput = nullptr; }
   const long per = finput ? g.N : images_per_group(g.N, bytes, kGroupScratch);
+  Records rec;
+  if constexpr (PREC == mm::kPairs) {
+    mm::RangeRec *rx = mm::new_range_rec(), *rw = mm::new_range_rec();
+    const mm::RangeJob jw = mm::range_job_flat(w, g.K * g.R, rw);
+    mm::launch_ranges(mm::range_job_flat(in, g.N * g.C * g.H * g.W, rx), &jw);
+    rec.act = rx; rec.weight = rw;
+  }
   for (long n0 = 0; n0 < g.N; n0 += per) {
     WsScope ws_scope;
     ConvGeom s = g;
     s.N = std::min(per, g.N - n0);
-    const void *act = restated_input<HALF>(s, u, in + n0 * g.C * g.H * g.W, finput);
-    window_product<HALF, false>(act, forward_windows(s, u), w, u, g.K, g.K, bias, out + n0 * g.K * g.P);
+    const float *x = in + n0 * g.C * g.H * g.W;
+    mm::PairForm form;
+    form.ranges = rec.joint(rec.act);
+    void *act = finput ? planes_in(finput, s, u, x, PREC) : nullptr;
+    if (act && PREC == mm::kPairs) form.keep = record_behind(act, s, u);
+    if (!act) act = ws_alloc(mm::planes_bytes(s.N, (long)u.Hs * u.Ws, u.Cs, PREC));
+    restate_input<PREC>(s, u, x, act, form);
+    window_product<PREC, false>(act, forward_windows(s, u), w, u, g.K, g.K, bias, out + n0 * g.K * g.P, rec);
   }
 }
 
@@ -290,25 +328,26 @@ static const float *transposed_weight(const ConvGeom &g, const float *w, bool tu
 // gradInput of a layer with few output planes stated as a layer of its own, whose input is gradOutput: padding two planes to a span of
 // channels multiplies the product by 16, which restate() knows to avoid (13 x 13 taps, 271 <- 2 planes of 110 x 118, four images in
 // BF16: 915 us over padded planes, 177 so; 9 x 9, 32 <- 2, 46 of 87 x 88: 516 and 121).  False: the padded planes cost less.
-static bool grad_input_layer(const ConvGeom &g, bool half, ConvGeom &t, mm::Cells &u) {
-  if (g.dH != 1 || g.dW != 1 || g.kH != g.kW || g.pad >= g.kH || 2 * g.K > mm::padded_channels(g.K, half)) return false;
+static bool grad_input_layer(const ConvGeom &g, int prec, ConvGeom &t, mm::Cells &u) {
+  if (g.dH != 1 || g.dW != 1 || g.kH != g.kW || g.pad >= g.kH || 2 * g.K > mm::padded_channels(g.K, prec)) return false;
   t = g;
   t.C = g.K; t.K = g.C; t.H = g.oH; t.W = g.oW; t.oH = g.H; t.oW = g.W; t.P = g.H * g.W;
   t.pad = g.kH - 1 - g.pad; t.R = g.K * g.kH * g.kW;
-  if (!restate(t, half, u) || u.direct) return false;
-  const double bytes = (double)mm::planes_bytes(g.N, (long)u.Hs * u.Ws, u.Cs, half);
-  const double own = windows_us(forward_windows(t, u), t.K, half) + 2 * bytes / 5e6 + 10;   // and two launches more
-  return own < windows_us(grad_input_windows(g, grad_input_cells(g, half), half), g.C, half);
+  if (!restate(t, prec, u) || u.direct) return false;
+  const double bytes = (double)mm::planes_bytes(g.N, (long)u.Hs * u.Ws, u.Cs, prec);
+  const double own = windows_us(forward_windows(t, u), t.K, prec) + 2 * bytes / 5e6 + 10;   // and two launches more
+  return own < windows_us(grad_input_windows(g, grad_input_cells(g, prec), prec), g.C, prec);
 }
 
 // gradInput = forward pass of gradOutput's planes under the filter rotated by 180 degrees with its plane roles swapped.
-template <bool HALF>
-static void conv_grad_input_tc(const ConvGeom &g, const mm::ActPlanes &pgo, const float *w, float *gin) {
-  const mm::Cells u = grad_input_cells(g, HALF);
-  const mm::Windows v = grad_input_windows(g, u, HALF);
-  if (u.direct) { window_product<HALF, true>(pgo.p, v, w, u, g.K, g.C, nullptr, gin); return; }
+template <int PREC>
+static void conv_grad_input_tc(const ConvGeom &g, const mm::ActPlanes &pgo, const float *w, float *gin, Records rec) {
+  rec.act = std::exchange(rec.gout, rec.act);   // the windows run over gradOutput here
+  const mm::Cells u = grad_input_cells(g, PREC);
+  const mm::Windows v = grad_input_windows(g, u, PREC);
+  if (u.direct) { window_product<PREC, true>(pgo.p, v, w, u, g.K, g.C, nullptr, gin, rec); return; }
   float *gS = (float *)ws_alloc(sizeof(float) * g.N * u.Cr * (long)(u.Hs * u.Ws));
-  window_product<HALF, true>(pgo.p, v, w, u, g.K, u.Cr, nullptr, gS);
+  window_product<PREC, true>(pgo.p, v, w, u, g.K, u.Cr, nullptr, gS, rec);
   const long planes = g.N * g.C;
   const unsigned bx = (unsigned)std::min<long>((g.H * g.W + 255) / 256, 64);
   const unsigned by = (unsigned)std::min<long>(planes, std::max<long>(1, ctx().sm_count * 32l / bx));
@@ -324,34 +363,36 @@ static void conv_grad_input_tc(const ConvGeom &g, const mm::ActPlanes &pgo, cons
 //        T[(bi, ch)][(j', ko)] = sum_{n, y, x'} S[n][y + bi][x'][ch] * gradOut[n][y][x' - (kWs - 1 - j')][ko]
 //      is the gradient of tap (bi, bj = kWs - 1 - j'): the column shift is a zero-padded window of the gradOutput
 //      plane, which TMA's im2col mode reads like any other.  For layers with few output planes and columns, whose
-//      64-wide tiles would run at half the tensor-pipe rate.
+//      64-wide tiles would run at prec the tensor-pipe rate.
 // and, for the column form (one tap), whose two operands are plain matrices of a few columns:
 //   3  f pixels side by side, rows = (pixel mod f, ko), columns = (pixel mod f, ch) of the same memory read as wider
 //      matrices: the f diagonal blocks of the result are the gradient's partial sums.  The other blocks are computed in
 //      vain, but a k tile costs the same however little of its 256 x 64 tile is used, and there are f times fewer.
-template <bool HALF>
-static void conv_acc_grad_tc(const ConvGeom &g, const mm::Cells &u, const void *act, const mm::ActPlanes &pgo, float *gw, float scale) {
+template <int PREC>
+static void conv_acc_grad_tc(const ConvGeom &g, const mm::Cells &u, const void *act, const mm::ActPlanes &pgo, float *gw, float scale,
+                             const Records &rec) {
   using namespace mm;
   const Windows v = forward_windows(g, u);
   const long Kp = pgo.Cp, Cs = u.Cs, Rp = (long)u.kHs * u.kWs * Cs, pixels = g.N * g.P;
   const long M2 = (long)u.kHs * Cs, N2 = (long)u.kWs * Kp;
   const Windows va{g.N, u.Hs, u.Ws, Cs, g.oH, u.Ws, u.kHs, 1, 1, 1, 0, 0};
   const Windows vb{g.N, g.oH, g.oW, Kp, g.oH, u.Ws, 1, u.kWs, 1, 1, 0, u.kWs - 1};
-  double us[3] = {tc2_product_us(g.K, Rp, pixels, HALF, true), tc2_product_us(Rp, g.K, pixels, HALF, true),
-                  !u.direct && u.kWs > 1 && windows_ok(va) && windows_ok(vb) ? tc2_product_us(M2, N2, g.N * g.oH * u.Ws, HALF, true) : 1e30};
+  double us[3] = {tc2_product_us(g.K, Rp, pixels, PREC, true), tc2_product_us(Rp, g.K, pixels, PREC, true),
+                  !u.direct && u.kWs > 1 && windows_ok(va) && windows_ok(vb) ? tc2_product_us(M2, N2, g.N * g.oH * u.Ws, PREC, true) : 1e30};
   int way = us[2] < us[0] && us[2] < us[1] ? 2 : us[1] < us[0] ? 1 : 0;
   long f = 1;
-  if (u.kHs == 1 && u.kWs == 1 && !u.direct)
+  if (PREC != kPairs && u.kHs == 1 && u.kWs == 1 && !u.direct)   // (a pair's halves lie side by side, not a pixel's neighbours)
     while (2 * f * Kp <= 256 && 2 * f * Cs <= 256 && pixels % (2 * f) == 0) f *= 2;
-  if (f > 1 && tc2_product_us(f * Kp, f * Cs, pixels / f, HALF, true) < us[way]) {
+  if (f > 1 && tc2_product_us(f * Kp, f * Cs, pixels / f, PREC, true) < us[way]) {
     const long Mf = f * Kp, Nf = f * Cs;
     float *T = (float *)ws_alloc(sizeof(float) * Mf * Nf);
-    Problem<RawOperand<true>, RawOperand<true>, false, HALF> p;
+    Problem<RawOperand<true, PREC>, RawOperand<true, PREC>, false, PREC> p;
+    p.range_a = rec.gout; p.range_b = rec.act; p.ranges = rec.joint(rec.act);
     p.epi = Epilogue{T, nullptr, 1.f, 0.f, 1, Nf, 1};                 // T[m * Nf + n]
     p.M = Mf; p.N = Nf; p.K = pixels / f;
     launch_raw(p, [&](auto &q, int bn2) {
-      attach_raw_map<HALF>(q.a, pgo.p, Mf, pixels / f, Mf, TC_BM);
-      attach_raw_map<HALF>(q.b, act, Nf, pixels / f, Nf, bn2 / 2);
+      attach_raw_map<PREC>(q.a, pgo.p, Mf, pixels / f, Mf, TC_BM);
+      attach_raw_map<PREC>(q.b, act, Nf, pixels / f, Nf, bn2 / 2);
     });
     const WgradPlace pl{Nf, 1, 0, 0, 0, (int)f, Kp * Nf + Cs};
     const long total = g.K * g.R;
@@ -363,23 +404,26 @@ static void conv_acc_grad_tc(const ConvGeom &g, const mm::Cells &u, const void *
   float *T = (float *)ws_alloc(sizeof(float) * rows * cols);
   WgradPlace pl;
   if (way == 0) {
-    Problem<RawOperand<true>, WindowRowsOperand, false, HALF> p;
-    attach_window_rows_map<HALF>(p.b, act, v);
+    Problem<RawOperand<true, PREC>, WindowRowsOperand<PREC>, false, PREC> p;
+    p.range_a = rec.gout; p.range_b = rec.act; p.ranges = rec.joint(rec.act);
+    attach_window_rows_map<PREC>(p.b, act, v);
     p.epi = Epilogue{T, nullptr, 1.f, 0.f, 1, Rp, 1};                 // T[m * Rp + n]
     p.M = g.K; p.N = Rp; p.K = pixels;
-    launch_raw(p, [&](auto &q, int) { attach_raw_map<HALF>(q.a, pgo.p, Kp, pixels, Kp, TC_BM); });
+    launch_raw(p, [&](auto &q, int) { attach_raw_map<PREC>(q.a, pgo.p, Kp, pixels, Kp, TC_BM); });
     pl = WgradPlace{Rp, 1, u.kWs * Cs, Cs, 0, 1, 0};
   } else if (way == 1) {
-    Problem<WindowRowsOperand, RawOperand<true>, false, HALF> p;
-    attach_window_rows_map<HALF>(p.a, act, v);
+    Problem<WindowRowsOperand<PREC>, RawOperand<true, PREC>, false, PREC> p;
+    p.range_a = rec.act; p.range_b = rec.gout; p.ranges = rec.joint(rec.act);
+    attach_window_rows_map<PREC>(p.a, act, v);
     p.epi = Epilogue{T, nullptr, 1.f, 0.f, LONG_MAX, 0, Rp};          // T[n * Rp + m]
     p.M = Rp; p.N = g.K; p.K = pixels;
-    launch_raw(p, [&](auto &q, int bn2) { attach_raw_map<HALF>(q.b, pgo.p, Kp, pixels, Kp, bn2 / 2); });
+    launch_raw(p, [&](auto &q, int bn2) { attach_raw_map<PREC>(q.b, pgo.p, Kp, pixels, Kp, bn2 / 2); });
     pl = WgradPlace{Rp, 1, u.kWs * Cs, Cs, 0, 1, 0};
   } else {
-    Problem<WindowRowsOperand, WindowRowsOperand, false, HALF> p;
-    attach_window_rows_map<HALF>(p.a, act, va);
-    attach_window_rows_map<HALF>(p.b, pgo.p, vb);
+    Problem<WindowRowsOperand<PREC>, WindowRowsOperand<PREC>, false, PREC> p;
+    p.range_a = rec.act; p.range_b = rec.gout; p.ranges = rec.joint(rec.act);
+    attach_window_rows_map<PREC>(p.a, act, va);
+    attach_window_rows_map<PREC>(p.b, pgo.p, vb);
     p.epi = Epilogue{T, nullptr, 1.f, 0.f, 1, N2, 1};                 // T[m * N2 + n]
     p.M = M2; p.N = N2; p.K = g.N * g.oH * u.Ws;
     launch_raw(p, [](auto &, int) {});
@@ -521,16 +565,36 @@ static bool half_acc_grad(const ConvGeom &g) {
   return ctx().math_mode == 2 && ((Kp > 128 && Rp > 64) || (Rp > 128 && Kp > 64));
 }
 
+// FP16 pairs or TF32 for the FP32-accurate products of a layer, all of which share its planes: by the forward product's time and
+// the pass that measures the input, with 10 us for the launches that measure and check (64 planes under 11 x 11 / 4 over 16 images,
+// 40 us a product: 201.5 us in TF32, 212.6 over pairs for the whole block; 128 images: 4020 -> 3160 us a training step).  The column
+// form stays in TF32, whose weight gradient stacks pixels.
+static bool restate_accurate(const ConvGeom &g, mm::Cells &u, int &prec) {
+  prec = mm::kTf32;
+  const bool ok = restate(g, mm::kTf32, u);
+  mm::Cells up;
+  if (!ok || ctx().math_mode != 0 || windows_us(forward_windows(g, u), g.K, prec) < 30 || !restate(g, mm::kPairs, up) ||
+      (up.kHs == 1 && up.kWs == 1 && !up.direct))
+    return ok;
+  auto us = [&](const mm::Cells &c, int pr) {
+    return windows_us(forward_windows(g, c), g.K, pr) + 2 * (double)mm::planes_bytes(g.N, (long)c.Hs * c.Ws, c.Cs, pr) / 5e6;
+  };
+  if (us(up, mm::kPairs) + 10 + 4e-6 / 5.5 * (double)(g.N * g.C * g.H * g.W) < us(u, mm::kTf32)) { u = up; prec = mm::kPairs; }
+  return ok;
+}
+
 static void conv_forward(const ConvGeom &g, const float *in, const float *w, const float *bias, float *out, THGPUTensor *finput) {
   mm::Cells u;
   const bool half = half_forward(g);
-  if (ctx().math_mode != 1 && restate(g, half, u)) {
+  int prec = mm::kBf16;
+  if (ctx().math_mode != 1 && (half ? restate(g, prec, u) : restate_accurate(g, u, prec))) {
     // kept for a weight gradient of the same precision only, no other reads them back: the BF16 column matrix of the 11 x 11 / 4
     // layer over 3 planes is 6.2 MB an image, and its weight gradient FP32-accurate
     THGPUTensor *keep = half == half_acc_grad(g) ? finput : nullptr;
     if (!keep) forget_planes(finput);
-    if (half) conv_forward_tc<true>(g, u, in, w, bias, out, keep);
-    else conv_forward_tc<false>(g, u, in, w, bias, out, keep);
+    if (prec == mm::kBf16) conv_forward_tc<mm::kBf16>(g, u, in, w, bias, out, keep);
+    else if (prec == mm::kPairs) conv_forward_tc<mm::kPairs>(g, u, in, w, bias, out, keep);
+    else conv_forward_tc<mm::kTf32>(g, u, in, w, bias, out, keep);
     return;
   }
   forget_planes(finput);   // this pass leaves finput alone: what it holds belongs to an earlier input
@@ -539,25 +603,32 @@ static void conv_forward(const ConvGeom &g, const float *in, const float *w, con
 
 // gradInput (when gin is given) and gradWeight / gradBias (when gw is) of one precision, sharing one transposition of gradOutput.
 // `act`: the input's planes, or null; w_ok / in_ok: whether the weight gradient / gradInput runs over planes.
-template <bool HALF>
+template <int PREC>
 static void conv_backward_group(const ConvGeom &g, const mm::Cells &u, bool in_ok, bool w_ok, const float *in, const void *act, const float *gout,
-                                const float *w, float *gin, float *gw, float *gb, float scale) {
+                                const float *w, float *gin, float *gw, float *gb, float scale, const Records &rec) {
   WsScope ws_scope;
   ConvGeom t;
   mm::Cells ut;
-  if (gin && grad_input_layer(g, HALF, t, ut)) {
-    conv_forward_tc<HALF>(t, ut, gout, transposed_weight(g, w, true), nullptr, gin, nullptr);
+  if (gin && grad_input_layer(g, PREC, t, ut)) {
+    conv_forward_tc<PREC>(t, ut, gout, transposed_weight(g, w, true), nullptr, gin, nullptr);
     gin = nullptr;
     in_ok = false;
   }
   mm::ActPlanes pgo;
-  if (in_ok || w_ok) pgo = mm::make_act_planes<HALF>(gout, g.N, g.K, g.oH, g.oW, nullptr, gw != nullptr);
-  if (in_ok) conv_grad_input_tc<HALF>(g, pgo, w, gin);
+  mm::PairForm form;
+  form.ranges = rec.joint(rec.gout);
+  if (in_ok || w_ok) pgo = mm::make_act_planes<PREC>(gout, g.N, g.K, g.oH, g.oW, nullptr, gw != nullptr, form);
+  if (in_ok) conv_grad_input_tc<PREC>(g, pgo, w, gin, rec);
   else if (gin) conv_grad_input_simt(g, gout, w, gin);
   if (!gw) return;
   if (w_ok) {
-    if (!act) act = restated_input<HALF>(g, u, in, nullptr);
-    conv_acc_grad_tc<HALF>(g, u, act, pgo, gw, scale);
+    if (!act) {
+      void *made = ws_alloc(mm::planes_bytes(g.N, (long)u.Hs * u.Ws, u.Cs, PREC));
+      form.ranges = rec.joint(rec.act);
+      restate_input<PREC>(g, u, in, made, form);
+      act = made;
+    }
+    conv_acc_grad_tc<PREC>(g, u, act, pgo, gw, scale, rec);
   } else {
     conv_acc_grad_simt(g, in, gout, gw, scale);
   }
@@ -568,26 +639,45 @@ static void conv_backward_group(const ConvGeom &g, const mm::Cells &u, bool in_o
     grad_bias(g, gout, gb, scale);
   }
 }
-template <bool HALF>
-static void conv_backward_tc(const ConvGeom &g, const float *in, const float *gout, const float *w, float *gin, float *gw, float *gb, float scale,
-                             const THGPUTensor *finput) {
-  mm::Cells u;
-  const mm::Cells ui = grad_input_cells(g, HALF);
-  const bool in_ok = gin && mm::windows_ok(grad_input_windows(g, ui, HALF)), w_ok = gw && restate(g, HALF, u);
+template <int PREC>
+static void conv_backward_tc(const ConvGeom &g, const mm::Cells &u, bool restated, const float *in, const float *gout, const float *w, float *gin,
+                             float *gw, float *gb, float scale, const THGPUTensor *finput) {
+  const mm::Cells ui = grad_input_cells(g, PREC);
+  const bool in_ok = gin && mm::windows_ok(grad_input_windows(g, ui, PREC)), w_ok = gw && restated;
   // the input's planes: those the forward pass left in finput (as the CPU nn path reuses its finput,
   // mcw_nn/generic/SpatialConvolutionMM.c:284-346), else made group by group
-  const char *act = w_ok ? (const char *)planes_made_from(finput, in, g, u, HALF) : nullptr;
-  const size_t act_image = w_ok ? mm::planes_bytes(1, (long)u.Hs * u.Ws, u.Cs, HALF) : 0;
+  const char *act = w_ok ? (const char *)planes_made_from(finput, in, g, u, PREC) : nullptr;
+  const size_t act_image = w_ok ? mm::planes_bytes(1, (long)u.Hs * u.Ws, u.Cs, PREC) : 0;
+  Records rec;
+  if constexpr (PREC == mm::kPairs) {
+    const long image = g.C * g.H * g.W;
+    mm::RangeRec *rg = mm::new_range_rec(), *rw = in_ok ? mm::new_range_rec() : nullptr;
+    const mm::RangeJob jg = mm::range_job_flat(gout, g.N * g.K * g.P, rg), jw = mm::range_job_flat(w, g.K * g.R, rw);
+    mm::launch_ranges(jg, rw ? &jw : nullptr);
+    rec.gout = rg; rec.weight = rw;
+    if (act) {
+      mm::RangeRec *kept = record_behind(act, g, u);
+      rec.act = kept;
+      mm::PairForm form;
+      form.ranges = rec.joint(kept);
+      form.remake = kept;
+      restate_input<PREC>(g, u, in, (void *)act, form);
+    } else if (w_ok) {
+      mm::RangeRec *rx = mm::new_range_rec();
+      mm::launch_ranges(mm::range_job_flat(in, g.N * image, rx), nullptr);
+      rec.act = rx;
+    }
+  }
   double bytes = 0;
-  if (in_ok || w_ok) bytes += (double)mm::planes_bytes(1, g.P, mm::padded_channels(g.K, HALF), HALF);
+  if (in_ok || w_ok) bytes += (double)mm::planes_bytes(1, g.P, mm::padded_channels(g.K, PREC), PREC);
   if (in_ok && !ui.direct) bytes += 4. * ui.Cr * ui.Hs * ui.Ws;
   if (w_ok && !act) bytes += (double)act_image;
   const long image = g.C * g.H * g.W, per = images_per_group(g.N, bytes, whole_scratch((double)g.N * (image + g.K * g.P)));
   for (long n0 = 0; n0 < g.N; n0 += per) {
     ConvGeom s = g;
     s.N = std::min(per, g.N - n0);
-    conv_backward_group<HALF>(s, u, in_ok, w_ok, in ? in + n0 * image : nullptr, act ? act + n0 * act_image : nullptr, gout + n0 * g.K * g.P, w,
-                              gin ? gin + n0 * image : nullptr, gw, gb, scale);
+    conv_backward_group<PREC>(s, u, in_ok, w_ok, in ? in + n0 * image : nullptr, act ? act + n0 * act_image : nullptr, gout + n0 * g.K * g.P, w,
+                              gin ? gin + n0 * image : nullptr, gw, gb, scale, rec);
   }
 }
 static void conv_backward(const ConvGeom &g, const float *in, const float *gout, const float *w, float *gin, float *gw, float *gb, float scale,
@@ -601,8 +691,17 @@ static void conv_backward(const ConvGeom &g, const float *in, const float *gout,
     return;
   }
   const bool hin = gin && half_grad_input(g), hw = gw && half_acc_grad(g);
-  if (hin || hw) conv_backward_tc<true>(g, in, gout, w, hin ? gin : nullptr, hw ? gw : nullptr, gb, scale, finput);
-  if ((gin && !hin) || (gw && !hw)) conv_backward_tc<false>(g, in, gout, w, hin ? nullptr : gin, hw ? nullptr : gw, gb, scale, finput);
+  mm::Cells u;
+  if (hin || hw) {
+    const bool ok = restate(g, mm::kBf16, u);
+    conv_backward_tc<mm::kBf16>(g, u, ok, in, gout, w, hin ? gin : nullptr, hw ? gw : nullptr, gb, scale, finput);
+  }
+  if ((gin && !hin) || (gw && !hw)) {
+    int prec;
+    const bool ok = restate_accurate(g, u, prec);
+    if (prec == mm::kPairs) conv_backward_tc<mm::kPairs>(g, u, ok, in, gout, w, hin ? nullptr : gin, hw ? nullptr : gw, gb, scale, finput);
+    else conv_backward_tc<mm::kTf32>(g, u, ok, in, gout, w, hin ? nullptr : gin, hw ? nullptr : gw, gb, scale, finput);
+  }
 }
 
 static void check_grad_output(const ConvGeom &g, const THGPUTensor *gradOutput) {

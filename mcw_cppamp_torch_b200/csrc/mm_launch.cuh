@@ -106,20 +106,31 @@ static bool raw_matrix_ok(const float *base, long ld) {
   return encode_tiled_fn() && ((uintptr_t)base & 15) == 0 && ld % 4 == 0 && ld > 0;
 }
 // Element (r, k) of the matrix at base[r * ld + k], or base[k * ld + r] for MN; tile_rows: K-major rows per load.
-template <bool HALF, bool MN>
-static void attach_raw_map(RawOperand<MN> &op, const void *base, long rows, long K, long ld, int tile_rows) {
-  constexpr int KV = HALF ? 64 : 32;
+static void encode_matrix(CUtensorMap *map, CUtensorMapDataType type, int size, const void *base, bool mn, long rows, long K, long ld, int tile_rows) {
+  const cuuint32_t kv = 128 / (cuuint32_t)size;
   EncodeTiledFn enc = encode_tiled_fn();
-  THC_CHECK(enc && ((uintptr_t)base & 15) == 0 && ld % (HALF ? 8 : 4) == 0, "internal: matrix not addressable by TMA");
-  const cuuint64_t dims[2] = {(cuuint64_t)(MN ? rows : K), (cuuint64_t)(MN ? K : rows)};
-  const cuuint64_t strides[1] = {(cuuint64_t)ld * (HALF ? 2 : 4)};
-  const cuuint32_t box[2] = {KV, (cuuint32_t)(MN ? KV : tile_rows)};
+  THC_CHECK(enc && ((uintptr_t)base & 15) == 0 && ld * size % 16 == 0, "internal: matrix not addressable by TMA");
+  const cuuint64_t dims[2] = {(cuuint64_t)(mn ? rows : K), (cuuint64_t)(mn ? K : rows)};
+  const cuuint64_t strides[1] = {(cuuint64_t)ld * size};
+  const cuuint32_t box[2] = {kv, mn ? kv : (cuuint32_t)tile_rows};
   const cuuint32_t estr[2] = {1, 1};
-  const CUresult r = enc(&op.tmap, HALF ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, (void *)base, dims, strides,
-                         box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                         MN && !HALF ? CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B : CU_TENSOR_MAP_SWIZZLE_128B,
+  const CUresult r = enc(map, type, 2, (void *)base, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                         mn && size == 4 ? CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B : CU_TENSOR_MAP_SWIZZLE_128B,
                          CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   THC_CHECK(r == CUDA_SUCCESS, "internal: cuTensorMapEncodeTiled failed");
+}
+// kPairs: `ld` is the padded length of a line's halves, whose FP32 form has that pitch.
+template <int PREC, bool MN>
+static void attach_raw_map(RawOperand<MN, PREC> &op, const void *base, long rows, long K, long ld, int tile_rows) {
+  if constexpr (PREC == kPairs) {
+    op.lo = (int)ld;
+    encode_matrix(&op.tmap, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, base, MN, MN ? 2 * ld : rows, MN ? K : 2 * ld, 2 * ld, tile_rows);
+    encode_matrix(&op.tmap_wide, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, base, MN, rows, K, ld, tile_rows);
+  } else if (PREC == kBf16) {
+    encode_matrix(&op.tmap, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, base, MN, rows, K, ld, tile_rows);
+  } else {
+    encode_matrix(&op.tmap, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, base, MN, rows, K, ld, tile_rows);
+  }
 }
 
 // Windows of kH x kW taps on an [oH, oW] grid at strides (dH, dW) under padding (padH, padW), over a channels-last plane
@@ -146,37 +157,48 @@ static void set_window_pixels(PixelMap &m, const Windows &v) {
   m.img_stride = m.y_stride = m.x_stride = m.off0 = 0;   // the TMA map knows the memory
   m.sy = v.dH; m.y0 = -v.padH; m.sx = v.dW; m.x0 = -v.padW;
 }
-template <bool HALF>
-static void encode_windows(CUtensorMap *map, const void *base, const Windows &v, int windows_per_load, bool mn) {
-  constexpr int KV = HALF ? 64 : 32, E = HALF ? 2 : 4;
+static void encode_windows(CUtensorMap *map, CUtensorMapDataType type, int size, const void *base, const Windows &v, long C, int windows_per_load,
+                           bool mn) {
+  const int kv = 128 / size;
   EncodeIm2colFn enc = encode_im2col_fn();
   int lower[2], upper[2];
-  THC_CHECK(enc && v.C % KV == 0 && ((uintptr_t)base & 15) == 0 && window_corners(v, lower, upper), "internal: windows not addressable by TMA");
-  const cuuint64_t dims[4] = {(cuuint64_t)v.C, (cuuint64_t)v.W, (cuuint64_t)v.H, (cuuint64_t)v.N};
-  const cuuint64_t strides[3] = {(cuuint64_t)v.C * E, (cuuint64_t)v.W * v.C * E, (cuuint64_t)v.H * v.W * v.C * E};
+  THC_CHECK(enc && C % kv == 0 && ((uintptr_t)base & 15) == 0 && window_corners(v, lower, upper), "internal: windows not addressable by TMA");
+  const cuuint64_t dims[4] = {(cuuint64_t)C, (cuuint64_t)v.W, (cuuint64_t)v.H, (cuuint64_t)v.N};
+  const cuuint64_t strides[3] = {(cuuint64_t)C * size, (cuuint64_t)v.W * C * size, (cuuint64_t)v.H * v.W * C * size};
   const cuuint32_t estr[4] = {1, (cuuint32_t)v.dW, (cuuint32_t)v.dH, 1};
-  const CUresult r = enc(map, HALF ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, (void *)base, dims, strides, lower,
-                         upper, KV, (cuuint32_t)windows_per_load, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                         mn && !HALF ? CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B : CU_TENSOR_MAP_SWIZZLE_128B,
+  const CUresult r = enc(map, type, 4, (void *)base, dims, strides, lower, upper, (cuuint32_t)kv, (cuuint32_t)windows_per_load, estr,
+                         CU_TENSOR_MAP_INTERLEAVE_NONE, mn && size == 4 ? CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B : CU_TENSOR_MAP_SWIZZLE_128B,
                          CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   THC_CHECK(r == CUDA_SUCCESS, "internal: cuTensorMapEncodeIm2col failed");
 }
-template <bool HALF>
-static void attach_window_map(PlanesWindowOperand &op, const void *base, const Windows &v) {
+// The maps of an operand of windows; per load `per` windows, or as many as a span has values (mn).
+template <int PREC, class Op>
+static void attach_windows(Op &op, const void *base, const Windows &v, int per, bool mn) {
   op.n_img = (int)v.N;
-  set_window_pixels(op.rows, v);
-  op.ctiles = FastDiv::make(v.C / (HALF ? 64 : 32)); op.kW = FastDiv::make(v.kW);
-  encode_windows<HALF>(&op.tmap, base, v, TC_BM, false);
+  if constexpr (PREC == kPairs) {
+    op.lo = (int)v.C;
+    encode_windows(&op.tmap, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, base, v, 2 * v.C, mn ? 64 : per, mn);
+    encode_windows(&op.tmap_wide, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, base, v, v.C, mn ? 32 : per, mn);
+  } else if (PREC == kBf16) {
+    encode_windows(&op.tmap, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, base, v, v.C, mn ? 64 : per, mn);
+  } else {
+    encode_windows(&op.tmap, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, base, v, v.C, mn ? 32 : per, mn);
+  }
 }
-template <bool HALF>
-static void attach_window_rows_map(WindowRowsOperand &op, const void *base, const Windows &v) {
-  op.n_img = (int)v.N;
+template <int PREC>
+static void attach_window_map(PlanesWindowOperand<PREC> &op, const void *base, const Windows &v) {
+  set_window_pixels(op.rows, v);
+  op.ctiles = FastDiv::make(v.C / (PREC != kTf32 ? 64 : 32)); op.ctiles_wide = FastDiv::make(v.C / 32); op.kW = FastDiv::make(v.kW);
+  attach_windows<PREC>(op, base, v, TC_BM, false);
+}
+template <int PREC>
+static void attach_window_rows_map(WindowRowsOperand<PREC> &op, const void *base, const Windows &v) {
   set_window_pixels(op.ks, v);
   op.C = FastDiv::make(v.C); op.kW = FastDiv::make(v.kW);
-  encode_windows<HALF>(&op.tmap, base, v, HALF ? 64 : 32, true);
+  attach_windows<PREC>(op, base, v, 0, true);
 }
 
-// Width of the two-SM tile that pads N least (wider wins ties).  An MN-major BF16 operand on the N side comes in blocks of
+// Width of the two-SM tile that pads N least (wider wins ties).  An MN-major 16-bit operand on the N side comes in blocks of
 // 64 rows per CTA, which leaves 256 and 128.
 static int tc2_tile_width(long N, bool half_mn = false) {
   int best = 0;
@@ -190,29 +212,30 @@ static int tc2_tile_width(long N, bool half_mn = false) {
   return best;
 }
 // Microseconds a cluster takes for one k tile of a tile of this width, as the convolution and addmm launches at full size show it.
-static double tc2_tile_us(int bn2, bool half) {
-  if (half) return bn2 == 256 ? 0.55 : bn2 == 192 ? 0.47 : 0.4;
+static double tc2_tile_us(int bn2, int prec) {
+  if (prec == kBf16) return bn2 == 256 ? 0.55 : bn2 == 192 ? 0.47 : 0.4;
+  if (prec == kPairs) return bn2 == 256 ? 1.3 : bn2 == 192 ? 1.1 : bn2 == 128 ? 0.9 : 0.8;
   return bn2 == 256 ? 1.25 : bn2 == 192 ? 1.0 : bn2 == 128 ? 0.79 : 0.7;
 }
 // Model of a product's time, for choices between ways of stating it.
-static double tc2_product_us(long M, long N, long K, bool half, bool half_mn = false) {
-  const int w = tc2_tile_width(N, half && half_mn), kv = half ? 64 : 32;
+static double tc2_product_us(long M, long N, long K, int prec, bool mn = false) {
+  const int w = tc2_tile_width(N, prec != kTf32 && mn), kv = prec != kTf32 ? 64 : 32;
   const double tiles = (double)((M + 255) / 256) * (double)((N + w - 1) / w), ktiles = (double)((K + kv - 1) / kv);
   // a tile's epilogue and hand-over take about as long as two k tiles; a tile cut along k keeps at least six
-  return std::max(tiles * (ktiles + 2) / (ctx().sm_count / 2), std::min(ktiles, 6.0) + 2) * tc2_tile_us(w, half) + 8;
+  return std::max(tiles * (ktiles + 2) / (ctx().sm_count / 2), std::min(ktiles, 6.0) + 2) * tc2_tile_us(w, prec) + 8;
 }
 
 // Clusters of the two-SM kernel that the device runs at once (the kernel is persistent: a launch has no more).
 template <class P, int BN2>
 static int tc2r_resident_clusters() {
-  typedef Tc2rCfg<BN2, P::HALF> Cfg;
+  constexpr int SMEM = tc2r_smem_bytes<BN2, P::PREC>();
   static PerDevice resident;
   return resident.get(ctx().device, [] {
-    THC_CUDA(cudaFuncSetAttribute(tc2r_kernel<P, BN2>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM_BYTES));
+    THC_CUDA(cudaFuncSetAttribute(tc2r_kernel<P, BN2>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM));
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(2 * ctx().sm_count, 1, 1);
     cfg.blockDim = dim3(T2_THREADS, 1, 1);
-    cfg.dynamicSmemBytes = Cfg::SMEM_BYTES;
+    cfg.dynamicSmemBytes = SMEM;
     int c = 0;
     if (cudaOccupancyMaxActiveClusters(&c, tc2r_kernel<P, BN2>, &cfg) != cudaSuccess || c < 1) {
       cudaGetLastError();
@@ -230,11 +253,10 @@ static int tc2r_resident_clusters() {
 }
 template <class P, int BN2>
 static void launch_tc2r_kernel(const P &p, long items) {
-  typedef Tc2rCfg<BN2, P::HALF> Cfg;
   const long clusters = std::min<long>(items, tc2r_resident_clusters<P, BN2>());
   // a long launch gains nothing from starting early, and measured 1.5 % slower when it did (4096^3: 671 -> 682 us)
-  const bool early = tc2_product_us(p.M, p.N, p.K, P::HALF, P::HALF && P::OpB::MN_MAJOR) < 100;
-  launch_on_stream(early, tc2r_kernel<P, BN2>, dim3((unsigned)(2 * clusters), 1, 1), T2_THREADS, Cfg::SMEM_BYTES, p, stall_ctl(), sched_counter());
+  const bool early = tc2_product_us(p.M, p.N, p.K, P::PREC, P::OpB::MN_MAJOR) < 100;
+  launch_on_stream(early, tc2r_kernel<P, BN2>, dim3((unsigned)(2 * clusters), 1, 1), T2_THREADS, tc2r_smem_bytes<BN2, P::PREC>(), p, stall_ctl(), sched_counter());
   check_launch("tc2r_kernel");
 }
 
@@ -243,12 +265,12 @@ template <class P, class Attach>
 static void launch_raw(P p, Attach attach) {
   if (p.M <= 0 || p.N <= 0) return;
   THC_CHECK(p.K > 0, "internal: matrix product with empty reduction");
-  constexpr bool HALF_MN = P::HALF && P::OpB::MN_MAJOR;
+  constexpr bool HALF_MN = P::PREC != kTf32 && P::OpB::MN_MAJOR;
   const int bn2 = tc2_tile_width(p.N, HALF_MN);
   attach(p, bn2);
   const long gm = (p.M + 255) / 256, gn = (p.N + bn2 - 1) / bn2, tiles = gm * gn;
   int slots = 0;
-  // the widths a problem can come to: BF16 MN-major 256 and 128, pixel pairs (at most 128 columns) 128 and 64
+  // the widths a problem can come to: 16-bit MN-major 256 and 128, pixel pairs (at most 128 columns) 128 and 64
   auto with_width = [&](auto f) {
     if (bn2 == 128) { f(std::integral_constant<int, 128>()); return; }
     if constexpr (!P::PAIR) {
@@ -266,9 +288,9 @@ static void launch_raw(P p, Attach attach) {
   // tiles than clusters) are cut along k so that they fill the clusters once more instead of leaving most idle.
   // BF16 products over K-major operands (whose results the next layer rounds to BF16 again) cut every tile alike, so that no
   // element's rounding depends on the tile it falls in.
-  constexpr bool EVEN = P::HALF && !P::OpB::MN_MAJOR;
+  constexpr bool EVEN = P::PREC == kBf16 && !P::OpB::MN_MAJOR;
   const long tail = EVEN ? tiles : tiles % slots;
-  const int splits = EVEN ? (int)choose_splits(tiles, ktiles, ctx().sm_count / 2) : tail ? choose_tail_splits(tail, ktiles, slots, P::HALF ? 0.5 : 1.2) : 1;
+  const int splits = EVEN ? (int)choose_splits(tiles, ktiles, ctx().sm_count / 2) : tail ? choose_tail_splits(tail, ktiles, slots, P::PREC == kBf16 ? 0.5 : 1.2) : 1;
   p.ws = nullptr;
   p.k_per_split = p.K;
   p.tail_first = tiles;
@@ -380,17 +402,17 @@ struct ActPlanes {
   float *chan_partial = nullptr;
   int chan_blocks = 0;
 };
-static long padded_channels(long C, bool half) { return half ? (C + 63) / 64 * 64 : (C + 31) / 32 * 32; }
-static size_t planes_bytes(long N, long HW, long Cp, bool half) { return (size_t)N * HW * Cp * (half ? 2 : 4); }
-// `dst`: room for planes_bytes(), or null for workspace.
-template <bool HALF>
-static ActPlanes make_act_planes(const float *src, long N, long C, long H, long W, void *dst, bool want_chan_sums) {
+static long padded_channels(long C, int prec) { return prec != kTf32 ? (C + 63) / 64 * 64 : (C + 31) / 32 * 32; }
+static size_t planes_bytes(long N, long HW, long Cp, int prec) { return (size_t)N * HW * Cp * (prec == kBf16 ? 2 : 4); }
+// `dst`: room for planes_bytes(), or null for workspace.  `form`: kPairs.
+template <int PREC>
+static ActPlanes make_act_planes(const float *src, long N, long C, long H, long W, void *dst, bool want_chan_sums, const PairForm &form) {
   ActPlanes ap;
   const long HW = H * W;
-  ap.N = N; ap.H = H; ap.W = W; ap.Cp = padded_channels(C, HALF);
-  ap.p = dst ? dst : ws_alloc(planes_bytes(N, HW, ap.Cp, HALF));
+  ap.N = N; ap.H = H; ap.W = W; ap.Cp = padded_channels(C, PREC);
+  ap.p = dst ? dst : ws_alloc(planes_bytes(N, HW, ap.Cp, PREC));
   const long cap = (long)ctx().sm_count * 16;
-  const long needed = HALF ? N * ((HW + 63) / 64) * (ap.Cp / 64) : N * ((HW + 127) / 128) * (ap.Cp / 32);
+  const long needed = PREC != kTf32 ? N * ((HW + 63) / 64) * (ap.Cp / 64) : N * ((HW + 127) / 128) * (ap.Cp / 32);
   long blocks = std::min(needed, cap);
   size_t smem = 0;
   if (want_chan_sums && C <= 4096) {
@@ -403,9 +425,29 @@ static ActPlanes make_act_planes(const float *src, long N, long C, long H, long 
     ap.chan_partial = (float *)ws_alloc(sizeof(float) * blocks * C);
     smem = sizeof(float) * C;
   }
-  pdl_launch(nchw_to_planes_kernel<HALF>, (unsigned)blocks, 256, smem, src, N, (int)C, (int)HW, (int)ap.Cp, ap.p, ap.chan_partial);
+  if constexpr (PREC == kPairs)
+    pdl_launch(nchw_to_pairs_kernel, (unsigned)blocks, 256, smem, src, N, (int)C, (int)HW, (int)ap.Cp, ap.p, ap.chan_partial, form);
+  else
+    pdl_launch(nchw_to_planes_kernel<PREC == kBf16>, (unsigned)blocks, 256, smem, src, N, (int)C, (int)HW, (int)ap.Cp, ap.p, ap.chan_partial);
   check_launch("nchw_to_planes");
   return ap;
+}
+
+// ---- FP16 pairs -------------------------------------------------------------------------------------------------------
+// A zeroed record for range_kernel.
+static RangeRec *new_range_rec() { return (RangeRec *)zeroed_words(kRangeWords); }
+// Neighbours in memory are neighbours along a line wherever lines are long or lie apart.
+static RangeJob range_job(const float *p, long lines, long run, long ld, RangeRec *rec) {
+  const bool flat = (ld == run || lines == 1) && (lines < 4 || run < 64);
+  return RangeJob{p, lines, run, ld, flat, ((uintptr_t)p & 15) == 0 && (flat || ld % 4 == 0), rec};
+}
+static RangeJob range_job_flat(const float *p, long n, RangeRec *rec) { return range_job(p, 1, n, n, rec); }
+static void launch_ranges(const RangeJob &a, const RangeJob *b) {
+  auto sets = [](const RangeJob &j) { return j.flat ? (j.lines * j.run + 511) / 512 : (j.run + 127) / 128 * ((j.lines + 3) / 4); };
+  const long most = std::max(sets(a), b ? sets(*b) : 0l);
+  const dim3 grid((unsigned)std::max(1l, std::min((most + 7) / 8, ctx().sm_count * 8l)), b ? 2 : 1);
+  pdl_launch(range_kernel, grid, 256, 0, a, b ? *b : a);
+  check_launch("range");
 }
 
 // One BF16 plane of a strided matrix, rows padded to 64 values.

@@ -15,6 +15,7 @@
 
 #include <cuda.h>
 #include <cuda_bf16.h>
+#include <cuda_fp16.h>
 
 #include "thc_internal.h"
 
@@ -26,6 +27,140 @@ struct Info {
   int y, x;  // box-test coordinates contribution
 };
 constexpr int kInvalid = -(1 << 29);
+
+// What the two-SM engine multiplies.  kTf32: FP32 values, split inside the SM.  kBf16: BF16 values (opt-in mode).  kPairs: FP32
+// values that a pass over the operand has split into two FP16 halves (see RangeRec), FP32-accurate like kTf32.
+enum : int { kTf32 = 0, kBf16 = 1, kPairs = 2 };
+
+// ---- FP16 pairs --------------------------------------------------------------------------------------------------
+// x * 2^e = hi + lo * 2^-11 with hi = fp16(x * 2^e), lo = fp16((x * 2^e - hi) * 2^11), where e puts the operand's largest value into
+// [2^14, 2^15): 22 bits of every value down to 2^-29 of the largest, one more than the two TF32 parts hold (whose hi is
+// truncated), at four bytes a value and twice the tensor pipe's TF32 rate.  Below that the error stays at 2^-51 of the
+// largest value.  FP16's exponents do not reach over operands of any range, so a pass (range_kernel) measures each operand
+// first, and where one
+//   holds an infinity or a NaN,
+//   has its largest value outside [2^-60, 2^60],
+//   has a value below 2^-38 of the largest (fewer than 13 bits left), or
+//   among 512 neighbours has two groups of four with values below 2^-29 of the largest
+// all operands of the product stay in FP32, in the same buffers, and the same launch multiplies them as kTf32.
+// (A group of four may hold stray small values because tensors of 10^8 values do: the density of a layer's outputs around
+// zero leaves a few below 2^-29 of the largest.)
+struct RangeRec {
+  unsigned max_bits;     // bits of the largest |x|; infinities and NaN rank above every number
+  unsigned low_inv;      // ~(bits of the smallest non-zero |x| - 1)
+  unsigned low2_inv;     // ~(the same of the second smallest group of four in any set of 512 - 1)
+  unsigned wide;         // the operand is in FP32 whatever the others say: another operand of its product asked for it
+  unsigned ticket;
+  unsigned pad[3];
+};
+constexpr int kRangeWords = sizeof(RangeRec) / 4;
+__device__ __forceinline__ bool range_is_wide(const RangeRec &r) {
+  if (r.wide) return true;
+  if (r.max_bits == 0) return false;   // zeros only
+  const unsigned e = r.max_bits >> 23;
+  if (e < 127 - 60 || e > 127 + 60) return true;
+  const float most = __uint_as_float(r.max_bits);
+  return ~r.low_inv < __float_as_uint(most * 0x1p-38f) - 1u || ~r.low2_inv < __float_as_uint(most * 0x1p-29f) - 1u;
+}
+// 2^e of an operand that is not wide, and 2^-e
+__device__ __forceinline__ float pair_scale(const RangeRec &r) { return r.max_bits ? __uint_as_float((127u + 14u + 127u - (r.max_bits >> 23)) << 23) : 1.f; }
+__device__ __forceinline__ float pair_unscale(const RangeRec &r) { return r.max_bits ? __uint_as_float(((r.max_bits >> 23) - 14u) << 23) : 1.f; }
+// The operands whose form is decided together.  [0]: the one at hand.
+struct Ranges {
+  const RangeRec *rec[3] = {nullptr, nullptr, nullptr};
+  __device__ __forceinline__ bool wide() const {
+    bool w = false;
+#pragma unroll
+    for (int i = 0; i < 3; i++) w = w || (rec[i] && range_is_wide(*rec[i]));
+    return w;
+  }
+};
+__device__ __forceinline__ void split_pair(float a, float b, __half2 &hi, __half2 &lo) {
+  hi = __floats2half2_rn(a, b);
+  const float2 h = __half22float2(hi);
+  lo = __floats2half2_rn((a - h.x) * 2048.f, (b - h.y) * 2048.f);
+}
+__device__ __forceinline__ unsigned half2_bits(const __half2 &h) { return *reinterpret_cast<const unsigned *>(&h); }
+
+// Ranges of up to two operands (blockIdx.y), `lines` x `run` values with pitch ld.  A warp looks at 512 values at a time, in four
+// groups of 128: neighbours in memory (`flat`), or 128 neighbours in each of four lines, so that a small row or column shows in
+// several groups.
+struct RangeJob { const float *p; long lines, run, ld; int flat, vec; RangeRec *rec; };
+static __global__ void __launch_bounds__(256) range_kernel(const RangeJob ja, const RangeJob jb) {
+  pdl_begin();
+  const RangeJob &j = blockIdx.y ? jb : ja;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const long warps = (long)gridDim.x * 8, total = j.lines * j.run;
+  const long segs = j.flat ? (total + 511) / 512 : (j.run + 127) / 128, sets = j.flat ? segs : segs * ((j.lines + 3) / 4);
+  unsigned most = 0, low = ~0u, low2 = ~0u;   // the lows as bits - 1: zero becomes the largest
+  for (long s = (long)blockIdx.x * 8 + warp; s < sets; s += warps) {
+    unsigned v[4][4];
+    const long q = j.flat ? 0 : s / segs, c0 = j.flat ? s * 512 : (s - q * segs) * 128;
+#pragma unroll
+    for (int g = 0; g < 4; g++) {
+      const long line = j.flat ? 0 : q * 4 + g, c = c0 + (j.flat ? g * 128 : 0) + lane * 4, end = j.flat ? total : line < j.lines ? j.run : 0;
+      const float *src = j.p + line * j.ld + c;
+      if (j.vec && c + 4 <= end) {
+        const uint4 u = __ldg(reinterpret_cast<const uint4 *>(src));
+        v[g][0] = u.x; v[g][1] = u.y; v[g][2] = u.z; v[g][3] = u.w;
+      } else {
+#pragma unroll
+        for (int i = 0; i < 4; i++) v[g][i] = c + i < end ? __float_as_uint(__ldg(src + i)) : 0u;
+      }
+    }
+    unsigned a = ~0u, b = ~0u;   // the two smallest groups of this lane
+#pragma unroll
+    for (int g = 0; g < 4; g++) {
+      unsigned m = ~0u;
+#pragma unroll
+      for (int i = 0; i < 4; i++) {
+        const unsigned x = v[g][i] & 0x7fffffffu;
+        most = max(most, x);
+        m = min(m, x - 1u);
+      }
+      b = min(b, max(a, m));
+      a = min(a, m);
+    }
+    const unsigned first = __reduce_min_sync(0xffffffffu, a);
+    const int owner = __ffs(__ballot_sync(0xffffffffu, a == first)) - 1;
+    low = min(low, first);
+    low2 = min(low2, __reduce_min_sync(0xffffffffu, lane == owner ? b : a));
+  }
+  __shared__ unsigned sm[3][8];
+  most = __reduce_max_sync(0xffffffffu, most);
+  if (lane == 0) { sm[0][warp] = most; sm[1][warp] = low; sm[2][warp] = low2; }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int w = 1; w < 8; w++) { most = max(most, sm[0][w]); low = min(low, sm[1][w]); low2 = min(low2, sm[2][w]); }
+    if (most) atomicMax(&j.rec->max_bits, most);
+    if (~low) atomicMax(&j.rec->low_inv, ~low);
+    if (~low2) atomicMax(&j.rec->low2_inv, ~low2);
+  }
+}
+
+// What a kernel that writes an operand's planes needs in kPairs.
+struct PairForm {
+  Ranges ranges;
+  RangeRec *keep = nullptr;     // where the planes' record goes when they outlive the call (their ranges[0] does not)
+  RangeRec *remake = nullptr;   // ranges[0] of kept planes: write only if they are pairs and must be FP32 now
+  // Whether to write anything, and in which form; every thread of the block calls it.
+  __device__ __forceinline__ bool begin(bool &wide) const {
+    wide = ranges.wide();
+    return !remake || (wide && !*const_cast<const volatile unsigned *>(&remake->wide));
+  }
+  // After the block's last look at the records: the last block to get here changes what `begin` looked at.
+  __device__ __forceinline__ void end(bool wide) const {
+    if (keep && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) {
+      RangeRec r = *ranges.rec[0];
+      r.wide = wide; r.ticket = 0;
+      *keep = r;
+    }
+    if (remake) {
+      __syncthreads();
+      if (threadIdx.x == 0 && atomicAdd(&remake->ticket, 1u) == gridDim.x * gridDim.y - 1) { remake->ticket = 0; remake->wide = 1; }
+    }
+  }
+};
 
 // Division of a non-negative 31-bit integer by a runtime constant as multiply-high + shift.
 struct FastDiv {
@@ -135,21 +270,33 @@ struct Operand {
 // A plain matrix: K-major (memory runs along k) or MN-major (memory runs along the rows).  tmap: K-major {K, rows} with
 // a {KV, tile rows} box and the 128-byte swizzle; MN-major {rows, K} with a {KV rows, KV k} box per KV-row block (FP32: the
 // 32-byte-granule swizzle).  Elements beyond either extent read as zeros.
-template <bool MN_>
-struct RawOperand {
-  static constexpr bool MN_MAJOR = MN_;
+// kPairs: a row of memory is [hi values | lo values], each padded to whole spans (`lo`: distance of the two); `tmap` is over the
+// FP16 values, `tmap_wide` over the FP32 values that the buffer holds instead when a range is too wide.
+template <int PREC> struct TensorMaps {
   CUtensorMap tmap;
+  __device__ __forceinline__ const CUtensorMap *map(bool) const { return &tmap; }
+  __device__ __forceinline__ int half(bool) const { return 0; }
+};
+template <> struct TensorMaps<kPairs> {
+  CUtensorMap tmap, tmap_wide;
+  int lo;
+  __device__ __forceinline__ const CUtensorMap *map(bool wide) const { return wide ? &tmap_wide : &tmap; }
+  __device__ __forceinline__ int half(bool is_lo) const { return is_lo ? lo : 0; }
+};
+template <bool MN_, int PREC = kTf32>
+struct RawOperand : TensorMaps<PREC> {
+  static constexpr bool MN_MAJOR = MN_;
 };
 
 // Convolution windows over a channels-last plane [n_img][H][W][C] (C a multiple of KV), as rows (K-major): row = window (img,
 // y, x) of the product's grid, k = (i, j, c).  tmap: im2col map {C, W, H, n_img}, KV channels of 128 consecutive windows at
 // one filter tap per load, padding read as zeros.
-struct PlanesWindowOperand {
+template <int PREC = kTf32>
+struct PlanesWindowOperand : TensorMaps<PREC> {
   static constexpr bool MN_MAJOR = false;
-  CUtensorMap tmap;
   int n_img;
   PixelMap rows;            // window -> coordinates of its corner
-  FastDiv ctiles, kW;       // C / KV
+  FastDiv ctiles, ctiles_wide, kW;   // C / KV
   // Corner (x, y) and image of row m, the start coordinates of an im2col load; rows past the end map beyond the last
   // image, where every read is out of bounds (zeros).
   __device__ __forceinline__ void tile_origin(long m, int &x, int &y, int &img) const {
@@ -162,9 +309,9 @@ struct PlanesWindowOperand {
     img = (int)im;
   }
   // Tap (i, j) and channel tile of k tile t.
-  __device__ __forceinline__ void tile_tap(unsigned t, int &i, int &j, int &ct) const {
+  __device__ __forceinline__ void tile_tap(const FastDiv &tiles, unsigned t, int &i, int &j, int &ct) const {
     unsigned tap, cb, ii, jj;
-    ctiles.divmod(t, tap, cb);
+    tiles.divmod(t, tap, cb);
     kW.divmod(tap, ii, jj);
     i = (int)ii; j = (int)jj; ct = (int)cb;
   }
@@ -172,9 +319,9 @@ struct PlanesWindowOperand {
 
 // The same windows as the MN-major operand of the weight-gradient product: rows = (tap, c), k = windows.  tmap: im2col
 // map, KV channels of KV consecutive windows per load (one KV-row block of a k tile).
-struct WindowRowsOperand {
+template <int PREC = kTf32>
+struct WindowRowsOperand : TensorMaps<PREC> {
   static constexpr bool MN_MAJOR = true;
-  CUtensorMap tmap;
   int n_img;
   PixelMap ks;              // window -> coordinates of its corner
   FastDiv C, kW;
@@ -258,6 +405,72 @@ static __global__ void __launch_bounds__(256) nchw_to_planes_kernel(const float 
   if (chan_partial)
     for (int c = threadIdx.x; c < C; c += blockDim.x) chan_partial[(long)blockIdx.x * C + c] = chan_sum[c];
 }
+// The same as FP16 pairs, [img][pixel][hi: Cp][lo: Cp], or FP32 values in the same place.
+static __global__ void __launch_bounds__(256) nchw_to_pairs_kernel(const float *__restrict__ src, long N, int C, int HW, int Cp,
+                                                                   void *__restrict__ dst, float *__restrict__ chan_partial,
+                                                                   const PairForm form) {
+  pdl_begin();
+  bool wide;
+  if (!form.begin(wide)) return;
+  const float scale = wide ? 1.f : pair_scale(*form.ranges.rec[0]);
+  constexpr int CT = 64, PT = 64;
+  __shared__ float tile[CT][PT + 1];
+  extern __shared__ float chan_sum[];   // [C] when chan_partial is given
+  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+  const unsigned ptiles = (unsigned)((HW + PT - 1) / PT), ctiles = (unsigned)(Cp / CT);
+  const long ntiles = N * ptiles * ctiles;
+  if (chan_partial) {
+    for (int c = threadIdx.x; c < C; c += blockDim.x) chan_sum[c] = 0.f;
+    __syncthreads();
+  }
+  for (long t = blockIdx.x; t < ntiles; t += gridDim.x) {
+    const unsigned r = (unsigned)(t % (ptiles * ctiles));
+    const long img = t / (ptiles * ctiles);
+    const int ct = (int)(r / ptiles), p0 = (int)(r - ct * ptiles) * PT, c0 = ct * CT;
+    const int np = min(HW - p0, PT), nc = min(C - c0, CT);
+    const float *s = src + (img * C + c0) * HW + p0 + tx;
+    float v[CT / 8][PT / 32];
+#pragma unroll
+    for (int j = 0; j < CT / 8; j++)
+#pragma unroll
+      for (int g = 0; g < PT / 32; g++)
+        v[j][g] = (g * 32 + tx < np && ty + 8 * j < nc) ? s[(long)(ty + 8 * j) * HW + g * 32] : 0.f;
+#pragma unroll
+    for (int j = 0; j < CT / 8; j++) {
+      float part = 0.f;
+#pragma unroll
+      for (int g = 0; g < PT / 32; g++) {
+        tile[ty + 8 * j][g * 32 + tx] = v[j][g];
+        part += v[j][g];
+      }
+      if (chan_partial) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
+        if (tx == 0 && ty + 8 * j < nc) chan_sum[c0 + ty + 8 * j] += part;
+      }
+    }
+    __syncthreads();
+    const long o0 = (img * HW + p0) * Cp;
+#pragma unroll 8
+    for (int j = ty; j < np; j += 8) {
+      const float a = tile[2 * tx][j] * scale, b = tile[2 * tx + 1][j] * scale;
+      float *px = reinterpret_cast<float *>(dst) + o0 + (long)j * Cp;
+      if (wide) {
+        reinterpret_cast<float2 *>(px + c0)[tx] = make_float2(a, b);
+      } else {
+        __half2 hi, lo;
+        split_pair(a, b, hi, lo);
+        __half2 *h = reinterpret_cast<__half2 *>(px) + c0 / 2 + tx;
+        h[0] = hi;
+        h[Cp / 2] = lo;
+      }
+    }
+    __syncthreads();
+  }
+  if (chan_partial)
+    for (int c = threadIdx.x; c < C; c += blockDim.x) chan_partial[(long)blockIdx.x * C + c] = chan_sum[c];
+  form.end(wide);
+}
 // out[c] += scale * sum_b partial[b][c]: 32 row slices per channel (one warp each, eight loads in flight per
 // thread), folded in a fixed order.  The partials are a few MB at most; what this kernel costs is the chain of
 // dependent loads per thread, hence the wide block.
@@ -322,23 +535,16 @@ struct Cells {
 // looks up in a table; neighbouring threads hold neighbouring channels, i.e. neighbouring columns of a few input rows.  More
 // channels than the table holds (kCellTable: 48 KB of it) are found by division, once per 16 bytes.
 constexpr int kCellTable = 6144;
-template <bool HALF, bool TABLE>
-static __global__ void __launch_bounds__(256) cells_input_kernel(const float *__restrict__ in, void *__restrict__ S, const Cells u) {
-  pdl_begin();
-  constexpr int V = HALF ? 8 : 4;
-  extern __shared__ int2 chan_src[];      // per channel: offset in the image, (dy << 16 | dx) or -1
-  if constexpr (TABLE) {
-    for (int ch = threadIdx.x; ch < u.Cs; ch += blockDim.x) {
-      int c, dy, dx;
-      chan_src[ch] = u.channel(ch, c, dy, dx) ? make_int2((c * u.H + dy) * u.W + dx, dy << 16 | dx) : make_int2(0, -1);
-    }
-    __syncthreads();
-  }
-  const long n = blockIdx.x / u.Hs;
-  const int Y = (int)(blockIdx.x - n * u.Hs);
+// kPairs: [pixel][hi: Cs][lo: Cs], 8 channels a thread.
+template <int PREC, bool TABLE>
+__device__ __forceinline__ void cells_row(const float *__restrict__ in, void *__restrict__ S, long row, const Cells &u, const int2 *chan_src, bool wide,
+                                          float scale) {
+  constexpr int V = PREC != kTf32 ? 8 : 4;
+  const long n = row / u.Hs;
+  const int Y = (int)(row - n * u.Hs);
   const int q = u.Cs / V, chunks = u.Ws * q, y0 = Y * u.dH - u.pad;
   const float *img = in + n * u.C * (long)u.H * u.W;
-  uint4 *dst = reinterpret_cast<uint4 *>(S) + ((n * u.Hs + Y) * u.Ws) * (long)q;
+  uint4 *dst = reinterpret_cast<uint4 *>(S) + ((n * u.Hs + Y) * u.Ws) * (long)q * (PREC == kPairs ? 2 : 1);
   for (int o = blockIdx.y * blockDim.x + threadIdx.x; o < chunks; o += gridDim.y * blockDim.x) {
     const int X = o / q, ch0 = (o - X * q) * V, x0 = X * u.dW - u.pad;
     float v[V];
@@ -364,14 +570,52 @@ static __global__ void __launch_bounds__(256) cells_input_kernel(const float *__
         }
       }
     }
-    if constexpr (HALF) {
+    if constexpr (PREC == kBf16) {
       __nv_bfloat162 h[4];
 #pragma unroll
       for (int e = 0; e < 4; e++) h[e] = __floats2bfloat162_rn(v[2 * e], v[2 * e + 1]);
       dst[o] = *reinterpret_cast<const uint4 *>(h);
+    } else if constexpr (PREC == kPairs) {
+      if (wide) {
+        float4 *d = reinterpret_cast<float4 *>(dst) + 2 * (long)o;
+        d[0] = make_float4(v[0], v[1], v[2], v[3]);
+        d[1] = make_float4(v[4], v[5], v[6], v[7]);
+      } else {
+        __half2 hi[4], lo[4];
+#pragma unroll
+        for (int e = 0; e < 4; e++) split_pair(v[2 * e] * scale, v[2 * e + 1] * scale, hi[e], lo[e]);
+        uint4 *d = dst + X * 2l * q + ch0 / V;
+        d[0] = *reinterpret_cast<const uint4 *>(hi);
+        d[q] = *reinterpret_cast<const uint4 *>(lo);
+      }
     } else {
       dst[o] = make_uint4(__float_as_uint(v[0]), __float_as_uint(v[1]), __float_as_uint(v[2]), __float_as_uint(v[3]));
     }
+  }
+}
+template <int PREC, bool TABLE>
+static __global__ void __launch_bounds__(256) cells_input_kernel(const float *__restrict__ in, void *__restrict__ S, long N, const Cells u,
+                                                                 const PairForm form) {
+  pdl_begin();
+  bool wide = false;
+  float scale = 1.f;
+  if constexpr (PREC == kPairs) {
+    if (!form.begin(wide)) return;
+    if (!wide) scale = pair_scale(*form.ranges.rec[0]);
+  }
+  extern __shared__ int2 chan_src[];      // per channel: offset in the image, (dy << 16 | dx) or -1
+  if constexpr (TABLE) {
+    for (int ch = threadIdx.x; ch < u.Cs; ch += blockDim.x) {
+      int c, dy, dx;
+      chan_src[ch] = u.channel(ch, c, dy, dx) ? make_int2((c * u.H + dy) * u.W + dx, dy << 16 | dx) : make_int2(0, -1);
+    }
+    __syncthreads();
+  }
+  if constexpr (PREC == kPairs) {
+    for (long row = blockIdx.x; row < N * u.Hs; row += gridDim.x) cells_row<PREC, TABLE>(in, S, row, u, chan_src, wide, scale);
+    form.end(wide);
+  } else {
+    cells_row<PREC, TABLE>(in, S, blockIdx.x, u, chan_src, wide, scale);   // (a loop over rows costs 98 -> 117 us at 256 images)
   }
 }
 
@@ -415,14 +659,22 @@ static __global__ void __launch_bounds__(256) columns8_kernel(const float *__res
 // pair_shift > 0 (pixel-pair mode, see Epilogue): the filter is widened to kWs + pair_shift columns and
 // stored twice, rows [0, rows) as it is (output parity 0) and rows [rows, 2 rows) shifted right by pair_shift
 // columns (parity 1, whose window starts one stride later); the new columns are zero.
-template <bool HALF, bool FLIP>
+// kPairs: a row is [hi: its values][lo: its values].
+template <int PREC, bool FLIP>
 static __global__ void __launch_bounds__(256) repack_weight_kernel(const float *__restrict__ w, const Cells u, int K, int rows, int chans,
-                                                                   int pair_shift, void *__restrict__ out) {
+                                                                   int pair_shift, void *__restrict__ out, const Ranges ranges) {
   pdl_begin();
+  bool wide = false;
+  float scale = 1.f;
+  if constexpr (PREC == kPairs) {
+    wide = ranges.wide();
+    if (!wide) scale = pair_scale(*ranges.rec[0]);
+  }
   const int kWe = u.kWs + pair_shift, quads = u.kHs * kWe * (chans / 4);
   const unsigned total = (unsigned)((pair_shift ? 2 : 1) * rows) * (unsigned)quads;
   for (unsigned t = blockIdx.x * blockDim.x + threadIdx.x; t < total; t += gridDim.x * blockDim.x) {
     int r = (int)(t / (unsigned)quads);
+    const long row = r;
     const int k = (int)(t - (unsigned)r * quads) * 4, tap = k / chans, k0 = k - tap * chans;
     const int par = r >= rows ? 1 : 0;
     r -= par * rows;
@@ -437,7 +689,14 @@ static __global__ void __launch_bounds__(256) repack_weight_kernel(const float *
       const int i = dy + bi * u.stepH, j = dx + bj * u.stepW;
       v[e] = real && ko < K && bj >= 0 && bj < u.kWs && i < u.kH && j < u.kW ? w[(((long)ko * u.C + c) * u.kH + i) * u.kW + j] : 0.f;
     }
-    if constexpr (HALF) {
+    if (PREC == kPairs && !wide) {
+      __half2 hi[2], lo[2];
+      split_pair(v[0] * scale, v[1] * scale, hi[0], lo[0]);
+      split_pair(v[2] * scale, v[3] * scale, hi[1], lo[1]);
+      uint2 *o = reinterpret_cast<uint2 *>(out) + row * 2 * quads + k / 4;
+      o[0] = make_uint2(half2_bits(hi[0]), half2_bits(hi[1]));
+      o[quads] = make_uint2(half2_bits(lo[0]), half2_bits(lo[1]));
+    } else if constexpr (PREC == kBf16) {
       const __nv_bfloat162 a = __floats2bfloat162_rn(v[0], v[1]), b = __floats2bfloat162_rn(v[2], v[3]);
       reinterpret_cast<uint2 *>(out)[t] = make_uint2(*reinterpret_cast<const unsigned *>(&a), *reinterpret_cast<const unsigned *>(&b));
     } else {
@@ -483,6 +742,45 @@ static __global__ void __launch_bounds__(256) unfold_grad_input_kernel(const flo
       float v = 0.f;
       if (Y < u.Hs && X < u.Ws && dy < u.eH && dx < u.eW) v = src[((long)((dy * u.eW + dx) * u.Cq + c) * u.Hs + Y) * u.Ws + X];
       gin[pl * HW + t] = v;
+    }
+  }
+}
+
+// Up to two matrices (blockIdx.y) as FP16 pairs: lines of `run` values become [hi: ldp][lo: ldp], ldp = run padded with zeros to whole
+// spans, or lines of ldp FP32 values.  A warp takes 512 values of a line, all loads in flight before the first store.
+struct PairJob { const float *src; void *dst; long lines, run, ld, ldp; int vec; Ranges ranges; };
+static __global__ void __launch_bounds__(256) split_matrix_kernel(const PairJob a, const PairJob b) {
+  pdl_begin();
+  const PairJob &j = blockIdx.y ? b : a;
+  const bool wide = j.ranges.wide();
+  const float scale = wide ? 1.f : pair_scale(*j.ranges.rec[0]);
+  const int lane = threadIdx.x & 31;
+  const long warps = (long)gridDim.x * 8, parts = (j.ldp + 511) / 512;
+  for (long w = (long)blockIdx.x * 8 + (threadIdx.x >> 5); w < j.lines * parts; w += warps) {
+    const long l = w / parts, c0 = (w - l * parts) * 512 + lane * 4;
+    const float *s = j.src + l * j.ld;
+    float4 v[4];
+#pragma unroll
+    for (int g = 0; g < 4; g++) {
+      const long c = c0 + g * 128;
+      if (j.vec && c + 4 <= j.run) v[g] = __ldg(reinterpret_cast<const float4 *>(s + c));
+      else v[g] = make_float4(c < j.run ? s[c] : 0.f, c + 1 < j.run ? s[c + 1] : 0.f, c + 2 < j.run ? s[c + 2] : 0.f, c + 3 < j.run ? s[c + 3] : 0.f);
+    }
+    float *d = reinterpret_cast<float *>(j.dst) + l * j.ldp;
+#pragma unroll
+    for (int g = 0; g < 4; g++) {
+      const long c = c0 + g * 128;
+      if (c >= j.ldp) break;
+      if (wide) {
+        *reinterpret_cast<float4 *>(d + c) = v[g];
+      } else {
+        __half2 hi[2], lo[2];
+        split_pair(v[g].x * scale, v[g].y * scale, hi[0], lo[0]);
+        split_pair(v[g].z * scale, v[g].w * scale, hi[1], lo[1]);
+        uint2 *h = reinterpret_cast<uint2 *>(reinterpret_cast<__half *>(d) + c);
+        h[0] = make_uint2(half2_bits(hi[0]), half2_bits(hi[1]));
+        h[j.ldp / 4] = make_uint2(half2_bits(lo[0]), half2_bits(lo[1]));
+      }
     }
   }
 }
@@ -604,13 +902,16 @@ struct Epilogue {
   }
 };
 
-template <class OpA_, class OpB_, bool PAIR_ = false, bool HALF_ = false>
+template <class OpA_, class OpB_, bool PAIR_ = false, int PREC_ = kTf32>
 struct Problem {
   typedef OpA_ OpA;
   typedef OpB_ OpB;
   static constexpr bool PAIR = PAIR_;   // pixel-pair epilogue (see Epilogue)
-  static constexpr bool HALF = HALF_;   // BF16 operands (two-SM engine)
-  static constexpr int KV = HALF_ ? 64 : 32;   // k per tile of the two-SM engine
+  static constexpr int PREC = PREC_;    // operands of the two-SM engine
+  static constexpr int KV = PREC_ != kTf32 ? 64 : 32;   // k per tile of the two-SM engine
+  // kPairs: the operands' records, and all that decide on the form
+  const RangeRec *range_a = nullptr, *range_b = nullptr;
+  Ranges ranges;
   OpA a;
   OpB b;
   Epilogue epi;

@@ -1,4 +1,5 @@
-// Two-SM tcgen05 engine over operands fetched by TMA: FP32 values as 3xTF32 products split inside the SM, or BF16 values.
+// Two-SM tcgen05 engine over operands fetched by TMA: FP32 values as 3xTF32 products split inside the SM, FP32 values that come as
+// FP16 pairs, or BF16 values.
 //
 // A cluster of two CTAs on neighbouring SMs computes one 256 x BN2 tile of D (BN2 = 64, 128, 192 or 256): CTA r of the pair
 // stages rows [128 r, 128 r + 128) of the A tile and rows [BN2/2 r, BN2/2 (r+1)) of the B tile in its own shared
@@ -11,6 +12,15 @@
 // the `lo` slot at the same offsets (both slots share one layout, K-major or MN-major alike).  Twelve MMAs per 32-k tile,
 // Alo*Bhi + Ahi*Blo + Ahi*Bhi, go into one of two TMEM buffers and are added into FP32 registers with
 // round-to-nearest (the tensor core's own accumulation truncates, so chains stay 12 MMAs long).
+//
+// FP16 pairs (RangeRec, mm_problem.cuh): the same three products from halves that a pass over the operands has made, at twice the
+// rate of TF32 and without the splitters' shared-memory traffic.  A ring slot holds one half of a 64-k tile, lo before hi, and
+// twelve kind::f16 MMAs multiply a tile: Alo*Bhi + Ahi*Blo at 2^11 times their size, which the first of Ahi*Bhi scales back
+// (scale-input-d).  Each tile has an accumulator of its own, as in TF32, whose chain of full-size additions is as long (four MMAs)
+// over twice the k, so that the error is smaller: 4096^3 of normal values 1.95e-7 of the result's norm against 2.94e-7 (2048^3
+// 1.70e-7 / 2.61e-7, 8192^3 2.44e-7 / 3.60e-7).  Time with the passes over the operands: 4096^3 659 -> 430 us, 8192^3 4.78 -> 2.69 ms;
+// the 256-wide convolution launches of 1024 images run 500-570 TFLOP/s where TF32 had 240-250 (its ceiling 277).
+// What bounds it: the wide tiles the tensor pipe under the power cap (570 TFLOP/s = 1.7 PFLOP/s of MMAs).
 //
 // BF16 (opt-in math mode): no splitters and no lo slots, four kind::f16 MMAs per 64-k tile, one MMA thread; products are exact
 // in FP32 and the tolerance of the mode is BF16's, so four k tiles (16 MMAs) chain in one accumulator before a drain.  In
@@ -50,7 +60,8 @@ constexpr int T2R_HALF_CHAIN = 4;   // BF16: k tiles accumulated in tensor memor
 constexpr int T2R_TMA_WARP = 5;
 constexpr int T2R_MMA_WARP2 = 6;
 
-template <int BN2, bool HALF> struct Tc2rCfg {
+template <int BN2, int PREC> struct Tc2rCfg {
+  static constexpr bool HALF = PREC != kTf32;
   static constexpr int BH = BN2 / 2;
   static constexpr int A_BYTES = TC_BM * 128;
   static constexpr int B_BYTES = BH * 128;
@@ -63,6 +74,12 @@ template <int BN2, bool HALF> struct Tc2rCfg {
   static_assert(HI_SLOTS >= LO_SLOTS, "ring sizes");
   static_assert(HALF || HI_SLOTS % 2 == 0 || HI_SLOTS <= LO_SLOTS + 2, "an odd hi ring must not be longer than the lo ring + 2 (parity waits of the two MMA threads)");
 };
+
+// What a launch asks for: one over pairs may have to run as kTf32.
+template <int BN2, int PREC> __host__ __device__ constexpr int tc2r_smem_bytes() {
+  constexpr int own = Tc2rCfg<BN2, PREC>::SMEM_BYTES, wide = Tc2rCfg<BN2, kTf32>::SMEM_BYTES;
+  return PREC == kPairs && wide > own ? wide : own;
+}
 
 // lo = tf32(x - trunc_tf32(x)) of four values
 __device__ __forceinline__ uint4 tf32_lo4(const uint4 &v) {
@@ -93,28 +110,34 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst, const void *tmap, int 
       ::"r"(dst), "l"((unsigned long long)tmap), "r"(mbar), "r"(x), "r"(y)
       : "memory");
 }
-template <int ROWS, int KV, bool MN>
-__device__ __forceinline__ void tma_issue(const RawOperand<MN> &op, uint32_t dst, long row0, long k0, uint32_t mbar) {
+// PREC: the form the operand's buffer is in; `lo`: the second half of a pair.
+template <int ROWS, int PREC, bool WIDE, bool MN, int OWN>
+__device__ __forceinline__ void tma_issue(const RawOperand<MN, OWN> &op, uint32_t dst, long row0, long k0, bool lo, uint32_t mbar) {
+  constexpr int KV = PREC == kTf32 ? 32 : 64;
+  const CUtensorMap *map = op.map(WIDE);
+  const int off = op.half(lo);
   if constexpr (MN) {
     static_assert(ROWS % KV == 0, "whole row blocks");
 #pragma unroll
-    for (int a = 0; a < ROWS / KV; a++) tma_load_2d(dst + a * KV * 128, &op.tmap, (int)row0 + KV * a, (int)k0, mbar);
+    for (int a = 0; a < ROWS / KV; a++) tma_load_2d(dst + a * KV * 128, map, (int)row0 + KV * a + off, (int)k0, mbar);
   } else {
-    tma_load_2d(dst, &op.tmap, (int)k0, (int)row0, mbar);
+    tma_load_2d(dst, map, (int)k0 + off, (int)row0, mbar);
   }
 }
 // Convolution windows as rows (K-major): one im2col load of KV channels of ROWS = 128 consecutive windows.
-template <int ROWS, int KV>
-__device__ __forceinline__ void tma_issue(const PlanesWindowOperand &op, uint32_t dst, long row0, long k0, uint32_t mbar) {
+template <int ROWS, int PREC, bool WIDE, int OWN>
+__device__ __forceinline__ void tma_issue(const PlanesWindowOperand<OWN> &op, uint32_t dst, long row0, long k0, bool lo, uint32_t mbar) {
+  constexpr int KV = PREC == kTf32 ? 32 : 64;
   static_assert(ROWS == TC_BM, "the window map loads 128 windows");
   int x, y, img, i, j, ct;
   op.tile_origin(row0, x, y, img);
-  op.tile_tap((unsigned)(k0 / KV), i, j, ct);
-  tma_load_windows(dst, &op.tmap, ct * KV, x, y, img, j, i, mbar);
+  op.tile_tap(WIDE ? op.ctiles_wide : op.ctiles, (unsigned)(k0 / KV), i, j, ct);
+  tma_load_windows(dst, op.map(WIDE), ct * KV + op.half(lo), x, y, img, j, i, mbar);
 }
 // Convolution windows as the reduction (MN-major): per KV-row block, KV channels of KV consecutive windows.
-template <int ROWS, int KV>
-__device__ __forceinline__ void tma_issue(const WindowRowsOperand &op, uint32_t dst, long row0, long k0, uint32_t mbar) {
+template <int ROWS, int PREC, bool WIDE, int OWN>
+__device__ __forceinline__ void tma_issue(const WindowRowsOperand<OWN> &op, uint32_t dst, long row0, long k0, bool lo, uint32_t mbar) {
+  constexpr int KV = PREC == kTf32 ? 32 : 64;
   static_assert(ROWS % KV == 0, "whole row blocks");
   int x, y, img;
   op.pixel_origin(k0, x, y, img);
@@ -122,7 +145,7 @@ __device__ __forceinline__ void tma_issue(const WindowRowsOperand &op, uint32_t 
   for (int a = 0; a < ROWS / KV; a++) {
     int i, j, c0;
     op.row_tap(row0 + KV * a, i, j, c0);
-    tma_load_windows(dst + a * KV * 128, &op.tmap, c0, x, y, img, j, i, mbar);
+    tma_load_windows(dst + a * KV * 128, op.map(WIDE), c0 + op.half(lo), x, y, img, j, i, mbar);
   }
 }
 
@@ -141,7 +164,7 @@ constexpr int T2R_SCHED = 8;
 constexpr int T2R_SCHED_WARP = 7;
 constexpr uint32_t T2R_NO_ITEM = 0xffffffffu;
 constexpr int T2R_ITEM_WAIT_SHIFT = 6;   // item-level waits may take 64 k-tile limits (see mbar_wait)
-// readers per slot: TMA thread, 4 splitter warps (BF16: one relay), 8 drain warps in each CTA, the MMA threads in the leader
+// readers per slot: TMA thread, 4 splitter warps (16-bit operands: one relay), 8 drain warps in each CTA, the MMA threads in the leader
 template <bool HALF> struct Tc2rReaders { static constexpr uint32_t count = 2 * (1 + (HALF ? 1 : 4) + T2_DRAIN_WARPS) + (HALF ? 1 : 2); };
 
 __device__ __forceinline__ void mbar_arrive_local(uint32_t bar) {
@@ -179,16 +202,18 @@ struct Tc2rItem {
 // rings, barrier phases and accumulator buffers run on with a k-tile count `g` that spans the items, so the
 // loads, splits and first MMAs of an item run under the previous item's epilogue stores, and the barrier and
 // tensor-memory set-up is paid once per launch.
-template <class P, int BN2>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(T2_THREADS, 1) tc2r_kernel(const __grid_constant__ P p, const StallCtl ctl,
-                                                                                                unsigned *sched_counter) {
-  constexpr bool HALF = P::HALF;
-  constexpr int KV = P::KV;
-  typedef Tc2rCfg<BN2, HALF> Cfg;
+// PREC: what is multiplied; WIDE: operands meant as FP16 pairs that are in FP32 (kTf32 then).
+template <class P, int BN2, int PREC, bool WIDE>
+__device__ __forceinline__ void tc2r_run(const P &p, const StallCtl &ctl, unsigned *sched_counter) {
+  constexpr bool HALF = PREC != kTf32;     // operands of 16 bits: nothing is split here
+  constexpr bool PAIRS = PREC == kPairs;
+  constexpr int PARTS = PAIRS ? 2 : 1;     // ring slots of a k tile: lo, then hi, which is needed longest
+  constexpr int KV = HALF ? 64 : 32;
+  constexpr int CHAIN = PAIRS ? 1 : T2R_HALF_CHAIN;
+  typedef Tc2rCfg<BN2, PREC> Cfg;
   constexpr int R = Cfg::HI_SLOTS, L = Cfg::LO_SLOTS, LM = L > 0 ? L : 1;
   constexpr int BH = Cfg::BH;
   extern __shared__ uint8_t smem_raw[];
-  pdl_wait();
   uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   uint8_t *lo_ring = smem + R * Cfg::SLOT_BYTES;
   uint8_t *aux = lo_ring + L * Cfg::SLOT_BYTES;
@@ -272,7 +297,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(T2_THREADS, 1) tc2r_
     setmaxnreg_dec<72>();
     const uint32_t full_leader = mapa_shared(bar_full, 0);
     if constexpr (HALF) {
-      // BF16 tiles are ready as they land: one thread tells CTA 0 so
+      // 16-bit tiles are ready as they land: one thread tells CTA 0 so
       if (warp == 0 && lane == 0) {
         int g0 = 0;
         for (uint32_t n = 0; ok; n++) {
@@ -281,7 +306,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(T2_THREADS, 1) tc2r_
           if (!ok) break;
           sched.done(n);
           if (w == T2R_NO_ITEM) break;
-          const int nk = item_at(w).num_k_tiles;
+          const int nk = item_at(w).num_k_tiles * PARTS;
           for (int it = 0; it < nk; it++) {
             const int g = g0 + it, s = g % R;
             ok = mbar_wait(bar_raw + 8 * s, (uint32_t)(g / R) & 1u, abort_flag, kWaitRawTile);
@@ -340,8 +365,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(T2_THREADS, 1) tc2r_
   } else if (warp < T2_DRAIN_WARP0) {
     setmaxnreg_dec<40>();
     if (HALF && warp == T2_MMA_WARP && lane == 0 && rank == 0) {
-      // ---------------------------------------------------------- MMA issuer, BF16: one thread, T2R_HALF_CHAIN k tiles per buffer
-      constexpr uint32_t idesc = umma2_idesc_bf16(BN2, P::OpA::MN_MAJOR, P::OpB::MN_MAJOR);
+      // ---------------------------------------------------------- MMA issuer of 16-bit operands: one thread, CHAIN k tiles per buffer
+      constexpr bool A_MN = P::OpA::MN_MAJOR, B_MN = P::OpB::MN_MAJOR;
+      constexpr uint32_t idesc = PAIRS ? umma2_idesc_f16(BN2, A_MN, B_MN) : umma2_idesc_bf16(BN2, A_MN, B_MN);
       int g = 0, grp = 0;
       for (uint32_t n = 0; ok; n++) {
         uint32_t w = T2R_NO_ITEM;
@@ -351,22 +377,45 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(T2_THREADS, 1) tc2r_
         if (w == T2R_NO_ITEM) break;
         const int nk = item_at(w).num_k_tiles;
         for (int it = 0; it < nk; it++, g++) {
-          const int s = g % R, buf = grp & 1;
-          const bool first = it % T2R_HALF_CHAIN == 0, last = it % T2R_HALF_CHAIN == T2R_HALF_CHAIN - 1 || it == nk - 1;
-          if (first) ok = mbar_wait_spin(bar_acc_empty + 8 * buf, ((uint32_t)(grp >> 1) & 1u) ^ 1u, abort_flag, kWaitAccEmpty);
-          ok = ok && mbar_wait_spin(bar_full + 8 * s, (uint32_t)(g / R) & 1u, abort_flag, kWaitTileFull);
-          if (!ok) break;
-          tc_fence_after();
-          const uint32_t st = smem_u32(smem + s * Cfg::SLOT_BYTES);
-          const uint64_t a_d = umma_desc_half<P::OpA::MN_MAJOR>(st), b_d = umma_desc_half<P::OpB::MN_MAJOR>(st + Cfg::A_BYTES);
+          const int buf = grp & 1;
+          const bool first = it % CHAIN == 0, last = it % CHAIN == CHAIN - 1 || it == nk - 1;
           const uint32_t d = tmem_base + (uint32_t)(buf * BN2);
+          if (first) ok = mbar_wait_spin(bar_acc_empty + 8 * buf, ((uint32_t)(grp >> 1) & 1u) ^ 1u, abort_flag, kWaitAccEmpty);
+          if constexpr (PAIRS) {
+            const int gl = 2 * g, sl = gl % R, sh = (gl + 1) % R;
+            ok = ok && mbar_wait_spin(bar_full + 8 * sl, (uint32_t)(gl / R) & 1u, abort_flag, kWaitTileFull);
+            ok = ok && mbar_wait_spin(bar_full + 8 * sh, (uint32_t)((gl + 1) / R) & 1u, abort_flag, kWaitTileFull);
+            if (!ok) break;
+            tc_fence_after();
+            const uint32_t lo = smem_u32(smem + sl * Cfg::SLOT_BYTES), hi = smem_u32(smem + sh * Cfg::SLOT_BYTES);
+            const uint64_t a_lo = umma_desc_half<A_MN>(lo), b_lo = umma_desc_half<B_MN>(lo + Cfg::A_BYTES);
+            const uint64_t a_hi = umma_desc_half<A_MN>(hi), b_hi = umma_desc_half<B_MN>(hi + Cfg::A_BYTES);
 #pragma unroll
-          for (int kk = 0; kk < 4; kk++) {   // 16 k per MMA
-            const uint64_t adv_a = (uint64_t)((kk * umma_kstep_bytes_half<P::OpA::MN_MAJOR>()) >> 4);
-            const uint64_t adv_b = (uint64_t)((kk * umma_kstep_bytes_half<P::OpB::MN_MAJOR>()) >> 4);
-            umma2_bf16(d, a_d + adv_a, b_d + adv_b, idesc, (kk || !first) ? 1u : 0u);
+            for (int kk = 0; kk < 4; kk++) {   // 16 k per MMA; these two carry 2^11
+              const uint64_t adv_a = (uint64_t)((kk * umma_kstep_bytes_half<A_MN>()) >> 4), adv_b = (uint64_t)((kk * umma_kstep_bytes_half<B_MN>()) >> 4);
+              umma2_f16(d, a_lo + adv_a, b_hi + adv_b, idesc, kk ? 1u : 0u);
+              umma2_f16(d, a_hi + adv_a, b_lo + adv_b, idesc, 1u);
+            }
+            umma2_commit_both(bar_empty + 8 * sl);
+            umma2_f16_scale11(d, a_hi, b_hi, idesc);
+#pragma unroll
+            for (int kk = 1; kk < 4; kk++)
+              umma2_f16(d, a_hi + (uint64_t)((kk * umma_kstep_bytes_half<A_MN>()) >> 4), b_hi + (uint64_t)((kk * umma_kstep_bytes_half<B_MN>()) >> 4), idesc, 1u);
+            umma2_commit_both(bar_empty + 8 * sh);
+          } else {
+            const int s = g % R;
+            ok = ok && mbar_wait_spin(bar_full + 8 * s, (uint32_t)(g / R) & 1u, abort_flag, kWaitTileFull);
+            if (!ok) break;
+            tc_fence_after();
+            const uint32_t st = smem_u32(smem + s * Cfg::SLOT_BYTES);
+            const uint64_t a_d = umma_desc_half<A_MN>(st), b_d = umma_desc_half<B_MN>(st + Cfg::A_BYTES);
+#pragma unroll
+            for (int kk = 0; kk < 4; kk++) {   // 16 k per MMA
+              const uint64_t adv_a = (uint64_t)((kk * umma_kstep_bytes_half<A_MN>()) >> 4), adv_b = (uint64_t)((kk * umma_kstep_bytes_half<B_MN>()) >> 4);
+              umma2_f16(d, a_d + adv_a, b_d + adv_b, idesc, (kk || !first) ? 1u : 0u);
+            }
+            umma2_commit_both(bar_empty + 8 * s);
           }
-          umma2_commit_both(bar_empty + 8 * s);
           if (last) { umma2_commit_both(bar_acc_full + 8 * buf); grp++; }
         }
       }
@@ -435,17 +484,19 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(T2_THREADS, 1) tc2r_
         if (rank == 0) mbar_arrive_local(bar_sched_go);   // item n is under way: time to fetch the number of item n + 1
         const Tc2rItem item = item_at(w);
         const long m0 = item.m_tile0 + (long)rank * TC_BM, n0 = item.n_tile0 + (long)rank * BH;
-        for (int t = 0; t < item.num_k_tiles; t++) {
+        const int parts = item.num_k_tiles * PARTS;
+        for (int t = 0; t < parts; t++) {
           const int g = g0 + t;
           const int s = g % R;
           if (g >= R && !mbar_wait(bar_empty + 8 * s, (uint32_t)((g - R) / R) & 1u, abort_flag, kWaitSlotEmpty)) { ok = false; break; }
-          const long k0 = item.k_begin + (long)t * KV;
+          const long k0 = item.k_begin + (long)(t / PARTS) * KV;
+          const bool lo = PAIRS && t % PARTS == 0;
           const uint32_t slot = smem_u32(smem + s * Cfg::SLOT_BYTES);
           mbar_arrive_expect_tx(bar_raw + 8 * s, (uint32_t)Cfg::SLOT_BYTES);
-          tma_issue<TC_BM, KV>(p.a, slot, m0, k0, bar_raw + 8 * s);
-          tma_issue<BH, KV>(p.b, slot + Cfg::A_BYTES, n0, k0, bar_raw + 8 * s);
+          tma_issue<TC_BM, PREC, WIDE>(p.a, slot, m0, k0, lo, bar_raw + 8 * s);
+          tma_issue<BH, PREC, WIDE>(p.b, slot + Cfg::A_BYTES, n0, k0, lo, bar_raw + 8 * s);
         }
-        g0 += item.num_k_tiles;
+        g0 += parts;
       }
     } else if (warp == T2R_SCHED_WARP && lane == 0 && rank == 0) {
       // ---------------------------------------------------------- item hand-out (one thread per cluster)
@@ -473,6 +524,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(T2_THREADS, 1) tc2r_
     // Pixel-pair products over 64 planes (a 128-column tile: parity 0 in columns 0-63, parity 1 in 64-127): this warp
     // takes 32 planes in both parities instead of 64 columns of one, for the whole-line epilogue
     const bool pair_capable = P::PAIR && BN2 == 128 && p.epi.pair_K == 64 && p.epi.beta == 0.f;
+    float unscale_a = 1.f, unscale_b = 1.f;
+    if constexpr (PAIRS) { unscale_a = pair_unscale(*p.range_a); unscale_b = pair_unscale(*p.range_b); }
     int g0 = 0;
     for (uint32_t n = 0; ok; n++) {
       uint32_t w = T2R_NO_ITEM;
@@ -485,7 +538,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(T2_THREADS, 1) tc2r_
       float acc[NCOL];
 #pragma unroll
       for (int j = 0; j < NCOL; j++) acc[j] = 0.f;
-      const int folds = HALF ? (item.num_k_tiles + T2R_HALF_CHAIN - 1) / T2R_HALF_CHAIN : item.num_k_tiles;   // accumulators of this item
+      const int folds = HALF ? (item.num_k_tiles + CHAIN - 1) / CHAIN : item.num_k_tiles;   // accumulators of this item
       for (int it = 0; it < folds; it++) {
         const int g = g0 + it;
         const int buf = g & 1;
@@ -508,6 +561,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(T2_THREADS, 1) tc2r_
         if (lane == 0) mbar_arrive_cluster(acc_empty_leader + 8 * buf);
       }
       g0 += folds;
+      if constexpr (PAIRS) {
+#pragma unroll
+        for (int j = 0; j < NCOL; j++) acc[j] = acc[j] * unscale_a * unscale_b;
+      }
       if (ok) {
         const long m = item.m_tile0 + (long)rank * TC_BM + q * 32 + lane;
         if (item.z >= 0) {
@@ -529,6 +586,17 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(T2_THREADS, 1) tc2r_
   __syncthreads();
   cluster_sync_all();
   if (warp == T2_MMA_WARP) tmem_dealloc2(tmem_base, Cfg::TMEM_COLS);
+}
+template <class P, int BN2>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(T2_THREADS, 1) tc2r_kernel(const __grid_constant__ P p, const StallCtl ctl,
+                                                                                                unsigned *sched_counter) {
+  pdl_wait();
+  if constexpr (P::PREC == kPairs) {
+    if (p.ranges.wide()) tc2r_run<P, BN2, kTf32, true>(p, ctl, sched_counter);
+    else tc2r_run<P, BN2, kPairs, false>(p, ctl, sched_counter);
+  } else {
+    tc2r_run<P, BN2, P::PREC, false>(p, ctl, sched_counter);
+  }
 }
 
 }  // namespace mm

@@ -55,8 +55,8 @@ static void gemm_raw_t(const float *a, long lda, const float *b, long ldb, long 
   p.epi = epi;
   p.M = m; p.N = n; p.K = k;
   launch_raw(p, [&](auto &q, int bn2) {
-    attach_raw_map<false>(q.a, a, m, k, lda, TC_BM);
-    attach_raw_map<false>(q.b, b, n, k, ldb, bn2 / 2);
+    attach_raw_map<kTf32>(q.a, a, m, k, lda, TC_BM);
+    attach_raw_map<kTf32>(q.b, b, n, k, ldb, bn2 / 2);
   });
 }
 // One side of a product: element (r, l) at p[l + r * ld] (along_k) or p[r + l * ld].
@@ -77,14 +77,14 @@ static mm::Epilogue gemm_sides(GemmSide &x, GemmSide &y, float alpha, float beta
 // than 32 columns; smaller ones stay FP32-accurate.
 static void gemm_half(GemmSide x, GemmSide y, long k, float alpha, float beta, float *c, long ldc, const float *row_bias) {
   using namespace mm;
-  Problem<RawOperand<false>, RawOperand<false>, false, true> p;
+  Problem<RawOperand<false, kBf16>, RawOperand<false, kBf16>, false, kBf16> p;
   p.epi = gemm_sides(x, y, alpha, beta, c, ldc, row_bias);
   const HalfMatrix hx = make_half_matrix(x.p, x.along_k ? x.ld : 1, x.along_k ? 1 : x.ld, x.rows, k);
   const HalfMatrix hy = make_half_matrix(y.p, y.along_k ? y.ld : 1, y.along_k ? 1 : y.ld, y.rows, k);
   p.M = x.rows; p.N = y.rows; p.K = hx.ld;
   launch_raw(p, [&](auto &q, int bn2) {
-    attach_raw_map<true>(q.a, hx.p, x.rows, hx.ld, hx.ld, TC_BM);
-    attach_raw_map<true>(q.b, hy.p, y.rows, hy.ld, hy.ld, bn2 / 2);
+    attach_raw_map<kBf16>(q.a, hx.p, x.rows, hx.ld, hx.ld, TC_BM);
+    attach_raw_map<kBf16>(q.b, hy.p, y.rows, hy.ld, hy.ld, bn2 / 2);
   });
 }
 static void gemm_raw(GemmSide x, GemmSide y, long k, float alpha, float beta, float *c, long ldc, const float *row_bias) {
@@ -110,6 +110,49 @@ static void gemm_raw(GemmSide x, GemmSide y, long k, float alpha, float beta, fl
   else if (x.along_k && y.along_k) gemm_raw_t<false, false>(x.p, x.ld, y.p, y.ld, x.rows, y.rows, k, epi);
   else if (!x.along_k) gemm_raw_t<true, true>(x.p, x.ld, y.p, y.ld, x.rows, y.rows, k, epi);
   else gemm_raw_t<false, true>(x.p, x.ld, y.p, y.ld, x.rows, y.rows, k, epi);
+}
+// The same over FP16 pairs: a pass measures both operands and one splits them, each as it lies in memory.
+template <bool A_MN, bool B_MN>
+static void gemm_pairs_t(const void *a, long lda, const void *b, long ldb, long m, long n, long k, const mm::Epilogue &epi, const mm::RangeRec *ra,
+                         const mm::RangeRec *rb) {
+  using namespace mm;
+  Problem<RawOperand<A_MN, kPairs>, RawOperand<B_MN, kPairs>, false, kPairs> p;
+  p.epi = epi;
+  p.M = m; p.N = n; p.K = k;
+  p.range_a = ra; p.range_b = rb; p.ranges.rec[0] = ra; p.ranges.rec[1] = rb;
+  launch_raw(p, [&](auto &q, int bn2) {
+    attach_raw_map<kPairs>(q.a, a, m, k, lda, TC_BM);
+    attach_raw_map<kPairs>(q.b, b, n, k, ldb, bn2 / 2);
+  });
+}
+static void gemm_pairs(GemmSide x, GemmSide y, long k, float alpha, float beta, float *c, long ldc, const float *row_bias) {
+  using namespace mm;
+  const Epilogue epi = gemm_sides(x, y, alpha, beta, c, ldc, row_bias);
+  RangeRec *rec[2] = {new_range_rec(), new_range_rec()};
+  RangeJob ranges[2];
+  PairJob jobs[2];
+  const GemmSide *sides[2] = {&x, &y};
+  long pieces = 0;
+  for (int i = 0; i < 2; i++) {
+    const GemmSide &s = *sides[i];
+    const long lines = s.along_k ? s.rows : k, run = s.along_k ? k : s.rows, ldp = (run + 63) / 64 * 64;
+    ranges[i] = range_job(s.p, lines, run, s.ld, rec[i]);
+    jobs[i] = PairJob{s.p, ws_alloc(sizeof(float) * lines * ldp), lines, run, s.ld, ldp, ((uintptr_t)s.p & 15) == 0 && s.ld % 4 == 0, {}};
+    jobs[i].ranges.rec[0] = rec[i]; jobs[i].ranges.rec[1] = rec[1 - i];
+    pieces = std::max(pieces, lines * ((ldp + 511) / 512));
+  }
+  launch_ranges(ranges[0], &ranges[1]);
+  pdl_launch(split_matrix_kernel, dim3((unsigned)std::min<long>((pieces + 7) / 8, ctx().sm_count * 8l), 2), 256, 0, jobs[0], jobs[1]);
+  check_launch("split_matrix");
+  if (!x.along_k && y.along_k) gemm_pairs_t<true, false>(jobs[0].dst, jobs[0].ldp, jobs[1].dst, jobs[1].ldp, x.rows, y.rows, k, epi, rec[0], rec[1]);
+  else if (x.along_k && y.along_k) gemm_pairs_t<false, false>(jobs[0].dst, jobs[0].ldp, jobs[1].dst, jobs[1].ldp, x.rows, y.rows, k, epi, rec[0], rec[1]);
+  else if (!x.along_k) gemm_pairs_t<true, true>(jobs[0].dst, jobs[0].ldp, jobs[1].dst, jobs[1].ldp, x.rows, y.rows, k, epi, rec[0], rec[1]);
+  else gemm_pairs_t<false, true>(jobs[0].dst, jobs[0].ldp, jobs[1].dst, jobs[1].ldp, x.rows, y.rows, k, epi, rec[0], rec[1]);
+}
+// Whether pairs finish before TF32, the passes over the operands included.
+static bool pairs_are_faster(long m, long n, long k) {
+  const double passes = 8 + 4e-6 * (double)k * (double)(m + n) * (1 / 5.5 + 2 / 5.0);
+  return mm::tc2_product_us(m, n, k, mm::kPairs, true) + passes < mm::tc2_product_us(m, n, k, mm::kTf32);
 }
 // Whether the warp-level engine (mm_small.cuh) finishes before the two-SM one.  The latter, as measured for the same sizes: 11 us to
 // start, then the fill and fold of its long pipeline (0.026 per k up to 512) and 2.9 per GFLOP, or the operands' bytes
@@ -182,6 +225,7 @@ void gemm(char transa, char transb, long m, long n, long k, float alpha, const f
   const bool aligned = mm::raw_matrix_ok(a, lda) && mm::raw_matrix_ok(b, ldb);
   if (mode == 2 && m > 128 && n > 32) gemm_half(x, y, k, alpha, beta, c, ldc, row_bias);
   else if (small_is_faster(m, n, k, aligned)) gemm_small(x, y, k, alpha, beta, c, ldc, row_bias);
+  else if (mode == 0 && pairs_are_faster(m, n, k)) gemm_pairs(x, y, k, alpha, beta, c, ldc, row_bias);
   else gemm_raw(x, y, k, alpha, beta, c, ldc, row_bias);
 }
 

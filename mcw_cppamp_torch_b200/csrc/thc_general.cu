@@ -99,11 +99,11 @@ mm::StallCtl stall_ctl() {
   return mm::StallCtl{c.stall_dev, c.stall_host_dev, c.stall_limit};
 }
 
-unsigned *sched_counter() {
+unsigned *zeroed_words(int n) {
   Context &c = ctx();
   constexpr int kBlock = 4096;
   if (!c.sched_counters) {
-    THC_CUDA(cudaMalloc((void **)&c.sched_counters, sizeof(unsigned) * kBlock));
+    THC_CUDA(cudaMalloc((void **)&c.sched_counters, sizeof(unsigned) * 2 * kBlock));
     c.sched_next = kBlock;
   }
   if (c.sched_stream != c.stream) {
@@ -112,12 +112,17 @@ unsigned *sched_counter() {
     c.sched_stream = c.stream;
     c.sched_next = kBlock;
   }
-  if (c.sched_next == kBlock) {
-    THC_CUDA(cudaMemsetAsync(c.sched_counters, 0, sizeof(unsigned) * kBlock, c.stream));
+  if (n > 1) c.sched_next = (c.sched_next + 7) & ~7;
+  if (c.sched_next + n > kBlock) {
+    c.sched_block ^= 1;
+    THC_CUDA(cudaMemsetAsync(c.sched_counters + c.sched_block * kBlock, 0, sizeof(unsigned) * kBlock, c.stream));
     c.sched_next = 0;
   }
-  return c.sched_counters + c.sched_next++;
+  unsigned *p = c.sched_counters + c.sched_block * kBlock + c.sched_next;
+  c.sched_next += n;
+  return p;
 }
+unsigned *sched_counter() { return zeroed_words(1); }
 
 // Names of the wait codes of mm_tc.cuh (kWait*), for the error message.
 static const char *wait_name(int code) {

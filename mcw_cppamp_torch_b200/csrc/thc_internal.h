@@ -83,7 +83,7 @@ struct Context {
   long allocs = 0;               // stream-ordered allocations requested from the driver (storages + arena growth)
   // item counters of the persistent matrix-multiply launches (see sched_counter)
   unsigned *sched_counters = nullptr;
-  int sched_next = 0;
+  int sched_next = 0, sched_block = 0;
   cudaStream_t sched_stream = nullptr;
 };
 
@@ -107,10 +107,13 @@ __device__ __forceinline__ void scalar_deliver(ScalarSlot *slot, double v, unsig
 }
 #endif
 mm::StallCtl stall_ctl();         // kernel parameter of the tensor-core kernels
-// A zeroed device word for one persistent launch to hand out its work items from.  The words come from a block of
-// 4096 that is cleared on the stream each time it has been used up (the launches that used it are ahead of the
-// clearing in the same stream).
+// A zeroed device word for one persistent launch to hand out its work items from.  The words come from two blocks of
+// 4096; when one has been used up the other is cleared on the stream and takes over (the launches that used it are ahead of
+// the clearing in the same stream).
 unsigned *sched_counter();
+// The same for other uses inside one entry point, `n` words side by side on a 32-byte boundary; they keep their values until
+// some thousand further words have been handed out.
+unsigned *zeroed_words(int n);
 int device_if_initialised();       // -1 before the first CUDA use on this thread; never initialises
 void *scratch(size_t bytes);      // grow-only device scratch of the reductions, zero-filled when (re)allocated
 // Device words that are zero between launches: tickets of kernels that put them back to zero when they are done.  One
