@@ -8,9 +8,10 @@
 #include <cmath>
 #include <type_traits>
 
+#include "mm_planes.cuh"
 #include "mm_simt.cuh"
 #include "mm_small.cuh"
-#include "mm_tc2r.cuh"
+#include "mm_tc.cuh"
 #include "per_device.h"
 
 namespace thc {
@@ -188,13 +189,18 @@ static void attach_windows(Op &op, const void *base, const Windows &v, int per, 
 template <int PREC>
 static void attach_window_map(PlanesWindowOperand<PREC> &op, const void *base, const Windows &v) {
   set_window_pixels(op.rows, v);
-  op.ctiles = FastDiv::make(v.C / (PREC != kTf32 ? 64 : 32)); op.ctiles_wide = FastDiv::make(v.C / 32); op.kW = FastDiv::make(v.kW);
+  op.C = FastDiv::make(v.C); op.kW = FastDiv::make(v.kW);
   attach_windows<PREC>(op, base, v, TC_BM, false);
 }
 template <int PREC>
 static void attach_window_rows_map(WindowRowsOperand<PREC> &op, const void *base, const Windows &v) {
   set_window_pixels(op.ks, v);
   op.C = FastDiv::make(v.C); op.kW = FastDiv::make(v.kW);
+  op.oH = (int)v.oH;
+  for (int i = 0; i < 2; i++) {
+    const long n = 32l << i, P = v.oH * v.oW;
+    op.step[i] = WindowStep{(int)(n % P % v.oW), (int)(n % P / v.oW), (int)(n / P)};
+  }
   attach_windows<PREC>(op, base, v, 0, true);
 }
 
@@ -225,40 +231,10 @@ static double tc2_product_us(long M, long N, long K, int prec, bool mn = false) 
   return std::max(tiles * (ktiles + 2) / (ctx().sm_count / 2), std::min(ktiles, 6.0) + 2) * tc2_tile_us(w, prec) + 8;
 }
 
-// Clusters of the two-SM kernel that the device runs at once (the kernel is persistent: a launch has no more).
-template <class P, int BN2>
-static int tc2r_resident_clusters() {
-  constexpr int SMEM = tc2r_smem_bytes<BN2, P::PREC>();
-  static PerDevice resident;
-  return resident.get(ctx().device, [] {
-    THC_CUDA(cudaFuncSetAttribute(tc2r_kernel<P, BN2>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM));
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(2 * ctx().sm_count, 1, 1);
-    cfg.blockDim = dim3(T2_THREADS, 1, 1);
-    cfg.dynamicSmemBytes = SMEM;
-    int c = 0;
-    if (cudaOccupancyMaxActiveClusters(&c, tc2r_kernel<P, BN2>, &cfg) != cudaSuccess || c < 1) {
-      cudaGetLastError();
-      cudaLaunchAttribute attr;
-      attr.id = cudaLaunchAttributeClusterDimension;
-      attr.val.clusterDim.x = 2; attr.val.clusterDim.y = 1; attr.val.clusterDim.z = 1;
-      cfg.attrs = &attr; cfg.numAttrs = 1;
-      if (cudaOccupancyMaxActiveClusters(&c, tc2r_kernel<P, BN2>, &cfg) != cudaSuccess || c < 1) {
-        cudaGetLastError();
-        c = ctx().sm_count / 2;
-      }
-    }
-    return std::min(c, ctx().sm_count / 2);
-  });
-}
-template <class P, int BN2>
-static void launch_tc2r_kernel(const P &p, long items) {
-  const long clusters = std::min<long>(items, tc2r_resident_clusters<P, BN2>());
-  // a long launch gains nothing from starting early, and measured 1.5 % slower when it did (4096^3: 671 -> 682 us)
-  const bool early = tc2_product_us(p.M, p.N, p.K, P::PREC, P::OpB::MN_MAJOR) < 100;
-  launch_on_stream(early, tc2r_kernel<P, BN2>, dim3((unsigned)(2 * clusters), 1, 1), T2_THREADS, tc2r_smem_bytes<BN2, P::PREC>(), p, stall_ctl(), sched_counter());
-  check_launch("tc2r_kernel");
-}
+// The two-SM kernel (mm_tc2r.cuh) is compiled in files of its own, mm_tc2r_*.cu, which list the problems and tile widths there are.
+// Clusters that the device runs at once (the kernel is persistent: a launch has no more), and a launch of `items` work items.
+template <class P, int BN2> int tc2r_resident_clusters();
+template <class P, int BN2> void launch_tc2r_kernel(const P &p, long items, bool early);
 
 // Products over operands that TMA can fetch.  `attach(p, bn2)` writes the operands' tensor maps for the chosen tile width.
 template <class P, class Attach>
@@ -306,7 +282,9 @@ static void launch_raw(P p, Attach attach) {
   }
   const long items = p.tail_first + (tiles - p.tail_first) * p.tail_splits;
   THC_CHECK(items < (1l << 31) - 4096, "matrix product with too many tiles for one launch");
-  with_width([&](auto w) { launch_tc2r_kernel<P, decltype(w)::value>(p, items); });
+  // a long launch gains nothing from starting early, and measured 1.5 % slower when it did (4096^3: 671 -> 682 us)
+  const bool early = tc2_product_us(p.M, p.N, p.K, P::PREC, P::OpB::MN_MAJOR) < 100;
+  with_width([&](auto w) { launch_tc2r_kernel<P, decltype(w)::value>(p, items, early); });
   if (p.ws) {
     // a few thousand blocks whatever the number of tail tiles: a lone tile cut into many slices gets a block per column
     const long by = std::min<long>(bn2, std::max<long>(32, ceil_div(8l * ctx().sm_count, tail)));

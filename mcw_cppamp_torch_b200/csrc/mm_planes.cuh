@@ -1,0 +1,637 @@
+// Passes over operands and results of the matrix-multiply engines: ranges and FP16 pairs, channels-last planes and cells, repacked
+// weights, folds of partial sums.
+#ifndef THC_MM_PLANES_CUH
+#define THC_MM_PLANES_CUH
+
+#include "mm_problem.cuh"
+
+namespace thc {
+namespace mm {
+
+__device__ __forceinline__ void split_pair(float a, float b, __half2 &hi, __half2 &lo) {
+  hi = __floats2half2_rn(a, b);
+  const float2 h = __half22float2(hi);
+  lo = __floats2half2_rn((a - h.x) * 2048.f, (b - h.y) * 2048.f);
+}
+__device__ __forceinline__ unsigned half2_bits(const __half2 &h) { return *reinterpret_cast<const unsigned *>(&h); }
+
+// Ranges of up to two operands (blockIdx.y), `lines` x `run` values with pitch ld.  A warp looks at 512 values at a time, in four
+// groups of 128: neighbours in memory (`flat`), or 128 neighbours in each of four lines, so that a small row or column shows in
+// several groups.
+struct RangeJob { const float *p; long lines, run, ld; int flat, vec; RangeRec *rec; };
+static __global__ void __launch_bounds__(256) range_kernel(const RangeJob ja, const RangeJob jb) {
+  pdl_begin();
+  const RangeJob &j = blockIdx.y ? jb : ja;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const long warps = (long)gridDim.x * 8, total = j.lines * j.run;
+  const long segs = j.flat ? (total + 511) / 512 : (j.run + 127) / 128, sets = j.flat ? segs : segs * ((j.lines + 3) / 4);
+  unsigned most = 0, low = ~0u, low2 = ~0u;   // the lows as bits - 1: zero becomes the largest
+  for (long s = (long)blockIdx.x * 8 + warp; s < sets; s += warps) {
+    unsigned v[4][4];
+    const long q = j.flat ? 0 : s / segs, c0 = j.flat ? s * 512 : (s - q * segs) * 128;
+#pragma unroll
+    for (int g = 0; g < 4; g++) {
+      const long line = j.flat ? 0 : q * 4 + g, c = c0 + (j.flat ? g * 128 : 0) + lane * 4, end = j.flat ? total : line < j.lines ? j.run : 0;
+      const float *src = j.p + line * j.ld + c;
+      if (j.vec && c + 4 <= end) {
+        const uint4 u = __ldg(reinterpret_cast<const uint4 *>(src));
+        v[g][0] = u.x; v[g][1] = u.y; v[g][2] = u.z; v[g][3] = u.w;
+      } else {
+#pragma unroll
+        for (int i = 0; i < 4; i++) v[g][i] = c + i < end ? __float_as_uint(__ldg(src + i)) : 0u;
+      }
+    }
+    unsigned a = ~0u, b = ~0u;   // the two smallest groups of this lane
+#pragma unroll
+    for (int g = 0; g < 4; g++) {
+      unsigned m = ~0u;
+#pragma unroll
+      for (int i = 0; i < 4; i++) {
+        const unsigned x = v[g][i] & 0x7fffffffu;
+        most = max(most, x);
+        m = min(m, x - 1u);
+      }
+      b = min(b, max(a, m));
+      a = min(a, m);
+    }
+    const unsigned first = __reduce_min_sync(0xffffffffu, a);
+    const int owner = __ffs(__ballot_sync(0xffffffffu, a == first)) - 1;
+    low = min(low, first);
+    low2 = min(low2, __reduce_min_sync(0xffffffffu, lane == owner ? b : a));
+  }
+  __shared__ unsigned sm[3][8];
+  most = __reduce_max_sync(0xffffffffu, most);
+  if (lane == 0) { sm[0][warp] = most; sm[1][warp] = low; sm[2][warp] = low2; }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int w = 1; w < 8; w++) { most = max(most, sm[0][w]); low = min(low, sm[1][w]); low2 = min(low2, sm[2][w]); }
+    if (most) atomicMax(&j.rec->max_bits, most);
+    if (~low) atomicMax(&j.rec->low_inv, ~low);
+    if (~low2) atomicMax(&j.rec->low2_inv, ~low2);
+  }
+}
+
+// What a kernel that writes an operand's planes needs in kPairs.
+struct PairForm {
+  Ranges ranges;
+  RangeRec *keep = nullptr;     // where the planes' record goes when they outlive the call (their ranges[0] does not)
+  RangeRec *remake = nullptr;   // ranges[0] of kept planes: write only if they are pairs and must be FP32 now
+  // Whether to write anything, and in which form; every thread of the block calls it.
+  __device__ __forceinline__ bool begin(bool &wide) const {
+    wide = ranges.wide();
+    return !remake || (wide && !*const_cast<const volatile unsigned *>(&remake->wide));
+  }
+  // After the block's last look at the records: the last block to get here changes what `begin` looked at.
+  __device__ __forceinline__ void end(bool wide) const {
+    if (keep && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) {
+      RangeRec r = *ranges.rec[0];
+      r.wide = wide; r.ticket = 0;
+      *keep = r;
+    }
+    if (remake) {
+      __syncthreads();
+      if (threadIdx.x == 0 && atomicAdd(&remake->ticket, 1u) == gridDim.x * gridDim.y - 1) { remake->ticket = 0; remake->wide = 1; }
+    }
+  }
+};
+
+// ---------------------------------------------------------------------------------------------
+// Channels-last planes of an activation tensor, FP32 or BF16, channels padded with zeros to Cp = a multiple of KV.
+//
+// NCHW fp32 -> [img][pixel][Cp].  CT channels x PT pixels per pass through shared memory, sixteen loads per thread in flight
+// before the barrier (32 x 32 tiles with four left the kernel at half the HBM rate): reads coalesced along pixels, writes in
+// whole 128-byte lines along channels.
+// `chan_partial` (optional): [gridDim.x][C] sums over the pixels this block transposed, per channel -- the gradBias
+// reduction of a convolution rides on the transposition of gradOutput instead of reading the tensor a second time.
+// A channel of a tile belongs to one warp, tiles are taken in a fixed order, so the sums are reproducible.
+template <bool HALF>
+static __global__ void __launch_bounds__(256) nchw_to_planes_kernel(const float *__restrict__ src, long N, int C, int HW, int Cp,
+                                                                    void *__restrict__ dst, float *__restrict__ chan_partial) {
+  pdl_begin();
+  constexpr int CT = HALF ? 64 : 32, PT = HALF ? 64 : 128;
+  __shared__ float tile[CT][PT + 1];
+  extern __shared__ float chan_sum[];   // [C] when chan_partial is given
+  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+  const unsigned ptiles = (unsigned)((HW + PT - 1) / PT), ctiles = (unsigned)(Cp / CT);
+  const long ntiles = N * ptiles * ctiles;
+  if (chan_partial) {
+    for (int c = threadIdx.x; c < C; c += blockDim.x) chan_sum[c] = 0.f;
+    __syncthreads();
+  }
+  for (long t = blockIdx.x; t < ntiles; t += gridDim.x) {
+    const unsigned r = (unsigned)(t % (ptiles * ctiles));
+    const long img = t / (ptiles * ctiles);
+    const int ct = (int)(r / ptiles), p0 = (int)(r - ct * ptiles) * PT, c0 = ct * CT;
+    const int np = min(HW - p0, PT), nc = min(C - c0, CT);
+    const float *s = src + (img * C + c0) * HW + p0 + tx;
+    float v[CT / 8][PT / 32];
+#pragma unroll
+    for (int j = 0; j < CT / 8; j++)
+#pragma unroll
+      for (int g = 0; g < PT / 32; g++)
+        v[j][g] = (g * 32 + tx < np && ty + 8 * j < nc) ? s[(long)(ty + 8 * j) * HW + g * 32] : 0.f;
+#pragma unroll
+    for (int j = 0; j < CT / 8; j++) {
+      float part = 0.f;
+#pragma unroll
+      for (int g = 0; g < PT / 32; g++) {
+        tile[ty + 8 * j][g * 32 + tx] = v[j][g];
+        part += v[j][g];
+      }
+      if (chan_partial) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
+        if (tx == 0 && ty + 8 * j < nc) chan_sum[c0 + ty + 8 * j] += part;
+      }
+    }
+    __syncthreads();
+    const long o0 = (img * HW + p0) * Cp + c0;
+#pragma unroll 8
+    for (int j = ty; j < np; j += 8) {
+      if constexpr (HALF)
+        reinterpret_cast<__nv_bfloat162 *>(dst)[(o0 + (long)j * Cp) / 2 + tx] = __floats2bfloat162_rn(tile[2 * tx][j], tile[2 * tx + 1][j]);
+      else
+        reinterpret_cast<float *>(dst)[o0 + (long)j * Cp + tx] = tile[tx][j];
+    }
+    __syncthreads();
+  }
+  if (chan_partial)
+    for (int c = threadIdx.x; c < C; c += blockDim.x) chan_partial[(long)blockIdx.x * C + c] = chan_sum[c];
+}
+// The same as FP16 pairs, [img][pixel][hi: Cp][lo: Cp], or FP32 values in the same place.
+static __global__ void __launch_bounds__(256) nchw_to_pairs_kernel(const float *__restrict__ src, long N, int C, int HW, int Cp,
+                                                                   void *__restrict__ dst, float *__restrict__ chan_partial,
+                                                                   const PairForm form) {
+  pdl_begin();
+  bool wide;
+  if (!form.begin(wide)) return;
+  const float scale = wide ? 1.f : pair_scale(*form.ranges.rec[0]);
+  constexpr int CT = 64, PT = 64;
+  __shared__ float tile[CT][PT + 1];
+  extern __shared__ float chan_sum[];   // [C] when chan_partial is given
+  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+  const unsigned ptiles = (unsigned)((HW + PT - 1) / PT), ctiles = (unsigned)(Cp / CT);
+  const long ntiles = N * ptiles * ctiles;
+  if (chan_partial) {
+    for (int c = threadIdx.x; c < C; c += blockDim.x) chan_sum[c] = 0.f;
+    __syncthreads();
+  }
+  for (long t = blockIdx.x; t < ntiles; t += gridDim.x) {
+    const unsigned r = (unsigned)(t % (ptiles * ctiles));
+    const long img = t / (ptiles * ctiles);
+    const int ct = (int)(r / ptiles), p0 = (int)(r - ct * ptiles) * PT, c0 = ct * CT;
+    const int np = min(HW - p0, PT), nc = min(C - c0, CT);
+    const float *s = src + (img * C + c0) * HW + p0 + tx;
+    float v[CT / 8][PT / 32];
+#pragma unroll
+    for (int j = 0; j < CT / 8; j++)
+#pragma unroll
+      for (int g = 0; g < PT / 32; g++)
+        v[j][g] = (g * 32 + tx < np && ty + 8 * j < nc) ? s[(long)(ty + 8 * j) * HW + g * 32] : 0.f;
+#pragma unroll
+    for (int j = 0; j < CT / 8; j++) {
+      float part = 0.f;
+#pragma unroll
+      for (int g = 0; g < PT / 32; g++) {
+        tile[ty + 8 * j][g * 32 + tx] = v[j][g];
+        part += v[j][g];
+      }
+      if (chan_partial) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
+        if (tx == 0 && ty + 8 * j < nc) chan_sum[c0 + ty + 8 * j] += part;
+      }
+    }
+    __syncthreads();
+    const long o0 = (img * HW + p0) * Cp;
+#pragma unroll 8
+    for (int j = ty; j < np; j += 8) {
+      const float a = tile[2 * tx][j] * scale, b = tile[2 * tx + 1][j] * scale;
+      float *px = reinterpret_cast<float *>(dst) + o0 + (long)j * Cp;
+      if (wide) {
+        reinterpret_cast<float2 *>(px + c0)[tx] = make_float2(a, b);
+      } else {
+        __half2 hi, lo;
+        split_pair(a, b, hi, lo);
+        __half2 *h = reinterpret_cast<__half2 *>(px) + c0 / 2 + tx;
+        h[0] = hi;
+        h[Cp / 2] = lo;
+      }
+    }
+    __syncthreads();
+  }
+  if (chan_partial)
+    for (int c = threadIdx.x; c < C; c += blockDim.x) chan_partial[(long)blockIdx.x * C + c] = chan_sum[c];
+  form.end(wide);
+}
+// out[c] += scale * sum_b partial[b][c]: 32 row slices per channel (one warp each, eight loads in flight per
+// thread), folded in a fixed order.  The partials are a few MB at most; what this kernel costs is the chain of
+// dependent loads per thread, hence the wide block.
+static __global__ void __launch_bounds__(1024) chan_partial_finish_kernel(const float *__restrict__ partial, int nblocks, long C,
+                                                                          float *out, float scale) {
+  pdl_begin();
+  __shared__ float sm[32][33];
+  const int lane = threadIdx.x & 31, s = threadIdx.x >> 5;
+  const long c = (long)blockIdx.x * 32 + lane;
+  float a[8];
+#pragma unroll
+  for (int i = 0; i < 8; i++) a[i] = 0.f;
+  if (c < C) {
+    int b = s;
+    for (; b + 7 * 32 < nblocks; b += 8 * 32) {
+      float v[8];
+#pragma unroll
+      for (int i = 0; i < 8; i++) v[i] = partial[(long)(b + 32 * i) * C + c];
+#pragma unroll
+      for (int i = 0; i < 8; i++) a[i] += v[i];
+    }
+    for (; b < nblocks; b += 32) a[0] += partial[(long)b * C + c];
+  }
+  const float a0 = a[0] + a[4], a1 = a[1] + a[5], a2 = a[2] + a[6], a3 = a[3] + a[7];
+  sm[s][lane] = (a0 + a1) + (a2 + a3);
+  __syncthreads();
+  if (s == 0 && c < C) {
+    float acc = 0.f;
+    for (int k = 0; k < 32; k++) acc += sm[k][lane];
+    out[c] += scale * acc;
+  }
+}
+
+
+// A convolution layer restated over "cells": pixel (Y, X) of the restated input carries, as channels, the eH x eW input
+// pixels at offsets (dy, dx) from (Y * dH - pad, X * dW - pad), all planes of each:
+//   S[n][Y][X][ch = (dy * eW + dx) * Cq + c] = in[n][c][Y * dH + dy - pad][X * dW + dx - pad]
+// and filter tap (i, j) is tap ((i - dy) / stepH, (j - dx) / stepW) at the channels of (dy, dx).  Per axis either
+//   fold    e = min(d, k): the pixels of a stride cell become channels, ceil(k / d) taps remain, or
+//   unfold  e = k: one tap remains (along both axes: the column matrix).
+// `direct`: the input's own planes (e = 1, all taps, stride and padding left to the TMA window map).
+// Which one costs least depends on how far the channel count is from a multiple of KV: see restate() in gpunn_conv.cu.
+struct Cells {
+  int C, kH, kW, dH, dW, pad;      // the layer
+  int H, W;
+  int eH, eW, kHs, kWs, stepH, stepW;
+  int Cq;                          // channels per offset: C, or padded where that costs no further span
+  int Cr, Cs;                      // eH * eW * Cq, and that padded to a multiple of KV
+  int Hs, Ws;                      // grid of S
+  bool direct;
+  // place of channel `ch`; false: padding
+  __host__ __device__ __forceinline__ bool channel(int ch, int &c, int &dy, int &dx) const {
+    const int q = ch / Cq;
+    c = ch - q * Cq;
+    dy = q / eW;
+    dx = q - dy * eW;
+    return ch < Cr && c < C;
+  }
+};
+
+// S of one image row per block.  A thread produces 16 bytes of a pixel: 4 FP32 or 8 BF16 channels, whose source offsets it
+// looks up in a table; neighbouring threads hold neighbouring channels, i.e. neighbouring columns of a few input rows.  More
+// channels than the table holds (kCellTable: 48 KB of it) are found by division, once per 16 bytes.
+constexpr int kCellTable = 6144;
+// kPairs: [pixel][hi: Cs][lo: Cs], 8 channels a thread.
+template <int PREC, bool TABLE>
+__device__ __forceinline__ void cells_row(const float *__restrict__ in, void *__restrict__ S, long row, const Cells &u, const int2 *chan_src, bool wide,
+                                          float scale) {
+  constexpr int V = PREC != kTf32 ? 8 : 4;
+  const long n = row / u.Hs;
+  const int Y = (int)(row - n * u.Hs);
+  const int q = u.Cs / V, chunks = u.Ws * q, y0 = Y * u.dH - u.pad;
+  const float *img = in + n * u.C * (long)u.H * u.W;
+  uint4 *dst = reinterpret_cast<uint4 *>(S) + ((n * u.Hs + Y) * u.Ws) * (long)q * (PREC == kPairs ? 2 : 1);
+  for (int o = blockIdx.y * blockDim.x + threadIdx.x; o < chunks; o += gridDim.y * blockDim.x) {
+    const int X = o / q, ch0 = (o - X * q) * V, x0 = X * u.dW - u.pad;
+    float v[V];
+    if constexpr (TABLE) {
+      const float *base = img + (long)y0 * u.W + x0;
+#pragma unroll
+      for (int e = 0; e < V; e++) {
+        const int2 s = chan_src[ch0 + e];
+        const int y = y0 + (s.y >> 16), x = x0 + (s.y & 0xffff);
+        v[e] = s.y >= 0 && (unsigned)y < (unsigned)u.H && (unsigned)x < (unsigned)u.W ? __ldg(base + s.x) : 0.f;
+      }
+    } else {
+      int c, dy, dx;
+      u.channel(ch0, c, dy, dx);
+#pragma unroll
+      for (int e = 0; e < V; e++) {
+        const int y = y0 + dy, x = x0 + dx;
+        v[e] = ch0 + e < u.Cr && c < u.C && (unsigned)y < (unsigned)u.H && (unsigned)x < (unsigned)u.W
+                   ? __ldg(img + ((long)c * u.H + y) * u.W + x) : 0.f;
+        if (++c == u.Cq) {
+          c = 0;
+          if (++dx == u.eW) { dx = 0; dy++; }
+        }
+      }
+    }
+    if constexpr (PREC == kBf16) {
+      __nv_bfloat162 h[4];
+#pragma unroll
+      for (int e = 0; e < 4; e++) h[e] = __floats2bfloat162_rn(v[2 * e], v[2 * e + 1]);
+      dst[o] = *reinterpret_cast<const uint4 *>(h);
+    } else if constexpr (PREC == kPairs) {
+      if (wide) {
+        float4 *d = reinterpret_cast<float4 *>(dst) + 2 * (long)o;
+        d[0] = make_float4(v[0], v[1], v[2], v[3]);
+        d[1] = make_float4(v[4], v[5], v[6], v[7]);
+      } else {
+        __half2 hi[4], lo[4];
+#pragma unroll
+        for (int e = 0; e < 4; e++) split_pair(v[2 * e] * scale, v[2 * e + 1] * scale, hi[e], lo[e]);
+        uint4 *d = dst + X * 2l * q + ch0 / V;
+        d[0] = *reinterpret_cast<const uint4 *>(hi);
+        d[q] = *reinterpret_cast<const uint4 *>(lo);
+      }
+    } else {
+      dst[o] = make_uint4(__float_as_uint(v[0]), __float_as_uint(v[1]), __float_as_uint(v[2]), __float_as_uint(v[3]));
+    }
+  }
+}
+template <int PREC, bool TABLE>
+static __global__ void __launch_bounds__(256) cells_input_kernel(const float *__restrict__ in, void *__restrict__ S, long N, const Cells u,
+                                                                 const PairForm form) {
+  pdl_begin();
+  bool wide = false;
+  float scale = 1.f;
+  if constexpr (PREC == kPairs) {
+    if (!form.begin(wide)) return;
+    if (!wide) scale = pair_scale(*form.ranges.rec[0]);
+  }
+  extern __shared__ int2 chan_src[];      // per channel: offset in the image, (dy << 16 | dx) or -1
+  if constexpr (TABLE) {
+    for (int ch = threadIdx.x; ch < u.Cs; ch += blockDim.x) {
+      int c, dy, dx;
+      chan_src[ch] = u.channel(ch, c, dy, dx) ? make_int2((c * u.H + dy) * u.W + dx, dy << 16 | dx) : make_int2(0, -1);
+    }
+    __syncthreads();
+  }
+  if constexpr (PREC == kPairs) {
+    for (long row = blockIdx.x; row < N * u.Hs; row += gridDim.x) cells_row<PREC, TABLE>(in, S, row, u, chan_src, wide, scale);
+    form.end(wide);
+  } else {
+    cells_row<PREC, TABLE>(in, S, blockIdx.x, u, chan_src, wide, scale);   // (a loop over rows costs 98 -> 117 us at 256 images)
+  }
+}
+
+// The column matrix in BF16 with eight channels per tap (Cq = 8, C <= 8): 16 bytes of S are one tap of one pixel.  A block makes
+// the rows of one output row: the kH input rows it needs go to shared memory once, as 16-byte pixels, and leave from there
+// kH * kW times over, so that the kernel is bound by the writes (gathering each value from the image took four times as
+// long: 1105 -> 280 us for 256 images under the 11 x 11 / 4 filter, 1.6 GB).
+static __global__ void __launch_bounds__(256) columns8_kernel(const float *__restrict__ in, uint4 *__restrict__ S, const Cells u) {
+  pdl_begin();
+  extern __shared__ uint4 px_rows[];   // [kH][W + 2 pad]
+  const long n = blockIdx.x / u.Hs;
+  const int Y = (int)(blockIdx.x - n * u.Hs), Wp = u.W + 2 * u.pad, taps = u.kH * u.kW, q = u.Cs / 8;
+  const float *img = in + n * u.C * (long)u.H * u.W;
+  for (int t = threadIdx.x; t < u.kH * Wp; t += blockDim.x) {
+    const int i = t / Wp, y = Y * u.dH + i - u.pad, x = t - i * Wp - u.pad;
+    float v[8];
+#pragma unroll
+    for (int c = 0; c < 8; c++)
+      v[c] = c < u.C && (unsigned)y < (unsigned)u.H && (unsigned)x < (unsigned)u.W ? __ldg(img + ((long)c * u.H + y) * u.W + x) : 0.f;
+    __nv_bfloat162 h[4];
+#pragma unroll
+    for (int e = 0; e < 4; e++) h[e] = __floats2bfloat162_rn(v[2 * e], v[2 * e + 1]);
+    px_rows[t] = *reinterpret_cast<const uint4 *>(h);
+  }
+  __syncthreads();
+  uint4 *dst = S + (n * u.Hs + Y) * u.Ws * (long)q;
+  const int chunks = u.Ws * q, step_x = (int)blockDim.x / q, step_t = (int)blockDim.x - step_x * q;
+  int X = (int)threadIdx.x / q, tap = (int)threadIdx.x - X * q;
+  for (int o = threadIdx.x; o < chunks; o += blockDim.x) {
+    const int i = tap / u.kW, j = tap - i * u.kW;
+    dst[o] = tap < taps ? px_rows[i * Wp + X * u.dW + j] : make_uint4(0, 0, 0, 0);
+    X += step_x; tap += step_t;
+    if (tap >= q) { tap -= q; X++; }
+  }
+}
+
+// Weights of the restated layer in the k order of the window operand, four values per thread:
+//   FLIP false: out[ko][(bi, bj, ch)]           (forward)
+//   FLIP true : out[ch][(bi', bj', ko)], bi' = kHs - 1 - bi: gradInput as a forward pass over gradOutput (channels padded to
+//               `chans`) under the filter rotated by 180 degrees
+// pair_shift > 0 (pixel-pair mode, see Epilogue): the filter is widened to kWs + pair_shift columns and
+// stored twice, rows [0, rows) as it is (output parity 0) and rows [rows, 2 rows) shifted right by pair_shift
+// columns (parity 1, whose window starts one stride later); the new columns are zero.
+// kPairs: a row is [hi: its values][lo: its values].
+template <int PREC, bool FLIP>
+static __global__ void __launch_bounds__(256) repack_weight_kernel(const float *__restrict__ w, const Cells u, int K, int rows, int chans,
+                                                                   int pair_shift, void *__restrict__ out, const Ranges ranges) {
+  pdl_begin();
+  bool wide = false;
+  float scale = 1.f;
+  if constexpr (PREC == kPairs) {
+    wide = ranges.wide();
+    if (!wide) scale = pair_scale(*ranges.rec[0]);
+  }
+  const int kWe = u.kWs + pair_shift, quads = u.kHs * kWe * (chans / 4);
+  const unsigned total = (unsigned)((pair_shift ? 2 : 1) * rows) * (unsigned)quads;
+  for (unsigned t = blockIdx.x * blockDim.x + threadIdx.x; t < total; t += gridDim.x * blockDim.x) {
+    int r = (int)(t / (unsigned)quads);
+    const long row = r;
+    const int k = (int)(t - (unsigned)r * quads) * 4, tap = k / chans, k0 = k - tap * chans;
+    const int par = r >= rows ? 1 : 0;
+    r -= par * rows;
+    int bi = tap / kWe, bj = tap - bi * kWe - par * pair_shift;
+    if (FLIP) { bi = u.kHs - 1 - bi; bj = u.kWs - 1 - bj; }
+    float v[4];
+#pragma unroll
+    for (int e = 0; e < 4; e++) {
+      const int ch = FLIP ? r : k0 + e, ko = FLIP ? k0 + e : r;
+      int c, dy, dx;
+      const bool real = u.channel(ch, c, dy, dx);
+      const int i = dy + bi * u.stepH, j = dx + bj * u.stepW;
+      v[e] = real && ko < K && bj >= 0 && bj < u.kWs && i < u.kH && j < u.kW ? w[(((long)ko * u.C + c) * u.kH + i) * u.kW + j] : 0.f;
+    }
+    if (PREC == kPairs && !wide) {
+      __half2 hi[2], lo[2];
+      split_pair(v[0] * scale, v[1] * scale, hi[0], lo[0]);
+      split_pair(v[2] * scale, v[3] * scale, hi[1], lo[1]);
+      uint2 *o = reinterpret_cast<uint2 *>(out) + row * 2 * quads + k / 4;
+      o[0] = make_uint2(half2_bits(hi[0]), half2_bits(hi[1]));
+      o[quads] = make_uint2(half2_bits(lo[0]), half2_bits(lo[1]));
+    } else if constexpr (PREC == kBf16) {
+      const __nv_bfloat162 a = __floats2bfloat162_rn(v[0], v[1]), b = __floats2bfloat162_rn(v[2], v[3]);
+      reinterpret_cast<uint2 *>(out)[t] = make_uint2(*reinterpret_cast<const unsigned *>(&a), *reinterpret_cast<const unsigned *>(&b));
+    } else {
+      reinterpret_cast<float4 *>(out)[t] = make_float4(v[0], v[1], v[2], v[3]);
+    }
+  }
+}
+
+// gw[ko][(c, i, j)] += scale * T at the restated tap and channel of (c, i, j).  ko_stride, ch_stride, bi_stride, bj_stride: where T
+// keeps them (bj counted from the other end when bj_stride is negative: `first` is then the place of tap (0, 0)).
+// `copies` partial sums of each, copy_stride apart.
+struct WgradPlace { long ko_stride, ch_stride, bi_stride, bj_stride, first; int copies; long copy_stride; };
+static __global__ void __launch_bounds__(256) unpack_grad_weight_kernel(const float *__restrict__ T, float *__restrict__ gw, const Cells u,
+                                                                        int K, const WgradPlace p, float scale) {
+  pdl_begin();
+  const unsigned kHW = (unsigned)(u.kH * u.kW), per = (unsigned)u.C * kHW, total = (unsigned)K * per;
+  for (unsigned t = blockIdx.x * blockDim.x + threadIdx.x; t < total; t += gridDim.x * blockDim.x) {
+    const unsigned ko = t / per, r = t - ko * per, c = r / kHW, tap = r - c * kHW, i = tap / (unsigned)u.kW, j = tap - i * u.kW;
+    const int bi = u.kHs > 1 ? (int)i / u.stepH : 0, bj = u.kWs > 1 ? (int)j / u.stepW : 0;
+    const int dy = (int)i - bi * u.stepH, dx = (int)j - bj * u.stepW;
+    const long ch = (dy * u.eW + dx) * u.Cq + (int)c;
+    const float *s = T + (p.first + ko * p.ko_stride + ch * p.ch_stride + bi * p.bi_stride + bj * p.bj_stride);
+    float sum = *s;
+    for (int q = 1; q < p.copies; q++) sum += s[q * p.copy_stride];
+    gw[t] += scale * sum;
+  }
+}
+
+// gin[n][c][h][w] = gS[n][ch][Y][X], the inverse of a fold along both axes (a bijection between the input pixels that any
+// window reaches and the cells' channels; the others get zero).  gS: [N][Cr][Hs][Ws].
+static __global__ void __launch_bounds__(256) unfold_grad_input_kernel(const float *__restrict__ gS, float *__restrict__ gin, long N,
+                                                                       const Cells u) {
+  pdl_begin();
+  const unsigned HW = (unsigned)(u.H * u.W);
+  const long planes = N * u.C;
+  for (long pl = blockIdx.y; pl < planes; pl += gridDim.y) {
+    const long n = pl / u.C;
+    const int c = (int)(pl - n * u.C);
+    const float *src = gS + n * u.Cr * (long)(u.Hs * u.Ws);
+    for (unsigned t = blockIdx.x * blockDim.x + threadIdx.x; t < HW; t += gridDim.x * blockDim.x) {
+      const int h = (int)(t / (unsigned)u.W) + u.pad, w = (int)(t % (unsigned)u.W) + u.pad;
+      const int Y = h / u.dH, dy = h - Y * u.dH, X = w / u.dW, dx = w - X * u.dW;
+      float v = 0.f;
+      if (Y < u.Hs && X < u.Ws && dy < u.eH && dx < u.eW) v = src[((long)((dy * u.eW + dx) * u.Cq + c) * u.Hs + Y) * u.Ws + X];
+      gin[pl * HW + t] = v;
+    }
+  }
+}
+
+// Up to two matrices (blockIdx.y) as FP16 pairs: lines of `run` values become [hi: ldp][lo: ldp], ldp = run padded with zeros to whole
+// spans, or lines of ldp FP32 values.  A warp takes 512 values of a line, all loads in flight before the first store.
+struct PairJob { const float *src; void *dst; long lines, run, ld, ldp; int vec; Ranges ranges; };
+static __global__ void __launch_bounds__(256) split_matrix_kernel(const PairJob a, const PairJob b) {
+  pdl_begin();
+  const PairJob &j = blockIdx.y ? b : a;
+  const bool wide = j.ranges.wide();
+  const float scale = wide ? 1.f : pair_scale(*j.ranges.rec[0]);
+  const int lane = threadIdx.x & 31;
+  const long warps = (long)gridDim.x * 8, parts = (j.ldp + 511) / 512;
+  for (long w = (long)blockIdx.x * 8 + (threadIdx.x >> 5); w < j.lines * parts; w += warps) {
+    const long l = w / parts, c0 = (w - l * parts) * 512 + lane * 4;
+    const float *s = j.src + l * j.ld;
+    float4 v[4];
+#pragma unroll
+    for (int g = 0; g < 4; g++) {
+      const long c = c0 + g * 128;
+      if (j.vec && c + 4 <= j.run) v[g] = __ldg(reinterpret_cast<const float4 *>(s + c));
+      else v[g] = make_float4(c < j.run ? s[c] : 0.f, c + 1 < j.run ? s[c + 1] : 0.f, c + 2 < j.run ? s[c + 2] : 0.f, c + 3 < j.run ? s[c + 3] : 0.f);
+    }
+    float *d = reinterpret_cast<float *>(j.dst) + l * j.ldp;
+#pragma unroll
+    for (int g = 0; g < 4; g++) {
+      const long c = c0 + g * 128;
+      if (c >= j.ldp) break;
+      if (wide) {
+        *reinterpret_cast<float4 *>(d + c) = v[g];
+      } else {
+        __half2 hi[2], lo[2];
+        split_pair(v[g].x * scale, v[g].y * scale, hi[0], lo[0]);
+        split_pair(v[g].z * scale, v[g].w * scale, hi[1], lo[1]);
+        uint2 *h = reinterpret_cast<uint2 *>(reinterpret_cast<__half *>(d) + c);
+        h[0] = make_uint2(half2_bits(hi[0]), half2_bits(hi[1]));
+        h[j.ldp / 4] = make_uint2(half2_bits(lo[0]), half2_bits(lo[1]));
+      }
+    }
+  }
+}
+
+// BF16 plane of a strided matrix: element (r, k) at src[r*rs + k*ks]; out [rows][ld], zero for k >= K (ld a multiple of 64).
+// 64 x 64 tiles: along k as they lie, else through shared memory.
+static __global__ void __launch_bounds__(256) bf16_rows_kernel(const float *__restrict__ src, long rs, long ks, long rows, long K,
+                                                               __nv_bfloat16 *__restrict__ out, long ld) {
+  pdl_begin();
+  __shared__ float tile[64][65];
+  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+  const long tiles_k = ld / 64;
+  const long ntiles = ((rows + 63) / 64) * tiles_k;
+  for (long t = blockIdx.x; t < ntiles; t += gridDim.x) {
+    const long r0 = (t / tiles_k) * 64, k0 = (t % tiles_k) * 64;
+    if (rs == 1 && ks != 1) {   // memory runs along the rows: warp = k, lanes = rows
+      float v[8][2];
+#pragma unroll
+      for (int j = 0; j < 8; j++)
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+          const long r = r0 + tx + 32 * h, k = k0 + ty + 8 * j;
+          v[j][h] = (r < rows && k < K) ? src[r + k * ks] : 0.f;
+        }
+#pragma unroll
+      for (int j = 0; j < 8; j++)
+#pragma unroll
+        for (int h = 0; h < 2; h++) tile[tx + 32 * h][ty + 8 * j] = v[j][h];
+      __syncthreads();
+#pragma unroll
+      for (int j = 0; j < 8; j++) {
+        const long r = r0 + ty + 8 * j;
+        if (r < rows)
+          *reinterpret_cast<__nv_bfloat162 *>(out + r * ld + k0 + 2 * tx) = __floats2bfloat162_rn(tile[ty + 8 * j][2 * tx], tile[ty + 8 * j][2 * tx + 1]);
+      }
+      __syncthreads();
+    } else {
+      float v[8][2];
+#pragma unroll
+      for (int j = 0; j < 8; j++)
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+          const long r = r0 + ty + 8 * j, k = k0 + 2 * tx + h;
+          v[j][h] = (r < rows && k < K) ? src[r * rs + k * ks] : 0.f;
+        }
+#pragma unroll
+      for (int j = 0; j < 8; j++) {
+        const long r = r0 + ty + 8 * j;
+        if (r < rows) *reinterpret_cast<__nv_bfloat162 *>(out + r * ld + k0 + 2 * tx) = __floats2bfloat162_rn(v[j][0], v[j][1]);
+      }
+    }
+  }
+}
+
+// Folds split-K partials (fixed order -> deterministic) and applies the epilogue.  grid.y walks n, threads walk
+// m, which is contiguous in the workspace.
+static __global__ void __launch_bounds__(256) splitk_finish_kernel(const float *__restrict__ ws, int splits, long M, long N,
+                                                            Epilogue epi) {
+  pdl_begin();
+  const long m = (long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (m >= M) return;
+  const bool pair = epi.pair_K != 0;
+  const long mo = pair ? epi.moff<true>(m) : epi.moff<false>(m);
+  const float row_b = epi.rb(m);
+  for (long n = blockIdx.y; n < N; n += gridDim.y) {
+    float acc = 0.f;
+    for (int z = 0; z < splits; z++) acc += ws[((long)z * N + n) * M + m];
+    if (pair) epi.store<true>(mo, n, acc);
+    else epi.store<false>(mo, n, acc, row_b);
+  }
+}
+
+// The same for the tile-local partials of the raw-operand engine (Problem::tail_first): block (t, y) folds columns
+// y, y + gridDim.y, ... of tail tile t; a thread owns one of the tile's 256 rows, which are contiguous in the
+// workspace.
+static __global__ void __launch_bounds__(256) tail_finish_kernel(const float *__restrict__ ws, int splits, int bn2, long tail_first,
+                                                          long gm, long M, long N, Epilogue epi) {
+  pdl_begin();
+  const long tile = tail_first + blockIdx.x;
+  const long nt = tile / gm, mt = tile - nt * gm;
+  const long m = mt * 256 + threadIdx.x;
+  if (m >= M) return;
+  const bool pair = epi.pair_K != 0;
+  const long mo = pair ? epi.moff<true>(m) : epi.moff<false>(m);
+  const float row_b = epi.rb(m);
+  const float *base = ws + (long)blockIdx.x * splits * bn2 * 256 + threadIdx.x;
+  for (int c = blockIdx.y; c < bn2; c += gridDim.y) {
+    const long n = nt * bn2 + c;
+    if (n >= N) break;
+    float acc = 0.f;
+#pragma unroll 8
+    for (int z = 0; z < splits; z++) acc += base[((long)z * bn2 + c) * 256];
+    if (pair) epi.store<true>(mo, n, acc);
+    else epi.store<false>(mo, n, acc, row_b);
+  }
+}
+
+}  // namespace mm
+}  // namespace thc
+
+#endif

@@ -20,11 +20,16 @@
 // over twice the k, so that the error is smaller: 4096^3 of normal values 1.95e-7 of the result's norm against 2.94e-7 (2048^3
 // 1.70e-7 / 2.61e-7, 8192^3 2.44e-7 / 3.60e-7).  Time with the passes over the operands: 4096^3 659 -> 430 us, 8192^3 4.78 -> 2.69 ms;
 // the 256-wide convolution launches of 1024 images run 500-570 TFLOP/s where TF32 had 240-250 (its ceiling 277).
-// What bounds it: the wide tiles the tensor pipe under the power cap (570 TFLOP/s = 1.7 PFLOP/s of MMAs).
+// What bounds it: the wide tiles the tensor pipe under the power cap (570-600 TFLOP/s = 1.7-1.8 PFLOP/s of MMAs).
+//
+// 16-bit operands of either kind: the loads of both CTAs complete on CTA 0's `full` barrier directly, tiles of up to 128 columns have
+// four accumulator buffers (they end an item every few microseconds, and the MMAs run on while its results are stored), and
+// the thread that issues the loads carries its coordinates on by additions.  A relayed barrier, two
+// buffers and divisions for every load took, at 1024 images: first layer forward 1121 -> 986 us, its weight gradient 971 -> 728,
+// gradInput 64 <- 192 1625 -> 1525, the 256-wide weight gradients 357 -> 340; 128 images 3207 -> 3115 us a step.
 //
 // BF16 (opt-in math mode): no splitters and no lo slots, four kind::f16 MMAs per 64-k tile, one MMA thread; products are exact
-// in FP32 and the tolerance of the mode is BF16's, so four k tiles (16 MMAs) chain in one accumulator before a drain.  In
-// each CTA one thread passes the arrival of a tile's bytes on to CTA 0's `full` barrier.  No pipe is
+// in FP32 and the tolerance of the mode is BF16's, so four k tiles (16 MMAs) chain in one accumulator before a drain.  No pipe is
 // full (4096^3: 136 us, 1.0 PFLOP/s, tensor pipe 47 % busy): 7.9 TB/s cross from L2 into the SMs, 64 KB per 256 x 256 x 64
 // step of the pair, near the most any engine here has moved.
 //
@@ -69,7 +74,8 @@ template <int BN2, int PREC> struct Tc2rCfg {
   static constexpr int LO_SLOTS = HALF ? 0 : 3;
   static constexpr int HI_MAX = (227 * 1024 - 1024 - 512) / SLOT_BYTES - LO_SLOTS;
   static constexpr int HI_SLOTS = HI_MAX > (HALF ? 8 : 6) ? (HALF ? 8 : 6) : HI_MAX;
-  static constexpr int TMEM_COLS = 2 * BN2 > 256 ? 512 : 256;
+  static constexpr int ACCS = HALF && BN2 <= 128 ? 4 : 2;       // accumulator buffers
+  static constexpr int TMEM_COLS = ACCS * BN2 > 256 ? 512 : 256;
   static constexpr int SMEM_BYTES = (HI_SLOTS + LO_SLOTS) * SLOT_BYTES + 512 + 1024;
   static_assert(HI_SLOTS >= LO_SLOTS, "ring sizes");
   static_assert(HALF || HI_SLOTS % 2 == 0 || HI_SLOTS <= LO_SLOTS + 2, "an odd hi ring must not be longer than the lo ring + 2 (parity waits of the two MMA threads)");
@@ -110,44 +116,77 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst, const void *tmap, int 
       ::"r"(dst), "l"((unsigned long long)tmap), "r"(mbar), "r"(x), "r"(y)
       : "memory");
 }
-// PREC: the form the operand's buffer is in; `lo`: the second half of a pair.
+// The loads of one CTA's share of an operand, ROWS rows from row0 on, k tile after k tile.  PREC: the form the operand's buffer is in;
+// `lo`: the second half of a pair.  One thread issues them all, and what it does between two loads is on the engine's
+// critical path: coordinates are found by division once per item and carried on by additions.
+template <int ROWS, int PREC, bool WIDE, class Op> struct TileLoader;
 template <int ROWS, int PREC, bool WIDE, bool MN, int OWN>
-__device__ __forceinline__ void tma_issue(const RawOperand<MN, OWN> &op, uint32_t dst, long row0, long k0, bool lo, uint32_t mbar) {
-  constexpr int KV = PREC == kTf32 ? 32 : 64;
-  const CUtensorMap *map = op.map(WIDE);
-  const int off = op.half(lo);
-  if constexpr (MN) {
-    static_assert(ROWS % KV == 0, "whole row blocks");
+struct TileLoader<ROWS, PREC, WIDE, RawOperand<MN, OWN>> {
+  static constexpr int KV = PREC == kTf32 ? 32 : 64;
+  int row, k;
+  __device__ __forceinline__ TileLoader(const RawOperand<MN, OWN> &, long row0, long k0) : row((int)row0), k((int)k0) {}
+  __device__ __forceinline__ void issue(const RawOperand<MN, OWN> &op, uint32_t dst, bool lo, uint32_t mbar) const {
+    if constexpr (MN) {
+      static_assert(ROWS % KV == 0, "whole row blocks");
 #pragma unroll
-    for (int a = 0; a < ROWS / KV; a++) tma_load_2d(dst + a * KV * 128, map, (int)row0 + KV * a + off, (int)k0, mbar);
-  } else {
-    tma_load_2d(dst, map, (int)k0 + off, (int)row0, mbar);
+      for (int a = 0; a < ROWS / KV; a++) tma_load_2d(dst + a * KV * 128, op.map(WIDE), row + KV * a + op.half(lo), k, mbar);
+    } else {
+      tma_load_2d(dst, op.map(WIDE), k + op.half(lo), row, mbar);
+    }
   }
-}
+  __device__ __forceinline__ void next(const RawOperand<MN, OWN> &) { k += KV; }
+};
 // Convolution windows as rows (K-major): one im2col load of KV channels of ROWS = 128 consecutive windows.
 template <int ROWS, int PREC, bool WIDE, int OWN>
-__device__ __forceinline__ void tma_issue(const PlanesWindowOperand<OWN> &op, uint32_t dst, long row0, long k0, bool lo, uint32_t mbar) {
-  constexpr int KV = PREC == kTf32 ? 32 : 64;
+struct TileLoader<ROWS, PREC, WIDE, PlanesWindowOperand<OWN>> {
+  static constexpr int KV = PREC == kTf32 ? 32 : 64;
   static_assert(ROWS == TC_BM, "the window map loads 128 windows");
-  int x, y, img, i, j, ct;
-  op.tile_origin(row0, x, y, img);
-  op.tile_tap(WIDE ? op.ctiles_wide : op.ctiles, (unsigned)(k0 / KV), i, j, ct);
-  tma_load_windows(dst, op.map(WIDE), ct * KV + op.half(lo), x, y, img, j, i, mbar);
-}
+  int x, y, img, i, j, c;
+  __device__ __forceinline__ TileLoader(const PlanesWindowOperand<OWN> &op, long row0, long k0) {
+    op.tile_origin(row0, x, y, img);
+    op.tile_tap((unsigned)k0, i, j, c);
+  }
+  __device__ __forceinline__ void issue(const PlanesWindowOperand<OWN> &op, uint32_t dst, bool lo, uint32_t mbar) const {
+    tma_load_windows(dst, op.map(WIDE), c + op.half(lo), x, y, img, j, i, mbar);
+  }
+  __device__ __forceinline__ void next(const PlanesWindowOperand<OWN> &op) {
+    c += KV;
+    if (c == (int)op.C.d) {
+      c = 0;
+      if (++j == (int)op.kW.d) { j = 0; i++; }
+    }
+  }
+};
 // Convolution windows as the reduction (MN-major): per KV-row block, KV channels of KV consecutive windows.
 template <int ROWS, int PREC, bool WIDE, int OWN>
-__device__ __forceinline__ void tma_issue(const WindowRowsOperand<OWN> &op, uint32_t dst, long row0, long k0, bool lo, uint32_t mbar) {
-  constexpr int KV = PREC == kTf32 ? 32 : 64;
+struct TileLoader<ROWS, PREC, WIDE, WindowRowsOperand<OWN>> {
+  static constexpr int KV = PREC == kTf32 ? 32 : 64, BLOCKS = ROWS / KV;
   static_assert(ROWS % KV == 0, "whole row blocks");
-  int x, y, img;
-  op.pixel_origin(k0, x, y, img);
-#pragma unroll
-  for (int a = 0; a < ROWS / KV; a++) {
-    int i, j, c0;
-    op.row_tap(row0 + KV * a, i, j, c0);
-    tma_load_windows(dst + a * KV * 128, op.map(WIDE), c0 + op.half(lo), x, y, img, j, i, mbar);
+  int x, y, img, i0, j0, c0;   // the other blocks' taps by addition each time: kept, they would spill
+  __device__ __forceinline__ TileLoader(const WindowRowsOperand<OWN> &op, long row0, long k0) {
+    op.pixel(k0, x, y, img);
+    op.row_tap(row0, i0, j0, c0);
   }
-}
+  __device__ __forceinline__ void issue(const WindowRowsOperand<OWN> &op, uint32_t dst, bool lo, uint32_t mbar) const {
+    const int cx = x * op.ks.sx + op.ks.x0, cy = y * op.ks.sy + op.ks.y0;
+    int i = i0, j = j0, c = c0;
+#pragma unroll
+    for (int a = 0; a < BLOCKS; a++) {
+      tma_load_windows(dst + a * KV * 128, op.map(WIDE), c + op.half(lo), cx, cy, img, j, i, mbar);
+      c += KV;
+      if (c == (int)op.C.d) {
+        c = 0;
+        if (++j == (int)op.kW.d) { j = 0; i++; }
+      }
+    }
+  }
+  __device__ __forceinline__ void next(const WindowRowsOperand<OWN> &op) {   // KV pixels on
+    const WindowStep &s = op.step[PREC == kTf32 ? 0 : 1];
+    x += s.x; y += s.y; img += s.img;
+    if (x >= (int)op.ks.XW.d) { x -= (int)op.ks.XW.d; y++; }
+    if (y >= op.oH) { y -= op.oH; img++; }
+  }
+};
 
 // ---- item hand-out ------------------------------------------------------------------------------------------
 // The clusters of a launch take their work items from a counter in device memory, first come first served, so a
@@ -165,7 +204,7 @@ constexpr int T2R_SCHED_WARP = 7;
 constexpr uint32_t T2R_NO_ITEM = 0xffffffffu;
 constexpr int T2R_ITEM_WAIT_SHIFT = 6;   // item-level waits may take 64 k-tile limits (see mbar_wait)
 // readers per slot: TMA thread, 4 splitter warps (16-bit operands: one relay), 8 drain warps in each CTA, the MMA threads in the leader
-template <bool HALF> struct Tc2rReaders { static constexpr uint32_t count = 2 * (1 + (HALF ? 1 : 4) + T2_DRAIN_WARPS) + (HALF ? 1 : 2); };
+template <bool HALF> struct Tc2rReaders { static constexpr uint32_t count = 2 * (1 + (HALF ? 0 : 4) + T2_DRAIN_WARPS) + (HALF ? 1 : 2); };
 
 __device__ __forceinline__ void mbar_arrive_local(uint32_t bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
@@ -211,18 +250,18 @@ __device__ __forceinline__ void tc2r_run(const P &p, const StallCtl &ctl, unsign
   constexpr int KV = HALF ? 64 : 32;
   constexpr int CHAIN = PAIRS ? 1 : T2R_HALF_CHAIN;
   typedef Tc2rCfg<BN2, PREC> Cfg;
-  constexpr int R = Cfg::HI_SLOTS, L = Cfg::LO_SLOTS, LM = L > 0 ? L : 1;
+  constexpr int R = Cfg::HI_SLOTS, L = Cfg::LO_SLOTS, LM = L > 0 ? L : 1, ACCS = Cfg::ACCS;
   constexpr int BH = Cfg::BH;
   extern __shared__ uint8_t smem_raw[];
   uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   uint8_t *lo_ring = smem + R * Cfg::SLOT_BYTES;
   uint8_t *aux = lo_ring + L * Cfg::SLOT_BYTES;
-  // full[R], empty[R], raw_full[R], acc_full[2], acc_empty[2], lo_empty[L], sched_full[T2R_SCHED], sched_empty[T2R_SCHED], sched_go
+  // full[R], empty[R], raw_full[R] (kTf32), acc_full[ACCS], acc_empty[ACCS], lo_empty[L], sched_full[T2R_SCHED], sched_empty[T2R_SCHED], sched_go
   uint64_t *bars = reinterpret_cast<uint64_t *>(aux);
-  uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + 3 * R + 4 + L + 2 * T2R_SCHED + 1);
+  uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + 3 * R + 2 * ACCS + L + 2 * T2R_SCHED + 1);
   volatile WaitCtl *abort_flag = reinterpret_cast<volatile WaitCtl *>(tmem_slot + 2);
   uint32_t *sched_ring = tmem_slot + 2 + sizeof(WaitCtl) / 4;
-  static_assert((3 * R + 4 + L + 2 * T2R_SCHED + 1) * 8 + 8 + sizeof(WaitCtl) + 4 * T2R_SCHED <= 512, "auxiliary shared memory");
+  static_assert((3 * R + 2 * ACCS + L + 2 * T2R_SCHED + 1) * 8 + 8 + sizeof(WaitCtl) + 4 * T2R_SCHED <= 512, "auxiliary shared memory");
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const uint32_t rank = cluster_ctarank();
@@ -255,9 +294,9 @@ __device__ __forceinline__ void tc2r_run(const P &p, const StallCtl &ctl, unsign
   };
 
   const uint32_t bar_full = smem_u32(bars), bar_empty = smem_u32(bars + R), bar_raw = smem_u32(bars + 2 * R);
-  const uint32_t bar_acc_full = smem_u32(bars + 3 * R), bar_acc_empty = smem_u32(bars + 3 * R + 2);
-  const uint32_t bar_lo_empty = smem_u32(bars + 3 * R + 4);
-  const uint32_t bar_sched_full = smem_u32(bars + 3 * R + 4 + L), bar_sched_empty = bar_sched_full + 8 * T2R_SCHED;
+  const uint32_t bar_acc_full = smem_u32(bars + 3 * R), bar_acc_empty = smem_u32(bars + 3 * R + ACCS);
+  const uint32_t bar_lo_empty = smem_u32(bars + 3 * R + 2 * ACCS);
+  const uint32_t bar_sched_full = smem_u32(bars + 3 * R + 2 * ACCS + L), bar_sched_empty = bar_sched_full + 8 * T2R_SCHED;
   const uint32_t bar_sched_go = bar_sched_empty + 8 * T2R_SCHED;
   Tc2rSched sched;
   sched.full = bar_sched_full;
@@ -265,7 +304,7 @@ __device__ __forceinline__ void tc2r_run(const P &p, const StallCtl &ctl, unsign
   sched.ring = smem_u32(sched_ring);
   if (tid == 0) {
     for (int s = 0; s < R; s++) {
-      mbar_init(bar_full + 8 * s, HALF ? 2 : 2 * T2_PRODUCERS / 64);   // one relay / group of two splitter warps in each CTA (used in CTA 0)
+      mbar_init(bar_full + 8 * s, HALF ? 1 : 2 * T2_PRODUCERS / 64);   // used in CTA 0: its TMA thread and both CTAs' bytes / a group of two splitter warps in each CTA
       mbar_init(bar_empty + 8 * s, 1);
       mbar_init(bar_raw + 8 * s, 1);                        // this CTA's TMA thread + the bytes it announces
     }
@@ -275,7 +314,7 @@ __device__ __forceinline__ void tc2r_run(const P &p, const StallCtl &ctl, unsign
       mbar_init(bar_sched_empty + 8 * k, Tc2rReaders<HALF>::count);   // used in CTA 0
     }
     mbar_init(bar_sched_go, 1);                                // used in CTA 0
-    for (int b = 0; b < 2; b++) {
+    for (int b = 0; b < ACCS; b++) {
       mbar_init(bar_acc_full + 8 * b, 1);
       mbar_init(bar_acc_empty + 8 * b, 2 * T2_DRAIN_WARPS);
     }
@@ -296,28 +335,7 @@ __device__ __forceinline__ void tc2r_run(const P &p, const StallCtl &ctl, unsign
     // ------------------------------------------------------------ splitters
     setmaxnreg_dec<72>();
     const uint32_t full_leader = mapa_shared(bar_full, 0);
-    if constexpr (HALF) {
-      // 16-bit tiles are ready as they land: one thread tells CTA 0 so
-      if (warp == 0 && lane == 0) {
-        int g0 = 0;
-        for (uint32_t n = 0; ok; n++) {
-          uint32_t w = T2R_NO_ITEM;
-          ok = sched.next(n, w, abort_flag);
-          if (!ok) break;
-          sched.done(n);
-          if (w == T2R_NO_ITEM) break;
-          const int nk = item_at(w).num_k_tiles * PARTS;
-          for (int it = 0; it < nk; it++) {
-            const int g = g0 + it, s = g % R;
-            ok = mbar_wait(bar_raw + 8 * s, (uint32_t)(g / R) & 1u, abort_flag, kWaitRawTile);
-            if (!ok) break;
-            mbar_arrive_cluster(full_leader + 8 * s);
-          }
-          g0 += nk;
-        }
-      }
-      __syncwarp();
-    } else {
+    if constexpr (!HALF) {
     // Two groups of two warps take alternate k tiles, so that one group's barrier round trips and proxy fence
     // overlap the other group's copying: under the MMAs' own shared-memory traffic every access here waits
     // hundreds of cycles.
@@ -368,7 +386,8 @@ __device__ __forceinline__ void tc2r_run(const P &p, const StallCtl &ctl, unsign
       // ---------------------------------------------------------- MMA issuer of 16-bit operands: one thread, CHAIN k tiles per buffer
       constexpr bool A_MN = P::OpA::MN_MAJOR, B_MN = P::OpB::MN_MAJOR;
       constexpr uint32_t idesc = PAIRS ? umma2_idesc_f16(BN2, A_MN, B_MN) : umma2_idesc_bf16(BN2, A_MN, B_MN);
-      int g = 0, grp = 0;
+      const uint32_t ring = smem_u32(smem);
+      uint32_t s = 0, phase = 0, buf = 0, acc_phase = 0;
       for (uint32_t n = 0; ok; n++) {
         uint32_t w = T2R_NO_ITEM;
         ok = sched.next(n, w, abort_flag);
@@ -376,18 +395,18 @@ __device__ __forceinline__ void tc2r_run(const P &p, const StallCtl &ctl, unsign
         sched.done(n);
         if (w == T2R_NO_ITEM) break;
         const int nk = item_at(w).num_k_tiles;
-        for (int it = 0; it < nk; it++, g++) {
-          const int buf = grp & 1;
+        for (int it = 0; it < nk; it++) {
           const bool first = it % CHAIN == 0, last = it % CHAIN == CHAIN - 1 || it == nk - 1;
-          const uint32_t d = tmem_base + (uint32_t)(buf * BN2);
-          if (first) ok = mbar_wait_spin(bar_acc_empty + 8 * buf, ((uint32_t)(grp >> 1) & 1u) ^ 1u, abort_flag, kWaitAccEmpty);
+          const uint32_t d = tmem_base + buf * BN2;
+          if (first) ok = mbar_wait_spin(bar_acc_empty + 8 * buf, acc_phase ^ 1u, abort_flag, kWaitAccEmpty);
+          ok = ok && mbar_wait_spin(bar_full + 8 * s, phase, abort_flag, kWaitTileFull);
           if constexpr (PAIRS) {
-            const int gl = 2 * g, sl = gl % R, sh = (gl + 1) % R;
-            ok = ok && mbar_wait_spin(bar_full + 8 * sl, (uint32_t)(gl / R) & 1u, abort_flag, kWaitTileFull);
-            ok = ok && mbar_wait_spin(bar_full + 8 * sh, (uint32_t)((gl + 1) / R) & 1u, abort_flag, kWaitTileFull);
+            const uint32_t sl = s;
+            if (++s == R) { s = 0; phase ^= 1u; }
+            ok = ok && mbar_wait_spin(bar_full + 8 * s, phase, abort_flag, kWaitTileFull);
             if (!ok) break;
             tc_fence_after();
-            const uint32_t lo = smem_u32(smem + sl * Cfg::SLOT_BYTES), hi = smem_u32(smem + sh * Cfg::SLOT_BYTES);
+            const uint32_t lo = ring + sl * Cfg::SLOT_BYTES, hi = ring + s * Cfg::SLOT_BYTES;
             const uint64_t a_lo = umma_desc_half<A_MN>(lo), b_lo = umma_desc_half<B_MN>(lo + Cfg::A_BYTES);
             const uint64_t a_hi = umma_desc_half<A_MN>(hi), b_hi = umma_desc_half<B_MN>(hi + Cfg::A_BYTES);
 #pragma unroll
@@ -401,22 +420,23 @@ __device__ __forceinline__ void tc2r_run(const P &p, const StallCtl &ctl, unsign
 #pragma unroll
             for (int kk = 1; kk < 4; kk++)
               umma2_f16(d, a_hi + (uint64_t)((kk * umma_kstep_bytes_half<A_MN>()) >> 4), b_hi + (uint64_t)((kk * umma_kstep_bytes_half<B_MN>()) >> 4), idesc, 1u);
-            umma2_commit_both(bar_empty + 8 * sh);
           } else {
-            const int s = g % R;
-            ok = ok && mbar_wait_spin(bar_full + 8 * s, (uint32_t)(g / R) & 1u, abort_flag, kWaitTileFull);
             if (!ok) break;
             tc_fence_after();
-            const uint32_t st = smem_u32(smem + s * Cfg::SLOT_BYTES);
+            const uint32_t st = ring + s * Cfg::SLOT_BYTES;
             const uint64_t a_d = umma_desc_half<A_MN>(st), b_d = umma_desc_half<B_MN>(st + Cfg::A_BYTES);
 #pragma unroll
             for (int kk = 0; kk < 4; kk++) {   // 16 k per MMA
               const uint64_t adv_a = (uint64_t)((kk * umma_kstep_bytes_half<A_MN>()) >> 4), adv_b = (uint64_t)((kk * umma_kstep_bytes_half<B_MN>()) >> 4);
               umma2_f16(d, a_d + adv_a, b_d + adv_b, idesc, (kk || !first) ? 1u : 0u);
             }
-            umma2_commit_both(bar_empty + 8 * s);
           }
-          if (last) { umma2_commit_both(bar_acc_full + 8 * buf); grp++; }
+          umma2_commit_both(bar_empty + 8 * s);
+          if (++s == R) { s = 0; phase ^= 1u; }
+          if (last) {
+            umma2_commit_both(bar_acc_full + 8 * buf);
+            if (++buf == ACCS) { buf = 0; acc_phase ^= 1u; }
+          }
         }
       }
     } else if (!HALF && (warp == T2_MMA_WARP || warp == T2R_MMA_WARP2) && lane == 0 && rank == 0) {
@@ -474,7 +494,11 @@ __device__ __forceinline__ void tc2r_run(const P &p, const StallCtl &ctl, unsign
       }
     } else if (warp == T2R_TMA_WARP && lane == 0) {
       // ---------------------------------------------------------- TMA issuer (one per CTA)
-      int g0 = 0;
+      // 16-bit tiles are ready as they land: the bytes of both CTAs complete on CTA 0's `full`.  The peer's may come before CTA 0 has
+      // announced them: the phase still waits for that arrival, and the peer's slot was free only after the phase before.
+      const uint32_t full_leader = mapa_shared(bar_full, 0), ring = smem_u32(smem);
+      uint32_t s = 0, phase = 0;
+      bool filled = false;   // every slot has been used
       for (uint32_t n = 0; ok; n++) {
         uint32_t w = T2R_NO_ITEM;
         ok = sched.next(n, w, abort_flag);
@@ -483,20 +507,28 @@ __device__ __forceinline__ void tc2r_run(const P &p, const StallCtl &ctl, unsign
         if (w == T2R_NO_ITEM) break;
         if (rank == 0) mbar_arrive_local(bar_sched_go);   // item n is under way: time to fetch the number of item n + 1
         const Tc2rItem item = item_at(w);
-        const long m0 = item.m_tile0 + (long)rank * TC_BM, n0 = item.n_tile0 + (long)rank * BH;
-        const int parts = item.num_k_tiles * PARTS;
-        for (int t = 0; t < parts; t++) {
-          const int g = g0 + t;
-          const int s = g % R;
-          if (g >= R && !mbar_wait(bar_empty + 8 * s, (uint32_t)((g - R) / R) & 1u, abort_flag, kWaitSlotEmpty)) { ok = false; break; }
-          const long k0 = item.k_begin + (long)(t / PARTS) * KV;
-          const bool lo = PAIRS && t % PARTS == 0;
-          const uint32_t slot = smem_u32(smem + s * Cfg::SLOT_BYTES);
-          mbar_arrive_expect_tx(bar_raw + 8 * s, (uint32_t)Cfg::SLOT_BYTES);
-          tma_issue<TC_BM, PREC, WIDE>(p.a, slot, m0, k0, lo, bar_raw + 8 * s);
-          tma_issue<BH, PREC, WIDE>(p.b, slot + Cfg::A_BYTES, n0, k0, lo, bar_raw + 8 * s);
+        TileLoader<TC_BM, PREC, WIDE, typename P::OpA> load_a(p.a, item.m_tile0 + (long)rank * TC_BM, item.k_begin);
+        TileLoader<BH, PREC, WIDE, typename P::OpB> load_b(p.b, item.n_tile0 + (long)rank * BH, item.k_begin);
+        for (int t = 0; ok && t < item.num_k_tiles; t++) {
+#pragma unroll
+          for (int part = 0; part < PARTS; part++) {
+            const bool lo = PAIRS && part == 0;
+            if (filled && !mbar_wait(bar_empty + 8 * s, phase ^ 1u, abort_flag, kWaitSlotEmpty)) { ok = false; break; }
+            const uint32_t slot = ring + s * Cfg::SLOT_BYTES;
+            uint32_t landed = bar_raw + 8 * s;
+            if constexpr (HALF) {
+              landed = full_leader + 8 * s;
+              if (rank == 0) mbar_arrive_expect_tx(bar_full + 8 * s, 2u * Cfg::SLOT_BYTES);
+            } else {
+              mbar_arrive_expect_tx(landed, (uint32_t)Cfg::SLOT_BYTES);
+            }
+            load_a.issue(p.a, slot, lo, landed);
+            load_b.issue(p.b, slot + Cfg::A_BYTES, lo, landed);
+            if (++s == R) { s = 0; phase ^= 1u; filled = true; }
+          }
+          load_a.next(p.a);
+          load_b.next(p.b);
         }
-        g0 += parts;
       }
     } else if (warp == T2R_SCHED_WARP && lane == 0 && rank == 0) {
       // ---------------------------------------------------------- item hand-out (one thread per cluster)
@@ -541,8 +573,8 @@ __device__ __forceinline__ void tc2r_run(const P &p, const StallCtl &ctl, unsign
       const int folds = HALF ? (item.num_k_tiles + CHAIN - 1) / CHAIN : item.num_k_tiles;   // accumulators of this item
       for (int it = 0; it < folds; it++) {
         const int g = g0 + it;
-        const int buf = g & 1;
-        const uint32_t acc_phase = (uint32_t)(g >> 1) & 1u;
+        const int buf = g % ACCS;
+        const uint32_t acc_phase = (uint32_t)(g / ACCS) & 1u;
         ok = mbar_wait(bar_acc_full + 8 * buf, acc_phase, abort_flag, kWaitAccFull);
         ok = __all_sync(0xffffffffu, ok);
         if (!ok) break;

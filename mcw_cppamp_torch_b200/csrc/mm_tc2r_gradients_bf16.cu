@@ -1,0 +1,12 @@
+// The two-SM engine over convolution windows as the reduction, BF16 values.
+#include "mm_tc2r_launch.cuh"
+
+namespace thc {
+namespace mm {
+
+TC2R_BLOCKS(Problem<RawOperand<true, kBf16>, WindowRowsOperand<kBf16>, false, kBf16>)
+TC2R_BLOCKS(Problem<WindowRowsOperand<kBf16>, RawOperand<true, kBf16>, false, kBf16>)
+TC2R_BLOCKS(Problem<WindowRowsOperand<kBf16>, WindowRowsOperand<kBf16>, false, kBf16>)
+
+}  // namespace mm
+}  // namespace thc
