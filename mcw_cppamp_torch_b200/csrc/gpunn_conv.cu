@@ -240,6 +240,15 @@ static void restate_input(const ConvGeom &g, const mm::Cells &u, const float *in
   const long rows = g.N * u.Hs, chunks = (long)u.Ws * u.Cs / (PREC != mm::kTf32 ? 8 : 4);
   const unsigned bx = (unsigned)(form.remake ? std::min(rows, 4l * ctx().sm_count) : rows);
   const unsigned parts = (unsigned)std::max(1l, std::min((chunks + 255) / 256, 4l * ctx().sm_count / rows));
+  if constexpr (PREC != mm::kBf16) {
+    const int q = u.Cs / (PREC == mm::kPairs ? 8 : 4);
+    const long Wp = (long)(u.Ws - 1) * u.dW + u.eW, ld = (Wp + 15) / 32 * 32 + 16, smem = 4l * u.C * u.eH * ld;
+    if (256 % q == 0 && smem <= 40 * 1024 && rows >= 2l * ctx().sm_count) {
+      pdl_launch(mm::cells_staged_kernel<PREC>, (unsigned)std::min(bx, 16u * ctx().sm_count), 256, smem, in, dst, g.N, u, (int)Wp, (int)ld, form);
+      check_launch("cells_staged");
+      return;
+    }
+  }
   if (u.Cs <= mm::kCellTable) pdl_launch(mm::cells_input_kernel<PREC, true>, dim3(bx, parts), 256, sizeof(int2) * u.Cs, in, dst, g.N, u, form);
   else pdl_launch(mm::cells_input_kernel<PREC, false>, dim3(bx, parts), 256, 0, in, dst, g.N, u, form);
   check_launch("cells_input");
