@@ -578,11 +578,11 @@ static bool half_acc_grad(const ConvGeom &g) {
 // the pass that measures the input, with 10 us for the launches that measure and check (64 planes under 11 x 11 / 4 over 16 images,
 // 40 us a product: 201.5 us in TF32, 212.6 over pairs for the whole block; 128 images: 4020 -> 3160 us a training step).  The column
 // form stays in TF32, whose weight gradient stacks pixels.
-static bool restate_accurate(const ConvGeom &g, mm::Cells &u, int &prec) {
+static bool restate_accurate(const ConvGeom &g, bool pairs, mm::Cells &u, int &prec) {
   prec = mm::kTf32;
   const bool ok = restate(g, mm::kTf32, u);
   mm::Cells up;
-  if (!ok || ctx().math_mode != 0 || windows_us(forward_windows(g, u), g.K, prec) < 30 || !restate(g, mm::kPairs, up) ||
+  if (!ok || !pairs || windows_us(forward_windows(g, u), g.K, prec) < 30 || !restate(g, mm::kPairs, up) ||
       (up.kHs == 1 && up.kWs == 1 && !up.direct))
     return ok;
   auto us = [&](const mm::Cells &c, int pr) {
@@ -596,7 +596,7 @@ static void conv_forward(const ConvGeom &g, const float *in, const float *w, con
   mm::Cells u;
   const bool half = half_forward(g);
   int prec = mm::kBf16;
-  if (ctx().math_mode != 1 && (half ? restate(g, prec, u) : restate_accurate(g, u, prec))) {
+  if (ctx().math_mode != 1 && (half ? restate(g, prec, u) : restate_accurate(g, ctx().math_mode == 0, u, prec))) {
     // kept for a weight gradient of the same precision only, no other reads them back: the BF16 column matrix of the 11 x 11 / 4
     // layer over 3 planes is 6.2 MB an image, and its weight gradient FP32-accurate
     THGPUTensor *keep = half == half_acc_grad(g) ? finput : nullptr;
@@ -707,7 +707,9 @@ static void conv_backward(const ConvGeom &g, const float *in, const float *gout,
   }
   if ((gin && !hin) || (gw && !hw)) {
     int prec;
-    const bool ok = restate_accurate(g, u, prec);
+    // in the BF16 mode only for weight gradients: another last bit of a layer's result or gradInput would turn into others where the
+    // next layer rounds it (the first layer's over 256 images: 385 -> 225 us)
+    const bool ok = restate_accurate(g, ctx().math_mode == 0 || !gin || hin, u, prec);
     if (prec == mm::kPairs) conv_backward_tc<mm::kPairs>(g, u, ok, in, gout, w, hin ? nullptr : gin, hw ? nullptr : gw, gb, scale, finput);
     else conv_backward_tc<mm::kTf32>(g, u, ok, in, gout, w, hin ? nullptr : gin, hw ? nullptr : gw, gb, scale, finput);
   }

@@ -287,8 +287,10 @@ static void launch_raw(P p, Attach attach) {
   with_width([&](auto w) { launch_tc2r_kernel<P, decltype(w)::value>(p, items, early); });
   if (p.ws) {
     // a few thousand blocks whatever the number of tail tiles: a lone tile cut into many slices gets a block per column
-    const long by = std::min<long>(bn2, std::max<long>(32, ceil_div(8l * ctx().sm_count, tail)));
-    pdl_launch(tail_finish_kernel, dim3((unsigned)tail, (unsigned)by), 256, 0, p.ws, p.tail_splits, bn2, p.tail_first, gm, p.M, p.N, p.epi);
+    const bool four = tail * (bn2 / 4) >= 2l * ctx().sm_count;
+    const long blocks = ceil_div(8l * ctx().sm_count, tail), by = four ? std::min<long>(bn2 / 4, std::max<long>(16, blocks)) : std::min<long>(bn2, std::max<long>(32, blocks));
+    pdl_launch(four ? tail_finish_kernel<4> : tail_finish_kernel<1>, dim3((unsigned)tail, (unsigned)by), 256, 0, p.ws, p.tail_splits, bn2, p.tail_first, gm, p.M, p.N,
+               p.epi);
     check_launch("tail_finish");
   }
 }

@@ -26,7 +26,8 @@ static __global__ void __launch_bounds__(256) range_kernel(const RangeJob ja, co
   const long warps = (long)gridDim.x * 8, total = j.lines * j.run;
   const long segs = j.flat ? (total + 511) / 512 : (j.run + 127) / 128, sets = j.flat ? segs : segs * ((j.lines + 3) / 4);
   unsigned most = 0, low = ~0u, low2 = ~0u;   // the lows as bits - 1: zero becomes the largest
-  for (long s = (long)blockIdx.x * 8 + warp; s < sets; s += warps) {
+  for (long at = (long)blockIdx.x * 8 + warp; at < sets; at += warps) {
+    const long s = sets - 1 - at;   // from the end, which whoever wrote the operand has left in L2, to the start, which the next pass reads first
     unsigned v[4][4];
     const long q = j.flat ? 0 : s / segs, c0 = j.flat ? s * 512 : (s - q * segs) * 128;
 #pragma unroll
@@ -685,28 +686,49 @@ static __global__ void __launch_bounds__(256) splitk_finish_kernel(const float *
   }
 }
 
-// The same for the tile-local partials of the raw-operand engine (Problem::tail_first): block (t, y) folds columns
-// y, y + gridDim.y, ... of tail tile t; a thread owns one of the tile's 256 rows, which are contiguous in the
-// workspace.
+// The same for the tile-local partials of the two-SM engine (Problem::tail_first): block (t, y) folds columns COLS * y .. + COLS - 1, COLS *
+// (y + gridDim.y), ... of tail tile t; a thread owns one of the tile's 256 rows, which are contiguous in the workspace.  Bound by
+// latency: four columns at once where that leaves blocks enough (8 -> 5 us for a round of tiles in two to four slices), one where
+// few tiles are cut into many slices (a tile in 70: 11.5 us, 18 with four).
+template <int COLS>
 static __global__ void __launch_bounds__(256) tail_finish_kernel(const float *__restrict__ ws, int splits, int bn2, long tail_first,
                                                           long gm, long M, long N, Epilogue epi) {
   pdl_begin();
   const long tile = tail_first + blockIdx.x;
-  const long nt = tile / gm, mt = tile - nt * gm;
+  const long nt = Epilogue::quotient(tile, gm), mt = tile - nt * gm;
   const long m = mt * 256 + threadIdx.x;
   if (m >= M) return;
   const bool pair = epi.pair_K != 0;
   const long mo = pair ? epi.moff<true>(m) : epi.moff<false>(m);
   const float row_b = epi.rb(m);
   const float *base = ws + (long)blockIdx.x * splits * bn2 * 256 + threadIdx.x;
-  for (int c = blockIdx.y; c < bn2; c += gridDim.y) {
+  for (int c = COLS * blockIdx.y; c < bn2; c += COLS * gridDim.y) {
     const long n = nt * bn2 + c;
     if (n >= N) break;
-    float acc = 0.f;
-#pragma unroll 8
-    for (int z = 0; z < splits; z++) acc += base[((long)z * bn2 + c) * 256];
-    if (pair) epi.store<true>(mo, n, acc);
-    else epi.store<false>(mo, n, acc, row_b);
+    float acc[COLS];
+#pragma unroll
+    for (int j = 0; j < COLS; j++) acc[j] = 0.f;
+#pragma unroll (COLS == 1 ? 8 : 4)
+    for (int z = 0; z < splits; z++)
+#pragma unroll
+      for (int j = 0; j < COLS; j++) acc[j] += base[((long)z * bn2 + c + j) * 256];
+    if constexpr (COLS == 4) {
+      float *o = epi.out + mo + n;
+      if (!pair && epi.nstride == 1 && n + 3 < N && (reinterpret_cast<uintptr_t>(o) & 15) == 0) {   // the columns are neighbours in memory
+        float4 old = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (epi.beta != 0.f) old = *reinterpret_cast<const float4 *>(o);
+        const float4 v = make_float4(epi.value(n, acc[0], row_b, old.x), epi.value(n + 1, acc[1], row_b, old.y), epi.value(n + 2, acc[2], row_b, old.z),
+                                     epi.value(n + 3, acc[3], row_b, old.w));
+        *reinterpret_cast<float4 *>(o) = v;
+        continue;
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < COLS; j++) {
+      if (n + j >= N) break;
+      if (pair) epi.store<true>(mo, n + j, acc[j]);
+      else epi.store<false>(mo, n + j, acc[j], row_b);
+    }
   }
 }
 

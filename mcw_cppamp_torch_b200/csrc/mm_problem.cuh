@@ -271,13 +271,15 @@ struct Epilogue {
   __device__ __forceinline__ float rb(long m) const { return row_bias ? __ldg(row_bias + m) : 0.f; }
   static constexpr long kLastOdd = 1l << 62;
   // PAIR is a compile-time property of the problem: the common path carries none of the pair arithmetic
+  // a / b, by the short division where it will do
+  static __device__ __forceinline__ long quotient(long a, long b) { return ((a | b) >> 32) == 0 ? (long)((unsigned)a / (unsigned)b) : a / b; }
   template <bool PAIR = false>
   __device__ __forceinline__ long moff(long m) const {
     if (PAIR) {
-      const long r = m / pair_oW2, x2 = m - r * pair_oW2, img = r / pair_oH, y = r - img * pair_oH;
+      const long r = quotient(m, pair_oW2), x2 = m - r * pair_oW2, img = quotient(r, pair_oH), y = r - img * pair_oH;
       return (img * pair_img + y * pair_oW + 2 * x2) | (2 * x2 + 1 >= pair_oW ? kLastOdd : 0);
     }
-    const long q = m / mdiv;
+    const long q = m < mdiv ? 0 : quotient(m, mdiv);
     return q * mouter + (m - q * mdiv);
   }
   // the same with the destination's previous value already in a register (never in pixel-pair mode)
@@ -316,10 +318,13 @@ struct Epilogue {
       return;
     }
     const long o = mo + n * nstride;
+    out[o] = value(n, acc, row_b, beta != 0.f ? out[o] : 0.f);
+  }
+  __device__ __forceinline__ float value(long n, float acc, float row_b, float old) const {
     float v = alpha * acc + row_b;
     if (bias) v += bias[n];
-    if (beta != 0.f) v += beta * out[o];
-    out[o] = v;
+    if (beta != 0.f) v += beta * old;
+    return v;
   }
 };
 
