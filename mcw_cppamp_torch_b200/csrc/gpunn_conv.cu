@@ -12,6 +12,7 @@
 
 #include <unordered_map>
 #include <utility>
+#include <vector>
 
 namespace thc {
 
@@ -49,15 +50,31 @@ static ConvGeom conv_geom(const THGPUTensor *input, const THGPUTensor *weight, i
 // that does not write `finput` forgets the entry, so planes of an earlier pass are never taken for fresh ones.
 // Keyed by the address of finput's data; one table per host thread, as the rest of the library's state.
 namespace {
-struct PlaneStamp { const float *input; int prec; long N, C, H, W, K; int kH, kW, dH, dW, pad; };
+// Pairs have a record (mm::RangeRec), `record` of the context's plane_records; the slots belong to the entries of this table.
+struct PlaneStamp { const float *input; int prec; long N, C, H, W, K; int kH, kW, dH, dW, pad; int record; long epoch; };
 thread_local std::unordered_map<const float *, PlaneStamp> g_plane_stamps;
+thread_local std::vector<int> g_free_records;   // of the slots below g_records
+thread_local int g_records = 0;
 void stamp_planes(const THGPUTensor *finput, const float *input, const ConvGeom &g, int prec) {
   if (!finput || !finput->storage) return;
-  if (g_plane_stamps.size() > 4096) g_plane_stamps.clear();
-  g_plane_stamps[data_ptr(finput)] = PlaneStamp{input, prec, g.N, g.C, g.H, g.W, g.K, g.kH, g.kW, g.dH, g.dW, g.pad};
+  int record = -1;
+  if (g_plane_stamps.size() >= kPlaneRecords) { g_plane_stamps.clear(); g_free_records.clear(); g_records = 0; }
+  if (prec == mm::kPairs) {
+    if (g_free_records.empty()) record = g_records++;
+    else { record = g_free_records.back(); g_free_records.pop_back(); }
+  }
+  g_plane_stamps[data_ptr(finput)] = PlaneStamp{input, prec, g.N, g.C, g.H, g.W, g.K, g.kH, g.kW, g.dH, g.dW, g.pad, record, ctx().plane_epoch};
 }
 void forget_planes(const THGPUTensor *finput) {
-  if (finput && finput->storage) g_plane_stamps.erase(data_ptr(finput));
+  if (!finput || !finput->storage) return;
+  auto it = g_plane_stamps.find(data_ptr(finput));
+  if (it == g_plane_stamps.end()) return;
+  if (it->second.record >= 0) g_free_records.push_back(it->second.record);
+  g_plane_stamps.erase(it);
+}
+// The record of planes that are known to be fresh.
+mm::RangeRec *planes_record(const void *planes) {
+  return (mm::RangeRec *)plane_records() + g_plane_stamps.at((const float *)planes).record;
 }
 }  // namespace
 
@@ -255,20 +272,15 @@ static void restate_input(const ConvGeom &g, const mm::Cells &u, const float *in
 }
 
 // Room for the restated input in `finput` (the counterpart of the column matrix the reference keeps there): a
-// [1, N, Hs, Ws, floats per pixel] tensor that accGradParameters reads back instead of making it again.  Pairs have their
-// record behind the tensor, in the same storage.  Null: no room that a TMA map can address.
+// [1, N, Hs, Ws, floats per pixel] tensor that accGradParameters reads back instead of making it again.  Null: no room that a
+// TMA map can address.
 static void *planes_in(THGPUTensor *finput, const ConvGeom &g, const mm::Cells &u, const float *in, int prec) {
-  const long s[5] = {1, g.N, u.Hs, u.Ws, prec == mm::kBf16 ? u.Cs / 2 : u.Cs}, n = s[1] * s[2] * s[3] * s[4];
+  const long s[5] = {1, g.N, u.Hs, u.Ws, prec == mm::kBf16 ? u.Cs / 2 : u.Cs};
   resize_nd(finput, 5, s, nullptr);
-  if (prec == mm::kPairs && finput->storage && finput->storage->size < finput->storageOffset + n + mm::kRangeWords)
-    storage_resize(finput->storage, finput->storageOffset + n + mm::kRangeWords);
   forget_planes(finput);
   if (!is_contiguous(finput) || ((uintptr_t)data_ptr(finput) & 15) != 0) return nullptr;
   stamp_planes(finput, in, g, prec);
   return data_ptr(finput);
-}
-static mm::RangeRec *record_behind(const void *planes, const ConvGeom &g, const mm::Cells &u) {
-  return (mm::RangeRec *)((char *)planes + mm::planes_bytes(g.N, (long)u.Hs * u.Ws, u.Cs, mm::kPairs));
 }
 
 // The planes the forward pass of this very layer over this very input left in `finput`, or null.  A `finput` that has been given
@@ -277,12 +289,11 @@ static const void *planes_made_from(const THGPUTensor *finput, const float *inpu
   if (!finput || !finput->storage || finput->nDimension != 5 || !is_contiguous(finput)) return nullptr;
   const long shape[5] = {1, g.N, u.Hs, u.Ws, prec == mm::kBf16 ? u.Cs / 2 : u.Cs};
   if (!std::equal(shape, shape + 5, finput->size)) return nullptr;
-  if (prec == mm::kPairs && finput->storage->size < finput->storageOffset + nelem(finput) + mm::kRangeWords) return nullptr;
   auto it = g_plane_stamps.find(data_ptr(finput));
   if (it == g_plane_stamps.end()) return nullptr;
   const PlaneStamp &s = it->second;
   const bool same = s.input == input && s.prec == prec && s.N == g.N && s.C == g.C && s.H == g.H && s.W == g.W && s.K == g.K &&
-                    s.kH == g.kH && s.kW == g.kW && s.dH == g.dH && s.dW == g.dW && s.pad == g.pad;
+                    s.kH == g.kH && s.kW == g.kW && s.dH == g.dH && s.dW == g.dW && s.pad == g.pad && s.epoch == ctx().plane_epoch;
   return same ? data_ptr(finput) : nullptr;
 }
 
@@ -307,7 +318,7 @@ static void conv_forward_tc(const ConvGeom &g, const mm::Cells &u, const float *
     mm::PairForm form;
     form.ranges = rec.joint(rec.act);
     void *act = finput ? planes_in(finput, s, u, x, PREC) : nullptr;
-    if (act && PREC == mm::kPairs) form.keep = record_behind(act, s, u);
+    if (act && PREC == mm::kPairs) form.keep = planes_record(act);
     if (!act) act = ws_alloc(mm::planes_bytes(s.N, (long)u.Hs * u.Ws, u.Cs, PREC));
     restate_input<PREC>(s, u, x, act, form);
     window_product<PREC, false>(act, forward_windows(s, u), w, u, g.K, g.K, bias, out + n0 * g.K * g.P, rec);
@@ -582,7 +593,8 @@ static bool restate_accurate(const ConvGeom &g, bool pairs, mm::Cells &u, int &p
   prec = mm::kTf32;
   const bool ok = restate(g, mm::kTf32, u);
   mm::Cells up;
-  if (!ok || !pairs || windows_us(forward_windows(g, u), g.K, prec) < 30 || !restate(g, mm::kPairs, up) ||
+  if (!ok || !pairs || g.R > 1l << 28 || g.K * g.kH * g.kW > 1l << 28 ||   // (a row of weights and its second half: 31 bits)
+      windows_us(forward_windows(g, u), g.K, prec) < 30 || !restate(g, mm::kPairs, up) ||
       (up.kHs == 1 && up.kWs == 1 && !up.direct))
     return ok;
   auto us = [&](const mm::Cells &c, int pr) {
@@ -665,7 +677,7 @@ static void conv_backward_tc(const ConvGeom &g, const mm::Cells &u, bool restate
     mm::launch_ranges(jg, rw ? &jw : nullptr);
     rec.gout = rg; rec.weight = rw;
     if (act) {
-      mm::RangeRec *kept = record_behind(act, g, u);
+      mm::RangeRec *kept = planes_record(act);
       rec.act = kept;
       mm::PairForm form;
       form.ranges = rec.joint(kept);

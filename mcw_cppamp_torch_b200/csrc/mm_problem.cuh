@@ -54,6 +54,7 @@ struct RangeRec {
   unsigned pad[3];
 };
 constexpr int kRangeWords = sizeof(RangeRec) / 4;
+static_assert(sizeof(RangeRec) == 32, "plane_records() hands out 32 bytes each");
 __device__ __forceinline__ bool range_is_wide(const RangeRec &r) {
   if (r.wide) return true;
   if (r.max_bits == 0) return false;   // zeros only

@@ -149,8 +149,9 @@ static void gemm_pairs(GemmSide x, GemmSide y, long k, float alpha, float beta, 
   else if (!x.along_k) gemm_pairs_t<true, true>(jobs[0].dst, jobs[0].ldp, jobs[1].dst, jobs[1].ldp, x.rows, y.rows, k, epi, rec[0], rec[1]);
   else gemm_pairs_t<false, true>(jobs[0].dst, jobs[0].ldp, jobs[1].dst, jobs[1].ldp, x.rows, y.rows, k, epi, rec[0], rec[1]);
 }
-// Whether pairs finish before TF32, the passes over the operands included.
+// Whether pairs finish before TF32, the passes over the operands included.  Their copies are scratch that TF32 does without: bounded.
 static bool pairs_are_faster(long m, long n, long k) {
+  if (4. * (double)k * (double)(m + n) > 16e9 || std::max(std::max(m, n), k) > 1l << 28) return false;
   const double passes = 8 + 4e-6 * (double)k * (double)(m + n) * (1 / 5.5 + 2 / 5.0);
   return mm::tc2_product_us(m, n, k, mm::kPairs, true) + passes < mm::tc2_product_us(m, n, k, mm::kTf32);
 }

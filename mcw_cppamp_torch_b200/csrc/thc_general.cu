@@ -53,6 +53,7 @@ static void init_device(Context &c, int device) {
   if (c.scratch) { cudaFree(c.scratch); c.scratch = nullptr; c.scratch_bytes = 0; }
   if (c.stall_dev) { cudaFree(c.stall_dev); c.stall_dev = nullptr; }
   if (c.sched_counters) { cudaFree(c.sched_counters); c.sched_counters = nullptr; c.sched_stream = nullptr; }
+  if (c.plane_records) { cudaFree(c.plane_records); c.plane_records = nullptr; c.plane_epoch++; }
   if (c.ws_base) { cudaFree(c.ws_base); c.ws_base = nullptr; c.ws_cap = c.ws_used = 0; c.ws_epoch++; }
   c.device = device;
   THC_CUDA(cudaStreamCreateWithFlags(&c.stream, cudaStreamNonBlocking));
@@ -120,9 +121,19 @@ unsigned *zeroed_words(int n) {
   }
   unsigned *p = c.sched_counters + c.sched_block * kBlock + c.sched_next;
   c.sched_next += n;
+  // a recorded launch runs many times over: its words are cleared each time
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(c.stream, &capture) == cudaSuccess && capture == cudaStreamCaptureStatusActive)
+    THC_CUDA(cudaMemsetAsync(p, 0, sizeof(unsigned) * n, c.stream));
   return p;
 }
 unsigned *sched_counter() { return zeroed_words(1); }
+
+void *plane_records() {
+  Context &c = ctx();
+  if (!c.plane_records) THC_CUDA(cudaMalloc(&c.plane_records, 32 * kPlaneRecords));
+  return c.plane_records;
+}
 
 // Names of the wait codes of mm_tc.cuh (kWait*), for the error message.
 static const char *wait_name(int code) {
