@@ -392,10 +392,12 @@ static ActPlanes make_act_planes(const float *src, long N, long C, long H, long 
   ap.N = N; ap.H = H; ap.W = W; ap.Cp = padded_channels(C, PREC);
   ap.p = dst ? dst : ws_alloc(planes_bytes(N, HW, ap.Cp, PREC));
   const long cap = (long)ctx().sm_count * 16;
-  const long needed = PREC != kTf32 ? N * ((HW + 63) / 64) * (ap.Cp / 64) : N * ((HW + 127) / 128) * (ap.Cp / 32);
+  const bool wide_tile = PREC == kPairs && (HW + 127) / 128 * 128 * 10 <= (HW + 63) / 64 * 64 * 11;
+  const int pt = PREC == kTf32 || wide_tile ? 128 : 64;
+  const long needed = N * ((HW + pt - 1) / pt) * (ap.Cp / (PREC != kTf32 ? 64 : 32));
   long blocks = std::min(needed, cap);
   size_t smem = 0;
-  if (want_chan_sums && C <= 4096) {
+  if (want_chan_sums && C <= (wide_tile ? 3968 : 4096)) {   // (with the tile, 48 KB)
     // every block leaves a row of per-channel sums for a second kernel to fold.  On a small tensor (a few tiles per
     // block) that fold costs as much as the transposition: a quarter of the blocks keeps it short (measured at
     // 128 images: fold 83 -> 33 us, transposition unchanged); on a large one the transposition wants all its
@@ -406,7 +408,7 @@ static ActPlanes make_act_planes(const float *src, long N, long C, long H, long 
     smem = sizeof(float) * C;
   }
   if constexpr (PREC == kPairs)
-    pdl_launch(nchw_to_pairs_kernel, (unsigned)blocks, 256, smem, src, N, (int)C, (int)HW, (int)ap.Cp, ap.p, ap.chan_partial, form);
+    pdl_launch(wide_tile ? nchw_to_pairs_kernel<128> : nchw_to_pairs_kernel<64>, (unsigned)blocks, 256, smem, src, N, (int)C, (int)HW, (int)ap.Cp, ap.p, ap.chan_partial, form);
   else
     pdl_launch(nchw_to_planes_kernel<PREC == kBf16>, (unsigned)blocks, 256, smem, src, N, (int)C, (int)HW, (int)ap.Cp, ap.p, ap.chan_partial);
   check_launch("nchw_to_planes");

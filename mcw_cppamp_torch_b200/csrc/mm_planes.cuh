@@ -159,7 +159,10 @@ static __global__ void __launch_bounds__(256) nchw_to_planes_kernel(const float 
   if (chan_partial)
     for (int c = threadIdx.x; c < C; c += blockDim.x) chan_partial[(long)blockIdx.x * C + c] = chan_sum[c];
 }
-// The same as FP16 pairs, [img][pixel][hi: Cp][lo: Cp], or FP32 values in the same place.
+// The same as FP16 pairs, [img][pixel][hi: Cp][lo: Cp], or FP32 values in the same place.  Bound by latency: 128 pixels a pass keep
+// twice the loads in flight (198 M values with channel sums, 1.6 GB: 322 -> 277 us), 64 where planes would leave much of the
+// wider tile empty (13 x 13: 92 us with 128, 83 with 64).
+template <int PT>
 static __global__ void __launch_bounds__(256) nchw_to_pairs_kernel(const float *__restrict__ src, long N, int C, int HW, int Cp,
                                                                    void *__restrict__ dst, float *__restrict__ chan_partial,
                                                                    const PairForm form) {
@@ -167,7 +170,7 @@ static __global__ void __launch_bounds__(256) nchw_to_pairs_kernel(const float *
   bool wide;
   if (!form.begin(wide)) return;
   const float scale = wide ? 1.f : pair_scale(*form.ranges.rec[0]);
-  constexpr int CT = 64, PT = 64;
+  constexpr int CT = 64;
   __shared__ float tile[CT][PT + 1];
   extern __shared__ float chan_sum[];   // [C] when chan_partial is given
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
