@@ -391,7 +391,7 @@ def tensor_math_report(gt, nn, torch, ts, hbm_gbs):
 # ------------------------------------------------------------------ the CUDA arm
 def tf32_yardstick(torch):
     """Dense TF32 rate of a LIBRARY GEMM in this very run (torch.matmul = cuBLAS with TF32 allowed, 8192^3, best of
-    10): the denominator the 3xTF32 engine is measured against.  It is outside the product, which never calls it."""
+    10): what three FP16 products are compared with beside the 16-bit peak.  It is outside the product, which never calls it."""
     prev = torch.backends.cuda.matmul.allow_tf32
     torch.backends.cuda.matmul.allow_tf32 = True
     try:
@@ -799,18 +799,18 @@ def run_ours(args):
         pk, src = peaks()
         tf32_run = tf32_yardstick(torch)
         ach = tot_f / tot_t / 1e12
-        roof = {"bound": "tensor", "achieved": ach, "peak": tf32_run, "unit": "TFLOP/s", "frac": ach / tf32_run,
+        roof = {"bound": "tensor", "achieved": ach, "peak": pk["bf16_tflops"], "unit": "TFLOP/s", "frac": ach / pk["bf16_tflops"],
                 # DRAM bytes of the GEMM-shaped launches of one step (ncu dram__bytes_read.sum + dram__bytes_write.sum
-                # over the 23 tc2r_kernel launches of a step captured at batch 128): 831 MB in the three classifier
-                # layers, whose traffic is their weights and does not grow with the batch, and 7.09 MB per image
-                # in the convolution layers, scaled to this rank's batch
+                # over the 23 tc2r_kernel launches of a step captured at batch 128, over FP32 operands; FP16 pairs have as many
+                # bytes): 831 MB in the three classifier layers, whose traffic is their weights and does not grow with the
+                # batch, and 7.09 MB per image in the convolution layers, scaled to this rank's batch
                 "traffic": 0.831e9 + 7.09e6 * nloc,
-                "kernel": "thc::mm::tc2r_kernel (persistent two-SM tcgen05 3xTF32 GEMM / implicit GEMM over raw FP32 operands)",
-                "peak_source": "dense TF32 rate of a library GEMM measured in this run (torch.matmul / cuBLAS, TF32 allowed, "
-                               "8192^3, best of 10; outside the product); %s bf16_tflops (burst) / 2 would be %.1f" % (
-                                   src, pk["bf16_tflops"] / 2.0),
-                "peak_bf16_half": pk["bf16_tflops"] / 2.0, "frac_of_bf16_half": ach / (pk["bf16_tflops"] / 2.0),
-                "executed_mma_frac": 3 * ach / tf32_run,
+                "kernel": "thc::mm::tc2r_kernel (persistent two-SM tcgen05 GEMM / implicit GEMM, FP32-accurate as three products of FP16 "
+                          "halves; three TF32 products for small layers)",
+                "peak_source": "%s bf16_tflops (burst, cuBLAS 8192^3): FP16 MMAs run at the same rate; three of them make one FP32-accurate "
+                               "product, so frac cannot exceed a third" % src,
+                "executed_mma_frac": 3 * ach / pk["bf16_tflops"],
+                "tf32_yardstick": tf32_run, "frac_of_tf32_yardstick": ach / tf32_run,
                 "conv_fwd_bwd_tflops": conv_f / conv_t / 1e12, "gemm_time_share_of_step": tot_t / (ms * 1e-3 / args.steps)}
 
     # the opt-in BF16 math mode, reported separately: the same step with every GEMM-shaped op on BF16 tensor
