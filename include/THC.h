@@ -104,6 +104,9 @@ THC_API long THGPUGetWaitLimit(void);
 THC_API int THGPUStallProbe(long limit_cycles);
 /* Count of kernels this library has launched on the calling thread since start. */
 THC_API long THGPUKernelLaunchCount(void);
+/* Count of products among them that ran on the two-SM tensor-core engine, by the form of their operands: 0 FP32 values, 1 BF16,
+ * 2 pairs of FP16 halves. */
+THC_API long THGPUProductCount(int form);
 /* Count of stream-ordered device allocations the library has requested from the driver on the calling thread
  * (storages, and growth of the workspace arena that holds the temporaries of the entry points). */
 THC_API long THGPUDeviceAllocCount(void);

@@ -285,6 +285,7 @@ static void launch_raw(P p, Attach attach) {
   // a long launch gains nothing from starting early, and measured 1.5 % slower when it did (4096^3: 671 -> 682 us)
   const bool early = tc2_product_us(p.M, p.N, p.K, P::PREC, P::OpB::MN_MAJOR) < 100;
   with_width([&](auto w) { launch_tc2r_kernel<P, decltype(w)::value>(p, items, early); });
+  ctx().products[P::PREC]++;
   if (p.ws) {
     // a few thousand blocks whatever the number of tail tiles: a lone tile cut into many slices gets a block per column
     const bool four = tail * (bn2 / 4) >= 2l * ctx().sm_count;

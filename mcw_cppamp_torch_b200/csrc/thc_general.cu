@@ -330,3 +330,4 @@ THC_API void THGPUBlas_setMathMode(int mode) {
 THC_API int THGPUBlas_getMathMode(void) { THC_BEGIN return ctx().math_mode; THC_END(-1) }
 THC_API long THGPUKernelLaunchCount(void) { return g_ctx.launches; }
 THC_API long THGPUDeviceAllocCount(void) { return g_ctx.allocs; }
+THC_API long THGPUProductCount(int form) { return form >= 0 && form < 3 ? g_ctx.products[form] : 0; }

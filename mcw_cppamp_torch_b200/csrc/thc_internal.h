@@ -60,6 +60,7 @@ struct Context {
   int sm_count = 0;
   int math_mode = 0;          // 0 fp32x3, 1 simt, 2 bf16
   long launches = 0;
+  long products[3] = {};      // launches of the two-SM engine by mm::kTf32, kBf16, kPairs
   // small device scratch reused by reductions and the GEMM error flag (lazy, per device)
   void *scratch = nullptr;
   size_t scratch_bytes = 0;

@@ -15,6 +15,11 @@ def gt():
     return gt
 
 
+def products(gt):
+    """Products so far over FP32 values and over pairs."""
+    return [gt.lib().THGPUProductCount(form) for form in (0, 2)]
+
+
 def randn(seed, *shape):
     g = torch.Generator(device="cuda")
     g.manual_seed(seed)
@@ -31,24 +36,26 @@ def wide_rows(t, dim, span):
     return t * s.view(shape)
 
 
-def addmm(gt, a, b, c, t1, t2, beta):
+def addmm(gt, a, b, c, t1, t2, beta, pairs=True):
     A, B, C = (gt.gpu(x.cpu().numpy()) for x in (a.t().contiguous() if t1 else a, b.t().contiguous() if t2 else b, c))
+    before = products(gt)
     C.addmm(beta, 1.0, A.t() if t1 else A, B.t() if t2 else B)
+    assert [n - b for n, b in zip(products(gt), before)] == ([0, 1] if pairs else [1, 0])
     return torch.from_numpy(C.float()).cuda().double()
 
 
-def check_addmm(gt, a, b, t1=False, t2=False, beta=0.0, rows=slice(None), cols=slice(None)):
+def check_addmm(gt, a, b, t1=False, t2=False, beta=0.0, rows=slice(None), cols=slice(None), pairs=True):
     c = randn(9, a.size(0), b.size(1))
-    got = addmm(gt, a, b, c, t1, t2, beta)[rows, cols]
+    got = addmm(gt, a, b, c, t1, t2, beta, pairs)[rows, cols]
     a, b, c = a[rows].double(), b[:, cols].double(), beta * c[rows, cols].double()
     assert torch.all((got - (a @ b + c)).abs() <= REL * (a.abs() @ b.abs() + c.abs()))
 
 
 @pytest.mark.parametrize("t1,t2", [(False, False), (False, True), (True, False), (True, True)])
 @pytest.mark.parametrize("m,n,k,beta", [(1500, 3001, 2222, 0.0), (2049, 1793, 2047, 1.0), (4097, 129, 4095, 0.0), (130, 4100, 4033, 1.0),
-                                        (2048, 2048, 2048, 0.0)])
+                                        (2048, 2048, 2048, 0.0), (2048, 2048, 2048, 1.0), (1500, 3001, 2222, 0.5), (4097, 1025, 4033, 1.0)])
 def test_layouts_and_remainders(gt, m, n, k, beta, t1, t2):
-    check_addmm(gt, randn(m, m, k), randn(n, k, n), t1, t2, beta)
+    check_addmm(gt, randn(m, m, k), randn(n, k, n), t1, t2, beta, pairs=(m, n) not in [(2049, 1793), (130, 4100)])
 
 
 @pytest.mark.parametrize("t1,t2", [(False, False), (True, True)])
@@ -81,19 +88,25 @@ def test_zeros_and_extreme_scales(gt):
         check_addmm(gt, a * 2.0 ** e, b * 2.0 ** -max(min(e, 60), -100))
 
 
-CONVS = [  # N, C, H, W, K, k, stride, pad
-    (32, 64, 56, 55, 64, 3, 1, 1),        # pixel pairs
-    (20, 100, 41, 37, 130, 3, 1, 1),      # channels padded to whole spans
-    (64, 3, 99, 101, 64, 11, 4, 2),       # cells
-    (24, 64, 31, 33, 192, 5, 1, 2),
-    (24, 128, 29, 29, 256, 3, 2, 1),      # strided windows, folded gradInput
+# N, C, H, W, K, k, stride, pad; how many products of forward, backward and a second accGradParameters run over FP32 values, and over pairs
+CONVS = [
+    ((32, 64, 56, 55, 64, 3, 1, 1), [0, 4]),       # pixel pairs
+    ((20, 100, 41, 37, 130, 3, 1, 1), [0, 4]),     # channels padded to whole spans
+    ((64, 3, 99, 101, 64, 11, 4, 2), [4, 0]),      # cells, too small for pairs
+    ((64, 3, 224, 224, 64, 11, 4, 2), [0, 4]),     # cells, rows staged in shared memory
+    ((21, 4, 211, 1903, 64, 11, 4, 2), [0, 4]),    # cells of rows that shared memory does not hold
+    ((64, 12, 131, 133, 64, 8, 4, 2), [0, 4]),     # cells whose chunks do not divide a block
+    ((24, 64, 31, 33, 192, 5, 1, 2), [0, 4]),
+    ((24, 128, 29, 29, 256, 3, 2, 1), [4, 0]),     # strided windows, folded gradInput
+    ((96, 128, 29, 29, 256, 3, 2, 1), [0, 4]),
+    ((4, 3, 500, 1000, 8, 11, 1, 5), [0, 4]),      # gradInput as a layer of its own
 ]
 
 
 @pytest.mark.parametrize("wide", ["", "input", "weight", "gradOutput", "inf"])
 @pytest.mark.parametrize("case", CONVS)
 def test_convolution(gt, case, wide):
-    N, C, H, W, K, k, stride, pad = case
+    (N, C, H, W, K, k, stride, pad), expected = case
     x, w, b = randn(1, N, C, H, W), randn(2, K, C, k, k) / (C * k * k) ** 0.5, randn(3, K)
     go = randn(4, N, K, (H + 2 * pad - k) // stride + 1, (W + 2 * pad - k) // stride + 1)
     x, w, go = (wide_rows(t, 0, 45) if wide == name else t for t, name in ((x, "input"), (w, "weight"), (go, "gradOutput")))
@@ -105,11 +118,13 @@ def test_convolution(gt, case, wide):
     m.gpu()
     xg, gog = gt.gpu(x.cpu().numpy()), gt.gpu(go.cpu().numpy())
     m.zeroGradParameters()
+    before = products(gt)
     out = torch.from_numpy(m.forward(xg).float()).cuda().double()
     gi = torch.from_numpy(m.backward(xg, gog).float()).cuda().double()
     gw = torch.from_numpy(m.gradWeight.float()).cuda().double().view_as(w)
     m.accGradParameters(xg, gog)            # the planes once more, whichever form they are in by now
     twice = torch.from_numpy(m.gradWeight.float()).cuda().double().view_as(w)
+    assert [n - b for n, b in zip(products(gt), before)] == expected
 
     def conv(x, w, b, go):
         x, w = x.double().requires_grad_(), w.double().requires_grad_()
