@@ -303,18 +303,18 @@ static void conv_forward_tc(const ConvGeom &g, const mm::Cells &u, const float *
   const double bytes = (double)mm::planes_bytes(1, (long)u.Hs * u.Ws, u.Cs, PREC), floats = (double)g.N * g.C * g.H * g.W;
   if (finput && bytes * (double)g.N > whole_scratch(floats)) { forget_planes(finput); finput = nullptr; }
   const long per = finput ? g.N : images_per_group(g.N, bytes, kGroupScratch);
-  Records rec;
-  if constexpr (PREC == mm::kPairs) {
-    mm::RangeRec *rx = mm::new_range_rec(), *rw = mm::new_range_rec();
-    const mm::RangeJob jw = mm::range_job_flat(w, g.K * g.R, rw);
-    mm::launch_ranges(mm::range_job_flat(in, g.N * g.C * g.H * g.W, rx), &jw);
-    rec.act = rx; rec.weight = rw;
-  }
   for (long n0 = 0; n0 < g.N; n0 += per) {
     WsScope ws_scope;
     ConvGeom s = g;
     s.N = std::min(per, g.N - n0);
     const float *x = in + n0 * g.C * g.H * g.W;
+    Records rec;
+    if constexpr (PREC == mm::kPairs) {   // (for each group: records last for some thousand words, see zeroed_words)
+      mm::RangeRec *rx = mm::new_range_rec(), *rw = mm::new_range_rec();
+      const mm::RangeJob jw = mm::range_job_flat(w, g.K * g.R, rw);
+      mm::launch_ranges(mm::range_job_flat(x, s.N * g.C * g.H * g.W, rx), &jw);
+      rec.act = rx; rec.weight = rw;
+    }
     mm::PairForm form;
     form.ranges = rec.joint(rec.act);
     void *act = finput ? planes_in(finput, s, u, x, PREC) : nullptr;
@@ -628,13 +628,6 @@ template <int PREC>
 static void conv_backward_group(const ConvGeom &g, const mm::Cells &u, bool in_ok, bool w_ok, const float *in, const void *act, const float *gout,
                                 const float *w, float *gin, float *gw, float *gb, float scale, const Records &rec) {
   WsScope ws_scope;
-  ConvGeom t;
-  mm::Cells ut;
-  if (gin && grad_input_layer(g, PREC, t, ut)) {
-    conv_forward_tc<PREC>(t, ut, gout, transposed_weight(g, w, true), nullptr, gin, nullptr);
-    gin = nullptr;
-    in_ok = false;
-  }
   mm::ActPlanes pgo;
   mm::PairForm form;
   form.ranges = rec.joint(rec.gout);
@@ -669,26 +662,6 @@ static void conv_backward_tc(const ConvGeom &g, const mm::Cells &u, bool restate
   // mcw_nn/generic/SpatialConvolutionMM.c:284-346), else made group by group
   const char *act = w_ok ? (const char *)planes_made_from(finput, in, g, u, PREC) : nullptr;
   const size_t act_image = w_ok ? mm::planes_bytes(1, (long)u.Hs * u.Ws, u.Cs, PREC) : 0;
-  Records rec;
-  if constexpr (PREC == mm::kPairs) {
-    const long image = g.C * g.H * g.W;
-    mm::RangeRec *rg = mm::new_range_rec(), *rw = in_ok ? mm::new_range_rec() : nullptr;
-    const mm::RangeJob jg = mm::range_job_flat(gout, g.N * g.K * g.P, rg), jw = mm::range_job_flat(w, g.K * g.R, rw);
-    mm::launch_ranges(jg, rw ? &jw : nullptr);
-    rec.gout = rg; rec.weight = rw;
-    if (act) {
-      mm::RangeRec *kept = planes_record(act);
-      rec.act = kept;
-      mm::PairForm form;
-      form.ranges = rec.joint(kept);
-      form.remake = kept;
-      restate_input<PREC>(g, u, in, (void *)act, form);
-    } else if (w_ok) {
-      mm::RangeRec *rx = mm::new_range_rec();
-      mm::launch_ranges(mm::range_job_flat(in, g.N * image, rx), nullptr);
-      rec.act = rx;
-    }
-  }
   double bytes = 0;
   if (in_ok || w_ok) bytes += (double)mm::planes_bytes(1, g.P, mm::padded_channels(g.K, PREC), PREC);
   if (in_ok && !ui.direct) bytes += 4. * ui.Cr * ui.Hs * ui.Ws;
@@ -697,8 +670,38 @@ static void conv_backward_tc(const ConvGeom &g, const mm::Cells &u, bool restate
   for (long n0 = 0; n0 < g.N; n0 += per) {
     ConvGeom s = g;
     s.N = std::min(per, g.N - n0);
-    conv_backward_group<PREC>(s, u, in_ok, w_ok, in ? in + n0 * image : nullptr, act ? act + n0 * act_image : nullptr, gout + n0 * g.K * g.P, w,
-                              gin ? gin + n0 * image : nullptr, gw, gb, scale, rec);
+    const float *x = in ? in + n0 * image : nullptr, *go = gout + n0 * g.K * g.P;
+    float *gi = gin ? gin + n0 * image : nullptr;
+    ConvGeom t;
+    mm::Cells ut;
+    const bool layer = gin && grad_input_layer(s, PREC, t, ut), own = gin && !layer, own_ok = own && in_ok;
+    if (own || gw) {
+      WsScope ws_scope;
+      Records rec;
+      if constexpr (PREC == mm::kPairs) {   // (for each group: records last for some thousand words, see zeroed_words)
+        mm::RangeRec *rg = mm::new_range_rec(), *rw = own_ok ? mm::new_range_rec() : nullptr;
+        const mm::RangeJob jg = mm::range_job_flat(go, s.N * g.K * g.P, rg), jw = mm::range_job_flat(w, g.K * g.R, rw);
+        mm::launch_ranges(jg, rw ? &jw : nullptr);
+        rec.gout = rg; rec.weight = rw;
+        if (act) {
+          mm::RangeRec *kept = planes_record(act);
+          rec.act = kept;
+          mm::PairForm form;
+          form.ranges = rec.joint(kept);
+          form.remake = kept;
+          restate_input<PREC>(g, u, in, (void *)act, form);
+        } else if (w_ok) {
+          mm::RangeRec *rx = mm::new_range_rec();
+          mm::launch_ranges(mm::range_job_flat(x, s.N * image, rx), nullptr);
+          rec.act = rx;
+        }
+      }
+      conv_backward_group<PREC>(s, u, own_ok, w_ok, x, act ? act + n0 * act_image : nullptr, go, w, own ? gi : nullptr, gw, gb, scale, rec);
+    }
+    if (layer) {   // last: its own groups use up words
+      WsScope ws_scope;
+      conv_forward_tc<PREC>(t, ut, go, transposed_weight(s, w, true), nullptr, gi, nullptr);
+    }
   }
 }
 static void conv_backward(const ConvGeom &g, const float *in, const float *gout, const float *w, float *gin, float *gw, float *gb, float scale,

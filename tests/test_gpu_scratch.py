@@ -1,0 +1,49 @@
+"""Device memory behind the products: records over many groups of images."""
+import pytest
+import torch
+
+from test_gpu_fp16_pairs import REL, gt, products, randn  # noqa: F401
+
+pytestmark = pytest.mark.gpu
+
+
+def wrap(gt, t):  # noqa: F811
+    """A torch.GPUTensor over a torch tensor's memory."""
+    L = gt.lib()
+    s = L.THGPUStorage_newWithData(t.data_ptr(), t.numel())
+    g = gt.GPUTensor(_ptr=L.THGPUTensor_newWithStorage1d(s, 0, t.numel(), 1)).view(*t.shape)
+    L.THGPUStorage_free(s)
+    return g
+
+
+def test_hundreds_of_groups(gt):  # noqa: F811
+    """A batch whose planes come to 350 groups of one image: an image's gradients are the same, bit for bit, wherever it stands."""
+    N, C, H, K, k = 350, 3, 1400, 1, 11
+    image, gout, w = randn(0, C, H, H), randn(1, K, H, H), randn(5, K, C, k, k)
+    x, go = torch.zeros(N, C, H, H, device="cuda"), torch.zeros(N, K, H, H, device="cuda")
+    m = gt.nn.SpatialConvolutionMM(C, K, k, k, 1, 1, k // 2)
+    m.weight.reshape(-1)[:] = w.cpu().numpy().reshape(-1)
+    m.gpu()
+    gi = torch.empty_like(x)
+    torch.cuda.synchronize()
+    m.gradInput = wrap(gt, gi)
+    X, GO = wrap(gt, x), wrap(gt, go)
+    got = []
+    for i in (0, N - 5):
+        x[i], go[i] = image, gout
+        torch.cuda.synchronize()
+        m.zeroGradParameters()
+        before = products(gt)
+        m.backward(X, GO)
+        gt.synchronize()
+        assert products(gt)[1] - before[1] == 2 * N
+        got.append((gi[i].clone(), torch.from_numpy(m.gradWeight.float())))
+        x[i], go[i] = 0, 0
+    assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1])
+
+    def grads(f):
+        xi, wi = f(image)[None].double().requires_grad_(), f(w).double().requires_grad_()
+        return torch.autograd.grad(torch.nn.functional.conv2d(xi, wi, None, 1, k // 2), (xi, wi), f(gout)[None].double())
+    (a, b), (am, bm) = grads(lambda t: t), grads(torch.abs)
+    assert torch.all((got[0][0].double() - a[0]).abs() <= REL * am[0])
+    assert torch.all((got[0][1].cuda().double().view_as(w) - b).abs() <= (REL + 2.0 ** -24 * (H * H / 32 + 64)) * bm)
