@@ -104,8 +104,20 @@ unsigned *zeroed_words(int n) {
   Context &c = ctx();
   constexpr int kBlock = 4096;
   if (!c.sched_counters) {
-    THC_CUDA(cudaMalloc((void **)&c.sched_counters, sizeof(unsigned) * 2 * kBlock));
+    THC_CUDA(cudaMalloc((void **)&c.sched_counters, sizeof(unsigned) * 3 * kBlock));
     c.sched_next = kBlock;
+  }
+  // A recorded launch runs many times over, whenever its recording does: its words are cleared each time, and come from a block
+  // of their own, so that no launch outside takes words for clear that a recording has written.
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(c.stream, &capture) != cudaSuccess) cudaGetLastError();
+  if (capture == cudaStreamCaptureStatusActive) {
+    if (n > 1) c.sched_recorded = (c.sched_recorded + 7) & ~7;
+    if (c.sched_recorded + n > kBlock) c.sched_recorded = 0;
+    unsigned *p = c.sched_counters + 2 * kBlock + c.sched_recorded;
+    c.sched_recorded += n;
+    THC_CUDA(cudaMemsetAsync(p, 0, sizeof(unsigned) * n, c.stream));
+    return p;
   }
   if (c.sched_stream != c.stream) {
     // the caller moved to another stream: launches of the old one may still be reading their counters
@@ -121,10 +133,6 @@ unsigned *zeroed_words(int n) {
   }
   unsigned *p = c.sched_counters + c.sched_block * kBlock + c.sched_next;
   c.sched_next += n;
-  // a recorded launch runs many times over: its words are cleared each time
-  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-  if (cudaStreamIsCapturing(c.stream, &capture) == cudaSuccess && capture == cudaStreamCaptureStatusActive)
-    THC_CUDA(cudaMemsetAsync(p, 0, sizeof(unsigned) * n, c.stream));
   return p;
 }
 unsigned *sched_counter() { return zeroed_words(1); }

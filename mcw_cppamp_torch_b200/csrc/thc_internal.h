@@ -84,7 +84,7 @@ struct Context {
   long allocs = 0;               // stream-ordered allocations requested from the driver (storages + arena growth)
   // item counters of the persistent matrix-multiply launches (see sched_counter)
   unsigned *sched_counters = nullptr;
-  int sched_next = 0, sched_block = 0;
+  int sched_next = 0, sched_block = 0, sched_recorded = 0;
   cudaStream_t sched_stream = nullptr;
   void *plane_records = nullptr;   // see plane_records()
   long plane_epoch = 0;            // bumped whenever they are given back
@@ -112,7 +112,8 @@ __device__ __forceinline__ void scalar_deliver(ScalarSlot *slot, double v, unsig
 mm::StallCtl stall_ctl();         // kernel parameter of the tensor-core kernels
 // A zeroed device word for one persistent launch to hand out its work items from.  The words come from two blocks of
 // 4096; when one has been used up the other is cleared on the stream and takes over (the launches that used it are ahead of
-// the clearing in the same stream).
+// the clearing in the same stream).  Launches that are being recorded take theirs from a third block, where each is cleared
+// by a node of the recording.  (Two recordings share it, as they share the workspace arena: they run one after the other.)
 unsigned *sched_counter();
 // The same for other uses inside one entry point, `n` words side by side on a 32-byte boundary; they keep their values until
 // some thousand further words have been handed out.

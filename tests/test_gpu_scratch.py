@@ -1,4 +1,6 @@
-"""Device memory behind the products: records over many groups of images."""
+"""Device memory behind the products: zeroed words inside recordings, records over many groups of images."""
+import ctypes
+
 import pytest
 import torch
 
@@ -14,6 +16,54 @@ def wrap(gt, t):  # noqa: F811
     g = gt.GPUTensor(_ptr=L.THGPUTensor_newWithStorage1d(s, 0, t.numel(), 1)).view(*t.shape)
     L.THGPUStorage_free(s)
     return g
+
+
+def test_recorded_products(gt):  # noqa: F811
+    """Enough products in a recording to use up the zeroed words several times over; launches outside it come before, between and after its runs."""
+    n, k = 3072, 2048                     # (more tiles than clusters: items are handed out)
+    a, b = [randn(i, n, k) * 2.0 ** (15 * i) for i in range(3)], [randn(i, k, n) * 2.0 ** (-15 * i) for i in range(3)]
+    want = [x.double() @ y.double() for x, y in zip(a, b)]
+    mass = [x.abs().double() @ y.abs().double() for x, y in zip(a, b)]
+    out = [torch.empty(n, n, device="cuda") for _ in a]
+    torch.cuda.synchronize()
+    stream = torch.cuda.Stream()
+    gt.lib().THGPUSetStream(ctypes.c_void_p(stream.cuda_stream))
+    try:
+        A, B, C = ([wrap(gt, t) for t in ts] for ts in (a, b, out))
+
+        def run(times):
+            for _ in range(times):
+                for x, y, z in zip(A, B, C):
+                    z.addmm(0.0, 1.0, x, y)
+
+        def check():
+            gt.synchronize()
+            for c, w, m in zip(out, want, mass):
+                assert torch.all((c.double() - w).abs() <= REL * m)
+                c.fill_(float("nan"))
+            torch.cuda.synchronize()
+
+        before = products(gt)
+        run(200)                          # every word has been used
+        assert products(gt)[1] - before[1] == 600
+        check()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=stream):
+            run(130)
+        torch.cuda.synchronize()
+        for _ in range(200):              # each result is looked at: a launch that missed its words leaves tiles out
+            run(1)
+            check()
+        with torch.cuda.stream(stream):
+            for _ in range(3):
+                graph.replay()
+                check()
+                run(7)
+                check()
+        del graph
+    finally:
+        gt.synchronize()
+        gt.lib().THGPUSetStream(None)
 
 
 def test_hundreds_of_groups(gt):  # noqa: F811
