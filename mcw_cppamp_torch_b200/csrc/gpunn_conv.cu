@@ -50,7 +50,7 @@ static ConvGeom conv_geom(const THGPUTensor *input, const THGPUTensor *weight, i
 // that does not write `finput` forgets the entry, so planes of an earlier pass are never taken for fresh ones.
 // Keyed by the address of finput's data; one table per host thread, as the rest of the library's state.
 namespace {
-// Pairs have a record (mm::RangeRec), `record` of the context's plane_records; the slots belong to the entries of this table.
+// Pairs have a record (mm::KeptRange), `record` of the context's (plane_record); the slots belong to the entries of this table.
 struct PlaneStamp { const float *input; int prec; long N, C, H, W, K; int kH, kW, dH, dW, pad; int record; long epoch; };
 thread_local std::unordered_map<const float *, PlaneStamp> g_plane_stamps;
 thread_local std::vector<int> g_free_records;   // of the slots below g_records
@@ -73,9 +73,7 @@ void forget_planes(const THGPUTensor *finput) {
   g_plane_stamps.erase(it);
 }
 // The record of planes that are known to be fresh.
-mm::RangeRec *planes_record(const void *planes) {
-  return (mm::RangeRec *)plane_records() + g_plane_stamps.at((const float *)planes).record;
-}
+mm::KeptRange *planes_record(const void *planes) { return (mm::KeptRange *)plane_record(g_plane_stamps.at((const float *)planes).record); }
 }  // namespace
 
 // ------------------------------------------------------------------------------------------------
@@ -189,19 +187,31 @@ static mm::Cells grad_input_cells(const ConvGeom &g, int prec) {
   return g.dH == 1 && g.dW == 1 ? direct_cells(g, prec) : cells_of(g, false, false, prec);
 }
 
-// kPairs: the records of the tensors that a call's products read, whose form is decided together (mm::RangeRec).
+// kPairs: the measures of the tensors that a call's products read, whose form is decided together (mm::RangeRec).
 struct Records {
-  const mm::RangeRec *act = nullptr, *weight = nullptr, *gout = nullptr;
+  mm::Measured act, weight, gout;
   // `own` first, then the others
-  mm::Ranges joint(const mm::RangeRec *own) const {
+  mm::Ranges joint(const mm::Measured &own) const {
     mm::Ranges r;
     int n = 0;
-    r.rec[n++] = own;
-    for (const mm::RangeRec *x : {act, weight, gout})
-      if (x != own) r.rec[n++] = x;
+    r.rec[n++] = own.rec;
+    for (const mm::RangeRec *x : {act.rec, weight.rec, gout.rec})
+      if (x != own.rec) r.rec[n++] = x;
     return r;
   }
 };
+static mm::LayerShape layer_shape(const ConvGeom &g) {
+  return mm::LayerShape{g.N, (int)g.C, (int)g.H, (int)g.W, (int)g.K, (int)g.oH, (int)g.oW, g.kH, g.kW, g.dH, g.dW, g.pad};
+}
+// What the strays of a forward product's (GRAD_INPUT: a gradInput product's) operands add to its result.
+template <bool GRAD_INPUT>
+static void add_strays(const ConvGeom &g, const float *src, const float *w, float *out, const Records &rec) {
+  const long planes = GRAD_INPUT ? g.C : g.K;
+  const dim3 grid((unsigned)std::min(g.N, 37l), (unsigned)std::min(planes, 8l));
+  pdl_launch(mm::window_strays_kernel<GRAD_INPUT>, grid, 256, 0, src, w, out, layer_shape(g), GRAD_INPUT ? rec.gout : rec.act, rec.weight,
+             rec.joint(rec.weight));
+  check_launch("window_strays");
+}
 
 // out[n, r, y, x] = bias[r] + the product of the windows `v` over `act` with rows r < rows of the repacked weights
 template <int PREC, bool FLIP, bool PAIR>
@@ -216,7 +226,7 @@ static void window_product_t(const void *act, const mm::Windows &full, const mm:
   pdl_launch(repack_weight_kernel<PREC, FLIP>, (unsigned)blocks, 256, 0, w, u, (int)K, (int)rows, (int)v.C, PAIR ? full.dW : 0, wp, rec.joint(rec.weight));
   check_launch("repack_weight");
   Problem<PlanesWindowOperand<PREC>, RawOperand<false, PREC>, PAIR, PREC> p;
-  p.range_a = rec.act; p.range_b = rec.weight; p.ranges = rec.joint(rec.act);
+  p.range_a = rec.act.rec; p.range_b = rec.weight.rec; p.ranges = rec.joint(rec.act);
   attach_window_map<PREC>(p.a, act, v);
   const long P = full.oH * full.oW;
   p.epi = Epilogue{out, bias, 1.f, 0.f, P, rows * P, P};
@@ -253,21 +263,20 @@ static void restate_input(const ConvGeom &g, const mm::Cells &u, const float *in
     }
   }
   // a block per row of cells; a row is shared by several blocks where the rows of few images leave SMs idle (one
-  // 224 x 224 image: 8.4 us with one block each).  Planes that are hardly ever made again get few blocks to find that out.
+  // 224 x 224 image: 8.4 us with one block each)
   const long rows = g.N * u.Hs, chunks = (long)u.Ws * u.Cs / (PREC != mm::kTf32 ? 8 : 4);
-  const unsigned bx = (unsigned)(form.remake ? std::min(rows, 4l * ctx().sm_count) : rows);
   const unsigned parts = (unsigned)std::max(1l, std::min((chunks + 255) / 256, 4l * ctx().sm_count / rows));
   if constexpr (PREC != mm::kBf16) {
     const int q = u.Cs / (PREC == mm::kPairs ? 8 : 4);
     const long Wp = (long)(u.Ws - 1) * u.dW + u.eW, ld = (Wp + 15) / 32 * 32 + 16, smem = 4l * u.C * u.eH * ld;
     if (256 % q == 0 && smem <= 40 * 1024 && rows >= 2l * ctx().sm_count) {
-      pdl_launch(mm::cells_staged_kernel<PREC>, (unsigned)std::min(bx, 16u * ctx().sm_count), 256, smem, in, dst, g.N, u, (int)Wp, (int)ld, form);
+      pdl_launch(mm::cells_staged_kernel<PREC>, (unsigned)std::min(rows, 16l * ctx().sm_count), 256, smem, in, dst, g.N, u, (int)Wp, (int)ld, form);
       check_launch("cells_staged");
       return;
     }
   }
-  if (u.Cs <= mm::kCellTable) pdl_launch(mm::cells_input_kernel<PREC, true>, dim3(bx, parts), 256, sizeof(int2) * u.Cs, in, dst, g.N, u, form);
-  else pdl_launch(mm::cells_input_kernel<PREC, false>, dim3(bx, parts), 256, 0, in, dst, g.N, u, form);
+  if (u.Cs <= mm::kCellTable) pdl_launch(mm::cells_input_kernel<PREC, true>, dim3((unsigned)rows, parts), 256, sizeof(int2) * u.Cs, in, dst, g.N, u, form);
+  else pdl_launch(mm::cells_input_kernel<PREC, false>, dim3((unsigned)rows, parts), 256, 0, in, dst, g.N, u, form);
   check_launch("cells_input");
 }
 
@@ -310,18 +319,18 @@ static void conv_forward_tc(const ConvGeom &g, const mm::Cells &u, const float *
     const float *x = in + n0 * g.C * g.H * g.W;
     Records rec;
     if constexpr (PREC == mm::kPairs) {   // (for each group: records last for some thousand words, see zeroed_words)
-      mm::RangeRec *rx = mm::new_range_rec(), *rw = mm::new_range_rec();
-      const mm::RangeJob jw = mm::range_job_flat(w, g.K * g.R, rw);
-      mm::launch_ranges(mm::range_job_flat(x, s.N * g.C * g.H * g.W, rx), &jw);
-      rec.act = rx; rec.weight = rw;
+      rec.act = mm::new_measured(); rec.weight = mm::new_measured();
+      mm::RangeJob jw = mm::range_job_flat(w, g.K * g.R, rec.weight);
+      mm::launch_ranges(mm::range_job_flat(x, s.N * g.C * g.H * g.W, rec.act), &jw);
     }
     mm::PairForm form;
     form.ranges = rec.joint(rec.act);
     void *act = finput ? planes_in(finput, s, u, x, PREC) : nullptr;
-    if (act && PREC == mm::kPairs) form.keep = planes_record(act);
+    if (act && PREC == mm::kPairs) { form.keep = planes_record(act); form.list = rec.act.list; }
     if (!act) act = ws_alloc(mm::planes_bytes(s.N, (long)u.Hs * u.Ws, u.Cs, PREC));
     restate_input<PREC>(s, u, x, act, form);
     window_product<PREC, false>(act, forward_windows(s, u), w, u, g.K, g.K, bias, out + n0 * g.K * g.P, rec);
+    if (PREC == mm::kPairs) add_strays<false>(s, x, w, out + n0 * g.K * g.P, rec);
   }
 }
 
@@ -361,8 +370,9 @@ static bool grad_input_layer(const ConvGeom &g, int prec, ConvGeom &t, mm::Cells
 
 // gradInput = forward pass of gradOutput's planes under the filter rotated by 180 degrees with its plane roles swapped.
 template <int PREC>
-static void conv_grad_input_tc(const ConvGeom &g, const mm::ActPlanes &pgo, const float *w, float *gin, Records rec) {
-  rec.act = std::exchange(rec.gout, rec.act);   // the windows run over gradOutput here
+static void conv_grad_input_tc(const ConvGeom &g, const mm::ActPlanes &pgo, const float *w, float *gin, const Records &records) {
+  Records rec = records;
+  std::swap(rec.act, rec.gout);   // the windows run over gradOutput here
   const mm::Cells u = grad_input_cells(g, PREC);
   const mm::Windows v = grad_input_windows(g, u, PREC);
   if (u.direct) { window_product<PREC, true>(pgo.p, v, w, u, g.K, g.C, nullptr, gin, rec); return; }
@@ -389,9 +399,10 @@ static void conv_grad_input_tc(const ConvGeom &g, const mm::ActPlanes &pgo, cons
 //      matrices: the f diagonal blocks of the result are the gradient's partial sums.  The other blocks are computed in
 //      vain, but a k tile costs the same however little of its 256 x 64 tile is used, and there are f times fewer.
 template <int PREC>
-static void conv_acc_grad_tc(const ConvGeom &g, const mm::Cells &u, const void *act, const mm::ActPlanes &pgo, float *gw, float scale,
-                             const Records &rec) {
+static void conv_acc_grad_tc(const ConvGeom &g, const mm::Cells &u, const void *act, const mm::ActPlanes &pgo, const float *gout, long n0, float *gw,
+                             float scale, const Records &rec) {
   using namespace mm;
+  const WgradStrays strays{rec.act, rec.gout, rec.joint(rec.act), n0, act, gout, layer_shape(g)};
   const Windows v = forward_windows(g, u);
   const long Kp = pgo.Cp, Cs = u.Cs, Rp = (long)u.kHs * u.kWs * Cs, pixels = g.N * g.P;
   const long M2 = (long)u.kHs * Cs, N2 = (long)u.kWs * Kp;
@@ -407,7 +418,7 @@ static void conv_acc_grad_tc(const ConvGeom &g, const mm::Cells &u, const void *
     const long Mf = f * Kp, Nf = f * Cs;
     float *T = (float *)ws_alloc(sizeof(float) * Mf * Nf);
     Problem<RawOperand<true, PREC>, RawOperand<true, PREC>, false, PREC> p;
-    p.range_a = rec.gout; p.range_b = rec.act; p.ranges = rec.joint(rec.act);
+    p.range_a = rec.gout.rec; p.range_b = rec.act.rec; p.ranges = rec.joint(rec.act);
     p.epi = Epilogue{T, nullptr, 1.f, 0.f, 1, Nf, 1};                 // T[m * Nf + n]
     p.M = Mf; p.N = Nf; p.K = pixels / f;
     launch_raw(p, [&](auto &q, int bn2) {
@@ -416,7 +427,7 @@ static void conv_acc_grad_tc(const ConvGeom &g, const mm::Cells &u, const void *
     });
     const WgradPlace pl{Nf, 1, 0, 0, 0, (int)f, Kp * Nf + Cs};
     const long total = g.K * g.R;
-    pdl_launch(unpack_grad_weight_kernel, (unsigned)std::min<long>((total + 255) / 256, ctx().sm_count * 8l), 256, 0, T, gw, u, (int)g.K, pl, scale);
+    pdl_launch(unpack_grad_weight_kernel<PREC == kPairs>, (unsigned)std::min<long>((total + 255) / 256, ctx().sm_count * 8l), 256, 0, T, gw, u, (int)g.K, pl, scale, strays);
     check_launch("unpack_grad_weight");
     return;
   }
@@ -425,7 +436,7 @@ static void conv_acc_grad_tc(const ConvGeom &g, const mm::Cells &u, const void *
   WgradPlace pl;
   if (way == 0) {
     Problem<RawOperand<true, PREC>, WindowRowsOperand<PREC>, false, PREC> p;
-    p.range_a = rec.gout; p.range_b = rec.act; p.ranges = rec.joint(rec.act);
+    p.range_a = rec.gout.rec; p.range_b = rec.act.rec; p.ranges = rec.joint(rec.act);
     attach_window_rows_map<PREC>(p.b, act, v);
     p.epi = Epilogue{T, nullptr, 1.f, 0.f, 1, Rp, 1};                 // T[m * Rp + n]
     p.M = g.K; p.N = Rp; p.K = pixels;
@@ -433,7 +444,7 @@ static void conv_acc_grad_tc(const ConvGeom &g, const mm::Cells &u, const void *
     pl = WgradPlace{Rp, 1, u.kWs * Cs, Cs, 0, 1, 0};
   } else if (way == 1) {
     Problem<WindowRowsOperand<PREC>, RawOperand<true, PREC>, false, PREC> p;
-    p.range_a = rec.act; p.range_b = rec.gout; p.ranges = rec.joint(rec.act);
+    p.range_a = rec.act.rec; p.range_b = rec.gout.rec; p.ranges = rec.joint(rec.act);
     attach_window_rows_map<PREC>(p.a, act, v);
     p.epi = Epilogue{T, nullptr, 1.f, 0.f, LONG_MAX, 0, Rp};          // T[n * Rp + m]
     p.M = Rp; p.N = g.K; p.K = pixels;
@@ -441,7 +452,7 @@ static void conv_acc_grad_tc(const ConvGeom &g, const mm::Cells &u, const void *
     pl = WgradPlace{Rp, 1, u.kWs * Cs, Cs, 0, 1, 0};
   } else {
     Problem<WindowRowsOperand<PREC>, WindowRowsOperand<PREC>, false, PREC> p;
-    p.range_a = rec.act; p.range_b = rec.gout; p.ranges = rec.joint(rec.act);
+    p.range_a = rec.act.rec; p.range_b = rec.gout.rec; p.ranges = rec.joint(rec.act);
     attach_window_rows_map<PREC>(p.a, act, va);
     attach_window_rows_map<PREC>(p.b, pgo.p, vb);
     p.epi = Epilogue{T, nullptr, 1.f, 0.f, 1, N2, 1};                 // T[m * N2 + n]
@@ -450,7 +461,7 @@ static void conv_acc_grad_tc(const ConvGeom &g, const mm::Cells &u, const void *
     pl = WgradPlace{1, N2, Cs * N2, -Kp, (u.kWs - 1) * Kp, 1, 0};
   }
   const long total = g.K * g.R;
-  pdl_launch(unpack_grad_weight_kernel, (unsigned)std::min<long>((total + 255) / 256, ctx().sm_count * 8l), 256, 0, T, gw, u, (int)g.K, pl, scale);
+  pdl_launch(unpack_grad_weight_kernel<PREC == kPairs>, (unsigned)std::min<long>((total + 255) / 256, ctx().sm_count * 8l), 256, 0, T, gw, u, (int)g.K, pl, scale, strays);
   check_launch("unpack_grad_weight");
 }
 
@@ -594,7 +605,7 @@ static bool restate_accurate(const ConvGeom &g, bool pairs, mm::Cells &u, int &p
   const bool ok = restate(g, mm::kTf32, u);
   mm::Cells up;
   if (!ok || !pairs || g.R > 1l << 28 || g.K * g.kH * g.kW > 1l << 28 ||   // (a row of weights and its second half: 31 bits)
-      windows_us(forward_windows(g, u), g.K, prec) < 30 || !restate(g, mm::kPairs, up) ||
+      windows_us(forward_windows(g, u), g.K, prec) < 30 || !restate(g, mm::kPairs, up) || up.Cs > 12288 ||   // (unpair_kernel: 48 KB)
       (up.kHs == 1 && up.kWs == 1 && !up.direct))
     return ok;
   auto us = [&](const mm::Cells &c, int pr) {
@@ -623,17 +634,21 @@ static void conv_forward(const ConvGeom &g, const float *in, const float *w, con
 }
 
 // gradInput (when gin is given) and gradWeight / gradBias (when gw is) of one precision, sharing one transposition of gradOutput.
-// `act`: the input's planes, or null; w_ok / in_ok: whether the weight gradient / gradInput runs over planes.
+// `act`: the input's planes, or null (n0: the image of their record that they start with); w_ok / in_ok: whether the weight gradient / gradInput runs over planes.
 template <int PREC>
 static void conv_backward_group(const ConvGeom &g, const mm::Cells &u, bool in_ok, bool w_ok, const float *in, const void *act, const float *gout,
-                                const float *w, float *gin, float *gw, float *gb, float scale, const Records &rec) {
+                                const float *w, float *gin, float *gw, float *gb, float scale, const Records &rec, long n0) {
   WsScope ws_scope;
   mm::ActPlanes pgo;
   mm::PairForm form;
   form.ranges = rec.joint(rec.gout);
   if (in_ok || w_ok) pgo = mm::make_act_planes<PREC>(gout, g.N, g.K, g.oH, g.oW, nullptr, gw != nullptr, form);
-  if (in_ok) conv_grad_input_tc<PREC>(g, pgo, w, gin, rec);
-  else if (gin) conv_grad_input_simt(g, gout, w, gin);
+  if (in_ok) {
+    conv_grad_input_tc<PREC>(g, pgo, w, gin, rec);
+    if (PREC == mm::kPairs) add_strays<true>(g, gout, w, gin, rec);
+  } else if (gin) {
+    conv_grad_input_simt(g, gout, w, gin);
+  }
   if (!gw) return;
   if (w_ok) {
     if (!act) {
@@ -642,7 +657,7 @@ static void conv_backward_group(const ConvGeom &g, const mm::Cells &u, bool in_o
       restate_input<PREC>(g, u, in, made, form);
       act = made;
     }
-    conv_acc_grad_tc<PREC>(g, u, act, pgo, gw, scale, rec);
+    conv_acc_grad_tc<PREC>(g, u, act, pgo, gout, n0, gw, scale, rec);
   } else {
     conv_acc_grad_simt(g, in, gout, gw, scale);
   }
@@ -679,24 +694,23 @@ static void conv_backward_tc(const ConvGeom &g, const mm::Cells &u, bool restate
       WsScope ws_scope;
       Records rec;
       if constexpr (PREC == mm::kPairs) {   // (for each group: records last for some thousand words, see zeroed_words)
-        mm::RangeRec *rg = mm::new_range_rec(), *rw = own_ok ? mm::new_range_rec() : nullptr;
-        const mm::RangeJob jg = mm::range_job_flat(go, s.N * g.K * g.P, rg), jw = mm::range_job_flat(w, g.K * g.R, rw);
-        mm::launch_ranges(jg, rw ? &jw : nullptr);
-        rec.gout = rg; rec.weight = rw;
+        rec.gout = mm::new_measured();
+        if (own_ok) rec.weight = mm::new_measured();
+        mm::RangeJob jw = mm::range_job_flat(w, g.K * g.R, rec.weight);
+        mm::launch_ranges(mm::range_job_flat(go, s.N * g.K * g.P, rec.gout), own_ok ? &jw : nullptr);
         if (act) {
-          mm::RangeRec *kept = planes_record(act);
-          rec.act = kept;
-          mm::PairForm form;
-          form.ranges = rec.joint(kept);
-          form.remake = kept;
-          restate_input<PREC>(g, u, in, (void *)act, form);
+          mm::KeptRange *kept = planes_record(act);
+          rec.act = mm::Measured{&kept->rec, kept->strays, true};
+          const long pixels = g.N * u.Hs * u.Ws, px = std::max(1, 6144 / u.Cs);
+          pdl_launch(mm::unpair_kernel, (unsigned)std::min((pixels + px - 1) / px, 4l * ctx().sm_count), 256, sizeof(float) * px * u.Cs, (void *)act, pixels, u.Cs,
+                     (int)px, rec.joint(rec.act), &kept->rec);
+          check_launch("unpair");
         } else if (w_ok) {
-          mm::RangeRec *rx = mm::new_range_rec();
-          mm::launch_ranges(mm::range_job_flat(x, s.N * image, rx), nullptr);
-          rec.act = rx;
+          rec.act = mm::new_measured();
+          mm::launch_ranges(mm::range_job_flat(x, s.N * image, rec.act), nullptr);
         }
       }
-      conv_backward_group<PREC>(s, u, own_ok, w_ok, x, act ? act + n0 * act_image : nullptr, go, w, own ? gi : nullptr, gw, gb, scale, rec);
+      conv_backward_group<PREC>(s, u, own_ok, w_ok, x, act ? act + n0 * act_image : nullptr, go, w, own ? gi : nullptr, gw, gb, scale, rec, act ? n0 : 0);
     }
     if (layer) {   // last: its own groups use up words
       WsScope ws_scope;

@@ -8,32 +8,47 @@
 namespace thc {
 namespace mm {
 
+// The halves of scaled values; strays (subnormal hi) leave zeros.
 __device__ __forceinline__ void split_pair(float a, float b, __half2 &hi, __half2 &lo) {
+  a = fabsf(a) < 0x1p-14f ? 0.f : a;
+  b = fabsf(b) < 0x1p-14f ? 0.f : b;
   hi = __floats2half2_rn(a, b);
   const float2 h = __half22float2(hi);
   lo = __floats2half2_rn((a - h.x) * 2048.f, (b - h.y) * 2048.f);
 }
+__device__ __forceinline__ float join_pair(__half hi, __half lo, float unscale) { return (__half2float(hi) + __half2float(lo) * 0x1p-11f) * unscale; }
 __device__ __forceinline__ unsigned half2_bits(const __half2 &h) { return *reinterpret_cast<const unsigned *>(&h); }
 
-// Ranges of up to two operands (blockIdx.y), `lines` x `run` values with pitch ld.  A warp looks at 512 values at a time, in four
-// groups of 128: neighbours in memory (`flat`), or 128 neighbours in each of four lines, so that a small row or column shows in
-// several groups.
-struct RangeJob { const float *p; long lines, run, ld; int flat, vec; RangeRec *rec; };
-static __global__ void __launch_bounds__(256) range_kernel(const RangeJob ja, const RangeJob jb) {
-  pdl_begin();
-  const RangeJob &j = blockIdx.y ? jb : ja;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const long warps = (long)gridDim.x * 8, total = j.lines * j.run;
-  const long segs = j.flat ? (total + 511) / 512 : (j.run + 127) / 128, sets = j.flat ? segs : segs * ((j.lines + 3) / 4);
-  unsigned most = 0, low = ~0u, low2 = ~0u;   // the lows as bits - 1: zero becomes the largest
-  for (long at = (long)blockIdx.x * 8 + warp; at < sets; at += warps) {
-    const long s = sets - 1 - at;   // from the end, which whoever wrote the operand has left in L2, to the start, which the next pass reads first
-    unsigned v[4][4];
+// Ranges of up to two operands (blockIdx.y), `lines` x `run` values with pitch ld.  A warp looks at a set of 512 values at a time, in
+// four groups of 128: neighbours in memory (`flat`), or 128 neighbours in each of four lines.  The last block to finish lists the
+// strays: from the smallest value of each block's sets and of each set (set_low) it knows where to look again, so that
+// the few strays of a large tensor cost it a few microseconds.  The list is in the order of `at`: results do not depend on who came first.
+struct RangeJob {
+  const float *p;
+  long lines, run, ld;
+  int flat, vec;
+  RangeRec *rec;
+  Stray *list;
+  uint2 *block_range;   // a block's largest and smallest
+  unsigned *set_low;
+};
+constexpr int kRangeBlocks = 2048;   // a launch has no more for an operand
+struct RangeSets {
+  const RangeJob &j;
+  long total, segs, count;
+  __device__ __forceinline__ RangeSets(const RangeJob &job) : j(job) {
+    total = j.lines * j.run;
+    segs = j.flat ? (total + 511) / 512 : (j.run + 127) / 128;
+    count = j.flat ? segs : segs * ((j.lines + 3) / 4);
+  }
+  // the 16 values of this lane; at[g]: the place of the first of group g
+  __device__ __forceinline__ void load(long s, int lane, unsigned (&v)[4][4], long (&at)[4]) const {
     const long q = j.flat ? 0 : s / segs, c0 = j.flat ? s * 512 : (s - q * segs) * 128;
 #pragma unroll
     for (int g = 0; g < 4; g++) {
       const long line = j.flat ? 0 : q * 4 + g, c = c0 + (j.flat ? g * 128 : 0) + lane * 4, end = j.flat ? total : line < j.lines ? j.run : 0;
       const float *src = j.p + line * j.ld + c;
+      at[g] = line * j.run + c;
       if (j.vec && c + 4 <= end) {
         const uint4 u = __ldg(reinterpret_cast<const uint4 *>(src));
         v[g][0] = u.x; v[g][1] = u.y; v[g][2] = u.z; v[g][3] = u.w;
@@ -42,59 +57,153 @@ static __global__ void __launch_bounds__(256) range_kernel(const RangeJob ja, co
         for (int i = 0; i < 4; i++) v[g][i] = c + i < end ? __float_as_uint(__ldg(src + i)) : 0u;
       }
     }
-    unsigned a = ~0u, b = ~0u;   // the two smallest groups of this lane
+  }
+};
+static __global__ void __launch_bounds__(256) range_kernel(const RangeJob ja, const RangeJob jb) {
+  pdl_begin();
+  const RangeJob &j = blockIdx.y ? jb : ja;
+  const RangeSets sets(j);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const long warps = (long)gridDim.x * 8, me = (long)blockIdx.x * 8 + warp;
+  unsigned most = 0, low = ~0u;   // the lows as bits - 1: zero becomes the largest
+  for (long k = me; k < sets.count; k += warps) {
+    const long s = sets.count - 1 - k;   // from the end, which whoever wrote the operand has left in L2, to the start, which the next pass reads first
+    unsigned v[4][4], m = ~0u;
+    long at[4];
+    sets.load(s, lane, v, at);
 #pragma unroll
-    for (int g = 0; g < 4; g++) {
-      unsigned m = ~0u;
+    for (int g = 0; g < 4; g++)
 #pragma unroll
       for (int i = 0; i < 4; i++) {
         const unsigned x = v[g][i] & 0x7fffffffu;
         most = max(most, x);
         m = min(m, x - 1u);
       }
-      b = min(b, max(a, m));
-      a = min(a, m);
-    }
-    const unsigned first = __reduce_min_sync(0xffffffffu, a);
-    const int owner = __ffs(__ballot_sync(0xffffffffu, a == first)) - 1;
-    low = min(low, first);
-    low2 = min(low2, __reduce_min_sync(0xffffffffu, lane == owner ? b : a));
+    m = __reduce_min_sync(0xffffffffu, m);
+    if (lane == 0) j.set_low[s] = m;
+    low = min(low, m);
   }
-  __shared__ unsigned sm[3][8];
+  __shared__ unsigned sm[2][8];
+  __shared__ int last, found, nblocks;
+  __shared__ Stray buf[kStrays];
+  __shared__ unsigned short blocks[kRangeBlocks];
   most = __reduce_max_sync(0xffffffffu, most);
-  if (lane == 0) { sm[0][warp] = most; sm[1][warp] = low; sm[2][warp] = low2; }
+  if (lane == 0) { sm[0][warp] = most; sm[1][warp] = low; }
   __syncthreads();
   if (threadIdx.x == 0) {
-    for (int w = 1; w < 8; w++) { most = max(most, sm[0][w]); low = min(low, sm[1][w]); low2 = min(low2, sm[2][w]); }
-    if (most) atomicMax(&j.rec->max_bits, most);
-    if (~low) atomicMax(&j.rec->low_inv, ~low);
-    if (~low2) atomicMax(&j.rec->low2_inv, ~low2);
+    for (int w = 1; w < 8; w++) { most = max(most, sm[0][w]); low = min(low, sm[1][w]); }
+    j.block_range[blockIdx.x] = make_uint2(most, low);
+    __threadfence();
+    last = atomicAdd(&j.rec->ticket, 1u) == gridDim.x - 1;
+    found = nblocks = 0;
   }
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  uint2 r[kRangeBlocks / 256];   // all of them on the way at once
+#pragma unroll
+  for (int i = 0; i < kRangeBlocks / 256; i++) r[i] = i * 256 + threadIdx.x < gridDim.x ? __ldcg(j.block_range + i * 256 + threadIdx.x) : make_uint2(0, ~0u);
+  most = 0;
+#pragma unroll
+  for (int i = 0; i < kRangeBlocks / 256; i++) most = max(most, r[i].x);
+  most = __reduce_max_sync(0xffffffffu, most);
+  if (lane == 0) sm[0][warp] = most;
+  __syncthreads();
+#pragma unroll
+  for (int w = 0; w < 8; w++) most = max(most, sm[0][w]);
+  if (threadIdx.x == 0) j.rec->max_bits = most;
+  const unsigned limit = stray_limit(most) - 1u;   // (as the lows: bits - 1)
+  if (!most || max_is_wide(most)) return;
+#pragma unroll
+  for (int i = 0; i < kRangeBlocks / 256; i++)
+    if (r[i].y < limit) blocks[atomicAdd(&nblocks, 1)] = (unsigned short)(i * 256 + threadIdx.x);
+  __syncthreads();
+  // a warp takes a block's sets, 128 at a time: set q is the block's warp q % 8's in its round q / 8
+  const long rounds = (sets.count + warps - 1) / warps;
+  bool stop = false;   // the same for a warp's lanes, as all that the loops below depend on
+  for (int b = warp; b < nblocks && !stop; b += 8) {
+    const long first = blocks[b] * 8l;
+    for (long q0 = 0; q0 < rounds * 8 && !stop; q0 += 128) {
+      unsigned l[4];
+#pragma unroll
+      for (int i = 0; i < 4; i++) {
+        const long q = q0 + i * 32 + lane, k = q / 8 * warps + first + q % 8;
+        l[i] = k < sets.count ? __ldcg(j.set_low + sets.count - 1 - k) : ~0u;
+      }
+#pragma unroll
+      for (int i = 0; i < 4; i++)
+        for (unsigned hit = __ballot_sync(0xffffffffu, l[i] < limit); hit && !stop; hit &= hit - 1) {
+          const long q = q0 + i * 32 + __ffs(hit) - 1;
+          unsigned v[4][4];
+          long at[4];
+          sets.load(sets.count - 1 - (q / 8 * warps + first + q % 8), lane, v, at);
+#pragma unroll
+          for (int g = 0; g < 4; g++)
+#pragma unroll
+            for (int e = 0; e < 4; e++)
+              if ((v[g][e] & 0x7fffffffu) - 1u < limit) {
+                const int n = atomicAdd(&found, 1);
+                if (n < kStrays) buf[n] = Stray{at[g] + e, __uint_as_float(v[g][e])};
+              }
+          __syncwarp();
+          stop = __shfl_sync(0xffffffffu, *const_cast<volatile int *>(&found), 0) > kStrays;
+        }
+    }
+  }
+  __syncthreads();
+  const int n = found;
+  if (n > kStrays) {
+    if (threadIdx.x == 0) j.rec->wide = 1;
+    return;
+  }
+  for (int i = threadIdx.x; i < n; i += 256) {
+    int rank = 0;
+    for (int o = 0; o < n; o++) rank += buf[o].at < buf[i].at;
+    j.list[rank] = buf[i];
+  }
+  if (threadIdx.x == 0) j.rec->strays = n;
 }
 
 // What a kernel that writes an operand's planes needs in kPairs.
 struct PairForm {
   Ranges ranges;
-  RangeRec *keep = nullptr;     // where the planes' record goes when they outlive the call (their ranges[0] does not)
-  RangeRec *remake = nullptr;   // ranges[0] of kept planes: write only if they are pairs and must be FP32 now
-  // Whether to write anything, and in which form; every thread of the block calls it.
-  __device__ __forceinline__ bool begin(bool &wide) const {
-    wide = ranges.wide();
-    return !remake || (wide && !*const_cast<const volatile unsigned *>(&remake->wide));
-  }
-  // After the block's last look at the records: the last block to get here changes what `begin` looked at.
+  KeptRange *keep = nullptr;     // where the operand's measures go when the planes outlive the call ...
+  const Stray *list = nullptr;   // ... and its list
   __device__ __forceinline__ void end(bool wide) const {
-    if (keep && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) {
-      RangeRec r = *ranges.rec[0];
-      r.wide = wide; r.ticket = 0;
-      *keep = r;
+    if (!keep || blockIdx.x || blockIdx.y) return;
+    const RangeRec r = *ranges.rec[0];
+    const int n = wide ? 0 : (int)r.strays;
+    if (threadIdx.x == 0) {
+      keep->rec = r;
+      keep->rec.wide = wide; keep->rec.ticket = 0; keep->rec.strays = n;
     }
-    if (remake) {
-      __syncthreads();
-      if (threadIdx.x == 0 && atomicAdd(&remake->ticket, 1u) == gridDim.x * gridDim.y - 1) { remake->ticket = 0; remake->wide = 1; }
-    }
+    for (int i = threadIdx.x; i < n; i += blockDim.x) keep->strays[i] = list[i];
   }
 };
+
+// Kept planes back to FP32, in place, where another operand asks for it: 24 bits of almost every value (22 next to the strays, whose
+// places stay zero).  A block takes `px` pixels of Cp channels at a time through shared memory.  Not made from the input again:
+// what the input's memory holds may have changed since the planes were written.
+static __global__ void __launch_bounds__(256) unpair_kernel(void *planes, long pixels, int Cp, int px, const Ranges ranges, RangeRec *kept) {
+  pdl_begin();
+  if (!ranges.wide() || *const_cast<const volatile unsigned *>(&kept->wide)) return;
+  extern __shared__ float4 raw[];
+  const __half *h = reinterpret_cast<const __half *>(raw);
+  const float unscale = pair_unscale(*kept);
+  for (long p0 = (long)blockIdx.x * px; p0 < pixels; p0 += (long)gridDim.x * px) {
+    const int n = (int)min((long)px, pixels - p0) * Cp;
+    float *d = reinterpret_cast<float *>(planes) + p0 * Cp;
+    for (int i = threadIdx.x; i < n / 4; i += 256) raw[i] = reinterpret_cast<const float4 *>(d)[i];
+    __syncthreads();
+    for (int i = threadIdx.x; i < n; i += 256) {
+      const int p = i / Cp, c = i - p * Cp;
+      d[i] = join_pair(h[2 * p * Cp + c], h[(2 * p + 1) * Cp + c], unscale);
+    }
+    __syncthreads();
+  }
+  // every block has looked at the flag before the last one sets it
+  if (threadIdx.x == 0 && atomicAdd(&kept->ticket, 1u) == gridDim.x - 1) { kept->ticket = 0; kept->wide = 1; }
+}
 
 // ---------------------------------------------------------------------------------------------
 // Channels-last planes of an activation tensor, FP32 or BF16, channels padded with zeros to Cp = a multiple of KV.
@@ -167,8 +276,7 @@ static __global__ void __launch_bounds__(256) nchw_to_pairs_kernel(const float *
                                                                    void *__restrict__ dst, float *__restrict__ chan_partial,
                                                                    const PairForm form) {
   pdl_begin();
-  bool wide;
-  if (!form.begin(wide)) return;
+  const bool wide = form.ranges.wide();
   const float scale = wide ? 1.f : pair_scale(*form.ranges.rec[0]);
   constexpr int CT = 64;
   __shared__ float tile[CT][PT + 1];
@@ -357,7 +465,7 @@ static __global__ void __launch_bounds__(256) cells_input_kernel(const float *__
   bool wide = false;
   float scale = 1.f;
   if constexpr (PREC == kPairs) {
-    if (!form.begin(wide)) return;
+    wide = form.ranges.wide();
     if (!wide) scale = pair_scale(*form.ranges.rec[0]);
   }
   extern __shared__ int2 chan_src[];      // per channel: offset in the image, (dy << 16 | dx) or -1
@@ -388,7 +496,7 @@ static __global__ void __launch_bounds__(256) cells_staged_kernel(const float *_
   bool wide = false;
   float scale = 1.f;
   if constexpr (PREC == kPairs) {
-    if (!form.begin(wide)) return;
+    wide = form.ranges.wide();
     if (!wide) scale = pair_scale(*form.ranges.rec[0]);
   }
   constexpr int V = PREC == kPairs ? 8 : 4;
@@ -545,9 +653,53 @@ static __global__ void __launch_bounds__(256) repack_weight_kernel(const float *
 // keeps them (bj counted from the other end when bj_stride is negative: `first` is then the place of tap (0, 0)).
 // `copies` partial sums of each, copy_stride apart.
 struct WgradPlace { long ko_stride, ch_stride, bi_stride, bj_stride, first; int copies; long copy_stride; };
+// The product that the strays of its operands are added to: a layer over N images, [N][C][H][W] -> [N][K][oH][oW].
+struct LayerShape { long N; int C, H, W, K, oH, oW, kH, kW, dH, dW, pad; };
+struct WgradStrays {
+  Measured act, gout;
+  Ranges ranges;
+  long n0;              // image of act's record and list that the planes start with
+  const void *planes;   // of the input (pairs, where gout has strays)
+  const float *go;
+  LayerShape l;
+};
+// One value of restated planes in pairs: input pixel (y, x) of plane c, which some window covers.
+__device__ __forceinline__ float plane_value(const void *planes, const Cells &u, long n, int c, int y, int x, float unscale) {
+  int ch = c;
+  if (!u.direct) {
+    y += u.pad; x += u.pad;
+    const int Y = min(y / u.dH, u.Hs - 1), X = min(x / u.dW, u.Ws - 1);
+    ch += ((y - Y * u.dH) * u.eW + x - X * u.dW) * u.Cq;
+    y = Y; x = X;
+  }
+  const __half *p = reinterpret_cast<const __half *>(planes) + ((n * u.Hs + y) * u.Ws + x) * 2 * u.Cs + ch;
+  return join_pair(p[0], p[u.Cs], unscale);
+}
+struct StrayPlaces { int n[kStrays], c[kStrays], y[kStrays], x[kStrays]; float v[kStrays]; };
+__device__ __forceinline__ void find_strays(StrayPlaces &s, const Stray *list, int count, int C, int H, int W, long n0) {
+  for (int i = threadIdx.x; i < count; i += blockDim.x) {
+    const long at = list[i].at, row = at / W, plane = row / H;
+    s.x[i] = (int)(at - row * W); s.y[i] = (int)(row - plane * H);
+    s.n[i] = (int)(plane / C - n0); s.c[i] = (int)(plane % C);
+    s.v[i] = list[i].v;
+  }
+}
+// kPairs: with the strays of the input against all of gradOutput, and those of gradOutput against what the planes hold of the input.
+template <bool PAIRS>
 static __global__ void __launch_bounds__(256) unpack_grad_weight_kernel(const float *__restrict__ T, float *__restrict__ gw, const Cells u,
-                                                                        int K, const WgradPlace p, float scale) {
+                                                                        int K, const WgradPlace p, float scale, const WgradStrays q) {
   pdl_begin();
+  __shared__ StrayPlaces sa, sg;   // (kPairs)
+  int na = 0, ng = 0;
+  float unscale = 1.f;
+  const LayerShape &l = q.l;
+  if constexpr (PAIRS) {
+    const bool wide = q.ranges.wide();
+    na = q.act.strays(wide); ng = q.gout.strays(wide);
+    if (na) find_strays(sa, q.act.list, na, l.C, l.H, l.W, q.n0);
+    if (ng) { find_strays(sg, q.gout.list, ng, l.K, l.oH, l.oW, 0); unscale = pair_unscale(*q.act.rec); }
+    __syncthreads();
+  }
   const unsigned kHW = (unsigned)(u.kH * u.kW), per = (unsigned)u.C * kHW, total = (unsigned)K * per;
   for (unsigned t = blockIdx.x * blockDim.x + threadIdx.x; t < total; t += gridDim.x * blockDim.x) {
     const unsigned ko = t / per, r = t - ko * per, c = r / kHW, tap = r - c * kHW, i = tap / (unsigned)u.kW, j = tap - i * u.kW;
@@ -556,7 +708,22 @@ static __global__ void __launch_bounds__(256) unpack_grad_weight_kernel(const fl
     const long ch = (dy * u.eW + dx) * u.Cq + (int)c;
     const float *s = T + (p.first + ko * p.ko_stride + ch * p.ch_stride + bi * p.bi_stride + bj * p.bj_stride);
     float sum = *s;
-    for (int q = 1; q < p.copies; q++) sum += s[q * p.copy_stride];
+    for (int b = 1; b < p.copies; b++) sum += s[b * p.copy_stride];
+    if constexpr (PAIRS) {
+      for (int e = 0; e < na; e++) {
+        const StrayPlaces &f = sa;
+        if (f.c[e] != (int)c || f.n[e] < 0 || f.n[e] >= l.N) continue;
+        const int ty = f.y[e] + l.pad - (int)i, tx = f.x[e] + l.pad - (int)j, oy = ty / l.dH, ox = tx / l.dW;
+        if (ty < 0 || tx < 0 || oy * l.dH != ty || ox * l.dW != tx || oy >= l.oH || ox >= l.oW) continue;
+        sum += f.v[e] * q.go[(((long)f.n[e] * l.K + ko) * l.oH + oy) * l.oW + ox];
+      }
+      for (int e = 0; e < ng; e++) {
+        const StrayPlaces &f = sg;
+        if (f.c[e] != (int)ko) continue;
+        const int y = f.y[e] * l.dH + (int)i - l.pad, x = f.x[e] * l.dW + (int)j - l.pad;
+        if ((unsigned)y < (unsigned)l.H && (unsigned)x < (unsigned)l.W) sum += f.v[e] * plane_value(q.planes, u, f.n[e], (int)c, y, x, unscale);
+      }
+    }
     gw[t] += scale * sum;
   }
 }

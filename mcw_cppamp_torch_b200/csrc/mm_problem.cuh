@@ -34,35 +34,32 @@ enum : int { kTf32 = 0, kBf16 = 1, kPairs = 2 };
 
 // ---- FP16 pairs --------------------------------------------------------------------------------------------------
 // x * 2^e = hi + lo * 2^-11 with hi = fp16(x * 2^e), lo = fp16((x * 2^e - hi) * 2^11), where e puts the operand's largest value into
-// [2^14, 2^15): 22 bits of every value down to 2^-29 of the largest, one more than the two TF32 parts hold (whose hi is
-// truncated), at four bytes a value and twice the tensor pipe's TF32 rate.  Below that the error stays at 2^-51 of the
-// largest value.  FP16's exponents do not reach over operands of any range, so a pass (range_kernel) measures each operand
-// first, and where one
-//   holds an infinity or a NaN,
-//   has its largest value outside [2^-60, 2^60],
-//   has a value below 2^-38 of the largest (fewer than 13 bits left), or
-//   among 512 neighbours has two groups of four with values below 2^-29 of the largest
-// all operands of the product stay in FP32, in the same buffers, and the same launch multiplies them as kTf32.
-// (A group of four may hold stray small values because tensors of 10^8 values do: the density of a layer's outputs around
-// zero leaves a few below 2^-29 of the largest.)
+// [2^14, 2^15): 22 bits of every value whose hi is a normal FP16 number, that is down to 2^-28 of the largest, as the two TF32 parts hold
+// (whose hi is truncated), at four bytes a value and twice the tensor pipe's TF32 rate.  FP16's exponents reach no further, and a
+// result may rest on smaller values alone (a row of zeros but one), so a pass (range_kernel) measures each operand first.
+//   Up to kStrays smaller values are listed; the pairs hold zeros in their place, and what they add to the result is added
+//   in FP32 (mm_strays.cuh).  Tensors of 10^8 values have a few: the density of a layer's outputs around zero leaves some
+//   below 2^-28 of the largest.
+//   More of them, an infinity or a NaN, or a largest value outside [2^-60, 2^60]: all operands of the product stay in FP32, in
+//   the same buffers, and the same launch multiplies them as kTf32.
+constexpr int kStrays = 512;
+struct Stray { long at; float v; };   // element `at` of the operand, in the order it was measured in
 struct RangeRec {
   unsigned max_bits;     // bits of the largest |x|; infinities and NaN rank above every number
-  unsigned low_inv;      // ~(bits of the smallest non-zero |x| - 1)
-  unsigned low2_inv;     // ~(the same of the second smallest group of four in any set of 512 - 1)
-  unsigned wide;         // the operand is in FP32 whatever the others say: another operand of its product asked for it
+  unsigned wide;         // the operand is in FP32 whatever the others say: too many strays, or another operand of its product asked for it
   unsigned ticket;
-  unsigned pad[3];
+  unsigned strays;       // length of the list that goes with the record
+  unsigned pad[4];
 };
 constexpr int kRangeWords = sizeof(RangeRec) / 4;
-static_assert(sizeof(RangeRec) == 32, "plane_records() hands out 32 bytes each");
-__device__ __forceinline__ bool range_is_wide(const RangeRec &r) {
-  if (r.wide) return true;
-  if (r.max_bits == 0) return false;   // zeros only
-  const unsigned e = r.max_bits >> 23;
-  if (e < 127 - 60 || e > 127 + 60) return true;
-  const float most = __uint_as_float(r.max_bits);
-  return ~r.low_inv < __float_as_uint(most * 0x1p-38f) - 1u || ~r.low2_inv < __float_as_uint(most * 0x1p-29f) - 1u;
-}
+static_assert(kRangeWords == 8, "zeroed_words() keeps 32-byte boundaries");
+// What stays of an operand's measures beside planes that outlive a call.
+struct KeptRange { RangeRec rec; Stray strays[kStrays]; };
+static_assert(sizeof(KeptRange) == kPlaneRecordBytes, "what plane_record() hands out");
+__device__ __forceinline__ bool max_is_wide(unsigned max_bits) { return max_bits && (max_bits >> 23 < 127 - 60 || max_bits >> 23 > 127 + 60); }
+__device__ __forceinline__ bool range_is_wide(const RangeRec &r) { return r.wide || max_is_wide(r.max_bits); }
+// Non-zero magnitudes below these bits are strays (of an operand that is not wide).
+__device__ __forceinline__ unsigned stray_limit(unsigned max_bits) { return max_bits ? ((max_bits >> 23) - 28u) << 23 : 0u; }
 // 2^e of an operand that is not wide, and 2^-e
 __device__ __forceinline__ float pair_scale(const RangeRec &r) { return r.max_bits ? __uint_as_float((127u + 14u + 127u - (r.max_bits >> 23)) << 23) : 1.f; }
 __device__ __forceinline__ float pair_unscale(const RangeRec &r) { return r.max_bits ? __uint_as_float(((r.max_bits >> 23) - 14u) << 23) : 1.f; }
@@ -75,6 +72,14 @@ struct Ranges {
     for (int i = 0; i < 3; i++) w = w || (rec[i] && range_is_wide(*rec[i]));
     return w;
   }
+};
+// An operand's record and list.  `kept`: of planes from an earlier call, which hold zeros for the strays also after they have been
+// brought back to FP32; planes that this call wrote in FP32 hold everything.
+struct Measured {
+  RangeRec *rec = nullptr;
+  Stray *list = nullptr;
+  bool kept = false;
+  __device__ __forceinline__ int strays(bool wide) const { return !rec || (wide && !kept) ? 0 : (int)rec->strays; }
 };
 // Division of a non-negative 31-bit integer by a runtime constant as multiply-high + shift.
 struct FastDiv {

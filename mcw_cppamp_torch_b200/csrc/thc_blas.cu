@@ -113,13 +113,13 @@ static void gemm_raw(GemmSide x, GemmSide y, long k, float alpha, float beta, fl
 }
 // The same over FP16 pairs: a pass measures both operands and one splits them, each as it lies in memory.
 template <bool A_MN, bool B_MN>
-static void gemm_pairs_t(const void *a, long lda, const void *b, long ldb, long m, long n, long k, const mm::Epilogue &epi, const mm::RangeRec *ra,
-                         const mm::RangeRec *rb) {
+static void gemm_pairs_t(const void *a, long lda, const void *b, long ldb, long m, long n, long k, const mm::Epilogue &epi,
+                         const mm::Ranges &ranges) {
   using namespace mm;
   Problem<RawOperand<A_MN, kPairs>, RawOperand<B_MN, kPairs>, false, kPairs> p;
   p.epi = epi;
   p.M = m; p.N = n; p.K = k;
-  p.range_a = ra; p.range_b = rb; p.ranges.rec[0] = ra; p.ranges.rec[1] = rb;
+  p.range_a = ranges.rec[0]; p.range_b = ranges.rec[1]; p.ranges = ranges;
   launch_raw(p, [&](auto &q, int bn2) {
     attach_raw_map<kPairs>(q.a, a, m, k, lda, TC_BM);
     attach_raw_map<kPairs>(q.b, b, n, k, ldb, bn2 / 2);
@@ -128,26 +128,31 @@ static void gemm_pairs_t(const void *a, long lda, const void *b, long ldb, long 
 static void gemm_pairs(GemmSide x, GemmSide y, long k, float alpha, float beta, float *c, long ldc, const float *row_bias) {
   using namespace mm;
   const Epilogue epi = gemm_sides(x, y, alpha, beta, c, ldc, row_bias);
-  RangeRec *rec[2] = {new_range_rec(), new_range_rec()};
+  const Measured m[2] = {new_measured(), new_measured()};
   RangeJob ranges[2];
   PairJob jobs[2];
+  StraySide strays[2];
   const GemmSide *sides[2] = {&x, &y};
   long pieces = 0;
   for (int i = 0; i < 2; i++) {
     const GemmSide &s = *sides[i];
     const long lines = s.along_k ? s.rows : k, run = s.along_k ? k : s.rows, ldp = (run + 63) / 64 * 64;
-    ranges[i] = range_job(s.p, lines, run, s.ld, rec[i]);
+    ranges[i] = range_job(s.p, lines, run, s.ld, m[i]);
     jobs[i] = PairJob{s.p, ws_alloc(sizeof(float) * lines * ldp), lines, run, s.ld, ldp, ((uintptr_t)s.p & 15) == 0 && s.ld % 4 == 0, {}};
-    jobs[i].ranges.rec[0] = rec[i]; jobs[i].ranges.rec[1] = rec[1 - i];
+    jobs[i].ranges.rec[0] = m[i].rec; jobs[i].ranges.rec[1] = m[1 - i].rec;
+    strays[i] = StraySide{s.p, s.ld, run, s.along_k, m[i]};
     pieces = std::max(pieces, lines * ((ldp + 511) / 512));
   }
   launch_ranges(ranges[0], &ranges[1]);
   pdl_launch(split_matrix_kernel, dim3((unsigned)std::min<long>((pieces + 7) / 8, ctx().sm_count * 8l), 2), 256, 0, jobs[0], jobs[1]);
   check_launch("split_matrix");
-  if (!x.along_k && y.along_k) gemm_pairs_t<true, false>(jobs[0].dst, jobs[0].ldp, jobs[1].dst, jobs[1].ldp, x.rows, y.rows, k, epi, rec[0], rec[1]);
-  else if (x.along_k && y.along_k) gemm_pairs_t<false, false>(jobs[0].dst, jobs[0].ldp, jobs[1].dst, jobs[1].ldp, x.rows, y.rows, k, epi, rec[0], rec[1]);
-  else if (!x.along_k) gemm_pairs_t<true, true>(jobs[0].dst, jobs[0].ldp, jobs[1].dst, jobs[1].ldp, x.rows, y.rows, k, epi, rec[0], rec[1]);
-  else gemm_pairs_t<false, true>(jobs[0].dst, jobs[0].ldp, jobs[1].dst, jobs[1].ldp, x.rows, y.rows, k, epi, rec[0], rec[1]);
+  const Ranges &r = jobs[0].ranges;
+  if (!x.along_k && y.along_k) gemm_pairs_t<true, false>(jobs[0].dst, jobs[0].ldp, jobs[1].dst, jobs[1].ldp, x.rows, y.rows, k, epi, r);
+  else if (x.along_k && y.along_k) gemm_pairs_t<false, false>(jobs[0].dst, jobs[0].ldp, jobs[1].dst, jobs[1].ldp, x.rows, y.rows, k, epi, r);
+  else if (!x.along_k) gemm_pairs_t<true, true>(jobs[0].dst, jobs[0].ldp, jobs[1].dst, jobs[1].ldp, x.rows, y.rows, k, epi, r);
+  else gemm_pairs_t<false, true>(jobs[0].dst, jobs[0].ldp, jobs[1].dst, jobs[1].ldp, x.rows, y.rows, k, epi, r);
+  pdl_launch(matrix_strays_kernel, dim3((unsigned)std::min(ceil_div(y.rows, 256), ctx().sm_count), 4), 256, 0, strays[0], strays[1], x.rows, y.rows, epi, r);
+  check_launch("matrix_strays");
 }
 // Whether pairs finish before TF32, the passes over the operands included.  Their copies are scratch that TF32 does without: bounded.
 static bool pairs_are_faster(long m, long n, long k) {

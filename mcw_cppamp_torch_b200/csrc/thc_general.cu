@@ -53,7 +53,9 @@ static void init_device(Context &c, int device) {
   if (c.scratch) { cudaFree(c.scratch); c.scratch = nullptr; c.scratch_bytes = 0; }
   if (c.stall_dev) { cudaFree(c.stall_dev); c.stall_dev = nullptr; }
   if (c.sched_counters) { cudaFree(c.sched_counters); c.sched_counters = nullptr; c.sched_stream = nullptr; }
-  if (c.plane_records) { cudaFree(c.plane_records); c.plane_records = nullptr; c.plane_epoch++; }
+  for (void *&r : c.plane_records)
+    if (r) { cudaFree(r); r = nullptr; }
+  c.plane_epoch++;
   if (c.ws_base) { cudaFree(c.ws_base); c.ws_base = nullptr; c.ws_cap = c.ws_used = 0; c.ws_epoch++; }
   c.device = device;
   THC_CUDA(cudaStreamCreateWithFlags(&c.stream, cudaStreamNonBlocking));
@@ -137,10 +139,11 @@ unsigned *zeroed_words(int n) {
 }
 unsigned *sched_counter() { return zeroed_words(1); }
 
-void *plane_records() {
-  Context &c = ctx();
-  if (!c.plane_records) THC_CUDA(cudaMalloc(&c.plane_records, 32 * kPlaneRecords));
-  return c.plane_records;
+void *plane_record(int i) {
+  constexpr int per = kPlaneRecords / kPlaneChunks;
+  void *&chunk = ctx().plane_records[i / per];
+  if (!chunk) THC_CUDA(cudaMalloc(&chunk, kPlaneRecordBytes * per));
+  return (char *)chunk + kPlaneRecordBytes * (i % per);
 }
 
 // Names of the wait codes of mm_tc.cuh (kWait*), for the error message.

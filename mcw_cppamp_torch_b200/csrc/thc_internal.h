@@ -86,7 +86,7 @@ struct Context {
   unsigned *sched_counters = nullptr;
   int sched_next = 0, sched_block = 0, sched_recorded = 0;
   cudaStream_t sched_stream = nullptr;
-  void *plane_records = nullptr;   // see plane_records()
+  void *plane_records[64] = {};    // see plane_record()
   long plane_epoch = 0;            // bumped whenever they are given back
 };
 
@@ -120,9 +120,10 @@ unsigned *sched_counter();
 unsigned *zeroed_words(int n);
 int device_if_initialised();       // -1 before the first CUDA use on this thread; never initialises
 void *scratch(size_t bytes);      // grow-only device scratch of the reductions, zero-filled when (re)allocated
-// kPlaneRecords records of 32 bytes for planes that outlive an entry point (mm::RangeRec; which belongs to whom is the caller's).
-constexpr int kPlaneRecords = 4096;
-void *plane_records();
+// Records for planes that outlive an entry point (mm::KeptRange; which belongs to whom is the caller's), allocated 64 at a time.
+constexpr int kPlaneRecords = 4096, kPlaneChunks = 64;
+constexpr size_t kPlaneRecordBytes = 8224;
+void *plane_record(int i);
 // Device words that are zero between launches: tickets of kernels that put them back to zero when they are done.  One
 // block for all of them, since the launches of a context run one after the other on its stream.
 constexpr int kZeroWords = 16384;
