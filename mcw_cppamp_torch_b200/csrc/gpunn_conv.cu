@@ -624,8 +624,15 @@ static void conv_forward(const ConvGeom &g, const float *in, const float *w, con
     // layer over 3 planes is 6.2 MB an image, and its weight gradient FP32-accurate
     THGPUTensor *keep = half == half_acc_grad(g) ? finput : nullptr;
     if (!keep) forget_planes(finput);
+    if (prec == mm::kPairs) {
+      try {
+        conv_forward_tc<mm::kPairs>(g, u, in, w, bias, out, keep);
+        return;
+      } catch (const OutOfMemory &) {   // FP32 planes may take half of it (channels in spans of 32, not 64)
+        restate(g, mm::kTf32, u);
+      }
+    }
     if (prec == mm::kBf16) conv_forward_tc<mm::kBf16>(g, u, in, w, bias, out, keep);
-    else if (prec == mm::kPairs) conv_forward_tc<mm::kPairs>(g, u, in, w, bias, out, keep);
     else conv_forward_tc<mm::kTf32>(g, u, in, w, bias, out, keep);
     return;
   }
@@ -668,8 +675,9 @@ static void conv_backward_group(const ConvGeom &g, const mm::Cells &u, bool in_o
     grad_bias(g, gout, gb, scale);
   }
 }
+// False: there is no room for planes of this precision (kPairs), and nothing has been done.
 template <int PREC>
-static void conv_backward_tc(const ConvGeom &g, const mm::Cells &u, bool restated, const float *in, const float *gout, const float *w, float *gin,
+static bool conv_backward_tc(const ConvGeom &g, const mm::Cells &u, bool restated, const float *in, const float *gout, const float *w, float *gin,
                              float *gw, float *gb, float scale, const THGPUTensor *finput) {
   const mm::Cells ui = grad_input_cells(g, PREC);
   const bool in_ok = gin && mm::windows_ok(grad_input_windows(g, ui, PREC)), w_ok = gw && restated;
@@ -682,6 +690,10 @@ static void conv_backward_tc(const ConvGeom &g, const mm::Cells &u, bool restate
   if (in_ok && !ui.direct) bytes += 4. * ui.Cr * ui.Hs * ui.Ws;
   if (w_ok && !act) bytes += (double)act_image;
   const long image = g.C * g.H * g.W, per = images_per_group(g.N, bytes, whole_scratch((double)g.N * (image + g.K * g.P)));
+  // with the weights' forms, the measures (under a hundredth of the planes) and the partial sums (see gemm_pairs)
+  if (PREC == mm::kPairs &&
+      !ws_reserve((size_t)(1.01 * bytes * (double)per + 16. * (double)(g.K + 64) * std::max(u.kHs * u.kWs * (double)u.Cs, (double)g.R) + 96e6)))
+    return false;
   for (long n0 = 0; n0 < g.N; n0 += per) {
     ConvGeom s = g;
     s.N = std::min(per, g.N - n0);
@@ -717,6 +729,7 @@ static void conv_backward_tc(const ConvGeom &g, const mm::Cells &u, bool restate
       conv_forward_tc<PREC>(t, ut, go, transposed_weight(s, w, true), nullptr, gi, nullptr);
     }
   }
+  return true;
 }
 static void conv_backward(const ConvGeom &g, const float *in, const float *gout, const float *w, float *gin, float *gw, float *gb, float scale,
                           const THGPUTensor *finput) {
@@ -739,8 +752,11 @@ static void conv_backward(const ConvGeom &g, const float *in, const float *gout,
     // in the BF16 mode only for weight gradients: another last bit of a layer's result or gradInput would turn into others where the
     // next layer rounds it (the first layer's over 256 images: 385 -> 225 us)
     const bool ok = restate_accurate(g, ctx().math_mode == 0 || !gin || hin, u, prec);
-    if (prec == mm::kPairs) conv_backward_tc<mm::kPairs>(g, u, ok, in, gout, w, hin ? nullptr : gin, hw ? nullptr : gw, gb, scale, finput);
-    else conv_backward_tc<mm::kTf32>(g, u, ok, in, gout, w, hin ? nullptr : gin, hw ? nullptr : gw, gb, scale, finput);
+    if (prec == mm::kPairs) {
+      if (conv_backward_tc<mm::kPairs>(g, u, ok, in, gout, w, hin ? nullptr : gin, hw ? nullptr : gw, gb, scale, finput)) return;
+      restate(g, mm::kTf32, u);
+    }
+    conv_backward_tc<mm::kTf32>(g, u, ok, in, gout, w, hin ? nullptr : gin, hw ? nullptr : gw, gb, scale, finput);
   }
 }
 

@@ -125,8 +125,14 @@ static void gemm_pairs_t(const void *a, long lda, const void *b, long ldb, long 
     attach_raw_map<kPairs>(q.b, b, n, k, ldb, bn2 / 2);
   });
 }
-static void gemm_pairs(GemmSide x, GemmSide y, long k, float alpha, float beta, float *c, long ldc, const float *row_bias) {
+// False: there is no room for the pairs, and nothing has been done.
+static bool gemm_pairs(GemmSide x, GemmSide y, long k, float alpha, float beta, float *c, long ldc, const float *row_bias) {
   using namespace mm;
+  // the copies, with a little for the measures (under a hundredth of them) and the partial sums (blocks of 256 KB, up to
+  // five rounds of clusters)
+  double need = 96e6;
+  for (const GemmSide &s : {x, y}) need += 4.1 * (double)(s.along_k ? s.rows : k) * (double)((s.along_k ? k : s.rows) + 64);
+  if (!ws_reserve((size_t)need)) return false;
   const Epilogue epi = gemm_sides(x, y, alpha, beta, c, ldc, row_bias);
   const Measured m[2] = {new_measured(), new_measured()};
   RangeJob ranges[2];
@@ -153,6 +159,7 @@ static void gemm_pairs(GemmSide x, GemmSide y, long k, float alpha, float beta, 
   else gemm_pairs_t<false, true>(jobs[0].dst, jobs[0].ldp, jobs[1].dst, jobs[1].ldp, x.rows, y.rows, k, epi, r);
   pdl_launch(matrix_strays_kernel, dim3((unsigned)std::min(ceil_div(y.rows, 256), ctx().sm_count), 4), 256, 0, strays[0], strays[1], x.rows, y.rows, epi, r);
   check_launch("matrix_strays");
+  return true;
 }
 // Whether pairs finish before TF32, the passes over the operands included.  Their copies are scratch that TF32 does without: bounded.
 static bool pairs_are_faster(long m, long n, long k) {
@@ -231,8 +238,8 @@ void gemm(char transa, char transb, long m, long n, long k, float alpha, const f
   const bool aligned = mm::raw_matrix_ok(a, lda) && mm::raw_matrix_ok(b, ldb);
   if (mode == 2 && m > 128 && n > 32) gemm_half(x, y, k, alpha, beta, c, ldc, row_bias);
   else if (small_is_faster(m, n, k, aligned)) gemm_small(x, y, k, alpha, beta, c, ldc, row_bias);
-  else if (mode == 0 && pairs_are_faster(m, n, k)) gemm_pairs(x, y, k, alpha, beta, c, ldc, row_bias);
-  else gemm_raw(x, y, k, alpha, beta, c, ldc, row_bias);
+  else if (!(mode == 0 && pairs_are_faster(m, n, k) && gemm_pairs(x, y, k, alpha, beta, c, ldc, row_bias)))
+    gemm_raw(x, y, k, alpha, beta, c, ldc, row_bias);
 }
 
 // y = beta*y + alpha*op(A)*x.  'n': A is m x n column-major, y has m entries: threads own rows

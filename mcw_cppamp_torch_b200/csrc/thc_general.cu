@@ -225,30 +225,47 @@ unsigned *zero_words() { return (unsigned *)((char *)scratch(1 << 20) + (1 << 17
 void *dev_alloc(size_t bytes) {
   if (bytes == 0) return nullptr;
   void *p = nullptr;
-  THC_CUDA(cudaMallocAsync(&p, bytes, stream()));
+  const cudaError_t e = cudaMallocAsync(&p, bytes, stream());
+  if (e == cudaErrorMemoryAllocation) {
+    cudaGetLastError();
+    throw OutOfMemory("CUDA error cudaErrorMemoryAllocation: no room for " + std::to_string(bytes) + " bytes of device memory");
+  }
+  THC_CUDA(e);
   g_ctx.allocs++;
   return p;
 }
 
+// Replaces the arena by one that holds what this call has taken so far plus `bytes`, with headroom.
+// Pointers handed out earlier in this call stay valid: the old arena is only freed when the call returns.
+static void ws_grow(Context &c, size_t bytes) {
+  THC_CHECK(c.ws_nretired < 8, "internal: workspace arena outgrown too often inside one call");
+  size_t want = c.ws_used + bytes;
+  if (want < c.ws_cap + c.ws_cap / 2) want = c.ws_cap + c.ws_cap / 2;
+  want = (want + ((size_t)64 << 20) - 1) & ~(((size_t)64 << 20) - 1);
+  char *nb = (char *)dev_alloc(want);
+  if (c.ws_base) c.ws_retired[c.ws_nretired++] = c.ws_base;
+  c.ws_base = nb; c.ws_cap = want; c.ws_used = 0; c.ws_epoch++;
+}
 void *ws_alloc(size_t bytes) {
   Context &c = ctx();
   THC_CHECK(c.ws_depth > 0, "internal: workspace request outside an entry point's scope");
   bytes = (bytes + 255) & ~(size_t)255;
   if (bytes == 0) bytes = 256;
-  if (c.ws_used + bytes > c.ws_cap) {
-    // Replace the arena by one that holds what this call has taken so far plus the request, with headroom.
-    // Pointers handed out earlier in this call stay valid: the old arena is only freed when the call returns.
-    THC_CHECK(c.ws_nretired < 8, "internal: workspace arena outgrown too often inside one call");
-    size_t want = c.ws_used + bytes;
-    if (want < c.ws_cap + c.ws_cap / 2) want = c.ws_cap + c.ws_cap / 2;
-    want = (want + ((size_t)64 << 20) - 1) & ~(((size_t)64 << 20) - 1);
-    char *nb = (char *)dev_alloc(want);
-    if (c.ws_base) c.ws_retired[c.ws_nretired++] = c.ws_base;
-    c.ws_base = nb; c.ws_cap = want; c.ws_used = 0; c.ws_epoch++;
-  }
+  if (c.ws_used + bytes > c.ws_cap) ws_grow(c, bytes);
   void *p = c.ws_base + c.ws_used;
   c.ws_used += bytes;
   return p;
+}
+bool ws_reserve(size_t bytes) {
+  Context &c = ctx();
+  THC_CHECK(c.ws_depth > 0, "internal: workspace request outside an entry point's scope");
+  if (c.ws_used + bytes <= c.ws_cap) return true;
+  try {
+    ws_grow(c, bytes);
+  } catch (const OutOfMemory &) {
+    return false;
+  }
+  return true;
 }
 WsScope::WsScope() {
   Context &c = ctx();

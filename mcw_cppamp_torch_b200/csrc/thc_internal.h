@@ -18,6 +18,10 @@ struct Error : std::runtime_error {
   using std::runtime_error::runtime_error;
 };
 
+struct OutOfMemory : Error {   // the device has no room for a request; nothing else is wrong
+  using Error::Error;
+};
+
 [[noreturn]] void fail(const char *fmt, ...);
 void record_error(const char *msg);  // thread-local message + user handler
 
@@ -137,6 +141,8 @@ void dev_free(void *p);
 // is freed in stream order once the entry point returns) until it fits the largest call, then no entry point
 // asks the driver for memory at all.
 void *ws_alloc(size_t bytes);
+// Whether the next requests of this scope, `bytes` in all, can be had; for callers with a way that takes less.
+bool ws_reserve(size_t bytes);
 struct WsScope {
   size_t mark;
   long epoch;

@@ -1,5 +1,8 @@
-"""Device memory behind the products: zeroed words inside recordings, records over many groups of images."""
+"""Device memory behind the products: zeroed words inside recordings, records over many groups of images, scratch that is not to be had."""
 import ctypes
+import os
+import subprocess
+import sys
 
 import pytest
 import torch
@@ -97,3 +100,88 @@ def test_hundreds_of_groups(gt):  # noqa: F811
     (a, b), (am, bm) = grads(lambda t: t), grads(torch.abs)
     assert torch.all((got[0][0].double() - a[0]).abs() <= REL * am[0])
     assert torch.all((got[0][1].cuda().double().view_as(w) - b).abs() <= (REL + 2.0 ** -24 * (H * H / 32 + 64)) * bm)
+
+
+FULL_DEVICE = """
+import torch, mcw_cppamp_torch_b200 as gt
+from test_gpu_fp16_pairs import REL, products, randn
+from test_gpu_scratch import wrap
+m, n, k = 16384, 8192, 16384
+a, b, c = randn(1, m, k), randn(2, k, n), torch.empty(m, n, device="cuda")
+rows = torch.arange(0, m, 511, device="cuda")
+want, mass = a[rows].double() @ b.double(), a[rows].abs().double() @ b.abs().double()
+A, B, C = wrap(gt, a), wrap(gt, b), wrap(gt, c)
+s = wrap(gt, torch.ones(256, 256, device="cuda"))
+wrap(gt, torch.empty(256, 256, device="cuda")).addmm(0.0, 1.0, s, s)
+gt.synchronize()
+torch.cuda.synchronize()
+torch.cuda.empty_cache()
+fill = torch.empty(torch.cuda.mem_get_info()[0] - (1 << 30), dtype=torch.uint8, device="cuda")     # the pairs take 1.6 GB
+for form in (0, 2):
+    before = products(gt)
+    C.addmm(0.0, 1.0, A, B)
+    gt.synchronize()
+    assert [x - y for x, y in zip(products(gt), before)] == [form == 0, form == 2], form
+    assert torch.all((c[rows].double() - want).abs() <= REL * mass)
+    fill = None
+    torch.cuda.empty_cache()
+"""
+
+
+FULL_DEVICE_CONVOLUTION = """
+import torch, mcw_cppamp_torch_b200 as gt
+from test_gpu_fp16_pairs import REL, products, randn
+from test_gpu_scratch import wrap
+N, C, H, K = 1024, 96, 56, 96
+x, w, go, gi = randn(1, N, C, H, H), randn(2, K, C, 3, 3), randn(3, N, K, H, H), torch.empty(N, C, H, H, device="cuda")
+out = torch.empty(N, K, H, H, device="cuda")
+m = gt.nn.SpatialConvolutionMM(C, K, 3, 3, 1, 1, 1)
+m.weight.reshape(-1)[:] = w.cpu().numpy().reshape(-1)
+m.bias[:] = 0
+m.gpu()
+m.output, m.gradInput = wrap(gt, out), wrap(gt, gi)
+X, GO = wrap(gt, x), wrap(gt, go)
+image = [0, N - 1]
+def grads(f):
+    xi, wi = f(x[image]).double().requires_grad_(), f(w).double().requires_grad_()
+    o = torch.nn.functional.conv2d(xi, wi, None, 1, 1)
+    return (o.detach(),) + torch.autograd.grad(o, xi, f(go[image]).double())
+want, mass = grads(lambda t: t), grads(torch.abs)
+def fill(room):
+    gt.synchronize()
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    return torch.empty(torch.cuda.mem_get_info()[0] - room, dtype=torch.uint8, device="cuda")
+s = wrap(gt, torch.ones(256, 256, device="cuda"))
+wrap(gt, torch.empty(256, 256, device="cuda")).addmm(0.0, 1.0, s, s)
+full = fill(1500 << 20)                # planes: 1.23 GB, as pairs 1.64
+before = products(gt)
+m.forward(X)
+del full
+full = fill(1500 << 20)                # gradOutput's planes likewise
+m.zeroGradParameters()
+m.backward(X, GO)
+gt.synchronize()
+assert [b - a for b, a in zip(products(gt), before)] == [3, 0], products(gt)
+for got, a, b in zip((out, gi), want, mass):
+    assert torch.all((got[image].double() - a).abs() <= REL * b)
+del full
+torch.cuda.empty_cache()
+before = products(gt)
+m.forward(X)
+m.backward(X, GO)
+gt.synchronize()
+assert [b - a for b, a in zip(products(gt), before)] == [0, 3], products(gt)
+for got, a, b in zip((out, gi), want, mass):
+    assert torch.all((got[image].double() - a).abs() <= REL * b)
+"""
+
+
+@pytest.mark.parametrize("program", [FULL_DEVICE, FULL_DEVICE_CONVOLUTION])
+def test_product_on_a_full_device(gt, program):  # noqa: F811
+    """Pairs are copies; where there is no room for them the product runs over the operands as they lie, or planes in FP32 where those are
+    smaller.  (A process of its own: this one's workspace has grown already.)"""
+    tests = os.path.dirname(os.path.abspath(__file__))
+    env = dict(os.environ, PYTHONPATH=os.pathsep.join([os.path.dirname(tests), tests]))
+    r = subprocess.run([sys.executable, "-c", program], env=env, capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stderr
