@@ -623,6 +623,12 @@ static void conv_forward(const ConvGeom &g, const float *in, const float *w, con
     // kept for a weight gradient of the same precision only, no other reads them back: the BF16 column matrix of the 11 x 11 / 4
     // layer over 3 planes is 6.2 MB an image, and its weight gradient FP32-accurate
     THGPUTensor *keep = half == half_acc_grad(g) ? finput : nullptr;
+    if (keep && ctx().math_mode == 2 && !half) {   // an FP32-accurate layer of that mode: its weight gradient may run over pairs (conv_backward)
+      mm::Cells uw;
+      int pw;
+      restate_accurate(g, true, uw, pw);
+      if (pw != prec) keep = nullptr;
+    }
     if (!keep) forget_planes(finput);
     if (prec == mm::kPairs) {
       try {

@@ -1,4 +1,5 @@
-"""Device memory behind the products: zeroed words inside recordings, records over many groups of images, scratch that is not to be had."""
+"""Device memory behind the products: zeroed words inside recordings, records over many groups of images, scratch that is not to be had,
+planes that are kept."""
 import ctypes
 import os
 import subprocess
@@ -185,3 +186,30 @@ def test_product_on_a_full_device(gt, program):  # noqa: F811
     env = dict(os.environ, PYTHONPATH=os.pathsep.join([os.path.dirname(tests), tests]))
     r = subprocess.run([sys.executable, "-c", program], env=env, capture_output=True, text=True, timeout=300)
     assert r.returncode == 0, r.stderr
+
+
+@pytest.mark.parametrize("N,kept", [(64, False), (4, True)])
+def test_planes_of_the_bf16_mode(gt, N, kept):  # noqa: F811
+    """A layer that the BF16 mode leaves FP32-accurate keeps planes for its weight gradient where that reads them, not where it runs over pairs."""
+    C, H, K, k = 64, 56, 32, 3
+    x, w, go = randn(1, N, C, H, H), randn(2, K, C, k, k), randn(3, N, K, H, H)
+    m = gt.nn.SpatialConvolutionMM(C, K, k, k, 1, 1, 1)
+    m.weight.reshape(-1)[:] = w.cpu().numpy().reshape(-1)
+    m.gpu()
+    gt.set_math_mode("bf16")
+    try:
+        xg, gog = gt.gpu(x.cpu().numpy()), gt.gpu(go.cpu().numpy())
+        m.forward(xg)
+        assert (m.finput.dim() > 0) == kept
+        m.zeroGradParameters()
+        before = products(gt)
+        m.accGradParameters(xg, gog)
+        assert [a - b for a, b in zip(products(gt), before)] == ([1, 0] if kept else [0, 1])
+        gw = torch.from_numpy(m.gradWeight.float()).cuda().double().view_as(w)
+    finally:
+        gt.set_math_mode("fp32x3")
+
+    def grad(f):
+        wi = f(w).double().requires_grad_()
+        return torch.autograd.grad(torch.nn.functional.conv2d(f(x).double(), wi, None, 1, 1), wi, f(go).double())[0]
+    assert torch.all((gw - grad(lambda t: t)).abs() <= (REL + 2.0 ** -24 * (go.numel() / K / 32 + 64)) * grad(torch.abs))
