@@ -269,7 +269,14 @@ static void restate_input(const ConvGeom &g, const mm::Cells &u, const float *in
   if constexpr (PREC != mm::kBf16) {
     const int q = u.Cs / (PREC == mm::kPairs ? 8 : 4);
     const long Wp = (long)(u.Ws - 1) * u.dW + u.eW, ld = (Wp + 15) / 32 * 32 + 16, smem = 4l * u.C * u.eH * ld;
-    if (256 % q == 0 && smem <= 40 * 1024 && rows >= 2l * ctx().sm_count) {
+    // Rows long enough to hide a block's barriers, of few input lines.  By units of 16 bytes a row, forward pass of the layer staged and
+    // not (us): 3 x 3 over 224 wide (1792 units) 451 / 510, 13 images 101 / 112, 7 x 7 / 2 (1840) 241 / 271, 500 wide
+    // (8000) 8239 / 8954, 128 wide 4 planes (1040) 224 / 228; 912 units 384 / 409 over 14592 rows, 132.5 / 132.6 over 3648, 48.4 / 47.7 over
+    // 912; 832 units 168.6 / 170.4 over 6400 rows, 768 183 / 194 over 12288; below, it loses: 608 112.3 / 109.5, 536 76.6 / 73.0, 464
+    // 44.1 / 38.2, 256 59.6 / 51.7 and 206 / 187.  45 lines of 85 columns (1360): 211.5 / 205.3, 21 lines gain.
+    const long units = chunks * (PREC == mm::kPairs ? 2 : 1);
+    if (256 % q == 0 && smem <= 40 * 1024 && rows >= 2l * ctx().sm_count && u.C * u.eH <= 24 &&
+        (units >= 1024 || (units >= 768 && rows >= 32l * ctx().sm_count))) {
       pdl_launch(mm::cells_staged_kernel<PREC>, (unsigned)std::min(rows, 16l * ctx().sm_count), 256, smem, in, dst, g.N, u, (int)Wp, (int)ld, form);
       check_launch("cells_staged");
       return;

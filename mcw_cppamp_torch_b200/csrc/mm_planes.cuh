@@ -487,7 +487,7 @@ static __global__ void __launch_bounds__(256) cells_input_kernel(const float *__
 // The same where a row's input fits shared memory and each thread keeps the channels it writes (Cs / V divides the block): the
 // C * eH input rows are read once, in order, with zeros around them, and every value leaves from there without a bounds check
 // or a table look-up.  Bound by the latency of a row's reads and by its shared-memory reads (lines 16 banks apart, the least
-// conflicts for cells of four columns).  3 planes of 224 x 224 as 4 x 4 cells: 1024 images as pairs (1.47 GB) 493 -> 338 us,
+// conflicts for cells of four columns); for long rows (see restate_input).  3 planes of 224 x 224 as 4 x 4 cells: 1024 images as pairs (1.47 GB) 493 -> 338 us,
 // 256 images in FP32 78 -> 70.
 template <int PREC>
 static __global__ void __launch_bounds__(256) cells_staged_kernel(const float *__restrict__ in, void *__restrict__ S, long N, const Cells u, int Wp, int ld,
