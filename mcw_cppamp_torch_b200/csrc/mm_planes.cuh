@@ -114,6 +114,7 @@ static __global__ void __launch_bounds__(256) range_kernel(const RangeJob ja, co
   if (threadIdx.x == 0) j.rec->max_bits = most;
   const unsigned limit = stray_limit(most) - 1u;   // (as the lows: bits - 1)
   if (!most || max_is_wide(most)) return;
+  const int allowed = (int)min((long)kStrays, stray_allowance(sets.total));
 #pragma unroll
   for (int i = 0; i < kRangeBlocks / 256; i++)
     if (r[i].y < limit) blocks[atomicAdd(&nblocks, 1)] = (unsigned short)(i * 256 + threadIdx.x);
@@ -146,13 +147,13 @@ static __global__ void __launch_bounds__(256) range_kernel(const RangeJob ja, co
                 if (n < kStrays) buf[n] = Stray{at[g] + e, __uint_as_float(v[g][e])};
               }
           __syncwarp();
-          stop = __shfl_sync(0xffffffffu, *const_cast<volatile int *>(&found), 0) > kStrays;
+          stop = __shfl_sync(0xffffffffu, *const_cast<volatile int *>(&found), 0) > allowed;
         }
     }
   }
   __syncthreads();
   const int n = found;
-  if (n > kStrays) {
+  if (n > allowed) {
     if (threadIdx.x == 0) j.rec->wide = 1;
     return;
   }

@@ -37,12 +37,15 @@ enum : int { kTf32 = 0, kBf16 = 1, kPairs = 2 };
 // [2^14, 2^15): 22 bits of every value whose hi is a normal FP16 number, that is down to 2^-28 of the largest, as the two TF32 parts hold
 // (whose hi is truncated), at four bytes a value and twice the tensor pipe's TF32 rate.  FP16's exponents reach no further, and a
 // result may rest on smaller values alone (a row of zeros but one), so a pass (range_kernel) measures each operand first.
-//   Up to kStrays smaller values are listed; the pairs hold zeros in their place, and what they add to the result is added
+//   A few smaller values (stray_allowance) are listed; the pairs hold zeros in their place, and what they add to the result is added
 //   in FP32 (mm_strays.cuh).  Tensors of 10^8 values have a few: the density of a layer's outputs around zero leaves some
 //   below 2^-28 of the largest.
 //   More of them, an infinity or a NaN, or a largest value outside [2^-60, 2^60]: all operands of the product stay in FP32, in
 //   the same buffers, and the same launch multiplies them as kTf32.
+// How many: two hundred times what 10^8 normal values have.  Each may cost the launch that adds it 2 us (4096 x 4096 x 512 with 512 of them in
+// a row: 1266 us, 88 over pairs without and about 120 in FP32), so that small operands are allowed few.
 constexpr int kStrays = 512;
+__host__ __device__ constexpr long stray_allowance(long values) { return values / (1 << 18) + 8; }   // (kStrays at most)
 struct Stray { long at; float v; };   // element `at` of the operand, in the order it was measured in
 struct RangeRec {
   unsigned max_bits;     // bits of the largest |x|; infinities and NaN rank above every number

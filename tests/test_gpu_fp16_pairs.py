@@ -53,9 +53,10 @@ def check_addmm(gt, a, b, t1=False, t2=False, beta=0.0, rows=slice(None), cols=s
 
 @pytest.mark.parametrize("t1,t2", [(False, False), (False, True), (True, False), (True, True)])
 @pytest.mark.parametrize("m,n,k,beta", [(1500, 3001, 2222, 0.0), (2049, 1793, 2047, 1.0), (4097, 129, 4095, 0.0), (130, 4100, 4033, 1.0),
-                                        (2048, 2048, 2048, 0.0), (2048, 2048, 2048, 1.0), (1500, 3001, 2222, 0.5), (4097, 1025, 4033, 1.0)])
+                                        (2048, 2048, 2048, 0.0), (2304, 2304, 2304, 0.0), (2304, 2304, 2304, 1.0), (1500, 3001, 2222, 0.5),
+                                        (4097, 1025, 4033, 1.0)])
 def test_layouts_and_remainders(gt, m, n, k, beta, t1, t2):
-    check_addmm(gt, randn(m, m, k), randn(n, k, n), t1, t2, beta, pairs=(m, n) not in [(2049, 1793), (130, 4100)])
+    check_addmm(gt, randn(m, m, k), randn(n, k, n), t1, t2, beta, pairs=(m, n) not in [(2049, 1793), (4097, 129), (130, 4100), (2048, 2048)])
 
 
 @pytest.mark.parametrize("t1,t2", [(False, False), (True, True)])

@@ -22,18 +22,18 @@ def test_rows_of_one_value(gt, e, t1, t2):  # noqa: F811
 @pytest.mark.parametrize("e", [30, 37])
 def test_diagonals(gt, e):  # noqa: F811
     """Both operands have one, and theirs meet: the product of two small values is a result of its own."""
-    a, b = torch.eye(2048, device="cuda"), torch.eye(2048, device="cuda")
-    perm = torch.randperm(2048, generator=torch.Generator().manual_seed(1)).cuda()
-    for i in (5, 777, 2047):
+    a, b = torch.eye(2304, device="cuda"), torch.eye(2304, device="cuda")
+    perm = torch.randperm(2304, generator=torch.Generator().manual_seed(1)).cuda()
+    for i in (5, 777, 2303):
         a[i, i] = 1.25 * 2.0 ** -e
         b[i, i] = 1.7 * 2.0 ** -e
     check_addmm(gt, a, b)
     check_addmm(gt, a[:, perm].contiguous(), b[perm].contiguous(), beta=1.0)
 
 
-@pytest.mark.parametrize("n", [0, 1, 40, 511, 512, 513, 3000])
+@pytest.mark.parametrize("n", [0, 1, 23, 24, 25, 3000])
 def test_many(gt, n):  # noqa: F811
-    """More of them than a list holds send the product to FP32 values."""
+    """More of them than are listed, 24 of this operand's, send the product to FP32 values."""
     a, b = randn(3, 2000, 2100), randn(4, 2100, 2200)
     at = torch.randperm(a.numel(), generator=torch.Generator().manual_seed(n))[:n].cuda()
     a.view(-1)[at] = 2.0 ** -(30 + torch.arange(n, device="cuda") % 20).float()
@@ -129,7 +129,7 @@ def test_input_written_over(gt):  # noqa: F811
 
 def test_repeats_exactly(gt):  # noqa: F811
     a, b = randn(3, 2000, 2100), randn(4, 2100, 2200)
-    at = torch.randperm(a.numel(), generator=torch.Generator().manual_seed(1))[:400].cuda()
+    at = torch.randperm(a.numel(), generator=torch.Generator().manual_seed(1))[:24].cuda()
     a.view(-1)[at] = 1.1 * 2.0 ** -31
     A, B = gt.gpu(a.cpu().numpy()), gt.gpu(b.cpu().numpy())
     r = [gt.GPUTensor(2000, 2200).addmm(0.0, 1.0, A, B).float() for _ in range(3)]
