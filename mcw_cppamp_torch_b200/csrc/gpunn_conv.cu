@@ -615,6 +615,9 @@ static bool restate_accurate(const ConvGeom &g, bool pairs, mm::Cells &u, int &p
       windows_us(forward_windows(g, u), g.K, prec) < 30 || !restate(g, mm::kPairs, up) || up.Cs > 12288 ||   // (unpair_kernel: 48 KB)
       (up.kHs == 1 && up.kWs == 1 && !up.direct))
     return ok;
+  // (window_product_t counts the repacked weights in 31 bits; channels in spans of 64 may make more of them than spans of 32)
+  const mm::Cells gi = grad_input_cells(g, mm::kPairs);
+  if (2. * g.K * up.kHs * up.kWs * up.Cs >= 0x1p31 || 2. * (gi.direct ? gi.C : gi.Cr) * gi.kHs * gi.kWs * mm::padded_channels(g.K, mm::kPairs) >= 0x1p31) return ok;
   auto us = [&](const mm::Cells &c, int pr) {
     return windows_us(forward_windows(g, c), g.K, pr) + 2 * (double)mm::planes_bytes(g.N, (long)c.Hs * c.Ws, c.Cs, pr) / 5e6;
   };

@@ -213,3 +213,20 @@ def test_planes_of_the_bf16_mode(gt, N, kept):  # noqa: F811
         wi = f(w).double().requires_grad_()
         return torch.autograd.grad(torch.nn.functional.conv2d(f(x).double(), wi, None, 1, 1), wi, f(go).double())[0]
     assert torch.all((gw - grad(lambda t: t)).abs() <= (REL + 2.0 ** -24 * (go.numel() / K / 32 + 64)) * grad(torch.abs))
+
+
+def test_filter_of_a_billion_weights(gt):  # noqa: F811
+    """65 output planes are 96 in spans of 32, for which 31 bits count the repacked weights, and 128 in spans of 64, for which they do not."""
+    N, C, H, K, k = 16, 4096, 64, 65, 64
+    w, go = randn(1, K, C * k * k), randn(2, N, K, 1, 1)
+    x, gi = torch.empty(N, C, H, H, device="cuda"), torch.empty(N, C, H, H, device="cuda")
+    m = gt.nn.SpatialConvolutionMM(1, 1, 1, 1)
+    m.gpu()
+    torch.cuda.synchronize()
+    m.kW = m.kH = k
+    m.weight, m.gradInput = wrap(gt, w), wrap(gt, gi)
+    m.updateGradInput(wrap(gt, x), wrap(gt, go))
+    gt.synchronize()
+    for at in (slice(0, 5000), slice(C * k * k - 5000, C * k * k)):
+        a, b = go.view(N, K).double(), w[:, at].double()
+        assert torch.all((gi.view(N, -1)[:, at].double() - a @ b).abs() <= REL * (a.abs() @ b.abs()))
