@@ -62,6 +62,7 @@ void stamp_planes(const THGPUTensor *finput, const float *input, const ConvGeom 
   if (prec == mm::kPairs) {
     if (g_free_records.empty()) record = g_records++;
     else { record = g_free_records.back(); g_free_records.pop_back(); }
+    plane_record(record);   // there before the entry is
   }
   g_plane_stamps[data_ptr(finput)] = PlaneStamp{input, prec, g.N, g.C, g.H, g.W, g.K, g.kH, g.kW, g.dH, g.dW, g.pad, record, ctx().plane_epoch};
 }

@@ -142,7 +142,14 @@ unsigned *sched_counter() { return zeroed_words(1); }
 void *plane_record(int i) {
   constexpr int per = kPlaneRecords / kPlaneChunks;
   void *&chunk = ctx().plane_records[i / per];
-  if (!chunk) THC_CUDA(cudaMalloc(&chunk, kPlaneRecordBytes * per));
+  if (!chunk) {
+    const cudaError_t e = cudaMalloc(&chunk, kPlaneRecordBytes * per);
+    if (e == cudaErrorMemoryAllocation) {
+      cudaGetLastError();
+      throw OutOfMemory("CUDA error cudaErrorMemoryAllocation: no room for the records of kept planes");
+    }
+    THC_CUDA(e);
+  }
   return (char *)chunk + kPlaneRecordBytes * (i % per);
 }
 
