@@ -109,7 +109,7 @@ static mm::Windows forward_windows(const ConvGeom &g, const mm::Cells &u) {
 }
 
 // A tcgen05.mma occupies the tensor pipe about 80 cycles however narrow it is, so with up to 64 output planes two horizontally
-// adjacent output pixels share a row of the product (pixel-pair mode): prec the rows, twice the columns, a window one
+// adjacent output pixels share a row of the product (pixel-pair mode): half the rows, twice the columns, a window one
 // stride wider.  Worth it when the wider window costs less than the rows save; not for windows of one column.
 // FP32 only: BF16 products are bound by their operands' bytes, which the wider window adds to.
 static bool pair_windows(const mm::Windows &v, long Kout, int prec, mm::Windows &p) {
@@ -401,7 +401,7 @@ static void conv_grad_input_tc(const ConvGeom &g, const mm::ActPlanes &pgo, cons
 //        T[(bi, ch)][(j', ko)] = sum_{n, y, x'} S[n][y + bi][x'][ch] * gradOut[n][y][x' - (kWs - 1 - j')][ko]
 //      is the gradient of tap (bi, bj = kWs - 1 - j'): the column shift is a zero-padded window of the gradOutput
 //      plane, which TMA's im2col mode reads like any other.  For layers with few output planes and columns, whose
-//      64-wide tiles would run at prec the tensor-pipe rate.
+//      64-wide tiles would run at half the tensor-pipe rate.
 // and, for the column form (one tap), whose two operands are plain matrices of a few columns:
 //   3  f pixels side by side, rows = (pixel mod f, ko), columns = (pixel mod f, ch) of the same memory read as wider
 //      matrices: the f diagonal blocks of the result are the gradient's partial sums.  The other blocks are computed in
@@ -605,9 +605,12 @@ static bool half_acc_grad(const ConvGeom &g) {
 }
 
 // FP16 pairs or TF32 for the FP32-accurate products of a layer, all of which share its planes: by the forward product's time and
-// the pass that measures the input, with 10 us for the launches that measure and check (64 planes under 11 x 11 / 4 over 16 images,
-// 40 us a product: 201.5 us in TF32, 212.6 over pairs for the whole block; 128 images: 4020 -> 3160 us a training step).  The column
-// form stays in TF32, whose weight gradient stacks pixels.
+// the pass that measures the input, with 10 us for the launches that measure and check.  Forward and backward near the line (us, pairs /
+// TF32): 64 planes under 11 x 11 / 4 over 32 images 259 / 255, over 64 398 / 508; 64 -> 128 of 112 x 112, 4 images, 210 / 211; 64 -> 192 under 5 x 5, 27 x
+// 27, 16 images, 175 / 247; 512 -> 512 of 14 x 14, 13 images, 223 / 244; 64 -> 64 of 56 x 56, 32 images, 259 / 267.  Where an operand has to stay
+// in FP32 a layer takes longer than in TF32, by the measuring passes, spans of 64 channels and tiles of 128 or 256: 1024 images
+// 64 -> 192 8.13 ms / 7.16, 384 -> 256 4.45 / 4.31; 13 images 256 -> 256 of 56 x 56 778 us / 705, 512 -> 512 of 14 x 14 290 / 244; 96 -> 96 (128 for 96
+// channels), 64 images, 1250 / 1000.  The column form stays in TF32, whose weight gradient stacks pixels.
 static bool restate_accurate(const ConvGeom &g, bool pairs, mm::Cells &u, int &prec) {
   prec = mm::kTf32;
   const bool ok = restate(g, mm::kTf32, u);
