@@ -423,17 +423,18 @@ static Measured new_measured() { return Measured{(RangeRec *)zeroed_words(kRange
 // Neighbours in memory are neighbours along a line wherever lines are long or lie apart.
 static RangeJob range_job(const float *p, long lines, long run, long ld, const Measured &m) {
   const bool flat = (ld == run || lines == 1) && (lines < 4 || run < 64);
-  return RangeJob{p, lines, run, ld, flat, ((uintptr_t)p & 15) == 0 && (flat || ld % 4 == 0), m.rec, m.list, nullptr, nullptr};
+  return RangeJob{p, lines, run, ld, flat, ((uintptr_t)p & 15) == 0 && (flat || ld % 4 == 0), m.rec, m.list, 0, nullptr, nullptr};
 }
 static RangeJob range_job_flat(const float *p, long n, const Measured &m) { return range_job(p, 1, n, n, m); }
 static void launch_ranges(RangeJob a, RangeJob *b) {
   auto sets = [](const RangeJob &j) { return j.flat ? (j.lines * j.run + 511) / 512 : (j.run + 127) / 128 * ((j.lines + 3) / 4); };
-  const long most = std::max(sets(a), b ? sets(*b) : 0l);
-  const dim3 grid((unsigned)std::max(1l, std::min((most + 7) / 8, std::min(ctx().sm_count * 8l, (long)kRangeBlocks))), b ? 2 : 1);
+  dim3 grid(1, b ? 2 : 1);
   for (RangeJob *j : {&a, b})
     if (j) {
-      j->block_range = (uint2 *)ws_alloc(sizeof(uint2) * grid.x + sizeof(unsigned) * sets(*j));
-      j->set_low = (unsigned *)(j->block_range + grid.x);
+      j->blocks = (unsigned)std::max(1l, std::min((sets(*j) + 7) / 8, std::min(ctx().sm_count * 5l, (long)kRangeBlocks)));
+      j->block_range = (uint2 *)ws_alloc(sizeof(uint2) * j->blocks + sizeof(unsigned) * sets(*j));
+      j->set_low = (unsigned *)(j->block_range + j->blocks);
+      grid.x = std::max(grid.x, j->blocks);
     }
   pdl_launch(range_kernel, grid, 256, 0, a, b ? *b : a);
   check_launch("range");

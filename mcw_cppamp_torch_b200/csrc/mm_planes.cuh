@@ -29,6 +29,7 @@ struct RangeJob {
   int flat, vec;
   RangeRec *rec;
   Stray *list;
+  unsigned blocks;      // that look at it, of the launch's
   uint2 *block_range;   // a block's largest and smallest
   unsigned *set_low;
 };
@@ -59,12 +60,13 @@ struct RangeSets {
     }
   }
 };
-static __global__ void __launch_bounds__(256) range_kernel(const RangeJob ja, const RangeJob jb) {
+static __global__ void __launch_bounds__(256, 5) range_kernel(const RangeJob ja, const RangeJob jb) {
   pdl_begin();
   const RangeJob &j = blockIdx.y ? jb : ja;
+  if (blockIdx.x >= j.blocks) return;
   const RangeSets sets(j);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const long warps = (long)gridDim.x * 8, me = (long)blockIdx.x * 8 + warp;
+  const long warps = j.blocks * 8l, me = (long)blockIdx.x * 8 + warp;
   unsigned most = 0, low = ~0u;   // the lows as bits - 1: zero becomes the largest
   for (long k = me; k < sets.count; k += warps) {
     const long s = sets.count - 1 - k;   // from the end, which whoever wrote the operand has left in L2, to the start, which the next pass reads first
@@ -94,7 +96,7 @@ static __global__ void __launch_bounds__(256) range_kernel(const RangeJob ja, co
     for (int w = 1; w < 8; w++) { most = max(most, sm[0][w]); low = min(low, sm[1][w]); }
     j.block_range[blockIdx.x] = make_uint2(most, low);
     __threadfence();
-    last = atomicAdd(&j.rec->ticket, 1u) == gridDim.x - 1;
+    last = atomicAdd(&j.rec->ticket, 1u) == j.blocks - 1;
     found = nblocks = 0;
   }
   __syncthreads();
@@ -102,7 +104,7 @@ static __global__ void __launch_bounds__(256) range_kernel(const RangeJob ja, co
   __threadfence();
   uint2 r[kRangeBlocks / 256];   // all of them on the way at once
 #pragma unroll
-  for (int i = 0; i < kRangeBlocks / 256; i++) r[i] = i * 256 + threadIdx.x < gridDim.x ? __ldcg(j.block_range + i * 256 + threadIdx.x) : make_uint2(0, ~0u);
+  for (int i = 0; i < kRangeBlocks / 256; i++) r[i] = i * 256 + threadIdx.x < j.blocks ? __ldcg(j.block_range + i * 256 + threadIdx.x) : make_uint2(0, ~0u);
   most = 0;
 #pragma unroll
   for (int i = 0; i < kRangeBlocks / 256; i++) most = max(most, r[i].x);
