@@ -803,7 +803,8 @@ def run_ours(args):
                 # DRAM bytes of the GEMM-shaped launches of one step (ncu dram__bytes_read.sum + dram__bytes_write.sum
                 # over the 23 tc2r_kernel launches of a step captured at batch 128, over FP32 operands; FP16 pairs have as many
                 # bytes): 831 MB in the three classifier layers, whose traffic is their weights and does not grow with the
-                # batch, and 7.09 MB per image in the convolution layers, scaled to this rank's batch
+                # batch, and 7.09 MB per image in the convolution layers, scaled to this rank's batch.  Not in it: the
+                # measuring, splitting and transposing passes (12 bytes a value, about 10 MB an image), whose time `achieved` has
                 "traffic": 0.831e9 + 7.09e6 * nloc,
                 "kernel": "thc::mm::tc2r_kernel (persistent two-SM tcgen05 GEMM / implicit GEMM, FP32-accurate as three products of FP16 "
                           "halves; three TF32 products for small layers)",

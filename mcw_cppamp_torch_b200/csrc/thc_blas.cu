@@ -163,7 +163,7 @@ static bool gemm_pairs(GemmSide x, GemmSide y, long k, float alpha, float beta, 
 }
 // Whether pairs finish before TF32, the passes over the operands included.  Their copies are scratch that TF32 does without: bounded.
 // Measured on both sides of the line (us, pairs / TF32): 2048^3 78.0 / 75.8, 2304^3 102.5 / 108.0, 2560^3 125 / 148, 1500 x 3001 x 2222 115 / 129, 4096 x 4096
-// x 512 88 / 98, 1024 x 4096 x 4096 131 / 167.  Operands that have to stay in FP32 take a quarter to a half longer than TF32 does
+// x 512 88 / 98, 1024 x 4096 x 4096 131 / 167.  Operands that have to stay in FP32 take up to two fifths longer than TF32 does
 // (2304^3 142, 1024 x 4096 x 4096 217, 4096^3 731 / 621, 8192^3 5030 / 5004): the measuring pass, a copy, wider tiles.
 static bool pairs_are_faster(long m, long n, long k) {
   if (4. * (double)k * (double)(m + n) > 16e9 || std::max(std::max(m, n), k) > 1l << 28) return false;
