@@ -24,11 +24,11 @@
 //
 // 16-bit operands of either kind: the loads of both CTAs complete on CTA 0's `full` barrier directly, tiles of up to 128 columns have
 // four accumulator buffers (they end an item every few microseconds, and the MMAs run on while its results are stored), and
-// the thread that issues the loads carries its coordinates on by additions.  A relayed barrier, two
+// the warp that issues the loads carries its coordinates on by additions.  A relayed barrier, two
 // buffers and divisions for every load took, at 1024 images: first layer forward 1121 -> 986 us, its weight gradient 971 -> 728,
 // gradInput 64 <- 192 1625 -> 1525, the 256-wide weight gradients 357 -> 340; 128 images 3207 -> 3115 us a step.
 //
-// BF16 (opt-in math mode): no splitters and no lo slots, four kind::f16 MMAs per 64-k tile, one MMA thread; products are exact
+// BF16 (opt-in math mode): no splitters and no lo slots, four kind::f16 MMAs per 64-k tile; products are exact
 // in FP32 and the tolerance of the mode is BF16's, so four k tiles (16 MMAs) chain in one accumulator before a drain.  No pipe is
 // full (4096^3: 136 us, 1.0 PFLOP/s, tensor pipe 47 % busy): 7.9 TB/s cross from L2 into the SMs, 64 KB per 256 x 256 x 64
 // step of the pair, near the most any engine here has moved.
@@ -40,10 +40,14 @@
 //   warps 0-3   splitters, two groups of two warps taking alternate k tiles: wait for the tile's TMA bytes
 //               (`raw_full`, CTA-local) and for its lo slot to be free, split, publish to the async proxy,
 //               arrive on CTA 0's `full`.
-//   warps 4, 6  (CTA 0) one MMA-issuing thread each, for the even and the odd k tiles.
-//   warp 5      one thread per CTA issues the TMA loads of this CTA's A rows and B rows, R - 1 tiles ahead,
+//   warps 4, 6  (CTA 0) issue the MMAs of the even and the odd k tiles (16-bit operands: warp 4 all).
+//   warp 5      issues the TMA loads of this CTA's A rows and B rows, R - 1 tiles ahead,
 //               as soon as the MMAs that read a slot have completed (`empty`).
 //   warps 8-15  drain: tcgen05.ld every finished partial tile and add it into FP32 registers; then the epilogue.
+// The issuing warps run their loops with all lanes and elect a thread for each tile's instructions (elect_one, mm_tc.cuh).  With a
+// single thread in the loop the MMAs of narrow tiles were bound by their issue: 512 images, forward 64 -> 192 (192 columns) 596 -> 500
+// us, gradInput 64 <- 192 (pixel pairs, 128) 839 -> 645, 64 -> 128 of 112 x 112 (128) 399 -> 320, in BF16 278 -> 240 and (64 columns)
+// 566 -> 464; tiles of 256 columns, which the power cap holds, 3 %.
 // Registers are rebalanced with setmaxnreg: the drain warps hold BN2/2 accumulators per thread.
 // The kernel is persistent: see tc2r_kernel.
 // Every wait is bounded; on expiry the CTA tells its peer, raises the stall flags (StallCtl, mm_tc.cuh), skips
@@ -117,7 +121,7 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst, const void *tmap, int 
       : "memory");
 }
 // The loads of one CTA's share of an operand, ROWS rows from row0 on, k tile after k tile.  PREC: the form the operand's buffer is in;
-// `lo`: the second half of a pair.  One thread issues them all, and what it does between two loads is on the engine's
+// `lo`: the second half of a pair.  One warp issues them all, and what it does between two loads is on the engine's
 // critical path: coordinates are found by division once per item and carried on by additions.
 template <int ROWS, int PREC, bool WIDE, class Op> struct TileLoader;
 template <int ROWS, int PREC, bool WIDE, bool MN, int OWN>
@@ -263,7 +267,7 @@ __device__ __forceinline__ void tc2r_run(const P &p, const StallCtl &ctl, unsign
   uint32_t *sched_ring = tmem_slot + 2 + sizeof(WaitCtl) / 4;
   static_assert((3 * R + 2 * ACCS + L + 2 * T2R_SCHED + 1) * 8 + 8 + sizeof(WaitCtl) + 4 * T2R_SCHED <= 512, "auxiliary shared memory");
 
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;   // warp: as a value that a warp has once
   const uint32_t rank = cluster_ctarank();
   // item counts fit 32 bits (checked by the launcher): the decode below runs once per item in every role
   const uint32_t gm = (uint32_t)((p.M + 255) / 256), gn = (uint32_t)((p.N + BN2 - 1) / BN2);
@@ -382,17 +386,18 @@ __device__ __forceinline__ void tc2r_run(const P &p, const StallCtl &ctl, unsign
     }
   } else if (warp < T2_DRAIN_WARP0) {
     setmaxnreg_dec<40>();
-    if (HALF && warp == T2_MMA_WARP && lane == 0 && rank == 0) {
-      // ---------------------------------------------------------- MMA issuer of 16-bit operands: one thread, CHAIN k tiles per buffer
+    if (HALF && warp == T2_MMA_WARP && rank == 0) {
+      // ---------------------------------------------------------- MMA issuer of 16-bit operands: one warp, CHAIN k tiles per buffer
       constexpr bool A_MN = P::OpA::MN_MAJOR, B_MN = P::OpB::MN_MAJOR;
       constexpr uint32_t idesc = PAIRS ? umma2_idesc_f16(BN2, A_MN, B_MN) : umma2_idesc_bf16(BN2, A_MN, B_MN);
       const uint32_t ring = smem_u32(smem);
       uint32_t s = 0, phase = 0, buf = 0, acc_phase = 0;
       for (uint32_t n = 0; ok; n++) {
         uint32_t w = T2R_NO_ITEM;
-        ok = sched.next(n, w, abort_flag);
+        ok = __all_sync(0xffffffffu, sched.next(n, w, abort_flag));
         if (!ok) break;
-        sched.done(n);
+        w = __shfl_sync(0xffffffffu, w, 0);
+        if (lane == 0) sched.done(n);
         if (w == T2R_NO_ITEM) break;
         const int nk = item_at(w).num_k_tiles;
         for (int it = 0; it < nk; it++) {
@@ -400,48 +405,50 @@ __device__ __forceinline__ void tc2r_run(const P &p, const StallCtl &ctl, unsign
           const uint32_t d = tmem_base + buf * BN2;
           if (first) ok = mbar_wait_spin(bar_acc_empty + 8 * buf, acc_phase ^ 1u, abort_flag, kWaitAccEmpty);
           ok = ok && mbar_wait_spin(bar_full + 8 * s, phase, abort_flag, kWaitTileFull);
+          const uint32_t sl = s;
           if constexpr (PAIRS) {
-            const uint32_t sl = s;
             if (++s == R) { s = 0; phase ^= 1u; }
             ok = ok && mbar_wait_spin(bar_full + 8 * s, phase, abort_flag, kWaitTileFull);
-            if (!ok) break;
-            tc_fence_after();
-            const uint32_t lo = ring + sl * Cfg::SLOT_BYTES, hi = ring + s * Cfg::SLOT_BYTES;
-            const uint64_t a_lo = umma_desc_half<A_MN>(lo), b_lo = umma_desc_half<B_MN>(lo + Cfg::A_BYTES);
-            const uint64_t a_hi = umma_desc_half<A_MN>(hi), b_hi = umma_desc_half<B_MN>(hi + Cfg::A_BYTES);
-#pragma unroll
-            for (int kk = 0; kk < 4; kk++) {   // 16 k per MMA; these two carry 2^11
-              const uint64_t adv_a = (uint64_t)((kk * umma_kstep_bytes_half<A_MN>()) >> 4), adv_b = (uint64_t)((kk * umma_kstep_bytes_half<B_MN>()) >> 4);
-              umma2_f16(d, a_lo + adv_a, b_hi + adv_b, idesc, kk ? 1u : 0u);
-              umma2_f16(d, a_hi + adv_a, b_lo + adv_b, idesc, 1u);
-            }
-            umma2_commit_both(bar_empty + 8 * sl);
-            umma2_f16_scale11(d, a_hi, b_hi, idesc);
-#pragma unroll
-            for (int kk = 1; kk < 4; kk++)
-              umma2_f16(d, a_hi + (uint64_t)((kk * umma_kstep_bytes_half<A_MN>()) >> 4), b_hi + (uint64_t)((kk * umma_kstep_bytes_half<B_MN>()) >> 4), idesc, 1u);
-          } else {
-            if (!ok) break;
-            tc_fence_after();
-            const uint32_t st = ring + s * Cfg::SLOT_BYTES;
-            const uint64_t a_d = umma_desc_half<A_MN>(st), b_d = umma_desc_half<B_MN>(st + Cfg::A_BYTES);
-#pragma unroll
-            for (int kk = 0; kk < 4; kk++) {   // 16 k per MMA
-              const uint64_t adv_a = (uint64_t)((kk * umma_kstep_bytes_half<A_MN>()) >> 4), adv_b = (uint64_t)((kk * umma_kstep_bytes_half<B_MN>()) >> 4);
-              umma2_f16(d, a_d + adv_a, b_d + adv_b, idesc, (kk || !first) ? 1u : 0u);
-            }
           }
-          umma2_commit_both(bar_empty + 8 * s);
+          ok = __all_sync(0xffffffffu, ok);
+          if (!ok) break;
+          tc_fence_after();
+          if (elect_one()) {
+            if constexpr (PAIRS) {
+              const uint32_t lo = ring + sl * Cfg::SLOT_BYTES, hi = ring + s * Cfg::SLOT_BYTES;
+              const uint64_t a_lo = umma_desc_half<A_MN>(lo), b_lo = umma_desc_half<B_MN>(lo + Cfg::A_BYTES);
+              const uint64_t a_hi = umma_desc_half<A_MN>(hi), b_hi = umma_desc_half<B_MN>(hi + Cfg::A_BYTES);
+#pragma unroll
+              for (int kk = 0; kk < 4; kk++) {   // 16 k per MMA; these two carry 2^11
+                const uint64_t adv_a = (uint64_t)((kk * umma_kstep_bytes_half<A_MN>()) >> 4), adv_b = (uint64_t)((kk * umma_kstep_bytes_half<B_MN>()) >> 4);
+                umma2_f16(d, a_lo + adv_a, b_hi + adv_b, idesc, kk ? 1u : 0u);
+                umma2_f16(d, a_hi + adv_a, b_lo + adv_b, idesc, 1u);
+              }
+              umma2_commit_both(bar_empty + 8 * sl);
+              umma2_f16_scale11(d, a_hi, b_hi, idesc);
+#pragma unroll
+              for (int kk = 1; kk < 4; kk++)
+                umma2_f16(d, a_hi + (uint64_t)((kk * umma_kstep_bytes_half<A_MN>()) >> 4), b_hi + (uint64_t)((kk * umma_kstep_bytes_half<B_MN>()) >> 4), idesc, 1u);
+            } else {
+              const uint32_t st = ring + s * Cfg::SLOT_BYTES;
+              const uint64_t a_d = umma_desc_half<A_MN>(st), b_d = umma_desc_half<B_MN>(st + Cfg::A_BYTES);
+#pragma unroll
+              for (int kk = 0; kk < 4; kk++) {   // 16 k per MMA
+                const uint64_t adv_a = (uint64_t)((kk * umma_kstep_bytes_half<A_MN>()) >> 4), adv_b = (uint64_t)((kk * umma_kstep_bytes_half<B_MN>()) >> 4);
+                umma2_f16(d, a_d + adv_a, b_d + adv_b, idesc, (kk || !first) ? 1u : 0u);
+              }
+            }
+            umma2_commit_both(bar_empty + 8 * s);
+            if (last) umma2_commit_both(bar_acc_full + 8 * buf);
+          }
+          __syncwarp();
           if (++s == R) { s = 0; phase ^= 1u; }
-          if (last) {
-            umma2_commit_both(bar_acc_full + 8 * buf);
-            if (++buf == ACCS) { buf = 0; acc_phase ^= 1u; }
-          }
+          if (last && ++buf == ACCS) { buf = 0; acc_phase ^= 1u; }
         }
       }
-    } else if (!HALF && (warp == T2_MMA_WARP || warp == T2R_MMA_WARP2) && lane == 0 && rank == 0) {
+    } else if (!HALF && (warp == T2_MMA_WARP || warp == T2R_MMA_WARP2) && rank == 0) {
       // ---------------------------------------------------------- MMA issuers
-      // Two threads take alternate k tiles (and with them alternate accumulator buffers): while one is blocked on
+      // Two warps take alternate k tiles (and with them alternate accumulator buffers): while one is blocked on
       // the tensor pipe's queue the other sits through its barrier polls, each a shared-memory round trip of
       // hundreds of cycles under the MMAs' own traffic.
       // With an odd number of hi slots a thread meets a slot only every second time round, so its parity wait for
@@ -456,9 +463,10 @@ __device__ __forceinline__ void tc2r_run(const P &p, const StallCtl &ctl, unsign
       int g0 = 0;
       for (uint32_t n = 0; ok; n++) {
         uint32_t w = T2R_NO_ITEM;
-        ok = sched.next(n, w, abort_flag);
+        ok = __all_sync(0xffffffffu, sched.next(n, w, abort_flag));
         if (!ok) break;
-        sched.done(n);
+        w = __shfl_sync(0xffffffffu, w, 0);
+        if (lane == 0) sched.done(n);
         if (w == T2R_NO_ITEM) break;
         const int nk = item_at(w).num_k_tiles;
         for (int it = (g0 + buf) & 1; it < nk; it += 2) {
@@ -466,34 +474,37 @@ __device__ __forceinline__ void tc2r_run(const P &p, const StallCtl &ctl, unsign
           const int s = g % R, ls = g % LM;
           const uint32_t phase = (uint32_t)(g / R) & 1u, acc_phase = (uint32_t)(g >> 1) & 1u;
           ok = mbar_wait_spin(bar_acc_empty + 8 * buf, acc_phase ^ 1u, abort_flag, kWaitAccEmpty);
-          ok = ok && mbar_wait_spin(bar_full + 8 * s, phase, abort_flag, kWaitTileFull);
+          ok = __all_sync(0xffffffffu, ok && mbar_wait_spin(bar_full + 8 * s, phase, abort_flag, kWaitTileFull));
           if (!ok) break;
           tc_fence_after();
-          const uint32_t hs = smem_u32(smem + s * Cfg::SLOT_BYTES), lsl = smem_u32(lo_ring + ls * Cfg::SLOT_BYTES);
-          const uint64_t a_hi = umma_desc_sw128<A_MN>(hs), a_lo = umma_desc_sw128<A_MN>(lsl);
-          const uint64_t b_hi = umma_desc_sw128<B_MN>(hs + Cfg::A_BYTES), b_lo = umma_desc_sw128<B_MN>(lsl + Cfg::A_BYTES);
-          const uint32_t d = tmem_base + (uint32_t)(buf * BN2);
+          if (elect_one()) {
+            const uint32_t hs = smem_u32(smem + s * Cfg::SLOT_BYTES), lsl = smem_u32(lo_ring + ls * Cfg::SLOT_BYTES);
+            const uint64_t a_hi = umma_desc_sw128<A_MN>(hs), a_lo = umma_desc_sw128<A_MN>(lsl);
+            const uint64_t b_hi = umma_desc_sw128<B_MN>(hs + Cfg::A_BYTES), b_lo = umma_desc_sw128<B_MN>(lsl + Cfg::A_BYTES);
+            const uint32_t d = tmem_base + (uint32_t)(buf * BN2);
 #pragma unroll
-          for (int kk = 0; kk < 4; kk++) {   // 8 k per MMA
-            const uint64_t adv_a = (uint64_t)((kk * umma_kstep_bytes<A_MN>()) >> 4);
-            const uint64_t adv_b = (uint64_t)((kk * umma_kstep_bytes<B_MN>()) >> 4);
-            umma2_tf32(d, a_lo + adv_a, b_hi + adv_b, idesc, kk ? 1u : 0u);
-            umma2_tf32(d, a_hi + adv_a, b_lo + adv_b, idesc, 1u);
-          }
+            for (int kk = 0; kk < 4; kk++) {   // 8 k per MMA
+              const uint64_t adv_a = (uint64_t)((kk * umma_kstep_bytes<A_MN>()) >> 4);
+              const uint64_t adv_b = (uint64_t)((kk * umma_kstep_bytes<B_MN>()) >> 4);
+              umma2_tf32(d, a_lo + adv_a, b_hi + adv_b, idesc, kk ? 1u : 0u);
+              umma2_tf32(d, a_hi + adv_a, b_lo + adv_b, idesc, 1u);
+            }
 #pragma unroll
-          for (int kk = 0; kk < 4; kk++) {   // 8 k per MMA
-            const uint64_t adv_a = (uint64_t)((kk * umma_kstep_bytes<A_MN>()) >> 4);
-            const uint64_t adv_b = (uint64_t)((kk * umma_kstep_bytes<B_MN>()) >> 4);
-            umma2_tf32(d, a_hi + adv_a, b_hi + adv_b, idesc, 1u);
+            for (int kk = 0; kk < 4; kk++) {   // 8 k per MMA
+              const uint64_t adv_a = (uint64_t)((kk * umma_kstep_bytes<A_MN>()) >> 4);
+              const uint64_t adv_b = (uint64_t)((kk * umma_kstep_bytes<B_MN>()) >> 4);
+              umma2_tf32(d, a_hi + adv_a, b_hi + adv_b, idesc, 1u);
+            }
+            umma2_commit_both(bar_empty + 8 * s);
+            umma2_commit_both(bar_lo_empty + 8 * ls);
+            umma2_commit_both(bar_acc_full + 8 * buf);
           }
-          umma2_commit_both(bar_empty + 8 * s);
-          umma2_commit_both(bar_lo_empty + 8 * ls);
-          umma2_commit_both(bar_acc_full + 8 * buf);
+          __syncwarp();
         }
         g0 += nk;
       }
-    } else if (warp == T2R_TMA_WARP && lane == 0) {
-      // ---------------------------------------------------------- TMA issuer (one per CTA)
+    } else if (warp == T2R_TMA_WARP) {
+      // ---------------------------------------------------------- TMA issuer (one warp per CTA)
       // 16-bit tiles are ready as they land: the bytes of both CTAs complete on CTA 0's `full`.  The peer's may come before CTA 0 has
       // announced them: the phase still waits for that arrival, and the peer's slot was free only after the phase before.
       const uint32_t full_leader = mapa_shared(bar_full, 0), ring = smem_u32(smem);
@@ -501,11 +512,12 @@ __device__ __forceinline__ void tc2r_run(const P &p, const StallCtl &ctl, unsign
       bool filled = false;   // every slot has been used
       for (uint32_t n = 0; ok; n++) {
         uint32_t w = T2R_NO_ITEM;
-        ok = sched.next(n, w, abort_flag);
+        ok = __all_sync(0xffffffffu, sched.next(n, w, abort_flag));
         if (!ok) break;
-        sched.done(n);
+        w = __shfl_sync(0xffffffffu, w, 0);
+        if (lane == 0) sched.done(n);
         if (w == T2R_NO_ITEM) break;
-        if (rank == 0) mbar_arrive_local(bar_sched_go);   // item n is under way: time to fetch the number of item n + 1
+        if (rank == 0 && lane == 0) mbar_arrive_local(bar_sched_go);   // item n is under way: time to fetch the number of item n + 1
         const Tc2rItem item = item_at(w);
         TileLoader<TC_BM, PREC, WIDE, typename P::OpA> load_a(p.a, item.m_tile0 + (long)rank * TC_BM, item.k_begin);
         TileLoader<BH, PREC, WIDE, typename P::OpB> load_b(p.b, item.n_tile0 + (long)rank * BH, item.k_begin);
@@ -513,24 +525,28 @@ __device__ __forceinline__ void tc2r_run(const P &p, const StallCtl &ctl, unsign
 #pragma unroll
           for (int part = 0; part < PARTS; part++) {
             const bool lo = PAIRS && part == 0;
-            if (filled && !mbar_wait(bar_empty + 8 * s, phase ^ 1u, abort_flag, kWaitSlotEmpty)) { ok = false; break; }
-            const uint32_t slot = ring + s * Cfg::SLOT_BYTES;
-            uint32_t landed = bar_raw + 8 * s;
-            if constexpr (HALF) {
-              landed = full_leader + 8 * s;
-              if (rank == 0) mbar_arrive_expect_tx(bar_full + 8 * s, 2u * Cfg::SLOT_BYTES);
-            } else {
-              mbar_arrive_expect_tx(landed, (uint32_t)Cfg::SLOT_BYTES);
+            if (filled) ok = __all_sync(0xffffffffu, mbar_wait(bar_empty + 8 * s, phase ^ 1u, abort_flag, kWaitSlotEmpty));
+            if (!ok) break;
+            if (elect_one()) {
+              const uint32_t slot = ring + s * Cfg::SLOT_BYTES;
+              uint32_t landed = bar_raw + 8 * s;
+              if constexpr (HALF) {
+                landed = full_leader + 8 * s;
+                if (rank == 0) mbar_arrive_expect_tx(bar_full + 8 * s, 2u * Cfg::SLOT_BYTES);
+              } else {
+                mbar_arrive_expect_tx(landed, (uint32_t)Cfg::SLOT_BYTES);
+              }
+              load_a.issue(p.a, slot, lo, landed);
+              load_b.issue(p.b, slot + Cfg::A_BYTES, lo, landed);
             }
-            load_a.issue(p.a, slot, lo, landed);
-            load_b.issue(p.b, slot + Cfg::A_BYTES, lo, landed);
+            __syncwarp();
             if (++s == R) { s = 0; phase ^= 1u; filled = true; }
           }
           load_a.next(p.a);
           load_b.next(p.b);
         }
       }
-    } else if (warp == T2R_SCHED_WARP && lane == 0 && rank == 0) {
+    } else if (warp == T2R_SCHED_WARP && rank == 0 && elect_one()) {
       // ---------------------------------------------------------- item hand-out (one thread per cluster)
       const uint32_t peer_ring = mapa_shared(sched.ring, 1), peer_full = mapa_shared(bar_sched_full, 1);
       for (uint32_t n = 0;; n++) {
