@@ -385,6 +385,13 @@ THC_API int THGPUNN_SpatialMaxPooling_updateGradInput(THGPUTensor *input, THGPUT
 THC_API int THGPUNN_Threshold_updateOutput(THGPUTensor *input, THGPUTensor *output, double threshold, double val);
 THC_API int THGPUNN_Threshold_updateGradInput(THGPUTensor *input, THGPUTensor *gradOutput,
     THGPUTensor *gradInput, double threshold);
+/* A Threshold and the SpatialMaxPooling behind it, both ways: the results of the two entry points above called in turn
+ * (`thresholded` is the first one's output, poolGradInput the second one's gradInput), for windows of 2 x 2 and 3 x 3
+ * at stride 2 in one pass.  What a container may call for two such neighbours; no counterpart function in the reference. */
+THC_API int THGPUNN_Threshold_SpatialMaxPooling_updateOutput(THGPUTensor *input, THGPUTensor *thresholded, THGPUTensor *output,
+    THGPUTensor *indices, double threshold, double val, int kW, int kH, int dW, int dH);
+THC_API int THGPUNN_Threshold_SpatialMaxPooling_updateGradInput(THGPUTensor *input, THGPUTensor *thresholded, THGPUTensor *gradOutput,
+    THGPUTensor *poolGradInput, THGPUTensor *gradInput, THGPUTensor *indices, double threshold, int kW, int kH, int dW, int dH);
 /* Classifier tail: gpunn-impl/LogSoftMax.cpp:116-194, gpunn-impl/ClassNLLCriterion.cpp:96-198
  * (targets are a float GPU tensor of 1-based class ids; loss averaged over the batch). */
 THC_API int THGPUNN_Linear_updateOutput(THGPUTensor *input, THGPUTensor *output, THGPUTensor *weight, THGPUTensor *bias);

@@ -184,6 +184,8 @@ SIGNATURES = {
     "THGPUNN_SpatialMaxPooling_updateOutput": (i, [TP, TP, TP, i, i, i, i]),
     "THGPUNN_SpatialMaxPooling_updateGradInput": (i, [TP, TP, TP, TP, i, i, i, i]),
     "THGPUNN_Threshold_updateOutput": (i, [TP, TP, d, d]), "THGPUNN_Threshold_updateGradInput": (i, [TP, TP, TP, d]),
+    "THGPUNN_Threshold_SpatialMaxPooling_updateOutput": (i, [TP, TP, TP, TP, d, d, i, i, i, i]),
+    "THGPUNN_Threshold_SpatialMaxPooling_updateGradInput": (i, [TP, TP, TP, TP, TP, TP, d, i, i, i, i]),
     "THGPUNN_Linear_updateOutput": (i, [TP, TP, TP, TP]),
     "THGPUNN_LogSoftMax_updateOutput": (i, [TP, TP]), "THGPUNN_LogSoftMax_updateGradInput": (i, [TP, TP, TP, TP]),
     "THGPUNN_ClassNLLCriterion_updateOutput": (i, [TP, TP, TP, i]),

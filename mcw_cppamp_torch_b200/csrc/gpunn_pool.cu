@@ -11,6 +11,7 @@
 // to the CPU result for overlapping windows too.
 #include <algorithm>
 #include <cfloat>
+#include <initializer_list>
 
 #include "thc_internal.h"
 
@@ -139,15 +140,49 @@ static __global__ void __launch_bounds__(256) maxpool_backward_kernel(const floa
 constexpr int kBand = 4;
 struct PoolGeom {
   long planes;
-  int H, W, oH, oW, xtiles, bands;   // bands of output rows (forward) or cell rows (backward)
+  int H, W, oH, oW, xtiles, bands;   // bands of output rows (forward) or cell rows (backward, and forward with a threshold)
+};
+// nn.Threshold and the pooling behind it in one pass (template parameter TH of the kernels below): the thresholded plane, which is the
+// pooling's input, is written while the pooling reads it, and on the way back the pooling's gradInput while the threshold reads it,
+// instead of being written by one kernel and read again by the next.  Every pixel belongs to one band and one lane there, so the
+// tiles cover whole planes and not only the windows.  Bound by HBM: of three passes over the plane forward and four backward one is
+// gone (64 images of 64 x 224 x 224, 2 x 2 windows: 267 + 216 -> 363 us forward, 233 + 365 -> 507 backward).
+struct ThresholdPass {
+  const float *in = nullptr;   // backward: what the threshold was applied to
+  float *out = nullptr;        // forward: the thresholded plane; backward: the threshold's gradInput
+  float th = 0.f, val = 0.f;
+};
+// Rows of pixel pairs, columns 2b and 2b + 1 of each lane, leave as 8-byte accesses: on odd addresses as the pairs one column to the left.
+// Every lane of the group takes part.  `first`: no lane of this tile stores the column to the left; `last`: nor the one to the right.
+template <int LP>
+struct PairStore {
+  float *dst;
+  bool odd;
+  __device__ __forceinline__ explicit PairStore(float *d) : dst(d), odd((reinterpret_cast<uintptr_t>(d) & 4) != 0) {}
+  __device__ __forceinline__ void row(float p0, float p1, bool c0, bool c1, bool first, bool last, int W) {
+    const float left = __shfl_up_sync(0xffffffffu, p1, 1, LP);
+    if (!odd) {
+      if (c1) *reinterpret_cast<float2 *>(dst) = make_float2(p0, p1);
+      else if (c0) dst[0] = p0;
+    } else {
+      if (c0) {
+        if (!first) *reinterpret_cast<float2 *>(dst - 1) = make_float2(left, p0);
+        else dst[0] = p0;
+      }
+      if (c1 && last) dst[1] = p1;
+    }
+    dst += W;
+    odd ^= (W & 1) != 0;
+  }
 };
 
 // Forward.  Lane `sub` owns window column x and reads input columns 2x and 2x + 1 of each row once (column 2x + 2 is the right-hand
 // lane's first); a row's maximum over the window's columns serves both windows it belongs to: 4.5 loads an output where a
 // thread per output issues 9.
-template <int K, int LP>
+template <int K, int LP, bool TH>
 static __global__ void __launch_bounds__(256) maxpool_forward_band_kernel(const float *__restrict__ in, float *__restrict__ out,
-                                                                          float *__restrict__ indy, float *__restrict__ indx, const PoolGeom p) {
+                                                                          float *__restrict__ indy, float *__restrict__ indx, const PoolGeom p,
+                                                                          const ThresholdPass t) {
   pdl_begin();
   constexpr int PPW = 32 / LP, ROWS = 2 * kBand + K - 2;
   const unsigned full = 0xffffffffu;
@@ -174,6 +209,19 @@ static __global__ void __launch_bounds__(256) maxpool_forward_band_kernel(const 
     if (K == 3) {
 #pragma unroll
       for (int k = 0; k < ROWS; k++) c[k] = edge && h0 + k < p.H ? src[k * p.W + 2] : none;
+    }
+    if constexpr (TH) {
+      auto pass = [&](bool there, float v) { return !there || v > t.th ? v : t.val; };
+#pragma unroll
+      for (int k = 0; k < ROWS; k++) {
+        const bool ok = h0 + k < p.H;
+        a[k] = pass(ok && l0, a[k]); b[k] = pass(ok && l1, b[k]);
+        if (K == 3) c[k] = pass(edge && ok, c[k]);
+      }
+      PairStore<LP> store(t.out + (plane * p.H + h0) * (long)p.W + 2 * x);
+#pragma unroll
+      for (int k = 0; k < 2 * kBand; k++)
+        if (h0 + k < p.H) store.row(a[k], b[k], l0, l1, sub == 0, sub == LP - 1 || 2 * x + 2 >= p.W, p.W);
     }
     // maximum and its column of every row of the band (first one wins, NaN never does)
     float m[ROWS];
@@ -213,9 +261,10 @@ static __global__ void __launch_bounds__(256) maxpool_forward_band_kernel(const 
 // the CPU's order of additions (ascending window row, then column), so the result is bit-equal to it.  A row of the result
 // leaves as 8-byte pairs, on odd addresses as the pairs one column to the left.
 // Planes of more than 32 cells: tiles of 31 cells whose first lane holds the window left of the tile.
-template <int LP>
+template <int LP, bool TH>
 static __global__ void __launch_bounds__(256) maxpool3_backward_kernel(const float *__restrict__ gout, const float *__restrict__ indy,
-                                                                       const float *__restrict__ indx, float *__restrict__ gin, const PoolGeom p) {
+                                                                       const float *__restrict__ indx, float *__restrict__ gin, const PoolGeom p,
+                                                                       const ThresholdPass th) {
   pdl_begin();
   constexpr int PPW = 32 / LP;
   const unsigned full = 0xffffffffu;
@@ -241,23 +290,21 @@ static __global__ void __launch_bounds__(256) maxpool3_backward_kernel(const flo
       const long o = w0 + (d - 1) * p.oW;
       iy[d] = ok ? indy[o] : 0.f; ix[d] = ok ? indx[o] : 0.f; v[d] = ok ? gout[o] : 0.f;
     }
-    float *dst = gin + (plane * p.H + 2 * y0) * (long)p.W + 2 * b;
-    bool odd = (reinterpret_cast<uintptr_t>(dst) & 4) != 0;
-    auto put = [&](float p0, float p1) {
-      const float left = __shfl_up_sync(full, p1, 1, LP);
-      if (!odd) {
-        if (c1) *reinterpret_cast<float2 *>(dst) = make_float2(p0, p1);
-        else if (c0) dst[0] = p0;
-      } else {
-        // the pair (2b - 1, 2b); the first lane of a row has no left column, the last column of an even row no right one
-        if (c0) {
-          if (sub > (halo ? 1 : 0)) *reinterpret_cast<float2 *>(dst - 1) = make_float2(left, p0);
-          else dst[0] = p0;
-        }
-        if (c1 && (sub == LP - 1 || 2 * b + 2 >= p.W)) dst[1] = p1;
+    const long at = (plane * p.H + 2 * y0) * (long)p.W + 2 * b;
+    float i0[2 * kBand], i1[2 * kBand];   // TH: what the threshold was applied to
+    if constexpr (TH) {
+#pragma unroll
+      for (int k = 0; k < 2 * kBand; k++) {
+        const bool ok = 2 * y0 + k < p.H;
+        i0[k] = ok && c0 ? th.in[at + k * p.W] : 0.f;
+        i1[k] = ok && c1 ? th.in[at + k * p.W + 1] : 0.f;
       }
-      dst += p.W;
-      odd ^= (p.W & 1) != 0;
+    }
+    PairStore<LP> store(gin + at), store_th(th.out + at);
+    const bool first = sub <= (halo ? 1 : 0), last = sub == LP - 1 || 2 * b + 2 >= p.W;
+    auto put = [&](int k, float p0, float p1) {
+      store.row(p0, p1, c0, c1, first, last, p.W);
+      if constexpr (TH) store_th.row(i0[k] > th.th ? p0 : 0.f, i1[k] > th.th ? p1 : 0.f, c0, c1, first, last, p.W);
     };
     auto add = [](float acc, bool hit, float x) { return hit ? acc + x : acc; };
     float pt = fmaf(3.f, iy[0], ix[0]), pv = v[0];
@@ -274,8 +321,8 @@ static __global__ void __launch_bounds__(256) maxpool3_backward_kernel(const flo
       const float p01 = add(add(0.f, pt == 11.f, pv), t == 5.f, x);
       const float p10 = add(add(0.f, lt == 9.f, lx), t == 7.f, x);
       const float p11 = add(0.f, t == 8.f, x);
-      put(p00, p01);
-      if (2 * (y0 + d - 1) + 1 < p.H) put(p10, p11);
+      put(2 * d - 2, p00, p01);
+      if (2 * (y0 + d - 1) + 1 < p.H) put(2 * d - 1, p10, p11);
       pt = t; pv = x; plt = lt; plv = lx;
     }
   }
@@ -283,10 +330,11 @@ static __global__ void __launch_bounds__(256) maxpool3_backward_kernel(const flo
 
 // Backward for windows of 2 x 2 at stride 2: every pixel belongs to one window.  A thread owns V neighbouring windows and writes
 // their 2 x 2V pixels (V = 2 where 16-byte stores are possible); rows and columns below and right of the last window are zero.
-template <int V>
+template <int V, bool TH>
 static __global__ void __launch_bounds__(256) maxpool2_backward_kernel(const float *__restrict__ gout, const float *__restrict__ indy,
                                                                        const float *__restrict__ indx, float *__restrict__ gin, long rows,
-                                                                       int H, int W, int oH, int oW, int cells_h, int cells_w, Div32 dcw) {
+                                                                       int H, int W, int oH, int oW, int cells_h, int cells_w, Div32 dcw,
+                                                                       const ThresholdPass th) {
   pdl_begin();
   // rows = planes * cells_h; a cell row has cells_w / V items
   const int per = cells_w / V;
@@ -297,7 +345,30 @@ static __global__ void __launch_bounds__(256) maxpool2_backward_kernel(const flo
       const int x = (int)(t - q * per) * V;
       const long row = row0 * 64 + q, plane = row / cells_h;
       const int y = (int)(row - plane * cells_h);
-      float top[2 * V], low[2 * V];
+      const long at = (plane * H + 2 * y) * (long)W + 2 * x;
+      const bool second = V == 2 || 2 * x + 1 < W, below = 2 * y + 1 < H;
+      float top[2 * V], low[2 * V], in_top[2 * V], in_low[2 * V];   // in_*, TH: what the threshold was applied to
+      auto load = [&](const float *s, float (&v)[2 * V]) {
+        if constexpr (V == 2) {
+          const float4 f = *reinterpret_cast<const float4 *>(s);
+          v[0] = f.x; v[1] = f.y; v[2] = f.z; v[3] = f.w;
+        } else {
+          v[0] = s[0];
+          v[1] = second ? s[1] : 0.f;
+        }
+      };
+      auto store = [&](float *d, const float (&v)[2 * V]) {
+        if constexpr (V == 2) {
+          *reinterpret_cast<float4 *>(d) = make_float4(v[0], v[1], v[2], v[3]);
+        } else {
+          d[0] = v[0];
+          if (second) d[1] = v[1];
+        }
+      };
+      if constexpr (TH) {
+        load(th.in + at, in_top);
+        if (below) load(th.in + at + W, in_low);
+      }
 #pragma unroll
       for (int k = 0; k < V; k++) {
         float iy = 0.f, ix = 0.f, v = 0.f;
@@ -309,26 +380,267 @@ static __global__ void __launch_bounds__(256) maxpool2_backward_kernel(const flo
         top[2 * k] = iy == 1.f && ix == 1.f ? v : 0.f; top[2 * k + 1] = iy == 1.f && ix == 2.f ? v : 0.f;
         low[2 * k] = iy == 2.f && ix == 1.f ? v : 0.f; low[2 * k + 1] = iy == 2.f && ix == 2.f ? v : 0.f;
       }
-      float *d = gin + (plane * H + 2 * y) * (long)W + 2 * x;
-      if constexpr (V == 2) {
-        *reinterpret_cast<float4 *>(d) = make_float4(top[0], top[1], top[2], top[3]);
-        if (2 * y + 1 < H) *reinterpret_cast<float4 *>(d + W) = make_float4(low[0], low[1], low[2], low[3]);
-      } else {
-        const bool second = 2 * x + 1 < W;
-        d[0] = top[0];
-        if (second) d[1] = top[1];
-        if (2 * y + 1 < H) {
-          d[W] = low[0];
-          if (second) d[W + 1] = low[1];
-        }
+      store(gin + at, top);
+      if (below) store(gin + at + W, low);
+      if constexpr (TH) {
+#pragma unroll
+        for (int k = 0; k < 2 * V; k++) { top[k] = in_top[k] > th.th ? top[k] : 0.f; low[k] = below && in_low[k] > th.th ? low[k] : 0.f; }
+        store(th.out + at, top);
+        if (below) store(th.out + at + W, low);
       }
     }
   }
 }
 
+// ---- the same windows over small planes -----------------------------------------------------------------------------------
+// A block takes G whole planes, one stretch of memory, through shared memory: whatever the width, global memory is read and written in
+// 16-byte pieces of that stretch.  Bound by HBM and by the barriers between a block's passes, of which other blocks of the SM make use.  The
+// kernels by rows touch parts of sectors and lines at both ends of a row, which costs most on short rows and, once the tensors have
+// left L2, in DRAM.  Threshold and 3 x 3 pooling in one pass, by rows -> by planes (us; the bytes at the copy rate): 65536 planes of
+// 55 x 55 forward 462 -> 415 (330), backward 584 -> 476 (452); 196608 of 27 x 27 440 -> 296 (236), 600 -> 371 (324); 262144 of 13 x 13
+// 150 -> 93 (72), 194 -> 125 (99).
+struct PlaneGeom {
+  long planes;
+  int G, H, W, HW, oH, oW, P;
+  Div32 dP, doW;                    // outputs of a plane, of a row
+  int cells, cw, ring;              // backward: 2 x 2 cells of a plane and of a row; windows of a plane with a ring of empty ones around
+  Div32 dcells, dcw, dring, dS;
+};
+constexpr int kPlanePieces = 4;   // 16-byte pieces of a thread in the backward kernel: at most 4096 pixels a group
+// f(i, n): global elements i .. i + n of [start, end), n = 4 on 16-byte boundaries, 1 at the ends; `U` pieces of a thread at once
+// (load, then use).
+template <int U, class Load, class Use>
+__device__ __forceinline__ void stretch(long start, long end, Load load, Use use) {
+  const long first = (start + 3) & ~3l, last = end & ~3l;
+  for (long i0 = first + 4l * threadIdx.x; i0 < last; i0 += 4l * U * blockDim.x) {
+    float4 v[U];
+#pragma unroll
+    for (int u = 0; u < U; u++)
+      if (i0 + 4l * u * blockDim.x < last) v[u] = load(i0 + 4l * u * blockDim.x);
+#pragma unroll
+    for (int u = 0; u < U; u++)
+      if (i0 + 4l * u * blockDim.x < last) use(i0 + 4l * u * blockDim.x, v[u]);
+  }
+}
+// the up to three elements on either side of the 16-byte pieces
+template <class One>
+__device__ __forceinline__ void stretch_ends(long start, long end, One one) {
+  const long first = min((start + 3) & ~3l, end), last = max(end & ~3l, first);
+  const int t = threadIdx.x;
+  if (t < first - start) one(start + t);
+  if (t >= 32 && t - 32 < end - last) one(last + t - 32);
+}
+
+template <int K, bool TH>
+static __global__ void __launch_bounds__(256) maxpool_forward_planes_kernel(const float *__restrict__ in, float *__restrict__ out,
+                                                                            float *__restrict__ indy, float *__restrict__ indx, const PlaneGeom q,
+                                                                            const ThresholdPass t) {
+  pdl_begin();
+  extern __shared__ float4 planes_sm[];
+  float *sm = reinterpret_cast<float *>(planes_sm);
+  const long groups = (q.planes + q.G - 1) / q.G;
+  auto pass = [&](float v) { return !TH || v > t.th ? v : t.val; };
+  for (long g = blockIdx.x; g < groups; g += gridDim.x) {
+    const long p0 = g * q.G, start = p0 * q.HW;
+    const int np = (int)min((long)q.G, q.planes - p0);
+    const long end = start + (long)np * q.HW, base = start & ~3l;
+    stretch<8>(start, end, [&](long i) { return __ldg(reinterpret_cast<const float4 *>(in + i)); }, [&](long i, float4 v) {
+      v = make_float4(pass(v.x), pass(v.y), pass(v.z), pass(v.w));
+      if (TH) *reinterpret_cast<float4 *>(t.out + i) = v;
+      *reinterpret_cast<float4 *>(sm + (i - base)) = v;
+    });
+    stretch_ends(start, end, [&](long i) {
+      const float v = pass(in[i]);
+      if (TH) t.out[i] = v;
+      sm[i - base] = v;
+    });
+    __syncthreads();
+    const float *src = sm + (start - base);
+    for (unsigned o = threadIdx.x; o < (unsigned)(np * q.P); o += blockDim.x) {
+      const unsigned pl = q.dP.div(o), r = o - pl * q.P, y = q.doW.div(r), x = r - y * q.oW;
+      const float *w = src + pl * q.HW + 2 * y * q.W + 2 * x;
+      float best = -INFINITY;   // as in the kernels above, nothing found included
+      int bi = 0, bj = -1;
+#pragma unroll
+      for (int i = 0; i < K; i++)
+#pragma unroll
+        for (int j = 0; j < K; j++) {
+          const float v = w[i * q.W + j];
+          if (v > best) { best = v; bi = i; bj = j; }
+        }
+      const long at = p0 * q.P + o;
+      out[at] = best;
+      indy[at] = (float)(bi + 1);
+      indx[at] = (float)(bj + 1);
+    }
+    __syncthreads();
+  }
+}
+// The windows' targets and values go to shared memory first, in a ring of empty windows; a thread then makes the four pixels of a cell from
+// the four windows that reach it (see maxpool3_backward_kernel; 2 x 2 windows: from the one), and the pixels leave as one stretch.
+template <int K, bool TH>
+static __global__ void __launch_bounds__(256) maxpool_backward_planes_kernel(const float *__restrict__ gout, const float *__restrict__ indy,
+                                                                             const float *__restrict__ indx, float *__restrict__ gin, const PlaneGeom q,
+                                                                             const ThresholdPass th) {
+  pdl_begin();
+  extern __shared__ float4 planes_sm[];
+  float *px = reinterpret_cast<float *>(planes_sm);
+  float2 *win = reinterpret_cast<float2 *>(px + (q.G * q.HW + 7) / 4 * 4);
+  const long groups = (q.planes + q.G - 1) / q.G;
+  const int S = q.oW + 2;
+  for (long g = blockIdx.x; g < groups; g += gridDim.x) {
+    const long p0 = g * q.G, start = p0 * q.HW;
+    const int np = (int)min((long)q.G, q.planes - p0);
+    const long end = start + (long)np * q.HW, base = start & ~3l;
+    // every load of the group is under way before the first is waited for
+    const long first = (start + 3) & ~3l, last = end & ~3l;
+    float4 x[kPlanePieces];
+    if constexpr (TH) {
+#pragma unroll
+      for (int u = 0; u < kPlanePieces; u++) {
+        const long i = first + 4l * (threadIdx.x + 256 * u);
+        if (i < last) x[u] = __ldg(reinterpret_cast<const float4 *>(th.in + i));
+      }
+    }
+    const unsigned rings = (unsigned)(np * q.ring);
+    for (unsigned c0 = threadIdx.x; c0 < rings; c0 += 256 * kPlanePieces) {
+      float iy[kPlanePieces], ix[kPlanePieces], v[kPlanePieces];
+#pragma unroll
+      for (int u = 0; u < kPlanePieces; u++) {
+        const unsigned c = c0 + 256 * u, pl = q.dring.div(c), r = c - pl * q.ring, yy = q.dS.div(r), xx = r - yy * S;
+        const bool there = c < rings && yy - 1 < (unsigned)q.oH && xx - 1 < (unsigned)q.oW;
+        const long o = (p0 + pl) * q.P + (int)(yy - 1) * q.oW + (int)(xx - 1);
+        iy[u] = there ? indy[o] : 0.f; ix[u] = there ? indx[o] : 0.f; v[u] = there ? gout[o] : 0.f;
+      }
+#pragma unroll
+      for (int u = 0; u < kPlanePieces; u++)   // 3 * row + column of the target, counted from 1 (4 .. 12; 0: no window), and value
+        if (c0 + 256 * u < rings) win[c0 + 256 * u] = make_float2(fmaf(3.f, iy[u], ix[u]), v[u]);
+    }
+    __syncthreads();
+    auto add = [](float acc, bool hit, float x) { return hit ? acc + x : acc; };
+    for (unsigned c = threadIdx.x; c < (unsigned)(np * q.cells); c += blockDim.x) {
+      const unsigned pl = q.dcells.div(c), r = c - pl * q.cells, cy = q.dcw.div(r), cx = r - cy * q.cw;
+      const float2 *b = win + pl * q.ring + (cy + 1) * S + cx + 1;
+      const float2 w = b[0];
+      float p00, p01, p10, p11;
+      if (K == 3) {
+        const float2 l = b[-1], u = b[-S], ul = b[-S - 1];
+        p00 = add(add(add(add(0.f, ul.x == 12.f, ul.y), u.x == 10.f, u.y), l.x == 6.f, l.y), w.x == 4.f, w.y);
+        p01 = add(add(0.f, u.x == 11.f, u.y), w.x == 5.f, w.y);
+        p10 = add(add(0.f, l.x == 9.f, l.y), w.x == 7.f, w.y);
+        p11 = add(0.f, w.x == 8.f, w.y);
+      } else {
+        p00 = add(0.f, w.x == 4.f, w.y); p01 = add(0.f, w.x == 5.f, w.y);
+        p10 = add(0.f, w.x == 7.f, w.y); p11 = add(0.f, w.x == 8.f, w.y);
+      }
+      float *d = px + (start - base) + pl * q.HW + 2 * cy * q.W + 2 * cx;
+      const bool right = 2 * cx + 1 < (unsigned)q.W, below = 2 * cy + 1 < (unsigned)q.H;
+      d[0] = p00;
+      if (right) d[1] = p01;
+      if (below) d[q.W] = p10;
+      if (below && right) d[q.W + 1] = p11;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int u = 0; u < kPlanePieces; u++) {
+      const long i = first + 4l * (threadIdx.x + 256 * u);
+      if (i >= last) break;
+      float4 v = *reinterpret_cast<const float4 *>(px + (i - base));
+      *reinterpret_cast<float4 *>(gin + i) = v;
+      if constexpr (TH) {
+        v = make_float4(x[u].x > th.th ? v.x : 0.f, x[u].y > th.th ? v.y : 0.f, x[u].z > th.th ? v.z : 0.f, x[u].w > th.th ? v.w : 0.f);
+        *reinterpret_cast<float4 *>(th.out + i) = v;
+      }
+    }
+    stretch_ends(start, end, [&](long i) {
+      const float v = px[i - base];
+      gin[i] = v;
+      if (TH) th.out[i] = th.in[i] > th.th ? v : 0.f;
+    });
+    __syncthreads();
+  }
+}
+// Planes per block, or G = 0 where the kernels by rows do better (us, by rows / by planes, threshold included).
+//   Few pixels: 1024 planes of 55 x 55 (3.1 M) forward 10.4 / 10.9, 8192 (25 M) 63.5 / 58.4; 174 of 43 x 35 backward 6.6 / 7.1.
+//   Forward: rows of more than 32 that start on 8-byte boundaries; 56 116 / 143 (its columns meet in the same banks), 62 12.4 / 13.1,
+//     54 114.6 / 105.5 (3 x 3) and 94 / 96 (2 x 2); 28 67 / 59, 101 225 / 183, 107 x 109 69 / 55.
+//   Backward: 3 x 3 by planes wherever a group fits; 28 82 / 71, 56 144 / 120.  2 x 2 by rows, which leave in whole sectors for
+//     widths of whole 16-byte pieces and meet in L2 otherwise, as long as the tensors stay there: 28 63 / 78, 14 17.7 / 22, 24576 of 27 x 27 (18 M pixels)
+//     48 / 53, 196608 (143 M) 418 / 354, 65536 of 55 x 55 570 / 468, 262144 of 13 x 13 122 / 129, 16384 of 54 x 54 (48 M) 130 / 119.
+static PlaneGeom plane_geom(long planes, long H, long W, long oH, long oW, int k, bool backward, size_t &smem) {
+  PlaneGeom q = {};
+  q.planes = planes; q.H = (int)H; q.W = (int)W; q.HW = (int)std::min(H * W, 1l << 30); q.oH = (int)oH; q.oW = (int)oW; q.P = (int)(oH * oW);
+  const long ch = (H + 1) / 2, cw = (W + 1) / 2, ring = (oH + 2) * (oW + 2), bytes = 4 * H * W + (backward ? 8 * ring : 0), pixels = planes * H * W;
+  if (bytes > 47 * 1024 || pixels < 4l << 20) return q;
+  if (!backward && W > 32 && W % 2 == 0) return q;
+  if (backward && H * W > 1024 * kPlanePieces) return q;
+  if (backward && k == 2 && (W % 4 == 0 || W <= 16 || pixels < 40l << 20)) return q;
+  q.G = (int)std::max(1l, std::min(backward ? std::min(1024 * kPlanePieces / (H * W), 47 * 1024 / bytes) : 24 * 1024 / bytes, planes / (4l * ctx().sm_count)));
+  q.cells = (int)(ch * cw); q.cw = (int)cw; q.ring = (int)ring;
+  q.dP = Div32::make(q.P); q.doW = Div32::make(oW); q.dcells = Div32::make(q.cells); q.dcw = Div32::make(cw); q.dring = Div32::make(ring); q.dS = Div32::make(oW + 2);
+  smem = (size_t)(4 * ((q.G * q.HW + 7) / 4 * 4) + (backward ? 8l * q.G * ring : 0));
+  return q;
+}
+static unsigned plane_blocks(const PlaneGeom &q) { return (unsigned)std::min((q.planes + q.G - 1) / q.G, (long)ctx().sm_count * 64); }
+
 static unsigned band_blocks(const PoolGeom &p, int planes_per_warp) {
   const long items = (p.planes + planes_per_warp - 1) / planes_per_warp * p.xtiles * p.bands;
   return (unsigned)std::min((items + 7) / 8, (long)ctx().sm_count * 64);
+}
+// The 2 x 2 and 3 x 3 windows at stride 2, behind a threshold (TH) or by themselves.
+template <bool TH>
+static void forward_bands(const float *src, float *o, float *iy, float *ix, long planes, long H, long W, long oH, long oW, int k, const ThresholdPass &t) {
+  size_t smem = 0;
+  const PlaneGeom q = plane_geom(planes, H, W, oH, oW, k, false, smem);
+  if (q.G && (((uintptr_t)src | (uintptr_t)t.out) & 15) == 0) {
+    auto go = [&](auto kernel) { pdl_launch(kernel, plane_blocks(q), 256, smem, src, o, iy, ix, q, t); };
+    if (k == 3) go(maxpool_forward_planes_kernel<3, TH>); else go(maxpool_forward_planes_kernel<2, TH>);
+    check_launch("maxpool_forward");
+    return;
+  }
+  // lanes per plane: as many as it has window columns, up to a warp; wider planes are cut into tiles of 32 columns
+  const long cells_h = (H + 1) / 2, cells_w = (W + 1) / 2;
+  const int LP = cells_w <= 8 ? 8 : cells_w <= 16 ? 16 : 32;
+  const PoolGeom pg{planes, (int)H, (int)W, (int)oH, (int)oW, (int)(((TH ? cells_w : oW) + LP - 1) / LP), (int)(((TH ? cells_h : oH) + kBand - 1) / kBand)};
+  auto go = [&](auto kernel) { pdl_launch(kernel, band_blocks(pg, 32 / LP), 256, 0, src, o, iy, ix, pg, t); };
+  if (k == 3) { if (LP == 8) go(maxpool_forward_band_kernel<3, 8, TH>); else if (LP == 16) go(maxpool_forward_band_kernel<3, 16, TH>); else go(maxpool_forward_band_kernel<3, 32, TH>); }
+  else { if (LP == 8) go(maxpool_forward_band_kernel<2, 8, TH>); else if (LP == 16) go(maxpool_forward_band_kernel<2, 16, TH>); else go(maxpool_forward_band_kernel<2, 32, TH>); }
+  check_launch("maxpool_forward");
+}
+static bool banded(int kW, int kH, int dW, int dH) { return dH == 2 && dW == 2 && kH == kW && (kH == 2 || kH == 3); }
+// False: windows or sizes of another kind, nothing has been done.
+template <bool TH>
+static bool backward_cells(const float *g, const float *iy, const float *ix, float *gi, long planes, long H, long W, long oH, long oW, int k,
+                           const ThresholdPass &t) {
+  size_t smem = 0;
+  const PlaneGeom q = plane_geom(planes, H, W, oH, oW, k, true, smem);
+  if (q.G && (((uintptr_t)gi | (uintptr_t)t.in | (uintptr_t)t.out) & 15) == 0) {
+    auto go = [&](auto kernel) { pdl_launch(kernel, plane_blocks(q), 256, smem, g, iy, ix, gi, q, t); };
+    if (k == 3) go(maxpool_backward_planes_kernel<3, TH>); else go(maxpool_backward_planes_kernel<2, TH>);
+    check_launch("maxpool_backward");
+    return true;
+  }
+  const long cells_h = (H + 1) / 2, cells_w = (W + 1) / 2;
+  if (k == 3) {
+    const int LP = cells_w <= 8 ? 8 : cells_w <= 16 ? 16 : 32;
+    const int xtiles = cells_w <= 32 ? 1 : (int)((cells_w + 30) / 31);
+    const PoolGeom pg{planes, (int)H, (int)W, (int)oH, (int)oW, xtiles, (int)((cells_h + kBand - 1) / kBand)};
+    auto go = [&](auto kernel) { pdl_launch(kernel, band_blocks(pg, 32 / LP), 256, 0, g, iy, ix, gi, pg, t); };
+    if (LP == 8) go(maxpool3_backward_kernel<8, TH>); else if (LP == 16) go(maxpool3_backward_kernel<16, TH>); else go(maxpool3_backward_kernel<32, TH>);
+    check_launch("maxpool_backward");
+    return true;
+  }
+  if (cells_w >= (1l << 24)) return false;
+  const bool vec = W % 4 == 0 && (((uintptr_t)gi | (uintptr_t)t.in | (uintptr_t)t.out) & 15) == 0;
+  const long rows = planes * cells_h, per = vec ? cells_w / 2 : cells_w;
+  const unsigned bx = (unsigned)std::min<long>((64 * per + 255) / 256, 16);
+  const unsigned by = (unsigned)std::min<long>((rows + 63) / 64, std::max<long>(1, ctx().sm_count * 32l / bx));
+  auto go = [&](auto kernel) {
+    pdl_launch(kernel, dim3(bx, by), 256, 0, g, iy, ix, gi, rows, (int)H, (int)W, (int)oH, (int)oW, (int)cells_h, (int)cells_w, Div32::make(per), t);
+  };
+  if (vec) go(maxpool2_backward_kernel<2, TH>); else go(maxpool2_backward_kernel<1, TH>);
+  check_launch("maxpool_backward");
+  return true;
 }
 static dim3 plane_grid(long planes, long per_plane) {
   long gx = (per_plane + 255) / 256;
@@ -416,20 +728,13 @@ THC_API int THGPUNN_SpatialMaxPooling_updateOutput(THGPUTensor *input, THGPUTens
   if (total > 0) {
     const float *src = data_ptr(in);
     float *o = data_ptr(output), *iy = data_ptr(indices), *ix = iy + total;
-    if (dH == 2 && dW == 2 && kH == kW && (kH == 2 || kH == 3)) {
-      // lanes per plane: as many as it has window columns, up to a warp; wider planes are cut into tiles of 32 columns
-      const int LP = (W + 1) / 2 <= 8 ? 8 : (W + 1) / 2 <= 16 ? 16 : 32;
-      const int xtiles = (int)((oW + LP - 1) / LP);
-      const PoolGeom pg{N * C, (int)H, (int)W, (int)oH, (int)oW, xtiles, (int)((oH + kBand - 1) / kBand)};
-#define THC_POOL_FWD(K, LPV) pdl_launch(maxpool_forward_band_kernel<K, LPV>, band_blocks(pg, 32 / LP), 256, 0, src, o, iy, ix, pg)
-      if (kH == 3) { if (LP == 8) THC_POOL_FWD(3, 8); else if (LP == 16) THC_POOL_FWD(3, 16); else THC_POOL_FWD(3, 32); }
-      else { if (LP == 8) THC_POOL_FWD(2, 8); else if (LP == 16) THC_POOL_FWD(2, 16); else THC_POOL_FWD(2, 32); }
-#undef THC_POOL_FWD
+    if (banded(kW, kH, dW, dH)) {
+      forward_bands<false>(src, o, iy, ix, N * C, H, W, oH, oW, kH, {});
     } else {
       pdl_launch(maxpool_forward_kernel, plane_grid(N * C, oH * oW), 256, 0, src, o, iy, ix, N * C, (int)H, (int)W, (int)oH, (int)oW,
                                                                                Div32::make(oW), kH, kW, dH, dW);
+      check_launch("maxpool_forward");
     }
-    check_launch("maxpool_forward");
   }
   return 0;
   THC_END(1)
@@ -455,27 +760,7 @@ THC_API int THGPUNN_SpatialMaxPooling_updateGradInput(THGPUTensor *input, THGPUT
   if (total > 0) {
     const float *g = data_ptr(go), *iy = data_ptr(ind), *ix = iy + ototal;
     float *gi = data_ptr(gradInput);
-    const long cells_h = (H + 1) / 2, cells_w = (W + 1) / 2;
-    if (dH == 2 && dW == 2 && kH == 3 && kW == 3) {
-      const int LP = cells_w <= 8 ? 8 : cells_w <= 16 ? 16 : 32;
-      const int xtiles = cells_w <= 32 ? 1 : (int)((cells_w + 30) / 31);
-      const PoolGeom pg{N * C, (int)H, (int)W, (int)oH, (int)oW, xtiles, (int)((cells_h + kBand - 1) / kBand)};
-#define THC_POOL_BWD3(LPV) pdl_launch(maxpool3_backward_kernel<LPV>, band_blocks(pg, 32 / LP), 256, 0, g, iy, ix, gi, pg)
-      if (LP == 8) THC_POOL_BWD3(8); else if (LP == 16) THC_POOL_BWD3(16); else THC_POOL_BWD3(32);
-#undef THC_POOL_BWD3
-      check_launch("maxpool_backward");
-      return 0;
-    }
-    if (dH == 2 && dW == 2 && kH == 2 && kW == 2 && cells_w < (1l << 24)) {
-      const bool vec = W % 4 == 0 && ((uintptr_t)gi & 15) == 0;
-      const long rows = N * C * cells_h, per = vec ? cells_w / 2 : cells_w;
-      const unsigned bx = (unsigned)std::min<long>((64 * per + 255) / 256, 16);
-      const unsigned by = (unsigned)std::min<long>((rows + 63) / 64, std::max<long>(1, ctx().sm_count * 32l / bx));
-      if (vec) pdl_launch(maxpool2_backward_kernel<2>, dim3(bx, by), 256, 0, g, iy, ix, gi, rows, (int)H, (int)W, (int)oH, (int)oW, (int)cells_h, (int)cells_w, Div32::make(per));
-      else pdl_launch(maxpool2_backward_kernel<1>, dim3(bx, by), 256, 0, g, iy, ix, gi, rows, (int)H, (int)W, (int)oH, (int)oW, (int)cells_h, (int)cells_w, Div32::make(per));
-      check_launch("maxpool_backward");
-      return 0;
-    }
+    if (banded(kW, kH, dW, dH) && backward_cells<false>(g, iy, ix, gi, N * C, H, W, oH, oW, kH, {})) return 0;
     // shared memory holds (position, value) of up to kMaxWin windows per work item
     const int kMaxWin = 5120;
     int G = 1, band_rows = (int)H, bands = 1;
@@ -504,6 +789,76 @@ THC_API int THGPUNN_SpatialMaxPooling_updateGradInput(THGPUTensor *input, THGPUT
     check_launch("maxpool_backward");
   }
   return 0;
+  THC_END(1)
+}
+
+// nn.Threshold followed by nn.SpatialMaxPooling.  What the two entry points in turn give, to the bit, and by them wherever the pass over
+// both does not apply: other windows, strided or overlapping tensors, arguments that one of them refuses.
+static bool own_storage(const THGPUTensor *t, std::initializer_list<const THGPUTensor *> others) {
+  for (const THGPUTensor *o : others)
+    if (o == t || (t->storage && o->storage == t->storage)) return false;
+  return true;
+}
+static bool apart(const float *a, long na, const float *b, long nb) { return a + na <= b || b + nb <= a; }
+static bool pooled_shape(const THGPUTensor *t, int kW, int kH, int dW, int dH, long s[6]) {   // planes, H, W, oH, oW, and N for a batch (else 0)
+  if ((t->nDimension != 3 && t->nDimension != 4) || !banded(kW, kH, dW, dH) || !is_contiguous(t)) return false;
+  const int o = t->nDimension - 3;
+  s[5] = o ? t->size[0] : 0;
+  s[0] = (o ? t->size[0] : 1) * t->size[o]; s[1] = t->size[o + 1]; s[2] = t->size[o + 2];
+  if (s[0] <= 0 || s[1] < kH || s[2] < kW || s[1] * s[2] >= (1l << 31)) return false;
+  s[3] = (s[1] - kH) / 2 + 1; s[4] = (s[2] - kW) / 2 + 1;
+  return true;
+}
+
+THC_API int THGPUNN_Threshold_SpatialMaxPooling_updateOutput(THGPUTensor *input, THGPUTensor *thresholded, THGPUTensor *output, THGPUTensor *indices,
+                                                             double threshold, double val, int kW, int kH, int dW, int dH) {
+  THC_BEGIN
+  long s[6];
+  if (pooled_shape(input, kW, kH, dW, dH, s) && own_storage(thresholded, {input, output, indices}) && own_storage(output, {input, indices}) &&
+      own_storage(indices, {input})) {
+    const long C = s[0] / (s[5] ? s[5] : 1), so[4] = {s[5], C, s[3], s[4]}, si[5] = {2, s[5], C, s[3], s[4]}, si3[4] = {2, C, s[3], s[4]};
+    tensor_resize_as(thresholded, input);
+    if (s[5]) { resize_nd(output, 4, so, nullptr); resize_nd(indices, 5, si, nullptr); }
+    else { resize_nd(output, 3, so + 1, nullptr); resize_nd(indices, 4, si3, nullptr); }
+    const long n = nelem(input), m = nelem(output);
+    const float *x = data_ptr(input);
+    float *r = data_ptr(thresholded), *o = data_ptr(output), *ind = data_ptr(indices);
+    if (is_contiguous(thresholded) && is_contiguous(output) && is_contiguous(indices) && apart(x, n, r, n) && apart(x, n, o, m) && apart(x, n, ind, 2 * m) &&
+        apart(r, n, o, m) && apart(r, n, ind, 2 * m) && apart(o, m, ind, 2 * m)) {
+      forward_bands<true>(x, o, ind, ind + m, s[0], s[1], s[2], s[3], s[4], kH, ThresholdPass{nullptr, r, (float)threshold, (float)val});
+      return 0;
+    }
+  }
+  const int bad = THGPUNN_Threshold_updateOutput(input, thresholded, threshold, val);
+  return bad ? bad : THGPUNN_SpatialMaxPooling_updateOutput(thresholded, output, indices, kW, kH, dW, dH);
+  THC_END(1)
+}
+
+THC_API int THGPUNN_Threshold_SpatialMaxPooling_updateGradInput(THGPUTensor *input, THGPUTensor *thresholded, THGPUTensor *gradOutput,
+                                                                THGPUTensor *poolGradInput, THGPUTensor *gradInput, THGPUTensor *indices,
+                                                                double threshold, int kW, int kH, int dW, int dH) {
+  THC_BEGIN
+  long s[6];
+  if (pooled_shape(input, kW, kH, dW, dH, s) && THGPUTensor_isSameSizeAs(input, thresholded) && gradOutput->nDimension == input->nDimension &&
+      is_contiguous(gradOutput) && is_contiguous(indices)) {
+    const int o = input->nDimension - 3;
+    const long n = nelem(input), m = s[0] * s[3] * s[4];
+    const bool sizes = (!o || gradOutput->size[0] == input->size[0]) && gradOutput->size[o] == input->size[o] && gradOutput->size[o + 1] == s[3] &&
+                       gradOutput->size[o + 2] == s[4] && nelem(indices) == 2 * m;
+    if (sizes && own_storage(poolGradInput, {input, thresholded, gradOutput, indices, gradInput}) &&
+        own_storage(gradInput, {input, thresholded, gradOutput, indices})) {
+      tensor_resize_as(poolGradInput, input);
+      tensor_resize_as(gradInput, input);
+      const float *x = data_ptr(input), *g = data_ptr(gradOutput), *ind = data_ptr(indices);
+      float *gp = data_ptr(poolGradInput), *gi = data_ptr(gradInput);
+      if (is_contiguous(poolGradInput) && is_contiguous(gradInput) && apart(gp, n, gi, n) && apart(x, n, gp, n) && apart(x, n, gi, n) && apart(g, m, gp, n) &&
+          apart(g, m, gi, n) && apart(ind, 2 * m, gp, n) && apart(ind, 2 * m, gi, n) &&
+          backward_cells<true>(g, ind, ind + m, gp, s[0], s[1], s[2], s[3], s[4], kH, ThresholdPass{x, gi, (float)threshold, 0.f}))
+        return 0;
+    }
+  }
+  const int bad = THGPUNN_SpatialMaxPooling_updateGradInput(thresholded, gradOutput, poolGradInput, indices, kW, kH, dW, dH);
+  return bad ? bad : THGPUNN_Threshold_updateGradInput(input, poolGradInput, gradInput, threshold);
   THC_END(1)
 }
 

@@ -127,6 +127,7 @@ const Entry kEntries[] = {
   E(THGPUNN_SpatialConvolutionMM_updateGradInput) E(THGPUNN_SpatialConvolutionMM_accGradParameters)
   E(THGPUNN_SpatialConvolutionMM_backward) E(THGPUNN_SpatialMaxPooling_updateOutput)
   E(THGPUNN_SpatialMaxPooling_updateGradInput) E(THGPUNN_Threshold_updateOutput) E(THGPUNN_Threshold_updateGradInput)
+  E(THGPUNN_Threshold_SpatialMaxPooling_updateOutput) E(THGPUNN_Threshold_SpatialMaxPooling_updateGradInput)
   E(THGPUNN_Linear_updateOutput) E(THGPUNN_LogSoftMax_updateOutput) E(THGPUNN_LogSoftMax_updateGradInput) E(THGPUNN_ClassNLLCriterion_updateOutput)
   E(THGPUNN_ClassNLLCriterion_updateGradInput) E(THGPUNN_SGD_update)
   UNARY(EU) COMPARE(EC)

@@ -159,19 +159,35 @@ class Sequential(Module):
         return self
 
     def updateOutput(self, input):
-        cur = input
-        for m in self.modules:
-            cur = m.updateOutput(cur)
+        cur, ms, i = input, self.modules, 0
+        while i < len(ms):
+            if i + 1 < len(ms) and _threshold_pool(ms[i], ms[i + 1], "forward"):
+                cur = _threshold_pool_forward(ms[i], ms[i + 1], cur)
+                i += 2
+            else:
+                cur = ms[i].updateOutput(cur)
+                i += 1
         self.output = cur
         return cur
 
-    def updateGradInput(self, input, gradOutput):
-        cur = gradOutput
-        for i in range(len(self.modules) - 1, 0, -1):
-            cur = self.modules[i].updateGradInput(self.modules[i - 1].output, cur)
-        cur = self.modules[0].updateGradInput(input, cur)
+    def _back(self, input, gradOutput, step):
+        """`step(module, its input, its gradOutput)` from the last module to the first"""
+        cur, ms = gradOutput, self.modules
+        i = len(ms) - 1
+        if i < 0:
+            raise IndexError("Sequential without modules")
+        while i >= 0:
+            if i > 0 and _threshold_pool(ms[i - 1], ms[i], "backward"):
+                cur = _threshold_pool_backward(ms[i - 1], ms[i], ms[i - 2].output if i > 1 else input, cur)
+                i -= 2
+            else:
+                cur = step(ms[i], ms[i - 1].output if i > 0 else input, cur)
+                i -= 1
         self.gradInput = cur
         return cur
+
+    def updateGradInput(self, input, gradOutput):
+        return self._back(input, gradOutput, lambda m, x, g: m.updateGradInput(x, g))
 
     def accGradParameters(self, input, gradOutput, scale=1.0):
         cur = gradOutput
@@ -183,12 +199,7 @@ class Sequential(Module):
 
     def backward(self, input, gradOutput, scale=1.0):
         # mcw_nn/Sequential.lua backward: each module's backward in reverse order
-        cur = gradOutput
-        for i in range(len(self.modules) - 1, 0, -1):
-            cur = self.modules[i].backward(self.modules[i - 1].output, cur, scale)
-        cur = self.modules[0].backward(input, cur, scale)
-        self.gradInput = cur
-        return cur
+        return self._back(input, gradOutput, lambda m, x, g: m.backward(x, g, scale))
 
     def zeroGradParameters(self):
         for m in self.modules:
@@ -300,6 +311,37 @@ class ReLU(Threshold):
 
     def __init__(self):
         super().__init__(0.0, 0.0)
+
+
+# A Threshold and the SpatialMaxPooling behind it in one library call, which leaves in both what their own calls leave.  Only for modules
+# of these very classes that nothing overrides.
+_FORWARD, _BACKWARD = ("updateOutput",), ("backward", "updateGradInput", "accGradParameters")
+_STOCK = {c: {n: getattr(c, n) for n in _FORWARD + _BACKWARD} for c in (Threshold, ReLU, SpatialMaxPooling)}
+
+
+def _stock(m, names):
+    c = type(m)
+    return all(getattr(c, n) is _STOCK[c][n] and n not in m.__dict__ for n in names)
+
+
+def _threshold_pool(a, b, way):
+    if type(b) is not SpatialMaxPooling or type(a) not in (Threshold, ReLU):
+        return False
+    names = _FORWARD if way == "forward" else _BACKWARD
+    return _stock(a, names) and _stock(b, names)
+
+
+def _threshold_pool_forward(a, b, input):
+    _need_gpu(input, "Threshold")
+    lib().THGPUNN_Threshold_SpatialMaxPooling_updateOutput(input._p, a.output._p, b.output._p, b.indices._p, a.threshold, a.val,
+                                                           b.kW, b.kH, b.dW, b.dH)
+    return b.output
+
+
+def _threshold_pool_backward(a, b, input, gradOutput):
+    lib().THGPUNN_Threshold_SpatialMaxPooling_updateGradInput(input._p, a.output._p, gradOutput._p, b.gradInput._p, a.gradInput._p, b.indices._p,
+                                                              a.threshold, b.kW, b.kH, b.dW, b.dH)
+    return a.gradInput
 
 
 class View(Module):

@@ -43,3 +43,90 @@ def test_negative_zero_gradients(k, W):
     out = p.forward(x).size()
     gi = p.updateGradInput(x, gt.gpu(np.full(out, -0.0, np.float32))).float()
     assert np.all(gi == 0) and not np.signbit(gi).any()
+
+
+@pytest.mark.parametrize("k", [2, 3])
+@pytest.mark.parametrize("shape", SHAPES + [(2, 3, 8, 64), (3, 4, 18, 65), (1, 2, 34, 66), (5, 24, 24), (2, 2, 9, 128)])
+def test_threshold_and_pooling_in_one_pass(shape, k):
+    """A container's pass over both modules leaves in each what their own calls leave, bit for bit (nothing is rounded)."""
+    import mcw_cppamp_torch_b200 as gt
+    g = np.random.default_rng(sum(shape) * 2 + k)
+    x = g.standard_normal(shape).astype(np.float32)
+    x.reshape(-1)[::5] = 0.25
+    x.reshape(-1)[1::17] = np.nan
+    x.reshape(-1)[2::29] = -np.inf
+    xg = gt.gpu(x)
+    for th, val in ((0.0, 0.0), (0.25, -1.5)):
+        one, two = [(gt.nn.Threshold(th, val), gt.nn.SpatialMaxPooling(k, k, 2, 2)) for _ in range(2)]
+        net = gt.nn.Sequential().add(one[0]).add(one[1])
+        n = gt.lib().THGPUKernelLaunchCount()
+        out = net.forward(xg)
+        assert gt.lib().THGPUKernelLaunchCount() == n + 1
+        want = two[1].forward(two[0].forward(xg))
+        go = gt.gpu(g.standard_normal(want.size()).astype(np.float32))
+        n = gt.lib().THGPUKernelLaunchCount()
+        gi = net.backward(xg, go)
+        assert gt.lib().THGPUKernelLaunchCount() == n + 1
+        two[0].backward(xg, two[1].backward(two[0].output, go))
+        for a, b in ((out, want), (one[0].output, two[0].output), (one[1].indices, two[1].indices), (one[1].gradInput, two[1].gradInput),
+                     (gi, two[0].gradInput)):
+            assert a.size() == b.size() and np.array_equal(a.float().view(np.uint32), b.float().view(np.uint32))
+
+
+# Tensors large enough for the kernels that take whole planes: widths on both sides of the rules, planes and groups that do not come out even.
+@pytest.mark.parametrize("k", [2, 3])
+@pytest.mark.parametrize("shape", [(67, 401, 13, 13), (23, 257, 27, 29), (31, 1000, 9, 16), (9, 191, 55, 55), (5, 101, 101, 97), (7, 230, 51, 54), (4700, 90, 10, 10),
+                                   (331, 170, 29, 27), (90000, 7, 9, 8), (5, 100000, 3, 3), (1501, 3, 31, 32)])
+def test_whole_planes(oracle_port, shape, k):
+    import mcw_cppamp_torch_b200 as gt
+    g = np.random.default_rng(sum(shape) + 3 * k)
+    x = g.standard_normal(shape, dtype=np.float32)
+    x.reshape(-1)[::7] = 0.5
+    relu = np.where(x > 0, x, np.float32(0))
+    xg, rg = gt.gpu(x), gt.gpu(relu)
+    net = gt.nn.Sequential().add(gt.nn.ReLU()).add(gt.nn.SpatialMaxPooling(k, k, 2, 2))
+    m = gt.nn.SpatialMaxPooling(k, k, 2, 2)
+    want, wind = oracle_port.maxpool_forward(relu, k, k, 2, 2)
+    go = g.standard_normal(want.shape, dtype=np.float32)
+    back = oracle_port.maxpool_backward(go, wind, x.shape, 2, 2)
+    gg = gt.gpu(go)
+    assert np.array_equal(net.forward(xg).float(), want) and np.array_equal(net.modules[1].indices.float(), wind)
+    assert np.array_equal(net.modules[0].output.float(), relu)
+    assert np.array_equal(net.backward(xg, gg).float(), np.where(x > 0, back, np.float32(0)))
+    assert np.array_equal(net.modules[1].gradInput.float(), back)
+    assert np.array_equal(m.forward(rg).float(), want) and np.array_equal(m.indices.float(), wind)
+    assert np.array_equal(m.updateGradInput(rg, gg).float(), back)
+    if shape[1] * shape[2] * shape[3] % 4:   # without the first image: an address that 16-byte pieces do not start on
+        tail = xg.narrow(1, 2, shape[0] - 1)
+        assert np.array_equal(net.forward(tail).float(), want[1:])
+
+
+def test_one_pass_only_for_what_it_knows():
+    """Other windows, strided inputs, results over their sources, overridden methods: the modules' own calls, same results."""
+    import mcw_cppamp_torch_b200 as gt
+    g = np.random.default_rng(5)
+    x = g.standard_normal((2, 3, 12, 11)).astype(np.float32)
+    relu = np.where(x > 0, x, np.float32(0))
+
+    def net(k, d):
+        return gt.nn.Sequential().add(gt.nn.ReLU()).add(gt.nn.SpatialMaxPooling(k, k, d, d))
+
+    def alone(k, d, data):
+        r, p = gt.nn.ReLU(), gt.nn.SpatialMaxPooling(k, k, d, d)
+        return p.forward(r.forward(gt.gpu(data))).float()
+
+    assert np.array_equal(net(3, 1).forward(gt.gpu(x)).float(), alone(3, 1, x))
+    t = gt.gpu(np.ascontiguousarray(x.transpose(0, 1, 3, 2))).transpose(3, 4)
+    assert np.array_equal(net(2, 2).forward(t).float(), alone(2, 2, x))
+    m, xg = net(3, 2), gt.gpu(x)
+    m.modules[0].output = xg                                        # in place
+    assert np.array_equal(m.forward(xg).float(), alone(3, 2, x)) and np.array_equal(xg.float(), relu)
+    m, calls = net(2, 2), []
+    m.modules[1].updateOutput = lambda v: calls.append(1) or v
+    assert m.forward(gt.gpu(x)) is m.modules[0].output and calls == [1]
+    with pytest.raises(gt.THCError):
+        net(2, 2).forward(gt.GPUTensor(1, 1, 1))
+    m = net(2, 2)
+    out = m.forward(gt.gpu(x))
+    with pytest.raises(gt.THCError):
+        m.backward(gt.gpu(x), gt.GPUTensor(*(v + 1 for v in out.size())))
