@@ -155,7 +155,7 @@ static bool restate(const ConvGeom &g, int prec, mm::Cells &best) {
     best.Cr = best.eH * best.eW * 8; best.Cs = (int)mm::padded_channels(best.Cr, mm::kBf16);
     if (mm::windows_ok(forward_windows(g, best)) && (double)mm::planes_bytes(1, g.P, best.Cs, mm::kBf16) < kImageScratch) return true;
   }
-  // Forms of more channels than the table of cells_input_kernel holds only where there is no other: strides beyond the eight
+  // Forms of more channels than the table of CellsPass holds only where there is no other: strides beyond the eight
   // that a window map takes, over many planes, and windows beyond 128 taps (as columns).  64 planes under 16 x 16 / 16, 16 images:
   // 300 us forward and 155 for the weight gradient, 1911 and 1870 on the FMA engine; 131 x 131 taps over 16 planes: 6.6 and
   // 2.2 ms, 13.6 and 11.9 there.
@@ -214,18 +214,34 @@ static void add_strays(const ConvGeom &g, const float *src, const float *w, floa
   check_launch("window_strays");
 }
 
-// out[n, r, y, x] = bias[r] + the product of the windows `v` over `act` with rows r < rows of the repacked weights
-template <int PREC, bool FLIP, bool PAIR>
-static void window_product_t(const void *act, const mm::Windows &full, const mm::Windows &v, const float *w, const mm::Cells &u, long K,
-                             long rows, const float *bias, float *out, const Records &rec) {
+// Repacked weights of a product of windows, rows r < rows: the buffer, and the pass that fills it (which shares a launch with the one that makes
+// the windows' planes).
+template <int PREC, bool FLIP>
+struct FilterForm {
+  mm::Windows full, v;   // the layer's windows, and those of the product (pixel pairs)
+  bool pair = false;
+  long rows = 0, wrows = 0, Kd = 0;
+  mm::RepackPass<PREC, FLIP> pass;
+};
+template <int PREC, bool FLIP>
+static FilterForm<PREC, FLIP> filter_form(const mm::Windows &full, const float *w, const mm::Cells &u, long K, long rows, const Records &rec) {
+  FilterForm<PREC, FLIP> f;
+  f.full = f.v = full;
+  mm::Windows p;
+  if (pair_windows(full, rows, PREC, p)) { f.pair = true; f.v = p; }
+  f.rows = rows; f.wrows = (f.pair ? 2 : 1) * rows; f.Kd = (long)f.v.kH * f.v.kW * f.v.C;
+  THC_CHECK(f.wrows * f.Kd < (1l << 31), "filter too large");
+  void *wp = ws_alloc((size_t)f.wrows * f.Kd * (PREC == mm::kBf16 ? 2 : 4));
+  const long blocks = std::min<long>((f.wrows * (f.Kd / 4) + 255) / 256, ctx().sm_count * 8l);
+  f.pass = mm::RepackPass<PREC, FLIP>{(unsigned)blocks, w, u, (int)K, (int)rows, (int)f.v.C, f.pair ? full.dW : 0, wp, rec.joint(rec.weight)};
+  return f;
+}
+// out[n, r, y, x] = bias[r] + the product of the windows over `act` with the repacked weights
+template <int PREC, bool PAIR, class Filter>
+static void window_product_t(const void *act, const Filter &f, const float *bias, float *out, const Records &rec) {
   using namespace mm;
-  const long Kd = (long)v.kH * v.kW * v.C;
-  const long wrows = (PAIR ? 2 : 1) * rows;
-  THC_CHECK(wrows * Kd < (1l << 31), "filter too large");
-  void *wp = ws_alloc((size_t)wrows * Kd * (PREC == mm::kBf16 ? 2 : 4));
-  const long blocks = std::min<long>((wrows * (Kd / 4) + 255) / 256, ctx().sm_count * 8l);
-  pdl_launch(repack_weight_kernel<PREC, FLIP>, (unsigned)blocks, 256, 0, w, u, (int)K, (int)rows, (int)v.C, PAIR ? full.dW : 0, wp, rec.joint(rec.weight));
-  check_launch("repack_weight");
+  const Windows &full = f.full, &v = f.v;
+  const long rows = f.rows;
   Problem<PlanesWindowOperand<PREC>, RawOperand<false, PREC>, PAIR, PREC> p;
   p.range_a = rec.act.rec; p.range_b = rec.weight.rec; p.ranges = rec.joint(rec.act);
   attach_window_map<PREC>(p.a, act, v);
@@ -234,32 +250,30 @@ static void window_product_t(const void *act, const mm::Windows &full, const mm:
   if (PAIR) {
     p.epi.pair_K = rows; p.epi.pair_oH = full.oH; p.epi.pair_oW2 = v.oW; p.epi.pair_oW = full.oW; p.epi.pair_img = rows * P;
   }
-  p.M = v.N * v.oH * v.oW; p.N = wrows; p.K = Kd;
-  launch_raw(p, [&](auto &q, int bn2) { attach_raw_map<PREC>(q.b, wp, wrows, Kd, Kd, bn2 / 2); });
+  p.M = v.N * v.oH * v.oW; p.N = f.wrows; p.K = f.Kd;
+  launch_raw(p, [&](auto &q, int bn2) { attach_raw_map<PREC>(q.b, f.pass.out, f.wrows, f.Kd, f.Kd, bn2 / 2); });
 }
 template <int PREC, bool FLIP>
-static void window_product(const void *act, const mm::Windows &v, const float *w, const mm::Cells &u, long K, long rows, const float *bias,
-                           float *out, const Records &rec) {
-  mm::Windows p;
+static void window_product(const void *act, const FilterForm<PREC, FLIP> &f, const float *bias, float *out, const Records &rec) {
   if constexpr (PREC != mm::kBf16)
-    if (pair_windows(v, rows, PREC, p)) { window_product_t<PREC, FLIP, true>(act, v, p, w, u, K, rows, bias, out, rec); return; }
-  window_product_t<PREC, FLIP, false>(act, v, v, w, u, K, rows, bias, out, rec);
+    if (f.pair) { window_product_t<PREC, true>(act, f, bias, out, rec); return; }
+  window_product_t<PREC, false>(act, f, bias, out, rec);
 }
 
-// The restated input in `dst`.
+// The restated input in `dst`, and the weights of `repack`.
 template <int PREC>
-static void restate_input(const ConvGeom &g, const mm::Cells &u, const float *in, void *dst, const mm::PairForm &form) {
-  if (u.direct) { mm::make_act_planes<PREC>(in, g.N, g.C, g.H, g.W, dst, false, form); return; }
+static void restate_input(const ConvGeom &g, const mm::Cells &u, const float *in, void *dst, const mm::PairForm &form,
+                          const mm::RepackPass<PREC, false> &repack) {
+  if (u.direct) { mm::make_act_planes<PREC>(in, g.N, g.C, g.H, g.W, dst, false, form, repack, mm::NoPass{}, 0); return; }
   if constexpr (PREC == mm::kBf16) {
     const size_t smem = sizeof(uint4) * g.kH * (g.W + 2 * g.pad);
     if (u.Cq == 8 && u.kHs == 1 && u.kWs == 1 && g.C <= 8 && smem <= 200 * 1024) {
       static thread_local int configured_for = -1;
       if (configured_for != ctx().device) {
-        THC_CUDA(cudaFuncSetAttribute(mm::columns8_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+        THC_CUDA(cudaFuncSetAttribute(mm::passes_kernel<mm::Columns8Pass, mm::RepackPass<PREC, false>, mm::NoPass>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
         configured_for = ctx().device;
       }
-      pdl_launch(mm::columns8_kernel, (unsigned)(g.N * u.Hs), 256, smem, in, (uint4 *)dst, u);
-      check_launch("columns8");
+      mm::launch_passes(mm::Columns8Pass{(unsigned)(g.N * u.Hs), in, (uint4 *)dst, u}, smem, "columns8", repack);
       return;
     }
   }
@@ -278,14 +292,13 @@ static void restate_input(const ConvGeom &g, const mm::Cells &u, const float *in
     const long units = chunks * (PREC == mm::kPairs ? 2 : 1);
     if (256 % q == 0 && smem <= 40 * 1024 && rows >= 2l * ctx().sm_count && u.C * u.eH <= 24 &&
         (units >= 1024 || (units >= 768 && rows >= 32l * ctx().sm_count))) {
-      pdl_launch(mm::cells_staged_kernel<PREC>, (unsigned)std::min(rows, 16l * ctx().sm_count), 256, smem, in, dst, g.N, u, (int)Wp, (int)ld, form);
-      check_launch("cells_staged");
+      mm::launch_passes(mm::StagedCellsPass<PREC>{(unsigned)std::min(rows, 16l * ctx().sm_count), in, dst, g.N, u, (int)Wp, (int)ld, form}, smem, "cells_staged", repack);
       return;
     }
   }
-  if (u.Cs <= mm::kCellTable) pdl_launch(mm::cells_input_kernel<PREC, true>, dim3((unsigned)rows, parts), 256, sizeof(int2) * u.Cs, in, dst, g.N, u, form);
-  else pdl_launch(mm::cells_input_kernel<PREC, false>, dim3((unsigned)rows, parts), 256, 0, in, dst, g.N, u, form);
-  check_launch("cells_input");
+  const unsigned blocks = (unsigned)rows * parts;
+  if (u.Cs <= mm::kCellTable) mm::launch_passes(mm::CellsPass<PREC, true>{blocks, (unsigned)rows, in, dst, u, form}, sizeof(int2) * u.Cs, "cells_input", repack);
+  else mm::launch_passes(mm::CellsPass<PREC, false>{blocks, (unsigned)rows, in, dst, u, form}, 0, "cells_input", repack);
 }
 
 // Room for the restated input in `finput` (the counterpart of the column matrix the reference keeps there): a
@@ -336,8 +349,9 @@ static void conv_forward_tc(const ConvGeom &g, const mm::Cells &u, const float *
     void *act = finput ? planes_in(finput, s, u, x, PREC) : nullptr;
     if (act && PREC == mm::kPairs) { form.keep = planes_record(act); form.list = rec.act.list; }
     if (!act) act = ws_alloc(mm::planes_bytes(s.N, (long)u.Hs * u.Ws, u.Cs, PREC));
-    restate_input<PREC>(s, u, x, act, form);
-    window_product<PREC, false>(act, forward_windows(s, u), w, u, g.K, g.K, bias, out + n0 * g.K * g.P, rec);
+    const auto filter = filter_form<PREC, false>(forward_windows(s, u), w, u, g.K, g.K, rec);
+    restate_input<PREC>(s, u, x, act, form, filter.pass);
+    window_product(act, filter, bias, out + n0 * g.K * g.P, rec);
     if (PREC == mm::kPairs) add_strays<false>(s, x, w, out + n0 * g.K * g.P, rec);
   }
 }
@@ -377,15 +391,23 @@ static bool grad_input_layer(const ConvGeom &g, int prec, ConvGeom &t, mm::Cells
 }
 
 // gradInput = forward pass of gradOutput's planes under the filter rotated by 180 degrees with its plane roles swapped.
-template <int PREC>
-static void conv_grad_input_tc(const ConvGeom &g, const mm::ActPlanes &pgo, const float *w, float *gin, const Records &records) {
+static Records grad_input_records(const Records &records) {
   Records rec = records;
   std::swap(rec.act, rec.gout);   // the windows run over gradOutput here
+  return rec;
+}
+template <int PREC>
+static FilterForm<PREC, true> grad_input_filter(const ConvGeom &g, const float *w, const Records &records) {
   const mm::Cells u = grad_input_cells(g, PREC);
-  const mm::Windows v = grad_input_windows(g, u, PREC);
-  if (u.direct) { window_product<PREC, true>(pgo.p, v, w, u, g.K, g.C, nullptr, gin, rec); return; }
+  return filter_form<PREC, true>(grad_input_windows(g, u, PREC), w, u, g.K, u.direct ? g.C : u.Cr, grad_input_records(records));
+}
+template <int PREC>
+static void conv_grad_input_tc(const ConvGeom &g, const mm::ActPlanes &pgo, const FilterForm<PREC, true> &filter, float *gin, const Records &records) {
+  const Records rec = grad_input_records(records);
+  const mm::Cells &u = filter.pass.u;
+  if (u.direct) { window_product(pgo.p, filter, nullptr, gin, rec); return; }
   float *gS = (float *)ws_alloc(sizeof(float) * g.N * u.Cr * (long)(u.Hs * u.Ws));
-  window_product<PREC, true>(pgo.p, v, w, u, g.K, u.Cr, nullptr, gS, rec);
+  window_product(pgo.p, filter, nullptr, gS, rec);
   const long planes = g.N * g.C;
   const unsigned bx = (unsigned)std::min<long>((g.H * g.W + 255) / 256, 64);
   const unsigned by = (unsigned)std::min<long>(planes, std::max<long>(1, ctx().sm_count * 32l / bx));
@@ -408,7 +430,7 @@ static void conv_grad_input_tc(const ConvGeom &g, const mm::ActPlanes &pgo, cons
 //      vain, but a k tile costs the same however little of its 256 x 64 tile is used, and there are f times fewer.
 template <int PREC>
 static void conv_acc_grad_tc(const ConvGeom &g, const mm::Cells &u, const void *act, const mm::ActPlanes &pgo, const float *gout, long n0, float *gw,
-                             float scale, const Records &rec) {
+                             float scale, const Records &rec, const mm::ChanFinishPass &bias) {
   using namespace mm;
   const WgradStrays strays{rec.act, rec.gout, rec.joint(rec.act), n0, act, gout, layer_shape(g)};
   const Windows v = forward_windows(g, u);
@@ -435,8 +457,7 @@ static void conv_acc_grad_tc(const ConvGeom &g, const mm::Cells &u, const void *
     });
     const WgradPlace pl{Nf, 1, 0, 0, 0, (int)f, Kp * Nf + Cs};
     const long total = g.K * g.R;
-    pdl_launch(unpack_grad_weight_kernel<PREC == kPairs>, (unsigned)std::min<long>((total + 255) / 256, ctx().sm_count * 8l), 256, 0, T, gw, u, (int)g.K, pl, scale, strays);
-    check_launch("unpack_grad_weight");
+    launch_passes(UnpackGradPass<PREC == kPairs>{(unsigned)std::min<long>((total + 255) / 256, ctx().sm_count * 8l), T, gw, u, (int)g.K, pl, scale, strays}, 0, "unpack_grad_weight", bias);
     return;
   }
   const long cols = way == 2 ? N2 : way == 1 ? g.K : Rp, rows = way == 2 ? M2 : way == 1 ? Rp : g.K;
@@ -469,8 +490,7 @@ static void conv_acc_grad_tc(const ConvGeom &g, const mm::Cells &u, const void *
     pl = WgradPlace{1, N2, Cs * N2, -Kp, (u.kWs - 1) * Kp, 1, 0};
   }
   const long total = g.K * g.R;
-  pdl_launch(unpack_grad_weight_kernel<PREC == kPairs>, (unsigned)std::min<long>((total + 255) / 256, ctx().sm_count * 8l), 256, 0, T, gw, u, (int)g.K, pl, scale, strays);
-  check_launch("unpack_grad_weight");
+  launch_passes(UnpackGradPass<PREC == kPairs>{(unsigned)std::min<long>((total + 255) / 256, ctx().sm_count * 8l), T, gw, u, (int)g.K, pl, scale, strays}, 0, "unpack_grad_weight", bias);
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -616,10 +636,10 @@ static bool restate_accurate(const ConvGeom &g, bool pairs, mm::Cells &u, int &p
   const bool ok = restate(g, mm::kTf32, u);
   mm::Cells up;
   if (!ok || !pairs || g.R > 1l << 28 || g.K * g.kH * g.kW > 1l << 28 ||   // (a row of weights and its second half: 31 bits)
-      windows_us(forward_windows(g, u), g.K, prec) < 30 || !restate(g, mm::kPairs, up) || up.Cs > 12288 ||   // (unpair_kernel: 48 KB)
+      windows_us(forward_windows(g, u), g.K, prec) < 30 || !restate(g, mm::kPairs, up) || up.Cs > 12288 ||   // (UnpairPass: 48 KB)
       (up.kHs == 1 && up.kWs == 1 && !up.direct))
     return ok;
-  // (window_product_t counts the repacked weights in 31 bits; channels in spans of 64 may make more of them than spans of 32)
+  // (filter_form counts the repacked weights in 31 bits; channels in spans of 64 may make more of them than spans of 32)
   const mm::Cells gi = grad_input_cells(g, mm::kPairs);
   if (2. * g.K * up.kHs * up.kWs * up.Cs >= 0x1p31 || 2. * (gi.direct ? gi.C : gi.Cr) * gi.kHs * gi.kWs * mm::padded_channels(g.K, mm::kPairs) >= 0x1p31) return ok;
   auto us = [&](const mm::Cells &c, int pr) {
@@ -664,36 +684,49 @@ static void conv_forward(const ConvGeom &g, const float *in, const float *w, con
 // `act`: the input's planes, or null (n0: the image of their record that they start with); w_ok / in_ok: whether the weight gradient / gradInput runs over planes.
 template <int PREC>
 static void conv_backward_group(const ConvGeom &g, const mm::Cells &u, bool in_ok, bool w_ok, const float *in, const void *act, const float *gout,
-                                const float *w, float *gin, float *gw, float *gb, float scale, const Records &rec, long n0) {
+                                const float *w, float *gin, float *gw, float *gb, float scale, const Records &rec, long n0, mm::UnpairPass unpair) {
   WsScope ws_scope;
   mm::ActPlanes pgo;
   mm::PairForm form;
   form.ranges = rec.joint(rec.gout);
-  if (in_ok || w_ok) pgo = mm::make_act_planes<PREC>(gout, g.N, g.K, g.oH, g.oW, nullptr, gw != nullptr, form);
+  FilterForm<PREC, true> filter;
+  if (in_ok) filter = grad_input_filter<PREC>(g, w, rec);
+  if (PREC == mm::kPairs) {
+    // planes are brought back to FP32 pixel by pixel where that needs no more shared memory than the transposition leaves
+    const size_t more = unpair.blocks ? sizeof(float) * std::max(1024, unpair.Cp) : 0;
+    if (more > 14 * 1024) {
+      unpair.px = 1;
+      mm::launch_passes(unpair, sizeof(float) * unpair.Cp, "unpair");
+      unpair.blocks = 0;
+    } else if (unpair.blocks) {
+      unpair.px = (int)(more / sizeof(float)) / unpair.Cp;
+    }
+    if (in_ok || w_ok) pgo = mm::make_act_planes<PREC>(gout, g.N, g.K, g.oH, g.oW, nullptr, gw != nullptr, form, filter.pass, unpair, unpair.blocks ? more : 0);
+  } else if (in_ok || w_ok) {
+    pgo = mm::make_act_planes<PREC>(gout, g.N, g.K, g.oH, g.oW, nullptr, gw != nullptr, form, filter.pass, mm::NoPass{}, 0);
+  }
   if (in_ok) {
-    conv_grad_input_tc<PREC>(g, pgo, w, gin, rec);
+    conv_grad_input_tc<PREC>(g, pgo, filter, gin, rec);
     if (PREC == mm::kPairs) add_strays<true>(g, gout, w, gin, rec);
   } else if (gin) {
     conv_grad_input_simt(g, gout, w, gin);
   }
   if (!gw) return;
+  mm::ChanFinishPass bias;   // gradBias comes along with the transposition of gradOutput
+  if (pgo.chan_partial) bias = mm::ChanFinishPass{(unsigned)((g.K + 7) / 8), pgo.chan_partial, pgo.chan_blocks, g.K, gb, scale};
   if (w_ok) {
     if (!act) {
       void *made = ws_alloc(mm::planes_bytes(g.N, (long)u.Hs * u.Ws, u.Cs, PREC));
       form.ranges = rec.joint(rec.act);
-      restate_input<PREC>(g, u, in, made, form);
+      restate_input<PREC>(g, u, in, made, form, {});
       act = made;
     }
-    conv_acc_grad_tc<PREC>(g, u, act, pgo, gout, n0, gw, scale, rec);
+    conv_acc_grad_tc<PREC>(g, u, act, pgo, gout, n0, gw, scale, rec, bias);
   } else {
     conv_acc_grad_simt(g, in, gout, gw, scale);
+    mm::launch_passes(bias, 0, "conv_grad_bias_finish");
   }
-  if (pgo.chan_partial) {   // gradBias came along with the transposition of gradOutput
-    pdl_launch(mm::chan_partial_finish_kernel, ceil_div(g.K, 32), 1024, 0, pgo.chan_partial, pgo.chan_blocks, g.K, gb, scale);
-    check_launch("conv_grad_bias_finish");
-  } else {
-    grad_bias(g, gout, gb, scale);
-  }
+  if (!bias.blocks) grad_bias(g, gout, gb, scale);
 }
 // False: there is no room for planes of this precision (kPairs), and nothing has been done.
 template <int PREC>
@@ -725,6 +758,7 @@ static bool conv_backward_tc(const ConvGeom &g, const mm::Cells &u, bool restate
     if (own || gw) {
       WsScope ws_scope;
       Records rec;
+      mm::UnpairPass unpair;
       if constexpr (PREC == mm::kPairs) {   // (for each group: records last for some thousand words, see zeroed_words)
         rec.gout = mm::new_measured();
         if (own_ok) rec.weight = mm::new_measured();
@@ -733,16 +767,14 @@ static bool conv_backward_tc(const ConvGeom &g, const mm::Cells &u, bool restate
         if (act) {
           mm::KeptRange *kept = planes_record(act);
           rec.act = mm::Measured{&kept->rec, kept->strays, true};
-          const long pixels = g.N * u.Hs * u.Ws, px = std::max(1, 6144 / u.Cs);
-          pdl_launch(mm::unpair_kernel, (unsigned)std::min((pixels + px - 1) / px, 4l * ctx().sm_count), 256, sizeof(float) * px * u.Cs, (void *)act, pixels, u.Cs,
-                     (int)px, rec.joint(rec.act), &kept->rec);
-          check_launch("unpair");
+          const long pixels = g.N * u.Hs * u.Ws;
+          unpair = mm::UnpairPass{(unsigned)std::min(pixels, 4l * ctx().sm_count), (void *)act, pixels, u.Cs, 1, rec.joint(rec.act), &kept->rec};
         } else if (w_ok) {
           rec.act = mm::new_measured();
           mm::launch_ranges(mm::range_job_flat(x, s.N * image, rec.act), nullptr);
         }
       }
-      conv_backward_group<PREC>(s, u, own_ok, w_ok, x, act ? act + n0 * act_image : nullptr, go, w, own ? gi : nullptr, gw, gb, scale, rec, act ? n0 : 0);
+      conv_backward_group<PREC>(s, u, own_ok, w_ok, x, act ? act + n0 * act_image : nullptr, go, w, own ? gi : nullptr, gw, gb, scale, rec, act ? n0 : 0, unpair);
     }
     if (layer) {   // last: its own groups use up words
       WsScope ws_scope;

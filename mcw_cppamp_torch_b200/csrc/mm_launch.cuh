@@ -376,19 +376,28 @@ static void launch_small(SmallProblem p, bool a_k, bool b_k) {
   else launch_small_layout<64, 2, 2>(p, a_k, b_k);
 }
 
+template <class Main, class First = NoPass, class Second = NoPass>
+static void launch_passes(const Main &main, size_t smem, const char *what, const First &first = {}, const Second &second = {}) {
+  const unsigned blocks = main.blocks + first.blocks + second.blocks;
+  if (!blocks) return;
+  pdl_launch(passes_kernel<Main, First, Second>, blocks, 256, smem, main, first, second);
+  check_launch(what);
+}
 // Channels-last planes of an NCHW activation tensor (or its cells), FP32 or BF16.
 struct ActPlanes {
   void *p = nullptr;
   long N = 0, H = 0, W = 0, Cp = 0;
-  // per-channel sums of the transposed tensor, when asked for: [chan_blocks][C] partials (see nchw_to_planes_kernel)
+  // per-channel sums of the transposed tensor, when asked for: [chan_blocks][C] partials (see PlanesPass)
   float *chan_partial = nullptr;
   int chan_blocks = 0;
 };
 static long padded_channels(long C, int prec) { return prec != kTf32 ? (C + 63) / 64 * 64 : (C + 31) / 32 * 32; }
 static size_t planes_bytes(long N, long HW, long Cp, int prec) { return (size_t)N * HW * Cp * (prec == kBf16 ? 2 : 4); }
-// `dst`: room for planes_bytes(), or null for workspace.  `form`: kPairs.
-template <int PREC>
-static ActPlanes make_act_planes(const float *src, long N, long C, long H, long W, void *dst, bool want_chan_sums, const PairForm &form) {
+// `dst`: room for planes_bytes(), or null for workspace.  `form`: kPairs.  `first`, `second` (with `more` bytes of shared memory): passes that
+// share the launch.
+template <int PREC, class First, class Second>
+static ActPlanes make_act_planes(const float *src, long N, long C, long H, long W, void *dst, bool want_chan_sums, const PairForm &form, const First &first,
+                                 const Second &second, size_t more) {
   ActPlanes ap;
   const long HW = H * W;
   ap.N = N; ap.H = H; ap.W = W; ap.Cp = padded_channels(C, PREC);
@@ -409,11 +418,13 @@ static ActPlanes make_act_planes(const float *src, long N, long C, long H, long 
     ap.chan_partial = (float *)ws_alloc(sizeof(float) * blocks * C);
     smem = sizeof(float) * C;
   }
-  if constexpr (PREC == kPairs)
-    pdl_launch(wide_tile ? nchw_to_pairs_kernel<128> : nchw_to_pairs_kernel<64>, (unsigned)blocks, 256, smem, src, N, (int)C, (int)HW, (int)ap.Cp, ap.p, ap.chan_partial, form);
-  else
-    pdl_launch(nchw_to_planes_kernel<PREC == kBf16>, (unsigned)blocks, 256, smem, src, N, (int)C, (int)HW, (int)ap.Cp, ap.p, ap.chan_partial);
-  check_launch("nchw_to_planes");
+  smem = std::max(smem, more);
+  if constexpr (PREC == kPairs) {
+    if (wide_tile) launch_passes(PairsPass<128>{(unsigned)blocks, src, N, (int)C, (int)HW, (int)ap.Cp, ap.p, ap.chan_partial, form}, smem, "nchw_to_pairs", first, second);
+    else launch_passes(PairsPass<64>{(unsigned)blocks, src, N, (int)C, (int)HW, (int)ap.Cp, ap.p, ap.chan_partial, form}, smem, "nchw_to_pairs", first, second);
+  } else {
+    launch_passes(PlanesPass<PREC == kBf16>{(unsigned)blocks, src, N, (int)C, (int)HW, (int)ap.Cp, ap.p, ap.chan_partial}, smem, "nchw_to_planes", first, second);
+  }
   return ap;
 }
 

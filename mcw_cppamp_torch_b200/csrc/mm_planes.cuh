@@ -167,13 +167,31 @@ static __global__ void __launch_bounds__(256, 5) range_kernel(const RangeJob ja,
   if (threadIdx.x == 0) j.rec->strays = n;
 }
 
+// Passes that do not read one another's results share a launch: the blocks of `first`, then those of `second`, then `main`'s.  Each is a
+// struct of its arguments with run(block) and its number of blocks, 256 threads each (none: not asked for).  A launch of its own, by the time
+// the next one has waited for it, costs a small pass two to four microseconds more than its work.
+struct NoPass {
+  static constexpr unsigned blocks = 0;
+  __device__ __forceinline__ void run(unsigned) const {}
+};
+template <class Main, class First, class Second>
+static __global__ void __launch_bounds__(256) passes_kernel(const __grid_constant__ Main main, const __grid_constant__ First first,
+                                                            const __grid_constant__ Second second) {
+  pdl_begin();
+  unsigned block = blockIdx.x;
+  if (block < first.blocks) { first.run(block); return; }
+  block -= first.blocks;
+  if (block < second.blocks) { second.run(block); return; }
+  main.run(block - second.blocks);
+}
+
 // What a kernel that writes an operand's planes needs in kPairs.
 struct PairForm {
   Ranges ranges;
   KeptRange *keep = nullptr;     // where the operand's measures go when the planes outlive the call ...
   const Stray *list = nullptr;   // ... and its list
-  __device__ __forceinline__ void end(bool wide) const {
-    if (!keep || blockIdx.x || blockIdx.y) return;
+  __device__ __forceinline__ void end(bool wide, unsigned block) const {
+    if (!keep || block) return;
     const RangeRec r = *ranges.rec[0];
     const int n = wide ? 0 : (int)r.strays;
     if (threadIdx.x == 0) {
@@ -187,26 +205,33 @@ struct PairForm {
 // Kept planes back to FP32, in place, where another operand asks for it: 24 bits of almost every value (22 next to the strays, whose
 // places stay zero).  A block takes `px` pixels of Cp channels at a time through shared memory.  Not made from the input again:
 // what the input's memory holds may have changed since the planes were written.
-static __global__ void __launch_bounds__(256) unpair_kernel(void *planes, long pixels, int Cp, int px, const Ranges ranges, RangeRec *kept) {
-  pdl_begin();
-  if (!ranges.wide() || *const_cast<const volatile unsigned *>(&kept->wide)) return;
-  extern __shared__ float4 raw[];
-  const __half *h = reinterpret_cast<const __half *>(raw);
-  const float unscale = pair_unscale(*kept);
-  for (long p0 = (long)blockIdx.x * px; p0 < pixels; p0 += (long)gridDim.x * px) {
-    const int n = (int)min((long)px, pixels - p0) * Cp;
-    float *d = reinterpret_cast<float *>(planes) + p0 * Cp;
-    for (int i = threadIdx.x; i < n / 4; i += 256) raw[i] = reinterpret_cast<const float4 *>(d)[i];
-    __syncthreads();
-    for (int i = threadIdx.x; i < n; i += 256) {
-      const int p = i / Cp, c = i - p * Cp;
-      d[i] = join_pair(h[2 * p * Cp + c], h[(2 * p + 1) * Cp + c], unscale);
+struct UnpairPass {
+  unsigned blocks = 0;
+  void *planes;
+  long pixels;
+  int Cp, px;
+  Ranges ranges;
+  RangeRec *kept;
+  __device__ __forceinline__ void run(unsigned block) const {
+    if (!ranges.wide() || *const_cast<const volatile unsigned *>(&kept->wide)) return;
+    extern __shared__ float4 pass_sm[];
+    const __half *h = reinterpret_cast<const __half *>(pass_sm);
+    const float unscale = pair_unscale(*kept);
+    for (long p0 = (long)block * px; p0 < pixels; p0 += (long)blocks * px) {
+      const int n = (int)min((long)px, pixels - p0) * Cp;
+      float *d = reinterpret_cast<float *>(planes) + p0 * Cp;
+      for (int i = threadIdx.x; i < n / 4; i += 256) pass_sm[i] = reinterpret_cast<const float4 *>(d)[i];
+      __syncthreads();
+      for (int i = threadIdx.x; i < n; i += 256) {
+        const int p = i / Cp, c = i - p * Cp;
+        d[i] = join_pair(h[2 * p * Cp + c], h[(2 * p + 1) * Cp + c], unscale);
+      }
+      __syncthreads();
     }
-    __syncthreads();
+    // every block has looked at the flag before the last one sets it
+    if (threadIdx.x == 0 && atomicAdd(&kept->ticket, 1u) == blocks - 1) { kept->ticket = 0; kept->wide = 1; }
   }
-  // every block has looked at the flag before the last one sets it
-  if (threadIdx.x == 0 && atomicAdd(&kept->ticket, 1u) == gridDim.x - 1) { kept->ticket = 0; kept->wide = 1; }
-}
+};
 
 // ---------------------------------------------------------------------------------------------
 // Channels-last planes of an activation tensor, FP32 or BF16, channels padded with zeros to Cp = a multiple of KV.
@@ -218,160 +243,191 @@ static __global__ void __launch_bounds__(256) unpair_kernel(void *planes, long p
 // reduction of a convolution rides on the transposition of gradOutput instead of reading the tensor a second time.
 // A channel of a tile belongs to one warp, tiles are taken in a fixed order, so the sums are reproducible.
 template <bool HALF>
-static __global__ void __launch_bounds__(256) nchw_to_planes_kernel(const float *__restrict__ src, long N, int C, int HW, int Cp,
-                                                                    void *__restrict__ dst, float *__restrict__ chan_partial) {
-  pdl_begin();
-  constexpr int CT = HALF ? 64 : 32, PT = HALF ? 64 : 128;
-  __shared__ float tile[CT][PT + 1];
-  extern __shared__ float chan_sum[];   // [C] when chan_partial is given
-  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-  const unsigned ptiles = (unsigned)((HW + PT - 1) / PT), ctiles = (unsigned)(Cp / CT);
-  const long ntiles = N * ptiles * ctiles;
-  if (chan_partial) {
-    for (int c = threadIdx.x; c < C; c += blockDim.x) chan_sum[c] = 0.f;
-    __syncthreads();
-  }
-  for (long t = blockIdx.x; t < ntiles; t += gridDim.x) {
-    const unsigned r = (unsigned)(t % (ptiles * ctiles));
-    const long img = t / (ptiles * ctiles);
-    const int ct = (int)(r / ptiles), p0 = (int)(r - ct * ptiles) * PT, c0 = ct * CT;
-    const int np = min(HW - p0, PT), nc = min(C - c0, CT);
-    const float *s = src + (img * C + c0) * HW + p0 + tx;
-    float v[CT / 8][PT / 32];
-#pragma unroll
-    for (int j = 0; j < CT / 8; j++)
-#pragma unroll
-      for (int g = 0; g < PT / 32; g++)
-        v[j][g] = (g * 32 + tx < np && ty + 8 * j < nc) ? s[(long)(ty + 8 * j) * HW + g * 32] : 0.f;
-#pragma unroll
-    for (int j = 0; j < CT / 8; j++) {
-      float part = 0.f;
-#pragma unroll
-      for (int g = 0; g < PT / 32; g++) {
-        tile[ty + 8 * j][g * 32 + tx] = v[j][g];
-        part += v[j][g];
-      }
-      if (chan_partial) {
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
-        if (tx == 0 && ty + 8 * j < nc) chan_sum[c0 + ty + 8 * j] += part;
-      }
+struct PlanesPass {
+  unsigned blocks = 0;
+  const float *src;
+  long N;
+  int C, HW, Cp;
+  void *dst;
+  float *chan_partial;
+  __device__ __forceinline__ void run(unsigned block) const {
+    constexpr int CT = HALF ? 64 : 32, PT = HALF ? 64 : 128;
+    __shared__ float tile[CT][PT + 1];
+    extern __shared__ float4 pass_sm[];
+    float *chan_sum = reinterpret_cast<float *>(pass_sm);   // [C] when chan_partial is given
+    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+    const unsigned ptiles = (unsigned)((HW + PT - 1) / PT), ctiles = (unsigned)(Cp / CT);
+    const long ntiles = N * ptiles * ctiles;
+    if (chan_partial) {
+      for (int c = threadIdx.x; c < C; c += blockDim.x) chan_sum[c] = 0.f;
+      __syncthreads();
     }
-    __syncthreads();
-    const long o0 = (img * HW + p0) * Cp + c0;
+    for (long t = block; t < ntiles; t += blocks) {
+      const unsigned r = (unsigned)(t % (ptiles * ctiles));
+      const long img = t / (ptiles * ctiles);
+      const int ct = (int)(r / ptiles), p0 = (int)(r - ct * ptiles) * PT, c0 = ct * CT;
+      const int np = min(HW - p0, PT), nc = min(C - c0, CT);
+      const float *s = src + (img * C + c0) * HW + p0 + tx;
+      float v[CT / 8][PT / 32];
+#pragma unroll
+      for (int j = 0; j < CT / 8; j++)
+#pragma unroll
+        for (int g = 0; g < PT / 32; g++)
+          v[j][g] = (g * 32 + tx < np && ty + 8 * j < nc) ? s[(long)(ty + 8 * j) * HW + g * 32] : 0.f;
+#pragma unroll
+      for (int j = 0; j < CT / 8; j++) {
+        float part = 0.f;
+#pragma unroll
+        for (int g = 0; g < PT / 32; g++) {
+          tile[ty + 8 * j][g * 32 + tx] = v[j][g];
+          part += v[j][g];
+        }
+        if (chan_partial) {
+#pragma unroll
+          for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
+          if (tx == 0 && ty + 8 * j < nc) chan_sum[c0 + ty + 8 * j] += part;
+        }
+      }
+      __syncthreads();
+      const long o0 = (img * HW + p0) * Cp + c0;
 #pragma unroll 8
-    for (int j = ty; j < np; j += 8) {
-      if constexpr (HALF)
-        reinterpret_cast<__nv_bfloat162 *>(dst)[(o0 + (long)j * Cp) / 2 + tx] = __floats2bfloat162_rn(tile[2 * tx][j], tile[2 * tx + 1][j]);
-      else
-        reinterpret_cast<float *>(dst)[o0 + (long)j * Cp + tx] = tile[tx][j];
+      for (int j = ty; j < np; j += 8) {
+        if constexpr (HALF)
+          reinterpret_cast<__nv_bfloat162 *>(dst)[(o0 + (long)j * Cp) / 2 + tx] = __floats2bfloat162_rn(tile[2 * tx][j], tile[2 * tx + 1][j]);
+        else
+          reinterpret_cast<float *>(dst)[o0 + (long)j * Cp + tx] = tile[tx][j];
+      }
+      __syncthreads();
     }
-    __syncthreads();
+    if (chan_partial)
+      for (int c = threadIdx.x; c < C; c += blockDim.x) chan_partial[(long)block * C + c] = chan_sum[c];
   }
-  if (chan_partial)
-    for (int c = threadIdx.x; c < C; c += blockDim.x) chan_partial[(long)blockIdx.x * C + c] = chan_sum[c];
-}
+};
 // The same as FP16 pairs, [img][pixel][hi: Cp][lo: Cp], or FP32 values in the same place.  Bound by latency: 128 pixels a pass keep
 // twice the loads in flight (198 M values with channel sums, 1.6 GB: 322 -> 277 us), 64 where planes would leave much of the
 // wider tile empty (13 x 13: 92 us with 128, 83 with 64).
 template <int PT>
-static __global__ void __launch_bounds__(256) nchw_to_pairs_kernel(const float *__restrict__ src, long N, int C, int HW, int Cp,
-                                                                   void *__restrict__ dst, float *__restrict__ chan_partial,
-                                                                   const PairForm form) {
-  pdl_begin();
-  const bool wide = form.ranges.wide();
-  const float scale = wide ? 1.f : pair_scale(*form.ranges.rec[0]);
-  constexpr int CT = 64;
-  __shared__ float tile[CT][PT + 1];
-  extern __shared__ float chan_sum[];   // [C] when chan_partial is given
-  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-  const unsigned ptiles = (unsigned)((HW + PT - 1) / PT), ctiles = (unsigned)(Cp / CT);
-  const long ntiles = N * ptiles * ctiles;
-  if (chan_partial) {
-    for (int c = threadIdx.x; c < C; c += blockDim.x) chan_sum[c] = 0.f;
-    __syncthreads();
-  }
-  for (long t = blockIdx.x; t < ntiles; t += gridDim.x) {
-    const unsigned r = (unsigned)(t % (ptiles * ctiles));
-    const long img = t / (ptiles * ctiles);
-    const int ct = (int)(r / ptiles), p0 = (int)(r - ct * ptiles) * PT, c0 = ct * CT;
-    const int np = min(HW - p0, PT), nc = min(C - c0, CT);
-    const float *s = src + (img * C + c0) * HW + p0 + tx;
-    float v[CT / 8][PT / 32];
-#pragma unroll
-    for (int j = 0; j < CT / 8; j++)
-#pragma unroll
-      for (int g = 0; g < PT / 32; g++)
-        v[j][g] = (g * 32 + tx < np && ty + 8 * j < nc) ? s[(long)(ty + 8 * j) * HW + g * 32] : 0.f;
-#pragma unroll
-    for (int j = 0; j < CT / 8; j++) {
-      float part = 0.f;
-#pragma unroll
-      for (int g = 0; g < PT / 32; g++) {
-        tile[ty + 8 * j][g * 32 + tx] = v[j][g];
-        part += v[j][g];
-      }
-      if (chan_partial) {
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
-        if (tx == 0 && ty + 8 * j < nc) chan_sum[c0 + ty + 8 * j] += part;
-      }
+struct PairsPass {
+  unsigned blocks = 0;
+  const float *src;
+  long N;
+  int C, HW, Cp;
+  void *dst;
+  float *chan_partial;
+  PairForm form;
+  __device__ __forceinline__ void run(unsigned block) const {
+    const bool wide = form.ranges.wide();
+    const float scale = wide ? 1.f : pair_scale(*form.ranges.rec[0]);
+    constexpr int CT = 64;
+    __shared__ float tile[CT][PT + 1];
+    extern __shared__ float4 pass_sm[];
+    float *chan_sum = reinterpret_cast<float *>(pass_sm);   // [C] when chan_partial is given
+    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+    const unsigned ptiles = (unsigned)((HW + PT - 1) / PT), ctiles = (unsigned)(Cp / CT);
+    const long ntiles = N * ptiles * ctiles;
+    if (chan_partial) {
+      for (int c = threadIdx.x; c < C; c += blockDim.x) chan_sum[c] = 0.f;
+      __syncthreads();
     }
-    __syncthreads();
-    const long o0 = (img * HW + p0) * Cp;
+    for (long t = block; t < ntiles; t += blocks) {
+      const unsigned r = (unsigned)(t % (ptiles * ctiles));
+      const long img = t / (ptiles * ctiles);
+      const int ct = (int)(r / ptiles), p0 = (int)(r - ct * ptiles) * PT, c0 = ct * CT;
+      const int np = min(HW - p0, PT), nc = min(C - c0, CT);
+      const float *s = src + (img * C + c0) * HW + p0 + tx;
+      float v[CT / 8][PT / 32];
+#pragma unroll
+      for (int j = 0; j < CT / 8; j++)
+#pragma unroll
+        for (int g = 0; g < PT / 32; g++)
+          v[j][g] = (g * 32 + tx < np && ty + 8 * j < nc) ? s[(long)(ty + 8 * j) * HW + g * 32] : 0.f;
+#pragma unroll
+      for (int j = 0; j < CT / 8; j++) {
+        float part = 0.f;
+#pragma unroll
+        for (int g = 0; g < PT / 32; g++) {
+          tile[ty + 8 * j][g * 32 + tx] = v[j][g];
+          part += v[j][g];
+        }
+        if (chan_partial) {
+#pragma unroll
+          for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
+          if (tx == 0 && ty + 8 * j < nc) chan_sum[c0 + ty + 8 * j] += part;
+        }
+      }
+      __syncthreads();
+      const long o0 = (img * HW + p0) * Cp;
 #pragma unroll 8
-    for (int j = ty; j < np; j += 8) {
-      const float a = tile[2 * tx][j] * scale, b = tile[2 * tx + 1][j] * scale;
-      float *px = reinterpret_cast<float *>(dst) + o0 + (long)j * Cp;
-      if (wide) {
-        reinterpret_cast<float2 *>(px + c0)[tx] = make_float2(a, b);
-      } else {
-        __half2 hi, lo;
-        split_pair(a, b, hi, lo);
-        __half2 *h = reinterpret_cast<__half2 *>(px) + c0 / 2 + tx;
-        h[0] = hi;
-        h[Cp / 2] = lo;
+      for (int j = ty; j < np; j += 8) {
+        const float a = tile[2 * tx][j] * scale, b = tile[2 * tx + 1][j] * scale;
+        float *px = reinterpret_cast<float *>(dst) + o0 + (long)j * Cp;
+        if (wide) {
+          reinterpret_cast<float2 *>(px + c0)[tx] = make_float2(a, b);
+        } else {
+          __half2 hi, lo;
+          split_pair(a, b, hi, lo);
+          __half2 *h = reinterpret_cast<__half2 *>(px) + c0 / 2 + tx;
+          h[0] = hi;
+          h[Cp / 2] = lo;
+        }
       }
+      __syncthreads();
     }
+    if (chan_partial)
+      for (int c = threadIdx.x; c < C; c += blockDim.x) chan_partial[(long)block * C + c] = chan_sum[c];
+    form.end(wide, block);
+  }
+};
+// out[c] += scale * sum_b partial[b][c], eight channels a block: 32 row slices per channel, folded in a fixed order.  The partials are a few
+// MB at most; what this pass costs is the chain of dependent loads per thread, hence a sector of channels per block and
+// sixteen loads in flight.
+struct ChanFinishPass {
+  unsigned blocks = 0;
+  const float *partial;
+  int nblocks;
+  long C;
+  float *out, scale;
+  __device__ __forceinline__ void run(unsigned block) const {
+    __shared__ float sm[32][9];
+    const int lane = threadIdx.x & 7, s = threadIdx.x >> 3;
+    const long c = (long)block * 8 + lane;
+    float a[8];
+#pragma unroll
+    for (int i = 0; i < 8; i++) a[i] = 0.f;
+    if (c < C) {
+      int b = s;
+      for (; b + 15 * 32 < nblocks; b += 16 * 32) {
+        float v[16];
+#pragma unroll
+        for (int i = 0; i < 16; i++) v[i] = partial[(long)(b + 32 * i) * C + c];
+#pragma unroll
+        for (int i = 0; i < 16; i++) a[i & 7] += v[i];
+      }
+      if (b + 7 * 32 < nblocks) {
+        float v[8];
+#pragma unroll
+        for (int i = 0; i < 8; i++) v[i] = partial[(long)(b + 32 * i) * C + c];
+#pragma unroll
+        for (int i = 0; i < 8; i++) a[i] += v[i];
+        b += 8 * 32;
+      }
+      float v[7];
+#pragma unroll
+      for (int i = 0; i < 7; i++) v[i] = b + 32 * i < nblocks ? partial[(long)(b + 32 * i) * C + c] : 0.f;
+#pragma unroll
+      for (int i = 0; i < 7; i++)
+        if (b + 32 * i < nblocks) a[0] += v[i];
+    }
+    const float a0 = a[0] + a[4], a1 = a[1] + a[5], a2 = a[2] + a[6], a3 = a[3] + a[7];
+    sm[s][lane] = (a0 + a1) + (a2 + a3);
     __syncthreads();
-  }
-  if (chan_partial)
-    for (int c = threadIdx.x; c < C; c += blockDim.x) chan_partial[(long)blockIdx.x * C + c] = chan_sum[c];
-  form.end(wide);
-}
-// out[c] += scale * sum_b partial[b][c]: 32 row slices per channel (one warp each, eight loads in flight per
-// thread), folded in a fixed order.  The partials are a few MB at most; what this kernel costs is the chain of
-// dependent loads per thread, hence the wide block.
-static __global__ void __launch_bounds__(1024) chan_partial_finish_kernel(const float *__restrict__ partial, int nblocks, long C,
-                                                                          float *out, float scale) {
-  pdl_begin();
-  __shared__ float sm[32][33];
-  const int lane = threadIdx.x & 31, s = threadIdx.x >> 5;
-  const long c = (long)blockIdx.x * 32 + lane;
-  float a[8];
-#pragma unroll
-  for (int i = 0; i < 8; i++) a[i] = 0.f;
-  if (c < C) {
-    int b = s;
-    for (; b + 7 * 32 < nblocks; b += 8 * 32) {
-      float v[8];
-#pragma unroll
-      for (int i = 0; i < 8; i++) v[i] = partial[(long)(b + 32 * i) * C + c];
-#pragma unroll
-      for (int i = 0; i < 8; i++) a[i] += v[i];
+    if (s == 0 && c < C) {
+      float acc = 0.f;
+      for (int k = 0; k < 32; k++) acc += sm[k][lane];
+      out[c] += scale * acc;
     }
-    for (; b < nblocks; b += 32) a[0] += partial[(long)b * C + c];
   }
-  const float a0 = a[0] + a[4], a1 = a[1] + a[5], a2 = a[2] + a[6], a3 = a[3] + a[7];
-  sm[s][lane] = (a0 + a1) + (a2 + a3);
-  __syncthreads();
-  if (s == 0 && c < C) {
-    float acc = 0.f;
-    for (int k = 0; k < 32; k++) acc += sm[k][lane];
-    out[c] += scale * acc;
-  }
-}
-
+};
 
 // A convolution layer restated over "cells": pixel (Y, X) of the restated input carries, as channels, the eH x eW input
 // pixels at offsets (dy, dx) from (Y * dH - pad, X * dW - pad), all planes of each:
@@ -406,14 +462,14 @@ constexpr int kCellTable = 6144;
 // kPairs: [pixel][hi: Cs][lo: Cs], 8 channels a thread.
 template <int PREC, bool TABLE>
 __device__ __forceinline__ void cells_row(const float *__restrict__ in, void *__restrict__ S, long row, const Cells &u, const int2 *chan_src, bool wide,
-                                          float scale) {
+                                          float scale, unsigned part, unsigned parts) {
   constexpr int V = PREC != kTf32 ? 8 : 4;
   const long n = row / u.Hs;
   const int Y = (int)(row - n * u.Hs);
   const int q = u.Cs / V, chunks = u.Ws * q, y0 = Y * u.dH - u.pad;
   const float *img = in + n * u.C * (long)u.H * u.W;
   uint4 *dst = reinterpret_cast<uint4 *>(S) + ((n * u.Hs + Y) * u.Ws) * (long)q * (PREC == kPairs ? 2 : 1);
-  for (int o = blockIdx.y * blockDim.x + threadIdx.x; o < chunks; o += gridDim.y * blockDim.x) {
+  for (int o = part * blockDim.x + threadIdx.x; o < chunks; o += parts * blockDim.x) {
     const int X = o / q, ch0 = (o - X * q) * V, x0 = X * u.dW - u.pad;
     float v[V];
     if constexpr (TABLE) {
@@ -462,30 +518,33 @@ __device__ __forceinline__ void cells_row(const float *__restrict__ in, void *__
   }
 }
 template <int PREC, bool TABLE>
-static __global__ void __launch_bounds__(256) cells_input_kernel(const float *__restrict__ in, void *__restrict__ S, long N, const Cells u,
-                                                                 const PairForm form) {
-  pdl_begin();
-  bool wide = false;
-  float scale = 1.f;
-  if constexpr (PREC == kPairs) {
-    wide = form.ranges.wide();
-    if (!wide) scale = pair_scale(*form.ranges.rec[0]);
-  }
-  extern __shared__ int2 chan_src[];      // per channel: offset in the image, (dy << 16 | dx) or -1
-  if constexpr (TABLE) {
-    for (int ch = threadIdx.x; ch < u.Cs; ch += blockDim.x) {
-      int c, dy, dx;
-      chan_src[ch] = u.channel(ch, c, dy, dx) ? make_int2((c * u.H + dy) * u.W + dx, dy << 16 | dx) : make_int2(0, -1);
+struct CellsPass {
+  unsigned blocks = 0, rows;   // a row of cells is shared by blocks / rows blocks
+  const float *in;
+  void *S;
+  Cells u;
+  PairForm form;
+  __device__ __forceinline__ void run(unsigned block) const {
+    bool wide = false;
+    float scale = 1.f;
+    if constexpr (PREC == kPairs) {
+      wide = form.ranges.wide();
+      if (!wide) scale = pair_scale(*form.ranges.rec[0]);
     }
-    __syncthreads();
+    extern __shared__ float4 pass_sm[];
+    int2 *chan_src = reinterpret_cast<int2 *>(pass_sm);      // per channel: offset in the image, (dy << 16 | dx) or -1
+    if constexpr (TABLE) {
+      for (int ch = threadIdx.x; ch < u.Cs; ch += blockDim.x) {
+        int c, dy, dx;
+        chan_src[ch] = u.channel(ch, c, dy, dx) ? make_int2((c * u.H + dy) * u.W + dx, dy << 16 | dx) : make_int2(0, -1);
+      }
+      __syncthreads();
+    }
+    const unsigned part = block / rows;
+    cells_row<PREC, TABLE>(in, S, block - part * rows, u, chan_src, wide, scale, part, blocks / rows);   // (a loop over rows costs 98 -> 117 us at 256 images)
+    if constexpr (PREC == kPairs) form.end(wide, block);
   }
-  if constexpr (PREC == kPairs) {
-    for (long row = blockIdx.x; row < N * u.Hs; row += gridDim.x) cells_row<PREC, TABLE>(in, S, row, u, chan_src, wide, scale);
-    form.end(wide);
-  } else {
-    cells_row<PREC, TABLE>(in, S, blockIdx.x, u, chan_src, wide, scale);   // (a loop over rows costs 98 -> 117 us at 256 images)
-  }
-}
+};
 
 // The same where a row's input fits shared memory and each thread keeps the channels it writes (Cs / V divides the block): the
 // C * eH input rows are read once, in order, with zeros around them, and every value leaves from there without a bounds check
@@ -493,111 +552,125 @@ static __global__ void __launch_bounds__(256) cells_input_kernel(const float *__
 // conflicts for cells of four columns); for long rows (see restate_input).  3 planes of 224 x 224 as 4 x 4 cells: 1024 images as pairs (1.47 GB) 493 -> 338 us,
 // 256 images in FP32 78 -> 70.
 template <int PREC>
-static __global__ void __launch_bounds__(256) cells_staged_kernel(const float *__restrict__ in, void *__restrict__ S, long N, const Cells u, int Wp, int ld,
-                                                                  const PairForm form) {
-  pdl_begin();
-  bool wide = false;
-  float scale = 1.f;
-  if constexpr (PREC == kPairs) {
-    wide = form.ranges.wide();
-    if (!wide) scale = pair_scale(*form.ranges.rec[0]);
-  }
-  constexpr int V = PREC == kPairs ? 8 : 4;
-  extern __shared__ float rows_in[];   // [C][eH][ld]
-  const int lines = u.C * u.eH, q = u.Cs / V, ch0 = (int)(threadIdx.x % q) * V, lane = threadIdx.x & 31;
-  int at[V];                           // this thread's channels within the window of column 0
-#pragma unroll
-  for (int e = 0; e < V; e++) {
-    int c, dy, dx;
-    at[e] = u.channel(ch0 + e, c, dy, dx) ? (c * u.eH + dy) * ld + dx : -1;
-  }
-  // a warp takes up to 128 columns of four lines at a time, all loads in flight before the first store; its first piece of the next
-  // row is on the way while this row leaves
-  const int warp = threadIdx.x >> 5, parts = (Wp + 127) / 128, pieces = (lines + 3) / 4 * parts;
-  float piece[4][4];
-  auto load = [&](long row, int g) {
-    const long n = row / u.Hs;
-    const int Y = (int)(row - n * u.Hs), y0 = Y * u.dH - u.pad, l0 = g / parts * 4, t0 = (g - g / parts * parts) * 128 + lane;
-    const float *img = in + n * u.C * (long)u.H * u.W;
-#pragma unroll
-    for (int a = 0; a < 4; a++) {
-      const int l = l0 + a, c = l / u.eH, y = y0 + l - c * u.eH;
-      const bool inside = l < lines && (unsigned)y < (unsigned)u.H;
-      const float *src = img + ((long)c * u.H + y) * u.W - u.pad;
-#pragma unroll
-      for (int b = 0; b < 4; b++) piece[a][b] = inside && (unsigned)(t0 + 32 * b - u.pad) < (unsigned)u.W ? __ldg(src + t0 + 32 * b) : 0.f;
+struct StagedCellsPass {
+  unsigned blocks = 0;
+  const float *in;
+  void *S;
+  long N;
+  Cells u;
+  int Wp, ld;
+  PairForm form;
+  __device__ __forceinline__ void run(unsigned block) const {
+    bool wide = false;
+    float scale = 1.f;
+    if constexpr (PREC == kPairs) {
+      wide = form.ranges.wide();
+      if (!wide) scale = pair_scale(*form.ranges.rec[0]);
     }
-  };
-  auto keep = [&](int g) {
-    const int l0 = g / parts * 4, t0 = (g - g / parts * parts) * 128 + lane;
+    constexpr int V = PREC == kPairs ? 8 : 4;
+    extern __shared__ float4 pass_sm[];
+    float *rows_in = reinterpret_cast<float *>(pass_sm);   // [C][eH][ld]
+    const int lines = u.C * u.eH, q = u.Cs / V, ch0 = (int)(threadIdx.x % q) * V, lane = threadIdx.x & 31;
+    int at[V];                           // this thread's channels within the window of column 0
 #pragma unroll
-    for (int a = 0; a < 4; a++)
+    for (int e = 0; e < V; e++) {
+      int c, dy, dx;
+      at[e] = u.channel(ch0 + e, c, dy, dx) ? (c * u.eH + dy) * ld + dx : -1;
+    }
+    // a warp takes up to 128 columns of four lines at a time, all loads in flight before the first store; its first piece of the next
+    // row is on the way while this row leaves
+    const int warp = threadIdx.x >> 5, parts = (Wp + 127) / 128, pieces = (lines + 3) / 4 * parts;
+    float piece[4][4];
+    auto load = [&](long row, int g) {
+      const long n = row / u.Hs;
+      const int Y = (int)(row - n * u.Hs), y0 = Y * u.dH - u.pad, l0 = g / parts * 4, t0 = (g - g / parts * parts) * 128 + lane;
+      const float *img = in + n * u.C * (long)u.H * u.W;
 #pragma unroll
-      for (int b = 0; b < 4; b++)
-        if (l0 + a < lines && t0 + 32 * b < Wp) rows_in[(l0 + a) * ld + t0 + 32 * b] = piece[a][b];
-  };
-  const long rows = N * u.Hs;
-  if (warp < pieces && blockIdx.x < rows) load(blockIdx.x, warp);
-  for (long row = blockIdx.x; row < rows; row += gridDim.x) {
-    if (warp < pieces) keep(warp);
-    for (int g = warp + 8; g < pieces; g += 8) { load(row, g); keep(g); }
-    __syncthreads();
-    if (warp < pieces && row + gridDim.x < rows) load(row + gridDim.x, warp);
-    uint4 *dst = reinterpret_cast<uint4 *>(S) + row * u.Ws * (long)q * (PREC == kPairs ? 2 : 1);
-    for (int X = (int)threadIdx.x / q; X < u.Ws; X += 256 / q) {
-      float v[V];
+      for (int a = 0; a < 4; a++) {
+        const int l = l0 + a, c = l / u.eH, y = y0 + l - c * u.eH;
+        const bool inside = l < lines && (unsigned)y < (unsigned)u.H;
+        const float *src = img + ((long)c * u.H + y) * u.W - u.pad;
 #pragma unroll
-      for (int e = 0; e < V; e++) v[e] = at[e] >= 0 ? rows_in[at[e] + X * u.dW] : 0.f;
-      if (PREC == kPairs && !wide) {
-        __half2 hi[4], lo[4];
-#pragma unroll
-        for (int e = 0; e < 4; e++) split_pair(v[(2 * e) % V] * scale, v[(2 * e + 1) % V] * scale, hi[e], lo[e]);
-        uint4 *d = dst + X * 2l * q + ch0 / V;
-        d[0] = *reinterpret_cast<const uint4 *>(hi);
-        d[q] = *reinterpret_cast<const uint4 *>(lo);
-      } else {
-        float4 *d = reinterpret_cast<float4 *>(dst) + ((long)X * q + ch0 / V) * (V / 4);
-#pragma unroll
-        for (int e = 0; e < V; e += 4) d[e / 4] = make_float4(v[e], v[e + 1], v[e + 2], v[e + 3]);
+        for (int b = 0; b < 4; b++) piece[a][b] = inside && (unsigned)(t0 + 32 * b - u.pad) < (unsigned)u.W ? __ldg(src + t0 + 32 * b) : 0.f;
       }
+    };
+    auto keep = [&](int g) {
+      const int l0 = g / parts * 4, t0 = (g - g / parts * parts) * 128 + lane;
+#pragma unroll
+      for (int a = 0; a < 4; a++)
+#pragma unroll
+        for (int b = 0; b < 4; b++)
+          if (l0 + a < lines && t0 + 32 * b < Wp) rows_in[(l0 + a) * ld + t0 + 32 * b] = piece[a][b];
+    };
+    const long rows = N * u.Hs;
+    if (warp < pieces && block < rows) load(block, warp);
+    for (long row = block; row < rows; row += blocks) {
+      if (warp < pieces) keep(warp);
+      for (int g = warp + 8; g < pieces; g += 8) { load(row, g); keep(g); }
+      __syncthreads();
+      if (warp < pieces && row + blocks < rows) load(row + blocks, warp);
+      uint4 *dst = reinterpret_cast<uint4 *>(S) + row * u.Ws * (long)q * (PREC == kPairs ? 2 : 1);
+      for (int X = (int)threadIdx.x / q; X < u.Ws; X += 256 / q) {
+        float v[V];
+#pragma unroll
+        for (int e = 0; e < V; e++) v[e] = at[e] >= 0 ? rows_in[at[e] + X * u.dW] : 0.f;
+        if (PREC == kPairs && !wide) {
+          __half2 hi[4], lo[4];
+#pragma unroll
+          for (int e = 0; e < 4; e++) split_pair(v[(2 * e) % V] * scale, v[(2 * e + 1) % V] * scale, hi[e], lo[e]);
+          uint4 *d = dst + X * 2l * q + ch0 / V;
+          d[0] = *reinterpret_cast<const uint4 *>(hi);
+          d[q] = *reinterpret_cast<const uint4 *>(lo);
+        } else {
+          float4 *d = reinterpret_cast<float4 *>(dst) + ((long)X * q + ch0 / V) * (V / 4);
+#pragma unroll
+          for (int e = 0; e < V; e += 4) d[e / 4] = make_float4(v[e], v[e + 1], v[e + 2], v[e + 3]);
+        }
+      }
+      __syncthreads();
     }
-    __syncthreads();
+    if constexpr (PREC == kPairs) form.end(wide, block);
   }
-  if constexpr (PREC == kPairs) form.end(wide);
-}
+};
 
 // The column matrix in BF16 with eight channels per tap (Cq = 8, C <= 8): 16 bytes of S are one tap of one pixel.  A block makes
 // the rows of one output row: the kH input rows it needs go to shared memory once, as 16-byte pixels, and leave from there
 // kH * kW times over, so that the kernel is bound by the writes (gathering each value from the image took four times as
 // long: 1105 -> 280 us for 256 images under the 11 x 11 / 4 filter, 1.6 GB).
-static __global__ void __launch_bounds__(256) columns8_kernel(const float *__restrict__ in, uint4 *__restrict__ S, const Cells u) {
-  pdl_begin();
-  extern __shared__ uint4 px_rows[];   // [kH][W + 2 pad]
-  const long n = blockIdx.x / u.Hs;
-  const int Y = (int)(blockIdx.x - n * u.Hs), Wp = u.W + 2 * u.pad, taps = u.kH * u.kW, q = u.Cs / 8;
-  const float *img = in + n * u.C * (long)u.H * u.W;
-  for (int t = threadIdx.x; t < u.kH * Wp; t += blockDim.x) {
-    const int i = t / Wp, y = Y * u.dH + i - u.pad, x = t - i * Wp - u.pad;
-    float v[8];
+struct Columns8Pass {
+  unsigned blocks = 0;
+  const float *in;
+  uint4 *S;
+  Cells u;
+  __device__ __forceinline__ void run(unsigned block) const {
+    extern __shared__ float4 pass_sm[];
+    uint4 *px_rows = reinterpret_cast<uint4 *>(pass_sm);   // [kH][W + 2 pad]
+    const long n = block / u.Hs;
+    const int Y = (int)(block - n * u.Hs), Wp = u.W + 2 * u.pad, taps = u.kH * u.kW, q = u.Cs / 8;
+    const float *img = in + n * u.C * (long)u.H * u.W;
+    for (int t = threadIdx.x; t < u.kH * Wp; t += blockDim.x) {
+      const int i = t / Wp, y = Y * u.dH + i - u.pad, x = t - i * Wp - u.pad;
+      float v[8];
 #pragma unroll
-    for (int c = 0; c < 8; c++)
-      v[c] = c < u.C && (unsigned)y < (unsigned)u.H && (unsigned)x < (unsigned)u.W ? __ldg(img + ((long)c * u.H + y) * u.W + x) : 0.f;
-    __nv_bfloat162 h[4];
+      for (int c = 0; c < 8; c++)
+        v[c] = c < u.C && (unsigned)y < (unsigned)u.H && (unsigned)x < (unsigned)u.W ? __ldg(img + ((long)c * u.H + y) * u.W + x) : 0.f;
+      __nv_bfloat162 h[4];
 #pragma unroll
-    for (int e = 0; e < 4; e++) h[e] = __floats2bfloat162_rn(v[2 * e], v[2 * e + 1]);
-    px_rows[t] = *reinterpret_cast<const uint4 *>(h);
+      for (int e = 0; e < 4; e++) h[e] = __floats2bfloat162_rn(v[2 * e], v[2 * e + 1]);
+      px_rows[t] = *reinterpret_cast<const uint4 *>(h);
+    }
+    __syncthreads();
+    uint4 *dst = S + (n * u.Hs + Y) * u.Ws * (long)q;
+    const int chunks = u.Ws * q, step_x = (int)blockDim.x / q, step_t = (int)blockDim.x - step_x * q;
+    int X = (int)threadIdx.x / q, tap = (int)threadIdx.x - X * q;
+    for (int o = threadIdx.x; o < chunks; o += blockDim.x) {
+      const int i = tap / u.kW, j = tap - i * u.kW;
+      dst[o] = tap < taps ? px_rows[i * Wp + X * u.dW + j] : make_uint4(0, 0, 0, 0);
+      X += step_x; tap += step_t;
+      if (tap >= q) { tap -= q; X++; }
+    }
   }
-  __syncthreads();
-  uint4 *dst = S + (n * u.Hs + Y) * u.Ws * (long)q;
-  const int chunks = u.Ws * q, step_x = (int)blockDim.x / q, step_t = (int)blockDim.x - step_x * q;
-  int X = (int)threadIdx.x / q, tap = (int)threadIdx.x - X * q;
-  for (int o = threadIdx.x; o < chunks; o += blockDim.x) {
-    const int i = tap / u.kW, j = tap - i * u.kW;
-    dst[o] = tap < taps ? px_rows[i * Wp + X * u.dW + j] : make_uint4(0, 0, 0, 0);
-    X += step_x; tap += step_t;
-    if (tap >= q) { tap -= q; X++; }
-  }
-}
+};
 
 // Weights of the restated layer in the k order of the window operand, four values per thread:
 //   FLIP false: out[ko][(bi, bj, ch)]           (forward)
@@ -608,49 +681,55 @@ static __global__ void __launch_bounds__(256) columns8_kernel(const float *__res
 // columns (parity 1, whose window starts one stride later); the new columns are zero.
 // kPairs: a row is [hi: its values][lo: its values].
 template <int PREC, bool FLIP>
-static __global__ void __launch_bounds__(256) repack_weight_kernel(const float *__restrict__ w, const Cells u, int K, int rows, int chans,
-                                                                   int pair_shift, void *__restrict__ out, const Ranges ranges) {
-  pdl_begin();
-  bool wide = false;
-  float scale = 1.f;
-  if constexpr (PREC == kPairs) {
-    wide = ranges.wide();
-    if (!wide) scale = pair_scale(*ranges.rec[0]);
-  }
-  const int kWe = u.kWs + pair_shift, quads = u.kHs * kWe * (chans / 4);
-  const unsigned total = (unsigned)((pair_shift ? 2 : 1) * rows) * (unsigned)quads;
-  for (unsigned t = blockIdx.x * blockDim.x + threadIdx.x; t < total; t += gridDim.x * blockDim.x) {
-    int r = (int)(t / (unsigned)quads);
-    const long row = r;
-    const int k = (int)(t - (unsigned)r * quads) * 4, tap = k / chans, k0 = k - tap * chans;
-    const int par = r >= rows ? 1 : 0;
-    r -= par * rows;
-    int bi = tap / kWe, bj = tap - bi * kWe - par * pair_shift;
-    if (FLIP) { bi = u.kHs - 1 - bi; bj = u.kWs - 1 - bj; }
-    float v[4];
+struct RepackPass {
+  unsigned blocks = 0;
+  const float *w;
+  Cells u;
+  int K, rows, chans, pair_shift;
+  void *out;
+  Ranges ranges;
+  __device__ __forceinline__ void run(unsigned block) const {
+    bool wide = false;
+    float scale = 1.f;
+    if constexpr (PREC == kPairs) {
+      wide = ranges.wide();
+      if (!wide) scale = pair_scale(*ranges.rec[0]);
+    }
+    const int kWe = u.kWs + pair_shift, quads = u.kHs * kWe * (chans / 4);
+    const unsigned total = (unsigned)((pair_shift ? 2 : 1) * rows) * (unsigned)quads;
+    for (unsigned t = block * blockDim.x + threadIdx.x; t < total; t += blocks * blockDim.x) {
+      int r = (int)(t / (unsigned)quads);
+      const long row = r;
+      const int k = (int)(t - (unsigned)r * quads) * 4, tap = k / chans, k0 = k - tap * chans;
+      const int par = r >= rows ? 1 : 0;
+      r -= par * rows;
+      int bi = tap / kWe, bj = tap - bi * kWe - par * pair_shift;
+      if (FLIP) { bi = u.kHs - 1 - bi; bj = u.kWs - 1 - bj; }
+      float v[4];
 #pragma unroll
-    for (int e = 0; e < 4; e++) {
-      const int ch = FLIP ? r : k0 + e, ko = FLIP ? k0 + e : r;
-      int c, dy, dx;
-      const bool real = u.channel(ch, c, dy, dx);
-      const int i = dy + bi * u.stepH, j = dx + bj * u.stepW;
-      v[e] = real && ko < K && bj >= 0 && bj < u.kWs && i < u.kH && j < u.kW ? w[(((long)ko * u.C + c) * u.kH + i) * u.kW + j] : 0.f;
-    }
-    if (PREC == kPairs && !wide) {
-      __half2 hi[2], lo[2];
-      split_pair(v[0] * scale, v[1] * scale, hi[0], lo[0]);
-      split_pair(v[2] * scale, v[3] * scale, hi[1], lo[1]);
-      uint2 *o = reinterpret_cast<uint2 *>(out) + row * 2 * quads + k / 4;
-      o[0] = make_uint2(half2_bits(hi[0]), half2_bits(hi[1]));
-      o[quads] = make_uint2(half2_bits(lo[0]), half2_bits(lo[1]));
-    } else if constexpr (PREC == kBf16) {
-      const __nv_bfloat162 a = __floats2bfloat162_rn(v[0], v[1]), b = __floats2bfloat162_rn(v[2], v[3]);
-      reinterpret_cast<uint2 *>(out)[t] = make_uint2(*reinterpret_cast<const unsigned *>(&a), *reinterpret_cast<const unsigned *>(&b));
-    } else {
-      reinterpret_cast<float4 *>(out)[t] = make_float4(v[0], v[1], v[2], v[3]);
+      for (int e = 0; e < 4; e++) {
+        const int ch = FLIP ? r : k0 + e, ko = FLIP ? k0 + e : r;
+        int c, dy, dx;
+        const bool real = u.channel(ch, c, dy, dx);
+        const int i = dy + bi * u.stepH, j = dx + bj * u.stepW;
+        v[e] = real && ko < K && bj >= 0 && bj < u.kWs && i < u.kH && j < u.kW ? w[(((long)ko * u.C + c) * u.kH + i) * u.kW + j] : 0.f;
+      }
+      if (PREC == kPairs && !wide) {
+        __half2 hi[2], lo[2];
+        split_pair(v[0] * scale, v[1] * scale, hi[0], lo[0]);
+        split_pair(v[2] * scale, v[3] * scale, hi[1], lo[1]);
+        uint2 *o = reinterpret_cast<uint2 *>(out) + row * 2 * quads + k / 4;
+        o[0] = make_uint2(half2_bits(hi[0]), half2_bits(hi[1]));
+        o[quads] = make_uint2(half2_bits(lo[0]), half2_bits(lo[1]));
+      } else if constexpr (PREC == kBf16) {
+        const __nv_bfloat162 a = __floats2bfloat162_rn(v[0], v[1]), b = __floats2bfloat162_rn(v[2], v[3]);
+        reinterpret_cast<uint2 *>(out)[t] = make_uint2(*reinterpret_cast<const unsigned *>(&a), *reinterpret_cast<const unsigned *>(&b));
+      } else {
+        reinterpret_cast<float4 *>(out)[t] = make_float4(v[0], v[1], v[2], v[3]);
+      }
     }
   }
-}
+};
 
 // gw[ko][(c, i, j)] += scale * T at the restated tap and channel of (c, i, j).  ko_stride, ch_stride, bi_stride, bj_stride: where T
 // keeps them (bj counted from the other end when bj_stride is negative: `first` is then the place of tap (0, 0)).
@@ -689,47 +768,55 @@ __device__ __forceinline__ void find_strays(StrayPlaces &s, const Stray *list, i
 }
 // kPairs: with the strays of the input against all of gradOutput, and those of gradOutput against what the planes hold of the input.
 template <bool PAIRS>
-static __global__ void __launch_bounds__(256) unpack_grad_weight_kernel(const float *__restrict__ T, float *__restrict__ gw, const Cells u,
-                                                                        int K, const WgradPlace p, float scale, const WgradStrays q) {
-  pdl_begin();
-  __shared__ StrayPlaces sa, sg;   // (kPairs)
-  int na = 0, ng = 0;
-  float unscale = 1.f;
-  const LayerShape &l = q.l;
-  if constexpr (PAIRS) {
-    const bool wide = q.ranges.wide();
-    na = q.act.strays(wide); ng = q.gout.strays(wide);
-    if (na) find_strays(sa, q.act.list, na, l.C, l.H, l.W, q.n0);
-    if (ng) { find_strays(sg, q.gout.list, ng, l.K, l.oH, l.oW, 0); unscale = pair_unscale(*q.act.rec); }
-    __syncthreads();
-  }
-  const unsigned kHW = (unsigned)(u.kH * u.kW), per = (unsigned)u.C * kHW, total = (unsigned)K * per;
-  for (unsigned t = blockIdx.x * blockDim.x + threadIdx.x; t < total; t += gridDim.x * blockDim.x) {
-    const unsigned ko = t / per, r = t - ko * per, c = r / kHW, tap = r - c * kHW, i = tap / (unsigned)u.kW, j = tap - i * u.kW;
-    const int bi = u.kHs > 1 ? (int)i / u.stepH : 0, bj = u.kWs > 1 ? (int)j / u.stepW : 0;
-    const int dy = (int)i - bi * u.stepH, dx = (int)j - bj * u.stepW;
-    const long ch = (dy * u.eW + dx) * u.Cq + (int)c;
-    const float *s = T + (p.first + ko * p.ko_stride + ch * p.ch_stride + bi * p.bi_stride + bj * p.bj_stride);
-    float sum = *s;
-    for (int b = 1; b < p.copies; b++) sum += s[b * p.copy_stride];
+struct UnpackGradPass {
+  unsigned blocks = 0;
+  const float *T;
+  float *gw;
+  Cells u;
+  int K;
+  WgradPlace p;
+  float scale;
+  WgradStrays q;
+  __device__ __forceinline__ void run(unsigned block) const {
+    __shared__ StrayPlaces sa, sg;   // (kPairs)
+    int na = 0, ng = 0;
+    float unscale = 1.f;
+    const LayerShape &l = q.l;
     if constexpr (PAIRS) {
-      for (int e = 0; e < na; e++) {
-        const StrayPlaces &f = sa;
-        if (f.c[e] != (int)c || f.n[e] < 0 || f.n[e] >= l.N) continue;
-        const int ty = f.y[e] + l.pad - (int)i, tx = f.x[e] + l.pad - (int)j, oy = ty / l.dH, ox = tx / l.dW;
-        if (ty < 0 || tx < 0 || oy * l.dH != ty || ox * l.dW != tx || oy >= l.oH || ox >= l.oW) continue;
-        sum += f.v[e] * q.go[(((long)f.n[e] * l.K + ko) * l.oH + oy) * l.oW + ox];
-      }
-      for (int e = 0; e < ng; e++) {
-        const StrayPlaces &f = sg;
-        if (f.c[e] != (int)ko) continue;
-        const int y = f.y[e] * l.dH + (int)i - l.pad, x = f.x[e] * l.dW + (int)j - l.pad;
-        if ((unsigned)y < (unsigned)l.H && (unsigned)x < (unsigned)l.W) sum += f.v[e] * plane_value(q.planes, u, f.n[e], (int)c, y, x, unscale);
-      }
+      const bool wide = q.ranges.wide();
+      na = q.act.strays(wide); ng = q.gout.strays(wide);
+      if (na) find_strays(sa, q.act.list, na, l.C, l.H, l.W, q.n0);
+      if (ng) { find_strays(sg, q.gout.list, ng, l.K, l.oH, l.oW, 0); unscale = pair_unscale(*q.act.rec); }
+      __syncthreads();
     }
-    gw[t] += scale * sum;
+    const unsigned kHW = (unsigned)(u.kH * u.kW), per = (unsigned)u.C * kHW, total = (unsigned)K * per;
+    for (unsigned t = block * blockDim.x + threadIdx.x; t < total; t += blocks * blockDim.x) {
+      const unsigned ko = t / per, r = t - ko * per, c = r / kHW, tap = r - c * kHW, i = tap / (unsigned)u.kW, j = tap - i * u.kW;
+      const int bi = u.kHs > 1 ? (int)i / u.stepH : 0, bj = u.kWs > 1 ? (int)j / u.stepW : 0;
+      const int dy = (int)i - bi * u.stepH, dx = (int)j - bj * u.stepW;
+      const long ch = (dy * u.eW + dx) * u.Cq + (int)c;
+      const float *s = T + (p.first + ko * p.ko_stride + ch * p.ch_stride + bi * p.bi_stride + bj * p.bj_stride);
+      float sum = *s;
+      for (int b = 1; b < p.copies; b++) sum += s[b * p.copy_stride];
+      if constexpr (PAIRS) {
+        for (int e = 0; e < na; e++) {
+          const StrayPlaces &f = sa;
+          if (f.c[e] != (int)c || f.n[e] < 0 || f.n[e] >= l.N) continue;
+          const int ty = f.y[e] + l.pad - (int)i, tx = f.x[e] + l.pad - (int)j, oy = ty / l.dH, ox = tx / l.dW;
+          if (ty < 0 || tx < 0 || oy * l.dH != ty || ox * l.dW != tx || oy >= l.oH || ox >= l.oW) continue;
+          sum += f.v[e] * q.go[(((long)f.n[e] * l.K + ko) * l.oH + oy) * l.oW + ox];
+        }
+        for (int e = 0; e < ng; e++) {
+          const StrayPlaces &f = sg;
+          if (f.c[e] != (int)ko) continue;
+          const int y = f.y[e] * l.dH + (int)i - l.pad, x = f.x[e] * l.dW + (int)j - l.pad;
+          if ((unsigned)y < (unsigned)l.H && (unsigned)x < (unsigned)l.W) sum += f.v[e] * plane_value(q.planes, u, f.n[e], (int)c, y, x, unscale);
+        }
+      }
+      gw[t] += scale * sum;
+    }
   }
-}
+};
 
 // gin[n][c][h][w] = gS[n][ch][Y][X], the inverse of a fold along both axes (a bijection between the input pixels that any
 // window reaches and the cells' channels; the others get zero).  gS: [N][Cr][Hs][Ws].

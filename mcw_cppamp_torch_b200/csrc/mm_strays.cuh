@@ -4,7 +4,7 @@
 // first.  A block owns the results it changes and takes the strays in their listed order, so that sums repeat exactly.  Without
 // strays, the usual case of all but the largest tensors, a launch looks at two counts and ends (about 2 us as a programmatic
 // dependent); each stray of an activation costs a block about a microsecond, one of the weights a pass over a plane.
-// The weight gradient's are added by unpack_grad_weight_kernel (mm_planes.cuh).
+// The weight gradient's are added by UnpackGradPass (mm_planes.cuh).
 #ifndef THC_MM_STRAYS_CUH
 #define THC_MM_STRAYS_CUH
 
