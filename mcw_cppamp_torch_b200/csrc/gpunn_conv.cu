@@ -327,6 +327,30 @@ static const void *planes_made_from(const THGPUTensor *finput, const float *inpu
   return same ? data_ptr(finput) : nullptr;
 }
 
+// BF16: the forward product of a layer of up to eight planes over windows that the engine gathers from an image of eight-plane pixels, in the
+// k order, the tiles and the k slices of the product over the column matrix, whose bits it gives.  Where nobody keeps that matrix (a weight
+// gradient of the same precision reads it) and its tiles are 64 wide, the widest that K <= 64 comes to.  False: another form.
+static bool gathered_forward(const ConvGeom &g, const mm::Cells &u, const float *in, const float *w, const float *bias, float *out) {
+  using namespace mm;
+  const long rows = (g.oH - 1) * g.dH + g.kH, pitch = (g.oW - 1) * g.dW + g.kW;
+  if (u.direct || u.Cq != 8 || u.kHs != 1 || u.kWs != 1 || g.C > 8 || g.K > 64 || rows * pitch >= 1l << 27 || 16. * (double)(g.N * rows * pitch) > kGroupScratch ||
+      (double)planes_bytes(g.N, g.P, u.Cs, kBf16) > kGroupScratch || !encode_tiled_fn())
+    return false;
+  const auto filter = filter_form<kBf16, false>(forward_windows(g, u), w, u, g.K, g.K, Records{});
+  uint4 *image = (uint4 *)ws_alloc(sizeof(uint4) * g.N * rows * pitch);
+  const long pieces = g.N * rows * ((pitch + 127) / 128);
+  launch_passes(Pixels8Pass{(unsigned)std::min((pieces + 7) / 8, 16l * ctx().sm_count), in, image, g.N, (int)g.C, (int)g.H, (int)g.W, g.pad, (int)rows, (int)pitch}, 0,
+                "pixels8", filter.pass);
+  Problem<GatheredWindowOperand, RawOperand<false, kBf16>, false, kBf16> p;
+  p.a.image = image; p.a.image_pixels = (int)(rows * pitch); p.a.pitch = (int)pitch; p.a.taps = g.kH * g.kW; p.a.kW = g.kW;
+  p.a.rows.set(g.N * g.P, g.P, g.oW);
+  p.a.rows.sy = g.dH; p.a.rows.sx = g.dW;
+  p.epi = Epilogue{out, bias, 1.f, 0.f, g.P, g.K * g.P, g.P};
+  p.M = g.N * g.P; p.N = g.K; p.K = filter.Kd;
+  launch_raw(p, [&](auto &q, int bn2) { attach_raw_map<kBf16>(q.b, filter.pass.out, filter.wrows, filter.Kd, filter.Kd, bn2 / 2); });
+  return true;
+}
+
 template <int PREC>
 static void conv_forward_tc(const ConvGeom &g, const mm::Cells &u, const float *in, const float *w, const float *bias, float *out,
                             THGPUTensor *finput) {
@@ -338,6 +362,7 @@ static void conv_forward_tc(const ConvGeom &g, const mm::Cells &u, const float *
     ConvGeom s = g;
     s.N = std::min(per, g.N - n0);
     const float *x = in + n0 * g.C * g.H * g.W;
+    if (PREC == mm::kBf16 && !finput && gathered_forward(s, u, x, w, bias, out + n0 * g.K * g.P)) continue;
     Records rec;
     if constexpr (PREC == mm::kPairs) {   // (for each group: records last for some thousand words, see zeroed_words)
       rec.act = mm::new_measured(); rec.weight = mm::new_measured();

@@ -247,10 +247,11 @@ static void launch_raw(P p, Attach attach) {
   attach(p, bn2);
   const long gm = (p.M + 255) / 256, gn = (p.N + bn2 - 1) / bn2, tiles = gm * gn;
   int slots = 0;
-  // the widths a problem can come to: 16-bit MN-major 256 and 128, pixel pairs (at most 128 columns) 128 and 64
+  // the widths a problem can come to: 16-bit MN-major 256 and 128, pixel pairs (at most 128 columns) 128 and 64, gathered windows 64
   auto with_width = [&](auto f) {
-    if (bn2 == 128) { f(std::integral_constant<int, 128>()); return; }
-    if constexpr (!P::PAIR) {
+    if constexpr (!P::OpA::GATHERED)
+      if (bn2 == 128) { f(std::integral_constant<int, 128>()); return; }
+    if constexpr (!P::PAIR && !P::OpA::GATHERED) {
       if (bn2 == 256) { f(std::integral_constant<int, 256>()); return; }
       if constexpr (!HALF_MN)
         if (bn2 == 192) { f(std::integral_constant<int, 192>()); return; }

@@ -672,6 +672,39 @@ struct Columns8Pass {
   }
 };
 
+// An image of eight-plane BF16 pixels (planes past C and pixels around the input are zeros) that the windows of a layer cover:
+// [n][rows][pitch], row (y, x) is input pixel (y - pad, x - pad).  See GatheredWindowOperand.  Bound by its writes.
+struct Pixels8Pass {
+  unsigned blocks = 0;
+  const float *in;
+  uint4 *out;
+  long N;
+  int C, H, W, pad, rows, pitch;
+  __device__ __forceinline__ void run(unsigned block) const {
+    const long lines = N * rows;
+    // a warp takes up to 128 pixels of a line, all loads on the way before the first store
+    const int lane = threadIdx.x & 31, parts = (pitch + 127) / 128;
+    for (long l = (long)block * 8 + (threadIdx.x >> 5); l < lines * parts; l += (long)blocks * 8) {
+      const long line = l / parts, n = line / rows;
+      const int x0 = (int)(l - line * parts) * 128 + lane, y = (int)(line - n * rows) - pad;
+      const float *src = in + (n * C * H + y) * (long)W - pad;
+      float v[4][8];
+#pragma unroll
+      for (int a = 0; a < 4; a++)
+#pragma unroll
+        for (int c = 0; c < 8; c++)
+          v[a][c] = c < C && (unsigned)y < (unsigned)H && (unsigned)(x0 + 32 * a - pad) < (unsigned)W ? __ldg(src + (long)c * H * W + x0 + 32 * a) : 0.f;
+#pragma unroll
+      for (int a = 0; a < 4; a++) {
+        __nv_bfloat162 h[4];
+#pragma unroll
+        for (int e = 0; e < 4; e++) h[e] = __floats2bfloat162_rn(v[a][2 * e], v[a][2 * e + 1]);
+        if (x0 + 32 * a < pitch) out[line * pitch + x0 + 32 * a] = *reinterpret_cast<const uint4 *>(h);
+      }
+    }
+  }
+};
+
 // Weights of the restated layer in the k order of the window operand, four values per thread:
 //   FLIP false: out[ko][(bi, bj, ch)]           (forward)
 //   FLIP true : out[ch][(bi', bj', ko)], bi' = kHs - 1 - bi: gradInput as a forward pass over gradOutput (channels padded to

@@ -207,7 +207,7 @@ template <> struct TensorMaps<kPairs> {
 };
 template <bool MN_, int PREC = kTf32>
 struct RawOperand : TensorMaps<PREC> {
-  static constexpr bool MN_MAJOR = MN_;
+  static constexpr bool MN_MAJOR = MN_, GATHERED = false;
 };
 
 // Convolution windows over a channels-last plane [n_img][H][W][C] (C a multiple of KV), as rows (K-major): row = window (img,
@@ -215,7 +215,7 @@ struct RawOperand : TensorMaps<PREC> {
 // one filter tap per load, padding read as zeros.
 template <int PREC = kTf32>
 struct PlanesWindowOperand : TensorMaps<PREC> {
-  static constexpr bool MN_MAJOR = false;
+  static constexpr bool MN_MAJOR = false, GATHERED = false;
   int n_img;
   PixelMap rows;            // window -> coordinates of its corner
   FastDiv C, kW;
@@ -239,12 +239,23 @@ struct PlanesWindowOperand : TensorMaps<PREC> {
   }
 };
 
+// Convolution windows of a layer of up to eight planes in BF16, as rows (K-major): k = (tap, plane), eight planes a tap.  Not by TMA: a tap of a
+// window is 16 bytes of an image of eight-plane pixels (zeros around it where the layer pads), and the engine's warps copy a tile's
+// taps, which lie side by side in the image as far as a filter row reaches, straight to their places in shared memory.
+struct GatheredWindowOperand {
+  static constexpr bool MN_MAJOR = false, GATHERED = true;
+  const uint4 *image;
+  int image_pixels, pitch;  // pixels of an image and of a row
+  int taps, kW;
+  PixelMap rows;            // window -> coordinates of its corner (count, PP, XW, sx, sy)
+};
+
 // The same windows as the MN-major operand of the weight-gradient product: rows = (tap, c), k = windows.  tmap: im2col
 // map, KV channels of KV consecutive windows per load (one KV-row block of a k tile).
 struct WindowStep { int x, y, img; };   // a number of windows as columns, rows and images
 template <int PREC = kTf32>
 struct WindowRowsOperand : TensorMaps<PREC> {
-  static constexpr bool MN_MAJOR = true;
+  static constexpr bool MN_MAJOR = true, GATHERED = false;
   int n_img, oH;
   WindowStep step[2];       // 32 and 64 windows
   PixelMap ks;              // window -> coordinates of its corner

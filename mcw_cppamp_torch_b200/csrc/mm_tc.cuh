@@ -121,6 +121,10 @@ __device__ __forceinline__ void cp_async4(uint32_t dst, const float *src, const 
   const unsigned n = src ? 4u : 0u;
   asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst), "l"((const void *)(src ? src : any_valid)), "r"(n) : "memory");
 }
+// 16 bytes, kept in L1 for the neighbours that read them again; `there` false: zeros, nothing is read
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void *src, bool there) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(there ? 16u : 0u) : "memory");
+}
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N> __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 

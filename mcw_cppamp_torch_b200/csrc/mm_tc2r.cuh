@@ -66,6 +66,7 @@ constexpr int T2_DRAIN_WARP0 = 8;
 constexpr int T2_DRAIN_WARPS = 8;
 constexpr int T2_THREADS = 512;
 constexpr int T2R_HALF_CHAIN = 4;   // BF16: k tiles accumulated in tensor memory before the drain warps fold them
+constexpr int kGatherAhead = 4;     // tiles on the way to a warp that gathers A
 constexpr int T2R_TMA_WARP = 5;
 constexpr int T2R_MMA_WARP2 = 6;
 
@@ -192,6 +193,14 @@ struct TileLoader<ROWS, PREC, WIDE, WindowRowsOperand<OWN>> {
   }
 };
 
+// Windows that the splitter warps gather.
+template <int ROWS, int PREC, bool WIDE>
+struct TileLoader<ROWS, PREC, WIDE, GatheredWindowOperand> {
+  __device__ __forceinline__ TileLoader(const GatheredWindowOperand &, long, long) {}
+  __device__ __forceinline__ void issue(const GatheredWindowOperand &, uint32_t, bool, uint32_t) const {}
+  __device__ __forceinline__ void next(const GatheredWindowOperand &) {}
+};
+
 // ---- item hand-out ------------------------------------------------------------------------------------------
 // The clusters of a launch take their work items from a counter in device memory, first come first served, so a
 // cluster that starts late (its SMs were still busy with another stream's kernel: a collective, a parameter
@@ -207,8 +216,8 @@ constexpr int T2R_SCHED = 8;
 constexpr int T2R_SCHED_WARP = 7;
 constexpr uint32_t T2R_NO_ITEM = 0xffffffffu;
 constexpr int T2R_ITEM_WAIT_SHIFT = 6;   // item-level waits may take 64 k-tile limits (see mbar_wait)
-// readers per slot: TMA thread, 4 splitter warps (16-bit operands: one relay), 8 drain warps in each CTA, the MMA threads in the leader
-template <bool HALF> struct Tc2rReaders { static constexpr uint32_t count = 2 * (1 + (HALF ? 0 : 4) + T2_DRAIN_WARPS) + (HALF ? 1 : 2); };
+// readers per slot: TMA thread, 4 splitter warps (16-bit operands: none, or the 4 that gather A), 8 drain warps in each CTA, the MMA threads in the leader
+template <bool HALF, bool GATHERED> struct Tc2rReaders { static constexpr uint32_t count = 2 * (1 + (HALF && !GATHERED ? 0 : 4) + T2_DRAIN_WARPS) + (HALF ? 1 : 2); };
 
 __device__ __forceinline__ void mbar_arrive_local(uint32_t bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
@@ -249,7 +258,7 @@ struct Tc2rItem {
 template <class P, int BN2, int PREC, bool WIDE>
 __device__ __forceinline__ void tc2r_run(const P &p, const StallCtl &ctl, unsigned *sched_counter) {
   constexpr bool HALF = PREC != kTf32;     // operands of 16 bits: nothing is split here
-  constexpr bool PAIRS = PREC == kPairs;
+  constexpr bool PAIRS = PREC == kPairs, GATHERED = P::OpA::GATHERED;
   constexpr int PARTS = PAIRS ? 2 : 1;     // ring slots of a k tile: lo, then hi, which is needed longest
   constexpr int KV = HALF ? 64 : 32;
   constexpr int CHAIN = PAIRS ? 1 : T2R_HALF_CHAIN;
@@ -308,14 +317,14 @@ __device__ __forceinline__ void tc2r_run(const P &p, const StallCtl &ctl, unsign
   sched.ring = smem_u32(sched_ring);
   if (tid == 0) {
     for (int s = 0; s < R; s++) {
-      mbar_init(bar_full + 8 * s, HALF ? 1 : 2 * T2_PRODUCERS / 64);   // used in CTA 0: its TMA thread and both CTAs' bytes / a group of two splitter warps in each CTA
+      mbar_init(bar_full + 8 * s, GATHERED ? 1 + 2 * T2_PRODUCERS / 32 : HALF ? 1 : 2 * T2_PRODUCERS / 64);   // used in CTA 0: its TMA thread and both CTAs' bytes (and the warps that gather) / a group of two splitter warps in each CTA
       mbar_init(bar_empty + 8 * s, 1);
       mbar_init(bar_raw + 8 * s, 1);                        // this CTA's TMA thread + the bytes it announces
     }
     for (int l = 0; l < L; l++) mbar_init(bar_lo_empty + 8 * l, 1);
     for (int k = 0; k < T2R_SCHED; k++) {
       mbar_init(bar_sched_full + 8 * k, 1);
-      mbar_init(bar_sched_empty + 8 * k, Tc2rReaders<HALF>::count);   // used in CTA 0
+      mbar_init(bar_sched_empty + 8 * k, Tc2rReaders<HALF, GATHERED>::count);   // used in CTA 0
     }
     mbar_init(bar_sched_go, 1);                                // used in CTA 0
     for (int b = 0; b < ACCS; b++) {
@@ -339,7 +348,61 @@ __device__ __forceinline__ void tc2r_run(const P &p, const StallCtl &ctl, unsign
     // ------------------------------------------------------------ splitters
     setmaxnreg_dec<72>();
     const uint32_t full_leader = mapa_shared(bar_full, 0);
-    if constexpr (!HALF) {
+    if constexpr (GATHERED) {
+      // A warp copies 32 windows' taps of a k tile: eight lanes the eight taps of one window, which are 128 bytes of the image where they
+      // belong to one filter row.  kGatherAhead tiles are on the way before the first is waited for, across items.  Bound by these copies, in
+      // L1 and what it misses: 256 images of the 11 x 11 / 4 layer over three planes (us) 305 with 4 tiles ahead, 330 with 2 and half the ring; past
+      // L1 345, and more with more on the way (6: 356, 8: 388).  With the pass that makes the image (54) 359, where the column matrix, written
+      // and read through DRAM at 1.6 GB, took 605.
+      static_assert(PREC == kBf16 && kGatherAhead < R, "k = (tap, 16 bytes); a slot is free before its turn to be announced comes");
+      const uint32_t ring = smem_u32(smem);
+      const int c = lane & 7, r0 = warp * 32 + (lane >> 3);
+      const uint32_t at[2] = {(uint32_t)(r0 * 128 + ((c ^ (lane >> 3)) << 4)), (uint32_t)((r0 + 4) * 128 + ((c ^ ((lane >> 3) + 4)) << 4))};   // 128-byte swizzle
+      uint32_t s = 0, phase = 0, told = 0;
+      int ahead = 0;
+      bool filled = false;
+      auto tell = [&]() {   // the oldest tile not announced yet has landed
+        fence_proxy_async_smem();
+        __syncwarp();
+        if (lane == 0) mbar_arrive_cluster(full_leader + 8 * told);
+        if (++told == R) told = 0;
+      };
+      for (uint32_t n = 0; ok; n++) {
+        uint32_t w = T2R_NO_ITEM;
+        ok = __all_sync(0xffffffffu, sched.next(n, w, abort_flag));
+        if (!ok) break;
+        if (lane == 0) sched.done(n);
+        if (w == T2R_NO_ITEM) break;
+        const Tc2rItem item = item_at(w);
+        const uint4 *row[8];
+#pragma unroll
+        for (int i = 0; i < 8; i++) {
+          const long m = min(item.m_tile0 + (long)rank * TC_BM + r0 + 4 * i, p.M - 1);   // (rows past the end are not stored)
+          unsigned img, px, y, x;
+          p.a.rows.PP.divmod((unsigned)m, img, px);
+          p.a.rows.XW.divmod(px, y, x);
+          row[i] = p.a.image + ((long)img * p.a.image_pixels + (int)y * p.a.rows.sy * p.a.pitch + (int)x * p.a.rows.sx);
+        }
+        int tap = (int)(item.k_begin >> 3) + c, ti = tap / p.a.kW, tj = tap - ti * p.a.kW;
+        for (int t = 0; t < item.num_k_tiles; t++) {
+          if (filled) ok = __all_sync(0xffffffffu, mbar_wait(bar_empty + 8 * s, phase ^ 1u, abort_flag, kWaitSlotEmpty));
+          if (!ok) break;
+          const bool there = tap < p.a.taps;
+          const int off = there ? ti * p.a.pitch + tj : 0;
+          const uint32_t slot = ring + s * Cfg::SLOT_BYTES;
+#pragma unroll
+          for (int i = 0; i < 8; i++) cp_async16(slot + at[i & 1] + (uint32_t)((i >> 1) * 1024), row[i] + off, there);
+          cp_async_commit();
+          if (ahead == kGatherAhead) { cp_async_wait<kGatherAhead>(); tell(); } else ahead++;
+          tap += 8; tj += 8;
+          while (tj >= p.a.kW) { tj -= p.a.kW; ti++; }
+          if (++s == R) { s = 0; phase ^= 1u; filled = true; }
+        }
+      }
+      cp_async_wait<0>();
+      if (ok)
+        for (; ahead > 0; ahead--) tell();
+    } else if constexpr (!HALF) {
     // Two groups of two warps take alternate k tiles, so that one group's barrier round trips and proxy fence
     // overlap the other group's copying: under the MMAs' own shared-memory traffic every access here waits
     // hundreds of cycles.
@@ -519,7 +582,7 @@ __device__ __forceinline__ void tc2r_run(const P &p, const StallCtl &ctl, unsign
         if (w == T2R_NO_ITEM) break;
         if (rank == 0 && lane == 0) mbar_arrive_local(bar_sched_go);   // item n is under way: time to fetch the number of item n + 1
         const Tc2rItem item = item_at(w);
-        TileLoader<TC_BM, PREC, WIDE, typename P::OpA> load_a(p.a, item.m_tile0 + (long)rank * TC_BM, item.k_begin);
+        TileLoader<TC_BM, PREC, WIDE, typename P::OpA> load_a(p.a, item.m_tile0 + (long)rank * TC_BM, item.k_begin);   // (gathered: nothing)
         TileLoader<BH, PREC, WIDE, typename P::OpB> load_b(p.b, item.n_tile0 + (long)rank * BH, item.k_begin);
         for (int t = 0; ok && t < item.num_k_tiles; t++) {
 #pragma unroll
@@ -532,7 +595,7 @@ __device__ __forceinline__ void tc2r_run(const P &p, const StallCtl &ctl, unsign
               uint32_t landed = bar_raw + 8 * s;
               if constexpr (HALF) {
                 landed = full_leader + 8 * s;
-                if (rank == 0) mbar_arrive_expect_tx(bar_full + 8 * s, 2u * Cfg::SLOT_BYTES);
+                if (rank == 0) mbar_arrive_expect_tx(bar_full + 8 * s, 2u * (GATHERED ? Cfg::B_BYTES : Cfg::SLOT_BYTES));
               } else {
                 mbar_arrive_expect_tx(landed, (uint32_t)Cfg::SLOT_BYTES);
               }

@@ -172,3 +172,29 @@ def test_grad_input_of_few_output_planes_does_not_pay_for_padding():
             times.append(a.elapsed_time(b) * 1e3)
         return sorted(times[2:])[2]
     assert us(2) < us(32) / 2
+
+
+@pytest.mark.parametrize("case", [(70, 3, 224, 224, 64, 11, 11, 4, 4, 2), (3, 8, 130, 97, 33, 3, 3, 1, 1, 1), (9, 1, 40, 61, 64, 1, 1, 1, 1, 0), (40, 2, 33, 47, 48, 8, 8, 2, 3, 3),
+                                  (5, 7, 64, 64, 64, 1, 17, 1, 1, 0), (6, 4, 60, 52, 50, 20, 2, 1, 1, 0), (300, 3, 32, 32, 64, 5, 5, 1, 1, 2), (20, 5, 12, 13, 40, 2, 2, 5, 6, 1)])   # (the mode leaves layers of up to 128 windows in FP32)
+def test_bf16_gathered_windows(case):
+    """First layers in BF16, whose taps the engine copies to shared memory itself: taps that fill no k tile, filter rows longer and shorter than one,
+    windows apart and overlapping, last tiles in part.  Products of BF16 values are exact in FP32; K sums, each rounded or truncated once."""
+    import torch
+    import mcw_cppamp_torch_b200 as gt
+    N, C, H, W, K, kH, kW, dH, dW, pad = case
+    g = torch.Generator().manual_seed(sum(case))
+    x, w, b = torch.randn(N, C, H, W, generator=g), torch.randn(K, C, kH, kW, generator=g), torch.randn(K, generator=g)
+    gt.set_math_mode("bf16")
+    try:
+        m = gt.nn.SpatialConvolutionMM(C, K, kW, kH, dW, dH, pad)
+        m.weight, m.bias = w.reshape(K, -1).numpy().copy(), b.numpy().copy()
+        m.gpu()
+        out = torch.from_numpy(m.forward(gt.gpu(x.numpy())).float()).cuda()
+        assert m.finput.dim() == 0
+    finally:
+        gt.set_math_mode("fp32x3")
+
+    def conv(f):
+        q = lambda t: f(t.bfloat16().double()).cuda()
+        return torch.nn.functional.conv2d(q(x), q(w), f(b.double()).cuda(), (dH, dW), pad)
+    assert torch.all((out - conv(lambda t: t)).abs() <= (C * kH * kW + 2) * 2.0 ** -23 * conv(torch.abs))
