@@ -264,7 +264,7 @@ static void window_product(const void *act, const FilterForm<PREC, FLIP> &f, con
 template <int PREC>
 static void restate_input(const ConvGeom &g, const mm::Cells &u, const float *in, void *dst, const mm::PairForm &form,
                           const mm::RepackPass<PREC, false> &repack) {
-  if (u.direct) { mm::make_act_planes<PREC>(in, g.N, g.C, g.H, g.W, dst, false, form, repack, mm::NoPass{}, 0); return; }
+  if (u.direct) { mm::make_act_planes<PREC, false>(in, g.N, g.C, g.H, g.W, dst, form, repack, mm::NoPass{}, 0); return; }
   if constexpr (PREC == mm::kBf16) {
     const size_t smem = sizeof(uint4) * g.kH * (g.W + 2 * g.pad);
     if (u.Cq == 8 && u.kHs == 1 && u.kWs == 1 && g.C <= 8 && smem <= 200 * 1024) {
@@ -716,6 +716,10 @@ static void conv_backward_group(const ConvGeom &g, const mm::Cells &u, bool in_o
   form.ranges = rec.joint(rec.gout);
   FilterForm<PREC, true> filter;
   if (in_ok) filter = grad_input_filter<PREC>(g, w, rec);
+  auto make = [&](const auto &second, size_t more) {
+    return gw ? mm::make_act_planes<PREC, true>(gout, g.N, g.K, g.oH, g.oW, nullptr, form, filter.pass, second, more)
+              : mm::make_act_planes<PREC, false>(gout, g.N, g.K, g.oH, g.oW, nullptr, form, filter.pass, second, more);
+  };
   if (PREC == mm::kPairs) {
     // planes are brought back to FP32 pixel by pixel where that needs no more shared memory than the transposition leaves
     const size_t more = unpair.blocks ? sizeof(float) * std::max(1024, unpair.Cp) : 0;
@@ -726,9 +730,9 @@ static void conv_backward_group(const ConvGeom &g, const mm::Cells &u, bool in_o
     } else if (unpair.blocks) {
       unpair.px = (int)(more / sizeof(float)) / unpair.Cp;
     }
-    if (in_ok || w_ok) pgo = mm::make_act_planes<PREC>(gout, g.N, g.K, g.oH, g.oW, nullptr, gw != nullptr, form, filter.pass, unpair, unpair.blocks ? more : 0);
+    if (in_ok || w_ok) pgo = make(unpair, unpair.blocks ? more : 0);
   } else if (in_ok || w_ok) {
-    pgo = mm::make_act_planes<PREC>(gout, g.N, g.K, g.oH, g.oW, nullptr, gw != nullptr, form, filter.pass, mm::NoPass{}, 0);
+    pgo = make(mm::NoPass{}, 0);
   }
   if (in_ok) {
     conv_grad_input_tc<PREC>(g, pgo, filter, gin, rec);

@@ -396,36 +396,27 @@ static long padded_channels(long C, int prec) { return prec != kTf32 ? (C + 63) 
 static size_t planes_bytes(long N, long HW, long Cp, int prec) { return (size_t)N * HW * Cp * (prec == kBf16 ? 2 : 4); }
 // `dst`: room for planes_bytes(), or null for workspace.  `form`: kPairs.  `first`, `second` (with `more` bytes of shared memory): passes that
 // share the launch.
-template <int PREC, class First, class Second>
-static ActPlanes make_act_planes(const float *src, long N, long C, long H, long W, void *dst, bool want_chan_sums, const PairForm &form, const First &first,
-                                 const Second &second, size_t more) {
+template <int PREC, bool SUMS, class First, class Second>
+static ActPlanes make_act_planes(const float *src, long N, long C, long H, long W, void *dst, const PairForm &form, const First &first, const Second &second,
+                                 size_t more) {
   ActPlanes ap;
   const long HW = H * W;
   ap.N = N; ap.H = H; ap.W = W; ap.Cp = padded_channels(C, PREC);
   ap.p = dst ? dst : ws_alloc(planes_bytes(N, HW, ap.Cp, PREC));
-  const long cap = (long)ctx().sm_count * 16;
-  const bool wide_tile = PREC == kPairs && (HW + 127) / 128 * 128 * 10 <= (HW + 63) / 64 * 64 * 11;
-  const int pt = PREC == kTf32 || wide_tile ? 128 : 64;
-  const long needed = N * ((HW + pt - 1) / pt) * (ap.Cp / (PREC != kTf32 ? 64 : 32));
-  long blocks = std::min(needed, cap);
-  size_t smem = 0;
-  if (want_chan_sums && C <= (wide_tile ? 3968 : 4096)) {   // (with the tile, 48 KB)
-    // every block leaves a row of per-channel sums for a second kernel to fold.  On a small tensor (a few tiles per
-    // block) that fold costs as much as the transposition: a quarter of the blocks keeps it short (measured at
-    // 128 images: fold 83 -> 33 us, transposition unchanged); on a large one the transposition wants all its
-    // blocks (at 1024 images the same cut cost it 3 %, more than the fold gained)
-    if (needed <= 4 * cap && blocks > cap / 4) blocks = cap / 4;
-    ap.chan_blocks = (int)blocks;
-    ap.chan_partial = (float *)ws_alloc(sizeof(float) * blocks * C);
-    smem = sizeof(float) * C;
+  const bool wide_tile = PREC == kTf32 || (HW + 127) / 128 * 128 * 10 <= (HW + 63) / 64 * 64 * 11;
+  const long tiles = N * ((HW + (wide_tile ? 127 : 63)) / (wide_tile ? 128 : 64)), ctiles = ap.Cp / (PREC != kTf32 ? 64 : 32);
+  const long shared = std::max(1l, std::min(tiles, ctx().sm_count * 16l / ctiles));   // blocks that share a tile of channels
+  if (SUMS) {
+    ap.chan_blocks = (int)shared;
+    ap.chan_partial = (float *)ws_alloc(sizeof(float) * shared * C);
   }
-  smem = std::max(smem, more);
-  if constexpr (PREC == kPairs) {
-    if (wide_tile) launch_passes(PairsPass<128>{(unsigned)blocks, src, N, (int)C, (int)HW, (int)ap.Cp, ap.p, ap.chan_partial, form}, smem, "nchw_to_pairs", first, second);
-    else launch_passes(PairsPass<64>{(unsigned)blocks, src, N, (int)C, (int)HW, (int)ap.Cp, ap.p, ap.chan_partial, form}, smem, "nchw_to_pairs", first, second);
-  } else {
-    launch_passes(PlanesPass<PREC == kBf16>{(unsigned)blocks, src, N, (int)C, (int)HW, (int)ap.Cp, ap.p, ap.chan_partial}, smem, "nchw_to_planes", first, second);
-  }
+  auto go = [&](auto pt) {
+    launch_passes(PlanesPass<PREC, decltype(pt)::value, SUMS>{(unsigned)(shared * ctiles), src, N, (int)C, (int)HW, (int)ap.Cp, ap.p, ap.chan_partial, form}, more, "nchw_to_planes", first,
+                  second);
+  };
+  if constexpr (PREC == kTf32) go(std::integral_constant<int, 128>());
+  else if (wide_tile) go(std::integral_constant<int, 128>());
+  else go(std::integral_constant<int, 64>());
   return ap;
 }
 

@@ -168,14 +168,16 @@ static __global__ void __launch_bounds__(256, 5) range_kernel(const RangeJob ja,
 }
 
 // Passes that do not read one another's results share a launch: the blocks of `first`, then those of `second`, then `main`'s.  Each is a
-// struct of its arguments with run(block) and its number of blocks, 256 threads each (none: not asked for).  A launch of its own, by the time
+// struct of its arguments with run(block), its number of blocks of 256 threads (none: not asked for) and how many an SM has to have room for
+// (kPerSM, of `main`).  A launch of its own, by the time
 // the next one has waited for it, costs a small pass two to four microseconds more than its work.
 struct NoPass {
+  static constexpr int kPerSM = 1;
   static constexpr unsigned blocks = 0;
   __device__ __forceinline__ void run(unsigned) const {}
 };
 template <class Main, class First, class Second>
-static __global__ void __launch_bounds__(256) passes_kernel(const __grid_constant__ Main main, const __grid_constant__ First first,
+static __global__ void __launch_bounds__(256, Main::kPerSM) passes_kernel(const __grid_constant__ Main main, const __grid_constant__ First first,
                                                             const __grid_constant__ Second second) {
   pdl_begin();
   unsigned block = blockIdx.x;
@@ -206,6 +208,7 @@ struct PairForm {
 // places stay zero).  A block takes `px` pixels of Cp channels at a time through shared memory.  Not made from the input again:
 // what the input's memory holds may have changed since the planes were written.
 struct UnpairPass {
+  static constexpr int kPerSM = 1;
   unsigned blocks = 0;
   void *planes;
   long pixels;
@@ -236,79 +239,19 @@ struct UnpairPass {
 // ---------------------------------------------------------------------------------------------
 // Channels-last planes of an activation tensor, FP32 or BF16, channels padded with zeros to Cp = a multiple of KV.
 //
-// NCHW fp32 -> [img][pixel][Cp].  CT channels x PT pixels per pass through shared memory, sixteen loads per thread in flight
-// before the barrier (32 x 32 tiles with four left the kernel at half the HBM rate): reads coalesced along pixels, writes in
-// whole 128-byte lines along channels.
-// `chan_partial` (optional): [gridDim.x][C] sums over the pixels this block transposed, per channel -- the gradBias
-// reduction of a convolution rides on the transposition of gradOutput instead of reading the tensor a second time.
-// A channel of a tile belongs to one warp, tiles are taken in a fixed order, so the sums are reproducible.
-template <bool HALF>
+// NCHW fp32 -> [img][pixel][Cp]; kPairs: [img][pixel][hi: Cp][lo: Cp], or FP32 values in the same place.  CT channels x PT pixels per pass through
+// shared memory: reads coalesced along pixels, writes in whole 128-byte lines along channels.  Bound by latency: a thread has 16 or 32
+// loads on the way before the barrier.  128 pixels a pass where they fill it (198 M values as pairs, 1.6 GB: 322 -> 277 us), 64 where
+// planes would leave much of the wider tile empty (13 x 13: 92 us with 128, 83 with 64).
+// SUMS: `chan_partial` is [blocks / channel tiles][C] sums over the pixels that a block transposed, per channel: the gradBias
+// reduction of a convolution rides on the transposition of gradOutput instead of reading the tensor a second time.  A block stays
+// with one tile of channels, so that a thread's sums wait in its registers for the end (folded over the lanes for every
+// tile, and to a row of all C for every block, which had to be fewer for it: 128 images' planes of 13 x 13 and 27 x 27 69 and 82 us for 60 and
+// 70, seven layers of VGG-A at 64 images 507 for 444).  Tiles are taken in a fixed order, the sums are reproducible.
+template <int PREC, int PT, bool SUMS>
 struct PlanesPass {
-  unsigned blocks = 0;
-  const float *src;
-  long N;
-  int C, HW, Cp;
-  void *dst;
-  float *chan_partial;
-  __device__ __forceinline__ void run(unsigned block) const {
-    constexpr int CT = HALF ? 64 : 32, PT = HALF ? 64 : 128;
-    __shared__ float tile[CT][PT + 1];
-    extern __shared__ float4 pass_sm[];
-    float *chan_sum = reinterpret_cast<float *>(pass_sm);   // [C] when chan_partial is given
-    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-    const unsigned ptiles = (unsigned)((HW + PT - 1) / PT), ctiles = (unsigned)(Cp / CT);
-    const long ntiles = N * ptiles * ctiles;
-    if (chan_partial) {
-      for (int c = threadIdx.x; c < C; c += blockDim.x) chan_sum[c] = 0.f;
-      __syncthreads();
-    }
-    for (long t = block; t < ntiles; t += blocks) {
-      const unsigned r = (unsigned)(t % (ptiles * ctiles));
-      const long img = t / (ptiles * ctiles);
-      const int ct = (int)(r / ptiles), p0 = (int)(r - ct * ptiles) * PT, c0 = ct * CT;
-      const int np = min(HW - p0, PT), nc = min(C - c0, CT);
-      const float *s = src + (img * C + c0) * HW + p0 + tx;
-      float v[CT / 8][PT / 32];
-#pragma unroll
-      for (int j = 0; j < CT / 8; j++)
-#pragma unroll
-        for (int g = 0; g < PT / 32; g++)
-          v[j][g] = (g * 32 + tx < np && ty + 8 * j < nc) ? s[(long)(ty + 8 * j) * HW + g * 32] : 0.f;
-#pragma unroll
-      for (int j = 0; j < CT / 8; j++) {
-        float part = 0.f;
-#pragma unroll
-        for (int g = 0; g < PT / 32; g++) {
-          tile[ty + 8 * j][g * 32 + tx] = v[j][g];
-          part += v[j][g];
-        }
-        if (chan_partial) {
-#pragma unroll
-          for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
-          if (tx == 0 && ty + 8 * j < nc) chan_sum[c0 + ty + 8 * j] += part;
-        }
-      }
-      __syncthreads();
-      const long o0 = (img * HW + p0) * Cp + c0;
-#pragma unroll 8
-      for (int j = ty; j < np; j += 8) {
-        if constexpr (HALF)
-          reinterpret_cast<__nv_bfloat162 *>(dst)[(o0 + (long)j * Cp) / 2 + tx] = __floats2bfloat162_rn(tile[2 * tx][j], tile[2 * tx + 1][j]);
-        else
-          reinterpret_cast<float *>(dst)[o0 + (long)j * Cp + tx] = tile[tx][j];
-      }
-      __syncthreads();
-    }
-    if (chan_partial)
-      for (int c = threadIdx.x; c < C; c += blockDim.x) chan_partial[(long)block * C + c] = chan_sum[c];
-  }
-};
-// The same as FP16 pairs, [img][pixel][hi: Cp][lo: Cp], or FP32 values in the same place.  Bound by latency: 128 pixels a pass keep
-// twice the loads in flight (198 M values with channel sums, 1.6 GB: 322 -> 277 us), 64 where planes would leave much of the
-// wider tile empty (13 x 13: 92 us with 128, 83 with 64).
-template <int PT>
-struct PairsPass {
-  unsigned blocks = 0;
+  static constexpr int CT = PREC == kTf32 ? 32 : 64, kPerSM = PT == 128 ? 4 : 5;   // (left alone, 128 registers with sums)
+  unsigned blocks = 0;   // a multiple of the channel tiles, Cp / CT
   const float *src;
   long N;
   int C, HW, Cp;
@@ -316,24 +259,22 @@ struct PairsPass {
   float *chan_partial;
   PairForm form;
   __device__ __forceinline__ void run(unsigned block) const {
-    const bool wide = form.ranges.wide();
-    const float scale = wide ? 1.f : pair_scale(*form.ranges.rec[0]);
-    constexpr int CT = 64;
-    __shared__ float tile[CT][PT + 1];
-    extern __shared__ float4 pass_sm[];
-    float *chan_sum = reinterpret_cast<float *>(pass_sm);   // [C] when chan_partial is given
-    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-    const unsigned ptiles = (unsigned)((HW + PT - 1) / PT), ctiles = (unsigned)(Cp / CT);
-    const long ntiles = N * ptiles * ctiles;
-    if (chan_partial) {
-      for (int c = threadIdx.x; c < C; c += blockDim.x) chan_sum[c] = 0.f;
-      __syncthreads();
+    bool wide = false;
+    float scale = 1.f;
+    if constexpr (PREC == kPairs) {
+      wide = form.ranges.wide();
+      if (!wide) scale = pair_scale(*form.ranges.rec[0]);
     }
-    for (long t = block; t < ntiles; t += blocks) {
-      const unsigned r = (unsigned)(t % (ptiles * ctiles));
-      const long img = t / (ptiles * ctiles);
-      const int ct = (int)(r / ptiles), p0 = (int)(r - ct * ptiles) * PT, c0 = ct * CT;
-      const int np = min(HW - p0, PT), nc = min(C - c0, CT);
+    __shared__ float tile[CT][PT + 1];
+    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+    const unsigned ptiles = (unsigned)((HW + PT - 1) / PT), step = blocks / (unsigned)(Cp / CT), ct = block / step, first = block - ct * step;
+    const int c0 = (int)ct * CT, nc = min(C - c0, CT);
+    float sum[CT / 8];
+#pragma unroll
+    for (int j = 0; j < CT / 8; j++) sum[j] = 0.f;
+    for (long t = first; t < N * ptiles; t += step) {
+      const long img = t / ptiles;
+      const int p0 = (int)(t - img * ptiles) * PT, np = min(HW - p0, PT);
       const float *s = src + (img * C + c0) * HW + p0 + tx;
       float v[CT / 8][PT / 32];
 #pragma unroll
@@ -347,41 +288,50 @@ struct PairsPass {
 #pragma unroll
         for (int g = 0; g < PT / 32; g++) {
           tile[ty + 8 * j][g * 32 + tx] = v[j][g];
-          part += v[j][g];
+          if (SUMS) part += v[j][g];
         }
-        if (chan_partial) {
-#pragma unroll
-          for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
-          if (tx == 0 && ty + 8 * j < nc) chan_sum[c0 + ty + 8 * j] += part;
-        }
+        if (SUMS) sum[j] += part;
       }
       __syncthreads();
-      const long o0 = (img * HW + p0) * Cp;
+      const long o0 = (img * HW + p0) * Cp + c0;
 #pragma unroll 8
       for (int j = ty; j < np; j += 8) {
-        const float a = tile[2 * tx][j] * scale, b = tile[2 * tx + 1][j] * scale;
-        float *px = reinterpret_cast<float *>(dst) + o0 + (long)j * Cp;
-        if (wide) {
-          reinterpret_cast<float2 *>(px + c0)[tx] = make_float2(a, b);
+        if constexpr (PREC == kBf16) {
+          reinterpret_cast<__nv_bfloat162 *>(dst)[(o0 + (long)j * Cp) / 2 + tx] = __floats2bfloat162_rn(tile[2 * tx][j], tile[2 * tx + 1][j]);
+        } else if constexpr (PREC == kPairs) {
+          const float a = tile[2 * tx][j] * scale, b = tile[2 * tx + 1][j] * scale;
+          float *px = reinterpret_cast<float *>(dst) + o0 - c0 + (long)j * Cp;
+          if (wide) {
+            reinterpret_cast<float2 *>(px + c0)[tx] = make_float2(a, b);
+          } else {
+            __half2 hi, lo;
+            split_pair(a, b, hi, lo);
+            __half2 *h = reinterpret_cast<__half2 *>(px) + c0 / 2 + tx;
+            h[0] = hi;
+            h[Cp / 2] = lo;
+          }
         } else {
-          __half2 hi, lo;
-          split_pair(a, b, hi, lo);
-          __half2 *h = reinterpret_cast<__half2 *>(px) + c0 / 2 + tx;
-          h[0] = hi;
-          h[Cp / 2] = lo;
+          reinterpret_cast<float *>(dst)[o0 + (long)j * Cp + tx] = tile[tx][j];
         }
       }
       __syncthreads();
     }
-    if (chan_partial)
-      for (int c = threadIdx.x; c < C; c += blockDim.x) chan_partial[(long)block * C + c] = chan_sum[c];
-    form.end(wide, block);
+    if constexpr (SUMS) {
+#pragma unroll
+      for (int j = 0; j < CT / 8; j++) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) sum[j] += __shfl_xor_sync(0xffffffffu, sum[j], o);
+        if (tx == 0 && ty + 8 * j < nc) chan_partial[(long)first * C + c0 + ty + 8 * j] = sum[j];
+      }
+    }
+    if constexpr (PREC == kPairs) form.end(wide, block);
   }
 };
 // out[c] += scale * sum_b partial[b][c], eight channels a block: 32 row slices per channel, folded in a fixed order.  The partials are a few
 // MB at most; what this pass costs is the chain of dependent loads per thread, hence a sector of channels per block and
 // sixteen loads in flight.
 struct ChanFinishPass {
+  static constexpr int kPerSM = 1;
   unsigned blocks = 0;
   const float *partial;
   int nblocks;
@@ -519,6 +469,7 @@ __device__ __forceinline__ void cells_row(const float *__restrict__ in, void *__
 }
 template <int PREC, bool TABLE>
 struct CellsPass {
+  static constexpr int kPerSM = 1;
   unsigned blocks = 0, rows;   // a row of cells is shared by blocks / rows blocks
   const float *in;
   void *S;
@@ -553,6 +504,7 @@ struct CellsPass {
 // 256 images in FP32 78 -> 70.
 template <int PREC>
 struct StagedCellsPass {
+  static constexpr int kPerSM = 1;
   unsigned blocks = 0;
   const float *in;
   void *S;
@@ -638,6 +590,7 @@ struct StagedCellsPass {
 // kH * kW times over, so that the kernel is bound by the writes (gathering each value from the image took four times as
 // long: 1105 -> 280 us for 256 images under the 11 x 11 / 4 filter, 1.6 GB).
 struct Columns8Pass {
+  static constexpr int kPerSM = 1;
   unsigned blocks = 0;
   const float *in;
   uint4 *S;
@@ -675,6 +628,7 @@ struct Columns8Pass {
 // An image of eight-plane BF16 pixels (planes past C and pixels around the input are zeros) that the windows of a layer cover:
 // [n][rows][pitch], row (y, x) is input pixel (y - pad, x - pad).  See GatheredWindowOperand.  Bound by its writes.
 struct Pixels8Pass {
+  static constexpr int kPerSM = 1;
   unsigned blocks = 0;
   const float *in;
   uint4 *out;
@@ -802,6 +756,7 @@ __device__ __forceinline__ void find_strays(StrayPlaces &s, const Stray *list, i
 // kPairs: with the strays of the input against all of gradOutput, and those of gradOutput against what the planes hold of the input.
 template <bool PAIRS>
 struct UnpackGradPass {
+  static constexpr int kPerSM = 1;
   unsigned blocks = 0;
   const float *T;
   float *gw;
