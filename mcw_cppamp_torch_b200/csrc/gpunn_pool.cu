@@ -397,8 +397,9 @@ static __global__ void __launch_bounds__(256) maxpool2_backward_kernel(const flo
 // 16-byte pieces of that stretch.  Bound by HBM and by the barriers between a block's passes, of which other blocks of the SM make use.  The
 // kernels by rows touch parts of sectors and lines at both ends of a row, which costs most on short rows and, once the tensors have
 // left L2, in DRAM.  Threshold and 3 x 3 pooling in one pass, by rows -> by planes (us; the bytes at the copy rate): 65536 planes of
-// 55 x 55 forward 462 -> 415 (330), backward 584 -> 476 (452); 196608 of 27 x 27 440 -> 296 (236), 600 -> 371 (324); 262144 of 13 x 13
-// 150 -> 93 (72), 194 -> 125 (99).
+// 55 x 55 forward 462 -> 335 (330), backward 584 -> 476 (452); 196608 of 27 x 27 440 -> 235 (236), 600 -> 371 (324); 262144 of 13 x 13
+// 150 -> 74 (72), 194 -> 125 (99).  Forward, five blocks an SM with six pieces of a thread on the way each: four pieces 340, 239, 77; eight without
+// a bound on registers (119 of them, two blocks) 415, 296, 93.
 struct PlaneGeom {
   long planes;
   int G, H, W, HW, oH, oW, P;
@@ -432,7 +433,7 @@ __device__ __forceinline__ void stretch_ends(long start, long end, One one) {
 }
 
 template <int K, bool TH>
-static __global__ void __launch_bounds__(256) maxpool_forward_planes_kernel(const float *__restrict__ in, float *__restrict__ out,
+static __global__ void __launch_bounds__(256, 5) maxpool_forward_planes_kernel(const float *__restrict__ in, float *__restrict__ out,
                                                                             float *__restrict__ indy, float *__restrict__ indx, const PlaneGeom q,
                                                                             const ThresholdPass t) {
   pdl_begin();
@@ -444,7 +445,7 @@ static __global__ void __launch_bounds__(256) maxpool_forward_planes_kernel(cons
     const long p0 = g * q.G, start = p0 * q.HW;
     const int np = (int)min((long)q.G, q.planes - p0);
     const long end = start + (long)np * q.HW, base = start & ~3l;
-    stretch<8>(start, end, [&](long i) { return __ldg(reinterpret_cast<const float4 *>(in + i)); }, [&](long i, float4 v) {
+    stretch<6>(start, end, [&](long i) { return __ldg(reinterpret_cast<const float4 *>(in + i)); }, [&](long i, float4 v) {
       v = make_float4(pass(v.x), pass(v.y), pass(v.z), pass(v.w));
       if (TH) *reinterpret_cast<float4 *>(t.out + i) = v;
       *reinterpret_cast<float4 *>(sm + (i - base)) = v;
@@ -561,9 +562,9 @@ static __global__ void __launch_bounds__(256) maxpool_backward_planes_kernel(con
   }
 }
 // Planes per block, or G = 0 where the kernels by rows do better (us, by rows / by planes, threshold included).
-//   Few pixels: 1024 planes of 55 x 55 (3.1 M) forward 10.4 / 10.9, 8192 (25 M) 63.5 / 58.4; 174 of 43 x 35 backward 6.6 / 7.1.
-//   Forward: rows of more than 32 that start on 8-byte boundaries; 56 116 / 143 (its columns meet in the same banks), 62 12.4 / 13.1,
-//     54 114.6 / 105.5 (3 x 3) and 94 / 96 (2 x 2); 28 67 / 59, 101 225 / 183, 107 x 109 69 / 55.
+//   Few pixels: 174 planes of 43 x 35 (0.3 M) forward 4.7 / 6.3, backward 5.2 / 7.0; 400 of 31 x 100 (1.2 M) 6.5 / 5.5, 6.6 / 5.9; 8192 of 13 x 13 (1.4 M) 8.2 /
+//     6.4, 11.3 / 7.5; 1024 of 55 x 55 (3.1 M) 10.3 / 8.5, 11.0 / 10.0.
+//   Forward: 54 114 / 80, 56 116 / 99 (its columns meet in the same banks), 100 216 / 175; 2 x 2 54 94 / 81, 60 109 / 102, but 100 164 / 169.
 //   Backward: 3 x 3 by planes wherever a group fits; 28 82 / 71, 56 144 / 120.  2 x 2 by rows, which leave in whole sectors for
 //     widths of whole 16-byte pieces and meet in L2 otherwise, as long as the tensors stay there: 28 63 / 78, 14 17.7 / 22, 24576 of 27 x 27 (18 M pixels)
 //     48 / 53, 196608 (143 M) 418 / 354, 65536 of 55 x 55 570 / 468, 262144 of 13 x 13 122 / 129, 16384 of 54 x 54 (48 M) 130 / 119.
@@ -571,8 +572,8 @@ static PlaneGeom plane_geom(long planes, long H, long W, long oH, long oW, int k
   PlaneGeom q = {};
   q.planes = planes; q.H = (int)H; q.W = (int)W; q.HW = (int)std::min(H * W, 1l << 30); q.oH = (int)oH; q.oW = (int)oW; q.P = (int)(oH * oW);
   const long ch = (H + 1) / 2, cw = (W + 1) / 2, ring = (oH + 2) * (oW + 2), bytes = 4 * H * W + (backward ? 8 * ring : 0), pixels = planes * H * W;
-  if (bytes > 47 * 1024 || pixels < 4l << 20) return q;
-  if (!backward && W > 32 && W % 2 == 0) return q;
+  if (bytes > 47 * 1024 || pixels < 1l << 20) return q;
+  if (!backward && k == 2 && W > 64 && W % 2 == 0) return q;
   if (backward && H * W > 1024 * kPlanePieces) return q;
   if (backward && k == 2 && (W % 4 == 0 || W <= 16 || pixels < 40l << 20)) return q;
   q.G = (int)std::max(1l, std::min(backward ? std::min(1024 * kPlanePieces / (H * W), 47 * 1024 / bytes) : 24 * 1024 / bytes, planes / (4l * ctx().sm_count)));

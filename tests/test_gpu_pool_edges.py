@@ -76,7 +76,7 @@ def test_threshold_and_pooling_in_one_pass(shape, k):
 # Tensors large enough for the kernels that take whole planes: widths on both sides of the rules, planes and groups that do not come out even.
 @pytest.mark.parametrize("k", [2, 3])
 @pytest.mark.parametrize("shape", [(67, 401, 13, 13), (23, 257, 27, 29), (31, 1000, 9, 16), (9, 191, 55, 55), (5, 101, 101, 97), (7, 230, 51, 54), (4700, 90, 10, 10),
-                                   (331, 170, 29, 27), (90000, 7, 9, 8), (5, 100000, 3, 3), (1501, 3, 31, 32)])
+                                   (331, 170, 29, 27), (90000, 7, 9, 8), (5, 100000, 3, 3), (1501, 3, 31, 32), (3, 100, 60, 62), (2, 99, 84, 66)])
 def test_whole_planes(oracle_port, shape, k):
     import mcw_cppamp_torch_b200 as gt
     g = np.random.default_rng(sum(shape) + 3 * k)
