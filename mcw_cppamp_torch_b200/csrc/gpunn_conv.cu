@@ -433,10 +433,8 @@ static void conv_grad_input_tc(const ConvGeom &g, const mm::ActPlanes &pgo, cons
   if (u.direct) { window_product(pgo.p, filter, nullptr, gin, rec); return; }
   float *gS = (float *)ws_alloc(sizeof(float) * g.N * u.Cr * (long)(u.Hs * u.Ws));
   window_product(pgo.p, filter, nullptr, gS, rec);
-  const long planes = g.N * g.C;
-  const unsigned bx = (unsigned)std::min<long>((g.H * g.W + 255) / 256, 64);
-  const unsigned by = (unsigned)std::min<long>(planes, std::max<long>(1, ctx().sm_count * 32l / bx));
-  pdl_launch(mm::unfold_grad_input_kernel, dim3(bx, by), 256, 0, gS, gin, g.N, u);
+  const long lines = g.N * g.C * g.H;
+  pdl_launch(mm::unfold_grad_input_kernel, (unsigned)std::min((lines + 7) / 8, ctx().sm_count * 16l), 256, 0, gS, gin, g.N, u, mm::FastDiv::make(u.dW));
   check_launch("unfold_grad_input");
 }
 

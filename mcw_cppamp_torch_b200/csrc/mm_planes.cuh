@@ -808,21 +808,23 @@ struct UnpackGradPass {
 
 // gin[n][c][h][w] = gS[n][ch][Y][X], the inverse of a fold along both axes (a bijection between the input pixels that any
 // window reaches and the cells' channels; the others get zero).  gS: [N][Cr][Hs][Ws].
+// A warp takes a line of the image: what belongs to the line is worked out once, and a column costs one division by multiplication (four in
+// hardware for every pixel: 14.7 us for 16 images of 3 x 224 x 224 from cold caches, 11.3 so).
 static __global__ void __launch_bounds__(256) unfold_grad_input_kernel(const float *__restrict__ gS, float *__restrict__ gin, long N,
-                                                                       const Cells u) {
+                                                                       const Cells u, const FastDiv ddW) {
   pdl_begin();
-  const unsigned HW = (unsigned)(u.H * u.W);
-  const long planes = N * u.C;
-  for (long pl = blockIdx.y; pl < planes; pl += gridDim.y) {
-    const long n = pl / u.C;
-    const int c = (int)(pl - n * u.C);
-    const float *src = gS + n * u.Cr * (long)(u.Hs * u.Ws);
-    for (unsigned t = blockIdx.x * blockDim.x + threadIdx.x; t < HW; t += gridDim.x * blockDim.x) {
-      const int h = (int)(t / (unsigned)u.W) + u.pad, w = (int)(t % (unsigned)u.W) + u.pad;
-      const int Y = h / u.dH, dy = h - Y * u.dH, X = w / u.dW, dx = w - X * u.dW;
-      float v = 0.f;
-      if (Y < u.Hs && X < u.Ws && dy < u.eH && dx < u.eW) v = src[((long)((dy * u.eW + dx) * u.Cq + c) * u.Hs + Y) * u.Ws + X];
-      gin[pl * HW + t] = v;
+  const int lane = threadIdx.x & 31;
+  const long lines = N * u.C * u.H, step = (long)u.Hs * u.Ws;
+  for (long line = (long)blockIdx.x * 8 + (threadIdx.x >> 5); line < lines; line += (long)gridDim.x * 8) {
+    const long pl = line / u.H, n = pl / u.C;
+    const int c = (int)(pl - n * u.C), h = (int)(line - pl * u.H) + u.pad, Y = h / u.dH, dy = h - Y * u.dH;
+    const bool reached = Y < u.Hs && dy < u.eH;
+    const float *src = gS + (n * u.Cr + (long)dy * u.eW * u.Cq + c) * step + (long)Y * u.Ws;
+#pragma unroll 4
+    for (int x = lane; x < u.W; x += 32) {
+      unsigned X, dx;
+      ddW.divmod((unsigned)(x + u.pad), X, dx);
+      gin[line * u.W + x] = reached && (int)X < u.Ws && (int)dx < u.eW ? __ldg(src + (long)dx * u.Cq * step + X) : 0.f;
     }
   }
 }
