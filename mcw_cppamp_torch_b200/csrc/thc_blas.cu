@@ -255,8 +255,21 @@ static __global__ void __launch_bounds__(1024) gemv_n_kernel(long m, long n, flo
   __shared__ float part[32][33];
   const long i = (long)blockIdx.x * 32 + threadIdx.x;
   float acc = 0.f;
-  if (i < m)
-    for (long j = threadIdx.y; j < n; j += 32) acc = fmaf(a[i + j * lda], x[j * incx], acc);
+  if (i < m) {
+    // eight columns on the way at once, added in their order (gradBias of three layers over 256 rows 21 -> 15 us)
+    for (long j0 = threadIdx.y; j0 < n; j0 += 8 * 32) {
+      float v[8], w[8];
+#pragma unroll
+      for (int k = 0; k < 8; k++) {
+        const long j = j0 + 32 * k;
+        v[k] = j < n ? a[i + j * lda] : 0.f;
+        w[k] = j < n ? x[j * incx] : 0.f;
+      }
+#pragma unroll
+      for (int k = 0; k < 8; k++)
+        if (j0 + 32 * k < n) acc = fmaf(v[k], w[k], acc);
+    }
+  }
   part[threadIdx.y][threadIdx.x] = acc;
   __syncthreads();
   if (threadIdx.y == 0 && i < m) {
