@@ -715,7 +715,8 @@ static void conv_backward_group(const ConvGeom &g, const mm::Cells &u, bool in_o
   FilterForm<PREC, true> filter;
   if (in_ok) filter = grad_input_filter<PREC>(g, w, rec);
   auto make = [&](const auto &second, size_t more) {
-    return gw ? mm::make_act_planes<PREC, true>(gout, g.N, g.K, g.oH, g.oW, nullptr, form, filter.pass, second, more)
+    // (the sums and the tile, 48 KB)
+    return gw && g.K <= 3968 ? mm::make_act_planes<PREC, true>(gout, g.N, g.K, g.oH, g.oW, nullptr, form, filter.pass, second, more)
               : mm::make_act_planes<PREC, false>(gout, g.N, g.K, g.oH, g.oW, nullptr, form, filter.pass, second, more);
   };
   if (PREC == mm::kPairs) {

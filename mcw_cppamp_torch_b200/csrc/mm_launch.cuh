@@ -403,15 +403,20 @@ static ActPlanes make_act_planes(const float *src, long N, long C, long H, long 
   const long HW = H * W;
   ap.N = N; ap.H = H; ap.W = W; ap.Cp = padded_channels(C, PREC);
   ap.p = dst ? dst : ws_alloc(planes_bytes(N, HW, ap.Cp, PREC));
-  const bool wide_tile = PREC == kTf32 || (HW + 127) / 128 * 128 * 10 <= (HW + 63) / 64 * 64 * 11;
-  const long tiles = N * ((HW + (wide_tile ? 127 : 63)) / (wide_tile ? 128 : 64)), ctiles = ap.Cp / (PREC != kTf32 ? 64 : 32);
-  const long shared = std::max(1l, std::min(tiles, ctx().sm_count * 16l / ctiles));   // blocks that share a tile of channels
+  // (BF16 with sums: 64 pixels, whose sums are as they always were)
+  const bool wide_tile = PREC == kTf32 || ((PREC == kPairs || !SUMS) && (HW + 127) / 128 * 128 * 10 <= (HW + 63) / 64 * 64 * 11);
+  const long cap = ctx().sm_count * 16l, needed = N * ((HW + (wide_tile ? 127 : 63)) / (wide_tile ? 128 : 64)) * (ap.Cp / (PREC != kTf32 ? 64 : 32));
+  long blocks = std::min(needed, cap);
   if (SUMS) {
-    ap.chan_blocks = (int)shared;
-    ap.chan_partial = (float *)ws_alloc(sizeof(float) * shared * C);
+    // every block leaves a row of per-channel sums to fold, which on a small tensor (a few tiles per block) costs as much as the
+    // transposition: a quarter of the blocks keeps it short; a large one wants all its blocks (at 1024 images the same cut cost it 3 %)
+    if (needed <= 4 * cap && blocks > cap / 4) blocks = cap / 4;
+    ap.chan_blocks = (int)blocks;
+    ap.chan_partial = (float *)ws_alloc(sizeof(float) * blocks * C);
+    more = std::max(more, sizeof(float) * C);
   }
   auto go = [&](auto pt) {
-    launch_passes(PlanesPass<PREC, decltype(pt)::value, SUMS>{(unsigned)(shared * ctiles), src, N, (int)C, (int)HW, (int)ap.Cp, ap.p, ap.chan_partial, form}, more, "nchw_to_planes", first,
+    launch_passes(PlanesPass<PREC, decltype(pt)::value, SUMS>{(unsigned)blocks, src, N, (int)C, (int)HW, (int)ap.Cp, ap.p, ap.chan_partial, form}, more, "nchw_to_planes", first,
                   second);
   };
   if constexpr (PREC == kTf32) go(std::integral_constant<int, 128>());

@@ -243,15 +243,15 @@ struct UnpairPass {
 // shared memory: reads coalesced along pixels, writes in whole 128-byte lines along channels.  Bound by latency: a thread has 16 or 32
 // loads on the way before the barrier.  128 pixels a pass where they fill it (198 M values as pairs, 1.6 GB: 322 -> 277 us), 64 where
 // planes would leave much of the wider tile empty (13 x 13: 92 us with 128, 83 with 64).
-// SUMS: `chan_partial` is [blocks / channel tiles][C] sums over the pixels that a block transposed, per channel: the gradBias
-// reduction of a convolution rides on the transposition of gradOutput instead of reading the tensor a second time.  A block stays
-// with one tile of channels, so that a thread's sums wait in its registers for the end (folded over the lanes for every
-// tile, and to a row of all C for every block, which had to be fewer for it: 128 images' planes of 13 x 13 and 27 x 27 69 and 82 us for 60 and
-// 70, seven layers of VGG-A at 64 images 507 for 444).  Tiles are taken in a fixed order, the sums are reproducible.
+// SUMS: `chan_partial` is [blocks][C] sums over the pixels that a block transposed, per channel: the gradBias
+// reduction of a convolution rides on the transposition of gradOutput instead of reading the tensor a second time.
+// A channel of a tile belongs to one warp, tiles are taken in a fixed order, so the sums are reproducible.  Blocks that stay with one tile of
+// channels and keep the sums in registers to the end save 15 % of the pass (a per cent of a step of 128 images), but another order of these
+// sums is another training run: of small batches, one that ends in NaN where this one does not, or the other way round.
 template <int PREC, int PT, bool SUMS>
 struct PlanesPass {
   static constexpr int CT = PREC == kTf32 ? 32 : 64, kPerSM = PT == 128 ? 4 : 5;   // (left alone, 128 registers with sums)
-  unsigned blocks = 0;   // a multiple of the channel tiles, Cp / CT
+  unsigned blocks = 0;
   const float *src;
   long N;
   int C, HW, Cp;
@@ -266,15 +266,20 @@ struct PlanesPass {
       if (!wide) scale = pair_scale(*form.ranges.rec[0]);
     }
     __shared__ float tile[CT][PT + 1];
+    extern __shared__ float4 pass_sm[];
+    float *chan_sum = reinterpret_cast<float *>(pass_sm);   // [C] (SUMS)
     const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-    const unsigned ptiles = (unsigned)((HW + PT - 1) / PT), step = blocks / (unsigned)(Cp / CT), ct = block / step, first = block - ct * step;
-    const int c0 = (int)ct * CT, nc = min(C - c0, CT);
-    float sum[CT / 8];
-#pragma unroll
-    for (int j = 0; j < CT / 8; j++) sum[j] = 0.f;
-    for (long t = first; t < N * ptiles; t += step) {
-      const long img = t / ptiles;
-      const int p0 = (int)(t - img * ptiles) * PT, np = min(HW - p0, PT);
+    const unsigned ptiles = (unsigned)((HW + PT - 1) / PT), ctiles = (unsigned)(Cp / CT);
+    const long ntiles = N * ptiles * ctiles;
+    if constexpr (SUMS) {
+      for (int c = threadIdx.x; c < C; c += blockDim.x) chan_sum[c] = 0.f;
+      __syncthreads();
+    }
+    for (long t = block; t < ntiles; t += blocks) {
+      const unsigned r = (unsigned)(t % (ptiles * ctiles));
+      const long img = t / (ptiles * ctiles);
+      const int ct = (int)(r / ptiles), p0 = (int)(r - ct * ptiles) * PT, c0 = ct * CT;
+      const int np = min(HW - p0, PT), nc = min(C - c0, CT);
       const float *s = src + (img * C + c0) * HW + p0 + tx;
       float v[CT / 8][PT / 32];
 #pragma unroll
@@ -290,7 +295,11 @@ struct PlanesPass {
           tile[ty + 8 * j][g * 32 + tx] = v[j][g];
           if (SUMS) part += v[j][g];
         }
-        if (SUMS) sum[j] += part;
+        if constexpr (SUMS) {
+#pragma unroll
+          for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
+          if (tx == 0 && ty + 8 * j < nc) chan_sum[c0 + ty + 8 * j] += part;
+        }
       }
       __syncthreads();
       const long o0 = (img * HW + p0) * Cp + c0;
@@ -316,14 +325,8 @@ struct PlanesPass {
       }
       __syncthreads();
     }
-    if constexpr (SUMS) {
-#pragma unroll
-      for (int j = 0; j < CT / 8; j++) {
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) sum[j] += __shfl_xor_sync(0xffffffffu, sum[j], o);
-        if (tx == 0 && ty + 8 * j < nc) chan_partial[(long)first * C + c0 + ty + 8 * j] = sum[j];
-      }
-    }
+    if constexpr (SUMS)
+      for (int c = threadIdx.x; c < C; c += blockDim.x) chan_partial[(long)block * C + c] = chan_sum[c];
     if constexpr (PREC == kPairs) form.end(wide, block);
   }
 };
