@@ -46,8 +46,9 @@ static ConvGeom conv_geom(const THGPUTensor *input, const THGPUTensor *weight, i
 }
 
 // What the planes kept in a module's `finput` were made from.  accGradParameters reuses them only when it is
-// handed the very input (same device memory, same layer and precision) that the forward pass transposed; a forward pass
-// that does not write `finput` forgets the entry, so planes of an earlier pass are never taken for fresh ones.
+// handed the very input (same device memory, same layer and precision) that the forward pass transposed; every forward pass
+// begins by forgetting the entry, so that planes of an earlier pass are never taken for those of one that does not write `finput`,
+// or that fails: what the input's memory holds may have changed since.
 // Keyed by the address of finput's data; one table per host thread, as the rest of the library's state.
 namespace {
 // Pairs have a record (mm::KeptRange), `record` of the context's (plane_record); the slots belong to the entries of this table.
@@ -73,6 +74,11 @@ void forget_planes(const THGPUTensor *finput) {
   if (it->second.record >= 0) g_free_records.push_back(it->second.record);
   g_plane_stamps.erase(it);
 }
+// Planes that are marked as made ahead of the launch that makes them: not any more, should that launch not come about.
+struct UnmadePlanes {
+  const THGPUTensor *finput;
+  ~UnmadePlanes() { forget_planes(finput); }
+};
 // The record of planes that are known to be fresh.
 mm::KeptRange *planes_record(const void *planes) { return (mm::KeptRange *)plane_record(g_plane_stamps.at((const float *)planes).record); }
 }  // namespace
@@ -355,7 +361,7 @@ template <int PREC>
 static void conv_forward_tc(const ConvGeom &g, const mm::Cells &u, const float *in, const float *w, const float *bias, float *out,
                             THGPUTensor *finput) {
   const double bytes = (double)mm::planes_bytes(1, (long)u.Hs * u.Ws, u.Cs, PREC), floats = (double)g.N * g.C * g.H * g.W;
-  if (finput && bytes * (double)g.N > whole_scratch(floats)) { forget_planes(finput); finput = nullptr; }
+  if (finput && bytes * (double)g.N > whole_scratch(floats)) finput = nullptr;
   const long per = finput ? g.N : images_per_group(g.N, bytes, kGroupScratch);
   for (long n0 = 0; n0 < g.N; n0 += per) {
     WsScope ws_scope;
@@ -371,11 +377,13 @@ static void conv_forward_tc(const ConvGeom &g, const mm::Cells &u, const float *
     }
     mm::PairForm form;
     form.ranges = rec.joint(rec.act);
+    const auto filter = filter_form<PREC, false>(forward_windows(s, u), w, u, g.K, g.K, rec);
     void *act = finput ? planes_in(finput, s, u, x, PREC) : nullptr;
+    UnmadePlanes unmade{act ? finput : nullptr};
     if (act && PREC == mm::kPairs) { form.keep = planes_record(act); form.list = rec.act.list; }
     if (!act) act = ws_alloc(mm::planes_bytes(s.N, (long)u.Hs * u.Ws, u.Cs, PREC));
-    const auto filter = filter_form<PREC, false>(forward_windows(s, u), w, u, g.K, g.K, rec);
     restate_input<PREC>(s, u, x, act, form, filter.pass);
+    unmade.finput = nullptr;
     window_product(act, filter, bias, out + n0 * g.K * g.P, rec);
     if (PREC == mm::kPairs) add_strays<false>(s, x, w, out + n0 * g.K * g.P, rec);
   }
@@ -686,7 +694,6 @@ static void conv_forward(const ConvGeom &g, const float *in, const float *w, con
       restate_accurate(g, true, uw, pw);
       if (pw != prec) keep = nullptr;
     }
-    if (!keep) forget_planes(finput);
     if (prec == mm::kPairs) {
       try {
         conv_forward_tc<mm::kPairs>(g, u, in, w, bias, out, keep);
@@ -699,7 +706,6 @@ static void conv_forward(const ConvGeom &g, const float *in, const float *w, con
     else conv_forward_tc<mm::kTf32>(g, u, in, w, bias, out, keep);
     return;
   }
-  forget_planes(finput);   // this pass leaves finput alone: what it holds belongs to an earlier input
   conv_forward_simt(g, in, w, bias, out);
 }
 
@@ -856,6 +862,7 @@ THC_API int THGPUNN_SpatialConvolutionMM_updateOutput(THGPUTensor *input, THGPUT
     THGPUTensor *bias, THGPUTensor *finput, THGPUTensor *fgradInput, int kW, int kH, int dW, int dH, int padding) {
   (void)fgradInput;
   THC_BEGIN
+  forget_planes(finput);
   WsScope ws_scope;
   const ConvGeom g = conv_geom(input, weight, kW, kH, dW, dH, padding);
   THC_ARG(bias->nDimension == 1 && bias->size[0] == g.K, 1, "bias must have nOutputPlane entries");

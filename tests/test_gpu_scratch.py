@@ -178,7 +178,54 @@ for got, a, b in zip((out, gi), want, mass):
 """
 
 
-@pytest.mark.parametrize("program", [FULL_DEVICE, FULL_DEVICE_CONVOLUTION])
+# A forward pass that fails leaves no planes: neither one that ends for want of memory (the filter's form comes before the planes are
+# made) nor one over new values in the input's memory (the planes of the old ones).
+REFUSED_FORWARD = """
+import torch, mcw_cppamp_torch_b200 as gt
+from test_gpu_fp16_pairs import randn
+from test_gpu_scratch import wrap
+N, C, H, K, k = 4, 1024, 8, 8192, 3
+x, w, go = randn(1, N, C, H, H), randn(2, K, C * k * k), randn(3, N, K, H, H)
+small, gs = randn(4, 256, C * k * k), randn(5, N, 256, H, H)
+out = [torch.empty(N, p, H, H, device="cuda") for p in (K, 256)]
+grad = [[torch.zeros_like(f) for f in (w, small)] for _ in range(2)]
+bias = torch.zeros(K, device="cuda")
+def layer(filters, output, gradWeight):
+    m = gt.nn.SpatialConvolutionMM(1, 1, 1, 1).gpu()
+    m.kW, m.kH, m.padding = k, k, 1
+    m.weight, m.bias, m.output, m.gradWeight = wrap(gt, filters), wrap(gt, bias[:len(filters)]), wrap(gt, output), wrap(gt, gradWeight)
+    m.gradBias = wrap(gt, torch.zeros(len(filters), device="cuda"))
+    return m
+X = wrap(gt, x)
+gt.set_math_mode("bf16")
+first, second = layer(w, out[0], grad[0][0]), layer(small, out[1], grad[0][1])
+second.forward(X)                      # 4.7 MB of filters, and planes of x
+assert second.finput.dim() == 5
+gt.synchronize()
+x.mul_(-1.5)
+torch.cuda.synchronize()
+torch.cuda.empty_cache()
+full = torch.empty(torch.cuda.mem_get_info()[0] - (96 << 20), dtype=torch.uint8, device="cuda")     # the filter's form: 151 MB
+second.bias = first.bias
+for m, why in ((first, "no room"), (second, "bias")):
+    try:
+        m.forward(X)
+    except gt.THCError as e:
+        assert why in str(e), e
+    else:
+        raise AssertionError("nothing failed")
+del full
+torch.cuda.empty_cache()
+for m, g in ((first, go), (second, gs)):
+    m.accGradParameters(X, wrap(gt, g))
+for m, f, g, o in ((layer(w, out[0], grad[1][0]), w, go, 0), (layer(small, out[1], grad[1][1]), small, gs, 1)):
+    m.accGradParameters(X, wrap(gt, g))
+    gt.synchronize()
+    assert grad[1][o].abs().max() > 1 and torch.equal(grad[0][o], grad[1][o]), o
+"""
+
+
+@pytest.mark.parametrize("program", [FULL_DEVICE, FULL_DEVICE_CONVOLUTION, REFUSED_FORWARD])
 def test_product_on_a_full_device(gt, program):  # noqa: F811
     """Pairs are copies; where there is no room for them the product runs over the operands as they lie, or planes in FP32 where those are
     smaller.  (A process of its own: this one's workspace has grown already.)"""
