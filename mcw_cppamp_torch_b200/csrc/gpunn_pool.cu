@@ -795,12 +795,20 @@ THC_API int THGPUNN_SpatialMaxPooling_updateGradInput(THGPUTensor *input, THGPUT
 
 // nn.Threshold followed by nn.SpatialMaxPooling.  What the two entry points in turn give, to the bit, and by them wherever the pass over
 // both does not apply: other windows, strided or overlapping tensors, arguments that one of them refuses.
-static bool own_storage(const THGPUTensor *t, std::initializer_list<const THGPUTensor *> others) {
-  for (const THGPUTensor *o : others)
-    if (o == t || (t->storage && o->storage == t->storage)) return false;
+// Whether resizing and writing any of `results` leaves the others and `sources` as they are: no storage is shared, and none of a result's memory,
+// which goes back when the result outgrows it, is borrowed by another (THGPUStorage_newWithData).  `sources`: contiguous.
+static bool apart(std::initializer_list<const THGPUTensor *> results, std::initializer_list<const THGPUTensor *> sources) {
+  auto meets = [](const THGPUTensor *r, const THGPUTensor *o, const float *a, long n) {
+    return o == r || (r->storage && (o->storage == r->storage || (a && a < r->storage->data + r->storage->size && r->storage->data < a + n)));
+  };
+  for (const THGPUTensor *r : results) {
+    for (const THGPUTensor *o : results)
+      if (o < r && meets(r, o, o->storage ? o->storage->data : nullptr, o->storage ? o->storage->size : 0)) return false;
+    for (const THGPUTensor *o : sources)
+      if (meets(r, o, data_ptr(o), nelem(o))) return false;
+  }
   return true;
 }
-static bool apart(const float *a, long na, const float *b, long nb) { return a + na <= b || b + nb <= a; }
 static bool pooled_shape(const THGPUTensor *t, int kW, int kH, int dW, int dH, long s[6]) {   // planes, H, W, oH, oW, and N for a batch (else 0)
   if ((t->nDimension != 3 && t->nDimension != 4) || !banded(kW, kH, dW, dH) || !is_contiguous(t)) return false;
   const int o = t->nDimension - 3;
@@ -815,18 +823,16 @@ THC_API int THGPUNN_Threshold_SpatialMaxPooling_updateOutput(THGPUTensor *input,
                                                              double threshold, double val, int kW, int kH, int dW, int dH) {
   THC_BEGIN
   long s[6];
-  if (pooled_shape(input, kW, kH, dW, dH, s) && own_storage(thresholded, {input, output, indices}) && own_storage(output, {input, indices}) &&
-      own_storage(indices, {input})) {
+  if (thresholded != output && thresholded != indices && output != indices && pooled_shape(input, kW, kH, dW, dH, s) &&
+      apart({thresholded, output, indices}, {input})) {
     const long C = s[0] / (s[5] ? s[5] : 1), so[4] = {s[5], C, s[3], s[4]}, si[5] = {2, s[5], C, s[3], s[4]}, si3[4] = {2, C, s[3], s[4]};
     tensor_resize_as(thresholded, input);
     if (s[5]) { resize_nd(output, 4, so, nullptr); resize_nd(indices, 5, si, nullptr); }
     else { resize_nd(output, 3, so + 1, nullptr); resize_nd(indices, 4, si3, nullptr); }
-    const long n = nelem(input), m = nelem(output);
-    const float *x = data_ptr(input);
-    float *r = data_ptr(thresholded), *o = data_ptr(output), *ind = data_ptr(indices);
-    if (is_contiguous(thresholded) && is_contiguous(output) && is_contiguous(indices) && apart(x, n, r, n) && apart(x, n, o, m) && apart(x, n, ind, 2 * m) &&
-        apart(r, n, o, m) && apart(r, n, ind, 2 * m) && apart(o, m, ind, 2 * m)) {
-      forward_bands<true>(x, o, ind, ind + m, s[0], s[1], s[2], s[3], s[4], kH, ThresholdPass{nullptr, r, (float)threshold, (float)val});
+    if (is_contiguous(thresholded) && is_contiguous(output) && is_contiguous(indices)) {
+      float *ind = data_ptr(indices);
+      forward_bands<true>(data_ptr(input), data_ptr(output), ind, ind + nelem(output), s[0], s[1], s[2], s[3], s[4], kH,
+                          ThresholdPass{nullptr, data_ptr(thresholded), (float)threshold, (float)val});
       return 0;
     }
   }
@@ -843,18 +849,17 @@ THC_API int THGPUNN_Threshold_SpatialMaxPooling_updateGradInput(THGPUTensor *inp
   if (pooled_shape(input, kW, kH, dW, dH, s) && THGPUTensor_isSameSizeAs(input, thresholded) && gradOutput->nDimension == input->nDimension &&
       is_contiguous(gradOutput) && is_contiguous(indices)) {
     const int o = input->nDimension - 3;
-    const long n = nelem(input), m = s[0] * s[3] * s[4];
+    const long m = s[0] * s[3] * s[4];
     const bool sizes = (!o || gradOutput->size[0] == input->size[0]) && gradOutput->size[o] == input->size[o] && gradOutput->size[o + 1] == s[3] &&
                        gradOutput->size[o + 2] == s[4] && nelem(indices) == 2 * m;
-    if (sizes && own_storage(poolGradInput, {input, thresholded, gradOutput, indices, gradInput}) &&
-        own_storage(gradInput, {input, thresholded, gradOutput, indices})) {
+    if (sizes && poolGradInput != gradInput && apart({poolGradInput, gradInput}, {input, gradOutput, indices}) && poolGradInput != thresholded &&
+        gradInput != thresholded) {
       tensor_resize_as(poolGradInput, input);
       tensor_resize_as(gradInput, input);
-      const float *x = data_ptr(input), *g = data_ptr(gradOutput), *ind = data_ptr(indices);
-      float *gp = data_ptr(poolGradInput), *gi = data_ptr(gradInput);
-      if (is_contiguous(poolGradInput) && is_contiguous(gradInput) && apart(gp, n, gi, n) && apart(x, n, gp, n) && apart(x, n, gi, n) && apart(g, m, gp, n) &&
-          apart(g, m, gi, n) && apart(ind, 2 * m, gp, n) && apart(ind, 2 * m, gi, n) &&
-          backward_cells<true>(g, ind, ind + m, gp, s[0], s[1], s[2], s[3], s[4], kH, ThresholdPass{x, gi, (float)threshold, 0.f}))
+      const float *ind = data_ptr(indices);
+      if (is_contiguous(poolGradInput) && is_contiguous(gradInput) &&
+          backward_cells<true>(data_ptr(gradOutput), ind, ind + m, data_ptr(poolGradInput), s[0], s[1], s[2], s[3], s[4], kH,
+                               ThresholdPass{data_ptr(input), data_ptr(gradInput), (float)threshold, 0.f}))
         return 0;
     }
   }

@@ -130,3 +130,36 @@ def test_one_pass_only_for_what_it_knows():
     out = m.forward(gt.gpu(x))
     with pytest.raises(gt.THCError):
         m.backward(gt.gpu(x), gt.GPUTensor(*(v + 1 for v in out.size())))
+
+
+def test_sources_that_borrow_a_results_memory():
+    """A result outgrows memory that a source lies in: what the source holds is read before that memory goes back."""
+    import mcw_cppamp_torch_b200 as gt
+    L = gt.lib()
+
+    def borrow(t, *shape):
+        s = L.THGPUStorage_newWithData(t.data_ptr(), int(np.prod(shape)))
+        v = gt.GPUTensor(_ptr=L.THGPUTensor_newWithStorage1d(s, 0, int(np.prod(shape)), 1)).view(*shape)
+        L.THGPUStorage_free(s)
+        return v
+
+    g = np.random.default_rng(9)
+    shape, pooled = (2, 3, 12, 11), (2, 3, 6, 5)
+    n, x, go = int(np.prod(shape)), g.standard_normal(shape).astype(np.float32), g.standard_normal(pooled).astype(np.float32)
+    r, p = gt.nn.ReLU(), gt.nn.SpatialMaxPooling(2, 2, 2, 2)
+    want = p.forward(r.forward(gt.gpu(x))).float()
+    back = r.backward(gt.gpu(x), p.backward(r.output, gt.gpu(go))).float()
+    for field in ("output", "indices"):
+        m = gt.nn.Sequential().add(gt.nn.ReLU()).add(gt.nn.SpatialMaxPooling(2, 2, 2, 2))
+        held = gt.GPUTensor(n + 8)
+        held.narrow(1, 1, n).copy(x.reshape(-1))
+        setattr(m.modules[1], field, held.narrow(1, n + 1, 8))      # its storage has no room for the result behind it
+        xg = borrow(held, *shape)
+        del held
+        assert np.array_equal(m.forward(xg).float(), want)
+    m = gt.nn.Sequential().add(gt.nn.ReLU()).add(gt.nn.SpatialMaxPooling(2, 2, 2, 2))
+    xg = gt.gpu(x)
+    m.forward(xg)
+    m.modules[0].gradInput = gt.gpu(go)
+    gg = borrow(m.modules[0].gradInput, *pooled)
+    assert np.array_equal(m.backward(xg, gg).float(), back)
