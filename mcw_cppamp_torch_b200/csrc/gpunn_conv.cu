@@ -441,8 +441,11 @@ static void conv_grad_input_tc(const ConvGeom &g, const mm::ActPlanes &pgo, cons
   if (u.direct) { window_product(pgo.p, filter, nullptr, gin, rec); return; }
   float *gS = (float *)ws_alloc(sizeof(float) * g.N * u.Cr * (long)(u.Hs * u.Ws));
   window_product(pgo.p, filter, nullptr, gS, rec);
-  const long lines = g.N * g.C * g.H;
-  pdl_launch(mm::unfold_grad_input_kernel, (unsigned)std::min((lines + 7) / 8, ctx().sm_count * 16l), 256, 0, gS, gin, g.N, u, mm::FastDiv::make(u.dW));
+  const long planes = g.N * g.C, HW = g.H * g.W, group = std::max(1l, 1024 / HW);
+  const unsigned by = (unsigned)std::min((planes + group - 1) / group, ctx().sm_count * 32l);
+  const unsigned bx = (unsigned)std::min((group * HW + 1023) / 1024, std::max(1l, ctx().sm_count * 32l / by));
+  pdl_launch(mm::unfold_grad_input_kernel, dim3(bx, by), 256, 0, gS, gin, u,
+             mm::UnfoldGeom{planes, (int)group, mm::FastDiv::make(HW), mm::FastDiv::make(g.C), mm::FastDiv::make(g.W), mm::FastDiv::make(u.dH), mm::FastDiv::make(u.dW)});
   check_launch("unfold_grad_input");
 }
 

@@ -811,23 +811,38 @@ struct UnpackGradPass {
 
 // gin[n][c][h][w] = gS[n][ch][Y][X], the inverse of a fold along both axes (a bijection between the input pixels that any
 // window reaches and the cells' channels; the others get zero).  gS: [N][Cr][Hs][Ws].
-// A warp takes a line of the image: what belongs to the line is worked out once, and a column costs one division by multiplication (four in
-// hardware for every pixel: 14.7 us for 16 images of 3 x 224 x 224 from cold caches, 11.3 so).
-static __global__ void __launch_bounds__(256) unfold_grad_input_kernel(const float *__restrict__ gS, float *__restrict__ gin, long N,
-                                                                       const Cells u, const FastDiv ddW) {
+// Blocks take groups of G planes pixel by pixel, whatever the planes' shape, four loads of a thread on the way, divisions by multiplication.
+// From cold caches (us; pixel by pixel with divisions in hardware / a warp per line / so): 16 images of 3 x 224 x 224 14.4 / 11.7 / 11.8; 512 of 512 x
+// 7 x 7 233 / 376 / 49; 256 of 256 x 14 x 14 92 / 186 / 48; one of 3 x 2048 x 2048 164 / 46 / 43, of 4 x 262144 51 / 2666 / 6.6.
+struct UnfoldGeom {
+  long planes;
+  int G;
+  FastDiv HW, C, W, dH, dW;
+};
+static __global__ void __launch_bounds__(256) unfold_grad_input_kernel(const float *__restrict__ gS, float *__restrict__ gin, const Cells u,
+                                                                       const UnfoldGeom q) {
   pdl_begin();
-  const int lane = threadIdx.x & 31;
-  const long lines = N * u.C * u.H, step = (long)u.Hs * u.Ws;
-  for (long line = (long)blockIdx.x * 8 + (threadIdx.x >> 5); line < lines; line += (long)gridDim.x * 8) {
-    const long pl = line / u.H, n = pl / u.C;
-    const int c = (int)(pl - n * u.C), h = (int)(line - pl * u.H) + u.pad, Y = h / u.dH, dy = h - Y * u.dH;
-    const bool reached = Y < u.Hs && dy < u.eH;
-    const float *src = gS + (n * u.Cr + (long)dy * u.eW * u.Cq + c) * step + (long)Y * u.Ws;
-#pragma unroll 4
-    for (int x = lane; x < u.W; x += 32) {
-      unsigned X, dx;
-      ddW.divmod((unsigned)(x + u.pad), X, dx);
-      gin[line * u.W + x] = reached && (int)X < u.Ws && (int)dx < u.eW ? __ldg(src + (long)dx * u.Cq * step + X) : 0.f;
+  const unsigned HW = q.HW.d;
+  const long step = (long)u.Hs * u.Ws;
+  for (long p0 = (long)blockIdx.y * q.G; p0 < q.planes; p0 += (long)gridDim.y * q.G) {
+    const long n0 = p0 / u.C;
+    const unsigned c0 = (unsigned)(p0 - n0 * u.C), pixels = (unsigned)min((long)q.G, q.planes - p0) * HW;
+    for (unsigned t0 = blockIdx.x * 1024 + threadIdx.x; t0 < pixels; t0 += gridDim.x * 1024) {
+      float v[4];
+#pragma unroll
+      for (int k = 0; k < 4; k++) {
+        unsigned pl, r, n, c, y, x, Y, dy, X, dx;
+        q.HW.divmod(t0 + 256 * k, pl, r);
+        q.C.divmod(c0 + pl, n, c);
+        q.W.divmod(r, y, x);
+        q.dH.divmod(y + u.pad, Y, dy);
+        q.dW.divmod(x + u.pad, X, dx);
+        const bool reached = t0 + 256 * k < pixels && (int)Y < u.Hs && (int)X < u.Ws && (int)dy < u.eH && (int)dx < u.eW;
+        v[k] = reached ? __ldg(gS + ((n0 + n) * u.Cr + (long)(dy * u.eW + dx) * u.Cq + c) * step + (long)Y * u.Ws + X) : 0.f;
+      }
+#pragma unroll
+      for (int k = 0; k < 4; k++)
+        if (t0 + 256 * k < pixels) gin[p0 * HW + t0 + 256 * k] = v[k];
     }
   }
 }

@@ -30,6 +30,8 @@ CASES = [
     (3, 33, 31, 30, 1, 9, 9, 1, 1, 0),
     (2, 70, 28, 33, 9, 7, 7, 1, 1, 6),
     (1, 7, 135, 140, 34, 131, 133, 1, 1, 0),  # a window beyond what a window map takes: columns
+    (7, 5, 6, 5, 40, 3, 3, 2, 2, 1),          # gradInput from cells: groups of 34 planes, the last of one
+    (1, 2, 3, 5000, 33, 2, 4, 2, 4, 0),       # and a plane shared by several blocks
 ]
 
 
@@ -198,3 +200,26 @@ def test_bf16_gathered_windows(case):
         q = lambda t: f(t.bfloat16().double()).cuda()
         return torch.nn.functional.conv2d(q(x), q(w), f(b.double()).cuda(), (dH, dW), pad)
     assert torch.all((out - conv(lambda t: t)).abs() <= (C * kH * kW + 2) * 2.0 ** -23 * conv(torch.abs))
+
+
+def test_grad_input_from_cells_by_pixels():
+    """Four rows of 262144 pixels take what 1024 rows of 1024 do; a lane or a block per row leaves the device idle."""
+    import torch
+    import mcw_cppamp_torch_b200 as gt
+
+    def us(H, W):
+        m = gt.nn.SpatialConvolutionMM(1, 33, 4, 4, 4, 4)
+        m.gpu()
+        x, go = gt.GPUTensor(1, 1, H, W), gt.GPUTensor(1, 33, H // 4, W // 4).fill(0.5)
+        a, b = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+        times = []
+        for _ in range(8):
+            gt.synchronize()
+            a.record()
+            m.updateGradInput(x, go)
+            gt.synchronize()
+            b.record()
+            b.synchronize()
+            times.append(a.elapsed_time(b) * 1e3)
+        return sorted(times[2:])[2]
+    assert us(4, 262144) < 4 * us(1024, 1024)
