@@ -449,6 +449,23 @@ static void conv_grad_input_tc(const ConvGeom &g, const mm::ActPlanes &pgo, cons
   check_launch("unfold_grad_input");
 }
 
+// Weights beyond which a pass over them is worth a launch of its own: next to another pass an SM holds half its blocks, by the other's registers or tile.
+constexpr long kManyWeights = 3l << 20;
+// gw += scale * T, and the fold of gradBias.  (us, together / apart: 9.4 M weights 49 / 33 + 4 from FP16 pairs or BF16, 2.4 M 23 / 23 + 6.)
+template <bool PAIRS>
+static void unpack_grad_weight(const ConvGeom &g, const mm::Cells &u, const float *T, float *gw, const mm::WgradPlace &pl, float scale, const mm::WgradStrays &strays,
+                               const mm::ChanFinishPass &bias) {
+  using namespace mm;
+  const long blocks = std::min((g.K * g.R + 255) / 256, ctx().sm_count * 32l);
+  auto pass = [&](auto alone) { return UnpackGradPass<PAIRS, decltype(alone)::value>{(unsigned)blocks, T, gw, u, (int)g.K, WgradDivs::of(u), pl, scale, strays}; };
+  if (g.K * g.R <= kManyWeights) {
+    launch_passes(pass(std::false_type()), 0, "unpack_grad_weight", bias);
+  } else {
+    launch_passes(bias, 0, "conv_grad_bias_finish");
+    launch_passes(pass(std::true_type()), 0, "unpack_grad_weight");
+  }
+}
+
 // gradW[ko][(c,i,j)] += scale * sum over windows of gradOut[ko] * S[tap, ch]: the reduction runs over pixels, along which
 // neither tensor is contiguous in channels-last form, so both enter as MN-major operands.  Three ways round, by cost:
 //   0  rows = output planes, columns = (tap, ch)
@@ -490,8 +507,7 @@ static void conv_acc_grad_tc(const ConvGeom &g, const mm::Cells &u, const void *
       attach_raw_map<PREC>(q.b, act, Nf, pixels / f, Nf, bn2 / 2);
     });
     const WgradPlace pl{Nf, 1, 0, 0, 0, (int)f, Kp * Nf + Cs};
-    const long total = g.K * g.R;
-    launch_passes(UnpackGradPass<PREC == kPairs>{(unsigned)std::min<long>((total + 255) / 256, ctx().sm_count * 8l), T, gw, u, (int)g.K, pl, scale, strays}, 0, "unpack_grad_weight", bias);
+    unpack_grad_weight<PREC == kPairs>(g, u, T, gw, pl, scale, strays, bias);
     return;
   }
   const long cols = way == 2 ? N2 : way == 1 ? g.K : Rp, rows = way == 2 ? M2 : way == 1 ? Rp : g.K;
@@ -523,8 +539,7 @@ static void conv_acc_grad_tc(const ConvGeom &g, const mm::Cells &u, const void *
     launch_raw(p, [](auto &, int) {});
     pl = WgradPlace{1, N2, Cs * N2, -Kp, (u.kWs - 1) * Kp, 1, 0};
   }
-  const long total = g.K * g.R;
-  launch_passes(UnpackGradPass<PREC == kPairs>{(unsigned)std::min<long>((total + 255) / 256, ctx().sm_count * 8l), T, gw, u, (int)g.K, pl, scale, strays}, 0, "unpack_grad_weight", bias);
+  unpack_grad_weight<PREC == kPairs>(g, u, T, gw, pl, scale, strays, bias);
 }
 
 // ------------------------------------------------------------------------------------------------

@@ -756,15 +756,25 @@ __device__ __forceinline__ void find_strays(StrayPlaces &s, const Stray *list, i
     s.v[i] = list[i].v;
   }
 }
+struct WgradDivs {
+  FastDiv per, kHW, kW, stepH, stepW;
+  static WgradDivs of(const Cells &u) {
+    const long kHW = (long)u.kH * u.kW;
+    return WgradDivs{FastDiv::make(u.C * kHW), FastDiv::make(kHW), FastDiv::make(u.kW), FastDiv::make(u.stepH), FastDiv::make(u.stepW)};
+  }
+};
 // kPairs: with the strays of the input against all of gradOutput, and those of gradOutput against what the planes hold of the input.
-template <bool PAIRS>
+// ALONE: not next to the fold of gradBias.  Bound by its instructions and by how many blocks an SM holds: 9.4 M weights took 80 us with the
+// fold's 56 registers and five divisions in hardware a weight, 57 with these by multiplication, 33 with 32 registers as well.
+template <bool PAIRS, bool ALONE>
 struct UnpackGradPass {
-  static constexpr int kPerSM = 1;
+  static constexpr int kPerSM = ALONE ? 8 : 4;
   unsigned blocks = 0;
   const float *T;
   float *gw;
   Cells u;
   int K;
+  WgradDivs div;
   WgradPlace p;
   float scale;
   WgradStrays q;
@@ -780,13 +790,17 @@ struct UnpackGradPass {
       if (ng) { find_strays(sg, q.gout.list, ng, l.K, l.oH, l.oW, 0); unscale = pair_unscale(*q.act.rec); }
       __syncthreads();
     }
-    const unsigned kHW = (unsigned)(u.kH * u.kW), per = (unsigned)u.C * kHW, total = (unsigned)K * per;
+    const unsigned total = (unsigned)K * div.per.d;
     for (unsigned t = block * blockDim.x + threadIdx.x; t < total; t += blocks * blockDim.x) {
-      const unsigned ko = t / per, r = t - ko * per, c = r / kHW, tap = r - c * kHW, i = tap / (unsigned)u.kW, j = tap - i * u.kW;
-      const int bi = u.kHs > 1 ? (int)i / u.stepH : 0, bj = u.kWs > 1 ? (int)j / u.stepW : 0;
-      const int dy = (int)i - bi * u.stepH, dx = (int)j - bj * u.stepW;
-      const long ch = (dy * u.eW + dx) * u.Cq + (int)c;
-      const float *s = T + (p.first + ko * p.ko_stride + ch * p.ch_stride + bi * p.bi_stride + bj * p.bj_stride);
+      unsigned ko, r, c, tap, i, j, bi = 0, dy, bj = 0, dx;
+      div.per.divmod(t, ko, r);
+      div.kHW.divmod(r, c, tap);
+      div.kW.divmod(tap, i, j);
+      dy = i; dx = j;
+      if (u.kHs > 1) div.stepH.divmod(i, bi, dy);
+      if (u.kWs > 1) div.stepW.divmod(j, bj, dx);
+      const long ch = (int)(dy * u.eW + dx) * u.Cq + (int)c;
+      const float *s = T + (p.first + ko * p.ko_stride + ch * p.ch_stride + (int)bi * p.bi_stride + (int)bj * p.bj_stride);
       float sum = *s;
       for (int b = 1; b < p.copies; b++) sum += s[b * p.copy_stride];
       if constexpr (PAIRS) {
