@@ -220,13 +220,17 @@ static void add_strays(const ConvGeom &g, const float *src, const float *w, floa
   check_launch("window_strays");
 }
 
-// Repacked weights of a product of windows, rows r < rows: the buffer, and the pass that fills it (which shares a launch with the one that makes
-// the windows' planes).
+// Weights beyond which a pass over them is worth a launch of its own: next to another pass an SM holds half its blocks, by the other's registers or tile.
+constexpr long kManyWeights = 3l << 20;
+// Repacked weights of a product of windows, rows r < rows: the buffer, and the pass that fills it, which shares a launch with the one that makes
+// the windows' planes or has one of its own ahead of the product.  (us, together / apart, turned filters: 103 M weights in BF16 593 / 431 + 4, 9.4 M 50 / 45 + 4; 4.1 M of
+// 1 x 1 forward 65 / 62 with their product; 2.4 M 15 / 13 + 7.)
 template <int PREC, bool FLIP>
 struct FilterForm {
   mm::Windows full, v;   // the layer's windows, and those of the product (pixel pairs)
   bool pair = false;
   long rows = 0, wrows = 0, Kd = 0;
+  unsigned alone = 0;    // the pass's blocks where it has a launch of its own
   mm::RepackPass<PREC, FLIP> pass;
 };
 template <int PREC, bool FLIP>
@@ -240,14 +244,20 @@ static FilterForm<PREC, FLIP> filter_form(const mm::Windows &full, const float *
   void *wp = ws_alloc((size_t)f.wrows * f.Kd * (PREC == mm::kBf16 ? 2 : 4));
   const long blocks = std::min<long>((f.wrows * (f.Kd / 4) + 255) / 256, ctx().sm_count * 8l);
   f.pass = mm::RepackPass<PREC, FLIP>{(unsigned)blocks, w, u, (int)K, (int)rows, (int)f.v.C, f.pair ? full.dW : 0, wp, rec.joint(rec.weight)};
+  if (f.wrows * f.Kd > kManyWeights) std::swap(f.alone, f.pass.blocks);
   return f;
 }
 // out[n, r, y, x] = bias[r] + the product of the windows over `act` with the repacked weights
-template <int PREC, bool PAIR, class Filter>
-static void window_product_t(const void *act, const Filter &f, const float *bias, float *out, const Records &rec) {
+template <int PREC, bool PAIR, bool FLIP>
+static void window_product_t(const void *act, const FilterForm<PREC, FLIP> &f, const float *bias, float *out, const Records &rec) {
   using namespace mm;
   const Windows &full = f.full, &v = f.v;
   const long rows = f.rows;
+  if (f.alone) {
+    const auto &w = f.pass;
+    pdl_launch(repack_weight_kernel<PREC, FLIP>, f.alone, 256, 0, w.w, w.u, w.K, w.rows, w.chans, w.pair_shift, w.out, w.ranges);
+    check_launch("repack_weight");
+  }
   Problem<PlanesWindowOperand<PREC>, RawOperand<false, PREC>, PAIR, PREC> p;
   p.range_a = rec.act.rec; p.range_b = rec.weight.rec; p.ranges = rec.joint(rec.act);
   attach_window_map<PREC>(p.a, act, v);
@@ -449,8 +459,6 @@ static void conv_grad_input_tc(const ConvGeom &g, const mm::ActPlanes &pgo, cons
   check_launch("unfold_grad_input");
 }
 
-// Weights beyond which a pass over them is worth a launch of its own: next to another pass an SM holds half its blocks, by the other's registers or tile.
-constexpr long kManyWeights = 3l << 20;
 // gw += scale * T, and the fold of gradBias.  (us, together / apart: 9.4 M weights 49 / 33 + 4 from FP16 pairs or BF16, 2.4 M 23 / 23 + 6.)
 template <bool PAIRS>
 static void unpack_grad_weight(const ConvGeom &g, const mm::Cells &u, const float *T, float *gw, const mm::WgradPlace &pl, float scale, const mm::WgradStrays &strays,

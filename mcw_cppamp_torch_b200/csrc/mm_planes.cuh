@@ -702,7 +702,7 @@ struct RepackPass {
         int c, dy, dx;
         const bool real = u.channel(ch, c, dy, dx);
         const int i = dy + bi * u.stepH, j = dx + bj * u.stepW;
-        v[e] = real && ko < K && bj >= 0 && bj < u.kWs && i < u.kH && j < u.kW ? w[(((long)ko * u.C + c) * u.kH + i) * u.kW + j] : 0.f;
+        v[e] = real && ko < K && bj >= 0 && bj < u.kWs && i < u.kH && j < u.kW ? __ldg(w + ((((long)ko * u.C + c) * u.kH + i) * u.kW + j)) : 0.f;
       }
       if (PREC == kPairs && !wide) {
         __half2 hi[2], lo[2];
@@ -720,6 +720,13 @@ struct RepackPass {
     }
   }
 };
+
+template <int PREC, bool FLIP>
+static __global__ void __launch_bounds__(256) repack_weight_kernel(const float *__restrict__ w, const Cells u, int K, int rows, int chans, int pair_shift,
+                                                                   void *__restrict__ out, const Ranges ranges) {
+  pdl_begin();
+  RepackPass<PREC, FLIP>{gridDim.x, w, u, K, rows, chans, pair_shift, out, ranges}.run(blockIdx.x);
+}
 
 // gw[ko][(c, i, j)] += scale * T at the restated tap and channel of (c, i, j).  ko_stride, ch_stride, bi_stride, bj_stride: where T
 // keeps them (bj counted from the other end when bj_stride is negative: `first` is then the place of tap (0, 0)).
