@@ -280,7 +280,7 @@ static void window_product(const void *act, const FilterForm<PREC, FLIP> &f, con
 template <int PREC>
 static void restate_input(const ConvGeom &g, const mm::Cells &u, const float *in, void *dst, const mm::PairForm &form,
                           const mm::RepackPass<PREC, false> &repack) {
-  if (u.direct) { mm::make_act_planes<PREC, false>(in, g.N, g.C, g.H, g.W, dst, form, repack, mm::NoPass{}, 0); return; }
+  if (u.direct) { mm::make_act_planes<PREC, false>(in, g.N, g.C, g.H, g.W, dst, form, repack, mm::NoPass{}); return; }
   if constexpr (PREC == mm::kBf16) {
     const size_t smem = sizeof(uint4) * g.kH * (g.W + 2 * g.pad);
     if (u.Cq == 8 && u.kHs == 1 && u.kWs == 1 && g.C <= 8 && smem <= 200 * 1024) {
@@ -693,7 +693,7 @@ static bool restate_accurate(const ConvGeom &g, bool pairs, mm::Cells &u, int &p
   const bool ok = restate(g, mm::kTf32, u);
   mm::Cells up;
   if (!ok || !pairs || g.R > 1l << 28 || g.K * g.kH * g.kW > 1l << 28 ||   // (a row of weights and its second half: 31 bits)
-      windows_us(forward_windows(g, u), g.K, prec) < 30 || !restate(g, mm::kPairs, up) || up.Cs > 12288 ||   // (UnpairPass: 48 KB)
+      windows_us(forward_windows(g, u), g.K, prec) < 30 || !restate(g, mm::kPairs, up) || up.Cs > mm::UnpairPass<6>::kMost ||
       (up.kHs == 1 && up.kWs == 1 && !up.direct))
     return ok;
   // (filter_form counts the repacked weights in 31 bits; channels in spans of 64 may make more of them than spans of 32)
@@ -739,31 +739,21 @@ static void conv_forward(const ConvGeom &g, const float *in, const float *w, con
 // `act`: the input's planes, or null (n0: the image of their record that they start with); w_ok / in_ok: whether the weight gradient / gradInput runs over planes.
 template <int PREC>
 static void conv_backward_group(const ConvGeom &g, const mm::Cells &u, bool in_ok, bool w_ok, const float *in, const void *act, const float *gout,
-                                const float *w, float *gin, float *gw, float *gb, float scale, const Records &rec, long n0, mm::UnpairPass unpair) {
+                                const float *w, float *gin, float *gw, float *gb, float scale, const Records &rec, long n0, const mm::UnpairPass<3> &unpair) {
   WsScope ws_scope;
   mm::ActPlanes pgo;
   mm::PairForm form;
   form.ranges = rec.joint(rec.gout);
   FilterForm<PREC, true> filter;
   if (in_ok) filter = grad_input_filter<PREC>(g, w, rec);
-  auto make = [&](const auto &second, size_t more) {
+  auto make = [&](const auto &second) {
     // (the sums and the tile, 48 KB)
-    return gw && g.K <= 3968 ? mm::make_act_planes<PREC, true>(gout, g.N, g.K, g.oH, g.oW, nullptr, form, filter.pass, second, more)
-              : mm::make_act_planes<PREC, false>(gout, g.N, g.K, g.oH, g.oW, nullptr, form, filter.pass, second, more);
+    return gw && g.K <= 3968 ? mm::make_act_planes<PREC, true>(gout, g.N, g.K, g.oH, g.oW, nullptr, form, filter.pass, second)
+              : mm::make_act_planes<PREC, false>(gout, g.N, g.K, g.oH, g.oW, nullptr, form, filter.pass, second);
   };
-  if (PREC == mm::kPairs) {
-    // planes are brought back to FP32 pixel by pixel where that needs no more shared memory than the transposition leaves
-    const size_t more = unpair.blocks ? sizeof(float) * std::max(1024, unpair.Cp) : 0;
-    if (more > 14 * 1024) {
-      unpair.px = 1;
-      mm::launch_passes(unpair, sizeof(float) * unpair.Cp, "unpair");
-      unpair.blocks = 0;
-    } else if (unpair.blocks) {
-      unpair.px = (int)(more / sizeof(float)) / unpair.Cp;
-    }
-    if (in_ok || w_ok) pgo = make(unpair, unpair.blocks ? more : 0);
-  } else if (in_ok || w_ok) {
-    pgo = make(mm::NoPass{}, 0);
+  if (in_ok || w_ok) {
+    if constexpr (PREC == mm::kPairs) pgo = make(unpair);
+    else pgo = make(mm::NoPass{});
   }
   if (in_ok) {
     conv_grad_input_tc<PREC>(g, pgo, filter, gin, rec);
@@ -818,7 +808,7 @@ static bool conv_backward_tc(const ConvGeom &g, const mm::Cells &u, bool restate
     if (own || gw) {
       WsScope ws_scope;
       Records rec;
-      mm::UnpairPass unpair;
+      mm::UnpairPass<3> unpair;
       if constexpr (PREC == mm::kPairs) {   // (for each group: records last for some thousand words, see zeroed_words)
         rec.gout = mm::new_measured();
         if (own_ok) rec.weight = mm::new_measured();
@@ -827,8 +817,9 @@ static bool conv_backward_tc(const ConvGeom &g, const mm::Cells &u, bool restate
         if (act) {
           mm::KeptRange *kept = planes_record(act);
           rec.act = mm::Measured{&kept->rec, kept->strays, true};
-          const long pixels = g.N * u.Hs * u.Ws;
-          unpair = mm::UnpairPass{(unsigned)std::min(pixels, 4l * ctx().sm_count), (void *)act, pixels, u.Cs, 1, rec.joint(rec.act), &kept->rec};
+          const long pixels = g.N * u.Hs * u.Ws, most = 4l * ctx().sm_count;
+          if (u.Cs <= mm::UnpairPass<3>::kMost) unpair = mm::UnpairPass<3>::of((void *)act, pixels, u.Cs, rec.joint(rec.act), &kept->rec, most);
+          else mm::launch_passes(mm::UnpairPass<6>::of((void *)act, pixels, u.Cs, rec.joint(rec.act), &kept->rec, most), 0, "unpair");
         } else if (w_ok) {
           rec.act = mm::new_measured();
           mm::launch_ranges(mm::range_job_flat(x, s.N * image, rec.act), nullptr);

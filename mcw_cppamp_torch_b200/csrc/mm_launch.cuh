@@ -394,11 +394,9 @@ struct ActPlanes {
 };
 static long padded_channels(long C, int prec) { return prec != kTf32 ? (C + 63) / 64 * 64 : (C + 31) / 32 * 32; }
 static size_t planes_bytes(long N, long HW, long Cp, int prec) { return (size_t)N * HW * Cp * (prec == kBf16 ? 2 : 4); }
-// `dst`: room for planes_bytes(), or null for workspace.  `form`: kPairs.  `first`, `second` (with `more` bytes of shared memory): passes that
-// share the launch.
+// `dst`: room for planes_bytes(), or null for workspace.  `form`: kPairs.  `first`, `second`: passes that share the launch.
 template <int PREC, bool SUMS, class First, class Second>
-static ActPlanes make_act_planes(const float *src, long N, long C, long H, long W, void *dst, const PairForm &form, const First &first, const Second &second,
-                                 size_t more) {
+static ActPlanes make_act_planes(const float *src, long N, long C, long H, long W, void *dst, const PairForm &form, const First &first, const Second &second) {
   ActPlanes ap;
   const long HW = H * W;
   ap.N = N; ap.H = H; ap.W = W; ap.Cp = padded_channels(C, PREC);
@@ -407,16 +405,17 @@ static ActPlanes make_act_planes(const float *src, long N, long C, long H, long 
   const bool wide_tile = PREC == kTf32 || ((PREC == kPairs || !SUMS) && (HW + 127) / 128 * 128 * 10 <= (HW + 63) / 64 * 64 * 11);
   const long cap = ctx().sm_count * 16l, needed = N * ((HW + (wide_tile ? 127 : 63)) / (wide_tile ? 128 : 64)) * (ap.Cp / (PREC != kTf32 ? 64 : 32));
   long blocks = std::min(needed, cap);
+  size_t smem = 0;
   if (SUMS) {
     // every block leaves a row of per-channel sums to fold, which on a small tensor (a few tiles per block) costs as much as the
     // transposition: a quarter of the blocks keeps it short; a large one wants all its blocks (at 1024 images the same cut cost it 3 %)
     if (needed <= 4 * cap && blocks > cap / 4) blocks = cap / 4;
     ap.chan_blocks = (int)blocks;
     ap.chan_partial = (float *)ws_alloc(sizeof(float) * blocks * C);
-    more = std::max(more, sizeof(float) * C);
+    smem = sizeof(float) * C;
   }
   auto go = [&](auto pt) {
-    launch_passes(PlanesPass<PREC, decltype(pt)::value, SUMS>{(unsigned)blocks, src, N, (int)C, (int)HW, (int)ap.Cp, ap.p, ap.chan_partial, form}, more, "nchw_to_planes", first,
+    launch_passes(PlanesPass<PREC, decltype(pt)::value, SUMS>{(unsigned)blocks, src, N, (int)C, (int)HW, (int)ap.Cp, ap.p, ap.chan_partial, form}, smem, "nchw_to_planes", first,
                   second);
   };
   if constexpr (PREC == kTf32) go(std::integral_constant<int, 128>());

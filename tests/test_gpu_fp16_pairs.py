@@ -101,6 +101,8 @@ CONVS = [
     ((24, 128, 29, 29, 256, 3, 2, 1), [4, 0]),     # strided windows, folded gradInput
     ((96, 128, 29, 29, 256, 3, 2, 1), [0, 4]),
     ((4, 3, 500, 1000, 8, 11, 1, 5), [0, 4]),      # gradInput as a layer of its own
+    ((14, 3001, 28, 29, 1024, 1, 1, 0), [0, 4]),   # kept planes of two pixels a block, brought back next to the transposition of gradOutput
+    ((6, 7001, 28, 29, 1024, 1, 1, 0), [0, 4]),    # of more channels than that takes
 ]
 
 
