@@ -747,9 +747,8 @@ static void conv_backward_group(const ConvGeom &g, const mm::Cells &u, bool in_o
   FilterForm<PREC, true> filter;
   if (in_ok) filter = grad_input_filter<PREC>(g, w, rec);
   auto make = [&](const auto &second) {
-    // (the sums and the tile, 48 KB)
-    return gw && g.K <= 3968 ? mm::make_act_planes<PREC, true>(gout, g.N, g.K, g.oH, g.oW, nullptr, form, filter.pass, second)
-              : mm::make_act_planes<PREC, false>(gout, g.N, g.K, g.oH, g.oW, nullptr, form, filter.pass, second);
+    return gw && g.K <= mm::most_sums<PREC>(g.oH * g.oW) ? mm::make_act_planes<PREC, true>(gout, g.N, g.K, g.oH, g.oW, nullptr, form, filter.pass, second)
+                                                         : mm::make_act_planes<PREC, false>(gout, g.N, g.K, g.oH, g.oW, nullptr, form, filter.pass, second);
   };
   if (in_ok || w_ok) {
     if constexpr (PREC == mm::kPairs) pgo = make(unpair);

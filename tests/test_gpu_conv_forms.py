@@ -223,3 +223,29 @@ def test_grad_input_from_cells_by_pixels():
             times.append(a.elapsed_time(b) * 1e3)
         return sorted(times[2:])[2]
     assert us(4, 262144) < 4 * us(1024, 1024)
+
+
+@pytest.mark.parametrize("mode,shape", [("bf16", (4, 64, 20, 18)), ("fp32x3", (4, 64, 20, 18)), ("fp32x3", (64, 512, 13, 13))])
+def test_grad_bias_of_4096_planes(mode, shape):
+    """Their sums come along with gradOutput's planes, as those of fewer planes do: as many launches."""
+    import mcw_cppamp_torch_b200 as gt
+    N, C, H, W = shape
+    g = np.random.default_rng(7)
+    x = gt.gpu(g.standard_normal(shape, dtype=np.float32))
+    gt.set_math_mode(mode)
+    try:
+        counts = []
+        for K in (3968, 4096):
+            m = gt.nn.SpatialConvolutionMM(C, K, 1, 1).gpu()
+            go = g.standard_normal((N, K, H, W), dtype=np.float32)
+            gg = gt.gpu(go)
+            m.zeroGradParameters()
+            n = gt.lib().THGPUKernelLaunchCount()
+            m.accGradParameters(x, gg)
+            counts.append(gt.lib().THGPUKernelLaunchCount() - n)
+            go = go.astype(np.float64)
+            # (partial sums of at most 16 pixels a lane, then trees and rows of blocks: far fewer roundings in turn than values)
+            assert np.all(np.abs(m.gradBias.float() - go.sum((0, 2, 3))) <= N * H * W * 2.0 ** -24 * np.abs(go).sum((0, 2, 3)))
+        assert counts[0] == counts[1]
+    finally:
+        gt.set_math_mode("fp32x3")
