@@ -399,7 +399,7 @@ static __global__ void __launch_bounds__(256) maxpool2_backward_kernel(const flo
 // left L2, in DRAM.  Threshold and 3 x 3 pooling in one pass, by rows -> by planes (us; the bytes at the copy rate): 65536 planes of
 // 55 x 55 forward 462 -> 335 (330), backward 584 -> 476 (452); 196608 of 27 x 27 440 -> 235 (236), 600 -> 371 (324); 262144 of 13 x 13
 // 150 -> 74 (72), 194 -> 125 (99).  Forward, five blocks an SM with six pieces of a thread on the way each: four pieces 340, 239, 77; eight without
-// a bound on registers (119 of them, two blocks) 415, 296, 93.
+// a bound on registers (119 of them, two blocks) 415, 296, 93.  Without a threshold, where five blocks spill, four: 315, 227, 78 -> 279, 202, 68.
 struct PlaneGeom {
   long planes;
   int G, H, W, HW, oH, oW, P;
@@ -433,7 +433,7 @@ __device__ __forceinline__ void stretch_ends(long start, long end, One one) {
 }
 
 template <int K, bool TH>
-static __global__ void __launch_bounds__(256, 5) maxpool_forward_planes_kernel(const float *__restrict__ in, float *__restrict__ out,
+static __global__ void __launch_bounds__(256, TH ? 5 : 4) maxpool_forward_planes_kernel(const float *__restrict__ in, float *__restrict__ out,
                                                                             float *__restrict__ indy, float *__restrict__ indx, const PlaneGeom q,
                                                                             const ThresholdPass t) {
   pdl_begin();
@@ -561,7 +561,7 @@ static __global__ void __launch_bounds__(256) maxpool_backward_planes_kernel(con
     __syncthreads();
   }
 }
-// Planes per block, or G = 0 where the kernels by rows do better (us, by rows / by planes, threshold included).
+// Planes per block, or G = 0 where the kernels by rows do better (us, by rows / by planes, threshold included; without one see rows_alone).
 //   Few pixels: 174 planes of 43 x 35 (0.3 M) forward 4.7 / 6.3, backward 5.2 / 7.0; 400 of 31 x 100 (1.2 M) 6.5 / 5.5, 6.6 / 5.9; 8192 of 13 x 13 (1.4 M) 8.2 /
 //     6.4, 11.3 / 7.5; 1024 of 55 x 55 (3.1 M) 10.3 / 8.5, 11.0 / 10.0.
 //   Forward: 54 114 / 80, 56 116 / 99 (its columns meet in the same banks), 100 216 / 175; 2 x 2 54 94 / 81, 60 109 / 102, but 100 164 / 169.
@@ -582,6 +582,21 @@ static PlaneGeom plane_geom(long planes, long H, long W, long oH, long oW, int k
   smem = (size_t)(4 * ((q.G * q.HW + 7) / 4 * 4) + (backward ? 8l * q.G * ring : 0));
   return q;
 }
+// Pooling by itself moves a third to a half less, and rows do better wherever they keep their lanes busy.  `fill`: lanes and band rows with work, in percent.
+// us, by rows / by planes, 24 M pixels (6 times as many: the same within a tenth, unless noted).
+//   Forward, 3 x 3: 9 columns (fill 50) 49 / 41, 13 (56) 47 / 41, 16 (77) 37 / 45, 19 (42) 59 / 43, 23 (63) 45 / 45, 25 (75) 41 / 46, 31 (88) 39 / 44,
+//     33 (50) 55 / 45, 42 (62) 45 / 45, 46 (63) 45 / 47, 55 (81) 39 / 45, 64 (94) 35 / 47, 72 (53) 47 / 40, 97 (75) 41 / 47.
+//     2 x 2: 14 (77) 39 / 37, six times as many 204 / 155; 16 (100) 35 / 38, 22 (63) 37 / 37 and 210 / 178, 27 (66) 39 / 37, 28 (77) 37 / 39, 39 (56) 37 / 37, 56 (88) 35 / 45.
+//   Backward, 3 x 3: even widths, whose rows leave in whole pairs, 12 (56) 1 / 0.94, 14 (77) 1 / 1.14, 22 (63) 1 / 0.92, 24 (75) 1 / 1.0, 28 (77) 43 / 45, 32 (100) 37 / 45, 36 (51) 53 / 43,
+//     44 (63) 45 / 43; odd ones 13 (77) 61 / 49, 15 (100) 45 / 51, 23 (75) 61 / 49, 29 (88) 53 / 43, 31 (100) 45 / 47, 45 (69) 47 / 45.  One plane a group, 46 to 64: 43 / 53 to 35 / 42.
+//     2 x 2: groups that fill little of a block, 46 and 47, 143 M pixels: 221 / 246, 213 / 240; 50 and more 1 / 0.84 to 1.
+static bool rows_alone(const PlaneGeom &q, int k, bool backward) {
+  auto fill = [](long w, long lanes, long h) { return 100 * w * h / (lanes * ((h + kBand - 1) / kBand * kBand)); };
+  const long ch = (q.H + 1) / 2, LP = q.cw <= 8 ? 8 : q.cw <= 16 ? 16 : 32;
+  if (!backward) return fill(q.oW, (q.oW + LP - 1) / LP * LP, q.oH) >= (LP == 32 ? 63 : k == 2 && LP == 8 ? 80 : 70);
+  if (k == 2) return 10l * q.G * q.HW < 6l * 1024 * kPlanePieces;
+  return q.G == 1 || fill(q.cw, q.cw <= 32 ? LP : (q.cw + 30) / 31 * 32, ch) >= (q.W % 2 ? 90 : 70);
+}
 static unsigned plane_blocks(const PlaneGeom &q) { return (unsigned)std::min((q.planes + q.G - 1) / q.G, (long)ctx().sm_count * 64); }
 
 static unsigned band_blocks(const PoolGeom &p, int planes_per_warp) {
@@ -593,7 +608,7 @@ template <bool TH>
 static void forward_bands(const float *src, float *o, float *iy, float *ix, long planes, long H, long W, long oH, long oW, int k, const ThresholdPass &t) {
   size_t smem = 0;
   const PlaneGeom q = plane_geom(planes, H, W, oH, oW, k, false, smem);
-  if (q.G && (((uintptr_t)src | (uintptr_t)t.out) & 15) == 0) {
+  if (q.G && (TH || !rows_alone(q, k, false)) && (((uintptr_t)src | (uintptr_t)t.out) & 15) == 0) {
     auto go = [&](auto kernel) { pdl_launch(kernel, plane_blocks(q), 256, smem, src, o, iy, ix, q, t); };
     if (k == 3) go(maxpool_forward_planes_kernel<3, TH>); else go(maxpool_forward_planes_kernel<2, TH>);
     check_launch("maxpool_forward");
@@ -615,7 +630,7 @@ static bool backward_cells(const float *g, const float *iy, const float *ix, flo
                            const ThresholdPass &t) {
   size_t smem = 0;
   const PlaneGeom q = plane_geom(planes, H, W, oH, oW, k, true, smem);
-  if (q.G && (((uintptr_t)gi | (uintptr_t)t.in | (uintptr_t)t.out) & 15) == 0) {
+  if (q.G && (TH || !rows_alone(q, k, true)) && (((uintptr_t)gi | (uintptr_t)t.in | (uintptr_t)t.out) & 15) == 0) {
     auto go = [&](auto kernel) { pdl_launch(kernel, plane_blocks(q), 256, smem, g, iy, ix, gi, q, t); };
     if (k == 3) go(maxpool_backward_planes_kernel<3, TH>); else go(maxpool_backward_planes_kernel<2, TH>);
     check_launch("maxpool_backward");

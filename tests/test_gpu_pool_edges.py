@@ -163,3 +163,34 @@ def test_sources_that_borrow_a_results_memory():
     m.modules[0].gradInput = gt.gpu(go)
     gg = borrow(m.modules[0].gradInput, *pooled)
     assert np.array_equal(m.backward(xg, gg).float(), back)
+
+
+@pytest.mark.parametrize("k,shape", [(3, (256, 64, 64, 64)), (2, (64, 256, 56, 56))])
+def test_pooling_by_itself_goes_by_rows(k, shape):
+    """Without a threshold, planes of these widths took a quarter to two fifths longer through shared memory than by rows, which memory off
+    a 16-byte boundary is taken by."""
+    import torch
+    import mcw_cppamp_torch_b200 as gt
+    stream = torch.cuda.ExternalStream(gt.lib().THGPUGetStream())
+    n = int(np.prod(shape))
+    m, held, back = gt.nn.SpatialMaxPooling(k, k, 2, 2).gpu(), gt.GPUTensor(n + 4).fill(0.5), gt.GPUTensor(n + 4)
+    at = lambda t, first: t.narrow(1, first, n).view(*shape)
+    go = m.forward(at(held, 1)).clone()
+
+    def ms(f):
+        a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        a.record(stream)
+        f()
+        b.record(stream)
+        b.synchronize()
+        return a.elapsed_time(b)
+
+    times = {}
+    for _ in range(7):
+        for first in (1, 2):
+            x = at(held, first)
+            m.gradInput = at(back, first)
+            times.setdefault((first, "forward"), []).append(ms(lambda: m.updateOutput(x)))
+            times.setdefault((first, "back"), []).append(ms(lambda: m.updateGradInput(x, go)))
+    for way in ("forward", "back"):
+        assert sorted(times[1, way])[3] < 1.12 * sorted(times[2, way])[3], way
