@@ -249,3 +249,22 @@ def test_grad_bias_of_4096_planes(mode, shape):
         assert counts[0] == counts[1]
     finally:
         gt.set_math_mode("fp32x3")
+
+
+@pytest.mark.parametrize("case", [(300, 3, 64, 64, 64, 11, 11, 4, 4, 2), (40, 2, 33, 47, 48, 8, 8, 2, 3, 3), (9, 1, 40, 61, 64, 1, 1, 1, 1, 0), (5, 7, 64, 64, 64, 1, 17, 1, 1, 0)])
+def test_bf16_gathered_windows_and_columns_agree(case):
+    """The same bits as over the column matrix, which a layer of 128 planes takes: its first planes have this layer's filters."""
+    import mcw_cppamp_torch_b200 as gt
+    N, C, H, W, K, kH, kW, dH, dW, pad = case
+    g = np.random.default_rng(sum(case))
+    x, w, b = (g.standard_normal(s, dtype=np.float32) for s in ((N, C, H, W), (128, C * kH * kW), (128,)))
+    xg, out = gt.gpu(x), []
+    gt.set_math_mode("bf16")
+    try:
+        for planes in (K, 128):
+            m = gt.nn.SpatialConvolutionMM(C, planes, kW, kH, dW, dH, pad)
+            m.weight, m.bias = w[:planes].copy(), b[:planes].copy()
+            out.append(m.gpu().forward(xg).float()[:, :K])
+    finally:
+        gt.set_math_mode("fp32x3")
+    assert np.array_equal(out[0].view(np.uint32), out[1].view(np.uint32))

@@ -194,3 +194,55 @@ def test_pooling_by_itself_goes_by_rows(k, shape):
             times.setdefault((first, "back"), []).append(ms(lambda: m.updateGradInput(x, go)))
     for way in ("forward", "back"):
         assert sorted(times[1, way])[3] < 1.12 * sorted(times[2, way])[3], way
+
+
+# (2 x 2 windows go back by planes from 40 M pixels on)
+@pytest.mark.parametrize("k,shape", [(3, (67, 401, 13, 13)), (3, (23, 257, 27, 29)), (3, (9, 191, 55, 55)), (2, (331, 170, 29, 27)), (3, (20, 64, 35, 33)),
+                                     (3, (40, 100, 21, 19)), (2, (60, 64, 20, 38))])
+def test_whole_planes_of_special_values(k, shape):
+    """NaN, infinities, windows without a maximum, ties, zeros of both signs: the same bits as by rows, which batches of few pixels and memory off
+    16-byte boundaries are taken by."""
+    import mcw_cppamp_torch_b200 as gt
+    g = np.random.default_rng(sum(shape))
+    x = g.standard_normal(shape, dtype=np.float32)
+    flat = x.reshape(-1)
+    for step, v in ((7, 0.5), (11, -np.inf), (13, np.nan), (17, 0.25), (19, -0.0), (1009, np.inf)):
+        flat[::step] = v
+    x[1, :, :8, :8] = -np.inf
+    x[2, :, 3:9, 2:9] = np.nan
+    xg, per = gt.gpu(x), (1 << 20) // int(np.prod(shape[1:]))
+    bits = lambda t: t.float().view(np.uint32)
+
+    def off(t):
+        """the same values, 4 bytes off a 16-byte boundary"""
+        size, n = t.size(), int(np.prod(t.size()))
+        u = gt.GPUTensor(n + 1).narrow(1, 2, n).view(*size)
+        return u.copy(t)
+
+    def run(make, outs, xs, go, before=None):
+        m = make()
+        if before:
+            before(m)
+        m.forward(xs)
+        m.backward(xs, go)
+        return [bits(f(m)) for f in outs]
+
+    net = lambda: gt.nn.Sequential().add(gt.nn.Threshold(0.25, -1.5)).add(gt.nn.SpatialMaxPooling(k, k, 2, 2))
+    fields = [lambda m: m.output, lambda m: m.modules[0].output, lambda m: m.modules[1].gradInput, lambda m: m.gradInput]
+    pool, one = lambda: gt.nn.SpatialMaxPooling(k, k, 2, 2), [lambda m: m.output, lambda m: m.gradInput]
+    go = g.standard_normal((*shape[:2], (shape[2] - k) // 2 + 1, (shape[3] - k) // 2 + 1), dtype=np.float32)
+    go.reshape(-1)[::5] = -0.0
+    gg = gt.gpu(go)
+    for make, outs in ((net, fields), (pool, one)):
+        whole = run(make, outs, xg, gg)
+        for n in range(0, shape[0], per):
+            c = min(per, shape[0] - n)
+            for a, b in zip(whole, run(make, outs, xg.narrow(1, n + 1, c), gg.narrow(1, n + 1, c))):
+                assert np.array_equal(a[n:n + c], b)
+    whole = run(net, fields, xg, gg)
+    for before in (lambda m: setattr(m.modules[1], "gradInput", off(xg)), lambda m: setattr(m.modules[0], "gradInput", off(xg)),
+                   lambda m: setattr(m.modules[0], "output", off(xg))):
+        for a, b in zip(whole, run(net, fields, xg, gg, before)):
+            assert np.array_equal(a, b)
+    for a, b in zip(whole, run(net, fields, off(xg), gg)):
+        assert np.array_equal(a, b)
