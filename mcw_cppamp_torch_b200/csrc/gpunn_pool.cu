@@ -399,7 +399,7 @@ static __global__ void __launch_bounds__(256) maxpool2_backward_kernel(const flo
 // left L2, in DRAM.  Threshold and 3 x 3 pooling in one pass, by rows -> by planes (us; the bytes at the copy rate): 65536 planes of
 // 55 x 55 forward 462 -> 335 (330), backward 584 -> 476 (452); 196608 of 27 x 27 440 -> 235 (236), 600 -> 371 (324); 262144 of 13 x 13
 // 150 -> 74 (72), 194 -> 125 (99).  Forward, five blocks an SM with six pieces of a thread on the way each: four pieces 340, 239, 77; eight without
-// a bound on registers (119 of them, two blocks) 415, 296, 93.  Without a threshold, where five blocks spill, four: 315, 227, 78 -> 279, 202, 68.
+// a bound on registers (119 of them, two blocks) 415, 296, 93.  Without a threshold, where five blocks spill 48 bytes a thread, four (8 bytes): 315, 227, 78 -> 279, 202, 68.
 struct PlaneGeom {
   long planes;
   int G, H, W, HW, oH, oW, P;
@@ -561,6 +561,9 @@ static __global__ void __launch_bounds__(256) maxpool_backward_planes_kernel(con
     __syncthreads();
   }
 }
+// By rows: lanes of a plane, and the share of lanes and band rows with work, in percent.
+static long rows_lanes(long cw) { return cw <= 8 ? 8 : cw <= 16 ? 16 : 32; }
+static long rows_fill(long w, long lanes, long h) { return 100 * w * h / (lanes * ((h + kBand - 1) / kBand * kBand)); }
 // Planes per block, or G = 0 where the kernels by rows do better (us, by rows / by planes, threshold included; without one see rows_alone).
 //   Few pixels: 174 planes of 43 x 35 (0.3 M) forward 4.7 / 6.3, backward 5.2 / 7.0; 400 of 31 x 100 (1.2 M) 6.5 / 5.5, 6.6 / 5.9; 8192 of 13 x 13 (1.4 M) 8.2 /
 //     6.4, 11.3 / 7.5; 1024 of 55 x 55 (3.1 M) 10.3 / 8.5, 11.0 / 10.0.
@@ -568,11 +571,14 @@ static __global__ void __launch_bounds__(256) maxpool_backward_planes_kernel(con
 //   Backward: 3 x 3 by planes wherever a group fits; 28 82 / 71, 56 144 / 120.  2 x 2 by rows, which leave in whole sectors for
 //     widths of whole 16-byte pieces and meet in L2 otherwise, as long as the tensors stay there: 28 63 / 78, 14 17.7 / 22, 24576 of 27 x 27 (18 M pixels)
 //     48 / 53, 196608 (143 M) 418 / 354, 65536 of 55 x 55 570 / 468, 262144 of 13 x 13 122 / 129, 16384 of 54 x 54 (48 M) 130 / 119.
-static PlaneGeom plane_geom(long planes, long H, long W, long oH, long oW, int k, bool backward, size_t &smem) {
+//   Below 2^20 pixels, behind a threshold, where rows leave half their lanes idle (from 2^18 on three fifths; the two modules by themselves / rows / planes): 0.6 M of
+//     11 x 5, 3 x 3 forward 6.9 / 8.5 / 4.4, backward 8.0 / 10.3 / 5.8, 2 x 2 forward 6.4 / 7.7 / 4.2; 0.3 M of 9 x 9 4.3 / 5.4 / 3.8, 5.9 / 6.2 / 5.0; 0.9 M of 17 x 17 6.6 / 8.3 / 5.0, 8.7 / 10.6 / 6.2.
+static PlaneGeom plane_geom(long planes, long H, long W, long oH, long oW, int k, bool backward, bool threshold, size_t &smem) {
   PlaneGeom q = {};
   q.planes = planes; q.H = (int)H; q.W = (int)W; q.HW = (int)std::min(H * W, 1l << 30); q.oH = (int)oH; q.oW = (int)oW; q.P = (int)(oH * oW);
   const long ch = (H + 1) / 2, cw = (W + 1) / 2, ring = (oH + 2) * (oW + 2), bytes = 4 * H * W + (backward ? 8 * ring : 0), pixels = planes * H * W;
-  if (bytes > 47 * 1024 || pixels < 1l << 20) return q;
+  if (bytes > 47 * 1024 || pixels < 1l << 18) return q;
+  if (pixels < 1l << 20 && (!threshold || rows_fill(cw, (cw + rows_lanes(cw) - 1) / rows_lanes(cw) * rows_lanes(cw), ch) >= (pixels < 1l << 19 ? 40 : 50))) return q;
   if (!backward && k == 2 && W > 64 && W % 2 == 0) return q;
   if (backward && H * W > 1024 * kPlanePieces) return q;
   if (backward && k == 2 && (W % 4 == 0 || W <= 16 || pixels < 40l << 20)) return q;
@@ -582,7 +588,7 @@ static PlaneGeom plane_geom(long planes, long H, long W, long oH, long oW, int k
   smem = (size_t)(4 * ((q.G * q.HW + 7) / 4 * 4) + (backward ? 8l * q.G * ring : 0));
   return q;
 }
-// Pooling by itself moves a third to a half less, and rows do better wherever they keep their lanes busy.  `fill`: lanes and band rows with work, in percent.
+// Pooling by itself moves a third to a half less, and rows do better wherever they keep their lanes busy (fill: rows_fill).
 // us, by rows / by planes, 24 M pixels (6 times as many: the same within a tenth, unless noted).
 //   Forward, 3 x 3: 9 columns (fill 50) 49 / 41, 13 (56) 47 / 41, 16 (77) 37 / 45, 19 (42) 59 / 43, 23 (63) 45 / 45, 25 (75) 41 / 46, 31 (88) 39 / 44,
 //     33 (50) 55 / 45, 42 (62) 45 / 45, 46 (63) 45 / 47, 55 (81) 39 / 45, 64 (94) 35 / 47, 72 (53) 47 / 40, 97 (75) 41 / 47.
@@ -591,11 +597,10 @@ static PlaneGeom plane_geom(long planes, long H, long W, long oH, long oW, int k
 //     44 (63) 45 / 43; odd ones 13 (77) 61 / 49, 15 (100) 45 / 51, 23 (75) 61 / 49, 29 (88) 53 / 43, 31 (100) 45 / 47, 45 (69) 47 / 45.  One plane a group, 46 to 64: 43 / 53 to 35 / 42.
 //     2 x 2: groups that fill little of a block, 46 and 47, 143 M pixels: 221 / 246, 213 / 240; 50 and more 1 / 0.84 to 1.
 static bool rows_alone(const PlaneGeom &q, int k, bool backward) {
-  auto fill = [](long w, long lanes, long h) { return 100 * w * h / (lanes * ((h + kBand - 1) / kBand * kBand)); };
-  const long ch = (q.H + 1) / 2, LP = q.cw <= 8 ? 8 : q.cw <= 16 ? 16 : 32;
-  if (!backward) return fill(q.oW, (q.oW + LP - 1) / LP * LP, q.oH) >= (LP == 32 ? 63 : k == 2 && LP == 8 ? 80 : 70);
+  const long ch = (q.H + 1) / 2, LP = rows_lanes(q.cw);
+  if (!backward) return rows_fill(q.oW, (q.oW + LP - 1) / LP * LP, q.oH) >= (LP == 32 ? 63 : k == 2 && LP == 8 ? 80 : 70);
   if (k == 2) return 10l * q.G * q.HW < 6l * 1024 * kPlanePieces;
-  return q.G == 1 || fill(q.cw, q.cw <= 32 ? LP : (q.cw + 30) / 31 * 32, ch) >= (q.W % 2 ? 90 : 70);
+  return q.G == 1 || rows_fill(q.cw, q.cw <= 32 ? LP : (q.cw + 30) / 31 * 32, ch) >= (q.W % 2 ? 90 : 70);
 }
 static unsigned plane_blocks(const PlaneGeom &q) { return (unsigned)std::min((q.planes + q.G - 1) / q.G, (long)ctx().sm_count * 64); }
 
@@ -607,7 +612,7 @@ static unsigned band_blocks(const PoolGeom &p, int planes_per_warp) {
 template <bool TH>
 static void forward_bands(const float *src, float *o, float *iy, float *ix, long planes, long H, long W, long oH, long oW, int k, const ThresholdPass &t) {
   size_t smem = 0;
-  const PlaneGeom q = plane_geom(planes, H, W, oH, oW, k, false, smem);
+  const PlaneGeom q = plane_geom(planes, H, W, oH, oW, k, false, TH, smem);
   if (q.G && (TH || !rows_alone(q, k, false)) && (((uintptr_t)src | (uintptr_t)t.out) & 15) == 0) {
     auto go = [&](auto kernel) { pdl_launch(kernel, plane_blocks(q), 256, smem, src, o, iy, ix, q, t); };
     if (k == 3) go(maxpool_forward_planes_kernel<3, TH>); else go(maxpool_forward_planes_kernel<2, TH>);
@@ -629,7 +634,7 @@ template <bool TH>
 static bool backward_cells(const float *g, const float *iy, const float *ix, float *gi, long planes, long H, long W, long oH, long oW, int k,
                            const ThresholdPass &t) {
   size_t smem = 0;
-  const PlaneGeom q = plane_geom(planes, H, W, oH, oW, k, true, smem);
+  const PlaneGeom q = plane_geom(planes, H, W, oH, oW, k, true, TH, smem);
   if (q.G && (TH || !rows_alone(q, k, true)) && (((uintptr_t)gi | (uintptr_t)t.in | (uintptr_t)t.out) & 15) == 0) {
     auto go = [&](auto kernel) { pdl_launch(kernel, plane_blocks(q), 256, smem, g, iy, ix, gi, q, t); };
     if (k == 3) go(maxpool_backward_planes_kernel<3, TH>); else go(maxpool_backward_planes_kernel<2, TH>);

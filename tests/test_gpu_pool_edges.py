@@ -198,7 +198,8 @@ def test_pooling_by_itself_goes_by_rows(k, shape):
 
 # (2 x 2 windows go back by planes from 40 M pixels on)
 @pytest.mark.parametrize("k,shape", [(3, (67, 401, 13, 13)), (3, (23, 257, 27, 29)), (3, (9, 191, 55, 55)), (2, (331, 170, 29, 27)), (3, (20, 64, 35, 33)),
-                                     (3, (40, 100, 21, 19)), (2, (60, 64, 20, 38))])
+                                     (3, (40, 100, 21, 19)), (2, (60, 64, 20, 38)), (3, (26, 420, 11, 5)),
+                                     (2, (90, 45, 9, 9))])
 def test_whole_planes_of_special_values(k, shape):
     """NaN, infinities, windows without a maximum, ties, zeros of both signs: the same bits as by rows, which batches of few pixels and memory off
     16-byte boundaries are taken by."""
@@ -210,7 +211,7 @@ def test_whole_planes_of_special_values(k, shape):
         flat[::step] = v
     x[1, :, :8, :8] = -np.inf
     x[2, :, 3:9, 2:9] = np.nan
-    xg, per = gt.gpu(x), (1 << 20) // int(np.prod(shape[1:]))
+    xg, per = gt.gpu(x), (1 << 20 if shape[3] > 9 else 1 << 18) // int(np.prod(shape[1:]))   # (narrow planes: from 2^18 pixels on)
     bits = lambda t: t.float().view(np.uint32)
 
     def off(t):
@@ -246,3 +247,25 @@ def test_whole_planes_of_special_values(k, shape):
             assert np.array_equal(a, b)
     for a, b in zip(whole, run(net, fields, off(xg), gg)):
         assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("k,shape", [(3, (1, 10909, 11, 5)), (2, (1, 16363, 11, 5)), (3, (1, 11111, 9, 9))])
+def test_one_pass_over_narrow_planes(k, shape):
+    """Threshold and pooling in one pass take no longer than one after the other; by rows, which planes of so few columns leave idle, they did."""
+    import torch
+    import mcw_cppamp_torch_b200 as gt
+    stream = torch.cuda.ExternalStream(gt.lib().THGPUGetStream())
+    x, net = gt.GPUTensor(*shape).fill(0.5), gt.nn.Sequential().add(gt.nn.ReLU()).add(gt.nn.SpatialMaxPooling(k, k, 2, 2)).gpu()
+    relu, pool = gt.nn.ReLU().gpu(), gt.nn.SpatialMaxPooling(k, k, 2, 2).gpu()
+
+    def ms(f):
+        a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        a.record(stream)
+        for _ in range(50):
+            f()
+        b.record(stream)
+        b.synchronize()
+        return a.elapsed_time(b)
+
+    one, two = (sorted(ms(f) for _ in range(9))[4] for f in (lambda: net.updateOutput(x), lambda: pool.updateOutput(relu.updateOutput(x))))
+    assert one < two
