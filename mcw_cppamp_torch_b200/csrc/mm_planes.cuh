@@ -271,7 +271,9 @@ struct UnpairPass {
 // sums is another training run: of small batches, one that ends in NaN where this one does not, or the other way round.
 template <int PREC, int PT, bool SUMS>
 struct PlanesPass {
-  static constexpr int CT = PREC == kTf32 ? 32 : 64, kPerSM = PT == 128 ? 4 : 5;   // (left alone, 128 registers with sums)
+  // (left alone, 128 registers with sums.  TF32 has half a tile and had 64 registers with four blocks, BF16 48 with five: 64 planes of 224 x 224, 16 images 69 -> 66 us, 512 planes of 62 x 62,
+  // 30 images, BF16 95 -> 85.  128 pixels: pairs 34 us with four blocks, 41 with five; BF16 34 with four or five, 42 with six, which spill.)
+  static constexpr int CT = PREC == kTf32 ? 32 : 64, kPerSM = PREC == kTf32 || (PREC == kBf16 && PT == 64) ? 6 : PT == 128 ? 4 : 5;
   unsigned blocks = 0;
   const float *src;
   long N;
@@ -493,7 +495,8 @@ __device__ __forceinline__ void cells_row(const float *__restrict__ in, void *__
 }
 template <int PREC, bool TABLE>
 struct CellsPass {
-  static constexpr int kPerSM = 1;
+  // as many as the pass has by itself: with the registers of the weights' repacking an SM held five (16 images of 3 x 224 x 224 as 4 x 4 cells 11.3 -> 9.6 us)
+  static constexpr int kPerSM = PREC == kTf32 ? 8 : PREC == kBf16 ? (TABLE ? 7 : 6) : TABLE ? 4 : 6;
   unsigned blocks = 0, rows;   // a row of cells is shared by blocks / rows blocks
   const float *in;
   void *S;
