@@ -271,9 +271,9 @@ struct UnpairPass {
 // sums is another training run: of small batches, one that ends in NaN where this one does not, or the other way round.
 template <int PREC, int PT, bool SUMS>
 struct PlanesPass {
-  // (left alone, 128 registers with sums.  TF32 has half a tile and had 64 registers with four blocks, BF16 48 with five: 64 planes of 224 x 224, 16 images 69 -> 66 us, 512 planes of 62 x 62,
-  // 30 images, BF16 95 -> 85.  128 pixels: pairs 34 us with four blocks, 41 with five; BF16 34 with four or five, 42 with six, which spill.)
-  static constexpr int CT = PREC == kTf32 ? 32 : 64, kPerSM = PREC == kTf32 || (PREC == kBf16 && PT == 64) ? 6 : PT == 128 ? 4 : 5;
+  // (left alone, 128 registers with sums.  Six blocks for TF32 and for BF16's 64 pixels are faster from cold caches, 512 planes of 62 x 62, 30 images 95 -> 85 us in BF16, but not
+  // behind the kernel that left the tensor in L2: a small TF32 block 68.6 -> 69.6, AlexNet's BF16 step 3350 -> 3366.)
+  static constexpr int CT = PREC == kTf32 ? 32 : 64, kPerSM = PT == 128 ? 4 : 5;
   unsigned blocks = 0;
   const float *src;
   long N;
