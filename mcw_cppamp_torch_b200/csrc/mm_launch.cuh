@@ -218,7 +218,9 @@ static int tc2_tile_width(long N, bool half_mn = false) {
   }
   return best;
 }
-// Microseconds a cluster takes for one k tile of a tile of this width, as the convolution and addmm launches at full size show it.
+// Microseconds a cluster takes for one k tile of a tile of this width, as the convolution and addmm launches at full size showed it when one
+// thread issued the MMAs.  Narrow tiles are faster since (pairs at 128 columns 0.6, see elect_one); the choices made by these values were within 2 % of the
+// better form when forms were forced, and other values move the bounds of k slices and with them the last bits of results.
 static double tc2_tile_us(int bn2, int prec) {
   if (prec == kBf16) return bn2 == 256 ? 0.55 : bn2 == 192 ? 0.47 : 0.4;
   if (prec == kPairs) return bn2 == 256 ? 1.3 : bn2 == 192 ? 1.1 : bn2 == 128 ? 0.9 : 0.8;

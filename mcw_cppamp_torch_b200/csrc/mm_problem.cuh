@@ -186,7 +186,7 @@ struct Operand {
 };
 
 // ---------------------------------------------------------------------------------------------
-// Operands of the two-SM engine, all fetched by TMA.  A tile row holds one swizzle span of 128 bytes: KV = 32 FP32 values
+// Operands of the two-SM engine, fetched by TMA (gathered windows: GatheredWindowOperand).  A tile row holds one swizzle span of 128 bytes: KV = 32 FP32 values
 // (3xTF32 products) or 64 BF16 values.
 //
 // A plain matrix: K-major (memory runs along k) or MN-major (memory runs along the rows).  tmap: K-major {K, rows} with

@@ -154,15 +154,15 @@ __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
 // One thread of a converged warp.  The tensor-core and TMA instructions take their descriptors, coordinates and barriers from registers
 // that a warp has once.  A warp that runs its loop with all lanes on values that all of them share, and issues under this predicate, has
 // them there; one thread alone (`lane == 0` around the loop, an election around the loop as well) pays for bringing them there
-// with every instruction.  tcgen05.mma of a CTA pair back to back: 107 cycles each at any width then, and 46, 68, 100 and 132 so, at
-// 64, 128, 192 and 256 columns.
+// with every instruction.  tcgen05.mma of a CTA pair back to back at 64, 128 and 192 columns: one every 107 cycles then, the cost of its issue, and
+// every 46, 68 and 100 so; 256 columns, which the pipe itself bounds, take some 130 either way.
 __device__ __forceinline__ bool elect_one() {
   uint32_t p;
   asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
   return p != 0;
 }
-// Bounded busy wait for the single MMA-issuing thread: polling without suspension answers within a few
-// cycles of the arrival, which is what keeps the tensor pipe fed; one spinning thread costs nothing.
+// Bounded busy wait for the warps that issue MMAs, all lanes of which poll: polling without suspension answers within a few
+// cycles of the arrival, which is what keeps the tensor pipe fed.  A poll is one instruction of the warp, as it was of a lone thread.
 __device__ __forceinline__ bool mbar_wait_spin(uint32_t bar, uint32_t parity, volatile WaitCtl *w, int code = kWaitOther) {
   long long t0 = 0;
   for (int polls = 0;; polls++) {

@@ -39,7 +39,8 @@
 // Roles (512 threads per CTA):
 //   warps 0-3   splitters, two groups of two warps taking alternate k tiles: wait for the tile's TMA bytes
 //               (`raw_full`, CTA-local) and for its lo slot to be free, split, publish to the async proxy,
-//               arrive on CTA 0's `full`.
+//               arrive on CTA 0's `full`.  16-bit operands have nothing to split: there these warps are idle, or (GatheredWindowOperand) copy
+//               the A rows of their CTA by cp.async, each a quarter of every tile, and arrive on CTA 0's `full` as the copies land.
 //   warps 4, 6  (CTA 0) issue the MMAs of the even and the odd k tiles (16-bit operands: warp 4 all).
 //   warp 5      issues the TMA loads of this CTA's A rows and B rows, R - 1 tiles ahead,
 //               as soon as the MMAs that read a slot have completed (`empty`).
@@ -83,7 +84,7 @@ template <int BN2, int PREC> struct Tc2rCfg {
   static constexpr int TMEM_COLS = ACCS * BN2 > 256 ? 512 : 256;
   static constexpr int SMEM_BYTES = (HI_SLOTS + LO_SLOTS) * SLOT_BYTES + 512 + 1024;
   static_assert(HI_SLOTS >= LO_SLOTS, "ring sizes");
-  static_assert(HALF || HI_SLOTS % 2 == 0 || HI_SLOTS <= LO_SLOTS + 2, "an odd hi ring must not be longer than the lo ring + 2 (parity waits of the two MMA threads)");
+  static_assert(HALF || HI_SLOTS % 2 == 0 || HI_SLOTS <= LO_SLOTS + 2, "an odd hi ring must not be longer than the lo ring + 2 (parity waits of the two MMA warps)");
 };
 
 // What a launch asks for: one over pairs may have to run as kTf32.
@@ -205,7 +206,7 @@ struct TileLoader<ROWS, PREC, WIDE, GatheredWindowOperand> {
 // The clusters of a launch take their work items from a counter in device memory, first come first served, so a
 // cluster that starts late (its SMs were still busy with another stream's kernel: a collective, a parameter
 // update) simply takes fewer items instead of leaving its fixed share to run alone at the end.  One thread of the
-// leader CTA fetches the next item number when the leader's TMA thread, the role that runs furthest ahead, starts on
+// leader CTA fetches the next item number when the leader's TMA warp, the role that runs furthest ahead, starts on
 // the current one (`go` barrier): one item of look-ahead hides the counter's round trip, and a cluster never holds
 // claims on work it is not about to do.  The numbers go into a ring of T2R_SCHED slots that exists in both CTAs;
 // every role of both CTAs reads the ring in the same order.  Slot protocol: `full` (one per CTA, count 1) completes
@@ -216,7 +217,7 @@ constexpr int T2R_SCHED = 8;
 constexpr int T2R_SCHED_WARP = 7;
 constexpr uint32_t T2R_NO_ITEM = 0xffffffffu;
 constexpr int T2R_ITEM_WAIT_SHIFT = 6;   // item-level waits may take 64 k-tile limits (see mbar_wait)
-// readers per slot: TMA thread, 4 splitter warps (16-bit operands: none, or the 4 that gather A), 8 drain warps in each CTA, the MMA threads in the leader
+// readers per slot: TMA warp, 4 splitter warps (16-bit operands: none, or the 4 that gather A), 8 drain warps in each CTA, the MMA warps in the leader
 template <bool HALF, bool GATHERED> struct Tc2rReaders { static constexpr uint32_t count = 2 * (1 + (HALF && !GATHERED ? 0 : 4) + T2_DRAIN_WARPS) + (HALF ? 1 : 2); };
 
 __device__ __forceinline__ void mbar_arrive_local(uint32_t bar) {
@@ -317,9 +318,9 @@ __device__ __forceinline__ void tc2r_run(const P &p, const StallCtl &ctl, unsign
   sched.ring = smem_u32(sched_ring);
   if (tid == 0) {
     for (int s = 0; s < R; s++) {
-      mbar_init(bar_full + 8 * s, GATHERED ? 1 + 2 * T2_PRODUCERS / 32 : HALF ? 1 : 2 * T2_PRODUCERS / 64);   // used in CTA 0: its TMA thread and both CTAs' bytes (and the warps that gather) / a group of two splitter warps in each CTA
+      mbar_init(bar_full + 8 * s, GATHERED ? 1 + 2 * T2_PRODUCERS / 32 : HALF ? 1 : 2 * T2_PRODUCERS / 64);   // used in CTA 0: its TMA warp and both CTAs' bytes (and the four warps of each CTA that gather) / a group of two splitter warps in each CTA
       mbar_init(bar_empty + 8 * s, 1);
-      mbar_init(bar_raw + 8 * s, 1);                        // this CTA's TMA thread + the bytes it announces
+      mbar_init(bar_raw + 8 * s, 1);                        // this CTA's TMA warp + the bytes it announces
     }
     for (int l = 0; l < L; l++) mbar_init(bar_lo_empty + 8 * l, 1);
     for (int k = 0; k < T2R_SCHED; k++) {
@@ -421,7 +422,7 @@ __device__ __forceinline__ void tc2r_run(const P &p, const StallCtl &ctl, unsign
         const uint32_t raw_bar = bar_raw + 8 * s, raw_par = (uint32_t)(g / R) & 1u;
         // The lo slot is free once the MMAs of tile g - L have read it.  It has a barrier of its own: the hi slots'
         // `empty` barriers can run two phases ahead of a splitter group that was slow to wake up (the other group and
-        // the other MMA thread do not wait for it), and a parity wait cannot tell two completed phases from none.
+        // the other MMA warp do not wait for it), and a parity wait cannot tell two completed phases from none.
         const uint32_t lo_bar = bar_lo_empty + 8 * ls, lo_par = (uint32_t)(g / LM + 1) & 1u;
         const bool r1 = mbar_try_wait(raw_bar, raw_par), r2 = g < L || mbar_try_wait(lo_bar, lo_par);
         ok = (r1 || mbar_wait(raw_bar, raw_par, abort_flag, kWaitRawTile)) && (r2 || mbar_wait(lo_bar, lo_par, abort_flag, kWaitLoSlot));
@@ -514,11 +515,11 @@ __device__ __forceinline__ void tc2r_run(const P &p, const StallCtl &ctl, unsign
       // Two warps take alternate k tiles (and with them alternate accumulator buffers): while one is blocked on
       // the tensor pipe's queue the other sits through its barrier polls, each a shared-memory round trip of
       // hundreds of cycles under the MMAs' own traffic.
-      // With an odd number of hi slots a thread meets a slot only every second time round, so its parity wait for
+      // With an odd number of hi slots a warp meets a slot only every second time round, so its parity wait for
       // tile g sees the phase of tile g - 2R as "the previous one".  That is safe because the phase of tile g - R
-      // is over by then: the thread has waited for tile g - 2, which was split only after the MMAs of tile g - 5
+      // is over by then: the warp has waited for tile g - 2, which was split only after the MMAs of tile g - 5
       // released its lo slot (three lo slots), and R = 5 is the only odd ring size in use (static_assert below).
-      // A scheme in which a thread skips whole revolutions (alternate ITEMS instead of alternate tiles) loses that
+      // A scheme in which a warp skips whole revolutions (alternate ITEMS instead of alternate tiles) loses that
       // guarantee and stalls.
       constexpr bool A_MN = P::OpA::MN_MAJOR, B_MN = P::OpB::MN_MAJOR;
       constexpr uint32_t idesc = umma2_idesc_tf32(BN2, A_MN, B_MN);
